@@ -135,7 +135,7 @@ struct AttnPrefillParams {
 };
 void attention_prefill_launch(const AttnPrefillParams& p, cudaStream_t stream);
 // tcgen05 / TMEM / TMA flash attention (attention_tc.cu), head_dim 128
-void attention_prefill_tc_launch(const void* q, const void* k, const void* v, void* out, const float* sinks, int B, int T, int Hq, int Hkv,
+void attention_prefill_tc_launch(const void* q, const void* k, const void* v, void* out, const float* sinks, int B, int T, int Hq, int Hkv, int D,
                                  float scale, int causal, int window, float softcap, cudaStream_t stream);
 
 // W8A8 fp8 path: dynamic per-token activation quantisation (quant.cu) + tcgen05 kind::f8f6f4 GEMM (gemm_tcgen05.cu)

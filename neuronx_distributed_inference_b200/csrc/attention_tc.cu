@@ -1,40 +1,59 @@
-// Flash attention (prefill) on the 5th-generation tensor cores: S = Q K^T and O += P V are tcgen05.mma instructions with their
-// accumulators in TENSOR MEMORY; Q / K / V tiles arrive through TMA (cp.async.bulk.tensor, SWIZZLE_128B); the softmax owns one
-// query row per thread (tcgen05.ld of its TMEM lane), so no cross-thread reductions exist anywhere.
+// Flash attention over prompts on the 5th-generation tensor cores: S = Q K^T and O += P V are tcgen05.mma instructions whose accumulators
+// AND whose probabilities live in TENSOR MEMORY; Q / K / V tiles arrive through TMA (SWIZZLE_128B); the softmax owns one query row per
+// thread (tcgen05.ld of its TMEM lane), so no cross-thread reductions exist anywhere.
 //
-//   CTA = one (batch, q head, 128-query tile).  192 threads: warp 0 = TMA producer, warp 1 = MMA issuer (one thread),
-//   warps 2..5 = softmax / correction / epilogue (TMEM lane quarter = warp % 4).
-//   per 128-key tile j:   S_j = Q K_j^T          8 x UMMA 128x128x16 (K-major A = Q, K-major B = K_j)        -> TMEM cols [0,128)
-//                         P_j = exp2(S_j*c - m)  registers -> bf16 -> shared memory (128B-swizzled, K-major A operand)
-//                         O  += P_j V_j          8 x UMMA 128x128x16 (B = V_j in its natural [key][d] layout = MN-major) -> TMEM cols [128,256)
-//   The running maximum is LAZY (FlashAttention-4 style): O and l are rescaled only when a row's maximum grows by more than 2^8,
-//   decided per warp, so the TMEM read-modify-write of O happens on a handful of tiles instead of all of them.
-//   S_{j+1} is issued right after P_j V_j, so the tensor pipe works on the next scores while the softmax of tile j+1 ... runs on
-//   the CUDA cores (single S / P buffers: the pipeline is MMA -> softmax -> MMA with the QK^T of the next tile overlapped).
-// Masks are arguments: causal, sliding window, bidirectional (causal = 0), per-head sink logit, tanh soft-cap.
+//   CTA = two 128-query tiles of one batch row that read the same keys: the same queries of two neighbouring q heads of a kv head (grouped
+//   heads), or 256 consecutive queries of one head.  384 threads: warps 0-3 softmax of tile a, warps 4-7 softmax of tile b, warp 8 MMA
+//   issuer (one thread), warp 9 TMA producer, warp 10 zeroes the value rows past the end of a paged row (see below).
+//   per 128-key tile j and query tile x:
+//     S_x = Q_x K_j^T     D/16 x UMMA 128x128x16 (shared-memory operands)                      -> TMEM cols [128 x, 128 x + 128)
+//     P_x = exp2(S_x c - m)   registers -> bf16 -> TMEM, over the first half of S_x (a thread has read its whole row before)
+//     O_x += P_x V_j      8 x UMMA 128xDx16 with A = P_x from TMEM, B = V_j in its natural [key][d] layout = MN-major
+//   The two query tiles take turns: while one is in its softmax the tensor pipe works on P V and the next Q K^T of the other.
+//   What bounds it: per pair of tiles (head size 128) the tensor pipe, the exponentials (16 per clock and SM) and shared memory each need
+//   about 2048 clocks; measured about 4400 (both pipes half busy: the chain scores -> softmax -> P V of a tile is longer than the turn of
+//   the other).  One 8192-token prompt, 32 / 8 heads x 128: 0.50 ms (1.1 PFLOP/s); the kernel before this one, one query tile per CTA with P
+//   through shared memory, took 0.95 ms.  Head size 64, 3 x 1000 tokens, window 128: 30 us against 55 us of the mma.sync kernel.
+//   Tried and slower: signalling P in two 64-key halves with the row sum after the second (0.53 ms: the sum no longer hides behind the
+//   exponentials); one query tile per CTA, 256 threads (0.59 ms).
+//   The running maximum is lazy: O and l are rescaled only when a row's maximum grows by more than 2^8, decided per warp, by the softmax
+//   warps themselves: S_j was issued after P V_{j-1}, so "S_j is complete" says that O is quiescent.
+//
+// Keys come from contiguous [B, T, Hkv, D] tensors or from a PAGED cache [blocks, page, Hkv, D] (page a power of two >= 8: a 128-key tile is
+// 128 / page boxes, whose 1024-byte swizzle atoms line up).  Pages past the last visible key are not fetched, and the rows after it in the
+// last tile are zeroed in shared memory before P V: probability 0 times whatever an unwritten cache row holds must stay 0.
+// Masks are arguments: causal or bidirectional, sliding window with kept first tokens, chunks, per-head sink logit, tanh soft cap.
 // reference kernel contract: attention_cte / flash_fwd (modules/attention/attention_base.py:603-630,722-744).
+#include <algorithm>
 #include <cfloat>
 #include <stdexcept>
 #include <string>
 
 #include "api.h"
 #include "common.cuh"
+#include "seqmix.h"
 
 namespace nxdi {
 
-constexpr int FA_BM = 128, FA_BN = 128, FA_D = 128;
-constexpr int FA_THREADS = 192;
-constexpr int FA_KV_STAGES = 2;
-constexpr int FA_TILE_BYTES = 128 * 128 * 2;   // one [128 rows][128 cols] bf16 tile = two 16 KB halves of 64 columns
+constexpr int FA_ROWS = 128;                   // queries per tile = keys per tile
+constexpr int FA_THREADS = 384;
 constexpr float FA_LOG2E = 1.4426950408889634f;
 
 struct FaParams {
-  CUtensorMap tm_q, tm_k, tm_v;   // 2-D views [B*T rows, H*D cols]; box {64, 128}, SWIZZLE_128B
-  __nv_bfloat16* out;             // [B, T, Hq, D]
-  const float* sinks;             // [Hq] or null
-  int B, T, Hq, Hkv, causal, window;
-  float scale_log2, softcap;
+  CUtensorMap tm_q, tm_k, tm_v, tm_o;   // q / o (and contiguous k / v): 4-D {D, heads, T, B}; paged k / v: 3-D {D, kv heads, slots}; boxes of 64 columns
+  const float* sinks;                   // [Hq] or null
+  const float* head_scale;              // [Hq] or null: a further factor of the scores of a head
+  const __nv_bfloat16* gate;            // [B, T, Hq * D] (or [B, T, Hq] with gate_per_head) with the strides below, or null
+  long long g_sb, g_st;
+  __nv_bfloat16* out;                   // [B, T, Hq, D]
+  const int *ctx_len, *q_len, *block_table;   // paged rows
+  int max_blocks, page_shift;
+  int gate_per_head, gate_vec;
+  int B, T, Hq, Hkv, causal, window, keep, chunk, pair_heads;
+  float scale, softcap;
 };
+
+__device__ unsigned fa_gave_up;         // waits that ran out (a protocol error; the results of that launch are not valid)
 
 __device__ __forceinline__ uint32_t fa_s32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void fa_mb_init(uint64_t* b, uint32_t n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(fa_s32(b)), "r"(n)); }
@@ -42,16 +61,34 @@ __device__ __forceinline__ void fa_mb_expect(uint64_t* b, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fa_s32(b)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void fa_mb_arrive(uint64_t* b) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(fa_s32(b)) : "memory"); }
-__device__ __forceinline__ void fa_mb_wait(uint64_t* b, uint32_t parity) {
-  uint32_t ok = 0;
-  while (!ok) {
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(fa_s32(b)), "r"(parity) : "memory");
-  }
+__device__ __forceinline__ bool fa_mb_try(uint64_t* b, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(fa_s32(b)), "r"(parity) : "memory");
+  return ok != 0u;
 }
-__device__ __forceinline__ void fa_tma_2d(void* dst, const CUtensorMap* tm, int c0, int c1, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(fa_s32(dst)),
-               "l"(tm), "r"(c0), "r"(c1), "r"(fa_s32(bar)) : "memory");
+// Bounded wait: after the limit (seconds) every role of the CTA stops waiting, issues no further copies or MMAs and runs to its end.
+__device__ __forceinline__ bool fa_mb_wait(uint64_t* b, uint32_t parity, volatile int* stop) {
+  if (fa_mb_try(b, parity)) return true;
+  for (int n = 0; n < (1 << 22); ++n) {
+    if (fa_mb_try(b, parity)) return true;
+    if (*stop) return false;
+  }
+  *stop = 1;
+  atomicAdd(&fa_gave_up, 1u);
+  return false;
+}
+__device__ __forceinline__ void fa_tma_4d(void* dst, const CUtensorMap* tm, int c0, int c1, int c2, int c3, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(fa_s32(dst)),
+               "l"(tm), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(fa_s32(bar)) : "memory");
+}
+__device__ __forceinline__ void fa_tma_3d(void* dst, const CUtensorMap* tm, int c0, int c1, int c2, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(fa_s32(dst)),
+               "l"(tm), "r"(c0), "r"(c1), "r"(c2), "r"(fa_s32(bar)) : "memory");
+}
+__device__ __forceinline__ void fa_tma_store_4d(const CUtensorMap* tm, const void* src, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(tm), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
+               "r"(fa_s32(src)) : "memory");
 }
 // K-major operand tile [rows][64 cols] of 128-byte rows, SWIZZLE_128B: 8-row groups 1024 B apart
 __device__ __forceinline__ uint64_t fa_desc_kmajor(const void* smem) {
@@ -69,24 +106,28 @@ __device__ __forceinline__ uint64_t fa_desc_kmajor(const void* smem) {
 __device__ __forceinline__ uint64_t fa_desc_mnmajor(const void* smem) {
   uint64_t d = 0;
   d |= (uint64_t)((fa_s32(smem) & 0x3FFFF) >> 4);
-  d |= (uint64_t)((FA_TILE_BYTES / 2) >> 4) << 16;   // leading byte offset: next 64-element block along MN
+  d |= (uint64_t)((FA_ROWS * 128) >> 4) << 16;       // leading byte offset: next 64-element block along MN
   d |= (uint64_t)(1024 >> 4) << 32;                  // stride byte offset: next 8-row (key) group
   d |= (uint64_t)1 << 46;
   d |= (uint64_t)2 << 61;
   return d;
 }
-// instruction descriptor: D = f32, A = B = bf16, M = 128, N = 128; bit 16 = B is MN-major
-__host__ __device__ constexpr uint32_t fa_idesc(bool b_mn_major) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn_major ? (1u << 16) : 0u) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+// instruction descriptor: D = f32, A = B = bf16, M = 128; bit 16 = B is MN-major
+__host__ __device__ constexpr uint32_t fa_idesc(int n, bool b_mn_major) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn_major ? (1u << 16) : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 __device__ __forceinline__ void fa_umma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
                "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
 }
+__device__ __forceinline__ void fa_umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+               "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc) : "memory");
+}
 __device__ __forceinline__ void fa_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(fa_s32(bar)) : "memory");
 }
-__device__ __forceinline__ void fa_tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+__device__ __forceinline__ void fa_tmem_ld32(uint32_t taddr, uint32_t* v) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
@@ -96,7 +137,7 @@ __device__ __forceinline__ void fa_tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) 
         "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
       : "r"(taddr));
 }
-__device__ __forceinline__ void fa_tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+__device__ __forceinline__ void fa_tmem_st32(uint32_t taddr, const uint32_t* v) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
       "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
@@ -107,292 +148,499 @@ __device__ __forceinline__ void fa_tmem_st32(uint32_t taddr, const uint32_t (&v)
       : "memory");
 }
 
+__device__ __forceinline__ float fa_ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// two fp32 operations per instruction
+__device__ __forceinline__ uint64_t fa_pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(__float_as_uint(a)), "r"(__float_as_uint(b)));
+  return r;
+}
+__device__ __forceinline__ void fa_unpack2(uint64_t v, float& a, float& b) {
+  uint32_t x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(x), "=r"(y) : "l"(v));
+  a = __uint_as_float(x);
+  b = __uint_as_float(y);
+}
+__device__ __forceinline__ uint64_t fa_fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t fa_mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fa_add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// tanh on |x| <= 1: x times a polynomial in x^2 (weighted least squares on Chebyshev nodes, relative error 1.7e-7 with fp32 arithmetic);
+// beyond: 1 - 2 / (e^2x + 1)
+__device__ __forceinline__ uint64_t fa_tanh2_small(uint64_t x) {
+  const uint64_t u = fa_mul2(x, x);
+  uint64_t r = fa_pack2(0.00104102155f, 0.00104102155f);
+  r = fa_fma2(r, u, fa_pack2(-0.00620337576f, -0.00620337576f));
+  r = fa_fma2(r, u, fa_pack2(0.0202899761f, 0.0202899761f));
+  r = fa_fma2(r, u, fa_pack2(-0.0534570292f, -0.0534570292f));
+  r = fa_fma2(r, u, fa_pack2(0.13325204f, 0.13325204f));
+  r = fa_fma2(r, u, fa_pack2(-0.333328396f, -0.333328396f));
+  r = fa_fma2(r, u, fa_pack2(0.99999994f, 0.99999994f));
+  return fa_mul2(x, r);
+}
+__device__ __forceinline__ float fa_tanh_any(float x) { return 1.f - __fdividef(2.f, __expf(2.f * x) + 1.f); }
+
+template <int D, bool PAGED, bool CAP>
 __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(const __grid_constant__ FaParams p) {
+  constexpr int TILE = FA_ROWS * D * 2;                  // bytes of a [128][D] tile: D / 64 blocks of [128 rows][128 bytes]
+  constexpr int HALF = FA_ROWS * 128;
+  constexpr int SLOTS = D == 128 ? 5 : 8;                // K and V tiles share one ring: K0 V0 K1 V1 ...
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = smem_raw + ((1024u - (fa_s32(smem_raw) & 1023u)) & 1023u);
-  uint8_t* sQ = smem;                                    // [2 d-halves][128 q][64 d]
-  uint8_t* sK = sQ + FA_TILE_BYTES;                      // [stages][2 d-halves][128 keys][64 d]
-  uint8_t* sV = sK + FA_KV_STAGES * FA_TILE_BYTES;       // [stages][2 d-halves][128 keys][64 d]
-  uint8_t* sP = sV + FA_KV_STAGES * FA_TILE_BYTES;       // [2 key-halves][128 q][64 keys]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + FA_TILE_BYTES);
-  uint64_t* q_full = bars;                 // 1
-  uint64_t* kv_full = bars + 1;            // [stages]  K and V of a stage landed
-  uint64_t* kv_empty = kv_full + FA_KV_STAGES;   // [stages]  P V of the stage retired
-  uint64_t* s_full = kv_empty + FA_KV_STAGES;    // S_j complete
-  uint64_t* p_full = s_full + 1;           // P_j written (and O rescaled): 4 softmax warps arrive
-  uint64_t* pv_done = p_full + 1;          // P_j V_j retired: P buffer and O accumulator are quiescent
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 1);
-
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_qt = (p.T + FA_BM - 1) / FA_BM;
-  const int qt = n_qt - 1 - (int)(blockIdx.x % n_qt);      // heavy (late) query tiles first
-  const int bh = blockIdx.x / n_qt;
-  const int b = bh / p.Hq, h = bh % p.Hq, hk = h / (p.Hq / p.Hkv);
-  const int q0 = qt * FA_BM;
-  // key tiles this query tile attends to
-  int j_hi = p.causal ? qt : (p.T + FA_BN - 1) / FA_BN - 1;
-  j_hi = min(j_hi, (p.T + FA_BN - 1) / FA_BN - 1);
-  int j_lo = 0;
-  if (p.window > 0) j_lo = max(0, q0 - p.window + 1) / FA_BN;
-  const int n_tiles = j_hi - j_lo + 1;
 
-  if (warp == 0 && lane == 0) {
+  uint8_t* smem = smem_raw + ((1024u - (fa_s32(smem_raw) & 1023u)) & 1023u);
+  uint8_t* sQ = smem;                                    // [2 tiles]; the outputs are staged here at the end
+  uint8_t* sKV = sQ + 2 * TILE;                          // [SLOTS]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + SLOTS * TILE);
+  uint64_t* q_full = bars;
+  uint64_t* kv_full = bars + 1;                          // [SLOTS]
+  uint64_t* kv_empty = kv_full + SLOTS;                  // [SLOTS]
+  uint64_t* s_full = kv_empty + SLOTS;                   // [2] S_x complete (and P V of the tile before retired)
+  uint64_t* p_full = s_full + 2;                         // [2] P_x written and O_x rescaled: four warps arrive
+  uint64_t* o_full = p_full + 2;                         // [2]
+  uint64_t* v_landed = o_full + 2;                       // the last value tile is there
+  uint64_t* v_clean = v_landed + 1;                      // its rows past the end are zeroed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_clean + 1);
+  volatile int* stop = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  if (warp == 9 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_q) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_k) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_v) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_o) : "memory");
     fa_mb_init(q_full, 1);
-    for (int s = 0; s < FA_KV_STAGES; ++s) {
+    for (int s = 0; s < SLOTS; ++s) {
       fa_mb_init(&kv_full[s], 1);
       fa_mb_init(&kv_empty[s], 1);
     }
-    fa_mb_init(s_full, 1);
-    fa_mb_init(p_full, 4);
-    fa_mb_init(pv_done, 1);
+    for (int x = 0; x < 2; ++x) {
+      fa_mb_init(&s_full[x], 1);
+      fa_mb_init(&p_full[x], 4);
+      fa_mb_init(&o_full[x], 1);
+    }
+    fa_mb_init(v_landed, 1);
+    fa_mb_init(v_clean, 1);
+    *stop = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(fa_s32(tmem_slot)), "n"(256));
+  if (warp == 8) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(fa_s32(tmem_slot)), "n"(512));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + 128;
-
+  const uint32_t tmem = *tmem_slot;
   pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait();               // from here on: what earlier kernels wrote
 
-  if (warp == 0) {
-    // ================= TMA producer =================
-    if (lane == 0) {
-      const int row_q = b * p.T + q0, colq = h * FA_D, colk = hk * FA_D;
-      fa_mb_expect(q_full, FA_TILE_BYTES);
-      fa_tma_2d(sQ, &p.tm_q, colq, row_q, q_full);
-      fa_tma_2d(sQ + FA_TILE_BYTES / 2, &p.tm_q, colq + 64, row_q, q_full);
-      for (int i = 0; i < n_tiles; ++i) {
-        const int s = i % FA_KV_STAGES;
-        const uint32_t ph = (uint32_t)((i / FA_KV_STAGES) & 1);
-        fa_mb_wait(&kv_empty[s], ph ^ 1u);
-        fa_mb_expect(&kv_full[s], 2 * FA_TILE_BYTES);
-        const int row_k = b * p.T + (j_lo + i) * FA_BN;
-        fa_tma_2d(sK + s * FA_TILE_BYTES, &p.tm_k, colk, row_k, &kv_full[s]);
-        fa_tma_2d(sK + s * FA_TILE_BYTES + FA_TILE_BYTES / 2, &p.tm_k, colk + 64, row_k, &kv_full[s]);
-        fa_tma_2d(sV + s * FA_TILE_BYTES, &p.tm_v, colk, row_k, &kv_full[s]);
-        fa_tma_2d(sV + s * FA_TILE_BYTES + FA_TILE_BYTES / 2, &p.tm_v, colk + 64, row_k, &kv_full[s]);
-      }
+  // ---- which queries: heavy (late) tiles first
+  const int n_hp = p.pair_heads ? p.Hq / 2 : p.Hq;
+  const int span = p.pair_heads ? FA_ROWS : 2 * FA_ROWS;
+  const int n_qt = (p.T + span - 1) / span;
+  const int per_qt = p.B * n_hp;
+  const int qt = n_qt - 1 - (int)(blockIdx.x / per_qt);
+  const int bh = blockIdx.x % per_qt, b = bh / n_hp, hp = bh % n_hp;
+  const int q0 = qt * span;
+  const int qn = PAGED ? min(p.q_len[b], p.T) : p.T, ctx = PAGED ? p.ctx_len[b] : 0;
+  if (PAGED && q0 >= qn) {                               // padding queries: zeros
+    const int rows = min(span, p.T - q0), heads = p.pair_heads ? 2 : 1, h0 = hp * heads;
+    for (int i = threadIdx.x; i < rows * heads * (D / 8); i += FA_THREADS) {
+      const int r = i / (heads * (D / 8)), c = i % (heads * (D / 8));
+      *reinterpret_cast<uint4*>(p.out + (((long long)b * p.T + q0 + r) * p.Hq + h0) * D + c * 8) = make_uint4(0u, 0u, 0u, 0u);
     }
-  } else if (warp == 1) {
-    // ================= MMA issuer =================
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = fa_idesc(false), idesc_pv = fa_idesc(true);
-      fa_mb_wait(q_full, 0);
-      auto issue_s = [&](int i) {   // S_i = Q K_i^T
-        const int s = i % FA_KV_STAGES;
-        fa_mb_wait(&kv_full[s], (uint32_t)((i / FA_KV_STAGES) & 1));
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-        for (int k = 0; k < FA_D / 16; ++k) {
-          // 16 d = 32 bytes inside the 128-byte swizzle atom; the second 64-d half is a separate 16 KB block
-          const uint64_t da = fa_desc_kmajor(sQ + (k >> 2) * (FA_TILE_BYTES / 2)) + (uint64_t)((k & 3) * 2);
-          const uint64_t db = fa_desc_kmajor(sK + s * FA_TILE_BYTES + (k >> 2) * (FA_TILE_BYTES / 2)) + (uint64_t)((k & 3) * 2);
-          fa_umma(tmem_S, da, db, idesc_qk, k != 0 ? 1u : 0u);
-        }
-        fa_commit(s_full);
+    if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512));
+    return;
+  }
+  const int h_first = p.pair_heads ? 2 * hp : hp, hk = h_first / (p.Hq / p.Hkv);
+  // ---- which keys: the kept first tokens below the window's reach (whole tiles), then [lo, hi]
+  const int p_first = ctx + q0, p_last = ctx + min(q0 + span, qn) - 1;
+  const int hi = p.causal ? p_last : qn - 1, end = hi + 1;
+  const int lo = p.window > 0 ? max(p_first - p.window + 1, 0) : p.chunk > 0 ? p_first / p.chunk * p.chunk : 0;
+  const int keep = p.window > 0 ? p.keep : 0;
+  const int t_lo = lo / FA_ROWS, nA = min((keep + FA_ROWS - 1) / FA_ROWS, t_lo);
+  const int n_tiles = nA + hi / FA_ROWS - t_lo + 1;
+  auto key_at = [&](int i) { return (i < nA ? i : t_lo + i - nA) * FA_ROWS; };
+  const bool dirty_end = PAGED && (end & (FA_ROWS - 1)) != 0;
+
+  if (warp >= 8) {
+    // registers: 384 threads x 168 at launch = 256 x 208 + 128 x 88
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    if (warp == 9) {
+      // ================= TMA producer =================
+      const int pieces = PAGED ? max(1, FA_ROWS >> p.page_shift) : 1;    // boxes per 64-column block
+      const int piece_rows = FA_ROWS / pieces;
+      const int* table = PAGED ? p.block_table + (long long)b * p.max_blocks : nullptr;
+      auto slot_at = [&](int key0) {                     // lane l: cache slot of the first key of piece l
+        const int k = key0 + lane * piece_rows;
+        if (!PAGED || lane >= pieces || k >= end) return 0;
+        const int pi = min(k >> p.page_shift, p.max_blocks - 1);
+        return (table[pi] << p.page_shift) + (k & ((1 << p.page_shift) - 1));
       };
-      issue_s(0);
-      for (int i = 0; i < n_tiles; ++i) {
-        const int s = i % FA_KV_STAGES;
-        fa_mb_wait(p_full, (uint32_t)(i & 1));     // P_i in shared memory, O rescaled, S_i fully read
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-        for (int k = 0; k < FA_BN / 16; ++k) {
-          // A = P: 16 keys = 32 bytes inside the atom, second 64-key half 16 KB further.
-          // B = V (MN-major): 16 keys = 16 rows of 128 bytes = 2048 bytes further in BOTH d halves (LBO covers the halves)
-          const uint64_t da = fa_desc_kmajor(sP + (k >> 2) * (FA_TILE_BYTES / 2)) + (uint64_t)((k & 3) * 2);
-          const uint64_t db = fa_desc_mnmajor(sV + s * FA_TILE_BYTES + k * 2048);
-          fa_umma(tmem_O, da, db, idesc_pv, (i | k) != 0 ? 1u : 0u);
+      if (lane == 0) {
+        fa_mb_expect(q_full, 2 * TILE);
+        for (int x = 0; x < 2; ++x)
+          for (int c = 0; c < D / 64; ++c)
+            fa_tma_4d(sQ + x * TILE + c * HALF, &p.tm_q, c * 64, p.pair_heads ? h_first + x : h_first, p.pair_heads ? q0 : q0 + x * FA_ROWS, b, q_full);
+      }
+      int next = slot_at(key_at(0));
+      bool go = true;
+      for (int i = 0; i < n_tiles && go; ++i) {
+        const int key0 = key_at(i), cur = next;
+        if (i + 1 < n_tiles) next = slot_at(key_at(i + 1));
+        const int live = PAGED ? min(pieces, (end - key0 + piece_rows - 1) / piece_rows) : 1;
+        for (int v = 0; v < 2 && go; ++v) {
+          const int it = 2 * i + v, s = it % SLOTS;
+          go = fa_mb_wait(&kv_empty[s], (uint32_t)((it / SLOTS) & 1) ^ 1u, stop);
+          go = __shfl_sync(0xffffffffu, (int)go, 0) != 0;
+          if (!go) break;
+          uint8_t* dst = sKV + s * TILE;
+          const CUtensorMap* tm = v ? &p.tm_v : &p.tm_k;
+          if (lane == 0) fa_mb_expect(&kv_full[s], (uint32_t)(live * piece_rows * D * 2));
+          if (PAGED) {
+            for (int u = 0; u < live; ++u) {
+              const int row = __shfl_sync(0xffffffffu, cur, u);
+              if (lane == 0)
+                for (int c = 0; c < D / 64; ++c) fa_tma_3d(dst + c * HALF + u * piece_rows * 128, tm, c * 64, hk, row, &kv_full[s]);
+            }
+          } else if (lane == 0) {
+            for (int c = 0; c < D / 64; ++c) fa_tma_4d(dst + c * HALF, tm, c * 64, hk, key0, b, &kv_full[s]);
+          }
         }
-        fa_commit(&kv_empty[s]);      // K_i / V_i stage reusable once these retire
-        fa_commit(pv_done);           // P buffer / O accumulator quiescent
-        if (i + 1 < n_tiles) issue_s(i + 1);
+      }
+    } else if (warp == 8) {
+      // ================= MMA issuer =================
+      if (lane == 0) {
+        constexpr uint32_t idesc_qk = fa_idesc(128, false), idesc_pv = fa_idesc(D, true);
+        auto issue_s = [&](int x, int i) {               // S_x = Q_x K_i^T
+          const uint8_t* k = sKV + ((2 * i) % SLOTS) * TILE;
+#pragma unroll
+          for (int c = 0; c < D / 16; ++c) {
+            // 16 d = 32 bytes inside the 128-byte swizzle atom; the second 64-d half is a separate 16 KB block
+            const uint64_t da = fa_desc_kmajor(sQ + x * TILE + (c >> 2) * HALF) + (uint64_t)((c & 3) * 2);
+            const uint64_t db = fa_desc_kmajor(k + (c >> 2) * HALF) + (uint64_t)((c & 3) * 2);
+            fa_umma(tmem + 128 * x, da, db, idesc_qk, c != 0 ? 1u : 0u);
+          }
+          fa_commit(&s_full[x]);
+        };
+        auto full = [&](int it) { return fa_mb_wait(&kv_full[it % SLOTS], (uint32_t)((it / SLOTS) & 1), stop); };
+        bool go = fa_mb_wait(q_full, 0, stop) && full(0);
+        if (go) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          issue_s(0, 0);
+          issue_s(1, 0);
+          fa_commit(&kv_empty[0]);
+        }
+        for (int i = 0; i < n_tiles && go; ++i) {
+          const bool more = i + 1 < n_tiles;
+          go = full(2 * i + 1);
+          if (go && dirty_end && !more) {
+            fa_mb_arrive(v_landed);
+            go = fa_mb_wait(v_clean, 0, stop);
+          }
+          for (int x = 0; x < 2 && go; ++x) {
+            go = fa_mb_wait(&p_full[x], (uint32_t)(i & 1), stop);       // P_x in TMEM, O_x rescaled, S_x fully read
+            if (!go) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint8_t* v = sKV + ((2 * i + 1) % SLOTS) * TILE;
+#pragma unroll
+            for (int c = 0; c < FA_ROWS / 16; ++c)
+              // A = P: 16 keys = 8 TMEM columns; B = V (MN-major): 16 keys = 16 rows of 128 bytes further in all blocks
+              fa_umma_ts(tmem + 256 + 128 * x, tmem + 128 * x + 8 * c, fa_desc_mnmajor(v + c * 2048), idesc_pv, (i | c) != 0 ? 1u : 0u);
+            if (x == 1) fa_commit(&kv_empty[(2 * i + 1) % SLOTS]);
+            if (more) {
+              if (x == 0) go = full(2 * i + 2);
+              if (!go) break;
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              issue_s(x, i + 1);
+              if (x == 1) fa_commit(&kv_empty[(2 * i + 2) % SLOTS]);
+            } else {
+              fa_commit(&o_full[x]);
+            }
+          }
+        }
+      }
+    } else if (warp == 10 && dirty_end) {
+      // ================= value rows past the last key of the last tile =================
+      const int valid = end - key_at(n_tiles - 1);
+      if (fa_mb_wait(v_landed, 0, stop)) {
+        uint8_t* v = sKV + ((2 * n_tiles - 1) % SLOTS) * TILE;
+        for (int c = lane; c < (FA_ROWS - valid) * 8; c += 32)
+#pragma unroll
+          for (int hf = 0; hf < D / 64; ++hf) *reinterpret_cast<uint4*>(v + hf * HALF + valid * 128 + c * 16) = make_uint4(0u, 0u, 0u, 0u);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) fa_mb_arrive(v_clean);
       }
     }
   } else {
-    // ================= softmax / correction / epilogue: one query row per thread =================
-    const int q = warp & 3;
-    const int r = q * 32 + lane;                  // row inside the tile = TMEM lane
-    const int qi = q0 + r;                        // query index inside the sequence
-    const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
+    // ================= softmax / rescale / epilogue: one query row per thread =================
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    const int x = warp >> 2, qd = warp & 3;
+    const int r = qd * 32 + lane;                        // row inside the tile = TMEM lane
+    const int t_tile = p.pair_heads ? q0 : q0 + x * FA_ROWS;
+    const int h = p.pair_heads ? h_first + x : h_first;
+    const int t = t_tile + r, pos = ctx + t;             // token of the batch row, position in the sequence
+    const uint32_t lanes = (uint32_t)(qd * 32) << 16;
+    const uint32_t tS = tmem + 128 * x + lanes, tO = tmem + 256 + 128 * x + lanes;
+    const int up = p.causal ? min(pos, end - 1) : end - 1;
+    const int lb = p.window > 0 ? pos - p.window + 1 : p.chunk > 0 ? pos / p.chunk * p.chunk : 0;
+    // tile-uniform bounds of the mask test: every row sees [lb_max, up_min]
+    const int up_min = p.causal ? min(ctx + t_tile, end - 1) : end - 1;
+    const int lb_max = p.window > 0 ? ctx + t_tile + FA_ROWS - p.window : p.chunk > 0 ? (ctx + t_tile + FA_ROWS - 1) / p.chunk * p.chunk : 0;
+    const float hs = p.head_scale ? p.scale * p.head_scale[h] : p.scale;
     float m_run = -INFINITY, l_run = 0.f;
-    const float sc = p.scale_log2;
     for (int i = 0; i < n_tiles; ++i) {
-      const int key0 = (j_lo + i) * FA_BN;
-      fa_mb_wait(s_full, (uint32_t)(i & 1));
+      const int key0 = key_at(i);
+      if (!fa_mb_wait(&s_full[x], (uint32_t)(i & 1), stop)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // ---- the whole S row of this thread -> registers (ONE TMEM read; 128 fp32)
-      uint32_t v[4][32];
+      uint32_t v[128];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) fa_tmem_ld32(tmem_S + lane_sel + 32 * c, v[c]);
+      for (int c = 0; c < 4; ++c) fa_tmem_ld32(tS + 32 * c, v + 32 * c);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      float scl = sc;
-      if (p.softcap > 0.f) {   // tanh soft-cap: scores move to the log2 domain here, the scale below becomes 1
+      float scl = hs * FA_LOG2E;                         // scores -> log2 domain
+      if (CAP) {
+        const float to_cap = hs / p.softcap;
+        float big = 0.f;
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int e = 0; e < 128; ++e) big = fmaxf(big, fabsf(__uint_as_float(v[e])));
+        if (!__any_sync(0xffffffffu, !(big * fabsf(to_cap) <= 1.f))) {
+          const uint64_t tc2 = fa_pack2(to_cap, to_cap);
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            v[c][e] = __float_as_uint(p.softcap * tanhf(__uint_as_float(v[c][e]) * (sc / FA_LOG2E) / p.softcap) * FA_LOG2E);
+          for (int e = 0; e < 128; e += 2) {
+            float a, c;
+            fa_unpack2(fa_tanh2_small(fa_mul2(fa_pack2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), tc2)), a, c);
+            v[e] = __float_as_uint(a);
+            v[e + 1] = __float_as_uint(c);
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 128; ++e) v[e] = __float_as_uint(fa_tanh_any(__uint_as_float(v[e]) * to_cap));
+        }
+        scl = p.softcap * FA_LOG2E;
+      } else if (!(scl > 0.f)) {                         // a head's factor may be zero or negative: the maximum below needs a positive scale
+#pragma unroll
+        for (int e = 0; e < 128; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * scl);
         scl = 1.f;
       }
-      // masks only where a tile can contain invisible keys (sequence end, causal diagonal, window edge): CTA-uniform test
-      const bool need_mask = (key0 + FA_BN > p.T) || (p.causal && key0 + FA_BN - 1 > q0) || (p.window > 0 && key0 <= q0 + FA_BM - 1 - p.window);
-      if (need_mask) {
+      // masks only where a tile can contain invisible keys: uniform test
+      if (key0 + FA_ROWS - 1 > up_min || (key0 < lb_max && key0 + FA_ROWS > keep)) {
+        const int e_hi = up - key0, e_lo = lb - key0, e_keep = keep - key0;
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const int kj = key0 + 32 * c + e;
-            const bool ok = kj < p.T && (!p.causal || kj <= qi) && (p.window <= 0 || kj > qi - p.window);
-            if (!ok) v[c][e] = 0xff800000u;   // -inf
-          }
+        for (int e = 0; e < 128; ++e)
+          if (!(e <= e_hi && (e >= e_lo || e < e_keep))) v[e] = 0xff800000u;   // -inf
       }
-      // row maximum in the RAW domain (the scale is positive), four independent chains
+      // row maximum in the domain of v (its scale is positive), four independent chains
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
+      for (int e = 0; e < 128; e += 8)
 #pragma unroll
-        for (int e = 0; e < 32; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], __uint_as_float(v[c][e]));
+        for (int c = 0; c < 4; ++c) mx4[c] = fmaxf(mx4[c], fmaxf(__uint_as_float(v[e + 2 * c]), __uint_as_float(v[e + 2 * c + 1])));
       const float mx_raw = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       const float mx = (mx_raw == -INFINITY) ? -INFINITY : mx_raw * scl;
-      // lazy running maximum: move it only when this tile exceeds it by more than 2^8 (decided per warp so that the TMEM
-      // read-modify-write below stays warp-uniform); rows that keep their maximum use alpha = 1
-      float m_new = m_run;
       const bool grow = mx > m_run + 8.f || (m_run == -INFINITY && mx > -INFINITY);
-      if (grow) m_new = mx;
-      const bool any = __any_sync(0xffffffffu, grow);
-      const float alpha = (m_run == -INFINITY) ? 0.f : exp2f(m_run - m_new);
-      // the previous P V must have retired before P is overwritten / O is touched
-      if (i > 0) fa_mb_wait(pv_done, (uint32_t)((i - 1) & 1));
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (any && i > 0) {
+      const float m_new = grow ? mx : m_run;
+      const float alpha = (m_run == -INFINITY) ? 0.f : fa_ex2(m_run - m_new);
+      if (i > 0 && __any_sync(0xffffffffu, grow)) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < FA_D; c0 += 32) {
+        for (int c0 = 0; c0 < D; c0 += 32) {
           uint32_t o[32];
-          fa_tmem_ld32(tmem_O + lane_sel + c0, o);
+          fa_tmem_ld32(tO + c0, o);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
           for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-          fa_tmem_st32(tmem_O + lane_sel + c0, o);
+          fa_tmem_st32(tO + c0, o);
         }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       }
-      l_run *= (grow ? alpha : 1.f);
+      l_run *= alpha;
       m_run = m_new;
-      // ---- P = exp2(s * scale - m) -> bf16 -> shared memory (row r of both 64-key halves, 16-byte chunks XOR-swizzled by r & 7)
+      // ---- P = exp2(v * scl - m) -> bf16 -> TMEM, over the scores
       const float neg_m = (m_run == -INFINITY) ? 0.f : -m_run;
-      float ls4[4] = {0.f, 0.f, 0.f, 0.f};
+      const uint64_t scl2 = fa_pack2(scl, scl), neg2 = fa_pack2(neg_m, neg_m);
+      uint64_t ls[2] = {0ull, 0ull};
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t pk[16];
+      for (int c = 0; c < 2; ++c) {
+        uint32_t pk[32];
 #pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-          const float p0 = exp2f(fmaf(__uint_as_float(v[c][e]), scl, neg_m));        // -inf -> 0
-          const float p1 = exp2f(fmaf(__uint_as_float(v[c][e + 1]), scl, neg_m));
+        for (int e = 0; e < 64; e += 2) {
+          float a, bb;
+          fa_unpack2(fa_fma2(fa_pack2(__uint_as_float(v[64 * c + e]), __uint_as_float(v[64 * c + e + 1])), scl2, neg2), a, bb);
+          const uint32_t w = pack_bf16(fa_ex2(a), fa_ex2(bb));            // -inf -> 0
           // the sum uses the bf16-rounded probabilities, exactly what the tensor core multiplies
-          const uint32_t w = pack_bf16(p0, p1);
-          ls4[(e >> 1) & 3] += bf16lo(w) + bf16hi(w);
+          ls[(e >> 1) & 1] = fa_add2(ls[(e >> 1) & 1], fa_pack2(bf16lo(w), bf16hi(w)));
           pk[e >> 1] = w;
         }
-        const int c0 = 32 * c;
-        uint8_t* rowp = sP + (c0 >> 6) * (FA_TILE_BYTES / 2) + r * 128;
-        const int ch0 = (c0 & 63) >> 3;   // first 16-byte chunk of this 32-key group inside the 128-byte row
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc)
-          *reinterpret_cast<uint4*>(rowp + (((ch0 + cc) ^ (r & 7)) << 4)) = make_uint4(pk[4 * cc], pk[4 * cc + 1], pk[4 * cc + 2], pk[4 * cc + 3]);
+        fa_tmem_st32(tS + 32 * c, pk);
       }
-      const float lsum = (ls4[0] + ls4[1]) + (ls4[2] + ls4[3]);
-      l_run += lsum;
-      // generic-proxy writes of P must be visible to the tensor core (async proxy); S reads are complete
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) fa_mb_arrive(p_full);
+      if (lane == 0) fa_mb_arrive(&p_full[x]);
+      float s0, s1;
+      fa_unpack2(fa_add2(ls[0], ls[1]), s0, s1);
+      l_run += s0 + s1;
     }
-    // ---- epilogue: O / l -> bf16 -> global
-    fa_mb_wait(pv_done, (uint32_t)((n_tiles - 1) & 1));
+    // ---- epilogue: O / l (times the gate) -> bf16 -> shared memory -> TMA store (rows past T are clipped, padding rows are zeros)
+    const bool done = fa_mb_wait(&o_full[x], 0, stop);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     float l = l_run;
-    if (p.sinks != nullptr) {
-      const float sk = p.sinks[h] * FA_LOG2E;
-      l = (m_run == -INFINITY) ? 1.f : l + exp2f(sk - m_run);
+    if (p.sinks != nullptr) l = (m_run == -INFINITY) ? 1.f : l + fa_ex2(p.sinks[h] * FA_LOG2E - m_run);
+    float inv = (m_run == -INFINITY || l == 0.f) ? 0.f : 1.f / l;
+    const bool live_row = t < qn;
+    const __nv_bfloat16* gp = nullptr;
+    if (p.gate != nullptr && live_row) {
+      gp = p.gate + (long long)b * p.g_sb + (long long)t * p.g_st + (p.gate_per_head ? h : h * D);
+      if (p.gate_per_head) inv *= 1.f / (1.f + __expf(-__bfloat162float(*gp)));
     }
-    const float inv = (m_run == -INFINITY || l == 0.f) ? 0.f : 1.f / l;
-    __nv_bfloat16* dst = p.out + (((size_t)b * p.T + qi) * p.Hq + h) * FA_D;
+    uint8_t* so = sQ + x * TILE + r * 128;
 #pragma unroll 1
-    for (int c0 = 0; c0 < FA_D; c0 += 32) {
-      uint32_t v[32];
-      fa_tmem_ld32(tmem_O + lane_sel + c0, v);
+    for (int c0 = 0; c0 < D; c0 += 32) {
+      uint32_t o[32];
+      fa_tmem_ld32(tO + c0, o);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (qi < p.T) {
 #pragma unroll
-        for (int e = 0; e < 32; e += 8) {
-          *reinterpret_cast<uint4*>(dst + c0 + e) =
-              make_uint4(pack_bf16(__uint_as_float(v[e]) * inv, __uint_as_float(v[e + 1]) * inv),
-                         pack_bf16(__uint_as_float(v[e + 2]) * inv, __uint_as_float(v[e + 3]) * inv),
-                         pack_bf16(__uint_as_float(v[e + 4]) * inv, __uint_as_float(v[e + 5]) * inv),
-                         pack_bf16(__uint_as_float(v[e + 6]) * inv, __uint_as_float(v[e + 7]) * inv));
+      for (int e = 0; e < 32; e += 8) {
+        float f[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) f[k] = live_row ? __uint_as_float(o[e + k]) * inv : 0.f;
+        if (gp != nullptr && !p.gate_per_head) {
+          float g[8];
+          if (p.gate_vec) {
+            const uint4 w = ldg_act(gp + c0 + e);
+            g[0] = bf16lo(w.x); g[1] = bf16hi(w.x); g[2] = bf16lo(w.y); g[3] = bf16hi(w.y);
+            g[4] = bf16lo(w.z); g[5] = bf16hi(w.z); g[6] = bf16lo(w.w); g[7] = bf16hi(w.w);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) g[k] = ldg_act_bf16(gp + c0 + e + k);
+          }
+#pragma unroll
+          for (int k = 0; k < 8; ++k) f[k] *= 1.f / (1.f + __expf(-g[k]));
         }
+        const int ch = ((c0 & 63) + e) >> 3;             // 16-byte chunk of the 128-byte row, XOR-swizzled like TMA does
+        *reinterpret_cast<uint4*>(so + (c0 >> 6) * HALF + ((ch ^ (r & 7)) << 4)) =
+            make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + x) : "memory");
+    if (r == 0 && done && t_tile < p.T) {
+      for (int c = 0; c < D / 64; ++c) fa_tma_store_4d(&p.tm_o, sQ + x * TILE + c * HALF, c * 64, h, t_tile, b);
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    }
   }
+  if (*stop) __nanosleep(1000000);        // gave up: let copies in flight land before the shared memory goes away
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 8) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(256));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512));
   }
 }
 
 typedef CUresult (*FaEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static void fa_make_map(CUtensorMap* tm, const void* ptr, long long rows, int cols) {
-  static FaEncodeFn fn = nullptr;
-  if (fn == nullptr) {
+static FaEncodeFn fa_encode_fn() {
+  static FaEncodeFn fn = [] {
     void* q = nullptr;
     cudaDriverEntryPointQueryResult r;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &q, cudaEnableDefault, &r) != cudaSuccess || q == nullptr)
       throw std::runtime_error("cuTensorMapEncodeTiled not available");
-    fn = reinterpret_cast<FaEncodeFn>(q);
-  }
-  cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t gstride[1] = {(cuuint64_t)cols * 2};
-  cuuint32_t box[2] = {64, 128};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return reinterpret_cast<FaEncodeFn>(q);
+  }();
+  return fn;
+}
+// dims / strides in elements of bf16, innermost first (its stride is 1); boxes of 64 columns x `rows` entries of dimension 2
+static void fa_make_map(CUtensorMap* tm, const void* ptr, int rank, const long long* dims, const long long* strides, int rows) {
+  cuuint64_t gdim[4], gstride[3];
+  cuuint32_t box[4] = {64, 1, (cuuint32_t)rows, 1}, estr[4] = {1, 1, 1, 1};
+  for (int i = 0; i < rank; ++i) gdim[i] = (cuuint64_t)dims[i];
+  for (int i = 1; i < rank; ++i) gstride[i - 1] = (cuuint64_t)strides[i] * 2;
+  CUresult r = fa_encode_fn()(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(ptr), gdim, gstride, box, estr,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled (attention) failed: " + std::to_string((int)r));
 }
+static void fa_map_rows(CUtensorMap* tm, const void* ptr, int B, int T, int H, int D) {      // [B, T, H, D]
+  const long long dims[4] = {D, H, T, B}, strides[4] = {1, D, (long long)H * D, (long long)T * H * D};
+  fa_make_map(tm, ptr, 4, dims, strides, FA_ROWS);
+}
 
-// q [B,T,Hq,128], k / v [B,T,Hkv,128] bf16 contiguous -> out [B,T,Hq,128]
-void attention_prefill_tc_launch(const void* q, const void* k, const void* v, void* out, const float* sinks, int B, int T, int Hq, int Hkv,
+template <int D, bool PAGED, bool CAP>
+static void fa_go(FaParams& p, cudaStream_t stream) {
+  constexpr int TILE = FA_ROWS * D * 2, SLOTS = D == 128 ? 5 : 8;
+  const size_t smem = (size_t)(2 + SLOTS) * TILE + 256 + 1024;
+  auto kernel = attention_prefill_tc_kernel<D, PAGED, CAP>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    throw std::runtime_error("attention (tensor cores): shared memory size refused");
+  // grouped heads share their keys two by two; a head of its own takes 256 queries instead
+  p.pair_heads = (p.Hq / p.Hkv) % 2 == 0 ? 1 : 0;
+  const int span = p.pair_heads ? FA_ROWS : 2 * FA_ROWS;
+  const long long blocks = (long long)((p.T + span - 1) / span) * p.B * (p.pair_heads ? p.Hq / 2 : p.Hq);
+  launch_pdl(kernel, dim3((unsigned)blocks), dim3(FA_THREADS), smem, stream, p);
+}
+
+// q [B,T,Hq,D], k / v [B,T,Hkv,D] bf16 contiguous, D = 64 or 128 -> out [B,T,Hq,D]
+void attention_prefill_tc_launch(const void* q, const void* k, const void* v, void* out, const float* sinks, int B, int T, int Hq, int Hkv, int D,
                                  float scale, int causal, int window, float softcap, cudaStream_t stream) {
+  if (B <= 0 || T <= 0) return;
   FaParams p{};
-  fa_make_map(&p.tm_q, q, (long long)B * T, Hq * FA_D);
-  fa_make_map(&p.tm_k, k, (long long)B * T, Hkv * FA_D);
-  fa_make_map(&p.tm_v, v, (long long)B * T, Hkv * FA_D);
+  fa_map_rows(&p.tm_q, q, B, T, Hq, D);
+  fa_map_rows(&p.tm_k, k, B, T, Hkv, D);
+  fa_map_rows(&p.tm_v, v, B, T, Hkv, D);
+  fa_map_rows(&p.tm_o, out, B, T, Hq, D);
   p.out = reinterpret_cast<__nv_bfloat16*>(out);
   p.sinks = sinks;
   p.B = B; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal; p.window = window;
-  p.scale_log2 = scale * FA_LOG2E;
-  p.softcap = softcap;
-  const size_t smem = (size_t)(2 + 2 * FA_KV_STAGES) * FA_TILE_BYTES + 256 + 1024;
-  static bool cfg = false;
-  if (!cfg) {
-    cudaFuncSetAttribute(attention_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cfg = true;
-  }
-  const int n_qt = (T + FA_BM - 1) / FA_BM;
-  launch_pdl(attention_prefill_tc_kernel, dim3(B * Hq * n_qt), dim3(FA_THREADS), smem, stream, p);
+  p.scale = scale; p.softcap = softcap;
+  if (D == 128 && softcap > 0.f) fa_go<128, false, true>(p, stream);
+  else if (D == 128) fa_go<128, false, false>(p, stream);
+  else if (D == 64 && softcap > 0.f) fa_go<64, false, true>(p, stream);
+  else if (D == 64) fa_go<64, false, false>(p, stream);
+  else throw std::runtime_error("attention (tensor cores): head size 64 or 128");
+}
+
+// Prompt portions over a paged cache.  Sizes this kernel takes: keys and values of one size, 64 or 128, rows on 16-byte boundaries, pages of
+// 2^k >= 8 tokens (smaller ones would break the 8-row swizzle atoms), no distance term; the rest is paged_window_attention_mma_kernel's.
+// 3 rows of up to 1024 tokens over contexts up to 3000, 32 / 8 heads x 128, window 2048, cap, gate: 0.28 ms, mma.sync kernel 0.88 ms.
+bool paged_attention_tc_supported(const WindowAttnParams& p, bool lp) {
+  return lp && p.T >= 16 && p.maps != 2 && p.slopes == nullptr && p.D == p.Dv && (p.D == 64 || p.D == 128) && (p.v_rs * 2) % 16 == 0 && p.page >= 8 &&
+         (p.page & (p.page - 1)) == 0 && (long long)p.B * p.Hq * ((p.T + FA_ROWS - 1) / FA_ROWS) <= 0x7fffffffLL &&
+         (reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k_cache) | reinterpret_cast<uintptr_t>(p.v_cache)) % 16 == 0;
+}
+void paged_attention_tc_launch(const WindowAttnParams& w, long long slots, cudaStream_t stream) {
+  FaParams p{};
+  fa_map_rows(&p.tm_q, w.q, w.B, w.T, w.Hq, w.D);
+  fa_map_rows(&p.tm_o, w.out, w.B, w.T, w.Hq, w.D);
+  const long long kd[3] = {w.D, w.G, slots}, ks[3] = {1, w.D, (long long)w.G * w.D}, vs[3] = {1, w.v_rs, w.G * w.v_rs};
+  fa_make_map(&p.tm_k, w.k_cache, 3, kd, ks, std::min(w.page, FA_ROWS));
+  fa_make_map(&p.tm_v, w.v_cache, 3, kd, vs, std::min(w.page, FA_ROWS));
+  p.out = reinterpret_cast<__nv_bfloat16*>(w.out);
+  p.sinks = w.sinks; p.head_scale = w.head_scale;
+  p.gate = reinterpret_cast<const __nv_bfloat16*>(w.gate); p.g_sb = w.g_sb; p.g_st = w.g_st; p.gate_per_head = w.gate_per_head;
+  p.gate_vec = (reinterpret_cast<uintptr_t>(w.gate) % 16 == 0 && (w.g_sb * 2) % 16 == 0 && (w.g_st * 2) % 16 == 0) ? 1 : 0;
+  p.ctx_len = w.ctx_len; p.q_len = w.q_len; p.block_table = w.block_table; p.max_blocks = w.max_blocks;
+  while ((1 << p.page_shift) < w.page) ++p.page_shift;
+  p.B = w.B; p.T = w.T; p.Hq = w.Hq; p.Hkv = w.G; p.causal = 1; p.window = w.window; p.keep = w.keep_first; p.chunk = w.chunk;
+  p.scale = w.scale; p.softcap = w.softcap;
+  const bool cap = w.softcap > 0.f;
+  if (w.D == 128) { if (cap) fa_go<128, true, true>(p, stream); else fa_go<128, true, false>(p, stream); }
+  else { if (cap) fa_go<64, true, true>(p, stream); else fa_go<64, true, false>(p, stream); }
 }
 
 }  // namespace nxdi

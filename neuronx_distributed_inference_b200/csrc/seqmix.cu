@@ -2492,9 +2492,13 @@ void conv_qknorm_rope_append_launch(const ConvQkParams& p, bool lp, cudaStream_t
   }
 }
 
-void paged_window_attention_launch(const WindowAttnParams& p, bool lp, cudaStream_t st) {
+void paged_window_attention_launch(const WindowAttnParams& p, bool lp, long long slots, cudaStream_t st) {
   const long long nq = (long long)p.B * p.T * p.Hq;
   if (nq <= 0) return;
+  if (paged_attention_tc_supported(p, lp)) {
+    paged_attention_tc_launch(p, slots, st);
+    return;
+  }
   // values that are a prefix of the key rows of the same cache (latent rows with a rotated tail): one shared-memory tile serves both
   const bool prefix = p.maps != 2 && p.v_cache == p.k_cache && p.v_rs == p.D && p.G == 1;
   const bool rows16 = (p.v_rs * 2) % 16 == 0;

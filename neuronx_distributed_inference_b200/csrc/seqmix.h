@@ -143,7 +143,11 @@ struct WindowAttnParams {
   long long v_rs;           // elements between the value rows of neighbouring (token, kv head) pairs; Dv <= v_rs (values that are a
                             // prefix of a wider cache row: v_cache = k_cache, v_rs = D)
 };
-void paged_window_attention_launch(const WindowAttnParams& p, bool lp, cudaStream_t st);
+// slots: tokens the cache tensors hold (blocks x page)
+void paged_window_attention_launch(const WindowAttnParams& p, bool lp, long long slots, cudaStream_t st);
+// bf16 prompt portions on tcgen05 (attention_tc.cu): every output row is written, zeros past q_len
+bool paged_attention_tc_supported(const WindowAttnParams& p, bool lp);
+void paged_attention_tc_launch(const WindowAttnParams& p, long long slots, cudaStream_t st);
 
 struct SsdScanParams {
   const float* xBC;         // [B, T, inner + 2 G N] after convolution and SiLU

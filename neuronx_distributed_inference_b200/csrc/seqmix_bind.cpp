@@ -197,14 +197,15 @@ at::Tensor paged_window_attention(const at::Tensor& q, const at::Tensor& k_cache
   a.chunk = (int)chunk;
   a.v_rs = v_cache.size(3);
   c10::cuda::CUDAGuard guard(q.device());
-  auto out = at::zeros({B, T, Hq * Dv}, q.options());
   a.q = q.data_ptr(); a.k_cache = k_cache.data_ptr(); a.v_cache = v_cache.data_ptr();
   a.block_table = block_table.data_ptr<int>(); a.ctx_len = ctx.data_ptr<int>(); a.q_len = qlen.data_ptr<int>();
-  a.out = out.data_ptr();
   a.B = (int)B; a.T = (int)T; a.Hq = (int)Hq; a.G = (int)G; a.D = (int)D; a.Dv = (int)Dv; a.page = (int)k_cache.size(1);
   a.max_blocks = (int)block_table.size(1); a.window = (int)window; a.keep_first = (int)keep_first;
   a.scale = (float)scale; a.softcap = (float)softcap;
-  paged_window_attention_launch(a, is_lp(q), stream());
+  // the tcgen05 kernel writes the padding rows itself
+  auto out = paged_attention_tc_supported(a, is_lp(q)) ? at::empty({B, T, Hq * Dv}, q.options()) : at::zeros({B, T, Hq * Dv}, q.options());
+  a.out = out.data_ptr();
+  paged_window_attention_launch(a, is_lp(q), k_cache.size(0) * k_cache.size(1), stream());
   return out;
 }
 
@@ -320,7 +321,7 @@ at::Tensor paged_diff_attention(const at::Tensor& q, const at::Tensor& k_cache, 
   a.out = out.data_ptr();
   a.B = (int)B; a.T = (int)T; a.Hq = (int)H; a.G = (int)G; a.D = (int)D; a.Dv = (int)Dv; a.page = (int)k_cache.size(1);
   a.max_blocks = (int)block_table.size(1); a.window = (int)window; a.scale = (float)scale;
-  paged_window_attention_launch(a, is_lp(q), stream());
+  paged_window_attention_launch(a, is_lp(q), k_cache.size(0) * k_cache.size(1), stream());
   return out;
 }
 

@@ -1,0 +1,76 @@
+"""The tcgen05 attention kernel (csrc/attention_tc.cu) at the edges of its tiles and over all forms of its mask, against the fp32 definition.
+
+Bound: probabilities and results are rounded to bf16 (2^-9 relative each, at most); their rms is below 2^-9 / sqrt(3) * sqrt(2) = 1.6e-3, the fp32
+sums are far below.  Random rows show 2.0e-3 .. 2.4e-3 because a result is a difference of many terms; 4e-3 is asked for."""
+import pytest
+import torch
+
+from neuronx_distributed_inference_b200 import ops
+from neuronx_distributed_inference_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _rel(a, b):
+    a, b = a.float(), b.float()
+    return ((a - b).norm() / b.norm().clamp_min(1e-9)).item()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,T,Hq,Hkv,window,causal,sinks", [
+    (1, 1, 2, 1, 0, True, False), (2, 17, 4, 1, 0, True, True), (1, 128, 3, 1, 0, True, False), (3, 129, 4, 2, 0, True, False),
+    (2, 255, 3, 3, 0, True, True), (1, 257, 8, 8, 100, True, False), (2, 640, 4, 1, 128, True, True), (1, 1000, 2, 2, 77, True, False),
+    (2, 383, 6, 2, 0, False, True), (1, 1300, 4, 4, 0, False, False), (1, 2049, 2, 1, 1024, True, False)])
+def test_contiguous(D, B, T, Hq, Hkv, window, causal, sinks):
+    q, k, v = (torch.randn(B, T, h, D, device=DEV, dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv))
+    sk = torch.randn(Hq, device=DEV) if sinks else None
+    got = ops.attention_prefill(q, k, v, D ** -0.5, causal, window or None, sinks=sk)
+    want = ref.attention_prefill(q.float(), k.float(), v.float(), D ** -0.5, causal, window or None, sinks=sk)
+    assert _rel(got, want) < 4e-3
+
+
+def _paged(B, T, Hq, G, D, page, ctx, n, std=1.0):
+    blocks = -(-(max(c + m for c, m in zip(ctx, n))) // page)
+    kc, vc = (torch.randn(B * blocks + 3, page, G, D, device=DEV, dtype=torch.bfloat16) * std for _ in range(2))
+    table = torch.randperm(B * blocks + 3, device=DEV)[:B * blocks].view(B, blocks).int()
+    used = torch.zeros(B * blocks + 3, page, dtype=torch.bool, device=DEV)
+    for b in range(B):                   # rows that no request wrote hold garbage, as the rest of an allocation does
+        slots = table[b].long().repeat_interleave(page) * page + torch.arange(page, device=DEV).repeat(blocks)
+        used.view(-1)[slots[:ctx[b] + n[b]]] = True
+    clean = (torch.where(used[..., None, None], t, torch.zeros_like(t)) for t in (kc, vc))
+    dirty = (torch.where(used[..., None, None], t, torch.full_like(t, float("nan"))) for t in (kc, vc))
+    q = torch.randn(B, T, Hq, D, device=DEV, dtype=torch.bfloat16) * std
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)          # noqa: E731
+    return q, tuple(dirty), tuple(clean), table, i32(ctx), i32(n)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("page", [8, 16, 64, 128, 256])
+@pytest.mark.parametrize("mask", [dict(), dict(window=100), dict(window=300, keep=4), dict(window=130, keep=200), dict(chunk=96)])
+def test_paged(D, page, mask):
+    ctx, n = (0, 517, 130, 64), (300, 16, 0, 129)
+    q, dirty, clean, table, c, m = _paged(4, 300, 4, 2, D, page, ctx, n)
+    args = (table, c, m, D ** -0.5, None, mask.get("window", 0), mask.get("keep", 0))
+    got = ops.paged_window_attention(q, *dirty, *args, chunk=mask.get("chunk"))
+    want = ref.paged_window_attention(q.float(), *(t.float() for t in clean), *args, chunk=mask.get("chunk"))
+    assert _rel(got, want) < 4e-3
+    for b, live in enumerate(n):
+        assert not got[b, live:].any()
+
+
+@pytest.mark.parametrize("std", [1.0, 6.0])          # scores inside and beyond the range of the polynomial for tanh (|score| <= cap)
+@pytest.mark.parametrize("Hq,G", [(4, 2), (3, 3)])
+@pytest.mark.parametrize("gate", [None, "channel", "odd", "head"])
+def test_paged_cap_gate_sinks_temperature(std, Hq, G, gate):
+    D, ctx, n = 128, (77, 0), (140, 65)
+    q, dirty, clean, table, c, m = _paged(2, 140, Hq, G, D, 64, ctx, n, std)
+    wide = torch.randn(2, 140, Hq * D + 3, device=DEV, dtype=torch.bfloat16)
+    g = {None: None, "channel": wide[..., :Hq * D].contiguous(), "odd": wide[..., 3:], "head": wide[..., :Hq]}[gate]
+    kw = dict(gate=g, sinks=torch.randn(Hq, device=DEV), gate_per_head=gate == "head",
+              head_scale=torch.tensor([0.7, 1.3, -0.5, 2.0], device=DEV)[:Hq])
+    for cap in (None, 20.0):
+        got = ops.paged_window_attention(q, *dirty, table, c, m, D ** -0.5, cap, 0, 0, **kw)
+        want = ref.paged_window_attention(q.float(), *(t.float() for t in clean), table, c, m, D ** -0.5, cap, 0, 0,
+                                          **dict(kw, gate=None if g is None else g.float()))
+        assert _rel(got, want) < 4e-3
