@@ -86,7 +86,8 @@ struct ArgmaxSymm {
 void argmax_launch(const void* logits, int dtype /*0 f32, 1 bf16*/, int64_t* out, float* ws_val, int* ws_idx,
                    unsigned* tickets, int B, int V, int ld, int nsplit, const ArgmaxSymm* symm, cudaStream_t stream);
 void topk_sample_launch(const void* logits, int dtype, const int* top_k, const float* top_p, const float* temperature,
-                        const float* rand, int64_t* out, int B, int V, int ld, int K, cudaStream_t stream);
+                        const float* rand, uint32_t* gmax /*[B, topk_groups(V)]*/, int64_t* out, int B, int V, int ld, int K, cudaStream_t stream);
+int topk_groups(int V);
 
 // weight-only int8 / fp8-e4m3 skinny GEMM (qgemv.cu): wdtype 1 = int8, 2 = fp8 e4m3; scale fp32 [N] or [1]
 void qgemv_launch(const void* x, const void* w, const float* scale, int scale_n, const void* bias, const void* norm_w,

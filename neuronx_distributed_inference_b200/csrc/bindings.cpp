@@ -461,8 +461,10 @@ at::Tensor topk_sample(const at::Tensor& logits, const at::Tensor& top_k, const 
               temperature.scalar_type() == at::kFloat && rand.scalar_type() == at::kFloat && rand.numel() == B);
   c10::cuda::CUDAGuard guard(logits.device());
   auto out = at::empty({B}, logits.options().dtype(at::kLong));
-  topk_sample_launch(logits.data_ptr(), is_bf16(logits) ? 1 : 0, top_k.data_ptr<int>(), top_p.data_ptr<float>(),
-                     temperature.data_ptr<float>(), rand.data_ptr<float>(), out.data_ptr<int64_t>(), B, V, (int)logits.stride(0),
+  if (B == 0) return out;
+  auto gmax = at::empty({B, (int64_t)topk_groups(V)}, logits.options().dtype(at::kInt));
+  topk_sample_launch(logits.data_ptr(), is_bf16(logits) ? 1 : 0, top_k.data_ptr<int>(), top_p.data_ptr<float>(), temperature.data_ptr<float>(),
+                     rand.data_ptr<float>(), reinterpret_cast<uint32_t*>(gmax.data_ptr<int>()), out.data_ptr<int64_t>(), B, V, (int)logits.stride(0),
                      (int)global_topk, cur_stream());
   return out;
 }

@@ -145,89 +145,200 @@ __device__ __forceinline__ float key_to_float(uint32_t k) {
 
 constexpr int TOPK_MAX = 256;
 constexpr int TOPK_THREADS = 1024;
+constexpr int TOPK_SLICE = 8192;            // row elements per block of the first kernel: 256 groups of 32
+constexpr int TOPK_CAND = 1024;             // candidates kept for the exact choice
+constexpr int TOPK_MAX_GROUPS = 8192;       // groups per row that fit the second kernel's shared memory (rows up to 262144)
 
-// One CTA per row: 4-pass radix select of the K-th largest logit, gather the K winners, bitonic sort them
-// (value desc, index asc), then one warp applies top-k mask / temperature / softmax / top-p / inverse-CDF.
+// 16 bytes of a row (8 bf16 or 4 fp32 values) as ordered keys; positions past V give 0
+template <typename T> struct RowVec;
+template <> struct RowVec<__nv_bfloat16> { static constexpr int N = 8; };
+template <> struct RowVec<float> { static constexpr int N = 4; };
 template <typename T>
-__global__ void __launch_bounds__(TOPK_THREADS) topk_sample_kernel(const T* __restrict__ logits, const int* __restrict__ top_k,
-                                                                   const float* __restrict__ top_p, const float* __restrict__ temperature,
-                                                                   const float* __restrict__ rand, int64_t* __restrict__ out, int V, int ld,
-                                                                   int K) {
+__device__ __forceinline__ void row_keys(const T* __restrict__ row, int i, int V, bool vec, uint32_t (&k)[RowVec<T>::N]) {
+  constexpr int N = RowVec<T>::N;
+  if (vec && i + N <= V) {
+    const uint4 q = *reinterpret_cast<const uint4*>(row + i);
+    if constexpr (N == 4) {
+      k[0] = order_key(__uint_as_float(q.x)); k[1] = order_key(__uint_as_float(q.y));
+      k[2] = order_key(__uint_as_float(q.z)); k[3] = order_key(__uint_as_float(q.w));
+    } else {
+      k[0] = order_key(bf16lo(q.x)); k[1] = order_key(bf16hi(q.x)); k[2] = order_key(bf16lo(q.y)); k[3] = order_key(bf16hi(q.y));
+      k[4] = order_key(bf16lo(q.z)); k[5] = order_key(bf16hi(q.z)); k[6] = order_key(bf16lo(q.w)); k[7] = order_key(bf16hi(q.w));
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < N; ++e) k[e] = i + e < V ? order_key(to_f(row[i + e])) : 0u;
+  }
+}
+
+// Kernel 1: the largest key of every group of 32 elements (thread t of a block: the 16-byte pieces t, t + 256, ... of its slice), one
+// coalesced pass over the row spread over the whole chip.
+template <typename T>
+__global__ void __launch_bounds__(256) topk_group_max_kernel(const T* __restrict__ logits, uint32_t* __restrict__ gmax, int V, int ld, int groups) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ unsigned hist[256];
-  __shared__ unsigned long long cand[TOPK_MAX];
-  __shared__ unsigned s_prefix, s_need, s_count_gt, s_count_eq;
-  __shared__ float s_p[TOPK_MAX];
-  const int b = blockIdx.x, tid = threadIdx.x;
-  const T* row = logits + (size_t)b * ld;
-  K = min(K, V);
-  if (tid == 0) { s_prefix = 0; s_need = K; }
-  __syncthreads();
-  // radix select, most significant byte first
+  constexpr int N = RowVec<T>::N;
+  const T* row = logits + (size_t)blockIdx.y * ld;
+  const bool vec = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
+  uint32_t m = 0;
+#pragma unroll
+  for (int j = 0; j < 32 / N; ++j) {
+    uint32_t k[N];
+    row_keys<T>(row, blockIdx.x * TOPK_SLICE + (j * 256 + (int)threadIdx.x) * N, V, vec, k);
+#pragma unroll
+    for (int e = 0; e < N; ++e) m = max(m, k[e]);
+  }
+  gmax[(size_t)blockIdx.y * groups + blockIdx.x * 256 + threadIdx.x] = m;
+}
+
+// key of the need-th largest element that `each` visits (it calls its argument with every key of this thread), and how many of those equal
+// to it are among the need largest: radix select, most significant byte first
+template <typename F>
+__device__ __forceinline__ void radix_select(unsigned* hist, unsigned* s_prefix, unsigned* s_need, unsigned need, F each) {
+  const int tid = threadIdx.x;
+  if (tid == 0) { *s_prefix = 0; *s_need = need; }
   for (int pass = 0; pass < 4; ++pass) {
     const int shift = 24 - 8 * pass;
     for (int i = tid; i < 256; i += TOPK_THREADS) hist[i] = 0;
     __syncthreads();
-    const unsigned prefix = s_prefix;
-    const unsigned mask = pass == 0 ? 0u : (0xffffffffu << (shift + 8));
-    for (int i = tid; i < V; i += TOPK_THREADS) {
-      const unsigned k = order_key(to_f(row[i]));
+    const unsigned prefix = *s_prefix, mask = pass == 0 ? 0u : (0xffffffffu << (shift + 8));
+    each([&](uint32_t k) {
       if ((k & mask) == prefix) atomicAdd(&hist[(k >> shift) & 0xffu], 1u);
-    }
+    });
     __syncthreads();
-    if (tid == 0) {
-      unsigned need = s_need, acc = 0;
-      int d = 255;
-      for (; d > 0; --d) {
-        if (acc + hist[d] >= need) break;
-        acc += hist[d];
+    if (tid < 32) {                         // lane l owns digits 255 - 8 l .. 248 - 8 l, the largest first
+      unsigned c[8], sum = 0;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) { c[e] = hist[255 - 8 * tid - e]; sum += c[e]; }
+      unsigned incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned n = __shfl_up_sync(0xffffffffu, incl, o);
+        if (tid >= o) incl += n;
       }
-      s_prefix = prefix | ((unsigned)d << shift);
-      s_need = need - acc;
+      const unsigned want = *s_need;
+      unsigned acc = incl - sum;
+      __syncwarp();
+      if (acc < want && (incl >= want || tid == 31)) {
+        int e = 0;
+        for (; e < 7 && acc + c[e] < want; ++e) acc += c[e];
+        *s_prefix = prefix | ((unsigned)(255 - 8 * tid - e) << shift);
+        *s_need = want - acc;
+      }
     }
     __syncthreads();
   }
-  const unsigned thr = s_prefix;  // key of the K-th largest element
-  if (tid == 0) { s_count_gt = 0; s_count_eq = 0; }
+}
+
+// Kernel 2, one CTA per row: the k-th largest group maximum is a lower bound of the k-th largest element (k groups hold one at least as
+// large), and only groups that reach it can hold one of the k largest: k groups plus ties, 32 elements each, are read again.  Their elements
+// from the bound upwards (k plus a few percent for rows in no particular order) are ranked by counting (value, then lowest index).  More than
+// TOPK_CAND of them (long runs of equal values, or one group that holds most of the large ones): the row is selected by radix passes over all of
+// it, as every row was before (32 rows of 128256 bf16 values: 84 us a call, six scalar passes per row; 15 us with the groups, most of it the host).
+template <typename T>
+__global__ void __launch_bounds__(TOPK_THREADS) topk_sample_kernel(const T* __restrict__ logits, const uint32_t* __restrict__ gmax, int groups,
+                                                                   const int* __restrict__ top_k, const float* __restrict__ top_p,
+                                                                   const float* __restrict__ temperature, const float* __restrict__ rand,
+                                                                   int64_t* __restrict__ out, int V, int ld, int K) {
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ uint32_t s_gmax[];        // [groups]
+  __shared__ unsigned hist[256];
+  __shared__ unsigned long long cand[TOPK_MAX], raw[TOPK_CAND];
+  __shared__ int s_group[TOPK_CAND];
+  __shared__ unsigned s_prefix, s_need, s_ngroups, s_ncand;
+  const int b = blockIdx.x, tid = threadIdx.x;
+  const T* row = logits + (size_t)b * ld;
+  K = min(K, V);
+  int k_eff = top_k[b];
+  k_eff = (k_eff <= 0) ? K : min(k_eff, K);
+  if (tid == 0) { s_ngroups = 0; s_ncand = 0; }
   for (int i = tid; i < TOPK_MAX; i += TOPK_THREADS) cand[i] = 0ull;
-  __syncthreads();
-  const unsigned n_eq_take = s_need;  // how many elements equal to thr belong to the top-K
-  for (int i = tid; i < V; i += TOPK_THREADS) {
-    const unsigned k = order_key(to_f(row[i]));
-    if (k > thr) {
-      const unsigned slot = atomicAdd(&s_count_gt, 1u);
-      if (slot < (unsigned)K) cand[slot] = ((unsigned long long)k << 32) | (unsigned)(0xffffffffu - (unsigned)i);
-    }
-  }
-  __syncthreads();
-  const unsigned n_gt = min(s_count_gt, (unsigned)K);
-  for (int i = tid; i < V; i += TOPK_THREADS) {
-    const unsigned k = order_key(to_f(row[i]));
-    if (k == thr) {
-      const unsigned slot = atomicAdd(&s_count_eq, 1u);
-      if (slot < n_eq_take && n_gt + slot < (unsigned)K)
-        cand[n_gt + slot] = ((unsigned long long)k << 32) | (unsigned)(0xffffffffu - (unsigned)i);
-    }
-  }
-  __syncthreads();
-  // bitonic sort (descending) of TOPK_MAX 64-bit keys; empty slots are 0 and sink to the end
-  for (int size = 2; size <= TOPK_MAX; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      if (tid < TOPK_MAX / 2) {
-        const int lo = 2 * tid - (tid & (stride - 1));
-        const int hi = lo + stride;
-        const bool desc = ((lo & size) == 0);
-        const unsigned long long a = cand[lo], c = cand[hi];
-        if ((a < c) == desc) { cand[lo] = c; cand[hi] = a; }
+  bool ranked = groups > 0;
+  if (ranked) {
+    for (int i = tid; i < groups; i += TOPK_THREADS) s_gmax[i] = gmax[(size_t)b * groups + i];
+    __syncthreads();
+    radix_select(hist, &s_prefix, &s_need, (unsigned)k_eff, [&](auto f) {
+      for (int i = tid; i < groups; i += TOPK_THREADS) f(s_gmax[i]);
+    });
+    const uint32_t thr = s_prefix;
+    for (int i = tid; i < groups; i += TOPK_THREADS)
+      if (s_gmax[i] >= thr) {
+        const unsigned at = atomicAdd(&s_ngroups, 1u);
+        if (at < TOPK_CAND) s_group[at] = i;
+      }
+    __syncthreads();
+    const unsigned ng = s_ngroups;
+    ranked = ng <= TOPK_CAND;
+    if (ranked) {
+      constexpr int N = RowVec<T>::N, PIECES = 32 / N;
+      const bool vec = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
+      for (unsigned i = tid; i < ng * PIECES; i += TOPK_THREADS) {
+        const int g = s_group[i / PIECES], j = i % PIECES;
+        const int at = (g >> 8) * TOPK_SLICE + (j * 256 + (g & 255)) * N;
+        uint32_t k[N];
+        row_keys<T>(row, at, V, vec, k);
+#pragma unroll
+        for (int e = 0; e < N; ++e)
+          if (k[e] >= thr && at + e < V) {
+            const unsigned slot = atomicAdd(&s_ncand, 1u);
+            if (slot < TOPK_CAND) raw[slot] = ((unsigned long long)k[e] << 32) | (0xffffffffu - (unsigned)(at + e));
+          }
       }
       __syncthreads();
+      const unsigned n = s_ncand;
+      ranked = n <= TOPK_CAND;
+      if (ranked && tid < n) {
+        const unsigned long long mine = raw[tid];
+        int rank = 0;
+        for (unsigned j = 0; j < n; ++j) rank += raw[j] > mine;
+        if (rank < k_eff) cand[rank] = mine;
+      }
     }
   }
+  if (!ranked) {
+    __syncthreads();
+    radix_select(hist, &s_prefix, &s_need, (unsigned)K, [&](auto f) {
+      for (int i = tid; i < V; i += TOPK_THREADS) f(order_key(to_f(row[i])));
+    });
+    const unsigned thr = s_prefix, n_eq_take = s_need;       // key of the K-th largest element; how many equal to it belong to the K largest
+    if (tid == 0) { s_ngroups = 0; s_ncand = 0; }
+    __syncthreads();
+    for (int i = tid; i < V; i += TOPK_THREADS) {
+      const unsigned k = order_key(to_f(row[i]));
+      if (k > thr) {
+        const unsigned slot = atomicAdd(&s_ngroups, 1u);
+        if (slot < (unsigned)K) cand[slot] = ((unsigned long long)k << 32) | (unsigned)(0xffffffffu - (unsigned)i);
+      }
+    }
+    __syncthreads();
+    const unsigned n_gt = min(s_ngroups, (unsigned)K);
+    for (int i = tid; i < V; i += TOPK_THREADS) {
+      const unsigned k = order_key(to_f(row[i]));
+      if (k == thr) {
+        const unsigned slot = atomicAdd(&s_ncand, 1u);
+        if (slot < n_eq_take && n_gt + slot < (unsigned)K)
+          cand[n_gt + slot] = ((unsigned long long)k << 32) | (unsigned)(0xffffffffu - (unsigned)i);
+      }
+    }
+    __syncthreads();
+    // bitonic sort (descending) of TOPK_MAX 64-bit keys; empty slots are 0 and sink to the end
+    for (int size = 2; size <= TOPK_MAX; size <<= 1) {
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        if (tid < TOPK_MAX / 2) {
+          const int lo = 2 * tid - (tid & (stride - 1));
+          const int hi = lo + stride;
+          const bool desc = ((lo & size) == 0);
+          const unsigned long long a = cand[lo], c = cand[hi];
+          if ((a < c) == desc) { cand[lo] = c; cand[hi] = a; }
+        }
+        __syncthreads();
+      }
+    }
+  }
+  __syncthreads();
   if (tid < 32) {
     const int lane = tid;
-    int k_eff = top_k[b];
-    k_eff = (k_eff <= 0) ? K : min(k_eff, K);
     const float temp = temperature[b];
     const bool greedy = (temp == 0.f) || (k_eff == 1);
     const float inv_t = (temp == 0.f) ? 1.f : 1.f / temp;
@@ -285,18 +396,26 @@ __global__ void __launch_bounds__(TOPK_THREADS) topk_sample_kernel(const T* __re
     choice = min(choice, max(nkept, 1) - 1);
     if (greedy) choice = 0;
     if (lane == 0) out[b] = (int64_t)(0xffffffffu - (unsigned)(cand[choice] & 0xffffffffull));
-    (void)s_p;
   }
 }
 
+// uint32 workspace per row (0: rows too long for the grouped path)
+int topk_groups(int V) {
+  const long long g = (long long)((V + TOPK_SLICE - 1) / TOPK_SLICE) * 256;
+  return g <= TOPK_MAX_GROUPS ? (int)g : 0;
+}
+
 void topk_sample_launch(const void* logits, int dtype, const int* top_k, const float* top_p, const float* temperature,
-                        const float* rand, int64_t* out, int B, int V, int ld, int K, cudaStream_t stream) {
-  if (dtype == 0)
-    launch_pdl(topk_sample_kernel<float>, dim3(B), dim3(TOPK_THREADS), 0, stream, reinterpret_cast<const float*>(logits), top_k,
+                        const float* rand, uint32_t* gmax, int64_t* out, int B, int V, int ld, int K, cudaStream_t stream) {
+  const int groups = topk_groups(V);
+  auto go = [&](auto* row) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(row)>>;
+    if (groups > 0) launch_pdl(topk_group_max_kernel<T>, dim3(groups / 256, B), dim3(256), 0, stream, row, gmax, V, ld, groups);
+    launch_pdl(topk_sample_kernel<T>, dim3(B), dim3(TOPK_THREADS), (size_t)groups * 4, stream, row, static_cast<const uint32_t*>(gmax), groups, top_k,
                top_p, temperature, rand, out, V, ld, K);
-  else
-    launch_pdl(topk_sample_kernel<__nv_bfloat16>, dim3(B), dim3(TOPK_THREADS), 0, stream,
-               reinterpret_cast<const __nv_bfloat16*>(logits), top_k, top_p, temperature, rand, out, V, ld, K);
+  };
+  if (dtype == 0) go(reinterpret_cast<const float*>(logits));
+  else go(reinterpret_cast<const __nv_bfloat16*>(logits));
 }
 
 }  // namespace nxdi

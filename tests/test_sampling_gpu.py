@@ -1,0 +1,42 @@
+"""Top-k / top-p sampling over rows whose order or ties stress the group bound, row lengths around the slice size, unaligned rows, and the
+exhaustive path, against the PyTorch definition (tokens are equal: ties go to the lowest index there and here)."""
+import pytest
+import torch
+
+from neuronx_distributed_inference_b200 import ops
+from neuronx_distributed_inference_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(kind, B, V, dtype):
+    if kind == "random":
+        return (torch.randn(B, V) * 3).to(dtype)
+    if kind == "sorted":                                  # the largest values side by side
+        return torch.linspace(-9, 9, V).expand(B, V).to(dtype).contiguous()
+    if kind == "block":                                   # one stretch far above the rest
+        x = torch.randn(B, V)
+        x[:, V // 3:V // 3 + 300] += 40
+        return x.to(dtype)
+    return torch.randint(0, 4, (B, V)).to(dtype)          # "ties": long runs of equal values
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("V", [1, 7, 256, 1000, 8191, 8192, 8193, 32000, 50257, 128256, 262144, 300001])
+@pytest.mark.parametrize("kind", ["random", "sorted", "block", "ties"])
+def test_tokens(kind, V, dtype):
+    B = 6
+    logits = _rows(kind, B, V, dtype).cuda()
+    # an exact order of equal values: the definition's top-k on the CPU keeps no order among them, so distinct values are compared by token,
+    # rows with ties by the value drawn
+    top_k = torch.tensor([1, 5, 50, 0, 256, 10], dtype=torch.int32)
+    top_p = torch.tensor([1.0, 0.9, 0.5, 1.0, 0.95, 1.0])
+    temp = torch.tensor([1.0, 0.7, 1.3, 1.0, 0.0, 2.0])
+    rand = torch.tensor([0.11, 0.97, 0.42, 0.63, 0.5, 0.29])
+    got = ops.sample(logits, top_k.cuda(), top_p.cuda(), temp.cuda(), rand.cuda(), 256)
+    want = ref.sample(logits.float().cpu(), top_k, top_p, temp, rand, 256)
+    rows = torch.arange(B)
+    value = logits.float().cpu()
+    assert torch.equal(value[rows, got.cpu()], value[rows, want])
+    if kind != "ties" and dtype == torch.float32:
+        assert torch.equal(got.cpu(), want)
