@@ -94,6 +94,32 @@ void qgemv_launch(const void* x, const void* w, const float* scale, int scale_n,
                   const void* residual, void* y, int T, int N, int K, int ldx, int ldy, int act, int wdtype, float eps,
                   float norm_offset, int n_sms, cudaStream_t stream);
 
+// few tokens x large weights with the weights streamed evenly over the SMs (skinny_gemm.cu): one weight [rows, K], or the experts that have tokens
+constexpr int SKINNY_MAX_T = 128;
+struct SkinnyGemm {
+  const void* x;              // [x_rows, K] bf16, row stride ldx
+  long long x_rows, ldx;
+  const void* w;              // [experts, rows, K] bf16, rows = n_out (2 * n_out = [gate; up] when act != 0)
+  const void* bias;           // [experts, rows] bf16 or null
+  const void* residual;       // [tokens, n_out] bf16 or null (one expert, act == 0)
+  void* y;                    // [x_rows, n_out] bf16, or fp32 with y_f32
+  int y_f32;
+  int experts, tokens;        // tokens: rows of x (one expert), or the most rows an expert can have
+  int n_out, K, act;
+  float limit, alpha;
+  const int *n_active, *active, *seg_start, *seg_count;   // grouped: experts with tokens, each expert's rows of x (contiguous); null: one expert
+  float* ws;                  // skinny_gemm_ws_floats
+  unsigned* tickets;          // skinny_gemm_tickets, zero at launch
+};
+long long skinny_gemm_ws_floats(int tokens, bool glu);
+int skinny_gemm_tickets();
+void skinny_clear_launch(unsigned* tickets, int n, cudaStream_t stream);
+void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream);
+void moe_small_gather_launch(const void* x, const float* topk_w, const int* topk_i, int entries, int k, int H, int expert_offset, int e_local,
+                             int scale_input, void* xp, int* pos, int* n_active, int* active, int* seg_start, int* seg_count, unsigned* tickets,
+                             int n_tickets, cudaStream_t stream);
+void moe_small_combine_launch(const float* y, const float* topk_w, const int* pos, void* out, int N, int H, int k, int scale_input, cudaStream_t stream);
+
 // MoE decode: routed experts for T <= 8 tokens as two batched streaming launches (moe_decode.cu)
 void moe_decode_launch(const void* x, const void* w_gate_up, const void* w_down, const float* topk_w, const int* topk_i, void* u,
                        float* y_acc, int T, int topk, int H, int I, int E, int expert_offset, int act /*1 silu*up, 4 clamped gate product*/, float limit,

@@ -158,6 +158,16 @@ at::Tensor gemv(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
 }
 
 // tcgen05 GEMM for T > 8 tokens (prefill, long speculation windows)
+// Where the swapped, evenly split GEMM (skinny_gemm.cu) beats the 128-row token tiles of gemm_tcgen05.cu (us, skinny / tiles; 37, 64 and 128 tokens):
+//   gate|up 28672 x 4096: 51 / 61, 55 / 62, 66 / 62     17280 x 3200: 33 / 33, 38 / 34, 46 / 34    16384 x 2048: 24 / 26, 26 / 26, 37 / 26
+//   plain 4096 x 14336:   34 / 52, 35 / 53, 42 / 54     6144 x 4096:  21 / 24, 21 / 24, 27 / 24    2048 x 8192:  20 / 35, 21 / 35, 29 / 36
+// Its last tile's epilogue grows with the tokens (a feature per lane, all tokens in turn, twice that with a gate product), while the tile kernel's
+// time does not change up to 128; deep K leaves the tile kernel few tiles.
+static bool skinny_pays(int M, int rows, int K, bool glu) {
+  if (glu) return M <= 32 || (M <= 64 && (long long)rows * K >= (64LL << 20));
+  return M <= 64 || (M <= SKINNY_MAX_T && K >= 2 * rows);
+}
+
 at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int64_t act,
                 const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& out) {
   TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1));
@@ -173,6 +183,19 @@ at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
   auto y = out.has_value() ? *out : at::empty({M, n_out}, x.options());
   if (residual.has_value())
     TORCH_CHECK(!glu && residual->is_contiguous() && residual->size(0) == M && residual->size(1) == n_out && is_bf16(*residual));
+  if (skinny_pays(M, N, K, glu)) {
+    auto fopt = x.options().dtype(at::kFloat);
+    const int64_t nt = skinny_gemm_tickets(), nf = skinny_gemm_ws_floats(M, glu);
+    auto ws = at::empty({nf + nt}, fopt);              // one per call: safe on any stream and inside captured graphs
+    SkinnyGemm a{};
+    a.x = x.data_ptr(); a.x_rows = M; a.ldx = x.stride(0); a.w = w.data_ptr(); a.bias = optr(bias); a.residual = optr(residual); a.y = y.data_ptr();
+    a.experts = 1; a.tokens = M; a.n_out = n_out; a.K = K; a.act = (int)act; a.limit = 7.f; a.alpha = 1.702f;
+    a.ws = ws.data_ptr<float>();
+    a.tickets = reinterpret_cast<unsigned*>(ws.data_ptr<float>() + nf);
+    skinny_clear_launch(a.tickets, (int)nt, cur_stream());
+    skinny_gemm_launch(a, cur_stream());
+    return y;
+  }
   gemm_tcgen05_launch(x.data_ptr(), (int)x.stride(0), w.data_ptr(), optr(bias), optr(residual), y.data_ptr(), n_out, M, N, K,
                       (int)act, cur_stream());
   return y;
@@ -237,6 +260,45 @@ at::Tensor moe_decode(const at::Tensor& x, const at::Tensor& w_gate_up, const at
   moe_decode_launch(x.data_ptr(), w_gate_up.data_ptr(), w_down.data_ptr(), topk_w.data_ptr<float>(), topk_i.data_ptr<int>(),
                     u.data_ptr(), y.data_ptr<float>(), T, k, H, I, E, (int)expert_offset, (int)act, (float)limit, (float)alpha, n_sms, cur_stream());
   return y.to(x.scalar_type());
+}
+
+// Routed experts of a step of up to 128 tokens: every expert's weights are streamed once for all its tokens (bf16; act and biases as moe_grouped)
+at::Tensor moe_small(const at::Tensor& x, const at::Tensor& w_gate_up, const at::Tensor& w_down, const at::Tensor& topk_w, const at::Tensor& topk_i,
+                     int64_t expert_offset, int64_t act, bool scale_input, const c10::optional<at::Tensor>& gate_up_bias,
+                     const c10::optional<at::Tensor>& down_bias, double limit, double alpha) {
+  TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.is_contiguous() && is_bf16(x) && is_bf16(w_gate_up) && is_bf16(w_down));
+  TORCH_CHECK(w_gate_up.dim() == 3 && w_down.dim() == 3 && w_gate_up.is_contiguous() && w_down.is_contiguous() && act >= 1 && act <= 4);
+  const int N = x.size(0), H = x.size(1), E = w_gate_up.size(0), I = w_gate_up.size(1) / 2, k = topk_i.size(1);
+  TORCH_CHECK(w_gate_up.size(1) == 2 * I && w_gate_up.size(2) == H && w_down.size(0) == E && w_down.size(1) == H && w_down.size(2) == I);
+  TORCH_CHECK(N >= 1 && N <= SKINNY_MAX_T && H % 64 == 0 && I % 64 == 0 && E <= 512, "moe_small: 1 .. 128 tokens, sizes in multiples of 64, <= 512 experts");
+  TORCH_CHECK(topk_w.scalar_type() == at::kFloat && topk_i.scalar_type() == at::kInt && topk_w.is_contiguous() && topk_i.is_contiguous() &&
+              topk_w.numel() == (int64_t)N * k && topk_i.size(0) == N);
+  if (gate_up_bias) TORCH_CHECK(is_bf16(*gate_up_bias) && gate_up_bias->is_contiguous() && gate_up_bias->numel() == (int64_t)E * 2 * I);
+  if (down_bias) TORCH_CHECK(is_bf16(*down_bias) && down_bias->is_contiguous() && down_bias->numel() == (int64_t)E * H);
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t R = (int64_t)N * k, nt = skinny_gemm_tickets();
+  auto iopt = x.options().dtype(at::kInt), fopt = x.options().dtype(at::kFloat);
+  auto xp = at::empty({R, H}, x.options()), h = at::empty({R, I}, x.options()), out = at::empty({N, H}, x.options());
+  auto y = at::empty({R, H}, fopt);
+  auto meta = at::empty({R + 1 + 3 * (int64_t)E + 2 * nt}, iopt);       // pos | n_active | active | seg_start | seg_count | tickets of both GEMMs
+  auto ws = at::empty({std::max(skinny_gemm_ws_floats(N, true), skinny_gemm_ws_floats(N, false))}, fopt);
+  int* pos = meta.data_ptr<int>();
+  int *n_active = pos + R, *active = n_active + 1, *seg_start = active + E, *seg_count = seg_start + E;
+  unsigned* tickets = reinterpret_cast<unsigned*>(seg_count + E);
+  auto st = cur_stream();
+  moe_small_gather_launch(x.data_ptr(), topk_w.data_ptr<float>(), topk_i.data_ptr<int>(), (int)R, k, H, (int)expert_offset, E, scale_input ? 1 : 0,
+                          xp.data_ptr(), pos, n_active, active, seg_start, seg_count, tickets, (int)(2 * nt), st);
+  SkinnyGemm a{};
+  a.x = xp.data_ptr(); a.x_rows = R; a.ldx = H; a.w = w_gate_up.data_ptr(); a.bias = optr(gate_up_bias); a.y = h.data_ptr();
+  a.experts = E; a.tokens = N; a.n_out = I; a.K = H; a.act = (int)act; a.limit = (float)limit; a.alpha = (float)alpha;
+  a.n_active = n_active; a.active = active; a.seg_start = seg_start; a.seg_count = seg_count;
+  a.ws = ws.data_ptr<float>(); a.tickets = tickets;
+  skinny_gemm_launch(a, st);
+  a.x = h.data_ptr(); a.ldx = I; a.w = w_down.data_ptr(); a.bias = optr(down_bias); a.y = y.data_ptr(); a.y_f32 = 1;
+  a.n_out = H; a.K = I; a.act = 0; a.tickets = tickets + nt;
+  skinny_gemm_launch(a, st);
+  moe_small_combine_launch(y.data_ptr<float>(), topk_w.data_ptr<float>(), pos, out.data_ptr(), N, H, k, scale_input ? 1 : 0, st);
+  return out;
 }
 
 // int8 / fp8 weight [N, K] x scale -> bf16 into `out` (a caller-owned scratch: one buffer serves every layer of a model)
@@ -756,6 +818,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemv2_supported", [](int64_t T, int64_t K, int64_t wt) { return nxdi::gemv2_supported((int)T, (int)K, (int)wt); },
         pybind11::arg("T"), pybind11::arg("K"), pybind11::arg("wt") = 0);
   m.def("moe_decode", &nxdi::moe_decode);
+  m.def("moe_small", &nxdi::moe_small);
   m.def("moe_grouped", &nxdi::moe_grouped);
   m.def("dequant_bf16", &nxdi::dequant_bf16);
   m.def("gemm", &nxdi::gemm);

@@ -1,0 +1,519 @@
+// GEMM of a few tokens with large weights (9 .. 128 tokens of a batched decode step; the tokens of one expert of a small MoE step):
+// Y[t, n] = act(X W^T).  The weights are the M operand of the tensor cores and the tokens the N operand (swapped against gemm_tcgen05.cu, whose
+// 128-row token tiles would be mostly padding and whose tile grid leaves a last wave nearly empty).
+//
+// What bounds it: the weight stream from HBM.  So
+//   * CTA c of G takes the k-blocks [total c / G, total (c + 1) / G) of the concatenated (expert, 128-feature tile, k) space: every SM streams the
+//     same number of bytes whatever the shape (stream-K).  Tiles cut by a boundary meet in fp32 partials; the CTA that arrives last adds them in
+//     k order (deterministic) and runs the epilogue.
+//   * a stage is a 128 x 64 weight box (two for gate | up) plus the tokens' 64 columns; the ring takes all of shared memory (100 .. 180 KB of weights
+//     in flight per SM), weights and tokens have a TMA producer warp each.
+//   * accumulators (128 features x tokens) sit in TMEM twice, so a tile's epilogue overlaps the stream of the next one.  A lane holds one output
+//     feature: a warp's store of one token is 64 contiguous bytes, gate and up of a feature meet in one thread.
+//   * eight epilogue warps: the last tile's epilogue is the tail of the launch (four warps: 56 instead of 51 us at 37 tokens, 28672 x 4096).
+// Measured (us, here / 128-row token tiles): see skinny_pays in bindings.cpp.  28672 x 4096 at 9 tokens 46 us = 5.1 TB/s; eight Mixtral-sized experts, 6
+// tokens: 407 us = 6.1 TB/s (one warp per weight row and (token, slot) pair: 760 us).
+#include <algorithm>
+#include <stdexcept>
+#include <string>
+
+#include "api.h"
+#include "common.cuh"
+
+namespace nxdi {
+
+constexpr int SK_BM = 128, SK_BK = 64;                 // weight rows, k elements per stage box (128-byte rows)
+constexpr int SK_W_BYTES = SK_BM * SK_BK * 2;
+constexpr int SK_THREADS = 384;                        // 4 warps: weights, MMA, TMEM, tokens; 8 epilogue warps
+constexpr int SK_MAX_STAGES = 12;
+constexpr int SK_SMEM = 220 * 1024;
+
+struct SkinnyKernelParams {
+  CUtensorMap tm_w;        // [experts * rows, K], box {64, 128}
+  CUtensorMap tm_x;        // [token rows, K], box {64, xbox}: xb rows for one expert, 16 when grouped (an expert loads as many as it has tokens for)
+  const int *n_active, *active, *seg_start, *seg_count;     // grouped: experts with tokens and their rows of x; null: one expert, T rows
+  const __nv_bfloat16 *bias, *residual;                      // [experts * rows]; [T, n_out] (one expert)
+  void* y;                 // [token rows, n_out] bf16, or fp32 (y_f32)
+  float* ws;               // [G][2][cols / 4][128][4] partial tiles
+  unsigned* tickets;       // [G], zero at launch
+  int T, n_out, rows, K, act, xb, xbox, stages, y_f32, tmem_cols;
+  float limit, alpha;
+};
+
+__device__ unsigned sk_gave_up;          // waits that ran out (a protocol error; the results of that launch are not valid)
+
+__device__ __forceinline__ uint32_t sk_s32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void sk_init(uint64_t* b, uint32_t n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sk_s32(b)), "r"(n)); }
+__device__ __forceinline__ void sk_expect(uint64_t* b, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sk_s32(b)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void sk_arrive(uint64_t* b) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sk_s32(b)) : "memory"); }
+__device__ __forceinline__ bool sk_try(uint64_t* b, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(sk_s32(b)), "r"(parity) : "memory");
+  return ok != 0u;
+}
+// bounded: after the limit (seconds) every role stops waiting, issues nothing more and runs to its end
+__device__ __forceinline__ bool sk_wait(uint64_t* b, uint32_t parity, volatile int* stop) {
+  if (sk_try(b, parity)) return true;
+  for (int n = 0; n < (1 << 22); ++n) {
+    if (sk_try(b, parity)) return true;
+    if (*stop) return false;
+  }
+  *stop = 1;
+  atomicAdd(&sk_gave_up, 1u);
+  return false;
+}
+__device__ __forceinline__ void sk_tma(void* dst, const CUtensorMap* tm, int c0, int c1, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(sk_s32(dst)), "l"(tm),
+               "r"(c0), "r"(c1), "r"(sk_s32(bar)) : "memory");
+}
+// K-major operand tile of 128-byte rows, SWIZZLE_128B; 8-row groups are 1024 B apart
+__device__ __forceinline__ uint64_t sk_desc(const void* smem) {
+  uint64_t d = 0;
+  d |= (uint64_t)((sk_s32(smem) & 0x3FFFF) >> 4);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+__device__ __forceinline__ void sk_umma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d), "l"(da),
+               "l"(db), "r"(idesc), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void sk_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sk_s32(bar)) : "memory");
+}
+__device__ __forceinline__ void sk_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+                 "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(taddr));
+}
+
+template <bool GLU>
+__global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid_constant__ SkinnyKernelParams p) {
+  constexpr int NW = GLU ? 2 : 1;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (sk_s32(smem_raw) & 1023u)) & 1023u);
+  __shared__ uint64_t full_bar[SK_MAX_STAGES], empty_bar[SK_MAX_STAGES], tmem_full[2], tmem_empty[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int s_stop, s_last;
+  volatile int* stop = &s_stop;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ST = p.stages, x_bytes = p.xb * SK_BK * 2, stage_bytes = NW * SK_W_BYTES + x_bytes;     // xb % 16 == 0: multiples of 1024
+
+  if (warp == 0 && lane == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_w) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_x) : "memory");
+    for (int s = 0; s < ST; ++s) {
+      sk_init(&full_bar[s], 2);         // the two producers
+      sk_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      sk_init(&tmem_full[b], 1);
+      sk_init(&tmem_empty[b], 8);
+    }
+    s_stop = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sk_s32(&tmem_slot)), "r"(p.tmem_cols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+  pdl_launch_dependents();
+  // dense weights do not depend on earlier kernels; everything else does
+  const bool grouped = p.n_active != nullptr;
+  if (!(warp == 0 && !grouped)) pdl_wait();
+
+  const int n_tiles = (p.n_out + SK_BM - 1) / SK_BM, nkb = p.K / SK_BK;
+  const long long total = (long long)(grouped ? *p.n_active : 1) * n_tiles * nkb;
+  const long long G = max(1ll, min((long long)gridDim.x, total / 4));                // at least four k-blocks per CTA that works
+  const long long u0 = blockIdx.x < G ? total * blockIdx.x / G : 0, u1 = blockIdx.x < G ? total * (blockIdx.x + 1) / G : 0;
+  const int acc_cols = NW * p.xb;
+
+  if (warp == 0 || warp == 3) {
+    // ================= TMA producers: weights, tokens =================
+    if (lane == 0) {
+      long long it = 0;
+      bool go = true;
+      for (long long u = u0; u < u1 && go;) {
+        const int tile = (int)(u / nkb), kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u));
+        const int ei = tile / n_tiles, n0 = (tile % n_tiles) * SK_BM, e = grouped ? p.active[ei] : 0;
+        const int row_w = e * p.rows + n0, row_x = grouped ? p.seg_start[e] : 0;
+        const int boxes = grouped ? (min(p.seg_count[e], p.xb) + p.xbox - 1) / p.xbox : 1, box_bytes = p.xbox * SK_BK * 2;
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const int s = (int)(it % ST);
+          go = sk_wait(&empty_bar[s], (uint32_t)((it / ST) & 1) ^ 1u, stop);
+          if (!go) break;
+          uint8_t* st = smem + (size_t)s * stage_bytes;
+          if (warp == 0) {
+            sk_expect(&full_bar[s], NW * SK_W_BYTES);
+            sk_tma(st, &p.tm_w, kb * SK_BK, row_w, &full_bar[s]);
+            if (GLU) sk_tma(st + SK_W_BYTES, &p.tm_w, kb * SK_BK, row_w + p.n_out, &full_bar[s]);
+          } else {
+            sk_expect(&full_bar[s], boxes * box_bytes);
+            for (int q = 0; q < boxes; ++q) sk_tma(st + NW * SK_W_BYTES + q * box_bytes, &p.tm_x, kb * SK_BK, row_x + q * p.xbox, &full_bar[s]);
+          }
+        }
+        u += kb1 - kb0;
+      }
+    }
+  } else if (warp == 1) {
+    // ================= MMA issuer =================
+    if (lane == 0) {
+      long long it = 0;
+      int seg = 0;
+      bool go = true;
+      for (long long u = u0; u < u1 && go; ++seg) {
+        const int kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u)), buf = seg & 1;
+        // D = f32, A = B = bf16, both K-major, M = 128, N = the tokens in whole boxes (a multiple of 16)
+        const int nx = grouped ? (min(p.seg_count[p.active[(int)(u / nkb) / n_tiles]], p.xb) + 15) / 16 * 16 : p.xb;
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nx >> 3) << 17) | ((uint32_t)(SK_BM >> 4) << 24);
+        go = sk_wait(&tmem_empty[buf], (uint32_t)((seg >> 1) & 1) ^ 1u, stop);
+        if (!go) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const int s = (int)(it % ST);
+          go = sk_wait(&full_bar[s], (uint32_t)((it / ST) & 1), stop);
+          if (!go) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint8_t* st = smem + (size_t)s * stage_bytes;
+          const uint64_t db = sk_desc(st + NW * SK_W_BYTES);
+#pragma unroll
+          for (int w = 0; w < NW; ++w) {
+            const uint64_t da = sk_desc(st + w * SK_W_BYTES);
+#pragma unroll
+            for (int k = 0; k < SK_BK / 16; ++k)      // 16 k = 32 bytes inside the swizzle atom
+              sk_umma(tmem + (uint32_t)(buf * acc_cols + w * p.xb), da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+          }
+          sk_commit(&empty_bar[s]);
+        }
+        if (go) sk_commit(&tmem_full[buf]);
+        u += kb1 - kb0;
+      }
+    }
+  } else if (warp >= 4) {
+    // ================= epilogue: lane = output feature =================
+    const int n_in = (warp & 3) * 32 + lane, c0 = warp >= 8 ? 16 : 0;      // two warps per 32 features: even and odd groups of 16 tokens
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+    int seg = 0;
+    for (long long u = u0; u < u1; ++seg) {
+      const int tile = (int)(u / nkb), kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u)), buf = seg & 1;
+      u += kb1 - kb0;
+      const int ei = tile / n_tiles, n = (tile % n_tiles) * SK_BM + n_in, e = grouped ? p.active[ei] : 0;
+      const int row0 = grouped ? p.seg_start[e] : 0, cnt = grouped ? min(p.seg_count[e], p.xb) : p.T;
+      if (!sk_wait(&tmem_full[buf], (uint32_t)((seg >> 1) & 1), stop)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t acc = tmem + lanes + (uint32_t)(buf * acc_cols);
+      const bool whole = kb0 == 0 && kb1 == nkb;
+      const float bg = (p.bias && n < p.n_out) ? __bfloat162float(p.bias[(size_t)e * p.rows + n]) : 0.f;
+      const float bu = (GLU && p.bias && n < p.n_out) ? __bfloat162float(p.bias[(size_t)e * p.rows + p.n_out + n]) : 0.f;
+      auto finish = [&](int t, float g, float up) {
+        if (n >= p.n_out || t >= cnt) return;
+        float r = g + bg;
+        if (GLU) {
+          up += bu;
+          if (p.act == 4) {       // clamped, shifted gate product
+            const float gc = fminf(r, p.limit), uc = fminf(fmaxf(up, -p.limit), p.limit);
+            r = (uc + 1.f) * gc * (1.f / (1.f + __expf(-p.alpha * gc)));
+          } else {
+            r = (p.act == 1 ? silu(r) : (p.act == 2 ? gelu_tanh(r) : gelu_erf(r))) * up;
+          }
+        }
+        const size_t at = (size_t)(row0 + t) * p.n_out + n;
+        if (!GLU && p.residual) r += ldg_act_bf16(p.residual + at);
+        if (p.y_f32) reinterpret_cast<float*>(p.y)[at] = r;
+        else reinterpret_cast<__nv_bfloat16*>(p.y)[at] = __float2bfloat16(r);
+      };
+      if (whole) {
+#pragma unroll 1
+        for (int c = c0; c < cnt; c += 32) {
+          uint32_t g[16], up[16];
+          sk_ld16(acc + c, g);
+          if (GLU) sk_ld16(acc + p.xb + c, up);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int k = 0; k < 16; ++k) finish(c + k, __uint_as_float(g[k]), GLU ? __uint_as_float(up[k]) : 0.f);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) sk_arrive(&tmem_empty[buf]);
+        continue;
+      }
+      // a part of the tile's k range.  CTAs that share the tile: those of its first and last k-block and all between
+      const long long f = (long long)tile * nkb;
+      const int c_first = (int)(((f + 1) * G - 1) / total), c_last = (int)(((f + nkb) * G - 1) / total);
+      // adds to the sums of 16 columns from column c the partials of CTAs q0 .. c_last (k order)
+      auto add_parts = [&](int c, int q0, float (&g)[16], float (&up)[16]) {
+#pragma unroll 2
+        for (int q = q0; q <= c_last; ++q) {              // 8 .. 16 16-byte loads in flight per thread: a round trip to L2 is most of the cost
+          const float4* src = reinterpret_cast<const float4*>(p.ws + ((size_t)q * 2 + (q == c_first ? 1 : 0)) * acc_cols * SK_BM) + n_in + (size_t)(c >> 2) * SK_BM;
+          float4 a[4], b[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            a[k] = __ldcg(src + k * SK_BM);
+            if (GLU) b[k] = __ldcg(src + (size_t)((p.xb >> 2) + k) * SK_BM);
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            g[4 * k] += a[k].x; g[4 * k + 1] += a[k].y; g[4 * k + 2] += a[k].z; g[4 * k + 3] += a[k].w;
+            if (GLU) { up[4 * k] += b[k].x; up[4 * k + 1] += b[k].y; up[4 * k + 2] += b[k].z; up[4 * k + 3] += b[k].w; }
+          }
+        }
+      };
+      if (kb0 == 0) {
+        // the tile's first part is its CTA's last segment, so the other parts are usually there already: then it takes them to its own sums
+        // in TMEM and needs neither slot nor ticket
+        if (threadIdx.x == 128) {
+          unsigned v;
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.tickets + c_first) : "memory");
+          s_last = v == (unsigned)(c_last - c_first);
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        const bool direct = s_last != 0;
+        asm volatile("bar.sync 1, 256;" ::: "memory");     // s_last reusable
+        if (direct) {
+          __threadfence();
+#pragma unroll 1
+          for (int c = c0; c < cnt; c += 32) {
+            uint32_t vg[16], vu[16];
+            sk_ld16(acc + c, vg);
+            if (GLU) sk_ld16(acc + p.xb + c, vu);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            float g[16], up[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+              g[k] = __uint_as_float(vg[k]);
+              up[k] = GLU ? __uint_as_float(vu[k]) : 0.f;
+            }
+            add_parts(c, c_first + 1, g, up);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) finish(c + k, g[k], up[k]);
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) sk_arrive(&tmem_empty[buf]);
+          continue;
+        }
+      }
+      // slot 0 of this CTA if the tile began in an earlier one, else slot 1
+      const int wcols = (cnt + 15) & ~15;
+      float* mine = p.ws + ((size_t)blockIdx.x * 2 + (kb0 == 0 ? 1 : 0)) * acc_cols * SK_BM;
+#pragma unroll 1
+      for (int w = 0; w < NW; ++w)
+#pragma unroll 1
+        for (int c = c0; c < wcols; c += 32) {
+          uint32_t v[16];
+          sk_ld16(acc + w * p.xb + c, v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int k = 0; k < 16; k += 4)
+            __stcg(reinterpret_cast<uint4*>(mine) + (size_t)((w * p.xb + c + k) >> 2) * SK_BM + n_in, make_uint4(v[k], v[k + 1], v[k + 2], v[k + 3]));
+        }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) sk_arrive(&tmem_empty[buf]);
+      __threadfence();
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (threadIdx.x == 128) s_last = atomicAdd(&p.tickets[c_first], 1u) == (unsigned)(c_last - c_first);
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (s_last) {
+        __threadfence();
+#pragma unroll 1
+        for (int c = c0; c < cnt; c += 32) {
+          float g[16], up[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) g[k] = up[k] = 0.f;
+          add_parts(c, c_first, g, up);
+#pragma unroll
+          for (int k = 0; k < 16; ++k) finish(c + k, g[k], up[k]);
+        }
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");     // s_last reusable
+    }
+  }
+  if (*stop) __nanosleep(1000000);        // gave up: let copies in flight land before the shared memory goes away
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 2) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(p.tmem_cols));
+  }
+}
+
+typedef CUresult (*SkEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                               const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static void sk_map(CUtensorMap* tm, const void* ptr, long long rows, int K, long long ld, int box_rows) {
+  static SkEncodeFn fn = [] {
+    void* q = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &q, cudaEnableDefault, &r) != cudaSuccess || q == nullptr)
+      throw std::runtime_error("cuTensorMapEncodeTiled not available");
+    return reinterpret_cast<SkEncodeFn>(q);
+  }();
+  cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)rows}, gstride[1] = {(cuuint64_t)ld * 2};
+  cuuint32_t box[2] = {(cuuint32_t)SK_BK, (cuuint32_t)box_rows}, estr[2] = {1, 1};
+  CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled (skinny gemm) failed: " + std::to_string((int)r));
+}
+
+static int sk_grid() {
+  static int n = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v;
+  }();
+  return n;
+}
+static int sk_xb(int tokens) { return std::max(16, (tokens + 15) / 16 * 16); }
+
+// floats of partial tiles a launch may need
+long long skinny_gemm_ws_floats(int tokens, bool glu) { return (long long)sk_grid() * 2 * sk_xb(tokens) * (glu ? 2 : 1) * SK_BM; }
+int skinny_gemm_tickets() { return sk_grid(); }
+
+// one block between the kernel that produces x and the GEMM: the GEMM's CTAs are already filling their rings meanwhile
+__global__ void __launch_bounds__(256) skinny_clear_kernel(unsigned* __restrict__ tickets, int n) {
+  pdl_launch_dependents();
+  pdl_wait();
+  for (int i = threadIdx.x; i < n; i += 256) tickets[i] = 0u;
+}
+void skinny_clear_launch(unsigned* tickets, int n, cudaStream_t stream) { launch_pdl(skinny_clear_kernel, dim3(1), dim3(256), 0, stream, tickets, n); }
+
+void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream) {
+  if (a.K % SK_BK != 0 || a.tokens < 1 || a.tokens > SKINNY_MAX_T) throw std::runtime_error("skinny gemm: K % 64 == 0, 1 .. 128 tokens per expert");
+  SkinnyKernelParams p{};
+  const bool glu = a.act != 0;
+  p.rows = glu ? 2 * a.n_out : a.n_out;
+  p.xb = sk_xb(a.tokens);
+  sk_map(&p.tm_w, a.w, (long long)a.experts * p.rows, a.K, a.K, SK_BM);
+  p.xbox = a.n_active ? 16 : p.xb;
+  sk_map(&p.tm_x, a.x, a.x_rows, a.K, a.ldx, p.xbox);
+  p.n_active = a.n_active; p.active = a.active; p.seg_start = a.seg_start; p.seg_count = a.seg_count;
+  p.bias = reinterpret_cast<const __nv_bfloat16*>(a.bias);
+  p.residual = reinterpret_cast<const __nv_bfloat16*>(a.residual);
+  p.y = a.y; p.y_f32 = a.y_f32; p.ws = a.ws; p.tickets = a.tickets;
+  p.T = a.tokens; p.n_out = a.n_out; p.K = a.K; p.act = a.act; p.limit = a.limit; p.alpha = a.alpha;
+  const int stage = (glu ? 2 : 1) * SK_W_BYTES + p.xb * SK_BK * 2;
+  p.stages = std::min(SK_MAX_STAGES, (SK_SMEM - 1024) / stage);
+  int cols = 32;
+  while (cols < 2 * (glu ? 2 : 1) * p.xb) cols *= 2;
+  p.tmem_cols = cols;
+  const size_t smem = (size_t)p.stages * stage + 1024;
+  auto kernel = glu ? skinny_gemm_kernel<true> : skinny_gemm_kernel<false>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM) != cudaSuccess)
+    throw std::runtime_error("skinny gemm: shared memory size refused");
+  launch_pdl(kernel, dim3(sk_grid()), dim3(SK_THREADS), smem, stream, p);
+}
+
+// ---- routed experts of a small step -------------------------------------------------------------------------------------------------------
+// One block per (token, slot) entry: its row among the entries sorted by (expert, entry) — counted, so the order is the same every time —
+// and a copy of the token's row to that place.  Block 0 also writes the experts' segments and clears the tickets of the two GEMMs.
+__global__ void __launch_bounds__(256) moe_small_gather_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ topk_w,
+                                                               const int* __restrict__ topk_i, int entries, int k, int H, int expert_offset, int e_local,
+                                                               int scale_input, __nv_bfloat16* __restrict__ xp, int* __restrict__ pos,
+                                                               int* __restrict__ n_active, int* __restrict__ active, int* __restrict__ seg_start,
+                                                               int* __restrict__ seg_count, unsigned* __restrict__ tickets, int n_tickets) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ int s_sum[8];
+  const int i = blockIdx.x, tid = threadIdx.x;
+  const int e = topk_i[i] - expert_offset;
+  const bool mine = e >= 0 && e < e_local;
+  int before = 0;
+  if (mine)
+    for (int j = tid; j < entries; j += 256) {
+      const int ej = topk_i[j] - expert_offset;
+      before += ej >= 0 && (ej < e || (ej == e && j < i));
+    }
+  before = __reduce_add_sync(0xffffffffu, before);
+  if ((tid & 31) == 0) s_sum[tid >> 5] = before;
+  __syncthreads();
+  int row = 0;
+  for (int w = 0; w < 8; ++w) row += s_sum[w];
+  if (tid == 0) pos[i] = mine ? row : -1;
+  if (mine) {
+    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(i / k) * H);
+    uint4* dst = reinterpret_cast<uint4*>(xp + (size_t)row * H);
+    const float w = scale_input ? topk_w[i] : 1.f;
+    for (int v = tid; v < H / 8; v += 256) {
+      uint4 q = ldg_act(src + v);
+      if (scale_input)
+        q = make_uint4(pack_bf16(bf16lo(q.x) * w, bf16hi(q.x) * w), pack_bf16(bf16lo(q.y) * w, bf16hi(q.y) * w),
+                       pack_bf16(bf16lo(q.z) * w, bf16hi(q.z) * w), pack_bf16(bf16lo(q.w) * w, bf16hi(q.w) * w));
+      dst[v] = q;
+    }
+  }
+  if (i == 0) {
+    __shared__ int s_cnt[512], s_act;
+    for (int c = tid; c < e_local; c += 256) s_cnt[c] = 0;
+    if (tid == 0) s_act = 0;
+    __syncthreads();
+    for (int j = tid; j < entries; j += 256) {
+      const int ej = topk_i[j] - expert_offset;
+      if (ej >= 0 && ej < e_local) atomicAdd(&s_cnt[ej], 1);
+    }
+    __syncthreads();
+    if (tid < 32) {                       // exclusive scans of the counts and of "has tokens", 32 experts at a time
+      int rows = 0, acts = 0;
+      for (int c0 = 0; c0 < e_local; c0 += 32) {
+        const int c = c0 + tid, n = c < e_local ? s_cnt[c] : 0;
+        int incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, incl, o);
+          if (tid >= o) incl += t;
+        }
+        const unsigned has = __ballot_sync(0xffffffffu, n > 0);
+        if (c < e_local) {
+          seg_start[c] = rows + incl - n;
+          seg_count[c] = n;
+        }
+        if (n > 0) active[acts + __popc(has & ((1u << tid) - 1u))] = c;
+        rows += __shfl_sync(0xffffffffu, incl, 31);
+        acts += __popc(has);
+      }
+      if (tid == 0) *n_active = acts;
+    }
+    for (int t = tid; t < n_tickets; t += 256) tickets[t] = 0u;
+  }
+}
+
+// out[token] = sum over slots of affinity * y[row of (token, slot)], fp32 rows, fixed slot order
+__global__ void __launch_bounds__(256) moe_small_combine_kernel(const float* __restrict__ y, const float* __restrict__ topk_w, const int* __restrict__ pos,
+                                                                __nv_bfloat16* __restrict__ out, int H, int k, int scale_input) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tok = blockIdx.y, v = blockIdx.x * 256 + threadIdx.x;
+  if (v >= H / 4) return;
+  float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s = 0; s < k; ++s) {
+    const int r = pos[tok * k + s];
+    if (r < 0) continue;
+    const float w = scale_input ? 1.f : topk_w[tok * k + s];
+    const float4 q = __ldcg(reinterpret_cast<const float4*>(y + (size_t)r * H) + v);
+    f.x += w * q.x; f.y += w * q.y; f.z += w * q.z; f.w += w * q.w;
+  }
+  *reinterpret_cast<uint2*>(out + (size_t)tok * H + v * 4) = make_uint2(pack_bf16(f.x, f.y), pack_bf16(f.z, f.w));
+}
+
+void moe_small_gather_launch(const void* x, const float* topk_w, const int* topk_i, int entries, int k, int H, int expert_offset, int e_local,
+                             int scale_input, void* xp, int* pos, int* n_active, int* active, int* seg_start, int* seg_count, unsigned* tickets,
+                             int n_tickets, cudaStream_t stream) {
+  if (e_local > 512 || H % 8 != 0) throw std::runtime_error("moe (small step): at most 512 experts, hidden size % 8 == 0");
+  launch_pdl(moe_small_gather_kernel, dim3(entries), dim3(256), 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), topk_w, topk_i, entries, k, H,
+             expert_offset, e_local, scale_input, reinterpret_cast<__nv_bfloat16*>(xp), pos, n_active, active, seg_start, seg_count, tickets, n_tickets);
+}
+void moe_small_combine_launch(const float* y, const float* topk_w, const int* pos, void* out, int N, int H, int k, int scale_input, cudaStream_t stream) {
+  launch_pdl(moe_small_combine_kernel, dim3((H / 4 + 255) / 256, N), dim3(256), 0, stream, y, topk_w, pos, reinterpret_cast<__nv_bfloat16*>(out), H, k,
+             scale_input);
+}
+
+}  // namespace nxdi

@@ -429,10 +429,21 @@ def moe_experts(x, w_gate_up, w_down, topk_w, topk_i, act="silu_mul", expert_off
                                gate_up_scale, down_scale)
     # activations with a kernel implementation: the named GLU ones, or a callable that names its kernel twin (``kernel_act``)
     kact = act if act_fn is None else getattr(act_fn, "kernel_act", None)
-    if (_use_cuda(x) and x.dtype in _FAST_DTYPES and w_gate_up.dtype == x.dtype and act in ("silu_mul", "clamped_glu")
-            and act_fn is None and gate_up_bias is None and down_bias is None and N <= GEMV_MAX_TOKENS and not scale_input
-            and w_gate_up.is_contiguous() and w_down.is_contiguous() and topk_i.dim() == 2
-            and x.shape[1] % 8 == 0 and w_down.shape[2] % 8 == 0 and max(x.shape[1], w_down.shape[2]) * 2 <= 65536):
+    # a handful of tokens through plain SwiGLU experts: one warp per weight row and (token, slot) pair
+    rows_kernel = (act in ("silu_mul", "clamped_glu") and act_fn is None and gate_up_bias is None and down_bias is None and not scale_input
+                   and x.shape[1] % 8 == 0 and w_down.shape[2] % 8 == 0 and max(x.shape[1], w_down.shape[2]) * 2 <= 65536)
+    # small steps: every expert's weights are streamed once for all its tokens, evenly over the SMs (csrc/skinny_gemm.cu)
+    if (_use_cuda(x) and _MOE_GROUPED and x.dtype == torch.bfloat16 and w_gate_up.dtype == x.dtype and w_down.dtype == x.dtype
+            and kact in _MOE_ACTS and (_MOE_ROWS_TOKENS if rows_kernel else 0) < N <= _MOE_SMALL_TOKENS and topk_i.dim() == 2 and topk_i.shape[1] <= 64
+            and w_gate_up.is_contiguous() and w_down.is_contiguous() and x.shape[1] % 64 == 0 and w_down.shape[2] % 64 == 0
+            and w_gate_up.shape[0] <= 512
+            and (gate_up_bias is None or gate_up_bias.dtype == x.dtype) and (down_bias is None or down_bias.dtype == x.dtype)):
+        stats["moe_decode" if rows_kernel and N <= GEMV_MAX_TOKENS else "moe_grouped"] += 1
+        return _C().moe_small(x.contiguous(), w_gate_up, w_down, topk_w.float().contiguous(), topk_i.to(torch.int32).contiguous(), int(expert_offset),
+                              _MOE_ACTS[kact], bool(scale_input), None if gate_up_bias is None else gate_up_bias.contiguous(),
+                              None if down_bias is None else down_bias.contiguous(), limit, alpha)
+    if (_use_cuda(x) and x.dtype in _FAST_DTYPES and w_gate_up.dtype == x.dtype and rows_kernel and N <= GEMV_MAX_TOKENS
+            and w_gate_up.is_contiguous() and w_down.is_contiguous() and topk_i.dim() == 2):
         stats["moe_decode"] += 1
         return _C().moe_decode(x.contiguous(), w_gate_up, w_down, topk_w.float().contiguous(),
                                topk_i.to(torch.int32).contiguous(), int(expert_offset), _MOE_ACTS[act], limit, alpha)
@@ -452,6 +463,10 @@ def moe_experts(x, w_gate_up, w_down, topk_w, topk_i, act="silu_mul", expert_off
 
 
 _MOE_GROUPED = os.environ.get("NXDI_B200_MOE_GROUPED", "1") == "1"
+# measured (us, rows kernel / small-step path): 128 experts, 8 chosen, 2048 x 768: 26 / 37, 39 / 59, 80 / 78, 141 / 113 at 1, 2, 4, 8 tokens; 8 experts, 2 chosen,
+# 4096 x 14336: 129 / 141, 209 / 195 and 686 / 412 at 1, 2 and 8.  Against the padded grouped GEMMs at 12, 48 and 128 tokens: 228 / 140, 346 / 223, 354 / 244 and
+# 510 / 464, 512 / 491, 575 / 509
+_MOE_ROWS_TOKENS, _MOE_SMALL_TOKENS = 2, 128
 _MOE_ACTS = {"silu_mul": 1, "gelu_tanh_mul": 2, "gelu_mul": 3, "gpt_oss_glu": 4, "clamped_glu": 4}      # 4 takes (limit, alpha); gpt_oss_glu: 7, 1.702
 _UNARY_ACTS = {"relu": 1, "relu2": 2, "silu": 3, "gelu_tanh": 4, "sigmoid": 5, "gelu": 6}         # codes of csrc/seqmix.cu (unary_act, moe_plain, gated_act_mul)
 _MOE_PLAIN_ACTS = _UNARY_ACTS
