@@ -94,6 +94,10 @@ void qgemv_launch(const void* x, const void* w, const float* scale, int scale_n,
                   const void* residual, void* y, int T, int N, int K, int ldx, int ldy, int act, int wdtype, float eps,
                   float norm_offset, int n_sms, cudaStream_t stream);
 
+// prompt-sized GEMM on CTA pairs (gemm_pair.cu); tile_expert: grouped, segments of whole 256-row tiles
+void gemm_pair_launch(const void* a, long long lda, const void* b, const void* bias, const void* residual, void* c, int M, int N, int K, int act,
+                      cudaStream_t stream, const int* tile_expert = nullptr, int experts = 1, float limit = 7.f, float alpha = 1.702f);
+
 // few tokens x large weights with the weights streamed evenly over the SMs (skinny_gemm.cu): one weight [rows, K], or the experts that have tokens
 constexpr int SKINNY_MAX_T = 128;
 struct SkinnyGemm {

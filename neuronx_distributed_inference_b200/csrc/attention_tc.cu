@@ -70,7 +70,7 @@ __device__ __forceinline__ bool fa_mb_try(uint64_t* b, uint32_t parity) {
 // Bounded wait: after the limit (seconds) every role of the CTA stops waiting, issues no further copies or MMAs and runs to its end.
 __device__ __forceinline__ bool fa_mb_wait(uint64_t* b, uint32_t parity, volatile int* stop) {
   if (fa_mb_try(b, parity)) return true;
-  for (int n = 0; n < (1 << 22); ++n) {
+  for (int n = 0; n < (1 << 20); ++n) {
     if (fa_mb_try(b, parity)) return true;
     if (*stop) return false;
   }

@@ -163,6 +163,14 @@ at::Tensor gemv(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
 //   plain 4096 x 14336:   34 / 52, 35 / 53, 42 / 54     6144 x 4096:  21 / 24, 21 / 24, 27 / 24    2048 x 8192:  20 / 35, 21 / 35, 29 / 36
 // Its last tile's epilogue grows with the tokens (a feature per lane, all tokens in turn, twice that with a gate product), while the tile kernel's
 // time does not change up to 128; deep K leaves the tile kernel few tiles.
+// Where 256 x 256 tiles on CTA pairs (gemm_pair.cu) beat the one-CTA tiles (us, pairs / one CTA, isolated):
+//   28672 x 4096 gate|up: 62 / 84 at 256 tokens, 99 / 133 at 512, 624 / 725 at 4096      4096 x 14336: 74 / 55 at 256, 76 / 77 at 512, 80 / 94 at 768
+//   6144 x 4096: 26 / 26 at 256, 29 / 41 at 400, 71 / 82 at 2048                         2048 x 8192: 45 / 36 at 512, 45 / 49 at 768, 98 / 110 at 4096
+// Up to 512 tokens the one-CTA kernel has smaller tiles and split-K to fill the chip; with 40 pair tiles or more (of 74 pairs) they are not needed.
+static bool pair_pays(int M, int n_out, bool glu) {
+  return M > 512 || (M > 128 && ((M + 255) / 256) * ((n_out + (glu ? 127 : 255)) / (glu ? 128 : 256)) >= 40);
+}
+
 static bool skinny_pays(int M, int rows, int K, bool glu) {
   if (glu) return M <= 32 || (M <= 64 && (long long)rows * K >= (64LL << 20));
   return M <= 64 || (M <= SKINNY_MAX_T && K >= 2 * rows);
@@ -194,6 +202,10 @@ at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
     a.tickets = reinterpret_cast<unsigned*>(ws.data_ptr<float>() + nf);
     skinny_clear_launch(a.tickets, (int)nt, cur_stream());
     skinny_gemm_launch(a, cur_stream());
+    return y;
+  }
+  if (pair_pays(M, n_out, glu)) {
+    gemm_pair_launch(x.data_ptr(), x.stride(0), w.data_ptr(), optr(bias), optr(residual), y.data_ptr(), M, N, K, (int)act, cur_stream());
     return y;
   }
   gemm_tcgen05_launch(x.data_ptr(), (int)x.stride(0), w.data_ptr(), optr(bias), optr(residual), y.data_ptr(), n_out, M, N, K,

@@ -57,7 +57,7 @@ __device__ __forceinline__ bool sk_try(uint64_t* b, uint32_t parity) {
 // bounded: after the limit (seconds) every role stops waiting, issues nothing more and runs to its end
 __device__ __forceinline__ bool sk_wait(uint64_t* b, uint32_t parity, volatile int* stop) {
   if (sk_try(b, parity)) return true;
-  for (int n = 0; n < (1 << 22); ++n) {
+  for (int n = 0; n < (1 << 20); ++n) {
     if (sk_try(b, parity)) return true;
     if (*stop) return false;
   }
