@@ -94,7 +94,7 @@ void qgemv_launch(const void* x, const void* w, const float* scale, int scale_n,
                   const void* residual, void* y, int T, int N, int K, int ldx, int ldy, int act, int wdtype, float eps,
                   float norm_offset, int n_sms, cudaStream_t stream);
 
-// prompt-sized GEMM on CTA pairs (gemm_pair.cu); tile_expert: grouped, segments of whole 256-row tiles
+// prompt-sized GEMM on CTA pairs (gemm_pair.cu); tile_expert: grouped, segments of whole 256-row tiles (moe_plan256)
 void gemm_pair_launch(const void* a, long long lda, const void* b, const void* bias, const void* residual, void* c, int M, int N, int K, int act,
                       cudaStream_t stream, const int* tile_expert = nullptr, int experts = 1, float limit = 7.f, float alpha = 1.702f);
 
@@ -177,6 +177,8 @@ void gemm_fp8_launch(const void* a, int lda, const void* b, const float* a_scale
                      const void* residual, void* c, int ldc, int M, int N, int K, int act, cudaStream_t stream);
 
 // mixture-of-experts prefill: device-side permutation (moe_grouped.cu) around the grouped tcgen05 GEMM (gemm_tcgen05.cu)
+void moe_plan256_launch(const int* topk_i, int entries, int expert_offset, int e_local, int tiles, int* pos, int* tile_expert, cudaStream_t stream);
+void moe_scatter_launch(const void* x, const float* topk_w, const int* pos, void* xp, int N, int H, int k, int scale_input, cudaStream_t stream);
 void moe_plan_launch(const int* topk_i, int entries, int expert_offset, int e_local, int R, int* pos, int* row_entry, int* tile_expert,
                      cudaStream_t stream);
 void moe_gather_launch(const void* x, const float* topk_w, const int* row_entry, const int* tile_expert, void* xp, int R, int H, int k,

@@ -356,8 +356,24 @@ at::Tensor moe_grouped(const at::Tensor& x, const at::Tensor& w_gate_up, const a
   if (gate_up_bias) TORCH_CHECK(is_bf16(*gate_up_bias) && gate_up_bias->is_contiguous() && gate_up_bias->numel() == (int64_t)E * 2 * I);
   if (down_bias) TORCH_CHECK(is_bf16(*down_bias) && down_bias->is_contiguous() && down_bias->numel() == (int64_t)E * H);
   c10::cuda::CUDAGuard guard(x.device());
-  const int64_t R = (((int64_t)N * k + (int64_t)E * 127) + 127) / 128 * 128;   // static bound: graph-stable shapes
   auto iopt = x.options().dtype(at::kInt);
+  if (!fp8) {
+    // static bound of 256-row tiles: graph-stable shapes
+    const int64_t entries = (int64_t)N * k, R = (entries + std::min<int64_t>(E, entries) * 255) / 256 * 256;
+    auto out = at::empty({N, H}, x.options());
+    if (entries == 0 || R == 0) return out.zero_();
+    auto st = cur_stream();
+    auto pos = at::empty({entries}, iopt), tile_expert = at::empty({R / 256}, iopt);
+    auto xp = at::empty({R, H}, x.options()), h = at::empty({R, I}, x.options()), y = at::empty({R, H}, x.options());
+    moe_plan256_launch(topk_i.data_ptr<int>(), (int)entries, (int)expert_offset, E, (int)(R / 256), pos.data_ptr<int>(), tile_expert.data_ptr<int>(), st);
+    moe_scatter_launch(x.data_ptr(), topk_w.data_ptr<float>(), pos.data_ptr<int>(), xp.data_ptr(), N, H, k, scale_input ? 1 : 0, st);
+    gemm_pair_launch(xp.data_ptr(), H, w_gate_up.data_ptr(), optr(gate_up_bias), nullptr, h.data_ptr(), (int)R, 2 * I, H, (int)act, st,
+                     tile_expert.data_ptr<int>(), E, (float)limit, (float)alpha);
+    gemm_pair_launch(h.data_ptr(), I, w_down.data_ptr(), optr(down_bias), nullptr, y.data_ptr(), (int)R, H, I, 0, st, tile_expert.data_ptr<int>(), E);
+    moe_combine_launch(y.data_ptr(), topk_w.data_ptr<float>(), pos.data_ptr<int>(), out.data_ptr(), N, H, k, scale_input ? 1 : 0, st);
+    return out;
+  }
+  const int64_t R = (((int64_t)N * k + (int64_t)E * 127) + 127) / 128 * 128;
   auto pos = at::empty({(int64_t)N * k}, iopt);
   auto row_entry = at::empty({R}, iopt);
   auto tile_expert = at::empty({R / 128}, iopt);
@@ -371,22 +387,15 @@ at::Tensor moe_grouped(const at::Tensor& x, const at::Tensor& w_gate_up, const a
   moe_gather_launch(x.data_ptr(), topk_w.data_ptr<float>(), row_entry.data_ptr<int>(), tile_expert.data_ptr<int>(), xp.data_ptr(), (int)R,
                     H, k, scale_input ? 1 : 0, st);
   const float inf = std::numeric_limits<float>::infinity();
-  if (fp8) {
-    auto bopt = x.options().dtype(at::kByte);
-    auto xq = at::empty({R, H}, bopt), hq = at::empty({R, I}, bopt);
-    auto xs = at::empty({R}, x.options().dtype(at::kFloat)), hs = at::empty({R}, x.options().dtype(at::kFloat));
-    rmsnorm_quant_launch(xp.data_ptr(), nullptr, xq.data_ptr(), xs.data_ptr<float>(), (int)R, H, 0.f, 0.f, inf, st);
-    gemm_grouped_launch(xq.data_ptr(), w_gate_up.data_ptr(), gate_up_bias ? gate_up_bias->data_ptr() : nullptr, h.data_ptr(), (int)R, 2 * I,
-                        H, E, (int)act, tile_expert.data_ptr<int>(), xs.data_ptr<float>(), gate_up_scale->data_ptr<float>(), st, (float)limit, (float)alpha);
-    rmsnorm_quant_launch(h.data_ptr(), nullptr, hq.data_ptr(), hs.data_ptr<float>(), (int)R, I, 0.f, 0.f, inf, st);
-    gemm_grouped_launch(hq.data_ptr(), w_down.data_ptr(), down_bias ? down_bias->data_ptr() : nullptr, y.data_ptr(), (int)R, H, I, E, 0,
-                        tile_expert.data_ptr<int>(), hs.data_ptr<float>(), down_scale->data_ptr<float>(), st);
-  } else {
-    gemm_grouped_launch(xp.data_ptr(), w_gate_up.data_ptr(), gate_up_bias ? gate_up_bias->data_ptr() : nullptr, h.data_ptr(), (int)R,
-                        2 * I, H, E, (int)act, tile_expert.data_ptr<int>(), nullptr, nullptr, st, (float)limit, (float)alpha);
-    gemm_grouped_launch(h.data_ptr(), w_down.data_ptr(), down_bias ? down_bias->data_ptr() : nullptr, y.data_ptr(), (int)R, H, I, E, 0,
-                        tile_expert.data_ptr<int>(), nullptr, nullptr, st);
-  }
+  auto bopt = x.options().dtype(at::kByte);
+  auto xq = at::empty({R, H}, bopt), hq = at::empty({R, I}, bopt);
+  auto xs = at::empty({R}, x.options().dtype(at::kFloat)), hs = at::empty({R}, x.options().dtype(at::kFloat));
+  rmsnorm_quant_launch(xp.data_ptr(), nullptr, xq.data_ptr(), xs.data_ptr<float>(), (int)R, H, 0.f, 0.f, inf, st);
+  gemm_grouped_launch(xq.data_ptr(), w_gate_up.data_ptr(), gate_up_bias ? gate_up_bias->data_ptr() : nullptr, h.data_ptr(), (int)R, 2 * I,
+                      H, E, (int)act, tile_expert.data_ptr<int>(), xs.data_ptr<float>(), gate_up_scale->data_ptr<float>(), st, (float)limit, (float)alpha);
+  rmsnorm_quant_launch(h.data_ptr(), nullptr, hq.data_ptr(), hs.data_ptr<float>(), (int)R, I, 0.f, 0.f, inf, st);
+  gemm_grouped_launch(hq.data_ptr(), w_down.data_ptr(), down_bias ? down_bias->data_ptr() : nullptr, y.data_ptr(), (int)R, H, I, E, 0,
+                      tile_expert.data_ptr<int>(), hs.data_ptr<float>(), down_scale->data_ptr<float>(), st);
   moe_combine_launch(y.data_ptr(), topk_w.data_ptr<float>(), pos.data_ptr<int>(), out.data_ptr(), N, H, k, scale_input ? 1 : 0, st);
   return out;
 }

@@ -9,8 +9,10 @@
 //   * warps 4..11: epilogue of the CTA's own 128 rows (two warps per 32 rows take turns at 64-column pieces: with four warps the gate products of
 //     2048-deep tiles took longer than their MMAs); bias / residual / gate products; rows leave (and residual rows come) through shared memory as
 //     whole 128-byte pieces
-//   * grouped (mixture of experts): A holds tokens permuted by expert in segments of whole 256-row tiles, tile_expert maps a row tile to its expert.
-//     Tiles are walked in bands of at most 32 MB of A rows, so that the permuted rows are read from HBM once and not once per n-tile.
+//   * grouped (mixture of experts): A holds tokens permuted by expert in segments of whole 256-row tiles; tile_expert gives a row tile's expert and how
+//     many of its rows hold tokens (a half without any is neither loaded nor stored).  Tiles are walked in bands of four row tiles, n-tile by n-tile
+//     inside a band: the permuted rows and an expert's weights are read from HBM once (128 experts of 2048 x 768, 4096 tokens, 8 each, both GEMMs with
+//     permutation: 456 us; bands of 32 row tiles 480, no bands 589; 8 experts of 4096 x 14336, 1024 tokens: 858, 951, 944).
 // Measured (isolated, us, here / 128 x 256 tiles of one CTA): 4096 tokens 28672 x 4096 gate|up 624 / 725 (1.54 PFLOP/s, 94 % of the measured cuBLAS burst),
 // 4096 x 14336 336 / 371, 16384 x 2048 gate|up 188 / 356 (290 with four epilogue warps).  256 x 128 tiles are slower wherever they were tried (960 us
 // for the first): their operand traffic per flop is that of the one-CTA tiles again.
@@ -37,7 +39,7 @@ struct PairParams {
   int M, N, K, n_out, act;        // act: 0 none, 1 silu*up, 2 gelu_tanh*up, 3 gelu*up, 4 clamped gate product (n_out = N / 2)
   float limit, alpha;
   int m_tiles, n_tiles, band;
-  const int* tile_expert;         // grouped: [m_tiles] expert of a 256-row tile, < 0: not in use; null: one weight
+  const int* tile_expert;         // grouped: [m_tiles] expert | rows with tokens << 10 of a 256-row tile, < 0: not in use; null: one weight
 };
 
 __device__ unsigned gp_gave_up;    // waits that ran out (a protocol error; the results of that launch are not valid)
@@ -167,9 +169,12 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
         int mt, nt;
         gp_tile(p, t, mt, nt);
         int e = 0;
+        bool second = true;              // the odd CTA's half has rows
         if (p.tile_expert != nullptr) {
           e = __ldg(p.tile_expert + mt);
           if (e < 0) continue;
+          second = (e >> 10) > 128;
+          e &= 1023;
         }
         const int row_a = mt * 256 + (int)rank * 128;
         const int row_b = e * p.N + (glu ? nt * (BN / 2) + (rank ? p.n_out : 0) : nt * BN + (int)rank * (BN / 2));
@@ -182,8 +187,8 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
           if (warp == 0) {
             gp_tma(st + GP_A_BYTES, &p.tma_b, kb * GP_BK, row_b, bar);
           } else {
-            if (rank == 0) gp_expect(&full_bar[s], 2 * STAGE);       // everything that both CTAs copy for this stage
-            gp_tma(st, &p.tma_a, kb * GP_BK, row_a, bar);
+            if (rank == 0) gp_expect(&full_bar[s], 2 * STAGE - (second ? 0 : GP_A_BYTES));       // everything that both CTAs copy for this stage
+            if (rank == 0 || second) gp_tma(st, &p.tma_a, kb * GP_BK, row_a, bar);
           }
         }
       }
@@ -227,12 +232,12 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
     uint8_t* stg = staging + (warp - 4) * 4096;             // 32 rows x 64 columns, 16-byte chunks XOR-swizzled
     auto stg_at = [&](int r, int ch) { return reinterpret_cast<uint4*>(stg + r * 128 + ((ch ^ (r & 7)) << 4)); };
     // rows row0 .. row0 + 31, columns col0 .. col0 + 63, lanes along the rows: residual in, results out
-    auto move_rows = [&](int row0, int col0, bool in) {
+    auto move_rows = [&](int row0, int row_end, int col0, bool in) {
       __syncwarp();
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int r = i * 4 + (lane >> 3), ch = lane & 7, row = row0 + r, col = col0 + ch * 8;
-        if (row < p.M && col < p.n_out) {           // n_out % 8 == 0: a chunk is inside or outside as a whole
+        if (row < row_end && col < p.n_out) {          // n_out % 8 == 0: a chunk is inside or outside as a whole
           if (in) *stg_at(r, ch) = ldg_act(p.residual + (size_t)row * p.n_out + col);
           else *reinterpret_cast<uint4*>(p.c + (size_t)row * p.n_out + col) = *stg_at(r, ch);
         }
@@ -243,19 +248,20 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
     for (int t = pair; t < total; t += pairs) {
       int mt, nt;
       gp_tile(p, t, mt, nt);
-      int eo = 0;
+      int eo = 0, row_end = p.M;
       if (p.tile_expert != nullptr) {
         const int e = __ldg(p.tile_expert + mt);
         if (e < 0) continue;
-        eo = e * p.N;
+        eo = (e & 1023) * p.N;
+        row_end = mt * 256 + (e >> 10);
       }
       const int buf = tc & 1, row0 = mt * 256 + (int)rank * 128 + q * 32, col_t = nt * tile_out;
       if (!gp_wait(&tmem_full[buf], (uint32_t)((tc >> 1) & 1), stop)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN);
 #pragma unroll 1
-      for (int c0 = warp >= 8 ? 64 : 0; c0 < tile_out; c0 += 128) {
-        if (p.residual != nullptr) move_rows(row0, col_t + c0, true);
+      for (int c0 = warp >= 8 ? 64 : 0; c0 < tile_out && row0 < row_end; c0 += 128) {
+        if (p.residual != nullptr) move_rows(row0, row_end, col_t + c0, true);
 #pragma unroll 1
         for (int c = c0; c < c0 + 64; c += 32) {
           uint32_t vg[32], vu[32];
@@ -301,7 +307,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
             *at = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
           }
         }
-        move_rows(row0, col_t + c0, false);
+        move_rows(row0, row_end, col_t + c0, false);
       }
       // this warp has read its lanes of the buffer: back to the pair's issuer
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -363,7 +369,7 @@ void gemm_pair_launch(const void* a, long long lda, const void* b, const void* b
   const int tile_out = glu ? GP_BN / 2 : GP_BN;
   p.m_tiles = (M + 255) / 256;
   p.n_tiles = (p.n_out + tile_out - 1) / tile_out;
-  p.band = tile_expert == nullptr ? p.m_tiles : std::max(1, std::min<int>(p.m_tiles, (int)((32LL << 20) / (256LL * K * 2))));
+  p.band = tile_expert == nullptr ? p.m_tiles : std::min(4, p.m_tiles);
   gp_map(&p.tma_a, a, M, K, lda, 128);
   gp_map(&p.tma_b, b, (long long)experts * N, K, K, GP_BN / 2);
   if (cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM) != cudaSuccess)

@@ -123,6 +123,93 @@ __global__ void __launch_bounds__(128) moe_combine_kernel(const __nv_bfloat16* _
   }
 }
 
+// ---- bf16 experts on CTA-pair tiles (gemm_pair.cu): segments of whole 256-row tiles ------------------------------------------------------
+// One CTA: the atomic that counts an expert's entries also ranks them, so one pass decides the rows and the second only adds the segment starts
+// (32768 entries, 128 experts: 11 us; with a second atomic pass, a serial scan and the inverse table 31 us).
+__global__ void __launch_bounds__(MOE_PLAN_THREADS) moe_plan256_kernel(const int* __restrict__ topk_i, int entries, int expert_offset, int e_local, int tiles,
+                                                                       int* __restrict__ pos, int* __restrict__ tile_expert) {
+  __shared__ int count[MOE_MAX_E], start[MOE_MAX_E + 1];
+  pdl_launch_dependents();
+  const int tid = threadIdx.x;
+  for (int e = tid; e < e_local; e += MOE_PLAN_THREADS) count[e] = 0;
+  __syncthreads();
+  pdl_wait();
+  constexpr int U = 8;             // entries in flight per thread
+  for (int i0 = tid; i0 < entries; i0 += U * MOE_PLAN_THREADS) {
+    int e[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) e[u] = i0 + u * MOE_PLAN_THREADS < entries ? topk_i[i0 + u * MOE_PLAN_THREADS] - expert_offset : -1;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * MOE_PLAN_THREADS < entries) pos[i0 + u * MOE_PLAN_THREADS] = (e[u] >= 0 && e[u] < e_local) ? atomicAdd(&count[e[u]], 1) : -1;
+  }
+  __syncthreads();
+  if (tid < 32) {
+    int at = 0;
+    for (int c0 = 0; c0 < e_local; c0 += 32) {
+      const int c = c0 + tid, n = c < e_local ? (count[c] + 255) & ~255 : 0;
+      int incl = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (tid >= o) incl += t;
+      }
+      if (c < e_local) start[c] = at + incl - n;
+      at += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (tid == 0) start[e_local] = at;
+  }
+  __syncthreads();
+  for (int e = tid; e < e_local; e += MOE_PLAN_THREADS)
+    for (int t = start[e] >> 8; t < start[e + 1] >> 8; ++t) tile_expert[t] = e | min(256, start[e] + count[e] - t * 256) << 10;
+  for (int t = (start[e_local] >> 8) + tid; t < tiles; t += MOE_PLAN_THREADS) tile_expert[t] = -1;
+  for (int i0 = tid; i0 < entries; i0 += U * MOE_PLAN_THREADS) {      // own entries again: written by this thread above
+    int e[U], r[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * MOE_PLAN_THREADS;
+      e[u] = i < entries ? topk_i[i] - expert_offset : -1;
+      r[u] = i < entries ? pos[i] : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (r[u] >= 0) pos[i0 + u * MOE_PLAN_THREADS] = start[e[u]] + r[u];
+  }
+}
+
+// one CTA per token: its row is read once and written to the k places of its experts (padding rows are left as they are: a row of the products
+// depends on its own row only, and no padding row is combined)
+__global__ void __launch_bounds__(256) moe_scatter_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ topk_w,
+                                                          const int* __restrict__ pos, __nv_bfloat16* __restrict__ xp, int H, int k, int scale_input) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tok = blockIdx.x;
+  const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)tok * H);
+  for (int v = threadIdx.x; v < H / 8; v += 256) {
+    const uint4 q = ldg_act(src + v);
+    for (int s = 0; s < k; ++s) {
+      const int r = pos[(size_t)tok * k + s];
+      if (r < 0) continue;
+      uint4 o = q;
+      if (scale_input) {
+        const float w = topk_w[(size_t)tok * k + s];
+        o = make_uint4(pack_bf16(bf16lo(q.x) * w, bf16hi(q.x) * w), pack_bf16(bf16lo(q.y) * w, bf16hi(q.y) * w),
+                       pack_bf16(bf16lo(q.z) * w, bf16hi(q.z) * w), pack_bf16(bf16lo(q.w) * w, bf16hi(q.w) * w));
+      }
+      *reinterpret_cast<uint4*>(xp + (size_t)r * H + v * 8) = o;
+    }
+  }
+}
+
+void moe_plan256_launch(const int* topk_i, int entries, int expert_offset, int e_local, int tiles, int* pos, int* tile_expert, cudaStream_t stream) {
+  if (e_local > MOE_MAX_E) throw std::runtime_error("moe_plan: more than 512 local experts");
+  launch_pdl(moe_plan256_kernel, dim3(1), dim3(MOE_PLAN_THREADS), 0, stream, topk_i, entries, expert_offset, e_local, tiles, pos, tile_expert);
+}
+void moe_scatter_launch(const void* x, const float* topk_w, const int* pos, void* xp, int N, int H, int k, int scale_input, cudaStream_t stream) {
+  launch_pdl(moe_scatter_kernel, dim3(N), dim3(256), 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), topk_w, pos,
+             reinterpret_cast<__nv_bfloat16*>(xp), H, k, scale_input);
+}
+
 void moe_plan_launch(const int* topk_i, int entries, int expert_offset, int e_local, int R, int* pos, int* row_entry, int* tile_expert,
                      cudaStream_t stream) {
   if (e_local > MOE_MAX_E) throw std::runtime_error("moe_plan: more than 512 local experts");

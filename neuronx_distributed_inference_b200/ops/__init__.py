@@ -366,6 +366,8 @@ def router_topk(x, weight, top_k, act="softmax", normalize=True, act_over_topk=F
     elementwise / sort launches.  -> (logits, weights [N, k] fp32, expert ids [N, k])."""
     E = weight.shape[0]
     plain_softmax = act == "softmax" and (not normalize or correction is not None or groups is not None)
+    if act == "softmax" and normalize and correction is None and groups is None and not act_over_topk:
+        plain_softmax, renorm_eps = True, 0.0 if renorm_eps is None else renorm_eps          # the chosen weights are divided by their sum
     over_topk = act == "softmax" and act_over_topk and correction is None and groups is None and renorm_eps is None and scale == 1.0
     if (_mix_cuda(x) and (over_topk or ((act == "sigmoid" or plain_softmax) and not act_over_topk)) and weight.dtype == torch.float32
             and x.dim() == 2 and (bias is None or bias.dtype == torch.float32) and top_k <= E and E <= 512 and (groups is None or (E % int(groups[0]) == 0 and int(groups[1]) <= int(groups[0])))):
