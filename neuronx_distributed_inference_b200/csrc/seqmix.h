@@ -94,7 +94,9 @@ struct RouterSelect {
   int groups, keep;          // groups <= 1: no group limit
   float renorm_eps, scale;
 };
-void router_topk_launch(const void* x, const float* w, float* logits, float* topk_w, int* topk_i, int N, int W, int E, int k,
+// `parts`: [router_parts - 1, N, E] partial logits
+int router_parts(int N, int W, int E, bool lp);
+void router_topk_launch(const void* x, const float* w, float* logits, float* parts, float* topk_w, int* topk_i, int N, int W, int E, int k,
                         const RouterSelect& sel, bool lp, cudaStream_t st);
 
 void short_conv_launch(const void* u, long long u_sb, long long u_st, const float* w, const float* bias, const void* state,

@@ -689,7 +689,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> router_topk(const at::Tensor& x, 
     sel.correction = correction->data_ptr<float>();
   }
   sel.groups = (int)groups; sel.keep = (int)keep; sel.renorm_eps = (float)renorm_eps; sel.scale = (float)scale;
-  router_topk_launch(x.data_ptr(), w.data_ptr<float>(), logits.data_ptr<float>(), tw.data_ptr<float>(), ti.data_ptr<int>(), N, W, E, (int)k, sel,
+  const int kparts = router_parts(N, W, E, is_lp(x));
+  auto parts = at::empty({kparts > 1 ? (int64_t)(kparts - 1) * N * E : 0}, f32);
+  router_topk_launch(x.data_ptr(), w.data_ptr<float>(), logits.data_ptr<float>(), parts.data_ptr<float>(), tw.data_ptr<float>(), ti.data_ptr<int>(), N, W, E, (int)k, sel,
                      is_lp(x), stream());
   return {logits, tw, ti};
 }

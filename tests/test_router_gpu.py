@@ -1,0 +1,33 @@
+"""fp32 router on tensor cores (csrc/moe_plain.cu): logits against 64 bits at the edges of its blocks and column parts; choice and weights against the definition.
+
+Bound: products of bf16 rows and split fp32 weights are exact in fp32, sums of at most 64 go through the tensor core (its adder drops bits below
+2^-23 of the running sum: 64 * 2^-23 relative at worst, 1e-7 seen), the rest are fp32 additions; 1e-6 is asked for."""
+import pytest
+import torch
+
+from neuronx_distributed_inference_b200 import ops
+from neuronx_distributed_inference_b200.modules.moe import RouterTopK
+from neuronx_distributed_inference_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("N", [1, 255, 256, 257, 1000, 4097])
+@pytest.mark.parametrize("E,W", [(8, 512), (64, 64), (65, 128), (128, 2048), (300, 192), (512, 1088)])
+def test_logits_and_choice(N, E, W):
+    x = torch.randn(N, W, device="cuda", dtype=torch.bfloat16)
+    w, b = torch.randn(E, W, device="cuda") * 0.05, torch.randn(E, device="cuda")
+    k = min(8, E)
+    for bias in (None, b):
+        logits, weights, ids = ops.router_topk(x, w, k, bias=bias)
+        exact = x.double() @ w.double().t() + (0 if bias is None else bias.double())
+        assert ((logits.double() - exact).norm() / exact.norm()).item() < 1e-6
+        want_w, want_i = ref.moe_route(logits, k)
+        assert torch.equal(ids.long().sort(-1).values, want_i.sort(-1).values)
+        assert torch.allclose(weights.sort(-1).values, want_w.sort(-1).values, rtol=1e-5, atol=1e-7)
+
+
+def test_module_ids_keep_their_type():
+    r = RouterTopK(16, 2, 256, device="cuda")
+    r.linear_router.weight.data.normal_()
+    assert r(torch.randn(5, 256, device="cuda", dtype=torch.bfloat16))[2].dtype == torch.int64
