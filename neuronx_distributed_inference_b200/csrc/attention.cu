@@ -40,6 +40,9 @@ void attention_decode_launch(const AttnDecodeParams& p, cudaStream_t stream) {
   a.tickets = p.tickets;
   a.B = p.B; a.T = p.T; a.Hq = p.Hq; a.Hkv = p.Hkv; a.S = p.S; a.L = p.L; a.nsplit = p.nsplit; a.window = p.window;
   a.block_size = p.block_size; a.max_blocks = p.max_blocks;
+  a.page_shift = -1;
+  for (int s = 0; s < 31; ++s)
+    if (p.block_size == 1 << s) a.page_shift = s;
   a.scale_log2 = p.scale * kLog2e;
   a.qkv = reinterpret_cast<const __nv_bfloat16*>(p.qkv);
   a.cos = p.cos; a.sin = p.sin;

