@@ -281,6 +281,63 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const T* __restrict_
     }
 }
 
+// Logits of up to sixteen experts: the kernel above gives a warp four of them and leaves the other warps of the block idle (eight experts: two of eight
+// warps work).  Here KW warps share the columns of four experts, read the rows and the weights straight from memory (no staging, no barrier in the loop;
+// the row of one warp is in L1 for the next) and their sums are added in order at the end.  Bound by the latency of a few rounds of loads.  Eight experts
+// of 4096 columns, logits and choice together: 6.9 us for 6 tokens, 8.4 for 300 (28 with the kernel above), 9.1 for 1000, 23 for 4096.
+constexpr int RS_EG = 4;
+template <typename T, int RT, int KW>
+__global__ void __launch_bounds__(256) router_logits_split_kernel(const T* __restrict__ x, const float* __restrict__ w, float* __restrict__ logits,
+                                                                  int N, int W, int E) {
+  __shared__ float part[8][RT * RS_EG];
+  const int t0 = blockIdx.x * RT, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int e0 = (warp / KW) * RS_EG;
+  float acc[RT][RS_EG] = {};
+  if (e0 < E) {
+    const float* wr[RS_EG];
+    const T* xr[RT];
+#pragma unroll
+    for (int g = 0; g < RS_EG; ++g) wr[g] = w + (size_t)min(e0 + g, E - 1) * W;
+#pragma unroll
+    for (int t = 0; t < RT; ++t) xr[t] = x + (size_t)min(t0 + t, N - 1) * W;
+#pragma unroll 2
+    for (int c = ((warp % KW) * 32 + lane) * 4; c < W; c += KW * 128) {
+      float4 wv[RS_EG], xv[RT];
+#pragma unroll
+      for (int g = 0; g < RS_EG; ++g) wv[g] = __ldg(reinterpret_cast<const float4*>(wr[g] + c));
+#pragma unroll
+      for (int t = 0; t < RT; ++t) {
+        if constexpr (std::is_same<T, float>::value) {
+          xv[t] = __ldg(reinterpret_cast<const float4*>(xr[t] + c));
+        } else {
+          const uint2 r = __ldg(reinterpret_cast<const uint2*>(xr[t] + c));
+          xv[t] = make_float4(bf16lo(r.x), bf16hi(r.x), bf16lo(r.y), bf16hi(r.y));
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < RT; ++t)
+#pragma unroll
+        for (int g = 0; g < RS_EG; ++g)
+          acc[t][g] = fmaf(xv[t].w, wv[g].w, fmaf(xv[t].z, wv[g].z, fmaf(xv[t].y, wv[g].y, fmaf(xv[t].x, wv[g].x, acc[t][g]))));
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < RT; ++t)
+#pragma unroll
+    for (int g = 0; g < RS_EG; ++g) {
+      const float v = warp_sum(acc[t][g]);
+      if (lane == 0) part[warp][t * RS_EG + g] = v;
+    }
+  __syncthreads();
+  const int i = threadIdx.x, grp = i / (RT * RS_EG), j = i % (RT * RS_EG), t = t0 + j / RS_EG, e = grp * RS_EG + j % RS_EG;
+  if (grp < 8 / KW && t < N && e < E) {
+    float v = part[grp * KW][j];
+#pragma unroll
+    for (int q = 1; q < KW; ++q) v += part[grp * KW + q][j];
+    logits[(size_t)t * E + e] = v;
+  }
+}
+
 // Logits of many bf16 rows on tensor cores at fp32 precision: a fp32 weight is the exact sum of three bf16 parts (8 + 8 + 8 bits), bf16 rows are exact,
 // so every product is exact in fp32 and only the sums round, as in the kernel above.  Block = 32 tokens x 128 experts, 64 columns per round; the
 // weights are split on their way into shared memory, the three partial sums stay apart until the end.  The kernel above is bound by reading the
@@ -488,6 +545,21 @@ void router_topk_launch(const void* x, const float* w, float* logits, float* par
     n_parts = kparts - 1;
     cudaFuncSetAttribute(router_logits_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RTC_SMEM);
     router_logits_tc_kernel<<<dim3((N + RTC_T - 1) / RTC_T, (E + RTC_E - 1) / RTC_E, kparts), RTC_THREADS, RTC_SMEM, st>>>((const __nv_bfloat16*)x, w, logits, parts, N, W, E);
+  } else if (E <= 16 && W % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
+    // tokens per block: one for a few tokens; then four, and eight (half the weight reads) once four would give every SM eight blocks
+    const int srt = few ? 1 : N <= 4 * 8 * kNumSMs ? 4 : 8;
+    auto split = [&](auto kernel, auto xp) { kernel<<<(N + srt - 1) / srt, 256, 0, st>>>(xp, w, logits, N, W, E); };
+    auto by_rows = [&](auto xp, auto kw) {
+      using X = std::remove_cv_t<std::remove_pointer_t<decltype(xp)>>;
+      constexpr int KW = decltype(kw)::value;
+      if (srt == 1) split(router_logits_split_kernel<X, 1, KW>, xp);
+      else if (srt == 4) split(router_logits_split_kernel<X, 4, KW>, xp);
+      else split(router_logits_split_kernel<X, 8, KW>, xp);
+    };
+    auto by_experts = [&](auto xp) {
+      if (E <= 8) by_rows(xp, std::integral_constant<int, 4>()); else by_rows(xp, std::integral_constant<int, 2>());
+    };
+    if (lp) by_experts((const __nv_bfloat16*)x); else by_experts((const float*)x);
   } else if (lp) {
     if (few) go(router_logits_kernel<__nv_bfloat16, 1, 8>, (const __nv_bfloat16*)x); else go(router_logits_kernel<__nv_bfloat16, 4, 8>, (const __nv_bfloat16*)x);
   } else {

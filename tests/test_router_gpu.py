@@ -27,6 +27,22 @@ def test_logits_and_choice(N, E, W):
         assert torch.allclose(weights.sort(-1).values, want_w.sort(-1).values, rtol=1e-5, atol=1e-7)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N", [1, 32, 33, 300, 4737])
+@pytest.mark.parametrize("E,W", [(1, 4), (4, 516), (5, 4096), (8, 132), (9, 1028), (16, 6144), (8, 130)])
+def test_few_experts_share_the_columns(N, E, W, dtype):
+    """Up to 16 experts: the warps of a block share the columns.  fp32 sums of W terms in 32 lanes and up to 4 parts: at most W / 128 + 9 additions in a
+    row, 57 * 2^-24 = 3.4e-6 at worst of the terms' size (4e-7 seen); 1e-6 of the result is asked for."""
+    x = torch.randn(N, W, device="cuda", dtype=dtype)
+    w = torch.randn(E, W, device="cuda") * 0.05
+    logits, weights, ids = ops.router_topk(x, w, min(2, E))
+    exact = x.double() @ w.double().t()
+    assert ((logits.double() - exact).norm() / exact.norm()).item() < 1e-6
+    want_w, want_i = ref.moe_route(logits, min(2, E))
+    assert torch.equal(ids.long().sort(-1).values, want_i.sort(-1).values)
+    assert torch.allclose(weights.sort(-1).values, want_w.sort(-1).values, rtol=1e-5, atol=1e-7)
+
+
 def test_module_ids_keep_their_type():
     r = RouterTopK(16, 2, 256, device="cuda")
     r.linear_router.weight.data.normal_()
