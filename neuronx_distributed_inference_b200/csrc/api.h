@@ -65,7 +65,7 @@ struct GemmRsArgs {
   void* cta_counter;
 };
 void gemm_tcgen05_launch(const void* a, int lda, const void* b, const void* bias, const void* residual, void* c, int ldc, int M,
-                         int N, int K, int act, cudaStream_t stream, const GemmRsArgs* rs = nullptr);
+                         int N, int K, int act, cudaStream_t stream, const GemmRsArgs* rs = nullptr, bool w_fresh = false);
 void rmsnorm_launch(const void* x, const void* res_in, const void* w, void* y, void* res_out, int rows, int H, float eps,
                     float offset, cudaStream_t stream);
 
@@ -96,7 +96,7 @@ void qgemv_launch(const void* x, const void* w, const float* scale, int scale_n,
 
 // prompt-sized GEMM on CTA pairs (gemm_pair.cu); tile_expert: grouped, segments of whole 256-row tiles (moe_plan256)
 void gemm_pair_launch(const void* a, long long lda, const void* b, const void* bias, const void* residual, void* c, int M, int N, int K, int act,
-                      cudaStream_t stream, const int* tile_expert = nullptr, int experts = 1, float limit = 7.f, float alpha = 1.702f);
+                      cudaStream_t stream, const int* tile_expert = nullptr, int experts = 1, float limit = 7.f, float alpha = 1.702f, bool w_fresh = false);
 
 // few tokens x large weights with the weights streamed evenly over the SMs (skinny_gemm.cu): one weight [rows, K], or the experts that have tokens
 constexpr int SKINNY_MAX_T = 128;
@@ -111,6 +111,7 @@ struct SkinnyGemm {
   int experts, tokens;        // tokens: rows of x (one expert), or the most rows an expert can have
   int n_out, K, act;
   float limit, alpha;
+  int w_fresh;                // w was written by a kernel just before: the weight producer waits for it
   const int *n_active, *active, *seg_start, *seg_count;   // grouped: experts with tokens, each expert's rows of x (contiguous); null: one expert
   float* ws;                  // skinny_gemm_ws_floats
   unsigned* tickets;          // skinny_gemm_tickets, zero at launch

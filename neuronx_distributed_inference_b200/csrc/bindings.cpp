@@ -176,8 +176,10 @@ static bool skinny_pays(int M, int rows, int K, bool glu) {
   return M <= 64 || (M <= SKINNY_MAX_T && K >= 2 * rows);
 }
 
+// fresh_weight: w was written by a kernel enqueued just before (an expanded 8-bit weight).  The kernels fetch a parameter's first tiles before the
+// kernels in front of them have finished; such a weight has to be waited for.
 at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int64_t act,
-                const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& out) {
+                const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& out, bool fresh_weight) {
   TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1));
   TORCH_CHECK(is_bf16(x) && is_bf16(w) && x.stride(1) == 1 && w.is_contiguous());
   const int M = x.size(0), K = x.size(1), N = w.size(0);
@@ -198,6 +200,7 @@ at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
     SkinnyGemm a{};
     a.x = x.data_ptr(); a.x_rows = M; a.ldx = x.stride(0); a.w = w.data_ptr(); a.bias = optr(bias); a.residual = optr(residual); a.y = y.data_ptr();
     a.experts = 1; a.tokens = M; a.n_out = n_out; a.K = K; a.act = (int)act; a.limit = 7.f; a.alpha = 1.702f;
+    a.w_fresh = fresh_weight ? 1 : 0;
     a.ws = ws.data_ptr<float>();
     a.tickets = reinterpret_cast<unsigned*>(ws.data_ptr<float>() + nf);
     skinny_clear_launch(a.tickets, (int)nt, cur_stream());
@@ -205,11 +208,12 @@ at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
     return y;
   }
   if (pair_pays(M, n_out, glu)) {
-    gemm_pair_launch(x.data_ptr(), x.stride(0), w.data_ptr(), optr(bias), optr(residual), y.data_ptr(), M, N, K, (int)act, cur_stream());
+    gemm_pair_launch(x.data_ptr(), x.stride(0), w.data_ptr(), optr(bias), optr(residual), y.data_ptr(), M, N, K, (int)act, cur_stream(),
+                     nullptr, 1, 7.f, 1.702f, fresh_weight);
     return y;
   }
   gemm_tcgen05_launch(x.data_ptr(), (int)x.stride(0), w.data_ptr(), optr(bias), optr(residual), y.data_ptr(), n_out, M, N, K,
-                      (int)act, cur_stream());
+                      (int)act, cur_stream(), nullptr, fresh_weight);
   return y;
 }
 
@@ -313,17 +317,18 @@ at::Tensor moe_small(const at::Tensor& x, const at::Tensor& w_gate_up, const at:
   return out;
 }
 
-// int8 / fp8 weight [N, K] x scale -> bf16 into `out` (a caller-owned scratch: one buffer serves every layer of a model)
-at::Tensor dequant_bf16(const at::Tensor& w, const at::Tensor& scale, at::Tensor out) {
+// int8 / fp8 weight [N, K] x scale -> bf16.  A result per call: two streams may expand weights at the same time, and the stream order of the caching
+// allocator hands the same memory to the next layer
+at::Tensor dequant_bf16(const at::Tensor& w, const at::Tensor& scale) {
   TORCH_CHECK(w.is_cuda() && w.dim() == 2 && w.is_contiguous() && scale.scalar_type() == at::kFloat && scale.is_contiguous());
   const bool i8 = w.scalar_type() == at::kChar;
   TORCH_CHECK(i8 || w.scalar_type() == at::kFloat8_e4m3fn, "dequant_bf16: int8 or float8_e4m3fn weights");
   TORCH_CHECK(scale.numel() == 1 || scale.numel() == w.size(0));
-  TORCH_CHECK(out.is_cuda() && is_bf16(out) && out.is_contiguous() && out.numel() >= w.numel());
   c10::cuda::CUDAGuard guard(w.device());
+  auto out = at::empty({w.size(0), w.size(1)}, w.options().dtype(at::kBFloat16));
   dequant_bf16_launch(w.data_ptr(), i8 ? 1 : 2, scale.data_ptr<float>(), (int)scale.numel(), out.data_ptr(), (int)w.size(0), (int)w.size(1),
                       cur_stream());
-  return out.flatten().narrow(0, 0, w.numel()).view({w.size(0), w.size(1)});
+  return out;
 }
 
 // Routed experts of a prefill-sized batch (any N): permutation on the device + two grouped tcgen05 GEMMs + weighted combine.
@@ -855,7 +860,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_small", &nxdi::moe_small);
   m.def("moe_grouped", &nxdi::moe_grouped);
   m.def("dequant_bf16", &nxdi::dequant_bf16);
-  m.def("gemm", &nxdi::gemm);
+  m.def("gemm", &nxdi::gemm, pybind11::arg("x"), pybind11::arg("w"), pybind11::arg("bias"), pybind11::arg("act"), pybind11::arg("residual"),
+        pybind11::arg("out"), pybind11::arg("fresh_weight") = false);
   m.def("symm_alloc", &nxdi::symm_alloc);
   m.def("symm_open", &nxdi::symm_open);
   m.def("symm_close", &nxdi::symm_close);

@@ -39,6 +39,7 @@ struct PairParams {
   int M, N, K, n_out, act;        // act: 0 none, 1 silu*up, 2 gelu_tanh*up, 3 gelu*up, 4 clamped gate product (n_out = N / 2)
   float limit, alpha;
   int m_tiles, n_tiles, band;
+  int w_fresh;                    // B was written by a kernel just before this one
   const int* tile_expert;         // grouped: [m_tiles] expert | rows with tokens << 10 of a 256-row tile, < 0: not in use; null: one weight
 };
 
@@ -157,8 +158,8 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
   pdl_launch_dependents();
-  // one weight does not depend on earlier kernels; everything else does
-  if (!(warp == 0 && p.tile_expert == nullptr)) pdl_wait();
+  // a weight that is a parameter does not depend on earlier kernels; everything else does
+  if (warp != 0 || p.tile_expert != nullptr || p.w_fresh) pdl_wait();
 
   if (warp == 0 || warp == 3) {
     // ================= TMA producers: B (warp 0), A (warp 3) of this CTA =================
@@ -356,7 +357,7 @@ static int gp_sms() {
 
 // a [M, K] (row stride lda), b [experts * N, K], c [M, n_out]; tile_expert (device, [M / 256]) for the grouped flavour
 void gemm_pair_launch(const void* a, long long lda, const void* b, const void* bias, const void* residual, void* c, int M, int N, int K, int act,
-                      cudaStream_t stream, const int* tile_expert, int experts, float limit, float alpha) {
+                      cudaStream_t stream, const int* tile_expert, int experts, float limit, float alpha, bool w_fresh) {
   if (K % GP_BK != 0 || M < 1) throw std::runtime_error("gemm pair: K must be a multiple of 64");
   if (tile_expert != nullptr && M % 256 != 0) throw std::runtime_error("gemm pair: the permuted row bound must be a multiple of 256");
   PairParams p{};
@@ -365,7 +366,7 @@ void gemm_pair_launch(const void* a, long long lda, const void* b, const void* b
   p.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   p.c = reinterpret_cast<__nv_bfloat16*>(c);
   p.M = M; p.N = N; p.K = K; p.act = act; p.n_out = glu ? N / 2 : N; p.limit = limit; p.alpha = alpha;
-  p.tile_expert = tile_expert;
+  p.tile_expert = tile_expert; p.w_fresh = w_fresh ? 1 : 0;
   const int tile_out = glu ? GP_BN / 2 : GP_BN;
   p.m_tiles = (M + 255) / 256;
   p.n_tiles = (p.n_out + tile_out - 1) / tile_out;

@@ -69,6 +69,7 @@ struct GemmParams {
   // with the rows of expert grp_tile_expert[mt] (< 0: tile not in use this step, skipped by every role).  M is the STATIC upper
   // bound of permuted rows, so the launch is shape-stable under CUDA graphs whatever the routing.
   const int* grp_tile_expert;
+  int w_fresh;                          // B was written by a kernel just before this one: its producer waits like the others
 };
 
 __device__ __forceinline__ uint32_t s_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -203,8 +204,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tcgen05_kernel(const __gri
     // kernel), warp 3 the ACTIVATION tile (one 256-row box when TM = 2) — both post to the same full barrier.
     if (lane == 0) {
       const bool is_b = warp == 0;
-      // (grouped: the routing plan comes from the preceding kernels, so the weight producer waits too)
-      if (!is_b || p.grp_tile_expert != nullptr) pdl_wait();
+      // (grouped: the routing plan comes from the preceding kernels; fresh: the weight does — the weight producer waits too)
+      if (!is_b || p.grp_tile_expert != nullptr || p.w_fresh) pdl_wait();
       long long it = 0;   // k-block counter across work items (ring position)
       for (int w = blockIdx.x; w < total_tiles; w += gridDim.x) {
         const int t = w / S, ks = w % S;
@@ -613,8 +614,10 @@ static unsigned* gemm_tickets() {
 
 static void gemm_launch_impl(const void* a, int lda, const void* b, const void* bias, const void* residual, void* c, int ldc, int M, int N,
                              int K, int act, cudaStream_t stream, const GemmRsArgs* rs, const float* a_scale, const float* w_scale,
-                             int w_scale_n, const int* tile_expert = nullptr, int n_experts = 1, float glu_limit = 7.f, float glu_alpha = 1.702f) {
+                             int w_scale_n, const int* tile_expert = nullptr, int n_experts = 1, float glu_limit = 7.f, float glu_alpha = 1.702f,
+                             bool w_fresh = false) {
   GemmParams p{};
+  p.w_fresh = w_fresh ? 1 : 0;
   p.grp_tile_expert = tile_expert;
   const bool glu = act != 0;
   const bool fp8 = a_scale != nullptr;
@@ -761,8 +764,8 @@ static void gemm_launch_impl(const void* a, int lda, const void* b, const void* 
 }
 
 void gemm_tcgen05_launch(const void* a, int lda, const void* b, const void* bias, const void* residual, void* c, int ldc, int M,
-                         int N, int K, int act, cudaStream_t stream, const GemmRsArgs* rs) {
-  gemm_launch_impl(a, lda, b, bias, residual, c, ldc, M, N, K, act, stream, rs, nullptr, nullptr, 0);
+                         int N, int K, int act, cudaStream_t stream, const GemmRsArgs* rs, bool w_fresh) {
+  gemm_launch_impl(a, lda, b, bias, residual, c, ldc, M, N, K, act, stream, rs, nullptr, nullptr, 0, nullptr, 1, 7.f, 1.702f, w_fresh);
 }
 
 // grouped GEMM of the mixture-of-experts layers: a [R, K] tokens permuted by expert (R % 128 == 0), b [E, N, K] stacked expert

@@ -99,11 +99,12 @@ void rmsnorm_quant_launch(const void* x, const void* gamma, void* q, float* scal
 
 // Weight-only 8-bit layers at prefill sizes without activation quantisation: expand W (int8 / fp8-e4m3, per-channel or per-tensor
 // scale) to bf16 ONCE per call into a scratch buffer (1 B read + 2 B written per weight; the copy is consumed from L2 by the
-// tcgen05 GEMM that follows) instead of the three elementwise passes of the PyTorch composite.
+// tcgen05 GEMM that follows, which therefore waits for it before its first weight tile: `fresh_weight`) instead of the three elementwise passes of the PyTorch composite.
 template <int WT>
 __global__ void __launch_bounds__(256) dequant_bf16_kernel(const uint8_t* __restrict__ w, const float* __restrict__ scale, int scale_n,
                                                            __nv_bfloat16* __restrict__ out, int N, int K) {
   pdl_launch_dependents();
+  pdl_wait();                                  // `out` is recycled memory: an earlier GEMM may still be reading what it held
   const int kv = K >> 4;                       // 16-byte vectors per row
   const long long total = (long long)N * kv;
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {

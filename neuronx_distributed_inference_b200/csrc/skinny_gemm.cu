@@ -36,7 +36,7 @@ struct SkinnyKernelParams {
   void* y;                 // [token rows, n_out] bf16, or fp32 (y_f32)
   float* ws;               // [G][2][cols / 4][128][4] partial tiles
   unsigned* tickets;       // [G], zero at launch
-  int T, n_out, rows, K, act, xb, xbox, stages, y_f32, tmem_cols;
+  int T, n_out, rows, K, act, xb, xbox, stages, y_f32, tmem_cols, w_fresh;
   float limit, alpha;
 };
 
@@ -127,9 +127,9 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
   pdl_launch_dependents();
-  // dense weights do not depend on earlier kernels; everything else does
+  // a dense weight that is a parameter does not depend on earlier kernels; everything else does
   const bool grouped = p.n_active != nullptr;
-  if (!(warp == 0 && !grouped)) pdl_wait();
+  if (warp != 0 || grouped || p.w_fresh) pdl_wait();
 
   const int n_tiles = (p.n_out + SK_BM - 1) / SK_BM, nkb = p.K / SK_BK;
   const long long total = (long long)(grouped ? *p.n_active : 1) * n_tiles * nkb;
@@ -400,7 +400,7 @@ void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream) {
   p.bias = reinterpret_cast<const __nv_bfloat16*>(a.bias);
   p.residual = reinterpret_cast<const __nv_bfloat16*>(a.residual);
   p.y = a.y; p.y_f32 = a.y_f32; p.ws = a.ws; p.tickets = a.tickets;
-  p.T = a.tokens; p.n_out = a.n_out; p.K = a.K; p.act = a.act; p.limit = a.limit; p.alpha = a.alpha;
+  p.T = a.tokens; p.n_out = a.n_out; p.K = a.K; p.act = a.act; p.limit = a.limit; p.alpha = a.alpha; p.w_fresh = a.w_fresh;
   const int stage = (glu ? 2 : 1) * SK_W_BYTES + p.xb * SK_BK * 2;
   p.stages = std::min(SK_MAX_STAGES, (SK_SMEM - 1024) / stage);
   int cols = 32;

@@ -91,7 +91,7 @@ def linear(x, w, bias=None, norm_weight=None, norm_eps: float = 1e-6, norm_offse
         wq = w.dtype in (torch.int8, torch.float8_e4m3fn)
         ok_w = (w.dtype == x.dtype and scale is None) or (wq and scale is not None and scale.dim() == 1)
         if ok_w and act in _ACT_CODES and w.is_contiguous():
-            x2 = x.reshape(T, K)
+            x2, fresh = x.reshape(T, K), False
             if wq and T <= GEMV_MAX_TOKENS and K % 16 == 0 and w.dim() == 2:
                 stats["qgemv"] += 1
                 r2 = residual.reshape(T, -1).contiguous() if (residual is not None and act is None) else None
@@ -117,16 +117,16 @@ def linear(x, w, bias=None, norm_weight=None, norm_eps: float = 1e-6, norm_offse
                 return y if (residual is None or r2 is not None) else y + residual
             if (wq and T > GEMV_MAX_TOKENS and w.dim() == 2 and K % 64 == 0 and n_out % 8 == 0 and _TCGEN05_GEMM
                     and x.dtype == torch.bfloat16):
-                # weight-only 8-bit prefill: one expansion pass into a shared bf16 scratch (stays in L2), then the bf16 tensor-core GEMM
+                # weight-only 8-bit prefill: one expansion pass to bf16 (stays in L2), then the bf16 tensor-core GEMM, which waits for it
                 stats["dequant_gemm"] += 1
-                w, scale, wq = _C().dequant_bf16(w, scale.float().contiguous(), _dequant_scratch(w)), None, False
+                w, scale, wq, fresh = _C().dequant_bf16(w, scale.float().contiguous()), None, False, True
             if not wq and n_out % 8 == 0 and K % 64 == 0 and _TCGEN05_GEMM and (T > GEMV_MAX_TOKENS or K % 64 != 0):
                 if norm_weight is not None:
                     x2 = rmsnorm(x2, norm_weight, norm_eps, norm_offset)
                 stats["gemm_tcgen05"] += 1
                 r2 = residual.reshape(T, -1) if (residual is not None and act is None) else None
                 o2 = out.view(T, -1) if out is not None else None
-                y = _C().gemm(x2.contiguous(), w, bias, _ACT_CODES[act], r2, o2)
+                y = _C().gemm(x2.contiguous(), w, bias, _ACT_CODES[act], r2, o2, fresh)
                 y = out if out is not None else y.view(*x.shape[:-1], y.shape[-1])
                 return y if (residual is None or r2 is not None) else y + residual
     if act in _GATE_PRODUCTS and _mix_cuda(x) and w.dtype == x.dtype and scale is None and x.dim() >= 2:
@@ -142,22 +142,6 @@ def linear(x, w, bias=None, norm_weight=None, norm_eps: float = 1e-6, norm_offse
         out.copy_(y)
         return out
     return y
-
-
-_DEQ_SCRATCH = {}
-_DEQ_RETIRED = []
-
-
-def _dequant_scratch(w):
-    """One bf16 scratch per device, grown to the largest 8-bit weight seen (consumed by the GEMM enqueued right after the expansion;
-    stream order makes the reuse by the next layer safe)."""
-    buf = _DEQ_SCRATCH.get(w.device)
-    if buf is None or buf.numel() < w.numel():
-        if buf is not None:
-            _DEQ_RETIRED.append(buf)      # never freed: CUDA graphs captured with the smaller scratch still hold its address
-        buf = torch.empty(w.numel(), dtype=torch.bfloat16, device=w.device)
-        _DEQ_SCRATCH[w.device] = buf
-    return buf
 
 
 def linear_allreduce(x, w, bias, group, residual=None, reduce_dtype=None, scale=None):

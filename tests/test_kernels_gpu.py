@@ -430,7 +430,7 @@ def test_quantized_gemv_matches_dequantized_reference(wdtype, T, N, K, act, norm
 
 @pytest.mark.parametrize("wdtype", [torch.int8, torch.float8_e4m3fn])
 def test_weight_only_prefill_expands_once_then_tensor_core_gemm(wdtype):
-    """T > 8 with 8-bit weights and no activation quantisation: one dequantise-to-bf16 pass into the shared scratch + tcgen05 GEMM."""
+    """T > 8 with 8-bit weights and no activation quantisation: one dequantise-to-bf16 pass + tcgen05 GEMM."""
     torch.manual_seed(0)
     T, N, K = 256, 2 * 1408, 1024
     q, s = ref.quantize_per_channel(torch.randn(N, K, device="cuda") * 0.05, wdtype)
