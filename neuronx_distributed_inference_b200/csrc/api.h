@@ -108,20 +108,21 @@ struct SkinnyGemm {
   const void* residual;       // [tokens, n_out] bf16 or null (one expert, act == 0)
   void* y;                    // [x_rows, n_out] bf16, or fp32 with y_f32
   int y_f32;
-  int experts, tokens;        // tokens: rows of x (one expert), or the most rows an expert can have
+  int experts, tokens;        // tokens: rows of x (one expert), or the most rows of a segment
   int n_out, K, act;
   float limit, alpha;
   int w_fresh;                // w was written by a kernel just before: the weight producer waits for it
-  const int *n_active, *active, *seg_start, *seg_count;   // grouped: experts with tokens, each expert's rows of x (contiguous); null: one expert
+  const int *n_active, *active, *seg_start, *seg_count;   // grouped: number of segments; each one's expert, first row of x and rows; null: one expert
   float* ws;                  // skinny_gemm_ws_floats
   unsigned* tickets;          // skinny_gemm_tickets, zero at launch
 };
+int skinny_gemm_rows(int tokens);          // `tokens` rounded up to what a segment may hold
 long long skinny_gemm_ws_floats(int tokens, bool glu);
 int skinny_gemm_tickets();
 void skinny_clear_launch(unsigned* tickets, int n, cudaStream_t stream);
 void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream);
 void moe_small_gather_launch(const void* x, const float* topk_w, const int* topk_i, int entries, int k, int H, int expert_offset, int e_local,
-                             int scale_input, void* xp, int* pos, int* n_active, int* active, int* seg_start, int* seg_count, unsigned* tickets,
+                             int seg_rows, int scale_input, void* xp, int* pos, int* n_active, int* active, int* seg_start, int* seg_count, unsigned* tickets,
                              int n_tickets, cudaStream_t stream);
 void moe_small_combine_launch(const float* y, const float* topk_w, const int* pos, void* out, int N, int H, int k, int scale_input, cudaStream_t stream);
 

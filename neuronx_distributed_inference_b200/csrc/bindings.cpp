@@ -296,14 +296,18 @@ at::Tensor moe_small(const at::Tensor& x, const at::Tensor& w_gate_up, const at:
   auto iopt = x.options().dtype(at::kInt), fopt = x.options().dtype(at::kFloat);
   auto xp = at::empty({R, H}, x.options()), h = at::empty({R, I}, x.options()), out = at::empty({N, H}, x.options());
   auto y = at::empty({R, H}, fopt);
-  auto meta = at::empty({R + 1 + 3 * (int64_t)E + 2 * nt}, iopt);       // pos | n_active | active | seg_start | seg_count | tickets of both GEMMs
+  // an expert has at most N entries when every token names it once, but nothing forbids a token to name it again (k times N): its rows are cut into
+  // segments of what the GEMM's token tile holds
+  const int seg_rows = skinny_gemm_rows(N);
+  const int64_t segs = std::min<int64_t>(E, R) + R / seg_rows;
+  auto meta = at::empty({R + 1 + 3 * segs + 2 * nt}, iopt);       // pos | n_active | active | seg_start | seg_count | tickets of both GEMMs
   auto ws = at::empty({std::max(skinny_gemm_ws_floats(N, true), skinny_gemm_ws_floats(N, false))}, fopt);
   int* pos = meta.data_ptr<int>();
-  int *n_active = pos + R, *active = n_active + 1, *seg_start = active + E, *seg_count = seg_start + E;
-  unsigned* tickets = reinterpret_cast<unsigned*>(seg_count + E);
+  int *n_active = pos + R, *active = n_active + 1, *seg_start = active + segs, *seg_count = seg_start + segs;
+  unsigned* tickets = reinterpret_cast<unsigned*>(seg_count + segs);
   auto st = cur_stream();
-  moe_small_gather_launch(x.data_ptr(), topk_w.data_ptr<float>(), topk_i.data_ptr<int>(), (int)R, k, H, (int)expert_offset, E, scale_input ? 1 : 0,
-                          xp.data_ptr(), pos, n_active, active, seg_start, seg_count, tickets, (int)(2 * nt), st);
+  moe_small_gather_launch(x.data_ptr(), topk_w.data_ptr<float>(), topk_i.data_ptr<int>(), (int)R, k, H, (int)expert_offset, E, seg_rows,
+                          scale_input ? 1 : 0, xp.data_ptr(), pos, n_active, active, seg_start, seg_count, tickets, (int)(2 * nt), st);
   SkinnyGemm a{};
   a.x = xp.data_ptr(); a.x_rows = R; a.ldx = H; a.w = w_gate_up.data_ptr(); a.bias = optr(gate_up_bias); a.y = h.data_ptr();
   a.experts = E; a.tokens = N; a.n_out = I; a.K = H; a.act = (int)act; a.limit = (float)limit; a.alpha = (float)alpha;

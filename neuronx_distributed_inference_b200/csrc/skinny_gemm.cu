@@ -3,7 +3,7 @@
 // 128-row token tiles would be mostly padding and whose tile grid leaves a last wave nearly empty).
 //
 // What bounds it: the weight stream from HBM.  So
-//   * CTA c of G takes the k-blocks [total c / G, total (c + 1) / G) of the concatenated (expert, 128-feature tile, k) space: every SM streams the
+//   * CTA c of G takes the k-blocks [total c / G, total (c + 1) / G) of the concatenated (segment, 128-feature tile, k) space: every SM streams the
 //     same number of bytes whatever the shape (stream-K).  Tiles cut by a boundary meet in fp32 partials; the CTA that arrives last adds them in
 //     k order (deterministic) and runs the epilogue.
 //   * a stage is a 128 x 64 weight box (two for gate | up) plus the tokens' 64 columns; the ring takes all of shared memory (100 .. 180 KB of weights
@@ -31,7 +31,7 @@ constexpr int SK_SMEM = 220 * 1024;
 struct SkinnyKernelParams {
   CUtensorMap tm_w;        // [experts * rows, K], box {64, 128}
   CUtensorMap tm_x;        // [token rows, K], box {64, xbox}: xb rows for one expert, 16 when grouped (an expert loads as many as it has tokens for)
-  const int *n_active, *active, *seg_start, *seg_count;     // grouped: experts with tokens and their rows of x; null: one expert, T rows
+  const int *n_active, *active, *seg_start, *seg_count;     // grouped: segments (expert, first row of x, rows <= xb); null: one expert, T rows
   const __nv_bfloat16 *bias, *residual;                      // [experts * rows]; [T, n_out] (one expert)
   void* y;                 // [token rows, n_out] bf16, or fp32 (y_f32)
   float* ws;               // [G][2][cols / 4][128][4] partial tiles
@@ -145,8 +145,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
       for (long long u = u0; u < u1 && go;) {
         const int tile = (int)(u / nkb), kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u));
         const int ei = tile / n_tiles, n0 = (tile % n_tiles) * SK_BM, e = grouped ? p.active[ei] : 0;
-        const int row_w = e * p.rows + n0, row_x = grouped ? p.seg_start[e] : 0;
-        const int boxes = grouped ? (min(p.seg_count[e], p.xb) + p.xbox - 1) / p.xbox : 1, box_bytes = p.xbox * SK_BK * 2;
+        const int row_w = e * p.rows + n0, row_x = grouped ? p.seg_start[ei] : 0;
+        const int boxes = grouped ? (p.seg_count[ei] + p.xbox - 1) / p.xbox : 1, box_bytes = p.xbox * SK_BK * 2;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = (int)(it % ST);
           go = sk_wait(&empty_bar[s], (uint32_t)((it / ST) & 1) ^ 1u, stop);
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
       for (long long u = u0; u < u1 && go; ++seg) {
         const int kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u)), buf = seg & 1;
         // D = f32, A = B = bf16, both K-major, M = 128, N = the tokens in whole boxes (a multiple of 16)
-        const int nx = grouped ? (min(p.seg_count[p.active[(int)(u / nkb) / n_tiles]], p.xb) + 15) / 16 * 16 : p.xb;
+        const int nx = grouped ? (p.seg_count[(int)(u / nkb) / n_tiles] + 15) / 16 * 16 : p.xb;
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nx >> 3) << 17) | ((uint32_t)(SK_BM >> 4) << 24);
         go = sk_wait(&tmem_empty[buf], (uint32_t)((seg >> 1) & 1) ^ 1u, stop);
         if (!go) break;
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
       const int tile = (int)(u / nkb), kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u)), buf = seg & 1;
       u += kb1 - kb0;
       const int ei = tile / n_tiles, n = (tile % n_tiles) * SK_BM + n_in, e = grouped ? p.active[ei] : 0;
-      const int row0 = grouped ? p.seg_start[e] : 0, cnt = grouped ? min(p.seg_count[e], p.xb) : p.T;
+      const int row0 = grouped ? p.seg_start[ei] : 0, cnt = grouped ? p.seg_count[ei] : p.T;
       if (!sk_wait(&tmem_full[buf], (uint32_t)((seg >> 1) & 1), stop)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem + lanes + (uint32_t)(buf * acc_cols);
@@ -373,10 +373,10 @@ static int sk_grid() {
   }();
   return n;
 }
-static int sk_xb(int tokens) { return std::max(16, (tokens + 15) / 16 * 16); }
+int skinny_gemm_rows(int tokens) { return std::max(16, (tokens + 15) / 16 * 16); }
 
 // floats of partial tiles a launch may need
-long long skinny_gemm_ws_floats(int tokens, bool glu) { return (long long)sk_grid() * 2 * sk_xb(tokens) * (glu ? 2 : 1) * SK_BM; }
+long long skinny_gemm_ws_floats(int tokens, bool glu) { return (long long)sk_grid() * 2 * skinny_gemm_rows(tokens) * (glu ? 2 : 1) * SK_BM; }
 int skinny_gemm_tickets() { return sk_grid(); }
 
 // one block between the kernel that produces x and the GEMM: the GEMM's CTAs are already filling their rings meanwhile
@@ -392,7 +392,7 @@ void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream) {
   SkinnyKernelParams p{};
   const bool glu = a.act != 0;
   p.rows = glu ? 2 * a.n_out : a.n_out;
-  p.xb = sk_xb(a.tokens);
+  p.xb = skinny_gemm_rows(a.tokens);
   sk_map(&p.tm_w, a.w, (long long)a.experts * p.rows, a.K, a.K, SK_BM);
   p.xbox = a.n_active ? 16 : p.xb;
   sk_map(&p.tm_x, a.x, a.x_rows, a.K, a.ldx, p.xbox);
@@ -415,10 +415,11 @@ void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream) {
 
 // ---- routed experts of a small step -------------------------------------------------------------------------------------------------------
 // One block per (token, slot) entry: its row among the entries sorted by (expert, entry) — counted, so the order is the same every time —
-// and a copy of the token's row to that place.  Block 0 also writes the experts' segments and clears the tickets of the two GEMMs.
+// and a copy of the token's row to that place.  Block 0 also writes the segments (an expert's rows, cut every seg_rows of them) and clears the tickets
+// of the two GEMMs.
 __global__ void __launch_bounds__(256) moe_small_gather_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ topk_w,
                                                                const int* __restrict__ topk_i, int entries, int k, int H, int expert_offset, int e_local,
-                                                               int scale_input, __nv_bfloat16* __restrict__ xp, int* __restrict__ pos,
+                                                               int seg_rows, int scale_input, __nv_bfloat16* __restrict__ xp, int* __restrict__ pos,
                                                                int* __restrict__ n_active, int* __restrict__ active, int* __restrict__ seg_start,
                                                                int* __restrict__ seg_count, unsigned* __restrict__ tickets, int n_tickets) {
   pdl_launch_dependents();
@@ -452,35 +453,37 @@ __global__ void __launch_bounds__(256) moe_small_gather_kernel(const __nv_bfloat
     }
   }
   if (i == 0) {
-    __shared__ int s_cnt[512], s_act;
+    __shared__ int s_cnt[512];
     for (int c = tid; c < e_local; c += 256) s_cnt[c] = 0;
-    if (tid == 0) s_act = 0;
     __syncthreads();
     for (int j = tid; j < entries; j += 256) {
       const int ej = topk_i[j] - expert_offset;
       if (ej >= 0 && ej < e_local) atomicAdd(&s_cnt[ej], 1);
     }
     __syncthreads();
-    if (tid < 32) {                       // exclusive scans of the counts and of "has tokens", 32 experts at a time
-      int rows = 0, acts = 0;
+    if (tid < 32) {                       // exclusive scans of the counts and of the segments, 32 experts at a time
+      int rows = 0, segs = 0;
       for (int c0 = 0; c0 < e_local; c0 += 32) {
         const int c = c0 + tid, n = c < e_local ? s_cnt[c] : 0;
-        int incl = n;
+        const int ns = (n + seg_rows - 1) / seg_rows;
+        int incl = n, sincl = ns;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-          const int t = __shfl_up_sync(0xffffffffu, incl, o);
-          if (tid >= o) incl += t;
+          const int t = __shfl_up_sync(0xffffffffu, incl, o), ts = __shfl_up_sync(0xffffffffu, sincl, o);
+          if (tid >= o) {
+            incl += t;
+            sincl += ts;
+          }
         }
-        const unsigned has = __ballot_sync(0xffffffffu, n > 0);
-        if (c < e_local) {
-          seg_start[c] = rows + incl - n;
-          seg_count[c] = n;
+        for (int j = 0, s = segs + sincl - ns; j < n; j += seg_rows, ++s) {
+          active[s] = c;
+          seg_start[s] = rows + incl - n + j;
+          seg_count[s] = min(seg_rows, n - j);
         }
-        if (n > 0) active[acts + __popc(has & ((1u << tid) - 1u))] = c;
         rows += __shfl_sync(0xffffffffu, incl, 31);
-        acts += __popc(has);
+        segs += __shfl_sync(0xffffffffu, sincl, 31);
       }
-      if (tid == 0) *n_active = acts;
+      if (tid == 0) *n_active = segs;
     }
     for (int t = tid; t < n_tickets; t += 256) tickets[t] = 0u;
   }
@@ -505,11 +508,11 @@ __global__ void __launch_bounds__(256) moe_small_combine_kernel(const float* __r
 }
 
 void moe_small_gather_launch(const void* x, const float* topk_w, const int* topk_i, int entries, int k, int H, int expert_offset, int e_local,
-                             int scale_input, void* xp, int* pos, int* n_active, int* active, int* seg_start, int* seg_count, unsigned* tickets,
+                             int seg_rows, int scale_input, void* xp, int* pos, int* n_active, int* active, int* seg_start, int* seg_count, unsigned* tickets,
                              int n_tickets, cudaStream_t stream) {
   if (e_local > 512 || H % 8 != 0) throw std::runtime_error("moe (small step): at most 512 experts, hidden size % 8 == 0");
   launch_pdl(moe_small_gather_kernel, dim3(entries), dim3(256), 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), topk_w, topk_i, entries, k, H,
-             expert_offset, e_local, scale_input, reinterpret_cast<__nv_bfloat16*>(xp), pos, n_active, active, seg_start, seg_count, tickets, n_tickets);
+             expert_offset, e_local, seg_rows, scale_input, reinterpret_cast<__nv_bfloat16*>(xp), pos, n_active, active, seg_start, seg_count, tickets, n_tickets);
 }
 void moe_small_combine_launch(const float* y, const float* topk_w, const int* pos, void* out, int N, int H, int k, int scale_input, cudaStream_t stream) {
   launch_pdl(moe_small_combine_kernel, dim3((H / 4 + 255) / 256, N), dim3(256), 0, stream, y, topk_w, pos, reinterpret_cast<__nv_bfloat16*>(out), H, k,

@@ -63,3 +63,24 @@ def test_experts(N, E, k, H, I, offset, local, form):
         assert not got.any()
     else:
         assert _rel(got, want) < 5e-3
+
+
+@pytest.mark.parametrize("N", [3, 16, 17, 33, 128])
+@pytest.mark.parametrize("form", ["twice", "all slots", "shard"])
+def test_a_token_may_name_an_expert_again(N, form):
+    """An expert then owns up to N * k rows, more than one token tile of the GEMM holds."""
+    E, k, H, I = 8, 4, 256, 192
+    x = torch.randn(N, H, device=DEV, dtype=BF)
+    wg = (torch.randn(E, 2 * I, H, device=DEV) / math.sqrt(H)).to(BF)
+    wd = (torch.randn(E, H, I, device=DEV) / math.sqrt(I)).to(BF)
+    w = torch.rand(N, k, device=DEV)
+    i = torch.randint(0, E, (N, k), device=DEV)
+    offset = 2 if form == "shard" else 0
+    if form == "all slots":
+        i[:] = 5
+    else:
+        i[:, 1] = i[:, 0] = 3
+    wg, wd = wg[:E - offset].contiguous(), wd[:E - offset].contiguous()
+    got = ops.moe_experts(x, wg, wd, w, i, "silu_mul", offset)
+    want = ref.moe_experts(x.float(), wg.float(), wd.float(), w, i, "silu_mul", offset)
+    assert _rel(got, want) < 5e-3
