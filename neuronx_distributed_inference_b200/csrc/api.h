@@ -94,6 +94,12 @@ void qgemv_launch(const void* x, const void* w, const float* scale, int scale_n,
                   const void* residual, void* y, int T, int N, int K, int ldx, int ldy, int act, int wdtype, float eps,
                   float norm_offset, int n_sms, cudaStream_t stream);
 
+// bounded waits of the tensor-core kernels (mbar_wait.cuh, kernel_status.cu): where a kernel reports a wait that ran out; raising for it on the host
+enum WaitKernel { WAIT_ATTENTION, WAIT_GEMM_PAIR, WAIT_SKINNY, WAIT_PROBE, WAIT_KERNELS };
+unsigned* wait_word(WaitKernel which);
+void check_waits();
+void wait_probe_launch(long long clocks, int* out, cudaStream_t stream);
+
 // prompt-sized GEMM on CTA pairs (gemm_pair.cu); tile_expert: grouped, segments of whole 256-row tiles (moe_plan256)
 void gemm_pair_launch(const void* a, long long lda, const void* b, const void* bias, const void* residual, void* c, int M, int N, int K, int act,
                       cudaStream_t stream, const int* tile_expert = nullptr, int experts = 1, float limit = 7.f, float alpha = 1.702f, bool w_fresh = false);

@@ -31,6 +31,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "mbar_wait.cuh"
 #include "seqmix.h"
 
 namespace nxdi {
@@ -51,49 +52,25 @@ struct FaParams {
   int gate_per_head, gate_vec;
   int B, T, Hq, Hkv, causal, window, keep, chunk, pair_heads;
   float scale, softcap;
+  unsigned* wait_word;                  // mbar_wait.cuh
 };
 
-__device__ unsigned fa_gave_up;         // waits that ran out (a protocol error; the results of that launch are not valid)
-
-__device__ __forceinline__ uint32_t fa_s32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void fa_mb_init(uint64_t* b, uint32_t n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(fa_s32(b)), "r"(n)); }
-__device__ __forceinline__ void fa_mb_expect(uint64_t* b, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fa_s32(b)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void fa_mb_arrive(uint64_t* b) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(fa_s32(b)) : "memory"); }
-__device__ __forceinline__ bool fa_mb_try(uint64_t* b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(ok) : "r"(fa_s32(b)), "r"(parity) : "memory");
-  return ok != 0u;
-}
-// Bounded wait: after the limit (seconds) every role of the CTA stops waiting, issues no further copies or MMAs and runs to its end.
-__device__ __forceinline__ bool fa_mb_wait(uint64_t* b, uint32_t parity, volatile int* stop) {
-  if (fa_mb_try(b, parity)) return true;
-  for (int n = 0; n < (1 << 20); ++n) {
-    if (fa_mb_try(b, parity)) return true;
-    if (*stop) return false;
-  }
-  *stop = 1;
-  atomicAdd(&fa_gave_up, 1u);
-  return false;
-}
 __device__ __forceinline__ void fa_tma_4d(void* dst, const CUtensorMap* tm, int c0, int c1, int c2, int c3, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(fa_s32(dst)),
-               "l"(tm), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(fa_s32(bar)) : "memory");
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(mbar_s32(dst)),
+               "l"(tm), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(mbar_s32(bar)) : "memory");
 }
 __device__ __forceinline__ void fa_tma_3d(void* dst, const CUtensorMap* tm, int c0, int c1, int c2, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(fa_s32(dst)),
-               "l"(tm), "r"(c0), "r"(c1), "r"(c2), "r"(fa_s32(bar)) : "memory");
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(mbar_s32(dst)),
+               "l"(tm), "r"(c0), "r"(c1), "r"(c2), "r"(mbar_s32(bar)) : "memory");
 }
 __device__ __forceinline__ void fa_tma_store_4d(const CUtensorMap* tm, const void* src, int c0, int c1, int c2, int c3) {
   asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(tm), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
-               "r"(fa_s32(src)) : "memory");
+               "r"(mbar_s32(src)) : "memory");
 }
 // K-major operand tile [rows][64 cols] of 128-byte rows, SWIZZLE_128B: 8-row groups 1024 B apart
 __device__ __forceinline__ uint64_t fa_desc_kmajor(const void* smem) {
   uint64_t d = 0;
-  d |= (uint64_t)((fa_s32(smem) & 0x3FFFF) >> 4);
+  d |= (uint64_t)((mbar_s32(smem) & 0x3FFFF) >> 4);
   d |= (uint64_t)1 << 16;
   d |= (uint64_t)(1024 >> 4) << 32;
   d |= (uint64_t)1 << 46;
@@ -105,7 +82,7 @@ __device__ __forceinline__ uint64_t fa_desc_kmajor(const void* smem) {
 // the second 64-column half of the tile sits LBO = 16 KB further.
 __device__ __forceinline__ uint64_t fa_desc_mnmajor(const void* smem) {
   uint64_t d = 0;
-  d |= (uint64_t)((fa_s32(smem) & 0x3FFFF) >> 4);
+  d |= (uint64_t)((mbar_s32(smem) & 0x3FFFF) >> 4);
   d |= (uint64_t)((FA_ROWS * 128) >> 4) << 16;       // leading byte offset: next 64-element block along MN
   d |= (uint64_t)(1024 >> 4) << 32;                  // stride byte offset: next 8-row (key) group
   d |= (uint64_t)1 << 46;
@@ -125,7 +102,7 @@ __device__ __forceinline__ void fa_umma_ts(uint32_t tmem_d, uint32_t tmem_a, uin
                "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc) : "memory");
 }
 __device__ __forceinline__ void fa_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(fa_s32(bar)) : "memory");
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar_s32(bar)) : "memory");
 }
 __device__ __forceinline__ void fa_tmem_ld32(uint32_t taddr, uint32_t* v) {
   asm volatile(
@@ -203,7 +180,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  uint8_t* smem = smem_raw + ((1024u - (fa_s32(smem_raw) & 1023u)) & 1023u);
+  uint8_t* smem = smem_raw + ((1024u - (mbar_s32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sQ = smem;                                    // [2 tiles]; the outputs are staged here at the end
   uint8_t* sKV = sQ + 2 * TILE;                          // [SLOTS]
   uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + SLOTS * TILE);
@@ -223,23 +200,23 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_k) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_v) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_o) : "memory");
-    fa_mb_init(q_full, 1);
+    mbar_init(q_full, 1);
     for (int s = 0; s < SLOTS; ++s) {
-      fa_mb_init(&kv_full[s], 1);
-      fa_mb_init(&kv_empty[s], 1);
+      mbar_init(&kv_full[s], 1);
+      mbar_init(&kv_empty[s], 1);
     }
     for (int x = 0; x < 2; ++x) {
-      fa_mb_init(&s_full[x], 1);
-      fa_mb_init(&p_full[x], 4);
-      fa_mb_init(&o_full[x], 1);
+      mbar_init(&s_full[x], 1);
+      mbar_init(&p_full[x], 4);
+      mbar_init(&o_full[x], 1);
     }
-    fa_mb_init(v_landed, 1);
-    fa_mb_init(v_clean, 1);
+    mbar_init(v_landed, 1);
+    mbar_init(v_clean, 1);
     *stop = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 8) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(fa_s32(tmem_slot)), "n"(512));
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(mbar_s32(tmem_slot)), "n"(512));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -293,7 +270,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
         return (table[pi] << p.page_shift) + (k & ((1 << p.page_shift) - 1));
       };
       if (lane == 0) {
-        fa_mb_expect(q_full, 2 * TILE);
+        mbar_expect(q_full, 2 * TILE);
         for (int x = 0; x < 2; ++x)
           for (int c = 0; c < D / 64; ++c)
             fa_tma_4d(sQ + x * TILE + c * HALF, &p.tm_q, c * 64, p.pair_heads ? h_first + x : h_first, p.pair_heads ? q0 : q0 + x * FA_ROWS, b, q_full);
@@ -306,12 +283,11 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
         const int live = PAGED ? min(pieces, (end - key0 + piece_rows - 1) / piece_rows) : 1;
         for (int v = 0; v < 2 && go; ++v) {
           const int it = 2 * i + v, s = it % SLOTS;
-          go = fa_mb_wait(&kv_empty[s], (uint32_t)((it / SLOTS) & 1) ^ 1u, stop);
-          go = __shfl_sync(0xffffffffu, (int)go, 0) != 0;
+          go = mbar_wait_warp(&kv_empty[s], (uint32_t)((it / SLOTS) & 1) ^ 1u, stop, p.wait_word);
           if (!go) break;
           uint8_t* dst = sKV + s * TILE;
           const CUtensorMap* tm = v ? &p.tm_v : &p.tm_k;
-          if (lane == 0) fa_mb_expect(&kv_full[s], (uint32_t)(live * piece_rows * D * 2));
+          if (lane == 0) mbar_expect(&kv_full[s], (uint32_t)(live * piece_rows * D * 2));
           if (PAGED) {
             for (int u = 0; u < live; ++u) {
               const int row = __shfl_sync(0xffffffffu, cur, u);
@@ -338,8 +314,8 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
           }
           fa_commit(&s_full[x]);
         };
-        auto full = [&](int it) { return fa_mb_wait(&kv_full[it % SLOTS], (uint32_t)((it / SLOTS) & 1), stop); };
-        bool go = fa_mb_wait(q_full, 0, stop) && full(0);
+        auto full = [&](int it) { return mbar_wait(&kv_full[it % SLOTS], (uint32_t)((it / SLOTS) & 1), stop, p.wait_word); };
+        bool go = mbar_wait(q_full, 0, stop, p.wait_word) && full(0);
         if (go) {
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           issue_s(0, 0);
@@ -350,11 +326,11 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
           const bool more = i + 1 < n_tiles;
           go = full(2 * i + 1);
           if (go && dirty_end && !more) {
-            fa_mb_arrive(v_landed);
-            go = fa_mb_wait(v_clean, 0, stop);
+            mbar_arrive(v_landed);
+            go = mbar_wait(v_clean, 0, stop, p.wait_word);
           }
           for (int x = 0; x < 2 && go; ++x) {
-            go = fa_mb_wait(&p_full[x], (uint32_t)(i & 1), stop);       // P_x in TMEM, O_x rescaled, S_x fully read
+            go = mbar_wait(&p_full[x], (uint32_t)(i & 1), stop, p.wait_word);       // P_x in TMEM, O_x rescaled, S_x fully read
             if (!go) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint8_t* v = sKV + ((2 * i + 1) % SLOTS) * TILE;
@@ -378,14 +354,14 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
     } else if (warp == 10 && dirty_end) {
       // ================= value rows past the last key of the last tile =================
       const int valid = end - key_at(n_tiles - 1);
-      if (fa_mb_wait(v_landed, 0, stop)) {
+      if (mbar_wait_warp(v_landed, 0, stop, p.wait_word)) {
         uint8_t* v = sKV + ((2 * n_tiles - 1) % SLOTS) * TILE;
         for (int c = lane; c < (FA_ROWS - valid) * 8; c += 32)
 #pragma unroll
           for (int hf = 0; hf < D / 64; ++hf) *reinterpret_cast<uint4*>(v + hf * HALF + valid * 128 + c * 16) = make_uint4(0u, 0u, 0u, 0u);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) fa_mb_arrive(v_clean);
+        if (lane == 0) mbar_arrive(v_clean);
       }
     }
   } else {
@@ -407,7 +383,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
     float m_run = -INFINITY, l_run = 0.f;
     for (int i = 0; i < n_tiles; ++i) {
       const int key0 = key_at(i);
-      if (!fa_mb_wait(&s_full[x], (uint32_t)(i & 1), stop)) break;
+      if (!mbar_wait_warp(&s_full[x], (uint32_t)(i & 1), stop, p.wait_word)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       uint32_t v[128];
 #pragma unroll
@@ -490,13 +466,13 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) fa_mb_arrive(&p_full[x]);
+      if (lane == 0) mbar_arrive(&p_full[x]);
       float s0, s1;
       fa_unpack2(fa_add2(ls[0], ls[1]), s0, s1);
       l_run += s0 + s1;
     }
     // ---- epilogue: O / l (times the gate) -> bf16 -> shared memory -> TMA store (rows past T are clipped, padding rows are zeros)
-    const bool done = fa_mb_wait(&o_full[x], 0, stop);
+    const bool done = mbar_wait_warp(&o_full[x], 0, stop, p.wait_word);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     float l = l_run;
     if (p.sinks != nullptr) l = (m_run == -INFINITY) ? 1.f : l + fa_ex2(p.sinks[h] * FA_LOG2E - m_run);
@@ -588,6 +564,8 @@ static void fa_go(FaParams& p, cudaStream_t stream) {
   auto kernel = attention_prefill_tc_kernel<D, PAGED, CAP>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     throw std::runtime_error("attention (tensor cores): shared memory size refused");
+  check_waits();
+  p.wait_word = wait_word(WAIT_ATTENTION);
   // grouped heads share their keys two by two; a head of its own takes 256 queries instead
   p.pair_heads = (p.Hq / p.Hkv) % 2 == 0 ? 1 : 0;
   const int span = p.pair_heads ? FA_ROWS : 2 * FA_ROWS;

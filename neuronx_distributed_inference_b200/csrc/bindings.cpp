@@ -862,6 +862,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         pybind11::arg("T"), pybind11::arg("K"), pybind11::arg("wt") = 0);
   m.def("moe_decode", &nxdi::moe_decode);
   m.def("moe_small", &nxdi::moe_small);
+  m.def("check_waits", &nxdi::check_waits);
+  m.def("wait_probe", [](int64_t clocks, at::Tensor out) {
+    TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kInt && out.numel() >= 1);
+    c10::cuda::CUDAGuard guard(out.device());
+    nxdi::wait_probe_launch(clocks, out.data_ptr<int>(), nxdi::cur_stream());
+  });
   m.def("moe_grouped", &nxdi::moe_grouped);
   m.def("dequant_bf16", &nxdi::dequant_bf16);
   m.def("gemm", &nxdi::gemm, pybind11::arg("x"), pybind11::arg("w"), pybind11::arg("bias"), pybind11::arg("act"), pybind11::arg("residual"),

@@ -22,6 +22,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "mbar_wait.cuh"
 
 namespace nxdi {
 
@@ -40,46 +41,23 @@ struct PairParams {
   float limit, alpha;
   int m_tiles, n_tiles, band;
   int w_fresh;                    // B was written by a kernel just before this one
+  unsigned* wait_word;            // mbar_wait.cuh
   const int* tile_expert;         // grouped: [m_tiles] expert | rows with tokens << 10 of a 256-row tile, < 0: not in use; null: one weight
 };
 
-__device__ unsigned gp_gave_up;    // waits that ran out (a protocol error; the results of that launch are not valid)
-
-__device__ __forceinline__ uint32_t gp_s32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void gp_init(uint64_t* b, uint32_t n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gp_s32(b)), "r"(n)); }
-__device__ __forceinline__ void gp_expect(uint64_t* b, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(gp_s32(b)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool gp_try(uint64_t* b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(ok) : "r"(gp_s32(b)), "r"(parity) : "memory");
-  return ok != 0u;
-}
-// bounded: after the limit (seconds) every role of this CTA stops waiting, issues nothing more and runs to its end
-__device__ __forceinline__ bool gp_wait(uint64_t* b, uint32_t parity, volatile int* stop) {
-  if (gp_try(b, parity)) return true;
-  for (int n = 0; n < (1 << 20); ++n) {
-    if (gp_try(b, parity)) return true;
-    if (*stop) return false;
-  }
-  *stop = 1;
-  atomicAdd(&gp_gave_up, 1u);
-  return false;
-}
 // shared::cluster address of a local shared-memory object in the pair's leader
 __device__ __forceinline__ uint32_t gp_leader(const void* p) {
   uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(gp_s32(p)));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(mbar_s32(p)));
   return r;
 }
 __device__ __forceinline__ void gp_tma(void* dst, const CUtensorMap* tm, int c0, int c1, uint32_t leader_bar) {
-  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(gp_s32(dst)),
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(mbar_s32(dst)),
                "l"(tm), "r"(c0), "r"(c1), "r"(leader_bar) : "memory");
 }
 __device__ __forceinline__ uint64_t gp_desc(const void* smem) {     // K-major, 128-byte rows, SWIZZLE_128B
   uint64_t d = 0;
-  d |= (uint64_t)((gp_s32(smem) & 0x3FFFF) >> 4);
+  d |= (uint64_t)((mbar_s32(smem) & 0x3FFFF) >> 4);
   d |= (uint64_t)1 << 16;
   d |= (uint64_t)(1024 >> 4) << 32;
   d |= (uint64_t)1 << 46;
@@ -91,7 +69,7 @@ __device__ __forceinline__ void gp_umma(uint32_t tmem_d, uint64_t da, uint64_t d
                "l"(db), "r"(idesc), "r"(acc) : "memory");
 }
 __device__ __forceinline__ void gp_commit_both(uint64_t* bar) {      // arrives on the barrier at this offset in both CTAs
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(gp_s32(bar)),
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(mbar_s32(bar)),
                "h"((unsigned short)3) : "memory");
 }
 __device__ __forceinline__ void gp_cluster_sync() {
@@ -118,7 +96,7 @@ __device__ __forceinline__ void gp_tile(const PairParams& p, int t, int& mt, int
 __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_constant__ PairParams p) {
   constexpr int BN = GP_BN, ST = GP_STAGES, STAGE = GP_STAGE;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = smem_raw + ((1024u - (gp_s32(smem_raw) & 1023u)) & 1023u);
+  uint8_t* smem = smem_raw + ((1024u - (mbar_s32(smem_raw) & 1023u)) & 1023u);
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + ST * STAGE);    // the leader's are used
   uint64_t* empty_bar = full_bar + ST;
   uint64_t* tmem_full = empty_bar + ST;     // [2]
@@ -138,18 +116,18 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tma_a) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tma_b) : "memory");
     for (int s = 0; s < ST; ++s) {
-      gp_init(&full_bar[s], 1);
-      gp_init(&empty_bar[s], 1);
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
-      gp_init(&tmem_full[b], 1);
-      gp_init(&tmem_empty[b], 2 * GP_EPI_WARPS);
+      mbar_init(&tmem_full[b], 1);
+      mbar_init(&tmem_empty[b], 2 * GP_EPI_WARPS);
     }
     *stop = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gp_s32(tmem_slot)), "n"(2 * BN));
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(mbar_s32(tmem_slot)), "n"(2 * BN));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -159,7 +137,8 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
   const uint32_t tmem = *tmem_slot;
   pdl_launch_dependents();
   // a weight that is a parameter does not depend on earlier kernels; everything else does
-  if (warp != 0 || p.tile_expert != nullptr || p.w_fresh) pdl_wait();
+  const bool early = warp == 0 && p.tile_expert == nullptr && !p.w_fresh;
+  if (!early) pdl_wait();
 
   if (warp == 0 || warp == 3) {
     // ================= TMA producers: B (warp 0), A (warp 3) of this CTA =================
@@ -181,14 +160,15 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
         const int row_b = e * p.N + (glu ? nt * (BN / 2) + (rank ? p.n_out : 0) : nt * BN + (int)rank * (BN / 2));
         for (int kb = 0; kb < nkb; ++kb, ++it) {
           const int s = (int)(it % ST);
-          go = gp_wait(&empty_bar[s], (uint32_t)((it / ST) & 1) ^ 1u, stop);
+          if (early && it == ST) pdl_wait();         // the ring is full: from here on a wait depends on the warps that wait for earlier kernels
+          go = mbar_wait<true>(&empty_bar[s], (uint32_t)((it / ST) & 1) ^ 1u, stop, p.wait_word);
           if (!go) break;
           uint8_t* st = smem + s * STAGE;
           const uint32_t bar = gp_leader(&full_bar[s]);
           if (warp == 0) {
             gp_tma(st + GP_A_BYTES, &p.tma_b, kb * GP_BK, row_b, bar);
           } else {
-            if (rank == 0) gp_expect(&full_bar[s], 2 * STAGE - (second ? 0 : GP_A_BYTES));       // everything that both CTAs copy for this stage
+            if (rank == 0) mbar_expect(&full_bar[s], 2 * STAGE - (second ? 0 : GP_A_BYTES));       // everything that both CTAs copy for this stage
             if (rank == 0 || second) gp_tma(st, &p.tma_a, kb * GP_BK, row_a, bar);
           }
         }
@@ -209,12 +189,12 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
           if (__ldg(p.tile_expert + mt) < 0) continue;
         }
         const int buf = tc & 1;
-        go = gp_wait(&tmem_empty[buf], (uint32_t)((tc >> 1) & 1) ^ 1u, stop);
+        go = mbar_wait<true>(&tmem_empty[buf], (uint32_t)((tc >> 1) & 1) ^ 1u, stop, p.wait_word);
         if (!go) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int kb = 0; kb < nkb; ++kb, ++it) {
           const int s = (int)(it % ST);
-          go = gp_wait(&full_bar[s], (uint32_t)((it / ST) & 1), stop);
+          go = mbar_wait<true>(&full_bar[s], (uint32_t)((it / ST) & 1), stop, p.wait_word);
           if (!go) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint64_t da = gp_desc(smem + s * STAGE), db = gp_desc(smem + s * STAGE + GP_A_BYTES);
@@ -257,7 +237,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
         row_end = mt * 256 + (e >> 10);
       }
       const int buf = tc & 1, row0 = mt * 256 + (int)rank * 128 + q * 32, col_t = nt * tile_out;
-      if (!gp_wait(&tmem_full[buf], (uint32_t)((tc >> 1) & 1), stop)) break;
+      if (!mbar_wait_warp<true>(&tmem_full[buf], (uint32_t)((tc >> 1) & 1), stop, p.wait_word)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN);
 #pragma unroll 1
@@ -366,6 +346,8 @@ void gemm_pair_launch(const void* a, long long lda, const void* b, const void* b
   p.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   p.c = reinterpret_cast<__nv_bfloat16*>(c);
   p.M = M; p.N = N; p.K = K; p.act = act; p.n_out = glu ? N / 2 : N; p.limit = limit; p.alpha = alpha;
+  check_waits();
+  p.wait_word = wait_word(WAIT_GEMM_PAIR);
   p.tile_expert = tile_expert; p.w_fresh = w_fresh ? 1 : 0;
   const int tile_out = glu ? GP_BN / 2 : GP_BN;
   p.m_tiles = (M + 255) / 256;

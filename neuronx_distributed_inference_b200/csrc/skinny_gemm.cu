@@ -19,6 +19,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "mbar_wait.cuh"
 
 namespace nxdi {
 
@@ -38,41 +39,17 @@ struct SkinnyKernelParams {
   unsigned* tickets;       // [G], zero at launch
   int T, n_out, rows, K, act, xb, xbox, stages, y_f32, tmem_cols, w_fresh;
   float limit, alpha;
+  unsigned* wait_word;     // mbar_wait.cuh
 };
 
-__device__ unsigned sk_gave_up;          // waits that ran out (a protocol error; the results of that launch are not valid)
-
-__device__ __forceinline__ uint32_t sk_s32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void sk_init(uint64_t* b, uint32_t n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sk_s32(b)), "r"(n)); }
-__device__ __forceinline__ void sk_expect(uint64_t* b, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sk_s32(b)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void sk_arrive(uint64_t* b) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sk_s32(b)) : "memory"); }
-__device__ __forceinline__ bool sk_try(uint64_t* b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(ok) : "r"(sk_s32(b)), "r"(parity) : "memory");
-  return ok != 0u;
-}
-// bounded: after the limit (seconds) every role stops waiting, issues nothing more and runs to its end
-__device__ __forceinline__ bool sk_wait(uint64_t* b, uint32_t parity, volatile int* stop) {
-  if (sk_try(b, parity)) return true;
-  for (int n = 0; n < (1 << 20); ++n) {
-    if (sk_try(b, parity)) return true;
-    if (*stop) return false;
-  }
-  *stop = 1;
-  atomicAdd(&sk_gave_up, 1u);
-  return false;
-}
 __device__ __forceinline__ void sk_tma(void* dst, const CUtensorMap* tm, int c0, int c1, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(sk_s32(dst)), "l"(tm),
-               "r"(c0), "r"(c1), "r"(sk_s32(bar)) : "memory");
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(mbar_s32(dst)), "l"(tm),
+               "r"(c0), "r"(c1), "r"(mbar_s32(bar)) : "memory");
 }
 // K-major operand tile of 128-byte rows, SWIZZLE_128B; 8-row groups are 1024 B apart
 __device__ __forceinline__ uint64_t sk_desc(const void* smem) {
   uint64_t d = 0;
-  d |= (uint64_t)((sk_s32(smem) & 0x3FFFF) >> 4);
+  d |= (uint64_t)((mbar_s32(smem) & 0x3FFFF) >> 4);
   d |= (uint64_t)1 << 16;
   d |= (uint64_t)(1024 >> 4) << 32;
   d |= (uint64_t)1 << 46;
@@ -84,7 +61,7 @@ __device__ __forceinline__ void sk_umma(uint32_t tmem_d, uint64_t da, uint64_t d
                "l"(db), "r"(idesc), "r"(acc) : "memory");
 }
 __device__ __forceinline__ void sk_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sk_s32(bar)) : "memory");
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar_s32(bar)) : "memory");
 }
 __device__ __forceinline__ void sk_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -96,7 +73,7 @@ template <bool GLU>
 __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid_constant__ SkinnyKernelParams p) {
   constexpr int NW = GLU ? 2 : 1;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = smem_raw + ((1024u - (sk_s32(smem_raw) & 1023u)) & 1023u);
+  uint8_t* smem = smem_raw + ((1024u - (mbar_s32(smem_raw) & 1023u)) & 1023u);
   __shared__ uint64_t full_bar[SK_MAX_STAGES], empty_bar[SK_MAX_STAGES], tmem_full[2], tmem_empty[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int s_stop, s_last;
@@ -108,18 +85,18 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_w) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_x) : "memory");
     for (int s = 0; s < ST; ++s) {
-      sk_init(&full_bar[s], 2);         // the two producers
-      sk_init(&empty_bar[s], 1);
+      mbar_init(&full_bar[s], 2);         // the two producers
+      mbar_init(&empty_bar[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
-      sk_init(&tmem_full[b], 1);
-      sk_init(&tmem_empty[b], 8);
+      mbar_init(&tmem_full[b], 1);
+      mbar_init(&tmem_empty[b], 8);
     }
     s_stop = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sk_s32(&tmem_slot)), "r"(p.tmem_cols));
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(mbar_s32(&tmem_slot)), "r"(p.tmem_cols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -128,8 +105,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
   const uint32_t tmem = tmem_slot;
   pdl_launch_dependents();
   // a dense weight that is a parameter does not depend on earlier kernels; everything else does
-  const bool grouped = p.n_active != nullptr;
-  if (warp != 0 || grouped || p.w_fresh) pdl_wait();
+  const bool grouped = p.n_active != nullptr, early = warp == 0 && !grouped && !p.w_fresh;
+  if (!early) pdl_wait();
 
   const int n_tiles = (p.n_out + SK_BM - 1) / SK_BM, nkb = p.K / SK_BK;
   const long long total = (long long)(grouped ? *p.n_active : 1) * n_tiles * nkb;
@@ -149,15 +126,16 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
         const int boxes = grouped ? (p.seg_count[ei] + p.xbox - 1) / p.xbox : 1, box_bytes = p.xbox * SK_BK * 2;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = (int)(it % ST);
-          go = sk_wait(&empty_bar[s], (uint32_t)((it / ST) & 1) ^ 1u, stop);
+          if (early && it == ST) pdl_wait();         // the ring is full: from here on a wait depends on the warps that wait for earlier kernels
+          go = mbar_wait(&empty_bar[s], (uint32_t)((it / ST) & 1) ^ 1u, stop, p.wait_word);
           if (!go) break;
           uint8_t* st = smem + (size_t)s * stage_bytes;
           if (warp == 0) {
-            sk_expect(&full_bar[s], NW * SK_W_BYTES);
+            mbar_expect(&full_bar[s], NW * SK_W_BYTES);
             sk_tma(st, &p.tm_w, kb * SK_BK, row_w, &full_bar[s]);
             if (GLU) sk_tma(st + SK_W_BYTES, &p.tm_w, kb * SK_BK, row_w + p.n_out, &full_bar[s]);
           } else {
-            sk_expect(&full_bar[s], boxes * box_bytes);
+            mbar_expect(&full_bar[s], boxes * box_bytes);
             for (int q = 0; q < boxes; ++q) sk_tma(st + NW * SK_W_BYTES + q * box_bytes, &p.tm_x, kb * SK_BK, row_x + q * p.xbox, &full_bar[s]);
           }
         }
@@ -175,12 +153,12 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
         // D = f32, A = B = bf16, both K-major, M = 128, N = the tokens in whole boxes (a multiple of 16)
         const int nx = grouped ? (p.seg_count[(int)(u / nkb) / n_tiles] + 15) / 16 * 16 : p.xb;
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nx >> 3) << 17) | ((uint32_t)(SK_BM >> 4) << 24);
-        go = sk_wait(&tmem_empty[buf], (uint32_t)((seg >> 1) & 1) ^ 1u, stop);
+        go = mbar_wait(&tmem_empty[buf], (uint32_t)((seg >> 1) & 1) ^ 1u, stop, p.wait_word);
         if (!go) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = (int)(it % ST);
-          go = sk_wait(&full_bar[s], (uint32_t)((it / ST) & 1), stop);
+          go = mbar_wait(&full_bar[s], (uint32_t)((it / ST) & 1), stop, p.wait_word);
           if (!go) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint8_t* st = smem + (size_t)s * stage_bytes;
@@ -203,12 +181,13 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
     const int n_in = (warp & 3) * 32 + lane, c0 = warp >= 8 ? 16 : 0;      // two warps per 32 features: even and odd groups of 16 tokens
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     int seg = 0;
+    bool live = true;          // false once a wait ran out: the warp still takes part in the barriers of the eight
     for (long long u = u0; u < u1; ++seg) {
       const int tile = (int)(u / nkb), kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u)), buf = seg & 1;
       u += kb1 - kb0;
       const int ei = tile / n_tiles, n = (tile % n_tiles) * SK_BM + n_in, e = grouped ? p.active[ei] : 0;
       const int row0 = grouped ? p.seg_start[ei] : 0, cnt = grouped ? p.seg_count[ei] : p.T;
-      if (!sk_wait(&tmem_full[buf], (uint32_t)((seg >> 1) & 1), stop)) break;
+      if (live) live = mbar_wait_warp(&tmem_full[buf], (uint32_t)((seg >> 1) & 1), stop, p.wait_word);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem + lanes + (uint32_t)(buf * acc_cols);
       const bool whole = kb0 == 0 && kb1 == nkb;
@@ -233,7 +212,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
       };
       if (whole) {
 #pragma unroll 1
-        for (int c = c0; c < cnt; c += 32) {
+        for (int c = c0; c < cnt && live; c += 32) {
           uint32_t g[16], up[16];
           sk_ld16(acc + c, g);
           if (GLU) sk_ld16(acc + p.xb + c, up);
@@ -243,7 +222,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) sk_arrive(&tmem_empty[buf]);
+        if (lane == 0) mbar_arrive(&tmem_empty[buf]);
         continue;
       }
       // a part of the tile's k range.  CTAs that share the tile: those of its first and last k-block and all between
@@ -281,7 +260,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
         if (direct) {
           __threadfence();
 #pragma unroll 1
-          for (int c = c0; c < cnt; c += 32) {
+          for (int c = c0; c < cnt && live; c += 32) {
             uint32_t vg[16], vu[16];
             sk_ld16(acc + c, vg);
             if (GLU) sk_ld16(acc + p.xb + c, vu);
@@ -298,7 +277,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
           }
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
-          if (lane == 0) sk_arrive(&tmem_empty[buf]);
+          if (lane == 0) mbar_arrive(&tmem_empty[buf]);
           continue;
         }
       }
@@ -308,7 +287,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
 #pragma unroll 1
       for (int w = 0; w < NW; ++w)
 #pragma unroll 1
-        for (int c = c0; c < wcols; c += 32) {
+        for (int c = c0; c < wcols && live; c += 32) {
           uint32_t v[16];
           sk_ld16(acc + w * p.xb + c, v);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -318,7 +297,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
         }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) sk_arrive(&tmem_empty[buf]);
+      if (lane == 0) mbar_arrive(&tmem_empty[buf]);
       __threadfence();
       asm volatile("bar.sync 1, 256;" ::: "memory");
       if (threadIdx.x == 128) s_last = atomicAdd(&p.tickets[c_first], 1u) == (unsigned)(c_last - c_first);
@@ -326,7 +305,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
       if (s_last) {
         __threadfence();
 #pragma unroll 1
-        for (int c = c0; c < cnt; c += 32) {
+        for (int c = c0; c < cnt && live; c += 32) {
           float g[16], up[16];
 #pragma unroll
           for (int k = 0; k < 16; ++k) g[k] = up[k] = 0.f;
@@ -401,6 +380,8 @@ void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream) {
   p.residual = reinterpret_cast<const __nv_bfloat16*>(a.residual);
   p.y = a.y; p.y_f32 = a.y_f32; p.ws = a.ws; p.tickets = a.tickets;
   p.T = a.tokens; p.n_out = a.n_out; p.K = a.K; p.act = a.act; p.limit = a.limit; p.alpha = a.alpha; p.w_fresh = a.w_fresh;
+  check_waits();
+  p.wait_word = wait_word(WAIT_SKINNY);
   const int stage = (glu ? 2 : 1) * SK_W_BYTES + p.xb * SK_BK * 2;
   p.stages = std::min(SK_MAX_STAGES, (SK_SMEM - 1024) / stage);
   int cols = 32;

@@ -14,6 +14,8 @@ from typing import List
 import torch
 import torch.nn as nn
 
+from .. import ops
+
 from ..modules.eagle.token_tree import TokenTree
 
 DEFAULT_MEDUSA_TREE = [[0], [0, 0], [1], [0, 1], [2], [0, 0, 0], [1, 0], [0, 2], [3], [0, 3], [4], [0, 4], [2, 0], [0, 5],
@@ -119,6 +121,7 @@ def medusa_generate(adapter, input_ids, attention_mask, max_length, eos: List[in
         acc, n_acc, root, heads, position = step(root, heads, seq_ids, position)
         stats["steps"] += 1
         stats["accepted"] += int(n_acc.sum())
+        ops.check_waits()
         for b, toks in enumerate(acc.cpu().tolist()):
             for t in toks:
                 if done[b] or t < 0:

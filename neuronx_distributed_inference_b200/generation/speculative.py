@@ -19,6 +19,8 @@ from typing import List, Optional, Tuple
 import torch
 import torch.nn as nn
 
+from .. import ops
+
 
 @torch.no_grad()
 def greedy_accept(draft_tokens: torch.Tensor, target_tokens: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -291,6 +293,7 @@ def assisted_generate(adapter, input_ids, attention_mask, max_length, eos: List[
         else:
             accepted, n_acc, tok, position, prev = step(tok, position, seq_ids, prev)[:5]
         acc = accepted.cpu()
+        ops.check_waits()
         stats["steps"] += 1
         stats["accepted"] += int(n_acc.sum())
         for b in range(B):

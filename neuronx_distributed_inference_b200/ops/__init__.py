@@ -14,7 +14,7 @@ from typing import Optional
 import torch
 
 from . import reference as ref
-from ._ext import load_extension, extension_available
+from ._ext import load_extension, loaded_extension, extension_available
 
 stats = Counter()
 _ALLOW_FALLBACK = os.environ.get("NXDI_B200_ALLOW_TORCH_FALLBACK", "0") == "1"
@@ -43,6 +43,14 @@ def _use_cuda(x: torch.Tensor) -> bool:
     raise RuntimeError("CUDA tensor but the sm_100a extension is not built: run "
                        "`python -c 'import __graft_entry__ as g; g.build()'` "
                        "(or set NXDI_B200_ALLOW_TORCH_FALLBACK=1)")
+
+
+def check_waits():
+    """Raise if a wait inside a tensor-core kernel ran out (csrc/mbar_wait.cuh): its results are invalid.  A read of a few words of host memory, no
+    synchronisation: call it where results have reached the host.  The launches of these kernels and every step of the engine do."""
+    mod = loaded_extension()
+    if mod is not None:
+        mod.check_waits()
 
 
 _FAST_DTYPES = (torch.bfloat16,)

@@ -107,6 +107,11 @@ def extension_available() -> bool:
     return load_extension(required=False) is not None
 
 
+def loaded_extension():
+    """The extension if something has loaded it already."""
+    return _mod
+
+
 def load_extension(required: bool = True):
     global _mod, _tried
     if _mod is not None:

@@ -22,6 +22,7 @@ from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
 
+from .. import ops
 from ..modules import autobucketing
 from ..models.model_base import ModelOutput
 
@@ -208,6 +209,7 @@ class SubModelRunner:
         return out
 
     def _call(self, input_ids, attention_mask, position_ids, seq_ids, sampling_params, _warmup=False, **kw):
+        ops.check_waits()                    # of the steps before: graph replays launch their kernels without the host
         B = input_ids.shape[0]
         if self.snapshot_hook is not None and not _warmup:
             if self.is_prefill and self.on_new_request is not None:

@@ -22,6 +22,8 @@ from typing import Sequence as Seq
 import numpy as np
 import torch
 
+from .. import ops
+
 
 class PagePool:
     def __init__(self, num_pages: int):
@@ -171,8 +173,11 @@ class PagedBatchEngine:
         for seq, (_, toks, _) in zip(seqs, entries):
             seq.length += len(toks)
         if sample:
-            return [int(t) for t in out.tokens.reshape(B, -1)[:, 0].tolist()]
+            toks = [int(t) for t in out.tokens.reshape(B, -1)[:, 0].tolist()]
+            ops.check_waits()
+            return toks
         logits = out.logits.float().cpu()
+        ops.check_waits()
         return [logits[b, :len(want)] for b, (_, _, want) in enumerate(entries)]
 
     # ---- scheduler ---------------------------------------------------------------------------------------------------

@@ -21,6 +21,7 @@ from typing import List, Optional, Union
 
 import torch
 
+from .. import ops
 from ..config import load_pretrained_config  # noqa: F401  (re-export, reference keeps it here)
 from ..modules.sampling import prepare_sampling_params
 
@@ -228,6 +229,7 @@ class HuggingFaceGenerationAdapter(_PreTrainedModel, _GenerationMixin):
                 nxt = self._host_sample(lg, gc, sequences)
             if want_logits and out.logits is not None:
                 all_logits.append(out.logits[:, -1].float().cpu())
+            ops.check_waits()
             nxt = torch.where(unfinished, nxt, torch.full_like(nxt, pad_id))
             # right padding: the new token goes right after each row's last valid token
             sequences, mask = _append_tokens(sequences, mask, nxt, pad_id, self.padding_side)
@@ -325,6 +327,7 @@ class HuggingFaceGenerationAdapter(_PreTrainedModel, _GenerationMixin):
                 nxt = torch.multinomial(torch.softmax(proc, -1), 1).squeeze(1) if generation_config.do_sample else proc.argmax(-1)
             else:
                 nxt = out.tokens.reshape(B, -1)[:, -1].to("cpu", torch.long)
+            ops.check_waits()
             nxt = torch.where(unfinished, nxt, torch.full_like(nxt, pad))
             sequences, mask = _append_tokens(sequences, mask, nxt, pad, self.padding_side)
             if streamer is not None:
