@@ -100,9 +100,10 @@ unsigned* wait_word(WaitKernel which);
 void check_waits();
 void wait_probe_launch(long long clocks, int* out, cudaStream_t stream);
 
-// prompt-sized GEMM on CTA pairs (gemm_pair.cu); tile_expert: grouped, segments of whole 256-row tiles (moe_plan256)
+// prompt-sized GEMM on CTA pairs (gemm_pair.cu); tile_expert / tile_row: grouped, m_tiles tiles of up to 256 rows of the M permuted ones (moe_plan256)
 void gemm_pair_launch(const void* a, long long lda, const void* b, const void* bias, const void* residual, void* c, int M, int N, int K, int act,
-                      cudaStream_t stream, const int* tile_expert = nullptr, int experts = 1, float limit = 7.f, float alpha = 1.702f, bool w_fresh = false);
+                      cudaStream_t stream, bool w_fresh = false, const int* tile_expert = nullptr, const int* tile_row = nullptr, int m_tiles = 0, int experts = 1,
+                      float limit = 7.f, float alpha = 1.702f);
 
 // few tokens x large weights with the weights streamed evenly over the SMs (skinny_gemm.cu): one weight [rows, K], or the experts that have tokens
 constexpr int SKINNY_MAX_T = 128;
@@ -185,7 +186,8 @@ void gemm_fp8_launch(const void* a, int lda, const void* b, const float* a_scale
                      const void* residual, void* c, int ldc, int M, int N, int K, int act, cudaStream_t stream);
 
 // mixture-of-experts prefill: device-side permutation (moe_grouped.cu) around the grouped tcgen05 GEMM (gemm_tcgen05.cu)
-void moe_plan256_launch(const int* topk_i, int entries, int expert_offset, int e_local, int tiles, int* pos, int* tile_expert, cudaStream_t stream);
+void moe_plan256_launch(const int* topk_i, int entries, int expert_offset, int e_local, int tiles, int* pos, int* tile_expert, int* tile_row,
+                        cudaStream_t stream);
 void moe_scatter_launch(const void* x, const float* topk_w, const int* pos, void* xp, int N, int H, int k, int scale_input, cudaStream_t stream);
 void moe_plan_launch(const int* topk_i, int entries, int expert_offset, int e_local, int R, int* pos, int* row_entry, int* tile_expert,
                      cudaStream_t stream);

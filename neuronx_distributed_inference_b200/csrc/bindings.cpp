@@ -209,7 +209,7 @@ at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
   }
   if (pair_pays(M, n_out, glu)) {
     gemm_pair_launch(x.data_ptr(), x.stride(0), w.data_ptr(), optr(bias), optr(residual), y.data_ptr(), M, N, K, (int)act, cur_stream(),
-                     nullptr, 1, 7.f, 1.702f, fresh_weight);
+                     fresh_weight);
     return y;
   }
   gemm_tcgen05_launch(x.data_ptr(), (int)x.stride(0), w.data_ptr(), optr(bias), optr(residual), y.data_ptr(), n_out, M, N, K,
@@ -367,18 +367,21 @@ at::Tensor moe_grouped(const at::Tensor& x, const at::Tensor& w_gate_up, const a
   c10::cuda::CUDAGuard guard(x.device());
   auto iopt = x.options().dtype(at::kInt);
   if (!fp8) {
-    // static bound of 256-row tiles: graph-stable shapes
-    const int64_t entries = (int64_t)N * k, R = (entries + std::min<int64_t>(E, entries) * 255) / 256 * 256;
+    // the permuted rows lie one after the other (an expert's last tile runs on into the next one's rows and stores its own only), so the three
+    // buffers hold one row per entry; the number of tiles is a static bound: graph-stable shapes
+    const int64_t R = (int64_t)N * k, tiles = (R + std::min<int64_t>(E, R) * 255) / 256;
     auto out = at::empty({N, H}, x.options());
-    if (entries == 0 || R == 0) return out.zero_();
+    if (R == 0) return out.zero_();
     auto st = cur_stream();
-    auto pos = at::empty({entries}, iopt), tile_expert = at::empty({R / 256}, iopt);
+    auto pos = at::empty({R}, iopt), tile_expert = at::empty({tiles}, iopt), tile_row = at::empty({tiles}, iopt);
     auto xp = at::empty({R, H}, x.options()), h = at::empty({R, I}, x.options()), y = at::empty({R, H}, x.options());
-    moe_plan256_launch(topk_i.data_ptr<int>(), (int)entries, (int)expert_offset, E, (int)(R / 256), pos.data_ptr<int>(), tile_expert.data_ptr<int>(), st);
+    moe_plan256_launch(topk_i.data_ptr<int>(), (int)R, (int)expert_offset, E, (int)tiles, pos.data_ptr<int>(), tile_expert.data_ptr<int>(),
+                       tile_row.data_ptr<int>(), st);
     moe_scatter_launch(x.data_ptr(), topk_w.data_ptr<float>(), pos.data_ptr<int>(), xp.data_ptr(), N, H, k, scale_input ? 1 : 0, st);
     gemm_pair_launch(xp.data_ptr(), H, w_gate_up.data_ptr(), optr(gate_up_bias), nullptr, h.data_ptr(), (int)R, 2 * I, H, (int)act, st,
-                     tile_expert.data_ptr<int>(), E, (float)limit, (float)alpha);
-    gemm_pair_launch(h.data_ptr(), I, w_down.data_ptr(), optr(down_bias), nullptr, y.data_ptr(), (int)R, H, I, 0, st, tile_expert.data_ptr<int>(), E);
+                     false, tile_expert.data_ptr<int>(), tile_row.data_ptr<int>(), (int)tiles, E, (float)limit, (float)alpha);
+    gemm_pair_launch(h.data_ptr(), I, w_down.data_ptr(), optr(down_bias), nullptr, y.data_ptr(), (int)R, H, I, 0, st, false,
+                     tile_expert.data_ptr<int>(), tile_row.data_ptr<int>(), (int)tiles, E);
     moe_combine_launch(y.data_ptr(), topk_w.data_ptr<float>(), pos.data_ptr<int>(), out.data_ptr(), N, H, k, scale_input ? 1 : 0, st);
     return out;
   }

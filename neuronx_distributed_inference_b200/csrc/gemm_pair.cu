@@ -9,8 +9,8 @@
 //   * warps 4..11: epilogue of the CTA's own 128 rows (two warps per 32 rows take turns at 64-column pieces: with four warps the gate products of
 //     2048-deep tiles took longer than their MMAs); bias / residual / gate products; rows leave (and residual rows come) through shared memory as
 //     whole 128-byte pieces
-//   * grouped (mixture of experts): A holds tokens permuted by expert in segments of whole 256-row tiles; tile_expert gives a row tile's expert and how
-//     many of its rows hold tokens (a half without any is neither loaded nor stored).  Tiles are walked in bands of four row tiles, n-tile by n-tile
+//   * grouped (mixture of experts): A holds tokens permuted by expert, one row per token and slot; tile_expert / tile_row give a row tile's expert, how many
+//     rows it stores (a half without any is neither loaded nor stored) and its first row; an expert's last tile reads on into the rows behind its own.  Tiles are walked in bands of four row tiles, n-tile by n-tile
 //     inside a band: the permuted rows and an expert's weights are read from HBM once (128 experts of 2048 x 768, 4096 tokens, 8 each, both GEMMs with
 //     permutation: 456 us; bands of 32 row tiles 480, no bands 589; 8 experts of 4096 x 14336, 1024 tokens: 858, 951, 944).
 // Measured (isolated, us, here / 128 x 256 tiles of one CTA): 4096 tokens 28672 x 4096 gate|up 624 / 725 (1.54 PFLOP/s, 94 % of the measured cuBLAS burst),
@@ -42,7 +42,8 @@ struct PairParams {
   int m_tiles, n_tiles, band;
   int w_fresh;                    // B was written by a kernel just before this one
   unsigned* wait_word;            // mbar_wait.cuh
-  const int* tile_expert;         // grouped: [m_tiles] expert | rows with tokens << 10 of a 256-row tile, < 0: not in use; null: one weight
+  const int* tile_expert;         // grouped: [m_tiles] expert | rows << 10 of a row tile, < 0: not in use; null: one weight
+  const int* tile_row;            // grouped: [m_tiles] first row of a row tile
 };
 
 // shared::cluster address of a local shared-memory object in the pair's leader
@@ -148,15 +149,16 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
       for (int t = pair; t < total && go; t += pairs) {
         int mt, nt;
         gp_tile(p, t, mt, nt);
-        int e = 0;
+        int e = 0, m0 = mt * 256;
         bool second = true;              // the odd CTA's half has rows
         if (p.tile_expert != nullptr) {
           e = __ldg(p.tile_expert + mt);
           if (e < 0) continue;
           second = (e >> 10) > 128;
           e &= 1023;
+          m0 = __ldg(p.tile_row + mt);
         }
-        const int row_a = mt * 256 + (int)rank * 128;
+        const int row_a = m0 + (int)rank * 128;
         const int row_b = e * p.N + (glu ? nt * (BN / 2) + (rank ? p.n_out : 0) : nt * BN + (int)rank * (BN / 2));
         for (int kb = 0; kb < nkb; ++kb, ++it) {
           const int s = (int)(it % ST);
@@ -229,14 +231,15 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
     for (int t = pair; t < total; t += pairs) {
       int mt, nt;
       gp_tile(p, t, mt, nt);
-      int eo = 0, row_end = p.M;
+      int eo = 0, m0 = mt * 256, row_end = p.M;
       if (p.tile_expert != nullptr) {
         const int e = __ldg(p.tile_expert + mt);
         if (e < 0) continue;
         eo = (e & 1023) * p.N;
-        row_end = mt * 256 + (e >> 10);
+        m0 = __ldg(p.tile_row + mt);
+        row_end = m0 + (e >> 10);
       }
-      const int buf = tc & 1, row0 = mt * 256 + (int)rank * 128 + q * 32, col_t = nt * tile_out;
+      const int buf = tc & 1, row0 = m0 + (int)rank * 128 + q * 32, col_t = nt * tile_out;
       if (!mbar_wait_warp<true>(&tmem_full[buf], (uint32_t)((tc >> 1) & 1), stop, p.wait_word)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN);
@@ -335,11 +338,10 @@ static int gp_sms() {
   return n;
 }
 
-// a [M, K] (row stride lda), b [experts * N, K], c [M, n_out]; tile_expert (device, [M / 256]) for the grouped flavour
+// a [M, K] (row stride lda), b [experts * N, K], c [M, n_out]; tile_expert / tile_row (device, [m_tiles]) for the grouped flavour
 void gemm_pair_launch(const void* a, long long lda, const void* b, const void* bias, const void* residual, void* c, int M, int N, int K, int act,
-                      cudaStream_t stream, const int* tile_expert, int experts, float limit, float alpha, bool w_fresh) {
+                      cudaStream_t stream, bool w_fresh, const int* tile_expert, const int* tile_row, int m_tiles, int experts, float limit, float alpha) {
   if (K % GP_BK != 0 || M < 1) throw std::runtime_error("gemm pair: K must be a multiple of 64");
-  if (tile_expert != nullptr && M % 256 != 0) throw std::runtime_error("gemm pair: the permuted row bound must be a multiple of 256");
   PairParams p{};
   const bool glu = act != 0;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
@@ -348,9 +350,9 @@ void gemm_pair_launch(const void* a, long long lda, const void* b, const void* b
   p.M = M; p.N = N; p.K = K; p.act = act; p.n_out = glu ? N / 2 : N; p.limit = limit; p.alpha = alpha;
   check_waits();
   p.wait_word = wait_word(WAIT_GEMM_PAIR);
-  p.tile_expert = tile_expert; p.w_fresh = w_fresh ? 1 : 0;
+  p.tile_expert = tile_expert; p.tile_row = tile_row; p.w_fresh = w_fresh ? 1 : 0;
   const int tile_out = glu ? GP_BN / 2 : GP_BN;
-  p.m_tiles = (M + 255) / 256;
+  p.m_tiles = tile_expert != nullptr ? m_tiles : (M + 255) / 256;
   p.n_tiles = (p.n_out + tile_out - 1) / tile_out;
   p.band = tile_expert == nullptr ? p.m_tiles : std::min(4, p.m_tiles);
   gp_map(&p.tma_a, a, M, K, lda, 128);

@@ -123,12 +123,12 @@ __global__ void __launch_bounds__(128) moe_combine_kernel(const __nv_bfloat16* _
   }
 }
 
-// ---- bf16 experts on CTA-pair tiles (gemm_pair.cu): segments of whole 256-row tiles ------------------------------------------------------
+// ---- bf16 experts on CTA-pair tiles (gemm_pair.cu): rows one after the other, up to 256 of an expert per tile ------------------------------------------------------
 // One CTA: the atomic that counts an expert's entries also ranks them, so one pass decides the rows and the second only adds the segment starts
 // (32768 entries, 128 experts: 11 us; with a second atomic pass, a serial scan and the inverse table 31 us).
 __global__ void __launch_bounds__(MOE_PLAN_THREADS) moe_plan256_kernel(const int* __restrict__ topk_i, int entries, int expert_offset, int e_local, int tiles,
-                                                                       int* __restrict__ pos, int* __restrict__ tile_expert) {
-  __shared__ int count[MOE_MAX_E], start[MOE_MAX_E + 1];
+                                                                       int* __restrict__ pos, int* __restrict__ tile_expert, int* __restrict__ tile_row) {
+  __shared__ int count[MOE_MAX_E], start[MOE_MAX_E], tile0[MOE_MAX_E + 1];
   pdl_launch_dependents();
   const int tid = threadIdx.x;
   for (int e = tid; e < e_local; e += MOE_PLAN_THREADS) count[e] = 0;
@@ -145,24 +145,34 @@ __global__ void __launch_bounds__(MOE_PLAN_THREADS) moe_plan256_kernel(const int
   }
   __syncthreads();
   if (tid < 32) {
-    int at = 0;
+    int at = 0, tile = 0;
     for (int c0 = 0; c0 < e_local; c0 += 32) {
-      const int c = c0 + tid, n = c < e_local ? (count[c] + 255) & ~255 : 0;
-      int incl = n;
+      const int c = c0 + tid, n = c < e_local ? count[c] : 0, nt = (n + 255) >> 8;
+      int incl = n, tincl = nt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (tid >= o) incl += t;
+        const int t = __shfl_up_sync(0xffffffffu, incl, o), tt = __shfl_up_sync(0xffffffffu, tincl, o);
+        if (tid >= o) {
+          incl += t;
+          tincl += tt;
+        }
       }
-      if (c < e_local) start[c] = at + incl - n;
+      if (c < e_local) {
+        start[c] = at + incl - n;
+        tile0[c] = tile + tincl - nt;
+      }
       at += __shfl_sync(0xffffffffu, incl, 31);
+      tile += __shfl_sync(0xffffffffu, tincl, 31);
     }
-    if (tid == 0) start[e_local] = at;
+    if (tid == 0) tile0[e_local] = tile;
   }
   __syncthreads();
   for (int e = tid; e < e_local; e += MOE_PLAN_THREADS)
-    for (int t = start[e] >> 8; t < start[e + 1] >> 8; ++t) tile_expert[t] = e | min(256, start[e] + count[e] - t * 256) << 10;
-  for (int t = (start[e_local] >> 8) + tid; t < tiles; t += MOE_PLAN_THREADS) tile_expert[t] = -1;
+    for (int t = tile0[e], r = 0; t < tile0[e + 1]; ++t, r += 256) {
+      tile_expert[t] = e | min(256, count[e] - r) << 10;
+      tile_row[t] = start[e] + r;
+    }
+  for (int t = tile0[e_local] + tid; t < tiles; t += MOE_PLAN_THREADS) tile_expert[t] = -1;
   for (int i0 = tid; i0 < entries; i0 += U * MOE_PLAN_THREADS) {      // own entries again: written by this thread above
     int e[U], r[U];
 #pragma unroll
@@ -177,8 +187,7 @@ __global__ void __launch_bounds__(MOE_PLAN_THREADS) moe_plan256_kernel(const int
   }
 }
 
-// one CTA per token: its row is read once and written to the k places of its experts (padding rows are left as they are: a row of the products
-// depends on its own row only, and no padding row is combined)
+// one CTA per token: its row is read once and written to the k places of its experts
 __global__ void __launch_bounds__(256) moe_scatter_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ topk_w,
                                                           const int* __restrict__ pos, __nv_bfloat16* __restrict__ xp, int H, int k, int scale_input) {
   pdl_launch_dependents();
@@ -201,9 +210,11 @@ __global__ void __launch_bounds__(256) moe_scatter_kernel(const __nv_bfloat16* _
   }
 }
 
-void moe_plan256_launch(const int* topk_i, int entries, int expert_offset, int e_local, int tiles, int* pos, int* tile_expert, cudaStream_t stream) {
+void moe_plan256_launch(const int* topk_i, int entries, int expert_offset, int e_local, int tiles, int* pos, int* tile_expert, int* tile_row,
+                        cudaStream_t stream) {
   if (e_local > MOE_MAX_E) throw std::runtime_error("moe_plan: more than 512 local experts");
-  launch_pdl(moe_plan256_kernel, dim3(1), dim3(MOE_PLAN_THREADS), 0, stream, topk_i, entries, expert_offset, e_local, tiles, pos, tile_expert);
+  launch_pdl(moe_plan256_kernel, dim3(1), dim3(MOE_PLAN_THREADS), 0, stream, topk_i, entries, expert_offset, e_local, tiles, pos, tile_expert,
+             tile_row);
 }
 void moe_scatter_launch(const void* x, const float* topk_w, const int* pos, void* xp, int N, int H, int k, int scale_input, cudaStream_t stream) {
   launch_pdl(moe_scatter_kernel, dim3(N), dim3(256), 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), topk_w, pos,
