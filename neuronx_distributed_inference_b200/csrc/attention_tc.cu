@@ -157,8 +157,7 @@ __device__ __forceinline__ uint64_t fa_add2(uint64_t a, uint64_t b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
-// tanh on |x| <= 1: x times a polynomial in x^2 (weighted least squares on Chebyshev nodes, relative error 1.7e-7 with fp32 arithmetic);
-// beyond: 1 - 2 / (e^2x + 1)
+// tanh on |x| <= 1: x times a polynomial in x^2 (weighted least squares on Chebyshev nodes, relative error 1.7e-7 with fp32 arithmetic)
 __device__ __forceinline__ uint64_t fa_tanh2_small(uint64_t x) {
   const uint64_t u = fa_mul2(x, x);
   uint64_t r = fa_pack2(0.00104102155f, 0.00104102155f);
@@ -170,7 +169,6 @@ __device__ __forceinline__ uint64_t fa_tanh2_small(uint64_t x) {
   r = fa_fma2(r, u, fa_pack2(0.99999994f, 0.99999994f));
   return fa_mul2(x, r);
 }
-__device__ __forceinline__ float fa_tanh_any(float x) { return 1.f - __fdividef(2.f, __expf(2.f * x) + 1.f); }
 
 template <int D, bool PAGED, bool CAP>
 __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(const __grid_constant__ FaParams p) {
@@ -390,11 +388,22 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
       for (int c = 0; c < 4; ++c) fa_tmem_ld32(tS + 32 * c, v + 32 * c);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       float scl = hs * FA_LOG2E;                         // scores -> log2 domain
+      // masks only where a tile can contain invisible keys: uniform test
+      const bool edge = key0 + FA_ROWS - 1 > up_min || (key0 < lb_max && key0 + FA_ROWS > keep);
+      const int e_hi = up - key0, e_lo = lb - key0, e_keep = keep - key0;
       if (CAP) {
+        // which form of tanh the warp takes must not depend on what a query does not see: later keys, rows of pages that were not fetched (whatever
+        // shared memory held), queries past the end
+        if (edge) {
+#pragma unroll
+          for (int e = 0; e < 128; ++e)
+            if (!(e <= e_hi && (e >= e_lo || e < e_keep))) v[e] = 0u;
+        }
         const float to_cap = hs / p.softcap;
         float big = 0.f;
 #pragma unroll
         for (int e = 0; e < 128; ++e) big = fmaxf(big, fabsf(__uint_as_float(v[e])));
+        if (t >= qn) big = 0.f;
         if (!__any_sync(0xffffffffu, !(big * fabsf(to_cap) <= 1.f))) {
           const uint64_t tc2 = fa_pack2(to_cap, to_cap);
 #pragma unroll
@@ -406,7 +415,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
           }
         } else {
 #pragma unroll
-          for (int e = 0; e < 128; ++e) v[e] = __float_as_uint(fa_tanh_any(__uint_as_float(v[e]) * to_cap));
+          for (int e = 0; e < 128; ++e) v[e] = __float_as_uint(tanhf(__uint_as_float(v[e]) * to_cap));
         }
         scl = p.softcap * FA_LOG2E;
       } else if (!(scl > 0.f)) {                         // a head's factor may be zero or negative: the maximum below needs a positive scale
@@ -414,9 +423,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
         for (int e = 0; e < 128; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * scl);
         scl = 1.f;
       }
-      // masks only where a tile can contain invisible keys: uniform test
-      if (key0 + FA_ROWS - 1 > up_min || (key0 < lb_max && key0 + FA_ROWS > keep)) {
-        const int e_hi = up - key0, e_lo = lb - key0, e_keep = keep - key0;
+      if (edge) {
 #pragma unroll
         for (int e = 0; e < 128; ++e)
           if (!(e <= e_hi && (e >= e_lo || e < e_keep))) v[e] = 0xff800000u;   // -inf

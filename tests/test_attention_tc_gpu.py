@@ -74,3 +74,25 @@ def test_paged_cap_gate_sinks_temperature(std, Hq, G, gate):
         want = ref.paged_window_attention(q.float(), *(t.float() for t in clean), table, c, m, D ** -0.5, cap, 0, 0,
                                           **dict(kw, gate=None if g is None else g.float()))
         assert _rel(got, want) < 4e-3
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_soft_cap_does_not_depend_on_unseen_keys(D):
+    """Bits must not change with cache rows past the end, later keys or queries past the end, whatever those hold."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    B, T, Hq, G, page, pages = 2, 200, 8, 2, 64, 8
+    k, v = (torch.randn(B * pages, page, G, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    q = torch.randn(B, T, Hq, D, device="cuda", generator=g).bfloat16()
+    table = torch.arange(B * pages, device="cuda", dtype=torch.int32).view(B, pages)
+    ctx, n = (torch.tensor(x, device="cuda", dtype=torch.int32) for x in ([100, 37], [T, 150]))
+    want = None
+    for fill in (0.0, 3.0, 400.0, -1e4):
+        kk, qq = k.clone(), q.clone()
+        for b in range(B):
+            rows = kk[b * pages:(b + 1) * pages].view(-1, G, D)
+            rows[int(ctx[b] + n[b]):] = fill
+            qq[b, int(n[b]):] = fill
+        torch.full((64 << 20,), fill, device="cuda").mul_(2)          # other kernels in between
+        got = ops.paged_window_attention(qq, kk, v, table, ctx, n, D ** -0.5, 30.0, 0, 0)
+        assert want is None or torch.equal(got, want)
+        want = got
