@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(RTC_THREADS, 2) router_logits_tc_kernel(const 
 }
 
 __global__ void __launch_bounds__(256) router_select_kernel(float* __restrict__ logits, const float* __restrict__ parts, int n_parts, float* __restrict__ topk_w,
-                                                            int* __restrict__ topk_i, int N, int E, int k, RouterSelect sel) {
+                                                            void* __restrict__ topk_i, int N, int E, int k, RouterSelect sel) {
   extern __shared__ float zsm[];                             // per warp: [E] scores, [E] choice scores, [groups] group bests
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tok = blockIdx.x * 8 + warp;
@@ -495,7 +495,8 @@ __global__ void __launch_bounds__(256) router_select_kernel(float* __restrict__ 
     sum += w;
     if (lane == 0) {
       topk_w[(size_t)tok * k + j] = w;
-      topk_i[(size_t)tok * k + j] = bi;
+      if (sel.wide_ids) static_cast<long long*>(topk_i)[(size_t)tok * k + j] = bi;
+      else static_cast<int*>(topk_i)[(size_t)tok * k + j] = bi;
       ch[bi] = -INFINITY;                                    // taken
     }
     __syncwarp();
@@ -525,7 +526,7 @@ int router_parts(int N, int W, int E, bool lp) {
   return (int)std::max<long long>(1, std::min<long long>({4, kNumSMs / blocks, W / RTC_K}));
 }
 
-void router_topk_launch(const void* x, const float* w, float* logits, float* parts, float* topk_w, int* topk_i, int N, int W, int E, int k,
+void router_topk_launch(const void* x, const float* w, float* logits, float* parts, float* topk_w, void* topk_i, int N, int W, int E, int k,
                         const RouterSelect& sel, bool lp, cudaStream_t st) {
   if (N <= 0) return;
   int n_parts = 0;

@@ -92,11 +92,12 @@ struct RouterSelect {
   const float* bias;         // [E] or null: added to the logits
   const float* correction;   // [E] or null: added to the scores for the choice only
   int groups, keep;          // groups <= 1: no group limit
+  int wide_ids;              // the ids are int64
   float renorm_eps, scale;
 };
 // `parts`: [router_parts - 1, N, E] partial logits
 int router_parts(int N, int W, int E, bool lp);
-void router_topk_launch(const void* x, const float* w, float* logits, float* parts, float* topk_w, int* topk_i, int N, int W, int E, int k,
+void router_topk_launch(const void* x, const float* w, float* logits, float* parts, float* topk_w, void* topk_i, int N, int W, int E, int k,
                         const RouterSelect& sel, bool lp, cudaStream_t st);
 
 void short_conv_launch(const void* u, long long u_sb, long long u_st, const float* w, const float* bias, const void* state,

@@ -665,7 +665,7 @@ at::Tensor moe_plain(const at::Tensor& x, const at::Tensor& w_up, const at::Tens
 }
 
 std::tuple<at::Tensor, at::Tensor, at::Tensor> router_topk(const at::Tensor& x, const at::Tensor& w, const OptT& bias, int64_t k, double renorm_eps,
-                                                           int64_t softmax, const OptT& correction, int64_t groups, int64_t keep, double scale) {
+                                                           int64_t softmax, const OptT& correction, int64_t groups, int64_t keep, double scale, bool wide_ids) {
   check_act(x, "router input");
   check_f32(w, "router weight");
   TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && w.dim() == 2 && w.size(1) == x.size(1) && k >= 1 && k <= w.size(0));
@@ -674,8 +674,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> router_topk(const at::Tensor& x, 
   auto f32 = x.options().dtype(at::kFloat);
   auto logits = at::empty({N, E}, f32);
   auto tw = at::empty({N, k}, f32);
-  auto ti = at::empty({N, k}, x.options().dtype(at::kInt));
+  auto ti = at::empty({N, k}, x.options().dtype(wide_ids ? at::kLong : at::kInt));
   RouterSelect sel{};
+  sel.wide_ids = wide_ids ? 1 : 0;
   TORCH_CHECK(softmax >= 0 && softmax <= 2);
   sel.softmax = (int)softmax;
   if (bias.has_value()) {
@@ -691,7 +692,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> router_topk(const at::Tensor& x, 
   sel.groups = (int)groups; sel.keep = (int)keep; sel.renorm_eps = (float)renorm_eps; sel.scale = (float)scale;
   const int kparts = router_parts(N, W, E, is_lp(x));
   auto parts = at::empty({kparts > 1 ? (int64_t)(kparts - 1) * N * E : 0}, f32);
-  router_topk_launch(x.data_ptr(), w.data_ptr<float>(), logits.data_ptr<float>(), parts.data_ptr<float>(), tw.data_ptr<float>(), ti.data_ptr<int>(), N, W, E, (int)k, sel,
+  router_topk_launch(x.data_ptr(), w.data_ptr<float>(), logits.data_ptr<float>(), parts.data_ptr<float>(), tw.data_ptr<float>(), ti.data_ptr(), N, W, E, (int)k, sel,
                      is_lp(x), stream());
   return {logits, tw, ti};
 }

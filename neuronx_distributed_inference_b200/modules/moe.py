@@ -53,16 +53,6 @@ class RouterTopK(nn.Module):
         self.compute_dtype = torch.float32      # router_config["dtype"] (reference RouterConfig): precision of the router GEMM
 
     def forward(self, x: torch.Tensor):
-        logits, w, idx = self.route(x)
-        return logits, w, idx.long() if self.long_ids else idx
-
-    @property
-    def long_ids(self) -> bool:
-        """Renormalised softmax routers hand out int64 ids (``torch.topk``'s), whatever kernel chose them."""
-        return self.act_fn == "softmax" and self.normalize and not self.act_over_topk and self.groups is None and self.score_correction is None
-
-    def route(self, x: torch.Tensor):
-        """:meth:`forward` with the ids in whatever integer type they were made in."""
         extra = (self.score_correction, self.groups, self.scale)
         if self.compute_dtype != torch.float32:
             cd = self.compute_dtype
@@ -178,11 +168,11 @@ class MoE(nn.Module):
         shape = x.shape
         xn = ops.rmsnorm(x, norm_weight, norm_eps, norm_offset) if norm_weight is not None else x
         x2 = xn.reshape(-1, shape[-1])
-        logits, w, idx = getattr(self.router, "route", self.router)(x2) if route is None else (None, *route)
+        logits, w, idx = self.router(x2) if route is None else (None, *route)
         if self.return_router_logits:
             self.last_router_logits = logits
         if self.return_expert_index:
-            self.last_expert_index = idx.long() if getattr(self.router, "long_ids", False) else idx
+            self.last_expert_index = idx
         if self.early_affinity_modulation:
             y = self.expert_mlps(x2, w.to(torch.float32), idx, scale_input=True)   # Llama-4: y = sum_j expert_j(x * w_j)
         else:

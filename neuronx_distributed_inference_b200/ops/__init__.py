@@ -352,13 +352,14 @@ def moe_route(router_logits, top_k, act="softmax", normalize=True, act_over_topk
 
 def router_topk(x, weight, top_k, act="softmax", normalize=True, act_over_topk=False, renorm_eps=None, correction=None, groups=None,
                 scale=1.0, bias=None):
-    """fp32 router: ``logits = x W^T + bias`` (W, bias fp32), then :func:`moe_route`.  Sigmoid routers, softmax routers that are not
-    renormalised or that choose by corrected scores among kept groups, and softmax over the chosen logits alone (``act_over_topk``) run as two kernels on CUDA (fp32 products with the rows in
-    shared memory; scores, group limit, selection and scaling, one warp per token) instead of a cast, a library GEMM and a chain of
-    elementwise / sort launches.  -> (logits, weights [N, k] fp32, expert ids [N, k])."""
+    """fp32 router: ``logits = x W^T + bias`` (W, bias fp32), then :func:`moe_route`, as two kernels on CUDA (fp32 products; scores, group limit,
+    selection and scaling, one warp per token) instead of a cast, a library GEMM and a chain of elementwise / sort launches.
+    -> (logits, weights [N, k] fp32, expert ids [N, k]: int64 from renormalised softmax routers, whose choice is ``torch.topk``'s on the CPU, int32 from the
+    other kernel routes)."""
     E = weight.shape[0]
     plain_softmax = act == "softmax" and (not normalize or correction is not None or groups is not None)
-    if act == "softmax" and normalize and correction is None and groups is None and not act_over_topk:
+    wide = act == "softmax" and normalize and correction is None and groups is None and not act_over_topk
+    if wide:
         plain_softmax, renorm_eps = True, 0.0 if renorm_eps is None else renorm_eps          # the chosen weights are divided by their sum
     over_topk = act == "softmax" and act_over_topk and correction is None and groups is None and renorm_eps is None and scale == 1.0
     if (_mix_cuda(x) and (over_topk or ((act == "sigmoid" or plain_softmax) and not act_over_topk)) and weight.dtype == torch.float32
@@ -366,7 +367,7 @@ def router_topk(x, weight, top_k, act="softmax", normalize=True, act_over_topk=F
         stats["router_topk"] += 1
         count, keep = (int(groups[0]), int(groups[1])) if groups is not None else (1, 1)
         return _C().router_topk(x.contiguous(), weight.contiguous(), None if bias is None else bias.contiguous(), int(top_k),
-                                -1.0 if renorm_eps is None else float(renorm_eps), 2 if over_topk else int(act == "softmax"), None if correction is None else correction.float().contiguous(), count, keep, float(scale))
+                                -1.0 if renorm_eps is None else float(renorm_eps), 2 if over_topk else int(act == "softmax"), None if correction is None else correction.float().contiguous(), count, keep, float(scale), wide)
     logits = torch.nn.functional.linear(x.float(), weight.float(), None if bias is None else bias.float())
     w, idx = moe_route(logits, top_k, act, normalize, act_over_topk, renorm_eps, correction, groups, scale)
     return logits, w, idx

@@ -46,4 +46,6 @@ def test_few_experts_share_the_columns(N, E, W, dtype):
 def test_module_ids_keep_their_type():
     r = RouterTopK(16, 2, 256, device="cuda")
     r.linear_router.weight.data.normal_()
-    assert r(torch.randn(5, 256, device="cuda", dtype=torch.bfloat16))[2].dtype == torch.int64
+    x = torch.randn(5, 256, device="cuda", dtype=torch.bfloat16)
+    assert r(x)[2].dtype == torch.int64 and ops.router_topk(x, r.linear_router.weight, 2)[2].dtype == torch.int64
+    assert ops.router_topk(x, r.linear_router.weight, 2, "sigmoid")[2].dtype == torch.int32
