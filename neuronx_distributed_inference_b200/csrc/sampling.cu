@@ -178,17 +178,17 @@ __global__ void __launch_bounds__(256) topk_group_max_kernel(const T* __restrict
   pdl_launch_dependents();
   pdl_wait();
   constexpr int N = RowVec<T>::N;
-  const T* row = logits + (size_t)blockIdx.y * ld;
+  const T* row = logits + (size_t)blockIdx.x * ld;
   const bool vec = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
   uint32_t m = 0;
 #pragma unroll
   for (int j = 0; j < 32 / N; ++j) {
     uint32_t k[N];
-    row_keys<T>(row, blockIdx.x * TOPK_SLICE + (j * 256 + (int)threadIdx.x) * N, V, vec, k);
+    row_keys<T>(row, blockIdx.y * TOPK_SLICE + (j * 256 + (int)threadIdx.x) * N, V, vec, k);
 #pragma unroll
     for (int e = 0; e < N; ++e) m = max(m, k[e]);
   }
-  gmax[(size_t)blockIdx.y * groups + blockIdx.x * 256 + threadIdx.x] = m;
+  gmax[(size_t)blockIdx.x * groups + blockIdx.y * 256 + threadIdx.x] = m;
 }
 
 // key of the need-th largest element that `each` visits (it calls its argument with every key of this thread), and how many of those equal
@@ -410,7 +410,7 @@ void topk_sample_launch(const void* logits, int dtype, const int* top_k, const f
   const int groups = topk_groups(V);
   auto go = [&](auto* row) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(row)>>;
-    if (groups > 0) launch_pdl(topk_group_max_kernel<T>, dim3(groups / 256, B), dim3(256), 0, stream, row, gmax, V, ld, groups);
+    if (groups > 0) launch_pdl(topk_group_max_kernel<T>, dim3(B, groups / 256), dim3(256), 0, stream, row, gmax, V, ld, groups);
     launch_pdl(topk_sample_kernel<T>, dim3(B), dim3(TOPK_THREADS), (size_t)groups * 4, stream, row, static_cast<const uint32_t*>(gmax), groups, top_k,
                top_p, temperature, rand, out, V, ld, K);
   };

@@ -40,3 +40,12 @@ def test_tokens(kind, V, dtype):
     assert torch.equal(value[rows, got.cpu()], value[rows, want])
     if kind != "ties" and dtype == torch.float32:
         assert torch.equal(got.cpu(), want)
+
+
+def test_more_rows_than_a_grid_dimension():
+    """66000 rows: more than the second dimension of a grid can count."""
+    B, V = 66000, 40
+    logits = torch.randn(B, V, device="cuda")
+    one = torch.ones(B, device="cuda")
+    got = ops.sample(logits, torch.ones(B, device="cuda", dtype=torch.int32), one, one, one * 0.5)
+    assert torch.equal(got, logits.argmax(-1))
