@@ -637,15 +637,22 @@ at::Tensor rope_attention_decode(const at::Tensor& qkv, const at::Tensor& cos, c
 }
 
 // Parts of a row's keys.  The fewer (row, kv head) pairs there are, the more parts fill the chip and shorten the longest row; a part costs a pipeline
-// fill and a share of the combine.  us at 1 / 2 / 4 / 8 / 16 parts (head size 128): 384 pairs, contexts up to 4096: 97 / 92 / 95 / 109; up to 1000: 30 / 37
-// / 49 / 72; 128 pairs up to 4096: 72 / 48 / 45 / 46; 32 pairs up to 4096: 60 / 36 / 25 / 18, up to 500: 12 / 11 / 10 / 10; 8 pairs, 4096: 59 / 35 / 22 / 15 / 14;
-// 1536 pairs up to 4096: 256 / 274 / 312 / 391.
+// fill and a share of the combine.  us of ragged rows, head size 128, at 1 / 2 / 4 / 8 / 16 / 24 / 37 / 64 parts:
+//   1 pair:    4096 keys 66 / 41 / 29 / 21 / 19 / 21 / 23 / 25     32768: 453 / 236 / 127 / 70 / 43 / 37 / 35 / 31      131072: 1776 / 893 / 455 / 236 / 127 / 92 / 72 / 53
+//   8 pairs:   4096 keys 64 / 39 / 27 / 21 / 19 / 21 / 23 / 31     32768: 453 / 234 / 127 / 72 / 49 / 47 / 45 / 53      131072: 1772 / 897 / 465 / 242 / 137 / 123 / 111 / 121
+//   12 pairs:  4096 keys 65 / 41 / 27 / 21 / 20 / 21 / 27 / 33     32768: 451 / 234 / 125 / 70 / 51 / 43 / 47 / 51      131072: 1778 / 895 / 465 / 242 / 168 / 129 / 137 / 131
+//   32 pairs:  1000 keys 23 / 21 / 18 / 16 / 23                    32768: 455 / 240 / 133 / 98 / 98 / 92                131072: 1778 / 918 / 471 / 322 / 268 / 256
+//   64 pairs:  500 keys 16 / 16 / 16 / 23 / 31    4096: 66 / 43 / 33 / 35 / 41    8192: 121 / 74 / 53 / 53 / 55         131072: 1788 / 918 / 598 / 518 / 467
+//   128 pairs: 500 keys 21 / 22 / 28 / 37         4096: 69 / 57 / 57 / 61         32768: 455 / 301 / 264 / 229 / 223
+//   384 pairs: 500 keys 29 / 37 / 49 / 74         4096: 103 / 98 / 100 / 117      32768: 639 / 537 / 475 / 453          1536 pairs, 4096 keys: 256 / 274 / 312 / 391
+// Head size 64 has its minima at the same numbers (32768 keys: 1 pair 303 / 172 / 92 / 52 / 33 / 29 / 27 / 25, 32 pairs 309 / 186 / 104 / 70 / 55 / 59 / 59 / 66).
 static int paged_nsplit(int pairs, int max_keys) {
   const int tiles = std::max(1, (max_keys + 63) / 64);
   if (pairs >= 1024) return 1;
   if (pairs >= 256) return max_keys >= 3072 ? 2 : 1;
   if (pairs >= 96) return std::max(1, std::min(4, max_keys / 1024));
-  return std::min(tiles, pairs > 8 ? 8 : 16);
+  const int some = std::min(tiles, pairs > 32 && max_keys <= 8192 ? 4 : pairs > 8 ? 8 : 16);
+  return std::max(some, std::min({64, 2 * 148 / pairs, max_keys / 512}));       // long rows: two CTAs per SM of at least 512 keys
 }
 
 at::Tensor paged_attention_decode(const at::Tensor& q, const at::Tensor& k_cache, const at::Tensor& v_cache,

@@ -27,3 +27,22 @@ def test_rows(B, T, Hq, Hkv, page, longest, window, sinks, D):
         got = ops.paged_attention_decode(q, kc, vc, table, pos, D ** -0.5, window or None, sk)
         want = ref.paged_attention_decode(q.float(), kc.float(), vc.float(), table, pos, D ** -0.5, window or None, sk)
         assert ((got.float() - want).norm() / want.norm()).item() < 4e-3
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Hkv", [1, 8])
+def test_few_requests_with_long_contexts(Hkv, D):
+    """One request takes up to 64 parts: the rows of the parts and their factors have to fit the workspace and the shared memory of the combine."""
+    Hq, page, ctx = 8 * Hkv if Hkv == 1 else 4 * Hkv, 64, 40001
+    n = -(-ctx // page)
+    k, v = (torch.randn(n, page, Hkv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    table = torch.randperm(n, device="cuda").view(1, n).int()
+    for T in (1, 64 // (Hq // Hkv)):
+        q = torch.randn(1, T, Hq, D, device="cuda", dtype=torch.bfloat16)
+        pos = torch.arange(ctx - T, ctx, device="cuda", dtype=torch.int32).view(1, T)
+        got = ops.paged_attention_decode(q, k, v, table, pos, D ** -0.5)
+        kk, vv = (t[table[0].long()].reshape(-1, Hkv, D)[:ctx].float().repeat_interleave(Hq // Hkv, 1) for t in (k, v))
+        sc = torch.einsum("thd,nhd->thn", q[0].float(), kk) * D ** -0.5
+        sc = sc.masked_fill(torch.arange(ctx, device="cuda") > pos[0].view(T, 1, 1), float("-inf"))
+        want = torch.einsum("thn,nhd->thd", torch.softmax(sc, -1), vv)
+        assert ((got[0].float() - want).norm() / want.norm()).item() < 4e-3
