@@ -105,7 +105,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
   const uint32_t tmem = tmem_slot;
   pdl_launch_dependents();
   // a dense weight that is a parameter does not depend on earlier kernels; everything else does
-  const bool grouped = p.n_active != nullptr, early = warp == 0 && !grouped && !p.w_fresh;
+  const bool grouped = p.n_active != nullptr;
+  bool early = warp == 0 && !grouped && !p.w_fresh;
   if (!early) pdl_wait();
 
   const int n_tiles = (p.n_out + SK_BM - 1) / SK_BM, nkb = p.K / SK_BK;
@@ -117,17 +118,20 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
   if (warp == 0 || warp == 3) {
     // ================= TMA producers: weights, tokens =================
     if (lane == 0) {
-      long long it = 0;
+      int s = 0;                 // counted, not divided out of a 64-bit count: 4096 x 14336, 9 tokens, 30.1 -> 26.1 us
+      uint32_t phase = 0;
       bool go = true;
       for (long long u = u0; u < u1 && go;) {
         const int tile = (int)(u / nkb), kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u));
         const int ei = tile / n_tiles, n0 = (tile % n_tiles) * SK_BM, e = grouped ? p.active[ei] : 0;
         const int row_w = e * p.rows + n0, row_x = grouped ? p.seg_start[ei] : 0;
         const int boxes = grouped ? (p.seg_count[ei] + p.xbox - 1) / p.xbox : 1, box_bytes = p.xbox * SK_BK * 2;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = (int)(it % ST);
-          if (early && it == ST) pdl_wait();         // the ring is full: from here on a wait depends on the warps that wait for earlier kernels
-          go = mbar_wait(&empty_bar[s], (uint32_t)((it / ST) & 1) ^ 1u, stop, p.wait_word);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (early && phase != 0) {       // the ring is full: from here on a wait depends on the warps that wait for earlier kernels
+            pdl_wait();
+            early = false;
+          }
+          go = mbar_wait(&empty_bar[s], phase ^ 1u, stop, p.wait_word);
           if (!go) break;
           uint8_t* st = smem + (size_t)s * stage_bytes;
           if (warp == 0) {
@@ -138,6 +142,10 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
             mbar_expect(&full_bar[s], boxes * box_bytes);
             for (int q = 0; q < boxes; ++q) sk_tma(st + NW * SK_W_BYTES + q * box_bytes, &p.tm_x, kb * SK_BK, row_x + q * p.xbox, &full_bar[s]);
           }
+          if (++s == ST) {
+            s = 0;
+            phase ^= 1u;
+          }
         }
         u += kb1 - kb0;
       }
@@ -145,8 +153,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
   } else if (warp == 1) {
     // ================= MMA issuer =================
     if (lane == 0) {
-      long long it = 0;
-      int seg = 0;
+      int seg = 0, s = 0;
+      uint32_t phase = 0;
       bool go = true;
       for (long long u = u0; u < u1 && go; ++seg) {
         const int kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u)), buf = seg & 1;
@@ -156,9 +164,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
         go = mbar_wait(&tmem_empty[buf], (uint32_t)((seg >> 1) & 1) ^ 1u, stop, p.wait_word);
         if (!go) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = (int)(it % ST);
-          go = mbar_wait(&full_bar[s], (uint32_t)((it / ST) & 1), stop, p.wait_word);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          go = mbar_wait(&full_bar[s], phase, stop, p.wait_word);
           if (!go) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint8_t* st = smem + (size_t)s * stage_bytes;
@@ -171,6 +178,10 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
               sk_umma(tmem + (uint32_t)(buf * acc_cols + w * p.xb), da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb != kb0 || k != 0) ? 1u : 0u);
           }
           sk_commit(&empty_bar[s]);
+          if (++s == ST) {
+            s = 0;
+            phase ^= 1u;
+          }
         }
         if (go) sk_commit(&tmem_full[buf]);
         u += kb1 - kb0;
