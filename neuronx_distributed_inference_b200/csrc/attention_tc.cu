@@ -12,12 +12,16 @@
 //   The two query tiles take turns: while one is in its softmax the tensor pipe works on P V and the next Q K^T of the other.
 //   What bounds it: per pair of tiles (head size 128) the tensor pipe, the exponentials (16 per clock and SM) and shared memory each need
 //   about 2048 clocks; measured about 4400 (both pipes half busy: the chain scores -> softmax -> P V of a tile is longer than the turn of
-//   the other).  One 8192-token prompt, 32 / 8 heads x 128: 0.50 ms (1.1 PFLOP/s); the kernel before this one, one query tile per CTA with P
-//   through shared memory, took 0.95 ms.  Head size 64, 3 x 1000 tokens, window 128: 30 us against 55 us of the mma.sync kernel.
-//   Tried and slower: signalling P in two 64-key halves with the row sum after the second (0.53 ms: the sum no longer hides behind the
-//   exponentials); one query tile per CTA, 256 threads (0.59 ms).
-//   The running maximum is lazy: O and l are rescaled only when a row's maximum grows by more than 2^8, decided per warp, by the softmax
-//   warps themselves: S_j was issued after P V_{j-1}, so "S_j is complete" says that O is quiescent.
+//   the other).  One 8192-token prompt, 32 / 8 heads x 128: 0.51 ms alone (1.08 PFLOP/s), 0.56 ms among others under the power cap; the kernel
+//   before this one, one query tile per CTA with P through shared memory, 1.03 and 1.02 ms.  Head size 64, 3 x 1000 tokens, window 128: 31 us
+//   against 56 us of the mma.sync kernel.
+//   Tried and slower: signalling P in two 64-key halves with the row sum after the second (6 % slower: the sum no longer hides behind the
+//   exponentials); one query tile per CTA, 256 threads (18 % slower).
+//   O and l are rescaled by the softmax warps themselves, decided per warp: S_j was issued after P V_{j-1}, so "S_j is complete" says that O
+//   is quiescent.  Contiguous rows of head size 128 move their maximum only when it grows by more than 2^8; the others move it at once, as the
+//   mma.sync kernels did that they ran on: then a row's largest probability is exactly 1 and takes no rounding (error against 64 bits of the mixed
+//   portions below 2.249e-3, with the lazy maximum 2.337e-3, mma.sync 2.248e-3; 3 x 1000 tokens of head size 64 2.088e-3, 2.143e-3, and 2.059e-3
+//   with that kernel's four maxima per row).  It costs 5 us of the mixed portions' 0.31 ms.
 //
 // Keys come from contiguous [B, T, Hkv, D] tensors or from a PAGED cache [blocks, page, Hkv, D] (page a power of two >= 8: a 128-key tile is
 // 128 / page boxes, whose 1024-byte swizzle atoms line up).  Pages past the last visible key are not fetched, and the rows after it in the
@@ -175,6 +179,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
   constexpr int TILE = FA_ROWS * D * 2;                  // bytes of a [128][D] tile: D / 64 blocks of [128 rows][128 bytes]
   constexpr int HALF = FA_ROWS * 128;
   constexpr int SLOTS = D == 128 ? 5 : 8;                // K and V tiles share one ring: K0 V0 K1 V1 ...
+  constexpr float SLACK = D == 128 && !PAGED ? 8.f : 0.f; // log2 of what a row's largest probability may exceed 1 by
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -388,17 +393,28 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
       for (int c = 0; c < 4; ++c) fa_tmem_ld32(tS + 32 * c, v + 32 * c);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       float scl = hs * FA_LOG2E;                         // scores -> log2 domain
-      // masks only where a tile can contain invisible keys: uniform test
-      const bool edge = key0 + FA_ROWS - 1 > up_min || (key0 < lb_max && key0 + FA_ROWS > keep);
-      const int e_hi = up - key0, e_lo = lb - key0, e_keep = keep - key0;
+      // masks only where a tile can contain invisible keys: uniform tests of its two ends
+      const bool above = key0 + FA_ROWS - 1 > up_min, below = key0 < lb_max && key0 + FA_ROWS > keep;
+      auto unseen = [&](uint32_t value) {
+        const int e_hi = up - key0, e_lo = lb - key0, e_keep = keep - key0;
+        if (above && below) {
+#pragma unroll
+          for (int e = 0; e < 128; ++e)
+            if (!(e <= e_hi && (e >= e_lo || e < e_keep))) v[e] = value;
+        } else if (above) {
+#pragma unroll
+          for (int e = 0; e < 128; ++e)
+            if (e > e_hi) v[e] = value;
+        } else if (below) {
+#pragma unroll
+          for (int e = 0; e < 128; ++e)
+            if (e < e_lo && e >= e_keep) v[e] = value;
+        }
+      };
       if (CAP) {
         // which form of tanh the warp takes must not depend on what a query does not see: later keys, rows of pages that were not fetched (whatever
         // shared memory held), queries past the end
-        if (edge) {
-#pragma unroll
-          for (int e = 0; e < 128; ++e)
-            if (!(e <= e_hi && (e >= e_lo || e < e_keep))) v[e] = 0u;
-        }
+        unseen(0u);
         const float to_cap = hs / p.softcap;
         float big = 0.f;
 #pragma unroll
@@ -423,11 +439,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
         for (int e = 0; e < 128; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * scl);
         scl = 1.f;
       }
-      if (edge) {
-#pragma unroll
-        for (int e = 0; e < 128; ++e)
-          if (!(e <= e_hi && (e >= e_lo || e < e_keep))) v[e] = 0xff800000u;   // -inf
-      }
+      unseen(0xff800000u);                               // -inf
       // row maximum in the domain of v (its scale is positive), four independent chains
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -436,10 +448,11 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
         for (int c = 0; c < 4; ++c) mx4[c] = fmaxf(mx4[c], fmaxf(__uint_as_float(v[e + 2 * c]), __uint_as_float(v[e + 2 * c + 1])));
       const float mx_raw = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       const float mx = (mx_raw == -INFINITY) ? -INFINITY : mx_raw * scl;
-      const bool grow = mx > m_run + 8.f || (m_run == -INFINITY && mx > -INFINITY);
+      const bool grow = mx > m_run + SLACK || (m_run == -INFINITY && mx > -INFINITY);
       const float m_new = grow ? mx : m_run;
       const float alpha = (m_run == -INFINITY) ? 0.f : fa_ex2(m_run - m_new);
-      if (i > 0 && __any_sync(0xffffffffu, grow)) {
+      const bool move = i > 0 && __any_sync(0xffffffffu, grow);
+      if (SLACK > 0.f && move) {                         // seldom: in few registers, beside the scores
 #pragma unroll 1
         for (int c0 = 0; c0 < D; c0 += 32) {
           uint32_t o[32];
@@ -470,6 +483,16 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
         }
         fa_tmem_st32(tS + 32 * c, pk);
       }
+      if (SLACK == 0.f && move) {                        // often: once the scores' registers are free, all of O in flight at once
+        uint32_t o[D];
+#pragma unroll
+        for (int c = 0; c < D; c += 32) fa_tmem_ld32(tO + c, o + c);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int e = 0; e < D; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+#pragma unroll
+        for (int c = 0; c < D; c += 32) fa_tmem_st32(tO + c, o + c);
+      }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -488,7 +511,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
     const __nv_bfloat16* gp = nullptr;
     if (p.gate != nullptr && live_row) {
       gp = p.gate + (long long)b * p.g_sb + (long long)t * p.g_st + (p.gate_per_head ? h : h * D);
-      if (p.gate_per_head) inv *= 1.f / (1.f + __expf(-__bfloat162float(*gp)));
+      if (p.gate_per_head) inv *= 1.f / (1.f + expf(-__bfloat162float(*gp)));
     }
     uint8_t* so = sQ + x * TILE + r * 128;
 #pragma unroll 1
@@ -512,7 +535,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
             for (int k = 0; k < 8; ++k) g[k] = ldg_act_bf16(gp + c0 + e + k);
           }
 #pragma unroll
-          for (int k = 0; k < 8; ++k) f[k] *= 1.f / (1.f + __expf(-g[k]));
+          for (int k = 0; k < 8; ++k) f[k] *= 1.f / (1.f + expf(-g[k]));
         }
         const int ch = ((c0 & 63) + e) >> 3;             // 16-byte chunk of the 128-byte row, XOR-swizzled like TMA does
         *reinterpret_cast<uint4*>(so + (c0 >> 6) * HALF + ((ch ^ (r & 7)) << 4)) =
@@ -602,7 +625,7 @@ void attention_prefill_tc_launch(const void* q, const void* k, const void* v, vo
 
 // Prompt portions over a paged cache.  Sizes this kernel takes: keys and values of one size, 64 or 128, rows on 16-byte boundaries, pages of
 // 2^k >= 8 tokens (smaller ones would break the 8-row swizzle atoms), no distance term; the rest is paged_window_attention_mma_kernel's.
-// 3 rows of up to 1024 tokens over contexts up to 3000, 32 / 8 heads x 128, window 2048, cap, gate: 0.28 ms, mma.sync kernel 0.88 ms.
+// 3 rows of up to 1024 tokens over contexts up to 3000, 32 / 8 heads x 128, window 2048, cap, gate: 0.31 ms, mma.sync kernel 0.90 ms.
 bool paged_attention_tc_supported(const WindowAttnParams& p, bool lp) {
   return lp && p.T >= 16 && p.maps != 2 && p.slopes == nullptr && p.D == p.Dv && (p.D == 64 || p.D == 128) && (p.v_rs * 2) % 16 == 0 && p.page >= 8 &&
          (p.page & (p.page - 1)) == 0 && (long long)p.B * p.Hq * ((p.T + FA_ROWS - 1) / FA_ROWS) <= 0x7fffffffLL &&
