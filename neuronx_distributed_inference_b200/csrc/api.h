@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <string>
+#include <utility>
 #include <vector>
 
 namespace nxdi {
@@ -99,6 +101,10 @@ enum WaitKernel { WAIT_ATTENTION, WAIT_GEMM_PAIR, WAIT_SKINNY, WAIT_PROBE, WAIT_
 unsigned* wait_word(WaitKernel which);
 void check_waits();
 void wait_probe_launch(long long clocks, int* out, cudaStream_t stream);
+// launches of the tensor-core kernels by the host (a graph replay is none): which route calls took
+enum CountedKernel { COUNT_ATTENTION, COUNT_GEMM_PAIR, COUNT_SKINNY, COUNT_GEMM_TCGEN05, COUNT_KERNELS };
+void count_launch(CountedKernel which);
+std::vector<std::pair<std::string, long long>> kernel_launches();
 
 // prompt-sized GEMM on CTA pairs (gemm_pair.cu); tile_expert / tile_row: grouped, m_tiles tiles of up to 256 rows of the M permuted ones (moe_plan256)
 void gemm_pair_launch(const void* a, long long lda, const void* b, const void* bias, const void* residual, void* c, int M, int N, int K, int act,
@@ -174,7 +180,7 @@ struct AttnPrefillParams {
   int causal;
 };
 void attention_prefill_launch(const AttnPrefillParams& p, cudaStream_t stream);
-// tcgen05 / TMEM / TMA flash attention (attention_tc.cu), head_dim 128
+// tcgen05 / TMEM / TMA flash attention (attention_tc.cu), head_dim 128, or 64 without a soft cap
 void attention_prefill_tc_launch(const void* q, const void* k, const void* v, void* out, const float* sinks, int B, int T, int Hq, int Hkv, int D,
                                  float scale, int causal, int window, float softcap, cudaStream_t stream);
 

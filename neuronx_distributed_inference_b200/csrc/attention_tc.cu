@@ -596,6 +596,7 @@ static void fa_go(FaParams& p, cudaStream_t stream) {
     throw std::runtime_error("attention (tensor cores): shared memory size refused");
   check_waits();
   p.wait_word = wait_word(WAIT_ATTENTION);
+  count_launch(COUNT_ATTENTION);
   // grouped heads share their keys two by two; a head of its own takes 256 queries instead
   p.pair_heads = (p.Hq / p.Hkv) % 2 == 0 ? 1 : 0;
   const int span = p.pair_heads ? FA_ROWS : 2 * FA_ROWS;
@@ -603,7 +604,7 @@ static void fa_go(FaParams& p, cudaStream_t stream) {
   launch_pdl(kernel, dim3((unsigned)blocks), dim3(FA_THREADS), smem, stream, p);
 }
 
-// q [B,T,Hq,D], k / v [B,T,Hkv,D] bf16 contiguous, D = 64 or 128 -> out [B,T,Hq,D]
+// q [B,T,Hq,D], k / v [B,T,Hkv,D] bf16 contiguous, D = 128, or 64 without a soft cap -> out [B,T,Hq,D]
 void attention_prefill_tc_launch(const void* q, const void* k, const void* v, void* out, const float* sinks, int B, int T, int Hq, int Hkv, int D,
                                  float scale, int causal, int window, float softcap, cudaStream_t stream) {
   if (B <= 0 || T <= 0) return;
@@ -618,9 +619,8 @@ void attention_prefill_tc_launch(const void* q, const void* k, const void* v, vo
   p.scale = scale; p.softcap = softcap;
   if (D == 128 && softcap > 0.f) fa_go<128, false, true>(p, stream);
   else if (D == 128) fa_go<128, false, false>(p, stream);
-  else if (D == 64 && softcap > 0.f) fa_go<64, false, true>(p, stream);
-  else if (D == 64) fa_go<64, false, false>(p, stream);
-  else throw std::runtime_error("attention (tensor cores): head size 64 or 128");
+  else if (D == 64 && softcap <= 0.f) fa_go<64, false, false>(p, stream);
+  else throw std::runtime_error("attention (tensor cores): head size 128, or 64 without a soft cap");
 }
 
 // Prompt portions over a paged cache.  Sizes this kernel takes: keys and values of one size, 64 or 128, rows on 16-byte boundaries, pages of

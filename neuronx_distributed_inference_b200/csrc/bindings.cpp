@@ -768,8 +768,8 @@ at::Tensor attention_prefill_tc(const at::Tensor& q, const at::Tensor& k, const 
                                 const c10::optional<at::Tensor>& sinks, bool causal, double softcap) {
   TORCH_CHECK(q.is_cuda() && q.dim() == 4 && q.is_contiguous() && k.is_contiguous() && v.is_contiguous() && is_bf16(q) && is_bf16(k) && is_bf16(v));
   const int B = q.size(0), T = q.size(1), Hq = q.size(2), D = q.size(3), Hkv = k.size(2);
-  TORCH_CHECK((D == 64 || D == 128) && k.size(0) == B && k.size(1) == T && k.size(3) == D && v.sizes() == k.sizes() && Hq % Hkv == 0,
-              "attention_prefill_tc: head_dim 64 or 128, equal q/k lengths");
+  TORCH_CHECK((D == 128 || (D == 64 && softcap <= 0.0)) && k.size(0) == B && k.size(1) == T && k.size(3) == D && v.sizes() == k.sizes() && Hq % Hkv == 0,
+              "attention_prefill_tc: head_dim 128, or 64 without a soft cap; equal q/k lengths");
   c10::cuda::CUDAGuard guard(q.device());
   auto out = at::empty_like(q);
   attention_prefill_tc_launch(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), sinks.has_value() ? sinks->data_ptr<float>() : nullptr,
@@ -873,6 +873,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_decode", &nxdi::moe_decode);
   m.def("moe_small", &nxdi::moe_small);
   m.def("check_waits", &nxdi::check_waits);
+  m.def("kernel_launches", &nxdi::kernel_launches);
   m.def("wait_probe", [](int64_t clocks, at::Tensor out) {
     TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kInt && out.numel() >= 1);
     c10::cuda::CUDAGuard guard(out.device());

@@ -350,6 +350,7 @@ void gemm_pair_launch(const void* a, long long lda, const void* b, const void* b
   p.M = M; p.N = N; p.K = K; p.act = act; p.n_out = glu ? N / 2 : N; p.limit = limit; p.alpha = alpha;
   check_waits();
   p.wait_word = wait_word(WAIT_GEMM_PAIR);
+  count_launch(COUNT_GEMM_PAIR);
   p.tile_expert = tile_expert; p.tile_row = tile_row; p.w_fresh = w_fresh ? 1 : 0;
   const int tile_out = glu ? GP_BN / 2 : GP_BN;
   p.m_tiles = tile_expert != nullptr ? m_tiles : (M + 255) / 256;

@@ -749,6 +749,7 @@ static void gemm_launch_impl(const void* a, int lda, const void* b, const void* 
     configured = true;
   }
   const int grid = std::min(n_sms, p.m_tiles * p.n_tiles * p.splits);
+  count_launch(COUNT_GEMM_TCGEN05);
   const dim3 g(grid), b3(GM_THREADS);
   if (fp8) {
     if (TM == 2) launch_pdl(gemm_tcgen05_kernel<2, 128, true>, g, b3, smem, stream, p);

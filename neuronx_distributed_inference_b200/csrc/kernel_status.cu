@@ -45,6 +45,15 @@ void check_waits() {
     }
 }
 
+static std::atomic<long long> g_launches[COUNT_KERNELS];
+void count_launch(CountedKernel which) { g_launches[which].fetch_add(1, std::memory_order_relaxed); }
+std::vector<std::pair<std::string, long long>> kernel_launches() {
+  static const char* const names[COUNT_KERNELS] = {"attention_prefill_tc", "gemm_pair", "skinny_gemm", "gemm_tcgen05"};
+  std::vector<std::pair<std::string, long long>> r;
+  for (int i = 0; i < COUNT_KERNELS; ++i) r.emplace_back(names[i], g_launches[i].load(std::memory_order_relaxed));
+  return r;
+}
+
 // one wait on a barrier that nobody arrives on, given up after `clocks`: what a kernel with such an error reports
 __global__ void __launch_bounds__(32) wait_probe_kernel(long long clocks, unsigned* word, int* out) {
   __shared__ uint64_t bar;

@@ -393,6 +393,7 @@ void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream) {
   p.T = a.tokens; p.n_out = a.n_out; p.K = a.K; p.act = a.act; p.limit = a.limit; p.alpha = a.alpha; p.w_fresh = a.w_fresh;
   check_waits();
   p.wait_word = wait_word(WAIT_SKINNY);
+  count_launch(COUNT_SKINNY);
   const int stage = (glu ? 2 : 1) * SK_W_BYTES + p.xb * SK_BK * 2;
   p.stages = std::min(SK_MAX_STAGES, (SK_SMEM - 1024) / stage);
   int cols = 32;

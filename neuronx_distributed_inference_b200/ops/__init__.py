@@ -45,6 +45,12 @@ def _use_cuda(x: torch.Tensor) -> bool:
                        "(or set NXDI_B200_ALLOW_TORCH_FALLBACK=1)")
 
 
+def kernel_launches():
+    """{kernel: launches by the host} of the tensor-core GEMM and attention kernels: ``stats`` counts calls (``gemm_tcgen05``: those of :func:`linear` that run
+    on tensor cores), this tells which kernel the rules of the extension chose."""
+    return dict(_C().kernel_launches())
+
+
 def check_waits():
     """Raise if a wait inside a tensor-core kernel ran out (csrc/mbar_wait.cuh): its results are invalid.  A read of a few words of host memory, no
     synchronisation: call it where results have reached the host.  The launches of these kernels and every step of the engine do."""
@@ -284,7 +290,7 @@ def attention_prefill(q, k, v, scale, causal: bool = True, window=None, chunk=No
     if (_use_cuda(q) and q.dtype in _FAST_DTYPES and (D == 128 or (D == 64 and softcap is None)) and _ATTN_TC and chunk is None and (causal or not window)
             and key_valid is None and q_pos is None and q.shape[1] == k.shape[1] and k.dtype == q.dtype):
         # Blackwell path: tcgen05 QK^T / PV with TMEM accumulators, TMA tiles (csrc/attention_tc.cu); soft-cap is an argument
-        stats["attn_prefill_tc" if D == 128 else "attn_prefill"] += 1
+        stats["attn_prefill_tc"] += 1
         return _C().attention_prefill_tc(q.contiguous(), k.contiguous(), v.contiguous(), float(scale), int(window or 0), sinks,
                                          bool(causal), float(softcap or 0.0))
     if (_use_cuda(q) and q.dtype in _FAST_DTYPES and D in (64, 128) and chunk is None and (causal or not window)
@@ -433,7 +439,7 @@ def moe_experts(x, w_gate_up, w_down, topk_w, topk_i, act="silu_mul", expert_off
             and w_gate_up.is_contiguous() and w_down.is_contiguous() and x.shape[1] % 64 == 0 and w_down.shape[2] % 64 == 0
             and w_gate_up.shape[0] <= 512
             and (gate_up_bias is None or gate_up_bias.dtype == x.dtype) and (down_bias is None or down_bias.dtype == x.dtype)):
-        stats["moe_decode" if rows_kernel and N <= GEMV_MAX_TOKENS else "moe_grouped"] += 1
+        stats["moe_small"] += 1
         return _C().moe_small(x.contiguous(), w_gate_up, w_down, topk_w.float().contiguous(), topk_i.to(torch.int32).contiguous(), int(expert_offset),
                               _MOE_ACTS[kact], bool(scale_input), None if gate_up_bias is None else gate_up_bias.contiguous(),
                               None if down_bias is None else down_bias.contiguous(), limit, alpha)

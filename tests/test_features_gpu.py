@@ -178,9 +178,9 @@ def test_gpt_oss_and_dbrx_run_under_cuda_graphs_with_grouped_moe():
                 t = a(t, position_ids=torch.full((2, 1), 20 + i, dtype=torch.int32)).tokens.view(2, 1).cpu()
                 out.append(t)
             return torch.cat(out, 1)
-        before = ops.stats["moe_grouped"]
+        before = ops.stats["moe_small"]
         got = run(app)
-        assert ops.stats["moe_grouped"] > before and len(app.token_generation_model._graphs) > 0, cls.__name__
+        assert ops.stats["moe_small"] > before and len(app.token_generation_model._graphs) > 0, cls.__name__
         assert torch.equal(got, run(mk(False))), cls.__name__
 
 
