@@ -134,13 +134,14 @@ long long skinny_gemm_ws_floats(int tokens, bool glu);
 int skinny_gemm_tickets();
 void skinny_clear_launch(unsigned* tickets, int n, cudaStream_t stream);
 void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream);
-void moe_small_gather_launch(const void* x, const float* topk_w, const int* topk_i, int entries, int k, int H, int expert_offset, int e_local,
+// id_step: 1, or 2 when topk_i points at int64 ids (their low words are read)
+void moe_small_gather_launch(const void* x, const float* topk_w, const int* topk_i, int id_step, int entries, int k, int H, int expert_offset, int e_local,
                              int seg_rows, int scale_input, void* xp, int* pos, int* n_active, int* active, int* seg_start, int* seg_count, unsigned* tickets,
                              int n_tickets, cudaStream_t stream);
 void moe_small_combine_launch(const float* y, const float* topk_w, const int* pos, void* out, int N, int H, int k, int scale_input, cudaStream_t stream);
 
 // MoE decode: routed experts for T <= 8 tokens as two batched streaming launches (moe_decode.cu)
-void moe_decode_launch(const void* x, const void* w_gate_up, const void* w_down, const float* topk_w, const int* topk_i, void* u,
+void moe_decode_launch(const void* x, const void* w_gate_up, const void* w_down, const float* topk_w, const int* topk_i, int id_step, void* u,
                        float* y_acc, int T, int topk, int H, int I, int E, int expert_offset, int act /*1 silu*up, 4 clamped gate product*/, float limit,
                        float alpha, int n_sms, cudaStream_t stream);
 
@@ -192,7 +193,7 @@ void gemm_fp8_launch(const void* a, int lda, const void* b, const float* a_scale
                      const void* residual, void* c, int ldc, int M, int N, int K, int act, cudaStream_t stream);
 
 // mixture-of-experts prefill: device-side permutation (moe_grouped.cu) around the grouped tcgen05 GEMM (gemm_tcgen05.cu)
-void moe_plan256_launch(const int* topk_i, int entries, int expert_offset, int e_local, int tiles, int* pos, int* tile_expert, int* tile_row,
+void moe_plan256_launch(const int* topk_i, int id_step, int entries, int expert_offset, int e_local, int tiles, int* pos, int* tile_expert, int* tile_row,
                         cudaStream_t stream);
 void moe_scatter_launch(const void* x, const float* topk_w, const int* pos, void* xp, int N, int H, int k, int scale_input, cudaStream_t stream);
 void moe_plan_launch(const int* topk_i, int entries, int expert_offset, int e_local, int R, int* pos, int* row_entry, int* tile_expert,

@@ -257,6 +257,11 @@ at::Tensor gemv_allreduce(const at::Tensor& x, const at::Tensor& w, const c10::o
   return y;
 }
 
+// Expert ids come as int32, or as int64 from torch.topk and renormalised softmax routers: the kernels read the low words
+static bool is_ids(const at::Tensor& t) { return t.scalar_type() == at::kInt || t.scalar_type() == at::kLong; }
+static int id_step(const at::Tensor& t) { return t.scalar_type() == at::kLong ? 2 : 1; }
+static const int* id_ptr(const at::Tensor& t) { return reinterpret_cast<const int*>(t.data_ptr()); }
+
 // Routed experts of a decode step: x [T,H], w_gate_up [E,2I,H], w_down [E,H,I], topk_w/topk_i [T,k] -> [T,H] (local experts only;
 // the caller all-reduces across EP/TP ranks).
 at::Tensor moe_decode(const at::Tensor& x, const at::Tensor& w_gate_up, const at::Tensor& w_down, const at::Tensor& topk_w,
@@ -266,14 +271,14 @@ at::Tensor moe_decode(const at::Tensor& x, const at::Tensor& w_gate_up, const at
   TORCH_CHECK(w_gate_up.dim() == 3 && w_down.dim() == 3 && w_gate_up.is_contiguous() && w_down.is_contiguous());
   const int T = x.size(0), H = x.size(1), E = w_gate_up.size(0), I = w_gate_up.size(1) / 2, k = topk_i.size(1);
   TORCH_CHECK(w_gate_up.size(2) == H && w_down.size(0) == E && w_down.size(1) == H && w_down.size(2) == I);
-  TORCH_CHECK(topk_w.scalar_type() == at::kFloat && topk_i.scalar_type() == at::kInt && topk_w.is_contiguous() &&
+  TORCH_CHECK(topk_w.scalar_type() == at::kFloat && is_ids(topk_i) && topk_w.is_contiguous() &&
               topk_i.is_contiguous() && topk_w.numel() == (int64_t)T * k && topk_i.size(0) == T);
   c10::cuda::CUDAGuard guard(x.device());
   auto u = at::empty({(int64_t)T * k, I}, x.options());
   auto y = at::zeros({T, H}, x.options().dtype(at::kFloat));
   static int n_sms = 0;
   if (n_sms == 0) n_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-  moe_decode_launch(x.data_ptr(), w_gate_up.data_ptr(), w_down.data_ptr(), topk_w.data_ptr<float>(), topk_i.data_ptr<int>(),
+  moe_decode_launch(x.data_ptr(), w_gate_up.data_ptr(), w_down.data_ptr(), topk_w.data_ptr<float>(), id_ptr(topk_i), id_step(topk_i),
                     u.data_ptr(), y.data_ptr<float>(), T, k, H, I, E, (int)expert_offset, (int)act, (float)limit, (float)alpha, n_sms, cur_stream());
   return y.to(x.scalar_type());
 }
@@ -287,7 +292,7 @@ at::Tensor moe_small(const at::Tensor& x, const at::Tensor& w_gate_up, const at:
   const int N = x.size(0), H = x.size(1), E = w_gate_up.size(0), I = w_gate_up.size(1) / 2, k = topk_i.size(1);
   TORCH_CHECK(w_gate_up.size(1) == 2 * I && w_gate_up.size(2) == H && w_down.size(0) == E && w_down.size(1) == H && w_down.size(2) == I);
   TORCH_CHECK(N >= 1 && N <= SKINNY_MAX_T && H % 64 == 0 && I % 64 == 0 && E <= 512, "moe_small: 1 .. 128 tokens, sizes in multiples of 64, <= 512 experts");
-  TORCH_CHECK(topk_w.scalar_type() == at::kFloat && topk_i.scalar_type() == at::kInt && topk_w.is_contiguous() && topk_i.is_contiguous() &&
+  TORCH_CHECK(topk_w.scalar_type() == at::kFloat && is_ids(topk_i) && topk_w.is_contiguous() && topk_i.is_contiguous() &&
               topk_w.numel() == (int64_t)N * k && topk_i.size(0) == N);
   if (gate_up_bias) TORCH_CHECK(is_bf16(*gate_up_bias) && gate_up_bias->is_contiguous() && gate_up_bias->numel() == (int64_t)E * 2 * I);
   if (down_bias) TORCH_CHECK(is_bf16(*down_bias) && down_bias->is_contiguous() && down_bias->numel() == (int64_t)E * H);
@@ -306,7 +311,7 @@ at::Tensor moe_small(const at::Tensor& x, const at::Tensor& w_gate_up, const at:
   int *n_active = pos + R, *active = n_active + 1, *seg_start = active + segs, *seg_count = seg_start + segs;
   unsigned* tickets = reinterpret_cast<unsigned*>(seg_count + segs);
   auto st = cur_stream();
-  moe_small_gather_launch(x.data_ptr(), topk_w.data_ptr<float>(), topk_i.data_ptr<int>(), (int)R, k, H, (int)expert_offset, E, seg_rows,
+  moe_small_gather_launch(x.data_ptr(), topk_w.data_ptr<float>(), id_ptr(topk_i), id_step(topk_i), (int)R, k, H, (int)expert_offset, E, seg_rows,
                           scale_input ? 1 : 0, xp.data_ptr(), pos, n_active, active, seg_start, seg_count, tickets, (int)(2 * nt), st);
   SkinnyGemm a{};
   a.x = xp.data_ptr(); a.x_rows = R; a.ldx = H; a.w = w_gate_up.data_ptr(); a.bias = optr(gate_up_bias); a.y = h.data_ptr();
@@ -360,7 +365,7 @@ at::Tensor moe_grouped(const at::Tensor& x, const at::Tensor& w_gate_up, const a
     TORCH_CHECK(H % 128 == 0 && I % 128 == 0 && H <= 16384 && I <= 16384, "moe_grouped (fp8): sizes must be multiples of 128, <= 16384");
     TORCH_CHECK(gate_up_scale->numel() == (int64_t)E * 2 * I && down_scale->numel() == (int64_t)E * H);
   }
-  TORCH_CHECK(topk_w.scalar_type() == at::kFloat && topk_i.scalar_type() == at::kInt && topk_w.is_contiguous() &&
+  TORCH_CHECK(topk_w.scalar_type() == at::kFloat && is_ids(topk_i) && (!fp8 || topk_i.scalar_type() == at::kInt) && topk_w.is_contiguous() &&
               topk_i.is_contiguous() && topk_w.numel() == (int64_t)N * k && topk_i.size(0) == N);
   if (gate_up_bias) TORCH_CHECK(is_bf16(*gate_up_bias) && gate_up_bias->is_contiguous() && gate_up_bias->numel() == (int64_t)E * 2 * I);
   if (down_bias) TORCH_CHECK(is_bf16(*down_bias) && down_bias->is_contiguous() && down_bias->numel() == (int64_t)E * H);
@@ -375,7 +380,7 @@ at::Tensor moe_grouped(const at::Tensor& x, const at::Tensor& w_gate_up, const a
     auto st = cur_stream();
     auto pos = at::empty({R}, iopt), tile_expert = at::empty({tiles}, iopt), tile_row = at::empty({tiles}, iopt);
     auto xp = at::empty({R, H}, x.options()), h = at::empty({R, I}, x.options()), y = at::empty({R, H}, x.options());
-    moe_plan256_launch(topk_i.data_ptr<int>(), (int)R, (int)expert_offset, E, (int)tiles, pos.data_ptr<int>(), tile_expert.data_ptr<int>(),
+    moe_plan256_launch(id_ptr(topk_i), id_step(topk_i), (int)R, (int)expert_offset, E, (int)tiles, pos.data_ptr<int>(), tile_expert.data_ptr<int>(),
                        tile_row.data_ptr<int>(), st);
     moe_scatter_launch(x.data_ptr(), topk_w.data_ptr<float>(), pos.data_ptr<int>(), xp.data_ptr(), N, H, k, scale_input ? 1 : 0, st);
     gemm_pair_launch(xp.data_ptr(), H, w_gate_up.data_ptr(), optr(gate_up_bias), nullptr, h.data_ptr(), (int)R, 2 * I, H, (int)act, st,

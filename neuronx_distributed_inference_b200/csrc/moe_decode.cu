@@ -21,7 +21,7 @@ constexpr int MOE_THREADS = 256;
 template <bool GLU>
 __global__ void __launch_bounds__(MOE_THREADS) moe_rows_kernel(const __nv_bfloat16* __restrict__ xin,   // K1: x [T,K]; K2: u [P,K]
                                                                 const __nv_bfloat16* __restrict__ W,     // [E, N_rows, K]
-                                                                const int* __restrict__ topk_i,           // [P]
+                                                                const int* __restrict__ topk_i, int id_step,   // [P]; 2: the low words of int64 ids
                                                                 const float* __restrict__ topk_w,         // [P] (K2 only)
                                                                 __nv_bfloat16* __restrict__ u_out,        // K1: [P, N]
                                                                 float* __restrict__ y_acc,                // K2: [T, N] fp32 (atomics)
@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_rows_kernel(const __nv_bfloat
   pdl_launch_dependents();
   pdl_wait();
   const int p = blockIdx.y, t = p / topk;
-  const int e = topk_i[p] - expert_offset;
+  const int e = topk_i[(size_t)p * id_step] - expert_offset;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rows_per = (N + gridDim.x - 1) / gridDim.x;
   const int r0 = blockIdx.x * rows_per, r1 = min(N, r0 + rows_per);
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_rows_kernel(const __nv_bfloat
   }
 }
 
-void moe_decode_launch(const void* x, const void* w_gate_up, const void* w_down, const float* topk_w, const int* topk_i, void* u,
+void moe_decode_launch(const void* x, const void* w_gate_up, const void* w_down, const float* topk_w, const int* topk_i, int id_step, void* u,
                        float* y_acc, int T, int topk, int H, int I, int E, int expert_offset, int act, float limit, float alpha, int n_sms,
                        cudaStream_t stream) {
   const int P = T * topk;
@@ -100,10 +100,10 @@ void moe_decode_launch(const void* x, const void* w_gate_up, const void* w_down,
   }
   if ((size_t)H * 2 > 64 * 1024 || (size_t)I * 2 > 64 * 1024) throw std::runtime_error("moe_decode: row too wide for shared memory");
   launch_pdl(k1, dim3(std::min(gx, I), P), dim3(MOE_THREADS), (size_t)H * 2, stream, reinterpret_cast<const __nv_bfloat16*>(x),
-             reinterpret_cast<const __nv_bfloat16*>(w_gate_up), topk_i, topk_w, reinterpret_cast<__nv_bfloat16*>(u),
+             reinterpret_cast<const __nv_bfloat16*>(w_gate_up), topk_i, id_step, topk_w, reinterpret_cast<__nv_bfloat16*>(u),
              static_cast<float*>(nullptr), H, I, topk, E, expert_offset, act, limit, alpha);
   launch_pdl(k2, dim3(std::min(gx, H), P), dim3(MOE_THREADS), (size_t)I * 2, stream, reinterpret_cast<const __nv_bfloat16*>(u),
-             reinterpret_cast<const __nv_bfloat16*>(w_down), topk_i, topk_w, static_cast<__nv_bfloat16*>(nullptr), y_acc, I, H, topk,
+             reinterpret_cast<const __nv_bfloat16*>(w_down), topk_i, id_step, topk_w, static_cast<__nv_bfloat16*>(nullptr), y_acc, I, H, topk,
              E, expert_offset, act, limit, alpha);
 }
 

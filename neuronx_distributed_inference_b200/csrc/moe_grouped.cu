@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(128) moe_combine_kernel(const __nv_bfloat16* _
 // ---- bf16 experts on CTA-pair tiles (gemm_pair.cu): rows one after the other, up to 256 of an expert per tile ------------------------------------------------------
 // One CTA: the atomic that counts an expert's entries also ranks them, so one pass decides the rows and the second only adds the segment starts
 // (32768 entries, 128 experts: 11 us; with a second atomic pass, a serial scan and the inverse table 31 us).
-__global__ void __launch_bounds__(MOE_PLAN_THREADS) moe_plan256_kernel(const int* __restrict__ topk_i, int entries, int expert_offset, int e_local, int tiles,
+__global__ void __launch_bounds__(MOE_PLAN_THREADS) moe_plan256_kernel(const int* __restrict__ topk_i, int id_step, int entries, int expert_offset, int e_local, int tiles,
                                                                        int* __restrict__ pos, int* __restrict__ tile_expert, int* __restrict__ tile_row) {
   __shared__ int count[MOE_MAX_E], start[MOE_MAX_E], tile0[MOE_MAX_E + 1];
   pdl_launch_dependents();
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(MOE_PLAN_THREADS) moe_plan256_kernel(const int
   for (int i0 = tid; i0 < entries; i0 += U * MOE_PLAN_THREADS) {
     int e[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) e[u] = i0 + u * MOE_PLAN_THREADS < entries ? topk_i[i0 + u * MOE_PLAN_THREADS] - expert_offset : -1;
+    for (int u = 0; u < U; ++u) e[u] = i0 + u * MOE_PLAN_THREADS < entries ? topk_i[(size_t)(i0 + u * MOE_PLAN_THREADS) * id_step] - expert_offset : -1;
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (i0 + u * MOE_PLAN_THREADS < entries) pos[i0 + u * MOE_PLAN_THREADS] = (e[u] >= 0 && e[u] < e_local) ? atomicAdd(&count[e[u]], 1) : -1;
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(MOE_PLAN_THREADS) moe_plan256_kernel(const int
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = i0 + u * MOE_PLAN_THREADS;
-      e[u] = i < entries ? topk_i[i] - expert_offset : -1;
+      e[u] = i < entries ? topk_i[(size_t)i * id_step] - expert_offset : -1;
       r[u] = i < entries ? pos[i] : -1;
     }
 #pragma unroll
@@ -210,10 +210,10 @@ __global__ void __launch_bounds__(256) moe_scatter_kernel(const __nv_bfloat16* _
   }
 }
 
-void moe_plan256_launch(const int* topk_i, int entries, int expert_offset, int e_local, int tiles, int* pos, int* tile_expert, int* tile_row,
+void moe_plan256_launch(const int* topk_i, int id_step, int entries, int expert_offset, int e_local, int tiles, int* pos, int* tile_expert, int* tile_row,
                         cudaStream_t stream) {
   if (e_local > MOE_MAX_E) throw std::runtime_error("moe_plan: more than 512 local experts");
-  launch_pdl(moe_plan256_kernel, dim3(1), dim3(MOE_PLAN_THREADS), 0, stream, topk_i, entries, expert_offset, e_local, tiles, pos, tile_expert,
+  launch_pdl(moe_plan256_kernel, dim3(1), dim3(MOE_PLAN_THREADS), 0, stream, topk_i, id_step, entries, expert_offset, e_local, tiles, pos, tile_expert,
              tile_row);
 }
 void moe_scatter_launch(const void* x, const float* topk_w, const int* pos, void* xp, int N, int H, int k, int scale_input, cudaStream_t stream) {

@@ -411,7 +411,7 @@ void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream) {
 // and a copy of the token's row to that place.  Block 0 also writes the segments (an expert's rows, cut every seg_rows of them) and clears the tickets
 // of the two GEMMs.
 __global__ void __launch_bounds__(256) moe_small_gather_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ topk_w,
-                                                               const int* __restrict__ topk_i, int entries, int k, int H, int expert_offset, int e_local,
+                                                               const int* __restrict__ topk_i, int id_step, int entries, int k, int H, int expert_offset, int e_local,
                                                                int seg_rows, int scale_input, __nv_bfloat16* __restrict__ xp, int* __restrict__ pos,
                                                                int* __restrict__ n_active, int* __restrict__ active, int* __restrict__ seg_start,
                                                                int* __restrict__ seg_count, unsigned* __restrict__ tickets, int n_tickets) {
@@ -419,12 +419,12 @@ __global__ void __launch_bounds__(256) moe_small_gather_kernel(const __nv_bfloat
   pdl_wait();
   __shared__ int s_sum[8];
   const int i = blockIdx.x, tid = threadIdx.x;
-  const int e = topk_i[i] - expert_offset;
+  const int e = topk_i[(size_t)i * id_step] - expert_offset;
   const bool mine = e >= 0 && e < e_local;
   int before = 0;
   if (mine)
     for (int j = tid; j < entries; j += 256) {
-      const int ej = topk_i[j] - expert_offset;
+      const int ej = topk_i[(size_t)j * id_step] - expert_offset;
       before += ej >= 0 && (ej < e || (ej == e && j < i));
     }
   before = __reduce_add_sync(0xffffffffu, before);
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(256) moe_small_gather_kernel(const __nv_bfloat
     for (int c = tid; c < e_local; c += 256) s_cnt[c] = 0;
     __syncthreads();
     for (int j = tid; j < entries; j += 256) {
-      const int ej = topk_i[j] - expert_offset;
+      const int ej = topk_i[(size_t)j * id_step] - expert_offset;
       if (ej >= 0 && ej < e_local) atomicAdd(&s_cnt[ej], 1);
     }
     __syncthreads();
@@ -500,11 +500,11 @@ __global__ void __launch_bounds__(256) moe_small_combine_kernel(const float* __r
   *reinterpret_cast<uint2*>(out + (size_t)tok * H + v * 4) = make_uint2(pack_bf16(f.x, f.y), pack_bf16(f.z, f.w));
 }
 
-void moe_small_gather_launch(const void* x, const float* topk_w, const int* topk_i, int entries, int k, int H, int expert_offset, int e_local,
+void moe_small_gather_launch(const void* x, const float* topk_w, const int* topk_i, int id_step, int entries, int k, int H, int expert_offset, int e_local,
                              int seg_rows, int scale_input, void* xp, int* pos, int* n_active, int* active, int* seg_start, int* seg_count, unsigned* tickets,
                              int n_tickets, cudaStream_t stream) {
   if (e_local > 512 || H % 8 != 0) throw std::runtime_error("moe (small step): at most 512 experts, hidden size % 8 == 0");
-  launch_pdl(moe_small_gather_kernel, dim3(entries), dim3(256), 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), topk_w, topk_i, entries, k, H,
+  launch_pdl(moe_small_gather_kernel, dim3(entries), dim3(256), 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), topk_w, topk_i, id_step, entries, k, H,
              expert_offset, e_local, seg_rows, scale_input, reinterpret_cast<__nv_bfloat16*>(xp), pos, n_active, active, seg_start, seg_count, tickets, n_tickets);
 }
 void moe_small_combine_launch(const float* y, const float* topk_w, const int* pos, void* out, int N, int H, int k, int scale_input, cudaStream_t stream) {

@@ -440,14 +440,14 @@ def moe_experts(x, w_gate_up, w_down, topk_w, topk_i, act="silu_mul", expert_off
             and w_gate_up.shape[0] <= 512
             and (gate_up_bias is None or gate_up_bias.dtype == x.dtype) and (down_bias is None or down_bias.dtype == x.dtype)):
         stats["moe_small"] += 1
-        return _C().moe_small(x.contiguous(), w_gate_up, w_down, topk_w.float().contiguous(), topk_i.to(torch.int32).contiguous(), int(expert_offset),
+        return _C().moe_small(x.contiguous(), w_gate_up, w_down, topk_w.float().contiguous(), _expert_ids(topk_i), int(expert_offset),
                               _MOE_ACTS[kact], bool(scale_input), None if gate_up_bias is None else gate_up_bias.contiguous(),
                               None if down_bias is None else down_bias.contiguous(), limit, alpha)
     if (_use_cuda(x) and x.dtype in _FAST_DTYPES and w_gate_up.dtype == x.dtype and rows_kernel and N <= GEMV_MAX_TOKENS
             and w_gate_up.is_contiguous() and w_down.is_contiguous() and topk_i.dim() == 2):
         stats["moe_decode"] += 1
         return _C().moe_decode(x.contiguous(), w_gate_up, w_down, topk_w.float().contiguous(),
-                               topk_i.to(torch.int32).contiguous(), int(expert_offset), _MOE_ACTS[act], limit, alpha)
+                               _expert_ids(topk_i), int(expert_offset), _MOE_ACTS[act], limit, alpha)
     # prefill-sized batches: device-side permutation + grouped tcgen05 GEMMs (static shapes: replays under CUDA graphs)
     if (_use_cuda(x) and _MOE_GROUPED and x.dtype == torch.bfloat16 and w_gate_up.dtype == x.dtype and w_down.dtype == x.dtype
             and kact in _MOE_ACTS and topk_i.dim() == 2 and topk_i.shape[1] <= 64
@@ -455,12 +455,17 @@ def moe_experts(x, w_gate_up, w_down, topk_w, topk_i, act="silu_mul", expert_off
             and w_gate_up.shape[0] <= 512
             and (gate_up_bias is None or gate_up_bias.dtype == x.dtype) and (down_bias is None or down_bias.dtype == x.dtype)):
         stats["moe_grouped"] += 1
-        return _C().moe_grouped(x.contiguous(), w_gate_up, w_down, topk_w.float().contiguous(), topk_i.to(torch.int32).contiguous(),
+        return _C().moe_grouped(x.contiguous(), w_gate_up, w_down, topk_w.float().contiguous(), _expert_ids(topk_i),
                                 int(expert_offset), _MOE_ACTS[kact], bool(scale_input),
                                 None if gate_up_bias is None else gate_up_bias.contiguous(),
                                 None if down_bias is None else down_bias.contiguous(), None, None, limit, alpha)
     return ref.moe_experts(x, w_gate_up, w_down, topk_w, topk_i, act, expert_offset, gate_up_bias, down_bias,
                            act_fn, scale_input, act_params=act_params)
+
+
+def _expert_ids(ids):
+    """Ids as these kernels read them: int32 or int64."""
+    return (ids if ids.dtype in (torch.int32, torch.int64) else ids.to(torch.int32)).contiguous()
 
 
 _MOE_GROUPED = os.environ.get("NXDI_B200_MOE_GROUPED", "1") == "1"

@@ -61,3 +61,13 @@ def test_workspaces_follow_the_entries():
     ops.moe_experts(x, wg, wd, w, i, "silu_mul")
     rows = 2 * N * k * (2 * H + I) + 2 * N * H               # permuted rows, products, intermediate rows and the result in bf16
     assert torch.cuda.max_memory_allocated() - base < rows + (1 << 20)
+
+
+@pytest.mark.parametrize("N", [2, 16, 200])            # a warp per weight row, weights as the M operand, CTA pairs
+def test_ids_of_either_width(N):
+    E, k, H, I = 8, 2, 256, 192
+    wg, wd = _experts(E, H, I)
+    x, w = torch.randn(N, H, device=DEV, dtype=BF), torch.rand(N, k, device=DEV)
+    i = torch.rand(N, E + 4, device=DEV).topk(k, -1).indices          # some experts live elsewhere
+    assert torch.equal(ops.moe_experts(x, wg, wd, w, i, "silu_mul", 2), ops.moe_experts(x, wg, wd, w, i.int(), "silu_mul", 2))
+    _check(x, wg, wd, w, i.int(), 2)
