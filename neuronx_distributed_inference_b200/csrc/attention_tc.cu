@@ -13,7 +13,7 @@
 //   What bounds it: per pair of tiles (head size 128) the tensor pipe, the exponentials (16 per clock and SM) and shared memory each need
 //   about 2048 clocks; measured about 4400 (both pipes half busy: the chain scores -> softmax -> P V of a tile is longer than the turn of
 //   the other).  One 8192-token prompt, 32 / 8 heads x 128: 0.51 ms alone (1.08 PFLOP/s), 0.56 ms among others under the power cap; the kernel
-//   before this one, one query tile per CTA with P through shared memory, 1.03 and 1.02 ms.  Head size 64, 3 x 1000 tokens, window 128: 31 us
+//   before this one, one query tile per CTA with P through shared memory, 1.03 and 1.02 ms.  Head size 64, 3 x 1000 tokens, window 128: 30 us
 //   against 56 us of the mma.sync kernel.
 //   Tried and slower: signalling P in two 64-key halves with the row sum after the second (6 % slower: the sum no longer hides behind the
 //   exponentials); one query tile per CTA, 256 threads (18 % slower).
@@ -21,7 +21,7 @@
 //   is quiescent.  Contiguous rows of head size 128 move their maximum only when it grows by more than 2^8; the others move it at once, as the
 //   mma.sync kernels did that they ran on: then a row's largest probability is exactly 1 and takes no rounding (error against 64 bits of the mixed
 //   portions below 2.249e-3, with the lazy maximum 2.337e-3, mma.sync 2.248e-3; 3 x 1000 tokens of head size 64 2.088e-3, 2.143e-3, and 2.059e-3
-//   with that kernel's four maxima per row).  It costs 5 us of the mixed portions' 0.31 ms.
+//   with that kernel's four maxima per row).  It costs 4 of 83 us at two portions of up to 969 tokens over contexts up to 2556 without a cap.
 //
 // Keys come from contiguous [B, T, Hkv, D] tensors or from a PAGED cache [blocks, page, Hkv, D] (page a power of two >= 8: a 128-key tile is
 // 128 / page boxes, whose 1024-byte swizzle atoms line up).  Pages past the last visible key are not fetched, and the rows after it in the
@@ -393,35 +393,15 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
       for (int c = 0; c < 4; ++c) fa_tmem_ld32(tS + 32 * c, v + 32 * c);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       float scl = hs * FA_LOG2E;                         // scores -> log2 domain
-      // masks only where a tile can contain invisible keys: uniform tests of its two ends
-      const bool above = key0 + FA_ROWS - 1 > up_min, below = key0 < lb_max && key0 + FA_ROWS > keep;
-      auto unseen = [&](uint32_t value) {
-        const int e_hi = up - key0, e_lo = lb - key0, e_keep = keep - key0;
-        if (above && below) {
-#pragma unroll
-          for (int e = 0; e < 128; ++e)
-            if (!(e <= e_hi && (e >= e_lo || e < e_keep))) v[e] = value;
-        } else if (above) {
-#pragma unroll
-          for (int e = 0; e < 128; ++e)
-            if (e > e_hi) v[e] = value;
-        } else if (below) {
-#pragma unroll
-          for (int e = 0; e < 128; ++e)
-            if (e < e_lo && e >= e_keep) v[e] = value;
-        }
-      };
       if (CAP) {
-        // which form of tanh the warp takes must not depend on what a query does not see: later keys, rows of pages that were not fetched (whatever
-        // shared memory held), queries past the end
-        unseen(0u);
         const float to_cap = hs / p.softcap;
         float big = 0.f;
 #pragma unroll
         for (int e = 0; e < 128; ++e) big = fmaxf(big, fabsf(__uint_as_float(v[e])));
-        if (t >= qn) big = 0.f;
+        const uint64_t tc2 = fa_pack2(to_cap, to_cap);
+        // the maximum is taken over scores that the row does not see too (later keys, rows of pages that were not fetched, whatever shared memory
+        // held): both ways give a score the same bits
         if (!__any_sync(0xffffffffu, !(big * fabsf(to_cap) <= 1.f))) {
-          const uint64_t tc2 = fa_pack2(to_cap, to_cap);
 #pragma unroll
           for (int e = 0; e < 128; e += 2) {
             float a, c;
@@ -431,7 +411,14 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
           }
         } else {
 #pragma unroll
-          for (int e = 0; e < 128; ++e) v[e] = __float_as_uint(tanhf(__uint_as_float(v[e]) * to_cap));
+          for (int e = 0; e < 128; e += 2) {
+            const uint64_t x2 = fa_mul2(fa_pack2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), tc2);
+            float x, y, a, c;
+            fa_unpack2(x2, x, y);
+            fa_unpack2(fa_tanh2_small(x2), a, c);
+            v[e] = __float_as_uint(fabsf(x) <= 1.f ? a : tanhf(x));
+            v[e + 1] = __float_as_uint(fabsf(y) <= 1.f ? c : tanhf(y));
+          }
         }
         scl = p.softcap * FA_LOG2E;
       } else if (!(scl > 0.f)) {                         // a head's factor may be zero or negative: the maximum below needs a positive scale
@@ -439,7 +426,20 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
         for (int e = 0; e < 128; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * scl);
         scl = 1.f;
       }
-      unseen(0xff800000u);                               // -inf
+      // masks only where a tile can contain invisible keys: uniform tests of its two ends
+      const bool above = key0 + FA_ROWS - 1 > up_min, below = key0 < lb_max && key0 + FA_ROWS > keep;
+      if (above || below) {
+        const int e_hi = up - key0, e_lo = lb - key0, e_keep = keep - key0;
+        if (!below) {
+#pragma unroll
+          for (int e = 0; e < 128; ++e)
+            if (e > e_hi) v[e] = 0xff800000u;            // -inf
+        } else {
+#pragma unroll
+          for (int e = 0; e < 128; ++e)
+            if (!(e <= e_hi && (e >= e_lo || e < e_keep))) v[e] = 0xff800000u;
+        }
+      }
       // row maximum in the domain of v (its scale is positive), four independent chains
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -489,7 +489,12 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
         for (int c = 0; c < D; c += 32) fa_tmem_ld32(tO + c, o + c);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int e = 0; e < D; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+        for (int e = 0; e < D; e += 2) {
+          float a, c;
+          fa_unpack2(fa_mul2(fa_pack2(__uint_as_float(o[e]), __uint_as_float(o[e + 1])), fa_pack2(alpha, alpha)), a, c);
+          o[e] = __float_as_uint(a);
+          o[e + 1] = __float_as_uint(c);
+        }
 #pragma unroll
         for (int c = 0; c < D; c += 32) fa_tmem_st32(tO + c, o + c);
       }
@@ -625,7 +630,7 @@ void attention_prefill_tc_launch(const void* q, const void* k, const void* v, vo
 
 // Prompt portions over a paged cache.  Sizes this kernel takes: keys and values of one size, 64 or 128, rows on 16-byte boundaries, pages of
 // 2^k >= 8 tokens (smaller ones would break the 8-row swizzle atoms), no distance term; the rest is paged_window_attention_mma_kernel's.
-// 3 rows of up to 1024 tokens over contexts up to 3000, 32 / 8 heads x 128, window 2048, cap, gate: 0.31 ms, mma.sync kernel 0.90 ms.
+// 3 rows of up to 1024 tokens over contexts up to 3000, 32 / 8 heads x 128, window 2048, cap, gate: 0.28 ms, mma.sync kernel 0.89 ms.
 bool paged_attention_tc_supported(const WindowAttnParams& p, bool lp) {
   return lp && p.T >= 16 && p.maps != 2 && p.slopes == nullptr && p.D == p.Dv && (p.D == 64 || p.D == 128) && (p.v_rs * 2) % 16 == 0 && p.page >= 8 &&
          (p.page & (p.page - 1)) == 0 && (long long)p.B * p.Hq * ((p.T + FA_ROWS - 1) / FA_ROWS) <= 0x7fffffffLL &&
