@@ -159,8 +159,8 @@ at::Tensor gemv(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
 
 // tcgen05 GEMM for T > 8 tokens (prefill, long speculation windows)
 // Where the swapped, evenly split GEMM (skinny_gemm.cu) beats the 128-row token tiles of gemm_tcgen05.cu (us, skinny / tiles; 37, 64 and 128 tokens):
-//   gate|up 28672 x 4096: 51 / 61, 55 / 62, 66 / 62     17280 x 3200: 33 / 33, 38 / 34, 46 / 34    16384 x 2048: 24 / 26, 26 / 26, 37 / 26
-//   plain 4096 x 14336:   34 / 52, 35 / 53, 42 / 54     6144 x 4096:  21 / 24, 21 / 24, 27 / 24    2048 x 8192:  20 / 35, 21 / 35, 29 / 36
+//   gate|up 28672 x 4096: 52 / 62, 55 / 63, 69 / 63     17280 x 3200: 33 / 34, 35 / 34, 46 / 34    16384 x 2048: 23 / 26, 26 / 26, 36 / 26
+//   plain 4096 x 14336:   30 / 52, 31 / 52, 39 / 54     6144 x 4096:  18 / 23, 19 / 23, 25 / 24    2048 x 8192:  19 / 34, 20 / 35, 27 / 36
 // Its last tile's epilogue grows with the tokens (a feature per lane, all tokens in turn, twice that with a gate product), while the tile kernel's
 // time does not change up to 128; deep K leaves the tile kernel few tiles.
 // Where 256 x 256 tiles on CTA pairs (gemm_pair.cu) beat the one-CTA tiles (us, pairs / one CTA, isolated):

@@ -11,8 +11,8 @@
 //   * accumulators (128 features x tokens) sit in TMEM twice, so a tile's epilogue overlaps the stream of the next one.  A lane holds one output
 //     feature: a warp's store of one token is 64 contiguous bytes, gate and up of a feature meet in one thread.
 //   * eight epilogue warps: the last tile's epilogue is the tail of the launch (four warps: 56 instead of 51 us at 37 tokens, 28672 x 4096).
-// Measured (us, here / 128-row token tiles): see skinny_pays in bindings.cpp.  28672 x 4096 at 9 tokens 46 us = 5.1 TB/s; eight Mixtral-sized experts, 6
-// tokens: 407 us = 6.1 TB/s (one warp per weight row and (token, slot) pair: 760 us).
+// Measured (us, here / 128-row token tiles): see skinny_pays in bindings.cpp.  28672 x 4096 at 9 tokens 46 us = 5.1 TB/s; six of eight Mixtral-sized
+// experts, 6 tokens, with permutation and sum: 336 us = 6.3 TB/s (one warp per weight row and (token, slot) pair: 744 us).
 #include <algorithm>
 #include <stdexcept>
 #include <string>

@@ -469,9 +469,9 @@ def _expert_ids(ids):
 
 
 _MOE_GROUPED = os.environ.get("NXDI_B200_MOE_GROUPED", "1") == "1"
-# measured (us, rows kernel / small-step path): 128 experts, 8 chosen, 2048 x 768: 26 / 37, 39 / 59, 80 / 78, 141 / 113 at 1, 2, 4, 8 tokens; 8 experts, 2 chosen,
-# 4096 x 14336: 129 / 141, 209 / 195 and 686 / 412 at 1, 2 and 8.  Against the padded grouped GEMMs at 12, 48 and 128 tokens: 228 / 140, 346 / 223, 354 / 244 and
-# 510 / 464, 512 / 491, 575 / 509
+# measured (us, rows kernel / small-step path): 128 experts, 8 chosen, 2048 x 768: 26 / 36, 37 / 57, 80 / 74, 137 / 105 at 1, 2, 4, 8 tokens; 8 experts, 2 chosen,
+# 4096 x 14336: 132 / 139, 222 / 185 and 697 / 386 at 1, 2 and 8.  Against the CTA-pair path at 12, 48 and 128 tokens: 147 / 129, 259 / 210, 271 / 219 and
+# 539 / 436, 568 / 461, 587 / 543; 16 experts, 4 chosen, 6144 x 1344: 254 / 186, 190 / 163, 201 / 175 at 16, 48 and 128
 _MOE_ROWS_TOKENS, _MOE_SMALL_TOKENS = 2, 128
 _MOE_ACTS = {"silu_mul": 1, "gelu_tanh_mul": 2, "gelu_mul": 3, "gpt_oss_glu": 4, "clamped_glu": 4}      # 4 takes (limit, alpha); gpt_oss_glu: 7, 1.702
 _UNARY_ACTS = {"relu": 1, "relu2": 2, "silu": 3, "gelu_tanh": 4, "sigmoid": 5, "gelu": 6}         # codes of csrc/seqmix.cu (unary_act, moe_plain, gated_act_mul)

@@ -34,3 +34,26 @@ def test_a_wait_that_runs_out_raises_once_and_leaves_the_context_usable(where):
         ops.check_waits() if where == "asked" else ops.linear(x, w)
     ops.check_waits()
     assert ((ops.linear(x, w).float() - x.float() @ w.float().t()).norm() / (x.float() @ w.float().t()).norm()).item() < 3e-3
+
+
+@pytest.mark.gpu
+def test_the_first_launch_of_a_process_may_be_captured():
+    """The words that kernels report to are allocated by the first launch, which may be inside a stream capture."""
+    import subprocess
+    import sys
+    code = """
+import torch
+from neuronx_distributed_inference_b200 import ops
+x, w = torch.randn(16, 256, device="cuda").bfloat16(), torch.randn(256, 256, device="cuda").bfloat16()
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    y = ops.linear(x, w)
+g.replay()
+torch.cuda.synchronize()
+ops.check_waits()
+want = x.float() @ w.float().t()
+assert ((y.float() - want).norm() / want.norm()).item() < 3e-3
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
