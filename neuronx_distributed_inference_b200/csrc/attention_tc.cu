@@ -2,21 +2,24 @@
 // AND whose probabilities live in TENSOR MEMORY; Q / K / V tiles arrive through TMA (SWIZZLE_128B); the softmax owns one query row per
 // thread (tcgen05.ld of its TMEM lane), so no cross-thread reductions exist anywhere.
 //
-//   CTA = two 128-query tiles of one batch row that read the same keys: the same queries of two neighbouring q heads of a kv head (grouped
-//   heads), or 256 consecutive queries of one head.  384 threads: warps 0-3 softmax of tile a, warps 4-7 softmax of tile b, warp 8 MMA
-//   issuer (one thread), warp 9 TMA producer, warp 10 zeroes the value rows past the end of a paged row (see below).
+//   CTA = one or two 128-query tiles of one batch row (NX; the rule stands at fa_go).  Two tiles read the same keys: the same queries of two neighbouring
+//   q heads of a kv head (grouped heads), or 256 consecutive queries of one head.  Per tile four softmax warps, then an MMA warp, a TMA warp, a warp
+//   that zeroes the value rows past the end of a paged row (see below).
 //   per 128-key tile j and query tile x:
 //     S_x = Q_x K_j^T     D/16 x UMMA 128x128x16 (shared-memory operands)                      -> TMEM cols [128 x, 128 x + 128)
 //     P_x = exp2(S_x c - m)   registers -> bf16 -> TMEM, over the first half of S_x (a thread has read its whole row before)
 //     O_x += P_x V_j      8 x UMMA 128xDx16 with A = P_x from TMEM, B = V_j in its natural [key][d] layout = MN-major
-//   The two query tiles take turns: while one is in its softmax the tensor pipe works on P V and the next Q K^T of the other.
+//   Query tiles take turns: while one is in its softmax the tensor pipe works on P V and the next Q K^T of the other.  P is handed over in two
+//   64-key halves: P V of the first runs while the second is exponentiated.
 //   What bounds it: per pair of tiles (head size 128) the tensor pipe, the exponentials (16 per clock and SM) and shared memory each need
-//   about 2048 clocks; measured about 4400 (both pipes half busy: the chain scores -> softmax -> P V of a tile is longer than the turn of
-//   the other).  One 8192-token prompt, 32 / 8 heads x 128: 0.51 ms alone (1.08 PFLOP/s), 0.56 ms among others under the power cap; the kernel
-//   before this one, one query tile per CTA with P through shared memory, 1.03 and 1.02 ms.  Head size 64, 3 x 1000 tokens, window 128: 30 us
-//   against 56 us of the mma.sync kernel.
-//   Tried and slower: signalling P in two 64-key halves with the row sum after the second (6 % slower: the sum no longer hides behind the
-//   exponentials); one query tile per CTA, 256 threads (18 % slower).
+//   about 2048 clocks; measured about 3100: the chain scores -> maximum (450) -> exponentials (1500) -> second half of P V and Q K^T (900) of a tile, with
+//   200 clocks for each hand-over.  One 8192-token prompt, 32 / 8 heads x 128: 0.44 ms alone (1.25 PFLOP/s).  Before: 0.495 ms; of that, 28 us from
+//   the MMA warp's code (fa_umma), 27 us from the halves of P, 7 us from the mixed-type sums (fa_add_bf16x2), 20 us from masks outside the tiles
+//   that need none.  3 x 1000 tokens of head size 64, window 128: 24 us, 30 before.
+//   Tried and slower: 64-key tiles with two score buffers per query tile (478 us: both tiles' softmax phases fall together, and a hand-over costs as
+//   much per 64 keys); sixteen softmax warps with half a row per thread (482 us); a share of the exponentials as polynomials on the FMA pipe (2 of 16: no
+//   gain, 4 of 16: 1 % slower: the fp32 pair operations cost more clocks than the exponentials they replace); the maximum beside the exponentials of
+//   the maximum before (493 us); four hand-overs of P (439 us).
 //   O and l are rescaled by the softmax warps themselves, decided per warp: S_j was issued after P V_{j-1}, so "S_j is complete" says that O
 //   is quiescent.  Contiguous rows of head size 128 move their maximum only when it grows by more than 2^8; the others move it at once, as the
 //   mma.sync kernels did that they ran on: then a row's largest probability is exactly 1 and takes no rounding (error against 64 bits of the mixed
@@ -32,6 +35,7 @@
 #include <cfloat>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 
 #include "api.h"
 #include "common.cuh"
@@ -41,7 +45,6 @@
 namespace nxdi {
 
 constexpr int FA_ROWS = 128;                   // queries per tile = keys per tile
-constexpr int FA_THREADS = 384;
 constexpr float FA_LOG2E = 1.4426950408889634f;
 
 struct FaParams {
@@ -97,16 +100,24 @@ __device__ __forceinline__ uint64_t fa_desc_mnmajor(const void* smem) {
 __host__ __device__ constexpr uint32_t fa_idesc(int n, bool b_mn_major) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn_major ? (1u << 16) : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
-__device__ __forceinline__ void fa_umma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-               "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
+// Called by a whole warp, issued by the lane whose `on` is 1: in code that all lanes run the descriptors stay in uniform registers.  (A branch
+// for one lane moves each of them there before every instruction: the issuing thread, not the tensor pipe, was what a key tile waited for.)
+__device__ __forceinline__ void fa_umma(uint32_t on, uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+               "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(on) : "memory");
 }
-__device__ __forceinline__ void fa_umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-               "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc) : "memory");
+__device__ __forceinline__ void fa_umma_ts(uint32_t on, uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+               "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc), "r"(on) : "memory");
 }
-__device__ __forceinline__ void fa_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar_s32(bar)) : "memory");
+__device__ __forceinline__ void fa_commit(uint32_t on, uint64_t* bar) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(mbar_s32(bar)),
+               "r"(on) : "memory");
+}
+__device__ __forceinline__ uint32_t fa_elect() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
 }
 __device__ __forceinline__ void fa_tmem_ld32(uint32_t taddr, uint32_t* v) {
   asm volatile(
@@ -161,6 +172,10 @@ __device__ __forceinline__ uint64_t fa_add2(uint64_t a, uint64_t b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+// s_lo, s_hi += the two bf16 halves of w
+__device__ __forceinline__ void fa_add_bf16x2(float& s_lo, float& s_hi, uint32_t w) {
+  asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.bf16 %0, l, %0;\n\tadd.rn.f32.bf16 %1, h, %1;\n\t}" : "+f"(s_lo), "+f"(s_hi) : "r"(w));
+}
 // tanh on |x| <= 1: x times a polynomial in x^2 (weighted least squares on Chebyshev nodes, relative error 1.7e-7 with fp32 arithmetic)
 __device__ __forceinline__ uint64_t fa_tanh2_small(uint64_t x) {
   const uint64_t u = fa_mul2(x, x);
@@ -174,31 +189,42 @@ __device__ __forceinline__ uint64_t fa_tanh2_small(uint64_t x) {
   return fa_mul2(x, r);
 }
 
-template <int D, bool PAGED, bool CAP>
-__global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(const __grid_constant__ FaParams p) {
-  constexpr int TILE = FA_ROWS * D * 2;                  // bytes of a [128][D] tile: D / 64 blocks of [128 rows][128 bytes]
+template <int D, int NX>
+struct FaShape {
+  static constexpr int THREADS = 128 * NX + 128;
+  static constexpr int TILE = FA_ROWS * D * 2;           // bytes of a [128][D] tile: D / 64 blocks of [128 rows][128 bytes]
+  static constexpr int SLOTS = NX == 2 ? (D == 128 ? 5 : 8) : D == 128 ? 2 : 5;     // K and V tiles share one ring: K0 V0 K1 V1 ...
+  static constexpr int SMEM = (NX + SLOTS) * TILE + 256 + 1024;                     // NX == 1: two CTAs per SM
+};
+
+// NX: query tiles of a CTA
+template <int D, int NX, bool PAGED, bool CAP>
+__global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_prefill_tc_kernel(const __grid_constant__ FaParams p) {
+  constexpr int TILE = FaShape<D, NX>::TILE, SLOTS = FaShape<D, NX>::SLOTS, THREADS = FaShape<D, NX>::THREADS;
   constexpr int HALF = FA_ROWS * 128;
-  constexpr int SLOTS = D == 128 ? 5 : 8;                // K and V tiles share one ring: K0 V0 K1 V1 ...
+  constexpr int W_MMA = 4 * NX, W_TMA = W_MMA + 1, W_CLEAN = W_MMA + 2;
+  constexpr uint32_t T_COLS = 256 * NX, T_OUT = 128 * NX;     // TMEM: S (and P) of every tile, then O
   constexpr float SLACK = D == 128 && !PAGED ? 8.f : 0.f; // log2 of what a row's largest probability may exceed 1 by
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   uint8_t* smem = smem_raw + ((1024u - (mbar_s32(smem_raw) & 1023u)) & 1023u);
-  uint8_t* sQ = smem;                                    // [2 tiles]; the outputs are staged here at the end
-  uint8_t* sKV = sQ + 2 * TILE;                          // [SLOTS]
+  uint8_t* sQ = smem;                                    // [NX]; the outputs are staged here at the end
+  uint8_t* sKV = sQ + NX * TILE;                         // [SLOTS]
   uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + SLOTS * TILE);
   uint64_t* q_full = bars;
   uint64_t* kv_full = bars + 1;                          // [SLOTS]
   uint64_t* kv_empty = kv_full + SLOTS;                  // [SLOTS]
   uint64_t* s_full = kv_empty + SLOTS;                   // [2] S_x complete (and P V of the tile before retired)
-  uint64_t* p_full = s_full + 2;                         // [2] P_x written and O_x rescaled: four warps arrive
+  uint64_t* p_half = s_full + 2;                         // [2] P_x of the first 64 keys written and O_x rescaled: four warps arrive
+  uint64_t* p_full = p_half + 2;                         // [2] the rest of P_x
   uint64_t* o_full = p_full + 2;                         // [2]
   uint64_t* v_landed = o_full + 2;                       // the last value tile is there
   uint64_t* v_clean = v_landed + 1;                      // its rows past the end are zeroed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_clean + 1);
   volatile int* stop = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  if (warp == 9 && lane == 0) {
+  if (warp == W_TMA && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_q) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_k) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_v) : "memory");
@@ -210,6 +236,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
     }
     for (int x = 0; x < 2; ++x) {
       mbar_init(&s_full[x], 1);
+      mbar_init(&p_half[x], 4);
       mbar_init(&p_full[x], 4);
       mbar_init(&o_full[x], 1);
     }
@@ -218,8 +245,8 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
     *stop = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 8) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(mbar_s32(tmem_slot)), "n"(512));
+  if (warp == W_MMA) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(mbar_s32(tmem_slot)), "n"(T_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -230,8 +257,9 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
   pdl_wait();               // from here on: what earlier kernels wrote
 
   // ---- which queries: heavy (late) tiles first
-  const int n_hp = p.pair_heads ? p.Hq / 2 : p.Hq;
-  const int span = p.pair_heads ? FA_ROWS : 2 * FA_ROWS;
+  const bool pair = NX == 2 && p.pair_heads;
+  const int n_hp = pair ? p.Hq / 2 : p.Hq;
+  const int span = pair ? FA_ROWS : NX * FA_ROWS;
   const int n_qt = (p.T + span - 1) / span;
   const int per_qt = p.B * n_hp;
   const int qt = n_qt - 1 - (int)(blockIdx.x / per_qt);
@@ -239,15 +267,15 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
   const int q0 = qt * span;
   const int qn = PAGED ? min(p.q_len[b], p.T) : p.T, ctx = PAGED ? p.ctx_len[b] : 0;
   if (PAGED && q0 >= qn) {                               // padding queries: zeros
-    const int rows = min(span, p.T - q0), heads = p.pair_heads ? 2 : 1, h0 = hp * heads;
-    for (int i = threadIdx.x; i < rows * heads * (D / 8); i += FA_THREADS) {
+    const int rows = min(span, p.T - q0), heads = pair ? 2 : 1, h0 = hp * heads;
+    for (int i = threadIdx.x; i < rows * heads * (D / 8); i += THREADS) {
       const int r = i / (heads * (D / 8)), c = i % (heads * (D / 8));
       *reinterpret_cast<uint4*>(p.out + (((long long)b * p.T + q0 + r) * p.Hq + h0) * D + c * 8) = make_uint4(0u, 0u, 0u, 0u);
     }
-    if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512));
+    if (warp == W_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(T_COLS));
     return;
   }
-  const int h_first = p.pair_heads ? 2 * hp : hp, hk = h_first / (p.Hq / p.Hkv);
+  const int h_first = pair ? 2 * hp : hp, hk = h_first / (p.Hq / p.Hkv);
   // ---- which keys: the kept first tokens below the window's reach (whole tiles), then [lo, hi]
   const int p_first = ctx + q0, p_last = ctx + min(q0 + span, qn) - 1;
   const int hi = p.causal ? p_last : qn - 1, end = hi + 1;
@@ -258,10 +286,11 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
   auto key_at = [&](int i) { return (i < nA ? i : t_lo + i - nA) * FA_ROWS; };
   const bool dirty_end = PAGED && (end & (FA_ROWS - 1)) != 0;
 
-  if (warp >= 8) {
-    // registers: 384 threads x 168 at launch = 256 x 208 + 128 x 88
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-    if (warp == 9) {
+  if (warp >= W_MMA) {
+    // registers: 384 threads x 168 at launch = 256 x 208 + 128 x 88; 256 x 128 = 128 x 200 + 128 x 56
+    if constexpr (NX == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if (warp == W_TMA) {
       // ================= TMA producer =================
       const int pieces = PAGED ? max(1, FA_ROWS >> p.page_shift) : 1;    // boxes per 64-column block
       const int piece_rows = FA_ROWS / pieces;
@@ -273,10 +302,10 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
         return (table[pi] << p.page_shift) + (k & ((1 << p.page_shift) - 1));
       };
       if (lane == 0) {
-        mbar_expect(q_full, 2 * TILE);
-        for (int x = 0; x < 2; ++x)
+        mbar_expect(q_full, NX * TILE);
+        for (int x = 0; x < NX; ++x)
           for (int c = 0; c < D / 64; ++c)
-            fa_tma_4d(sQ + x * TILE + c * HALF, &p.tm_q, c * 64, p.pair_heads ? h_first + x : h_first, p.pair_heads ? q0 : q0 + x * FA_ROWS, b, q_full);
+            fa_tma_4d(sQ + x * TILE + c * HALF, &p.tm_q, c * 64, pair ? h_first + x : h_first, pair ? q0 : q0 + x * FA_ROWS, b, q_full);
       }
       int next = slot_at(key_at(0));
       bool go = true;
@@ -302,59 +331,76 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
           }
         }
       }
-    } else if (warp == 8) {
+    } else if (warp == W_MMA) {
       // ================= MMA issuer =================
-      if (lane == 0) {
-        constexpr uint32_t idesc_qk = fa_idesc(128, false), idesc_pv = fa_idesc(D, true);
-        auto issue_s = [&](int x, int i) {               // S_x = Q_x K_i^T
-          const uint8_t* k = sKV + ((2 * i) % SLOTS) * TILE;
-#pragma unroll
-          for (int c = 0; c < D / 16; ++c) {
-            // 16 d = 32 bytes inside the 128-byte swizzle atom; the second 64-d half is a separate 16 KB block
-            const uint64_t da = fa_desc_kmajor(sQ + x * TILE + (c >> 2) * HALF) + (uint64_t)((c & 3) * 2);
-            const uint64_t db = fa_desc_kmajor(k + (c >> 2) * HALF) + (uint64_t)((c & 3) * 2);
-            fa_umma(tmem + 128 * x, da, db, idesc_qk, c != 0 ? 1u : 0u);
-          }
-          fa_commit(&s_full[x]);
-        };
-        auto full = [&](int it) { return mbar_wait(&kv_full[it % SLOTS], (uint32_t)((it / SLOTS) & 1), stop, p.wait_word); };
-        bool go = mbar_wait(q_full, 0, stop, p.wait_word) && full(0);
-        if (go) {
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          issue_s(0, 0);
-          issue_s(1, 0);
-          fa_commit(&kv_empty[0]);
+      constexpr uint32_t idesc_qk = fa_idesc(128, false), idesc_pv = fa_idesc(D, true);
+      const uint32_t on = fa_elect();
+      const uint64_t dq0 = fa_desc_kmajor(sQ), dk0 = fa_desc_kmajor(sKV), dv0 = fa_desc_mnmajor(sKV);
+      int slot = 0;                                      // the ring's next tile
+      uint32_t par = 0;
+      auto full = [&] { return mbar_wait_warp(&kv_full[slot], par, stop, p.wait_word); };
+      auto pop = [&] {
+        if (++slot == SLOTS) {
+          slot = 0;
+          par ^= 1u;
         }
-        for (int i = 0; i < n_tiles && go; ++i) {
-          const bool more = i + 1 < n_tiles;
-          go = full(2 * i + 1);
-          if (go && dirty_end && !more) {
-            mbar_arrive(v_landed);
-            go = mbar_wait(v_clean, 0, stop, p.wait_word);
-          }
-          for (int x = 0; x < 2 && go; ++x) {
-            go = mbar_wait(&p_full[x], (uint32_t)(i & 1), stop, p.wait_word);       // P_x in TMEM, O_x rescaled, S_x fully read
+      };
+      auto issue_s = [&](int x) {                        // S_x = Q_x K^T with the keys at `slot`
+        const uint64_t dq = dq0 + (uint64_t)(x * (TILE >> 4)), dk = dk0 + (uint64_t)(slot * (TILE >> 4));
+#pragma unroll
+        for (int c = 0; c < D / 16; ++c) {
+          // 16 d = 32 bytes inside the 128-byte swizzle atom; the second 64-d half is a separate 16 KB block
+          const uint64_t off = (uint64_t)((c >> 2) * (HALF >> 4) + (c & 3) * 2);
+          fa_umma(on, tmem + 128 * x, dq + off, dk + off, idesc_qk, c != 0 ? 1u : 0u);
+        }
+        fa_commit(on, &s_full[x]);
+        if (x == NX - 1) fa_commit(on, &kv_empty[slot]);
+      };
+      bool go = mbar_wait_warp(q_full, 0, stop, p.wait_word) && full();
+      if (go) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int x = 0; x < NX; ++x) issue_s(x);
+        pop();
+      }
+      for (int i = 0; i < n_tiles && go; ++i) {
+        const bool more = i + 1 < n_tiles;
+        go = full();
+        const int sv = slot;
+        pop();
+        if (go && dirty_end && !more) {
+          if (lane == 0) mbar_arrive(v_landed);
+          go = mbar_wait_warp(v_clean, 0, stop, p.wait_word);
+        }
+        const uint64_t dv = dv0 + (uint64_t)(sv * (TILE >> 4));
+#pragma unroll
+        for (int x = 0; x < NX; ++x) {
+          // O_x += P_x V: A = P: 16 keys = 8 TMEM columns; B = V (MN-major): 16 keys = 16 rows of 128 bytes further in all blocks
+          if (go) go = mbar_wait_warp(&p_half[x], (uint32_t)(i & 1), stop, p.wait_word);       // first half of P_x in TMEM, O_x rescaled, S_x fully read
+          if (!go) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+          for (int c = 0; c < FA_ROWS / 32; ++c)
+            fa_umma_ts(on, tmem + T_OUT + 128 * x, tmem + 128 * x + 8 * c, dv + (uint64_t)(c * 128), idesc_pv, (i | c) != 0 ? 1u : 0u);
+          go = mbar_wait_warp(&p_full[x], (uint32_t)(i & 1), stop, p.wait_word);
+          if (!go) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+          for (int c = FA_ROWS / 32; c < FA_ROWS / 16; ++c)
+            fa_umma_ts(on, tmem + T_OUT + 128 * x, tmem + 128 * x + 8 * c, dv + (uint64_t)(c * 128), idesc_pv, 1u);
+          if (x == NX - 1) fa_commit(on, &kv_empty[sv]);
+          if (more) {
+            if (x == 0) go = full();
             if (!go) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint8_t* v = sKV + ((2 * i + 1) % SLOTS) * TILE;
-#pragma unroll
-            for (int c = 0; c < FA_ROWS / 16; ++c)
-              // A = P: 16 keys = 8 TMEM columns; B = V (MN-major): 16 keys = 16 rows of 128 bytes further in all blocks
-              fa_umma_ts(tmem + 256 + 128 * x, tmem + 128 * x + 8 * c, fa_desc_mnmajor(v + c * 2048), idesc_pv, (i | c) != 0 ? 1u : 0u);
-            if (x == 1) fa_commit(&kv_empty[(2 * i + 1) % SLOTS]);
-            if (more) {
-              if (x == 0) go = full(2 * i + 2);
-              if (!go) break;
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              issue_s(x, i + 1);
-              if (x == 1) fa_commit(&kv_empty[(2 * i + 2) % SLOTS]);
-            } else {
-              fa_commit(&o_full[x]);
-            }
+            issue_s(x);
+            if (x == NX - 1) pop();
+          } else {
+            fa_commit(on, &o_full[x]);
           }
         }
       }
-    } else if (warp == 10 && dirty_end) {
+    } else if (warp == W_CLEAN && dirty_end) {
       // ================= value rows past the last key of the last tile =================
       const int valid = end - key_at(n_tiles - 1);
       if (mbar_wait_warp(v_landed, 0, stop, p.wait_word)) {
@@ -369,55 +415,69 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
     }
   } else {
     // ================= softmax / rescale / epilogue: one query row per thread =================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    if constexpr (NX == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    else asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
     const int x = warp >> 2, qd = warp & 3;
     const int r = qd * 32 + lane;                        // row inside the tile = TMEM lane
-    const int t_tile = p.pair_heads ? q0 : q0 + x * FA_ROWS;
-    const int h = p.pair_heads ? h_first + x : h_first;
+    const int t_tile = pair ? q0 : q0 + x * FA_ROWS;
+    const int h = pair ? h_first + x : h_first;
     const int t = t_tile + r, pos = ctx + t;             // token of the batch row, position in the sequence
     const uint32_t lanes = (uint32_t)(qd * 32) << 16;
-    const uint32_t tS = tmem + 128 * x + lanes, tO = tmem + 256 + 128 * x + lanes;
+    const uint32_t tS = tmem + 128 * x + lanes, tO = tmem + T_OUT + 128 * x + lanes;
     const int up = p.causal ? min(pos, end - 1) : end - 1;
-    const int lb = p.window > 0 ? pos - p.window + 1 : p.chunk > 0 ? pos / p.chunk * p.chunk : 0;
-    // tile-uniform bounds of the mask test: every row sees [lb_max, up_min]
-    const int up_min = p.causal ? min(ctx + t_tile, end - 1) : end - 1;
-    const int lb_max = p.window > 0 ? ctx + t_tile + FA_ROWS - p.window : p.chunk > 0 ? (ctx + t_tile + FA_ROWS - 1) / p.chunk * p.chunk : 0;
+    auto reach = [&](int at) { return p.window > 0 ? at - p.window + 1 : p.chunk > 0 ? at / p.chunk * p.chunk : 0; };
+    const int lb = reach(pos);                           // a row sees [lb, up] and the first `keep` keys
+    // bounds over the rows of this warp
+    const int w_pos = ctx + t_tile + 32 * qd;
+    const int up_min = p.causal ? min(w_pos, end - 1) : end - 1, up_max = p.causal ? min(w_pos + 31, end - 1) : end - 1;
+    const int lb_min = reach(w_pos), lb_max = reach(w_pos + 31);
     const float hs = p.head_scale ? p.scale * p.head_scale[h] : p.scale;
     float m_run = -INFINITY, l_run = 0.f;
-    for (int i = 0; i < n_tiles; ++i) {
-      const int key0 = key_at(i);
-      if (!mbar_wait_warp(&s_full[x], (uint32_t)(i & 1), stop, p.wait_word)) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    auto tile = [&](auto masked, int i, int key0) {
+      constexpr bool MASKED = decltype(masked)::value;
       uint32_t v[128];
 #pragma unroll
       for (int c = 0; c < 4; ++c) fa_tmem_ld32(tS + 32 * c, v + 32 * c);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       float scl = hs * FA_LOG2E;                         // scores -> log2 domain
+      // halves of 64 keys that no row of the warp sees: probability 0 without looking at the scores
+      bool dead[2] = {false, false};
+      if constexpr (MASKED) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int k0 = key0 + 64 * c;
+          dead[c] = k0 > up_max || (k0 + 63 < lb_min && k0 >= keep);
+        }
+      }
       if (CAP) {
         const float to_cap = hs / p.softcap;
-        float big = 0.f;
-#pragma unroll
-        for (int e = 0; e < 128; ++e) big = fmaxf(big, fabsf(__uint_as_float(v[e])));
         const uint64_t tc2 = fa_pack2(to_cap, to_cap);
-        // the maximum is taken over scores that the row does not see too (later keys, rows of pages that were not fetched, whatever shared memory
-        // held): both ways give a score the same bits
-        if (!__any_sync(0xffffffffu, !(big * fabsf(to_cap) <= 1.f))) {
 #pragma unroll
-          for (int e = 0; e < 128; e += 2) {
-            float a, c;
-            fa_unpack2(fa_tanh2_small(fa_mul2(fa_pack2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), tc2)), a, c);
-            v[e] = __float_as_uint(a);
-            v[e + 1] = __float_as_uint(c);
-          }
-        } else {
+        for (int c0 = 0; c0 < 128; c0 += 64) {
+          if (dead[c0 >> 6]) continue;
+          float big = 0.f;
 #pragma unroll
-          for (int e = 0; e < 128; e += 2) {
-            const uint64_t x2 = fa_mul2(fa_pack2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), tc2);
-            float x, y, a, c;
-            fa_unpack2(x2, x, y);
-            fa_unpack2(fa_tanh2_small(x2), a, c);
-            v[e] = __float_as_uint(fabsf(x) <= 1.f ? a : tanhf(x));
-            v[e + 1] = __float_as_uint(fabsf(y) <= 1.f ? c : tanhf(y));
+          for (int e = c0; e < c0 + 64; ++e) big = fmaxf(big, fabsf(__uint_as_float(v[e])));
+          // the maximum is taken over scores that the row does not see too (later keys, rows of pages that were not fetched, whatever shared memory
+          // held): both ways give a score the same bits
+          if (!__any_sync(0xffffffffu, !(big * fabsf(to_cap) <= 1.f))) {
+#pragma unroll
+            for (int e = c0; e < c0 + 64; e += 2) {
+              float a, c;
+              fa_unpack2(fa_tanh2_small(fa_mul2(fa_pack2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), tc2)), a, c);
+              v[e] = __float_as_uint(a);
+              v[e + 1] = __float_as_uint(c);
+            }
+          } else {
+#pragma unroll
+            for (int e = c0; e < c0 + 64; e += 2) {
+              const uint64_t x2 = fa_mul2(fa_pack2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), tc2);
+              float x, y, a, c;
+              fa_unpack2(x2, x, y);
+              fa_unpack2(fa_tanh2_small(x2), a, c);
+              v[e] = __float_as_uint(fabsf(x) <= 1.f ? a : tanhf(x));
+              v[e + 1] = __float_as_uint(fabsf(y) <= 1.f ? c : tanhf(y));
+            }
           }
         }
         scl = p.softcap * FA_LOG2E;
@@ -426,85 +486,99 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
         for (int e = 0; e < 128; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * scl);
         scl = 1.f;
       }
-      // masks only where a tile can contain invisible keys: uniform tests of its two ends
-      const bool above = key0 + FA_ROWS - 1 > up_min, below = key0 < lb_max && key0 + FA_ROWS > keep;
-      if (above || below) {
-        const int e_hi = up - key0, e_lo = lb - key0, e_keep = keep - key0;
-        if (!below) {
+      if constexpr (MASKED) {
+      // masks only where 32 keys are visible to some rows of the warp and not to others (a tile on the diagonal: one of four)
 #pragma unroll
-          for (int e = 0; e < 128; ++e)
-            if (e > e_hi) v[e] = 0xff800000u;            // -inf
-        } else {
+      for (int c = 0; c < 4; ++c) {
+        const int k0 = key0 + 32 * c;
+        if (!(k0 + 31 <= up_min && (k0 >= lb_max || k0 + 31 < keep)) && !dead[c >> 1]) {
+          const int e_hi = up - k0, e_lo = lb - k0, e_keep = keep - k0;
+          const uint32_t m_hi = e_hi >= 31 ? ~0u : e_hi < 0 ? 0u : (2u << e_hi) - 1u;
+          const uint32_t m_lo = e_lo <= 0 ? ~0u : e_lo > 31 ? 0u : ~0u << e_lo;
+          const uint32_t m_keep = e_keep > 31 ? ~0u : e_keep <= 0 ? 0u : (1u << e_keep) - 1u;
+          const uint32_t see = m_hi & (m_lo | m_keep);
 #pragma unroll
-          for (int e = 0; e < 128; ++e)
-            if (!(e <= e_hi && (e >= e_lo || e < e_keep))) v[e] = 0xff800000u;
+          for (int e = 0; e < 32; ++e)
+            if (!(see & (1u << e))) v[32 * c + e] = 0xff800000u;      // -inf
         }
+      }
       }
       // row maximum in the domain of v (its scale is positive), four independent chains
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int e = 0; e < 128; e += 8)
+      for (int c0 = 0; c0 < 128; c0 += 64) {
+        if (dead[c0 >> 6]) continue;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) mx4[c] = fmaxf(mx4[c], fmaxf(__uint_as_float(v[e + 2 * c]), __uint_as_float(v[e + 2 * c + 1])));
+        for (int e = c0; e < c0 + 64; e += 8)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) mx4[c] = fmaxf(mx4[c], fmaxf(__uint_as_float(v[e + 2 * c]), __uint_as_float(v[e + 2 * c + 1])));
+      }
       const float mx_raw = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       const float mx = (mx_raw == -INFINITY) ? -INFINITY : mx_raw * scl;
       const bool grow = mx > m_run + SLACK || (m_run == -INFINITY && mx > -INFINITY);
       const float m_new = grow ? mx : m_run;
       const float alpha = (m_run == -INFINITY) ? 0.f : fa_ex2(m_run - m_new);
       const bool move = i > 0 && __any_sync(0xffffffffu, grow);
-      if (SLACK > 0.f && move) {                         // seldom: in few registers, beside the scores
-#pragma unroll 1
-        for (int c0 = 0; c0 < D; c0 += 32) {
-          uint32_t o[32];
-          fa_tmem_ld32(tO + c0, o);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-          fa_tmem_st32(tO + c0, o);
-        }
-      }
       l_run *= alpha;
       m_run = m_new;
-      // ---- P = exp2(v * scl - m) -> bf16 -> TMEM, over the scores
+      // O = alpha O: P V of the tile before has retired
+      auto rescale = [&](auto cols) {
+        constexpr int C = decltype(cols)::value;
+#pragma unroll 1
+        for (int c0 = 0; c0 < D; c0 += C) {
+          uint32_t o[C];
+#pragma unroll
+          for (int c = 0; c < C; c += 32) fa_tmem_ld32(tO + c0 + c, o + c);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int e = 0; e < C; e += 2) {
+            float a, d;
+            fa_unpack2(fa_mul2(fa_pack2(__uint_as_float(o[e]), __uint_as_float(o[e + 1])), fa_pack2(alpha, alpha)), a, d);
+            o[e] = __float_as_uint(a);
+            o[e + 1] = __float_as_uint(d);
+          }
+#pragma unroll
+          for (int c = 0; c < C; c += 32) fa_tmem_st32(tO + c0 + c, o + c);
+        }
+      };
+      if (SLACK > 0.f && move) rescale(std::integral_constant<int, 32>{});       // seldom: in few registers, beside the scores
+      // ---- P = exp2(v * scl - m) -> bf16 -> TMEM, over the scores, 64 keys at a time: their P V runs while the next are exponentiated
       const float neg_m = (m_run == -INFINITY) ? 0.f : -m_run;
       const uint64_t scl2 = fa_pack2(scl, scl), neg2 = fa_pack2(neg_m, neg_m);
-      uint64_t ls[2] = {0ull, 0ull};
+      float ls[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t pk[32];
+        if (dead[c]) {
 #pragma unroll
-        for (int e = 0; e < 64; e += 2) {
-          float a, bb;
-          fa_unpack2(fa_fma2(fa_pack2(__uint_as_float(v[64 * c + e]), __uint_as_float(v[64 * c + e + 1])), scl2, neg2), a, bb);
-          const uint32_t w = pack_bf16(fa_ex2(a), fa_ex2(bb));            // -inf -> 0
-          // the sum uses the bf16-rounded probabilities, exactly what the tensor core multiplies
-          ls[(e >> 1) & 1] = fa_add2(ls[(e >> 1) & 1], fa_pack2(bf16lo(w), bf16hi(w)));
-          pk[e >> 1] = w;
+          for (int e = 0; e < 32; ++e) pk[e] = 0u;
+        } else {
+#pragma unroll
+          for (int e = 0; e < 64; e += 2) {
+            float a, bb;
+            fa_unpack2(fa_fma2(fa_pack2(__uint_as_float(v[64 * c + e]), __uint_as_float(v[64 * c + e + 1])), scl2, neg2), a, bb);
+            const uint32_t w = pack_bf16(fa_ex2(a), fa_ex2(bb));          // -inf -> 0
+            // the sum uses the bf16-rounded probabilities, exactly what the tensor core multiplies
+            fa_add_bf16x2(ls[e & 2], ls[(e & 2) + 1], w);
+            pk[e >> 1] = w;
+          }
         }
         fa_tmem_st32(tS + 32 * c, pk);
+        if (SLACK == 0.f && c == 0 && move) rescale(std::integral_constant<int, 64>{});      // often: in the registers of the first scores
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(c == 0 ? &p_half[x] : &p_full[x]);
       }
-      if (SLACK == 0.f && move) {                        // often: once the scores' registers are free, all of O in flight at once
-        uint32_t o[D];
-#pragma unroll
-        for (int c = 0; c < D; c += 32) fa_tmem_ld32(tO + c, o + c);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-        for (int e = 0; e < D; e += 2) {
-          float a, c;
-          fa_unpack2(fa_mul2(fa_pack2(__uint_as_float(o[e]), __uint_as_float(o[e + 1])), fa_pack2(alpha, alpha)), a, c);
-          o[e] = __float_as_uint(a);
-          o[e + 1] = __float_as_uint(c);
-        }
-#pragma unroll
-        for (int c = 0; c < D; c += 32) fa_tmem_st32(tO + c, o + c);
-      }
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[x]);
-      float s0, s1;
-      fa_unpack2(fa_add2(ls[0], ls[1]), s0, s1);
-      l_run += s0 + s1;
+      l_run += (ls[0] + ls[1]) + (ls[2] + ls[3]);
+    };
+    for (int i = 0; i < n_tiles; ++i) {
+      const int key0 = key_at(i);
+      if (!mbar_wait_warp(&s_full[x], (uint32_t)(i & 1), stop, p.wait_word)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // masks only in a tile that has keys which some row of the warp does not see
+      if (key0 + FA_ROWS - 1 <= up_min && (key0 >= lb_max || key0 + FA_ROWS <= keep)) tile(std::false_type{}, i, key0);
+      else tile(std::true_type{}, i, key0);
     }
     // ---- epilogue: O / l (times the gate) -> bf16 -> shared memory -> TMA store (rows past T are clipped, padding rows are zeros)
     const bool done = mbar_wait_warp(&o_full[x], 0, stop, p.wait_word);
@@ -558,9 +632,9 @@ __global__ void __launch_bounds__(FA_THREADS, 1) attention_prefill_tc_kernel(con
   }
   if (*stop) __nanosleep(1000000);        // gave up: let copies in flight land before the shared memory goes away
   __syncthreads();
-  if (warp == 8) {
+  if (warp == W_MMA) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(T_COLS));
   }
 }
 
@@ -592,21 +666,34 @@ static void fa_map_rows(CUtensorMap* tm, const void* ptr, int B, int T, int H, i
   fa_make_map(tm, ptr, 4, dims, strides, FA_ROWS);
 }
 
-template <int D, bool PAGED, bool CAP>
-static void fa_go(FaParams& p, cudaStream_t stream) {
-  constexpr int TILE = FA_ROWS * D * 2, SLOTS = D == 128 ? 5 : 8;
-  const size_t smem = (size_t)(2 + SLOTS) * TILE + 256 + 1024;
-  auto kernel = attention_prefill_tc_kernel<D, PAGED, CAP>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+template <int D, int NX, bool PAGED, bool CAP>
+static void fa_run(FaParams& p, cudaStream_t stream) {
+  using Shape = FaShape<D, NX>;
+  auto kernel = attention_prefill_tc_kernel<D, NX, PAGED, CAP>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM) != cudaSuccess)
     throw std::runtime_error("attention (tensor cores): shared memory size refused");
   check_waits();
   p.wait_word = wait_word(WAIT_ATTENTION);
   count_launch(COUNT_ATTENTION);
   // grouped heads share their keys two by two; a head of its own takes 256 queries instead
   p.pair_heads = (p.Hq / p.Hkv) % 2 == 0 ? 1 : 0;
-  const int span = p.pair_heads ? FA_ROWS : 2 * FA_ROWS;
-  const long long blocks = (long long)((p.T + span - 1) / span) * p.B * (p.pair_heads ? p.Hq / 2 : p.Hq);
-  launch_pdl(kernel, dim3((unsigned)blocks), dim3(FA_THREADS), smem, stream, p);
+  const bool pair = NX == 2 && p.pair_heads;
+  const int span = pair ? FA_ROWS : NX * FA_ROWS;
+  const long long blocks = (long long)((p.T + span - 1) / span) * p.B * (pair ? p.Hq / 2 : p.Hq);
+  launch_pdl(kernel, dim3((unsigned)blocks), dim3(Shape::THREADS), Shape::SMEM, stream, p);
+}
+// One query tile per CTA and two CTAs per SM where a tile reads few keys (a CTA's first loads, its epilogue and its masks then overlap the other's
+// work), or where pairs of tiles would not fill the SMs; two tiles per CTA, which share the keys they load, for long rows.  us, two tiles / one, 32 / 8
+// heads x 128, causal: 512 tokens 15.0 / 13.3, 4 x 1024 57.4 / 53.1, 2048 41.3 / 42.4, 8192 444 / 481; 2 x 3000 with a window of 128 67.8 / 59.9, 8192 with
+// 1024 161 / 160; 8 / 1 heads, 4096: 63.1 / 58.4 (128 CTAs of two tiles).  Head size 64: 13.1 / 11.5, 48.0 / 45.2, 36.5 / 38.3; 49.5 / 43.7, 143 / 138.
+template <int D, bool PAGED, bool CAP>
+static void fa_go(FaParams& p, long long keys, cudaStream_t stream) {
+  if (p.window > 0) keys = std::min(keys, (long long)p.window + p.keep + FA_ROWS);
+  else if (p.chunk > 0) keys = std::min(keys, (long long)p.chunk + FA_ROWS);
+  const bool pair = (p.Hq / p.Hkv) % 2 == 0;
+  const long long blocks = pair ? (long long)((p.T + FA_ROWS - 1) / FA_ROWS) * p.B * (p.Hq / 2) : (long long)((p.T + 2 * FA_ROWS - 1) / (2 * FA_ROWS)) * p.B * p.Hq;
+  if (keys <= 9 * FA_ROWS || blocks < kNumSMs) fa_run<D, 1, PAGED, CAP>(p, stream);
+  else fa_run<D, 2, PAGED, CAP>(p, stream);
 }
 
 // q [B,T,Hq,D], k / v [B,T,Hkv,D] bf16 contiguous, D = 128, or 64 without a soft cap -> out [B,T,Hq,D]
@@ -622,9 +709,9 @@ void attention_prefill_tc_launch(const void* q, const void* k, const void* v, vo
   p.sinks = sinks;
   p.B = B; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal; p.window = window;
   p.scale = scale; p.softcap = softcap;
-  if (D == 128 && softcap > 0.f) fa_go<128, false, true>(p, stream);
-  else if (D == 128) fa_go<128, false, false>(p, stream);
-  else if (D == 64 && softcap <= 0.f) fa_go<64, false, false>(p, stream);
+  if (D == 128 && softcap > 0.f) fa_go<128, false, true>(p, T, stream);
+  else if (D == 128) fa_go<128, false, false>(p, T, stream);
+  else if (D == 64 && softcap <= 0.f) fa_go<64, false, false>(p, T, stream);
   else throw std::runtime_error("attention (tensor cores): head size 128, or 64 without a soft cap");
 }
 
@@ -652,8 +739,9 @@ void paged_attention_tc_launch(const WindowAttnParams& w, long long slots, cudaS
   p.B = w.B; p.T = w.T; p.Hq = w.Hq; p.Hkv = w.G; p.causal = 1; p.window = w.window; p.keep = w.keep_first; p.chunk = w.chunk;
   p.scale = w.scale; p.softcap = w.softcap;
   const bool cap = w.softcap > 0.f;
-  if (w.D == 128) { if (cap) fa_go<128, true, true>(p, stream); else fa_go<128, true, false>(p, stream); }
-  else { if (cap) fa_go<64, true, true>(p, stream); else fa_go<64, true, false>(p, stream); }
+  const long long keys = (long long)w.max_blocks * w.page;       // contexts are known on the device alone
+  if (w.D == 128) { if (cap) fa_go<128, true, true>(p, keys, stream); else fa_go<128, true, false>(p, keys, stream); }
+  else { if (cap) fa_go<64, true, true>(p, keys, stream); else fa_go<64, true, false>(p, keys, stream); }
 }
 
 }  // namespace nxdi

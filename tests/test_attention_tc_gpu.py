@@ -96,3 +96,27 @@ def test_soft_cap_does_not_depend_on_unseen_keys(D):
         got = ops.paged_window_attention(qq, kk, v, table, ctx, n, D ** -0.5, 30.0, 0, 0)
         assert want is None or torch.equal(got, want)
         want = got
+
+
+# rows of more than 1152 keys and at least 148 CTAs take two query tiles per CTA: one tile more or less than that, whole and odd lengths, heads in pairs
+# and alone; the bound above
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,T,Hq,Hkv,window,causal,sinks", [
+    (1, 1152, 34, 17, 0, True, False), (1, 1153, 32, 8, 0, True, True), (1, 1281, 30, 30, 0, True, False), (2, 1290, 16, 4, 1025, True, True),
+    (2, 1290, 16, 4, 1024, True, False), (1, 1217, 32, 16, 0, False, False), (2, 1408, 15, 5, 0, False, True)])
+def test_two_tiles(D, B, T, Hq, Hkv, window, causal, sinks):
+    test_contiguous(D, B, T, Hq, Hkv, window, causal, sinks)
+
+
+@pytest.mark.parametrize("D,cap", [(64, 20.0), (128, 20.0), (64, None), (128, None)])
+@pytest.mark.parametrize("Hq,G", [(16, 4), (17, 17)])
+@pytest.mark.parametrize("mask", [dict(), dict(window=1300, keep=70), dict(window=200, keep=4), dict(chunk=1200)])
+def test_two_tiles_paged(D, cap, Hq, G, mask):
+    ctx, n = (0, 1517, 130, 64, 1000), (300, 16, 0, 257, 290)
+    q, dirty, clean, table, c, m = _paged(5, 300, Hq, G, D, 64, ctx, n)
+    args = (table, c, m, D ** -0.5, cap, mask.get("window", 0), mask.get("keep", 0))
+    got = ops.paged_window_attention(q, *dirty, *args, chunk=mask.get("chunk"))
+    want = ref.paged_window_attention(q.float(), *(t.float() for t in clean), *args, chunk=mask.get("chunk"))
+    assert _rel(got, want) < 4e-3
+    for b, live in enumerate(n):
+        assert not got[b, live:].any()
