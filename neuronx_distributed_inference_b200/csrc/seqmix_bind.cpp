@@ -227,15 +227,21 @@ at::Tensor ssd_scan(const at::Tensor& xBC, const at::Tensor& dt_raw, const at::T
   TORCH_CHECK(state.dim() == 4 && state.size(1) == nh && state.size(2) == N && state.size(3) == P, "ssd_scan: state [lines, heads, N, head_dim]");
   check_i32(lines, B, "lines"); check_i32(ctx, B, "ctx_len"); check_i32(qlen, B, "q_len");
   c10::cuda::CUDAGuard guard(xBC.device());
-  auto y = at::zeros({B, T, inner}, xBC.options());
   SsdScanParams a{};
   a.xBC = xBC.data_ptr<float>(); a.dt_raw = dt_raw.data_ptr(); a.z = z.data_ptr();
   a.dt_sb = dt_raw.stride(0); a.dt_st = dt_raw.stride(1); a.z_sb = z.stride(0); a.z_st = z.stride(1);
   a.A_log = A_log.data_ptr<float>(); a.dt_bias = dt_bias.data_ptr<float>(); a.D_skip = D_skip.data_ptr<float>();
   a.state = state.data_ptr<float>(); a.lines = lines.data_ptr<int>(); a.ctx_len = ctx.data_ptr<int>(); a.q_len = qlen.data_ptr<int>();
-  a.y = y.data_ptr<float>();
   a.B = (int)B; a.T = (int)T; a.nh = (int)nh; a.P = (int)P; a.N = (int)N; a.G = (int)G;
-  ssd_scan_launch(a, is_lp(dt_raw), stream());
+  const bool chunked = B > 0 && ssd_chunk_supported(a);
+  auto y = chunked ? at::empty({B, T, inner}, xBC.options()) : at::zeros({B, T, inner}, xBC.options());
+  a.y = y.data_ptr<float>();
+  if (chunked) {
+    auto ws = at::empty({ssd_chunk_workspace(a)}, xBC.options().dtype(at::kByte));
+    ssd_chunk_launch(a, ws.data_ptr(), is_lp(dt_raw), stream());
+  } else {
+    ssd_scan_launch(a, is_lp(dt_raw), stream());
+  }
   return y;
 }
 

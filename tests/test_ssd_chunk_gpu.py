@@ -1,0 +1,67 @@
+"""Mamba-2 scan in chunks on tensor cores (csrc/ssd_chunk.cu) at the edges of its chunks, against the definition in 64 bits.
+
+Bound: all operands carry at least 24 bits (three bf16 parts), sums are fp32.  A term of an output passes about 8 roundings as in the step-by-step kernel, a
+sum of 128 terms in the tensor core's fp32 accumulator adds 8 more that all go towards zero: 16 * 2^-24 = 1e-6 of the sizes of the terms.  The state does
+not cancel: 1e-6 of its norm."""
+import pytest
+import torch
+
+from neuronx_distributed_inference_b200 import ops
+from tests.test_ssd_pair_gpu import _definition
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(nh, G, T, lens, dtype):
+    B, P, N = len(lens), 64, 128
+    inner = nh * P
+    xbc = torch.randn(B, T, inner + 2 * G * N, device="cuda")
+    wide = torch.randn(B, T, inner + nh + 5, device="cuda", dtype=dtype)          # strided views of one projection
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")             # noqa: E731
+    return dict(xBC=xbc, dt_raw=wide[..., inner:inner + nh], z=wide[..., :inner], A_log=torch.rand(nh, device="cuda") * 3, dt_bias=torch.randn(nh, device="cuda") - 1,
+                D_skip=torch.randn(nh, device="cuda"), state=torch.randn(B + 2, nh, N, P, device="cuda"), slots=i32([3, 0, 1, 2][:B]), ctx_len=i32([5, 0, 7, 1][:B]),
+                q_len=i32(lens)), (nh, P, N, G)
+
+
+def _run(args, sizes):
+    before = dict(ops.kernel_launches())["ssd_chunk"]
+    y = ops.ssd_scan(*args.values(), *sizes)
+    assert dict(ops.kernel_launches())["ssd_chunk"] == before + 1
+    torch.cuda.synchronize()
+    ops.check_waits()
+    return y
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("nh,G", [(2, 1), (4, 2), (8, 1)])
+@pytest.mark.parametrize("T,lens", [(48, (48, 1, 0)), (64, (64, 63)), (65, (65, 64, 2)), (300, (300, 129, 0, 191)), (1000, (1000, 128))])
+def test_scan(nh, G, T, lens, dtype):
+    args, sizes = _inputs(nh, G, T, lens, dtype)
+    want_state = args["state"].clone()
+    want, size = _definition(*(dict(args, state=want_state)).values(), *sizes)
+    got = _run(args, sizes)
+    for b, live in enumerate(lens):
+        if live:
+            assert ((got[b, :live].double() - want[b, :live]).norm() / size[b, :live].norm()).item() < 1e-6
+        assert not got[b, live:].any()
+    assert ((args["state"].double() - want_state.double()).norm() / want_state.double().norm()).item() < 1e-6
+
+
+@pytest.mark.parametrize("where", ["x", "B", "C", "dt", "state"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_values_that_are_not_finite_reach_no_earlier_token_and_no_other_row(where, value):
+    args, sizes = _inputs(4, 2, 200, (200, 200), torch.float32)
+    want = _run({k: v.clone() for k, v in args.items()}, sizes)
+    at, inner = 100, 4 * 64
+    if where == "dt":
+        args["dt_raw"][0, at, 1] = value
+    elif where == "state":
+        args["state"][3, 1, 5, 7], at = value, 0
+    else:
+        args["xBC"][0, at, {"x": 70, "B": inner + 3, "C": inner + 2 * 128 + 3}[where]] = value
+    got = _run(args, sizes)
+    assert torch.equal(got[1], want[1])
+    rel = ((got[0, :at] - want[0, :at]).norm() / want[0, :at].norm().clamp_min(1e-9)).item()
+    assert at == 0 or rel < 1e-6
+    assert not torch.isfinite(got[0, at:]).all()
+    assert torch.isfinite(got[0, :, 128:]).all()                                  # heads 2 and 3: another group
