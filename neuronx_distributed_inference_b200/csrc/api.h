@@ -97,12 +97,12 @@ void qgemv_launch(const void* x, const void* w, const float* scale, int scale_n,
                   float norm_offset, int n_sms, cudaStream_t stream);
 
 // bounded waits of the tensor-core kernels (mbar_wait.cuh, kernel_status.cu): where a kernel reports a wait that ran out; raising for it on the host
-enum WaitKernel { WAIT_ATTENTION, WAIT_GEMM_PAIR, WAIT_SKINNY, WAIT_SSD, WAIT_PROBE, WAIT_KERNELS };
+enum WaitKernel { WAIT_ATTENTION, WAIT_GEMM_PAIR, WAIT_SKINNY, WAIT_SSD, WAIT_ROUTER, WAIT_PROBE, WAIT_KERNELS };
 unsigned* wait_word(WaitKernel which);
 void check_waits();
 void wait_probe_launch(long long clocks, int* out, cudaStream_t stream);
 // launches of the tensor-core kernels by the host (a graph replay is none): which route calls took
-enum CountedKernel { COUNT_ATTENTION, COUNT_GEMM_PAIR, COUNT_SKINNY, COUNT_GEMM_TCGEN05, COUNT_SSD, COUNT_KERNELS };
+enum CountedKernel { COUNT_ATTENTION, COUNT_GEMM_PAIR, COUNT_SKINNY, COUNT_GEMM_TCGEN05, COUNT_SSD, COUNT_ROUTER, COUNT_KERNELS };
 void count_launch(CountedKernel which);
 std::vector<std::pair<std::string, long long>> kernel_launches();
 

@@ -338,85 +338,6 @@ __global__ void __launch_bounds__(256) router_logits_split_kernel(const T* __res
   }
 }
 
-// Logits of many bf16 rows on tensor cores at fp32 precision: a fp32 weight is the exact sum of three bf16 parts (8 + 8 + 8 bits), bf16 rows are exact,
-// so every product is exact in fp32 and only the sums round, as in the kernel above.  Block = 32 tokens x 128 experts, 64 columns per round; the
-// weights are split on their way into shared memory, the three partial sums stay apart until the end.  The kernel above is bound by reading the
-// weights from L2 once per 8 tokens (512 MB for 4096 tokens x 128 experts x 2048: 85 us, here 52 us; a cast and a library fp32 product 77 us).
-// The tensor core adds without rounding to nearest (2e-6 .. 7e-6 off over 2048 .. 6144 columns when it carries the sum alone): its sums are taken over
-// 64 columns and added up in fp32 registers.
-constexpr int RTC_T = 32, RTC_E = 128, RTC_K = 64, RTC_LD = RTC_K + 8, RTC_THREADS = 512;
-constexpr int RTC_SMEM = (RTC_T + 3 * RTC_E) * RTC_LD * 2;
-__global__ void __launch_bounds__(RTC_THREADS, 2) router_logits_tc_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
-                                                                          float* __restrict__ logits, float* __restrict__ parts, int N, int W, int E) {
-  extern __shared__ __align__(16) __nv_bfloat16 rtc_sm[];
-  __nv_bfloat16* xs = rtc_sm;                                // [RTC_T][LD]
-  __nv_bfloat16* ws = xs + RTC_T * RTC_LD;                   // [3][RTC_E][LD]
-  const int t0 = blockIdx.x * RTC_T, e0 = blockIdx.y * RTC_E, tid = threadIdx.x, lane = tid & 31;
-  const int wm = tid >> 8, we = (tid >> 5) & 7;              // this warp's 16 tokens and 16 experts
-  float sum[2][4] = {}, low[2][4] = {};                      // high parts; middle and low parts
-  uint4 xr = make_uint4(0u, 0u, 0u, 0u);
-  float4 wr[4];
-  auto fetch = [&](int k0) {
-    const int xt = tid >> 3, xc = (tid & 7) * 8;
-    if (tid < RTC_T * 8 && t0 + xt < N) xr = *reinterpret_cast<const uint4*>(x + (size_t)(t0 + xt) * W + k0 + xc);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int i = tid + RTC_THREADS * j, e = e0 + (i >> 4);
-      wr[j] = e < E ? __ldg(reinterpret_cast<const float4*>(w + (size_t)e * W + k0) + (i & 15)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  };
-  // this block's part of the columns: part 0 goes to `logits`, the others to `parts`, router_select_kernel adds them in order
-  const int rounds = W / RTC_K, ks = (int)((long long)rounds * blockIdx.z / gridDim.z) * RTC_K, ke = (int)((long long)rounds * (blockIdx.z + 1) / gridDim.z) * RTC_K;
-  if (blockIdx.z > 0) logits = parts + (size_t)(blockIdx.z - 1) * N * E;
-  fetch(ks);
-  for (int k0 = ks; k0 < ke; k0 += RTC_K) {
-    __syncthreads();                      // the readers of the round before are done
-    if (tid < RTC_T * 8) *reinterpret_cast<uint4*>(xs + (tid >> 3) * RTC_LD + (tid & 7) * 8) = xr;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int i = tid + RTC_THREADS * j;
-      __nv_bfloat16* dst = ws + (i >> 4) * RTC_LD + (i & 15) * 4;
-      float v[4] = {wr[j].x, wr[j].y, wr[j].z, wr[j].w};
-#pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        const uint32_t a = pack_bf16(v[0], v[1]), b = pack_bf16(v[2], v[3]);
-        *reinterpret_cast<uint2*>(dst + s * RTC_E * RTC_LD) = make_uint2(a, b);
-        v[0] -= bf16lo(a); v[1] -= bf16hi(a); v[2] -= bf16lo(b); v[3] -= bf16hi(b);
-      }
-    }
-    __syncthreads();
-    if (k0 + RTC_K < ke) fetch(k0 + RTC_K);
-    float acc[2][2][4] = {};              // [high | middle and low][8 experts]
-#pragma unroll
-    for (int k = 0; k < RTC_K; k += 16) {
-      uint32_t a[4];
-      ldmatrix_x4(a, xs + (wm * 16 + (lane & 15)) * RTC_LD + k + (lane >> 4) * 8);
-#pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        uint32_t b[4];                    // two 8-expert tiles x two 8-column halves
-        ldmatrix_x4(b, ws + (s * RTC_E + we * 16 + (lane & 7) + (lane >> 4) * 8) * RTC_LD + k + ((lane >> 3) & 1) * 8);
-        const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
-        mma_bf16_16816(acc[s > 0][0], a, b0);
-        mma_bf16_16816(acc[s > 0][1], a, b1);
-      }
-    }
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        sum[n][c] += acc[0][n][c];
-        low[n][c] += acc[1][n][c];
-      }
-  }
-#pragma unroll
-  for (int n = 0; n < 2; ++n)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int t = t0 + wm * 16 + (lane >> 2) + (c >> 1) * 8, e = e0 + we * 16 + n * 8 + (lane & 3) * 2 + (c & 1);
-      if (t < N && e < E) logits[(size_t)t * E + e] = sum[n][c] + low[n][c];
-    }
-}
-
 __global__ void __launch_bounds__(256) router_select_kernel(float* __restrict__ logits, const float* __restrict__ parts, int n_parts, float* __restrict__ topk_w,
                                                             void* __restrict__ topk_i, int N, int E, int k, RouterSelect sel) {
   extern __shared__ float zsm[];                             // per warp: [E] scores, [E] choice scores, [groups] group bests
@@ -429,13 +350,23 @@ __global__ void __launch_bounds__(256) router_select_kernel(float* __restrict__ 
   float* gb = ch + E;
   // scores: sigmoid, softmax over all router outputs, or the logits themselves (softmax over the chosen ones at the end)
   float mx = -INFINITY;
-  for (int e = lane; e < E; e += 32) {
-    float v = logits[(size_t)tok * E + e];
-    for (int z = 0; z < n_parts; ++z) v += parts[((size_t)z * N + tok) * E + e];
-    if (sel.bias) v += sel.bias[e];
-    if (sel.bias || n_parts) logits[(size_t)tok * E + e] = v;
-    sc[e] = v;
-    mx = fmaxf(mx, v);
+  for (int c0 = lane; c0 < E; c0 += 128) {                    // four experts a lane: the loads of all parts in flight together
+    float v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = c0 + 32 * u < E ? logits[(size_t)tok * E + c0 + 32 * u] : 0.f;
+#pragma unroll 8
+    for (int z = 0; z < n_parts; ++z)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] += c0 + 32 * u < E ? __ldg(parts + ((size_t)z * N + tok) * E + c0 + 32 * u) : 0.f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int e = c0 + 32 * u;
+      if (e >= E) break;
+      if (sel.bias) v[u] += sel.bias[e];
+      if (sel.bias || n_parts) logits[(size_t)tok * E + e] = v[u];
+      sc[e] = v[u];
+      mx = fmaxf(mx, v[u]);
+    }
   }
   mx = warp_max(mx);
   if (sel.softmax == 2) {
@@ -450,21 +381,19 @@ __global__ void __launch_bounds__(256) router_select_kernel(float* __restrict__ 
   }
   for (int e = lane; e < E; e += 32) ch[e] = sc[e] + (sel.correction ? sel.correction[e] : 0.f);
   __syncwarp();
-  // largest value of an array of n floats, lowest index on ties; every lane gets (value, index)
-  auto arg_max = [&](const float* a, int n, float& best, int& bi) {
-    best = -INFINITY;
-    bi = 0x7fffffff;
+  // index of the largest value of an array of n floats, the lowest on ties; every lane gets it
+  auto arg_max = [&](const float* a, int n) {
+    float best = -INFINITY;
+    int bi = 0x7fffffff;
     for (int e = lane; e < n; e += 32) {
       const float v = a[e];
       if (v > best || (v == best && e < bi)) { best = v; bi = e; }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
-    if (bi >= n) bi = 0;                                     // nothing left to choose from (or not a number): stay inside the array
+    // order-preserving integers (-0 as 0): the largest, then the lowest index that holds it
+    const int bits = __float_as_int(best + 0.f);
+    const unsigned key = (unsigned)(bits ^ ((bits >> 31) | 0x80000000)), top = __reduce_max_sync(0xffffffffu, key);
+    bi = __reduce_min_sync(0xffffffffu, key == top ? bi : 0x7fffffff);
+    return bi >= n ? 0 : bi;                                 // nothing left to choose from (or not a number): stay inside the array
   };
   if (G) {
     // a group is as good as its best choice score; experts outside the `keep` best groups cannot be chosen
@@ -476,9 +405,7 @@ __global__ void __launch_bounds__(256) router_select_kernel(float* __restrict__ 
     }
     __syncwarp();
     for (int j = 0; j < sel.keep; ++j) {
-      float best;
-      int bg;
-      arg_max(gb, G, best, bg);
+      const int bg = arg_max(gb, G);
       if (lane == 0) gb[bg] = NAN;                           // marks the group as kept; NaN never wins a later comparison
       __syncwarp();
     }
@@ -488,9 +415,7 @@ __global__ void __launch_bounds__(256) router_select_kernel(float* __restrict__ 
   }
   float sum = 0.f;
   for (int j = 0; j < k; ++j) {
-    float best;
-    int bi;
-    arg_max(ch, E, best, bi);
+    const int bi = arg_max(ch, E);
     const float w = sel.softmax == 2 ? expf(sc[bi] - mx) : sc[bi];
     sum += w;
     if (lane == 0) {
@@ -518,14 +443,6 @@ __global__ void __launch_bounds__(256) gate_mul_rows_kernel(const T* __restrict_
 
 }  // namespace
 
-// Column parts of the tensor-core kernel, up to one block per SM (two: 59 instead of 56 us at 4096 tokens, 44 instead of 35 at 1000 x 512 experts); 0: the CUDA-core kernel.  A block computes 128 experts whether they exist or not, so
-// fewer than 64 stay with the CUDA cores, and so do a few tokens (N = 128: 17 us there).
-int router_parts(int N, int W, int E, bool lp) {
-  if (!lp || N < 256 || E < 64 || W % RTC_K != 0) return 0;
-  const long long blocks = (long long)((N + RTC_T - 1) / RTC_T) * ((E + RTC_E - 1) / RTC_E);
-  return (int)std::max<long long>(1, std::min<long long>({4, kNumSMs / blocks, W / RTC_K}));
-}
-
 void router_topk_launch(const void* x, const float* w, float* logits, float* parts, float* topk_w, void* topk_i, int N, int W, int E, int k,
                         const RouterSelect& sel, bool lp, cudaStream_t st) {
   if (N <= 0) return;
@@ -544,8 +461,7 @@ void router_topk_launch(const void* x, const float* w, float* logits, float* par
   const int kparts = router_parts(N, W, E, lp);
   if (kparts > 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
     n_parts = kparts - 1;
-    cudaFuncSetAttribute(router_logits_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RTC_SMEM);
-    router_logits_tc_kernel<<<dim3((N + RTC_T - 1) / RTC_T, (E + RTC_E - 1) / RTC_E, kparts), RTC_THREADS, RTC_SMEM, st>>>((const __nv_bfloat16*)x, w, logits, parts, N, W, E);
+    router_logits_tc_launch(x, w, logits, parts, N, W, E, kparts, st);
   } else if (E <= 16 && W % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
     // tokens per block: one for a few tokens; then four, and eight (half the weight reads) once four would give every SM eight blocks
     const int srt = few ? 1 : N <= 4 * 8 * kNumSMs ? 4 : 8;

@@ -97,6 +97,7 @@ struct RouterSelect {
 };
 // `parts`: [router_parts - 1, N, E] partial logits
 int router_parts(int N, int W, int E, bool lp);
+void router_logits_tc_launch(const void* x, const float* w, float* logits, float* parts, int N, int W, int E, int n_parts, cudaStream_t st);      // router_tc.cu
 void router_topk_launch(const void* x, const float* w, float* logits, float* parts, float* topk_w, void* topk_i, int N, int W, int E, int k,
                         const RouterSelect& sel, bool lp, cudaStream_t st);
 
