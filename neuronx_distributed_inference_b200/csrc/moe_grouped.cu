@@ -124,30 +124,51 @@ __global__ void __launch_bounds__(128) moe_combine_kernel(const __nv_bfloat16* _
 }
 
 // ---- bf16 experts on CTA-pair tiles (gemm_pair.cu): rows one after the other, up to 256 of an expert per tile ------------------------------------------------------
-// One CTA: the atomic that counts an expert's entries also ranks them, so one pass decides the rows and the second only adds the segment starts
-// (32768 entries, 128 experts: 11 us; with a second atomic pass, a serial scan and the inverse table 31 us).
+// A cluster of 8 CTAs, each with an eighth of the entries: the atomic that counts an expert's entries also ranks them, so one pass decides the rows and the
+// second only adds the starts.  A start needs the counts of the other CTAs, read from their shared memory; every CTA scans the totals for itself.
+// Bound by the latency of two passes over the ids: 32768 entries, 128 experts 7.2 us, one CTA for all 15.3 (cold caches).
+constexpr int MOE_PLAN_CTAS = 8;
 __global__ void __launch_bounds__(MOE_PLAN_THREADS) moe_plan256_kernel(const int* __restrict__ topk_i, int id_step, int entries, int expert_offset, int e_local, int tiles,
                                                                        int* __restrict__ pos, int* __restrict__ tile_expert, int* __restrict__ tile_row) {
-  __shared__ int count[MOE_MAX_E], start[MOE_MAX_E], tile0[MOE_MAX_E + 1];
+  __shared__ int count[MOE_MAX_E], total[MOE_MAX_E], start[MOE_MAX_E], tile0[MOE_MAX_E + 1];
   pdl_launch_dependents();
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, rank = blockIdx.x;
   for (int e = tid; e < e_local; e += MOE_PLAN_THREADS) count[e] = 0;
   __syncthreads();
   pdl_wait();
-  constexpr int U = 8;             // entries in flight per thread
-  for (int i0 = tid; i0 < entries; i0 += U * MOE_PLAN_THREADS) {
+  const int first = (int)((long long)entries * rank / MOE_PLAN_CTAS), end = (int)((long long)entries * (rank + 1) / MOE_PLAN_CTAS);
+  constexpr int U = 4;             // entries in flight per thread
+  for (int i0 = first + tid; i0 < end; i0 += U * MOE_PLAN_THREADS) {
     int e[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) e[u] = i0 + u * MOE_PLAN_THREADS < entries ? topk_i[(size_t)(i0 + u * MOE_PLAN_THREADS) * id_step] - expert_offset : -1;
+    for (int u = 0; u < U; ++u) e[u] = i0 + u * MOE_PLAN_THREADS < end ? topk_i[(size_t)(i0 + u * MOE_PLAN_THREADS) * id_step] - expert_offset : -1;
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (i0 + u * MOE_PLAN_THREADS < entries) pos[i0 + u * MOE_PLAN_THREADS] = (e[u] >= 0 && e[u] < e_local) ? atomicAdd(&count[e[u]], 1) : -1;
+      if (i0 + u * MOE_PLAN_THREADS < end) pos[i0 + u * MOE_PLAN_THREADS] = (e[u] >= 0 && e[u] < e_local) ? atomicAdd(&count[e[u]], 1) : -1;
   }
-  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  for (int e = tid; e < e_local; e += MOE_PLAN_THREADS) {
+    int n = 0, before = 0;
+#pragma unroll
+    for (int r = 0; r < MOE_PLAN_CTAS; ++r) {
+      uint32_t at;
+      int v;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&count[e]))), "r"(r));
+      asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+      if (r < rank) before += v;
+      n += v;
+    }
+    total[e] = n;
+    start[e] = before;
+  }
+  // the others have read this CTA's counts: they may be written over, and the CTA may end
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (tid < 32) {
     int at = 0, tile = 0;
     for (int c0 = 0; c0 < e_local; c0 += 32) {
-      const int c = c0 + tid, n = c < e_local ? count[c] : 0, nt = (n + 255) >> 8;
+      const int c = c0 + tid, n = c < e_local ? total[c] : 0, nt = (n + 255) >> 8;
       int incl = n, tincl = nt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -158,7 +179,7 @@ __global__ void __launch_bounds__(MOE_PLAN_THREADS) moe_plan256_kernel(const int
         }
       }
       if (c < e_local) {
-        start[c] = at + incl - n;
+        count[c] = at + incl - n;              // the expert's first row
         tile0[c] = tile + tincl - nt;
       }
       at += __shfl_sync(0xffffffffu, incl, 31);
@@ -167,23 +188,25 @@ __global__ void __launch_bounds__(MOE_PLAN_THREADS) moe_plan256_kernel(const int
     if (tid == 0) tile0[e_local] = tile;
   }
   __syncthreads();
-  for (int e = tid; e < e_local; e += MOE_PLAN_THREADS)
-    for (int t = tile0[e], r = 0; t < tile0[e + 1]; ++t, r += 256) {
-      tile_expert[t] = e | min(256, count[e] - r) << 10;
-      tile_row[t] = start[e] + r;
-    }
-  for (int t = tile0[e_local] + tid; t < tiles; t += MOE_PLAN_THREADS) tile_expert[t] = -1;
-  for (int i0 = tid; i0 < entries; i0 += U * MOE_PLAN_THREADS) {      // own entries again: written by this thread above
+  if (rank == 0) {
+    for (int e = tid; e < e_local; e += MOE_PLAN_THREADS)
+      for (int t = tile0[e], r = 0; t < tile0[e + 1]; ++t, r += 256) {
+        tile_expert[t] = e | min(256, total[e] - r) << 10;
+        tile_row[t] = count[e] + r;
+      }
+    for (int t = tile0[e_local] + tid; t < tiles; t += MOE_PLAN_THREADS) tile_expert[t] = -1;
+  }
+  for (int i0 = first + tid; i0 < end; i0 += U * MOE_PLAN_THREADS) {      // own entries again: written by this thread above
     int e[U], r[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = i0 + u * MOE_PLAN_THREADS;
-      e[u] = i < entries ? topk_i[(size_t)i * id_step] - expert_offset : -1;
-      r[u] = i < entries ? pos[i] : -1;
+      e[u] = i < end ? topk_i[(size_t)i * id_step] - expert_offset : -1;
+      r[u] = i < end ? pos[i] : -1;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (r[u] >= 0) pos[i0 + u * MOE_PLAN_THREADS] = start[e[u]] + r[u];
+      if (r[u] >= 0) pos[i0 + u * MOE_PLAN_THREADS] = count[e[u]] + start[e[u]] + r[u];
   }
 }
 
@@ -213,8 +236,21 @@ __global__ void __launch_bounds__(256) moe_scatter_kernel(const __nv_bfloat16* _
 void moe_plan256_launch(const int* topk_i, int id_step, int entries, int expert_offset, int e_local, int tiles, int* pos, int* tile_expert, int* tile_row,
                         cudaStream_t stream) {
   if (e_local > MOE_MAX_E) throw std::runtime_error("moe_plan: more than 512 local experts");
-  launch_pdl(moe_plan256_kernel, dim3(1), dim3(MOE_PLAN_THREADS), 0, stream, topk_i, id_step, entries, expert_offset, e_local, tiles, pos, tile_expert,
-             tile_row);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(MOE_PLAN_CTAS);
+  cfg.blockDim = dim3(MOE_PLAN_THREADS);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = MOE_PLAN_CTAS;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, moe_plan256_kernel, topk_i, id_step, entries, expert_offset, e_local, tiles, pos, tile_expert, tile_row);
+  if (e != cudaSuccess) throw std::runtime_error(std::string("moe_plan launch failed: ") + cudaGetErrorString(e));
 }
 void moe_scatter_launch(const void* x, const float* topk_w, const int* pos, void* xp, int N, int H, int k, int scale_input, cudaStream_t stream) {
   launch_pdl(moe_scatter_kernel, dim3(N), dim3(256), 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), topk_w, pos,
