@@ -35,6 +35,12 @@ def test_rmsnorm(rows, H):
     assert _rel(r2, rr2) < 1e-6 and _rel(y2, yr2) < 8e-3
 
 
+# one, two or four warps per row from 1024 rows on, H <= 8192: row counts that do not fill a block, rows shorter than a warp's pieces, the sizes' edges
+@pytest.mark.parametrize("rows,H", [(1023, 2048), (1024, 2048), (1025, 2056), (1031, 4096), (1024, 4104), (1030, 8192), (1024, 8200), (3000, 8), (1024, 264)])
+def test_rmsnorm_of_many_rows(rows, H):
+    test_rmsnorm(rows, H)
+
+
 @pytest.mark.parametrize("T", [1, 2, 3, 8])
 @pytest.mark.parametrize("N,K", [(4096, 4096), (6144, 4096), (1000 * 16, 2048), (4096, 14336), (512, 512), (40, 256),
                                  (3072, 4096), (64128, 4096), (4096, 7168), (4096, 2048), (4096, 1792), (768, 4096), (4096, 320), (400, 512)])
