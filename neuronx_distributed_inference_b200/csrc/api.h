@@ -158,6 +158,7 @@ struct AttnDecodeParams {
   float* ws_ml;            // [B*Hkv, nsplit, R, 2]
   unsigned* tickets;       // [B*Hkv]
   int B, T, Hq, Hkv, D, S, L, nsplit, window, block_size, max_blocks;
+  int part_tiles;          // paged: > 0: 64-key tiles of a part, every row has as many parts as it needs (at most nsplit)
   float scale;
   // fused prologue (contiguous decode): q unused; q/k/v taken from the QKV projection output
   const void* qkv;        // [B, T, (Hq + 2 Hkv) * D] bf16 or null

@@ -41,6 +41,7 @@ void attention_decode_launch(const AttnDecodeParams& p, cudaStream_t stream) {
   a.B = p.B; a.T = p.T; a.Hq = p.Hq; a.Hkv = p.Hkv; a.S = p.S; a.L = p.L; a.nsplit = p.nsplit; a.window = p.window;
   a.block_size = p.block_size; a.max_blocks = p.max_blocks;
   a.page_shift = -1;
+  a.part_tiles = p.part_tiles;
   for (int s = 0; s < 31; ++s)
     if (p.block_size == 1 << s) a.page_shift = s;
   a.scale_log2 = p.scale * kLog2e;

@@ -41,6 +41,7 @@ struct AttnArgs {
   unsigned* tickets;
   int B, T, Hq, Hkv, S, L, nsplit, window, block_size, max_blocks;
   int page_shift;  // paged: log2(block_size), -1 when it is no power of two
+  int part_tiles;  // paged: > 0: key tiles of a part, a row has as many parts as it needs (at most nsplit); 0: nsplit equal parts of every row
   float scale_log2;
   // fused decode prologue (ATTN_DECODE only): q/k/v come straight from the QKV projection; per-head RMSNorm + RoPE are
   // applied here, the new K/V rows are written to the cache by this CTA before it reads the cache
@@ -150,7 +151,11 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
   int t_lo = 0;
   if (p.window > 0) t_lo = max(0, pos_min - p.window + 1) / ATT_TILE;
   const int span = max(nt - t_lo, 0);
-  const int tps = (span + p.nsplit - 1) / p.nsplit;
+  // parts of this row
+  const bool sized = MODE == ATTN_PAGED && p.part_tiles > 0;
+  const int n_parts = sized ? max(1, (span + p.part_tiles - 1) / p.part_tiles) : p.nsplit;
+  if (sized && split >= n_parts) return;
+  const int tps = (span + n_parts - 1) / n_parts;
   const int t_beg = t_lo + split * tps;
   const int t_end = min(nt, t_beg + tps);
 
@@ -466,7 +471,7 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
   group_sync();
 
   const int bh = (MODE == ATTN_PREFILL) ? 0 : bx;
-  const bool direct = (MODE == ATTN_PREFILL) || p.nsplit == 1;
+  const bool direct = (MODE == ATTN_PREFILL) || n_parts == 1;
   const int ws_rows = p.T * G;               // rows of a piece in the workspace
   // per-row merge factors once (row max over the KS key-split warps, rescale factor of each, denominator incl. the sink):
   // sF[k2][r] = exp2(m_k2 - M) (/ L when written directly), so the element loop below is KS multiply-adds per output
@@ -534,7 +539,6 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
   if (direct) return;
 
   // ---- split-KV combine by the last-arriving CTA of this (batch, kv head) ------------------------------------
-  const int n_parts = p.nsplit;
   __threadfence();
   group_sync();
   if (tid == 0) s_last = (atomicAdd(&p.tickets[bh], 1u) == (unsigned)(n_parts - 1));

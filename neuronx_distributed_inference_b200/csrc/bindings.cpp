@@ -651,13 +651,22 @@ at::Tensor rope_attention_decode(const at::Tensor& qkv, const at::Tensor& cos, c
 //   128 pairs: 500 keys 21 / 22 / 28 / 37         4096: 69 / 57 / 57 / 61         32768: 455 / 301 / 264 / 229 / 223
 //   384 pairs: 500 keys 29 / 37 / 49 / 74         4096: 103 / 98 / 100 / 117      32768: 639 / 537 / 475 / 453          1536 pairs, 4096 keys: 256 / 274 / 312 / 391
 // Head size 64 has its minima at the same numbers (32768 keys: 1 pair 303 / 172 / 92 / 52 / 33 / 29 / 27 / 25, 32 pairs 309 / 186 / 104 / 70 / 55 / 59 / 59 / 66).
-static int paged_nsplit(int pairs, int max_keys) {
+// From 96 pairs on the parts are of one size, about 1024 keys, and a row has as many as it needs: with equal parts of every row the longest rows' parts
+// finished last.  us, parts of 512 / 768 / 1024 / 1536 / 2048 keys, equal parts as above; contexts of one request at the limit, the others anywhere up to it:
+//   384 pairs, 4096 keys: 95 / 87 / 83 / 85 / 83, 91    320, 3000: 66 / 61 / 57 / 59 / 59, 59    192, 4096: 52 / 48 / 50 / 53 / 48, 55
+//   128 pairs, 4096 keys: 37 / 41 / 41 / 36 / 45, 43    768, 2000, head size 64: 56 / 55 / 51 / 51 / 51, 56    1536, 4096: 327 / 298 / 275 / 263 / 264, 256 (one part)
+struct PagedParts {
+  int most, tiles;          // parts of the longest row; 64-key tiles of a part, 0: equal parts of every row
+};
+static PagedParts paged_parts(int pairs, int max_keys) {
   const int tiles = std::max(1, (max_keys + 63) / 64);
-  if (pairs >= 1024) return 1;
-  if (pairs >= 256) return max_keys >= 3072 ? 2 : 1;
-  if (pairs >= 96) return std::max(1, std::min(4, max_keys / 1024));
+  if (pairs >= 1024) return {1, 0};
+  if (pairs >= 96) {
+    const int n = std::max(1, std::min(16, (tiles + 8) / 16));
+    return {n, (tiles + n - 1) / n};
+  }
   const int some = std::min(tiles, pairs > 32 && max_keys <= 8192 ? 4 : pairs > 8 ? 8 : 16);
-  return std::max(some, std::min({64, 2 * 148 / pairs, max_keys / 512}));       // long rows: two CTAs per SM of at least 512 keys
+  return {std::max(some, std::min({64, 2 * 148 / pairs, max_keys / 512})), 0};       // long rows: two CTAs per SM of at least 512 keys
 }
 
 at::Tensor paged_attention_decode(const at::Tensor& q, const at::Tensor& k_cache, const at::Tensor& v_cache,
@@ -678,7 +687,8 @@ at::Tensor paged_attention_decode(const at::Tensor& q, const at::Tensor& k_cache
   p.sinks = sinks.has_value() ? sinks->data_ptr<float>() : nullptr;
   p.B = B; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.S = 0; p.L = 0; p.window = window; p.scale = (float)scale;
   p.block_size = bs; p.max_blocks = block_table.size(1);
-  p.nsplit = paged_nsplit(B * Hkv, p.max_blocks * bs);
+  const PagedParts parts = paged_parts(B * Hkv, p.max_blocks * bs);
+  p.nsplit = parts.most; p.part_tiles = parts.tiles;
   const int64_t rows = (int64_t)B * Hkv * p.nsplit * T * (Hq / Hkv);
   auto& ws = scratch(q.device(), rows * (D + 2), 0, (int64_t)B * Hkv);
   p.ws_o = ws.f.data_ptr<float>();

@@ -46,3 +46,22 @@ def test_few_requests_with_long_contexts(Hkv, D):
         sc = sc.masked_fill(torch.arange(ctx, device="cuda") > pos[0].view(T, 1, 1), float("-inf"))
         want = torch.einsum("thn,nhd->thd", torch.softmax(sc, -1), vv)
         assert ((got[0].float() - want).norm() / want.norm()).item() < 4e-3
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Hkv,window,most", [(1, 0, 4096), (2, 0, 2600), (1, 1500, 4096), (1, 0, 65536 + 64)])
+def test_parts_of_one_size(Hkv, window, most, D):
+    """From 96 (row, kv head) pairs on a row has as many parts as it needs: rows at the edges of the parts, the shortest and the longest that the table holds."""
+    ctx = [most, 1] + [c + d for c in (1024, 2048, 3072) for d in (-1, 0, 1) if c + d <= most] * 9 + [63, 64, 65, 500, most - 1]
+    B = 96 // Hkv + 3
+    ctx = (ctx * 3)[:B]
+    page, Hq = 64, 4 * Hkv
+    n = -(-most // page)
+    kc, vc = (torch.randn(n + 7, page, Hkv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    table = torch.stack([torch.randperm(n + 7, device="cuda")[:n] for _ in range(B)]).int()          # rows share pages
+    q, pos = torch.randn(B, 1, Hq, D, device="cuda", dtype=torch.bfloat16), torch.tensor(ctx, device="cuda", dtype=torch.int32).view(B, 1) - 1
+    for _ in range(2):
+        got = ops.paged_attention_decode(q, kc, vc, table, pos, D ** -0.5, window or None)
+        for b in range(0, B, 1 if most <= 4096 else 17):
+            want = ref.paged_attention_decode(q[b:b + 1].float(), kc.float(), vc.float(), table[b:b + 1], pos[b:b + 1], D ** -0.5, window or None, None)
+            assert ((got[b:b + 1].float() - want).norm() / want.norm()).item() < 4e-3
