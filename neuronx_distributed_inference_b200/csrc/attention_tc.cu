@@ -16,6 +16,8 @@
 //   200 clocks for each hand-over.  One 8192-token prompt, 32 / 8 heads x 128: 0.44 ms alone (1.25 PFLOP/s).  Before: 0.495 ms; of that, 28 us from
 //   the MMA warp's code (fa_umma), 27 us from the halves of P, 7 us from the mixed-type sums (fa_add_bf16x2), 20 us from masks outside the tiles
 //   that need none.  3 x 1000 tokens of head size 64, window 128: 24 us, 30 before.
+//   A soft cap (tanh) needs eight more fp32 pair operations per pair of scores, which bound those tiles; they run beside the exponentials and end in the
+//   exponent's multiply-add, the maximum is taken before the cap.  Three portions with cap, gate and window: 255 us; 267 with the cap as a pass of its own.
 //   Tried and slower: 64-key tiles with two score buffers per query tile (478 us: both tiles' softmax phases fall together, and a hand-over costs as
 //   much per 64 keys); sixteen softmax warps with half a row per thread (482 us); a share of the exponentials as polynomials on the FMA pipe (2 of 16: no
 //   gain, 4 of 16: 1 % slower: the fp32 pair operations cost more clocks than the exponentials they replace); the maximum beside the exponentials of
@@ -176,18 +178,24 @@ __device__ __forceinline__ uint64_t fa_add2(uint64_t a, uint64_t b) {
 __device__ __forceinline__ void fa_add_bf16x2(float& s_lo, float& s_hi, uint32_t w) {
   asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.bf16 %0, l, %0;\n\tadd.rn.f32.bf16 %1, h, %1;\n\t}" : "+f"(s_lo), "+f"(s_hi) : "r"(w));
 }
-// tanh on |x| <= 1: x times a polynomial in x^2 (weighted least squares on Chebyshev nodes, relative error 1.7e-7 with fp32 arithmetic)
-__device__ __forceinline__ uint64_t fa_tanh2_small(uint64_t x) {
-  const uint64_t u = fa_mul2(x, x);
-  uint64_t r = fa_pack2(0.00104102155f, 0.00104102155f);
-  r = fa_fma2(r, u, fa_pack2(-0.00620337576f, -0.00620337576f));
-  r = fa_fma2(r, u, fa_pack2(0.0202899761f, 0.0202899761f));
-  r = fa_fma2(r, u, fa_pack2(-0.0534570292f, -0.0534570292f));
-  r = fa_fma2(r, u, fa_pack2(0.13325204f, 0.13325204f));
-  r = fa_fma2(r, u, fa_pack2(-0.333328396f, -0.333328396f));
-  r = fa_fma2(r, u, fa_pack2(0.99999994f, 0.99999994f));
-  return fa_mul2(x, r);
-}
+// Soft cap: c tanh(x) on |x| <= 1 as x times a polynomial in x^2 (weighted least squares on Chebyshev nodes, relative error 1.7e-7 with fp32 arithmetic), c in
+// its coefficients
+struct FaCap {
+  uint64_t k[7];
+  __device__ __forceinline__ explicit FaCap(float c) {
+    const float t[7] = {0.00104102155f, -0.00620337576f, 0.0202899761f, -0.0534570292f, 0.13325204f, -0.333328396f, 0.99999994f};
+#pragma unroll
+    for (int i = 0; i < 7; ++i) k[i] = fa_pack2(t[i] * c, t[i] * c);
+  }
+  // c tanh(x) + add
+  __device__ __forceinline__ uint64_t operator()(uint64_t x, uint64_t add) const {
+    const uint64_t u = fa_mul2(x, x);
+    uint64_t r = k[0];
+#pragma unroll
+    for (int i = 1; i < 7; ++i) r = fa_fma2(r, u, k[i]);
+    return fa_fma2(x, r, add);
+  }
+};
 
 template <int D, int NX>
 struct FaShape {
@@ -431,6 +439,7 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
     const int w_pos = ctx + t_tile + 32 * qd;
     const int up_min = p.causal ? min(w_pos, end - 1) : end - 1, up_max = p.causal ? min(w_pos + 31, end - 1) : end - 1;
     const int lb_min = reach(w_pos), lb_max = reach(w_pos + 31);
+    const FaCap cap(CAP ? p.softcap * FA_LOG2E : 0.f);
     const float hs = p.head_scale ? p.scale * p.head_scale[h] : p.scale;
     float m_run = -INFINITY, l_run = 0.f;
     auto tile = [&](auto masked, int i, int key0) {
@@ -449,36 +458,26 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
           dead[c] = k0 > up_max || (k0 + 63 < lb_min && k0 >= keep);
         }
       }
+      bool slow[2] = {false, false};                     // halves with scores beyond the cap (|x| > 1): tanhf for those scores
       if (CAP) {
+        // v = score / cap from here on; the cap itself is taken beside the exponentials, the maximum's alone before them (it is increasing)
         const float to_cap = hs / p.softcap;
         const uint64_t tc2 = fa_pack2(to_cap, to_cap);
 #pragma unroll
-        for (int c0 = 0; c0 < 128; c0 += 64) {
-          if (dead[c0 >> 6]) continue;
+        for (int c = 0; c < 2; ++c) {
+          if (dead[c]) continue;
           float big = 0.f;
 #pragma unroll
-          for (int e = c0; e < c0 + 64; ++e) big = fmaxf(big, fabsf(__uint_as_float(v[e])));
-          // the maximum is taken over scores that the row does not see too (later keys, rows of pages that were not fetched, whatever shared memory
-          // held): both ways give a score the same bits
-          if (!__any_sync(0xffffffffu, !(big * fabsf(to_cap) <= 1.f))) {
-#pragma unroll
-            for (int e = c0; e < c0 + 64; e += 2) {
-              float a, c;
-              fa_unpack2(fa_tanh2_small(fa_mul2(fa_pack2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), tc2)), a, c);
-              v[e] = __float_as_uint(a);
-              v[e + 1] = __float_as_uint(c);
-            }
-          } else {
-#pragma unroll
-            for (int e = c0; e < c0 + 64; e += 2) {
-              const uint64_t x2 = fa_mul2(fa_pack2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), tc2);
-              float x, y, a, c;
-              fa_unpack2(x2, x, y);
-              fa_unpack2(fa_tanh2_small(x2), a, c);
-              v[e] = __float_as_uint(fabsf(x) <= 1.f ? a : tanhf(x));
-              v[e + 1] = __float_as_uint(fabsf(y) <= 1.f ? c : tanhf(y));
-            }
+          for (int e = 64 * c; e < 64 * c + 64; e += 2) {
+            float a, d;
+            fa_unpack2(fa_mul2(fa_pack2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), tc2), a, d);
+            v[e] = __float_as_uint(a);
+            v[e + 1] = __float_as_uint(d);
+            big = fmaxf(big, fmaxf(fabsf(a), fabsf(d)));
           }
+          // taken over scores that the row does not see too (later keys, rows of pages that were not fetched, whatever shared memory held): both
+          // ways give a score the same bits
+          slow[c] = __any_sync(0xffffffffu, !(big <= 1.f));
         }
         scl = p.softcap * FA_LOG2E;
       } else if (!(scl > 0.f)) {                         // a head's factor may be zero or negative: the maximum below needs a positive scale
@@ -486,22 +485,23 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
         for (int e = 0; e < 128; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * scl);
         scl = 1.f;
       }
+      uint32_t see[4] = {~0u, ~0u, ~0u, ~0u};
       if constexpr (MASKED) {
-      // masks only where 32 keys are visible to some rows of the warp and not to others (a tile on the diagonal: one of four)
+        // masks only where 32 keys are visible to some rows of the warp and not to others (a tile on the diagonal: one of four)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int k0 = key0 + 32 * c;
-        if (!(k0 + 31 <= up_min && (k0 >= lb_max || k0 + 31 < keep)) && !dead[c >> 1]) {
-          const int e_hi = up - k0, e_lo = lb - k0, e_keep = keep - k0;
-          const uint32_t m_hi = e_hi >= 31 ? ~0u : e_hi < 0 ? 0u : (2u << e_hi) - 1u;
-          const uint32_t m_lo = e_lo <= 0 ? ~0u : e_lo > 31 ? 0u : ~0u << e_lo;
-          const uint32_t m_keep = e_keep > 31 ? ~0u : e_keep <= 0 ? 0u : (1u << e_keep) - 1u;
-          const uint32_t see = m_hi & (m_lo | m_keep);
+        for (int c = 0; c < 4; ++c) {
+          const int k0 = key0 + 32 * c;
+          if (!(k0 + 31 <= up_min && (k0 >= lb_max || k0 + 31 < keep)) && !dead[c >> 1]) {
+            const int e_hi = up - k0, e_lo = lb - k0, e_keep = keep - k0;
+            const uint32_t m_hi = e_hi >= 31 ? ~0u : e_hi < 0 ? 0u : (2u << e_hi) - 1u;
+            const uint32_t m_lo = e_lo <= 0 ? ~0u : e_lo > 31 ? 0u : ~0u << e_lo;
+            const uint32_t m_keep = e_keep > 31 ? ~0u : e_keep <= 0 ? 0u : (1u << e_keep) - 1u;
+            see[c] = m_hi & (m_lo | m_keep);
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (!(see & (1u << e))) v[32 * c + e] = 0xff800000u;      // -inf
+            for (int e = 0; e < 32; ++e)
+              if (!(see[c] & (1u << e))) v[32 * c + e] = 0xff800000u;      // -inf
+          }
         }
-      }
       }
       // row maximum in the domain of v (its scale is positive), four independent chains
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -514,7 +514,12 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
           for (int c = 0; c < 4; ++c) mx4[c] = fmaxf(mx4[c], fmaxf(__uint_as_float(v[e + 2 * c]), __uint_as_float(v[e + 2 * c + 1])));
       }
       const float mx_raw = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      const float mx = (mx_raw == -INFINITY) ? -INFINITY : mx_raw * scl;
+      float mx = (mx_raw == -INFINITY) ? -INFINITY : mx_raw * scl;
+      if (CAP) {
+        float t, unused;
+        fa_unpack2(cap(fa_pack2(mx_raw, mx_raw), 0ull), t, unused);
+        if (mx > -INFINITY) mx = fabsf(mx_raw) <= 1.f ? t : tanhf(mx_raw) * scl;
+      }
       const bool grow = mx > m_run + SLACK || (m_run == -INFINITY && mx > -INFINITY);
       const float m_new = grow ? mx : m_run;
       const float alpha = (m_run == -INFINITY) ? 0.f : fa_ex2(m_run - m_new);
@@ -552,11 +557,32 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
         if (dead[c]) {
 #pragma unroll
           for (int e = 0; e < 32; ++e) pk[e] = 0u;
+        } else if (CAP && slow[c]) {
+#pragma unroll
+          for (int e = 0; e < 64; e += 2) {
+            const float s0 = __uint_as_float(v[64 * c + e]), s1 = __uint_as_float(v[64 * c + e + 1]);
+            float a, bb;
+            fa_unpack2(cap(fa_pack2(s0, s1), neg2), a, bb);
+            if (!(fabsf(s0) <= 1.f)) a = fmaf(tanhf(s0), scl, neg_m);
+            if (!(fabsf(s1) <= 1.f)) bb = fmaf(tanhf(s1), scl, neg_m);
+            if (MASKED) {
+              if (!(see[2 * c + (e >> 5)] & (1u << (e & 31)))) a = -INFINITY;
+              if (!(see[2 * c + (e >> 5)] & (2u << (e & 31)))) bb = -INFINITY;
+            }
+            const uint32_t w = pack_bf16(fa_ex2(a), fa_ex2(bb));
+            fa_add_bf16x2(ls[e & 2], ls[(e & 2) + 1], w);
+            pk[e >> 1] = w;
+          }
         } else {
 #pragma unroll
           for (int e = 0; e < 64; e += 2) {
+            const uint64_t v2 = fa_pack2(__uint_as_float(v[64 * c + e]), __uint_as_float(v[64 * c + e + 1]));
             float a, bb;
-            fa_unpack2(fa_fma2(fa_pack2(__uint_as_float(v[64 * c + e]), __uint_as_float(v[64 * c + e + 1])), scl2, neg2), a, bb);
+            fa_unpack2(CAP ? cap(v2, neg2) : fa_fma2(v2, scl2, neg2), a, bb);
+            if (CAP && MASKED) {                         // the cap of a masked score is no -inf
+              if (!(see[2 * c + (e >> 5)] & (1u << (e & 31)))) a = -INFINITY;
+              if (!(see[2 * c + (e >> 5)] & (2u << (e & 31)))) bb = -INFINITY;
+            }
             const uint32_t w = pack_bf16(fa_ex2(a), fa_ex2(bb));          // -inf -> 0
             // the sum uses the bf16-rounded probabilities, exactly what the tensor core multiplies
             fa_add_bf16x2(ls[e & 2], ls[(e & 2) + 1], w);
@@ -717,7 +743,7 @@ void attention_prefill_tc_launch(const void* q, const void* k, const void* v, vo
 
 // Prompt portions over a paged cache.  Sizes this kernel takes: keys and values of one size, 64 or 128, rows on 16-byte boundaries, pages of
 // 2^k >= 8 tokens (smaller ones would break the 8-row swizzle atoms), no distance term; the rest is paged_window_attention_mma_kernel's.
-// 3 rows of up to 1024 tokens over contexts up to 3000, 32 / 8 heads x 128, window 2048, cap, gate: 0.28 ms, mma.sync kernel 0.89 ms.
+// 3 rows of up to 1024 tokens over contexts up to 3000, 32 / 8 heads x 128, window 2048, cap, gate: 0.255 ms, mma.sync kernel 0.89 ms.
 bool paged_attention_tc_supported(const WindowAttnParams& p, bool lp) {
   return lp && p.T >= 16 && p.maps != 2 && p.slopes == nullptr && p.D == p.Dv && (p.D == 64 || p.D == 128) && (p.v_rs * 2) % 16 == 0 && p.page >= 8 &&
          (p.page & (p.page - 1)) == 0 && (long long)p.B * p.Hq * ((p.T + FA_ROWS - 1) / FA_ROWS) <= 0x7fffffffLL &&
