@@ -17,7 +17,7 @@
 //            8 warps hold the state (64 values a thread) and form its parts and those of x~, 4 warps form M and the parts of x, 8 warps finish the outputs,
 //            one warp issues the MMAs, one the copies, two (one per head) the step sizes and exponents.
 //   What bounds it: the chain of a chunk, about 9000 clocks: update (1500 and a hand-over), the state's parts (2500), inter and intra (3100), outputs (1400); the
-//   144 MMAs alone are 4600.  us, here / step by step: 64 heads, state 128, 4 rows of up to 1024 tokens 108 / 423, one row of 1024 89 / 254, of 128 27 / 41,
+//   144 MMAs alone are 4600.  us, here / step by step: 64 heads, state 128, 4 rows of up to 1024 tokens 106 / 423, one row of 1024 89 / 254, of 128 27 / 41,
 //   4 rows of 64 23.5 / 37.5, one of 48 23 / 22 (the host); 128 heads in 8 groups, 4 rows of up to 1024 207 / 734.  Error against 64 bits, 4 rows of up to
 //   1024: 1.0e-7, step by step 1.1e-7.  Tried: everything unrolled 217 us (2.3 warps waiting for instructions at every issue); four warps for
 //   the outputs 142; conditional loads of x, z 136 and more (the compiler waits for each).
@@ -91,7 +91,8 @@ __device__ __forceinline__ float silu_acc(float z) {
 __device__ __forceinline__ uint32_t swz(int row, int piece) { return (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
 
 // ---- prepare ---------------------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) ssd_prepare_kernel(SsdScanParams p, uint8_t* __restrict__ ws, int* __restrict__ odd, int chunks) {
+constexpr int SP_THREADS = 512;
+__global__ void __launch_bounds__(SP_THREADS) ssd_prepare_kernel(SsdScanParams p, uint8_t* __restrict__ ws, int* __restrict__ odd, int chunks) {
   extern __shared__ __align__(16) float pm[];              // B, C [64][132]
   constexpr int LD = SN + 4;
   const int c = blockIdx.x, g = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
@@ -104,7 +105,7 @@ __global__ void __launch_bounds__(256) ssd_prepare_kernel(SsdScanParams p, uint8
   const float* src = p.xBC + ((long long)b * p.T + c * SQ) * Cd + inner + g * SN;
   bool bad = false;
 #pragma unroll 4
-  for (int i = tid; i < 2 * SQ * SN / 8; i += 256) {       // 8 columns of a token
+  for (int i = tid; i < 2 * SQ * SN / 8; i += SP_THREADS) {       // 8 columns of a token
     const int which = i >> 10, t = (i >> 4) & 63, n0 = (i & 15) * 8;
     float v[8] = {};
     if (t < n) {
@@ -122,37 +123,34 @@ __global__ void __launch_bounds__(256) ssd_prepare_kernel(SsdScanParams p, uint8
   }
   const int any = __syncthreads_or(bad);
   if (tid == 0) odd[slot] = any;
-  // G[t][s], stored [s / 4][t][4]; 4 x 4 outputs of a thread, sums over 16 columns added up in order
+  // G[t][s], stored [s / 4][t][4]; 2 x 4 outputs of a thread (lanes along t: their rows of C miss each other's banks), sums over 16 columns added up in order
   const float *Bs = pm, *Cs = pm + SQ * LD;
-  const int t0 = (tid & 15) * 4, s0 = (tid >> 4) * 4;
-  float tot[4][4] = {};
-  if (s0 <= t0 + 3) {
+  const int t0 = tid & 31, s0 = (tid >> 5) * 4;
+  float tot[2][4] = {};
 #pragma unroll 1
-    for (int n0 = 0; n0 < SN; n0 += 16) {
-      float acc[4][4] = {};
+  for (int n0 = 0; n0 < SN; n0 += 16) {
+    float acc[2][4] = {};
 #pragma unroll
-      for (int k = 0; k < 16; k += 4) {
-        float4 bv[4], cv[4];
+    for (int k = 0; k < 16; k += 4) {
+      float4 bv[4], cv[2];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          bv[j] = *reinterpret_cast<const float4*>(Bs + (s0 + j) * LD + n0 + k);
-          cv[j] = *reinterpret_cast<const float4*>(Cs + (t0 + j) * LD + n0 + k);
-        }
+      for (int j = 0; j < 4; ++j) bv[j] = *reinterpret_cast<const float4*>(Bs + (s0 + j) * LD + n0 + k);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 2; ++i) cv[i] = *reinterpret_cast<const float4*>(Cs + (t0 + 32 * i) * LD + n0 + k);
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            acc[i][j] = fmaf(cv[i].w, bv[j].w, fmaf(cv[i].z, bv[j].z, fmaf(cv[i].y, bv[j].y, fmaf(cv[i].x, bv[j].x, acc[i][j]))));
-      }
+      for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) tot[i][j] += acc[i][j];
+        for (int j = 0; j < 4; ++j)
+          acc[i][j] = fmaf(cv[i].w, bv[j].w, fmaf(cv[i].z, bv[j].z, fmaf(cv[i].y, bv[j].y, fmaf(cv[i].x, bv[j].x, acc[i][j]))));
     }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) tot[i][j] += acc[i][j];
   }
   float4* G = reinterpret_cast<float4*>(img + 2 * S_IMG);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) G[(s0 >> 2) * SQ + t0 + i] = make_float4(tot[i][0], tot[i][1], tot[i][2], tot[i][3]);
+  for (int i = 0; i < 2; ++i) G[(s0 >> 2) * SQ + t0 + 32 * i] = make_float4(tot[i][0], tot[i][1], tot[i][2], tot[i][3]);
 }
 
 // ---- scan ------------------------------------------------------------------------------------------------------------------------
@@ -687,7 +685,7 @@ void ssd_chunk_launch(const SsdScanParams& p, void* workspace, bool lp, cudaStre
     if (cudaFuncSetAttribute(ssd_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PREP_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SC_SMEM) != cudaSuccess)
       throw std::runtime_error("ssd scan: shared memory size refused");
-    ssd_prepare_kernel<<<dim3(a.chunks, p.G, p.B), 256, PREP_SMEM, st>>>(p, static_cast<uint8_t*>(workspace), const_cast<int*>(a.odd), a.chunks);
+    ssd_prepare_kernel<<<dim3(a.chunks, p.G, p.B), SP_THREADS, PREP_SMEM, st>>>(p, static_cast<uint8_t*>(workspace), const_cast<int*>(a.odd), a.chunks);
     launch_pdl(kernel, dim3(p.nh / 2, p.B), dim3(SC_THREADS), SC_SMEM, st, a);
   };
   if (lp) go(ssd_chunk_kernel<__nv_bfloat16>); else go(ssd_chunk_kernel<float>);
