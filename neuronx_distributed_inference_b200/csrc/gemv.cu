@@ -101,21 +101,21 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const __nv_bfloat16* __res
 }
 
 // Many rows: WR warps per row, the row in registers as it came, eight 16-byte pieces a lane, so that an SM has 128 KB of reads in flight (one block per
-// row: 32 KB).  Bound by HBM and a load's latency; us, here / one block per row, inputs larger than L2: 4096 x 4096 12.8 / 23.6, 4096 x 2048 7.1 / 20.1,
-// 2048 x 6144 10.5 / 14.0, 1024 x 4096 5.4 / 6.1; a warp per row with 16 or 32 pieces a lane: 23.1 and 19.9 for the first and the third.
+// row: 32 KB).  Bound by HBM and a load's latency; us, here / one block per row, inputs larger than L2, launches one after the other: 4096 x 4096 15.2 / 26.0,
+// 4096 x 2048 8.1 / 21.1, 2048 x 6144 12.0 / 16.0, 1024 x 4096 6.8 / 8.3 (0.1 to 0.6 of that for the sums in the other kernel's order); a warp per row with 16
+// or 32 pieces a lane: 23.1 and 19.9 for the first and the third.
 template <int WR>
 __global__ void __launch_bounds__(256, 4) rmsnorm_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res_in, const __nv_bfloat16* __restrict__ w,
                                                               __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ res_out, int rows, int H, float eps,
                                                               float offset) {
   constexpr int NV = 8;
-  __shared__ float part[8];
+  __shared__ float part[8 / WR][8];
   pdl_launch_dependents();
   pdl_wait();
   const int warp = threadIdx.x >> 5, row = blockIdx.x * (8 / WR) + warp / WR, i0 = (warp % WR) * 32 + (threadIdx.x & 31);
   const int nvec = row < rows ? H >> 3 : 0;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * H);
   uint4 v[NV];
-  float acc = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) v[i] = i0 + i * 32 * WR < nvec ? xr[i0 + i * 32 * WR] : make_uint4(0u, 0u, 0u, 0u);
   if (res_in) {
@@ -131,21 +131,29 @@ __global__ void __launch_bounds__(256, 4) rmsnorm_rows_kernel(const __nv_bfloat1
       if (ro) ro[idx] = v[i];
     }
   }
+  // The sums of rmsnorm_kernel, in its order, so that a row has the same bits however many rows a call has: piece i of this lane belongs to that kernel's
+  // thread (i0 + 32 WR i) mod 256, whose warp is warp % WR + WR (i mod NS).
+  constexpr int NS = NV / WR;
+  float s[NS] = {};
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const float f[8] = {bf16lo(v[i].x), bf16hi(v[i].x), bf16lo(v[i].y), bf16hi(v[i].y), bf16lo(v[i].z), bf16hi(v[i].z), bf16lo(v[i].w), bf16hi(v[i].w)};
-    float s = 0.f;                                // sums of eight, added up
 #pragma unroll
-    for (int j = 0; j < 8; ++j) s += f[j] * f[j];
-    acc += s;
+    for (int j = 0; j < 8; ++j) s[i % NS] += f[j] * f[j];
   }
-  acc = warp_sum(acc);
-  if (WR > 1) {
-    if ((threadIdx.x & 31) == 0) part[warp] = acc;
-    __syncthreads();
-    acc = 0.f;
 #pragma unroll
-    for (int i = 0; i < WR; ++i) acc += part[warp / WR * WR + i];
+  for (int i = 0; i < NS; ++i) s[i] = warp_sum(s[i]);
+  float acc = 0.f;
+  if (WR == 1) {
+#pragma unroll
+    for (int i = 0; i < NS; ++i) acc += s[i];
+  } else {
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+      for (int i = 0; i < NS; ++i) part[warp / WR][warp % WR + WR * i] = s[i];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc += part[warp / WR][i];
   }
   const float rstd = rsqrtf(acc / (float)H + eps);
   const uint4* wr = reinterpret_cast<const uint4*>(w);

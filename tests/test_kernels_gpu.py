@@ -41,6 +41,18 @@ def test_rmsnorm_of_many_rows(rows, H):
     test_rmsnorm(rows, H)
 
 
+@pytest.mark.parametrize("H", [8, 264, 2048, 2056, 3200, 4096, 4104, 6144, 8192])
+@pytest.mark.parametrize("with_residual", [False, True])
+def test_rmsnorm_of_a_row_does_not_depend_on_the_number_of_rows(H, with_residual):
+    x, w = torch.randn(1037, H, device=DEV, dtype=torch.bfloat16), torch.randn(H, device=DEV, dtype=torch.bfloat16)
+    r = torch.randn_like(x) if with_residual else None
+    both = lambda a, b: ops.rmsnorm(a, w, 1e-5, residual=b) if with_residual else (ops.rmsnorm(a, w, 1e-5),)          # noqa: E731
+    many = both(x, r)
+    few = [both(x[i:i + 300], None if r is None else r[i:i + 300]) for i in range(0, 1037, 300)]
+    for j, got in enumerate(many):
+        assert torch.equal(got, torch.cat([f[j] for f in few]))
+
+
 @pytest.mark.parametrize("T", [1, 2, 3, 8])
 @pytest.mark.parametrize("N,K", [(4096, 4096), (6144, 4096), (1000 * 16, 2048), (4096, 14336), (512, 512), (40, 256),
                                  (3072, 4096), (64128, 4096), (4096, 7168), (4096, 2048), (4096, 1792), (768, 4096), (4096, 320), (400, 512)])
