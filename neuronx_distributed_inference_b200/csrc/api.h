@@ -145,6 +145,7 @@ void moe_decode_launch(const void* x, const void* w_gate_up, const void* w_down,
                        float* y_acc, int T, int topk, int H, int I, int E, int expert_offset, int act /*1 silu*up, 4 clamped gate product*/, float limit,
                        float alpha, int n_sms, cudaStream_t stream);
 
+constexpr int ATT_MAX_ORDER = 64;      // rows that a warp orders in two registers a lane
 struct AttnDecodeParams {
   const void* q;        // [B, T, Hq, D] bf16
   const void* k_cache;  // contiguous [L, Hkv, S, D] or paged [nblk, bs, Hkv, D]
@@ -158,7 +159,7 @@ struct AttnDecodeParams {
   float* ws_ml;            // [B*Hkv, nsplit, R, 2]
   unsigned* tickets;       // [B*Hkv]
   int B, T, Hq, Hkv, D, S, L, nsplit, window, block_size, max_blocks;
-  int part_tiles;          // paged: > 0: 64-key tiles of a part, every row has as many parts as it needs (at most nsplit)
+  int by_length;           // paged, at most ATT_MAX_ORDER rows: the longest rows start first
   float scale;
   // fused prologue (contiguous decode): q unused; q/k/v taken from the QKV projection output
   const void* qkv;        // [B, T, (Hq + 2 Hkv) * D] bf16 or null

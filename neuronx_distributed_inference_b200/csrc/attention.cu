@@ -3,15 +3,15 @@
 
 namespace nxdi {
 
-template <int D, int MODE, int ATT_STAGES>
+template <int D, int MODE, int ATT_STAGES, bool BY_LENGTH>
 __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnArgs p) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
-  attention_body<D, MODE, ATT_STAGES>(p, smem_raw, threadIdx.x, blockIdx.x, blockIdx.y, gridDim.x, 0, true, [] { pdl_wait(); });
+  attention_body<D, MODE, ATT_STAGES, BY_LENGTH>(p, smem_raw, threadIdx.x, blockIdx.x, blockIdx.y, gridDim.x, 0, true, [] { pdl_wait(); });
 }
 
-template <int D, int MODE, int ATT_STAGES>
+template <int D, int MODE, int ATT_STAGES, bool BY_LENGTH = false>
 static void launch_attn(const AttnArgs& a, dim3 grid, cudaStream_t stream) {
-  auto kern = attention_kernel<D, MODE, ATT_STAGES>;
+  auto kern = attention_kernel<D, MODE, ATT_STAGES, BY_LENGTH>;
   // + this step's K/V rows (fused decode: [2][T][D], patched into the resident tiles)
   const size_t extra = (MODE == ATTN_DECODE && a.qkv != nullptr) ? (size_t)2 * a.T * D * sizeof(__nv_bfloat16) : 0;
   const size_t smem = (size_t)(64 * D + 2 * ATT_STAGES * 64 * D) * sizeof(__nv_bfloat16) + extra;
@@ -41,7 +41,6 @@ void attention_decode_launch(const AttnDecodeParams& p, cudaStream_t stream) {
   a.B = p.B; a.T = p.T; a.Hq = p.Hq; a.Hkv = p.Hkv; a.S = p.S; a.L = p.L; a.nsplit = p.nsplit; a.window = p.window;
   a.block_size = p.block_size; a.max_blocks = p.max_blocks;
   a.page_shift = -1;
-  a.part_tiles = p.part_tiles;
   for (int s = 0; s < 31; ++s)
     if (p.block_size == 1 << s) a.page_shift = s;
   a.scale_log2 = p.scale * kLog2e;
@@ -55,10 +54,14 @@ void attention_decode_launch(const AttnDecodeParams& p, cudaStream_t stream) {
   a.norm_eps = p.norm_eps;
   a.prof = (grid_fits_prof(p.B * p.Hkv * p.nsplit)) ? prof_slot_ptr(prof_next_slot()) : nullptr;
   if (p.T * (p.Hq / p.Hkv) > 64) throw std::runtime_error("attention_decode: T * group size must be <= 64");
-  dim3 grid(p.B * p.Hkv, p.nsplit);
+  const dim3 grid = p.by_length ? dim3(p.Hkv, p.nsplit, p.B) : dim3(p.B * p.Hkv, p.nsplit);
   const bool paged = p.block_table != nullptr;
   const bool deep = p.nsplit == 1;  // short context, single split: latency bound -> deep prefetch
-  if (p.D == 128) {
+  if (paged && p.by_length) {
+    if (p.D == 128) { if (deep) launch_attn<128, ATTN_PAGED, 3, true>(a, grid, stream); else launch_attn<128, ATTN_PAGED, 2, true>(a, grid, stream); }
+    else if (p.D == 64) { if (deep) launch_attn<64, ATTN_PAGED, 3, true>(a, grid, stream); else launch_attn<64, ATTN_PAGED, 2, true>(a, grid, stream); }
+    else throw std::runtime_error("attention_decode: head_dim must be 64 or 128");
+  } else if (p.D == 128) {
     if (paged) { if (deep) launch_attn<128, ATTN_PAGED, 3>(a, grid, stream); else launch_attn<128, ATTN_PAGED, 2>(a, grid, stream); }
     else { if (deep) launch_attn<128, ATTN_DECODE, 3>(a, grid, stream); else launch_attn<128, ATTN_DECODE, 2>(a, grid, stream); }
   } else if (p.D == 64) {

@@ -41,7 +41,6 @@ struct AttnArgs {
   unsigned* tickets;
   int B, T, Hq, Hkv, S, L, nsplit, window, block_size, max_blocks;
   int page_shift;  // paged: log2(block_size), -1 when it is no power of two
-  int part_tiles;  // paged: > 0: key tiles of a part, a row has as many parts as it needs (at most nsplit); 0: nsplit equal parts of every row
   float scale_log2;
   // fused decode prologue (ATTN_DECODE only): q/k/v come straight from the QKV projection; per-head RMSNorm + RoPE are
   // applied here, the new K/V rows are written to the cache by this CTA before it reads the cache
@@ -71,7 +70,8 @@ __device__ __forceinline__ int swz(int row, int chunk) {  // element offset of a
 // coordinates in the (batch x kv-head, split) grid, `bar_id` the named barrier of the group (0 == __syncthreads for a
 // 128-thread CTA), `standalone` whether the programmatic-dependent-launch trigger belongs to this code; `wait_dep()` blocks until the
 // producer of q / qkv has finished (everything before it only touches step inputs and cache rows of earlier steps).
-template <int D, int MODE, int ATT_STAGES, class WaitDep>
+// BY_LENGTH (paged, at most ATT_MAX_ORDER rows, grid (kv head, part, rank)): the longest rows start first.
+template <int D, int MODE, int ATT_STAGES, bool BY_LENGTH = false, class WaitDep>
 __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_raw, const int tid, const int bx, const int by,
                                                const int gdx, const int bar_id, const bool standalone, WaitDep&& wait_dep) {
   constexpr int CH = D / 8;  // 16-byte chunks per row
@@ -105,8 +105,8 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
   if (!fused) wait_dep();
 
   // ---- work decomposition ----------------------------------------------------------------------------
-  int b, kvh, split = 0, R, qh0 = 0, tok0 = 0;
-  if (MODE == ATTN_PREFILL) {
+  int b, kvh, split = 0, R, qh0 = 0, tok0 = 0, last = 0;
+  if constexpr (MODE == ATTN_PREFILL) {
     const int n_qt = (p.T + 63) / 64;
     const int qt = n_qt - 1 - (int)(bx % n_qt);  // heavy (late) tiles first
     const int bh = bx / n_qt;
@@ -115,6 +115,30 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
     kvh = qh0 / G;
     tok0 = qt * 64;
     R = min(64, p.T - tok0);
+  } else if constexpr (BY_LENGTH) {
+    // rows in eight classes of length, the longest class first; every warp finds its row for itself
+    const int r0 = lane < p.B ? p.positions[lane * p.T + p.T - 1] : -1, r1 = lane + 32 < p.B ? p.positions[(lane + 32) * p.T + p.T - 1] : -1;
+    const int most = max(max(__reduce_max_sync(0xffffffffu, r0), __reduce_max_sync(0xffffffffu, r1)), 0);
+    const float to_class = 8.f / ((float)most + 1.f);
+    const int c0 = lane < p.B ? min((int)((float)max(r0, 0) * to_class), 7) : -1, c1 = lane + 32 < p.B ? min((int)((float)max(r1, 0) * to_class), 7) : -1;
+    int k = blockIdx.z;
+    b = 0;
+#pragma unroll 1
+    for (int c = 7; c >= 0; --c) {
+      const unsigned m0 = __ballot_sync(0xffffffffu, c0 == c), m1 = __ballot_sync(0xffffffffu, c1 == c);
+      const int n0 = __popc(m0), n1 = __popc(m1);
+      if (k < n0 + n1) {
+        const unsigned m = k < n0 ? m0 : m1;
+        const unsigned hit = __ballot_sync(0xffffffffu, (m >> lane & 1u) && __popc(m & ((1u << lane) - 1u)) == (k < n0 ? k : k - n0));
+        b = __ffs(hit) - 1 + (k < n0 ? 0 : 32);
+        break;
+      }
+      k -= n0 + n1;
+    }
+    last = __shfl_sync(0xffffffffu, b < 32 ? r0 : r1, b & 31);
+    kvh = bx;
+    split = by;
+    R = p.T * G;
   } else {
     b = bx / p.Hkv;
     kvh = bx % p.Hkv;
@@ -131,7 +155,7 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
   int pos_max = -1, pos_min = 0x7fffffff;
   for (int r = tid; r < 64; r += ATT_THREADS) {
     int ps = -1;
-    if (r < R) ps = (MODE == ATTN_PREFILL) ? (p.causal ? tok0 + r : p.T - 1) : p.positions[b * p.T + r / G];
+    if (r < R) ps = (MODE == ATTN_PREFILL) ? (p.causal ? tok0 + r : p.T - 1) : BY_LENGTH && p.T == 1 ? last : p.positions[b * p.T + r / G];
     s_pos[r] = ps;
   }
   group_sync();
@@ -151,11 +175,7 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
   int t_lo = 0;
   if (p.window > 0) t_lo = max(0, pos_min - p.window + 1) / ATT_TILE;
   const int span = max(nt - t_lo, 0);
-  // parts of this row
-  const bool sized = MODE == ATTN_PAGED && p.part_tiles > 0;
-  const int n_parts = sized ? max(1, (span + p.part_tiles - 1) / p.part_tiles) : p.nsplit;
-  if (sized && split >= n_parts) return;
-  const int tps = (span + n_parts - 1) / n_parts;
+  const int tps = (span + p.nsplit - 1) / p.nsplit;
   const int t_beg = t_lo + split * tps;
   const int t_end = min(nt, t_beg + tps);
 
@@ -470,8 +490,8 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
   }
   group_sync();
 
-  const int bh = (MODE == ATTN_PREFILL) ? 0 : bx;
-  const bool direct = (MODE == ATTN_PREFILL) || n_parts == 1;
+  const int bh = (MODE == ATTN_PREFILL) ? 0 : BY_LENGTH ? b * p.Hkv + kvh : bx;
+  const bool direct = (MODE == ATTN_PREFILL) || p.nsplit == 1;
   const int ws_rows = p.T * G;               // rows of a piece in the workspace
   // per-row merge factors once (row max over the KS key-split warps, rescale factor of each, denominator incl. the sink):
   // sF[k2][r] = exp2(m_k2 - M) (/ L when written directly), so the element loop below is KS multiply-adds per output
@@ -539,6 +559,7 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
   if (direct) return;
 
   // ---- split-KV combine by the last-arriving CTA of this (batch, kv head) ------------------------------------
+  const int n_parts = p.nsplit;
   __threadfence();
   group_sync();
   if (tid == 0) s_last = (atomicAdd(&p.tickets[bh], 1u) == (unsigned)(n_parts - 1));

@@ -651,22 +651,20 @@ at::Tensor rope_attention_decode(const at::Tensor& qkv, const at::Tensor& cos, c
 //   128 pairs: 500 keys 21 / 22 / 28 / 37         4096: 69 / 57 / 57 / 61         32768: 455 / 301 / 264 / 229 / 223
 //   384 pairs: 500 keys 29 / 37 / 49 / 74         4096: 103 / 98 / 100 / 117      32768: 639 / 537 / 475 / 453          1536 pairs, 4096 keys: 256 / 274 / 312 / 391
 // Head size 64 has its minima at the same numbers (32768 keys: 1 pair 303 / 172 / 92 / 52 / 33 / 29 / 27 / 25, 32 pairs 309 / 186 / 104 / 70 / 55 / 59 / 59 / 66).
-// From 96 pairs on the parts are of one size, about 1024 keys, and a row has as many as it needs: with equal parts of every row the longest rows' parts
-// finished last.  us, parts of 512 / 768 / 1024 / 1536 / 2048 keys, equal parts as above; contexts of one request at the limit, the others anywhere up to it:
-//   384 pairs, 4096 keys: 95 / 87 / 83 / 85 / 83, 91    320, 3000: 66 / 61 / 57 / 59 / 59, 59    192, 4096: 52 / 48 / 50 / 53 / 48, 55
-//   128 pairs, 4096 keys: 37 / 41 / 41 / 36 / 45, 43    768, 2000, head size 64: 56 / 55 / 51 / 51 / 51, 56    1536, 4096: 327 / 298 / 275 / 263 / 264, 256 (one part)
-struct PagedParts {
-  int most, tiles;          // parts of the longest row; 64-key tiles of a part, 0: equal parts of every row
-};
-static PagedParts paged_parts(int pairs, int max_keys) {
+// With 96 to 1023 pairs and up to 64 rows the longest rows start first (eight classes of length): in the order of the rows the parts of the longest ones finished
+// last.  us, by length / in their order, at 96, 128, 256, 384 and 512 pairs (8 kv heads; 4 at 256 and 128), head size 128:
+//   500 .. 8000 keys: 61 / 75, 63 / 78, 107 / 144, 133 / 157, 210 / 225    1 .. 4096: 34 / 38, 40 / 46, 59 / 73, 86 / 102, 106 / 116
+//   1 .. 1500: 20 / 20, 27 / 28, 37 / 41, 52 / 51, 62 / 62    all 4096: 60 / 59, 63 / 63, 104 / 104, 152 / 153, 199 / 199    all 300: 19.5 / 17.9, 21.0 / 20.0, 24.6 / 22.5, 33 / 32, 41.5 / 41.0
+// Every CTA finds its row for itself, which costs 0.5 us; an exact rank from keys in shared memory cost 2 .. 5 us.  More rows than a warp holds in two registers:
+// in their order.  Parts of one size for all rows (a row as many as it needs) were as fast, but short rows then had fewer parts and errors against 64 bits
+// up to 2 % larger: the largest probability of a part is exactly 1 and takes no rounding.
+static int paged_nsplit(int pairs, int max_keys) {
   const int tiles = std::max(1, (max_keys + 63) / 64);
-  if (pairs >= 1024) return {1, 0};
-  if (pairs >= 96) {
-    const int n = std::max(1, std::min(16, (tiles + 8) / 16));
-    return {n, (tiles + n - 1) / n};
-  }
+  if (pairs >= 1024) return 1;
+  if (pairs >= 256) return max_keys >= 3072 ? 2 : 1;
+  if (pairs >= 96) return std::max(1, std::min(4, max_keys / 1024));
   const int some = std::min(tiles, pairs > 32 && max_keys <= 8192 ? 4 : pairs > 8 ? 8 : 16);
-  return {std::max(some, std::min({64, 2 * 148 / pairs, max_keys / 512})), 0};       // long rows: two CTAs per SM of at least 512 keys
+  return std::max(some, std::min({64, 2 * 148 / pairs, max_keys / 512}));       // long rows: two CTAs per SM of at least 512 keys
 }
 
 at::Tensor paged_attention_decode(const at::Tensor& q, const at::Tensor& k_cache, const at::Tensor& v_cache,
@@ -687,8 +685,8 @@ at::Tensor paged_attention_decode(const at::Tensor& q, const at::Tensor& k_cache
   p.sinks = sinks.has_value() ? sinks->data_ptr<float>() : nullptr;
   p.B = B; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.S = 0; p.L = 0; p.window = window; p.scale = (float)scale;
   p.block_size = bs; p.max_blocks = block_table.size(1);
-  const PagedParts parts = paged_parts(B * Hkv, p.max_blocks * bs);
-  p.nsplit = parts.most; p.part_tiles = parts.tiles;
+  p.nsplit = paged_nsplit(B * Hkv, p.max_blocks * bs);
+  p.by_length = B > 1 && B <= ATT_MAX_ORDER && B * Hkv >= 96 && B * Hkv < 1024 ? 1 : 0;
   const int64_t rows = (int64_t)B * Hkv * p.nsplit * T * (Hq / Hkv);
   auto& ws = scratch(q.device(), rows * (D + 2), 0, (int64_t)B * Hkv);
   p.ws_o = ws.f.data_ptr<float>();

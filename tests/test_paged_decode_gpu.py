@@ -65,3 +65,38 @@ def test_parts_of_one_size(Hkv, window, most, D):
         for b in range(0, B, 1 if most <= 4096 else 17):
             want = ref.paged_attention_decode(q[b:b + 1].float(), kc.float(), vc.float(), table[b:b + 1], pos[b:b + 1], D ** -0.5, window or None, None)
             assert ((got[b:b + 1].float() - want).norm() / want.norm()).item() < 4e-3
+
+
+@pytest.mark.parametrize("Hkv,B", [(8, 12), (8, 33), (1, 100)])
+def test_parts_do_not_depend_on_the_width_of_the_table(Hkv, B):
+    """A serving layer may pass its full table: rows of a few thousand keys are cut as under a table of their own length."""
+    page, D, n, Hq = 32, 128, 4096 // 32, 4 * Hkv
+    kc, vc = (torch.randn(B * n, page, Hkv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    table = torch.randperm(B * n, device="cuda").view(B, n).int()
+    ctx = [(4096, 1, 1025, 3000, 2049, 1024)[b % 6] for b in range(B)]
+    q, pos = torch.randn(B, 1, Hq, D, device="cuda", dtype=torch.bfloat16), torch.tensor(ctx, device="cuda", dtype=torch.int32).view(B, 1) - 1
+    want = ops.paged_attention_decode(q, kc, vc, table, pos, D ** -0.5)
+    for slots in (32768, 131072):
+        wide = torch.zeros(B, slots // page, device="cuda", dtype=torch.int32)
+        wide[:, :n] = table
+        assert torch.equal(ops.paged_attention_decode(q, kc, vc, wide, pos, D ** -0.5), want)
+
+
+@pytest.mark.parametrize("B,T,Hkv,window", [(13, 1, 8, 0), (96, 1, 1, 0), (129, 2, 1, 100), (256, 1, 1, 0), (257, 1, 1, 0), (50, 3, 2, 700)])
+def test_order_of_the_rows(B, T, Hkv, window):
+    """The longest rows start first from 96 (row, kv head) pairs on: a row's bits do not depend on its place, equal lengths and empty rows among them."""
+    page, D, longest, Hq = 64, 64, 3500, 4 * Hkv
+    n = -(-longest // page)
+    kc, vc = (torch.randn(3 * n, page, Hkv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    table = torch.stack([torch.randperm(3 * n, device="cuda")[:n] for _ in range(B)]).int()
+    ctx = [(longest, 1, 700, 1200, 700, 64, 2049)[b % 7] for b in range(B)]
+    pos = torch.tensor(ctx, device="cuda", dtype=torch.int32).view(B, 1) - T + torch.arange(T, device="cuda", dtype=torch.int32)
+    q = torch.randn(B, T, Hq, D, device="cuda", dtype=torch.bfloat16)
+    got = ops.paged_attention_decode(q, kc, vc, table, pos, D ** -0.5, window or None)
+    i = torch.randperm(B, device="cuda")
+    again = ops.paged_attention_decode(q[i].contiguous(), kc, vc, table[i].contiguous(), pos[i].contiguous(), D ** -0.5, window or None)
+    assert torch.equal(again, got[i])
+    for b in range(0, B, 11):
+        if ctx[b] >= T:
+            want = ref.paged_attention_decode(q[b:b + 1].float(), kc.float(), vc.float(), table[b:b + 1], pos[b:b + 1], D ** -0.5, window or None, None)
+            assert ((got[b:b + 1].float() - want).norm() / want.norm()).item() < 4e-3
