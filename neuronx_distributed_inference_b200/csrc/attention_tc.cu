@@ -16,8 +16,9 @@
 //   200 clocks for each hand-over.  One 8192-token prompt, 32 / 8 heads x 128: 0.44 ms alone (1.25 PFLOP/s).  Before: 0.495 ms; of that, 28 us from
 //   the MMA warp's code (fa_umma), 27 us from the halves of P, 7 us from the mixed-type sums (fa_add_bf16x2), 20 us from masks outside the tiles
 //   that need none.  3 x 1000 tokens of head size 64, window 128: 24 us, 30 before.
-//   A soft cap (tanh) needs eight more fp32 pair operations per pair of scores, which bound those tiles; they run beside the exponentials and end in the
-//   exponent's multiply-add, the maximum is taken before the cap.  Three portions with cap, gate and window: 255 us; 267 with the cap as a pass of its own.
+//   A soft cap (tanh) needs nine more fp32 pair operations per pair of scores; they run beside the exponentials, the maximum is taken before the cap and capped
+//   alone.  Three portions with cap, gate and window: 257 us; 267 with the cap as a pass of its own, 255 with the cap's size in the polynomial's coefficients
+//   (other bits for no gain in error).
 //   Tried and slower: 64-key tiles with two score buffers per query tile (478 us: both tiles' softmax phases fall together, and a hand-over costs as
 //   much per 64 keys); sixteen softmax warps with half a row per thread (482 us); a share of the exponentials as polynomials on the FMA pipe (2 of 16: no
 //   gain, 4 of 16: 1 % slower: the fp32 pair operations cost more clocks than the exponentials they replace); the maximum beside the exponentials of
@@ -169,33 +170,19 @@ __device__ __forceinline__ uint64_t fa_mul2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
-__device__ __forceinline__ uint64_t fa_add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
 // s_lo, s_hi += the two bf16 halves of w
 __device__ __forceinline__ void fa_add_bf16x2(float& s_lo, float& s_hi, uint32_t w) {
   asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.bf16 %0, l, %0;\n\tadd.rn.f32.bf16 %1, h, %1;\n\t}" : "+f"(s_lo), "+f"(s_hi) : "r"(w));
 }
-// Soft cap: c tanh(x) on |x| <= 1 as x times a polynomial in x^2 (weighted least squares on Chebyshev nodes, relative error 1.7e-7 with fp32 arithmetic), c in
-// its coefficients
-struct FaCap {
-  uint64_t k[7];
-  __device__ __forceinline__ explicit FaCap(float c) {
-    const float t[7] = {0.00104102155f, -0.00620337576f, 0.0202899761f, -0.0534570292f, 0.13325204f, -0.333328396f, 0.99999994f};
+// tanh on |x| <= 1: x times a polynomial in x^2 (weighted least squares on Chebyshev nodes, relative error 1.7e-7 with fp32 arithmetic)
+__device__ __forceinline__ uint64_t fa_tanh2_small(uint64_t x) {
+  const float t[7] = {0.00104102155f, -0.00620337576f, 0.0202899761f, -0.0534570292f, 0.13325204f, -0.333328396f, 0.99999994f};
+  const uint64_t u = fa_mul2(x, x);
+  uint64_t r = fa_pack2(t[0], t[0]);
 #pragma unroll
-    for (int i = 0; i < 7; ++i) k[i] = fa_pack2(t[i] * c, t[i] * c);
-  }
-  // c tanh(x) + add
-  __device__ __forceinline__ uint64_t operator()(uint64_t x, uint64_t add) const {
-    const uint64_t u = fa_mul2(x, x);
-    uint64_t r = k[0];
-#pragma unroll
-    for (int i = 1; i < 7; ++i) r = fa_fma2(r, u, k[i]);
-    return fa_fma2(x, r, add);
-  }
-};
+  for (int i = 1; i < 7; ++i) r = fa_fma2(r, u, fa_pack2(t[i], t[i]));
+  return fa_mul2(x, r);
+}
 
 template <int D, int NX>
 struct FaShape {
@@ -439,7 +426,6 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
     const int w_pos = ctx + t_tile + 32 * qd;
     const int up_min = p.causal ? min(w_pos, end - 1) : end - 1, up_max = p.causal ? min(w_pos + 31, end - 1) : end - 1;
     const int lb_min = reach(w_pos), lb_max = reach(w_pos + 31);
-    const FaCap cap(CAP ? p.softcap * FA_LOG2E : 0.f);
     const float hs = p.head_scale ? p.scale * p.head_scale[h] : p.scale;
     float m_run = -INFINITY, l_run = 0.f;
     auto tile = [&](auto masked, int i, int key0) {
@@ -517,8 +503,8 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
       float mx = (mx_raw == -INFINITY) ? -INFINITY : mx_raw * scl;
       if (CAP) {
         float t, unused;
-        fa_unpack2(cap(fa_pack2(mx_raw, mx_raw), 0ull), t, unused);
-        if (mx > -INFINITY) mx = fabsf(mx_raw) <= 1.f ? t : tanhf(mx_raw) * scl;
+        fa_unpack2(fa_tanh2_small(fa_pack2(mx_raw, mx_raw)), t, unused);
+        if (mx > -INFINITY) mx = (fabsf(mx_raw) <= 1.f ? t : tanhf(mx_raw)) * scl;
       }
       const bool grow = mx > m_run + SLACK || (m_run == -INFINITY && mx > -INFINITY);
       const float m_new = grow ? mx : m_run;
@@ -562,7 +548,7 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
           for (int e = 0; e < 64; e += 2) {
             const float s0 = __uint_as_float(v[64 * c + e]), s1 = __uint_as_float(v[64 * c + e + 1]);
             float a, bb;
-            fa_unpack2(cap(fa_pack2(s0, s1), neg2), a, bb);
+            fa_unpack2(fa_fma2(fa_tanh2_small(fa_pack2(s0, s1)), scl2, neg2), a, bb);
             if (!(fabsf(s0) <= 1.f)) a = fmaf(tanhf(s0), scl, neg_m);
             if (!(fabsf(s1) <= 1.f)) bb = fmaf(tanhf(s1), scl, neg_m);
             if (MASKED) {
@@ -578,7 +564,7 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
           for (int e = 0; e < 64; e += 2) {
             const uint64_t v2 = fa_pack2(__uint_as_float(v[64 * c + e]), __uint_as_float(v[64 * c + e + 1]));
             float a, bb;
-            fa_unpack2(CAP ? cap(v2, neg2) : fa_fma2(v2, scl2, neg2), a, bb);
+            fa_unpack2(fa_fma2(CAP ? fa_tanh2_small(v2) : v2, scl2, neg2), a, bb);
             if (CAP && MASKED) {                         // the cap of a masked score is no -inf
               if (!(see[2 * c + (e >> 5)] & (1u << (e & 31)))) a = -INFINITY;
               if (!(see[2 * c + (e >> 5)] & (2u << (e & 31)))) bb = -INFINITY;
@@ -596,7 +582,7 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
         __syncwarp();
         if (lane == 0) mbar_arrive(c == 0 ? &p_half[x] : &p_full[x]);
       }
-      l_run += (ls[0] + ls[1]) + (ls[2] + ls[3]);
+      l_run += (ls[0] + ls[2]) + (ls[1] + ls[3]);
     };
     for (int i = 0; i < n_tiles; ++i) {
       const int key0 = key_at(i);
@@ -743,7 +729,7 @@ void attention_prefill_tc_launch(const void* q, const void* k, const void* v, vo
 
 // Prompt portions over a paged cache.  Sizes this kernel takes: keys and values of one size, 64 or 128, rows on 16-byte boundaries, pages of
 // 2^k >= 8 tokens (smaller ones would break the 8-row swizzle atoms), no distance term; the rest is paged_window_attention_mma_kernel's.
-// 3 rows of up to 1024 tokens over contexts up to 3000, 32 / 8 heads x 128, window 2048, cap, gate: 0.255 ms, mma.sync kernel 0.89 ms.
+// 3 rows of up to 1024 tokens over contexts up to 3000, 32 / 8 heads x 128, window 2048, cap, gate: 0.257 ms, mma.sync kernel 0.89 ms.
 bool paged_attention_tc_supported(const WindowAttnParams& p, bool lp) {
   return lp && p.T >= 16 && p.maps != 2 && p.slopes == nullptr && p.D == p.Dv && (p.D == 64 || p.D == 128) && (p.v_rs * 2) % 16 == 0 && p.page >= 8 &&
          (p.page & (p.page - 1)) == 0 && (long long)p.B * p.Hq * ((p.T + FA_ROWS - 1) / FA_ROWS) <= 0x7fffffffLL &&
