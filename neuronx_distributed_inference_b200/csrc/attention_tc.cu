@@ -502,9 +502,11 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
       const float mx_raw = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       float mx = (mx_raw == -INFINITY) ? -INFINITY : mx_raw * scl;
       if (CAP) {
+        // a row that sees keys has a maximum, of scores below fp32's range too: -cap
+        const bool any = !MASKED || (!dead[0] && (see[0] | see[1]) != 0u) || (!dead[1] && (see[2] | see[3]) != 0u);
         float t, unused;
         fa_unpack2(fa_tanh2_small(fa_pack2(mx_raw, mx_raw)), t, unused);
-        if (mx > -INFINITY) mx = (fabsf(mx_raw) <= 1.f ? t : tanhf(mx_raw)) * scl;
+        mx = any ? (fabsf(mx_raw) <= 1.f ? t : tanhf(mx_raw)) * scl : -INFINITY;
       }
       const bool grow = mx > m_run + SLACK || (m_run == -INFINITY && mx > -INFINITY);
       const float m_new = grow ? mx : m_run;

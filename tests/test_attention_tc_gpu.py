@@ -120,3 +120,18 @@ def test_two_tiles_paged(D, cap, Hq, G, mask):
     assert _rel(got, want) < 4e-3
     for b, live in enumerate(n):
         assert not got[b, live:].any()
+
+
+def test_soft_cap_of_scores_below_the_range():
+    """Scores that overflow to -inf are capped to -cap like all others, also where a row sees nothing else in its first tiles."""
+    B, T, Hq, G, D, page = 1, 300, 4, 2, 128, 64
+    q, dirty, _, table, c, m = _paged(B, T, Hq, G, D, page, (0,), (T,))
+    k, v = (t.nan_to_num(0.0) for t in dirty)
+    low = table[0].long().repeat_interleave(page)[:200] * page + torch.arange(page, device=DEV).repeat(5)[:200]
+    q[..., 0] = 1e20
+    k[..., 0] = 0.0
+    k.view(-1, G, D)[low, :, 0] = -1e20
+    for cap in (1.0, 4.0):
+        got = ops.paged_window_attention(q, k, v, table, c, m, D ** -0.5, cap, 0, 0)
+        want = ref.paged_window_attention(q.float(), k.float(), v.float(), table, c, m, D ** -0.5, cap, 0, 0)
+        assert _rel(got, want) < 4e-3
