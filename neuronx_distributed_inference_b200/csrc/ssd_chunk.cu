@@ -78,14 +78,24 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// z / (1 + e^-z) without branches: -z log2(e) in two terms, the reciprocal with one Newton step
-__device__ __forceinline__ float silu_acc(float z) {
-  const float x = fmaxf(z, -87.f), t = x * -1.44269502f, rest = fmaf(x, -1.44269502f, -t) + x * -1.92596303e-8f;
+// z / (1 + e^-z), the reciprocal with one step of Newton's method.  For |z| <= 80 e^-z = 2^t (1 + rest ln 2), t and rest the parts of -z log2(e), which is rounded
+// to two fp32 terms (Cody and Waite's reduction)
+constexpr float SILU_FAST = 80.f;
+__device__ __forceinline__ float silu_fast(float z) {
+  const float t = z * -1.44269502f, rest = fmaf(z, -1.44269502f, -t) + z * -1.92596303e-8f;
   const float d = 1.f + ex2(t) * fmaf(rest, 0.69314718f, 1.f);
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
   r = fmaf(fmaf(-d, r, 1.f), r, r);
   return z * r;
+}
+// any z, from e^-|z|: nothing leaves the range on the way to the definition's values (-inf: not a number)
+__device__ __forceinline__ float silu_any(float z) {
+  const float q = expf(-fabsf(z)), d = 1.f + q;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  r = fmaf(fmaf(-d, r, 1.f), r, r);
+  return fabsf(z) <= SILU_FAST ? silu_fast(z) : (z < 0.f ? z * q : z) * r;
 }
 // byte of a 16-byte piece in a tile of 128-byte rows, SWIZZLE_128B
 __device__ __forceinline__ uint32_t swz(int row, int piece) { return (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
@@ -505,8 +515,16 @@ __global__ void __launch_bounds__(SC_THREADS, 1) ssd_chunk_kernel(const __grid_c
         s[t] = ld_ahead(zt, t < n);
         zt += p.z_st;
       }
+      float big = 0.f;
 #pragma unroll
-      for (int t = 0; t < 32; ++t) s[t] = silu_acc(s[t]);
+      for (int t = 0; t < 32; ++t) big = fmaxf(big, fabsf(s[t]));
+      if (__any_sync(0xffffffffu, big > SILU_FAST)) {
+#pragma unroll
+        for (int t = 0; t < 32; ++t) s[t] = silu_any(s[t]);
+      } else {
+#pragma unroll
+        for (int t = 0; t < 32; ++t) s[t] = silu_fast(s[t]);
+      }
       if (!wait(&sh.intra_done, c)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const bool mine = !is_odd(c);

@@ -65,3 +65,23 @@ def test_values_that_are_not_finite_reach_no_earlier_token_and_no_other_row(wher
     assert at == 0 or rel < 1e-6
     assert not torch.isfinite(got[0, at:]).all()
     assert torch.isfinite(got[0, :, 128:]).all()                                  # heads 2 and 3: another group
+
+
+def test_gate_at_the_ends_of_its_range():
+    """silu(z) from -inf to inf: the outputs are those of z = 30 (whose silu is 30 to 1e-13) times silu(z) / 30.  Bound: the error of a gate, 6 * 2^-24, on both sides;
+    gates below 1e-37 carry the fewer bits of subnormal numbers."""
+    args, sizes = _inputs(2, 1, 64, (64,), torch.float32)
+    args["slots"].fill_(1)
+    inf = float("inf")
+    z = torch.tensor([0.0, -0.0, 1.0, -1.0, 20.0, -20.0, 80.0, -80.0, 86.9, -86.9, 87.1, -87.1, 88.0, -88.0, 100.0, -100.0, 1e4, -1e4, 3e35, -1e38, inf, -inf],
+                     device="cuda")
+    args["xBC"] *= 0.1
+    args["state"].zero_()
+    args["z"] = torch.full_like(args["z"], 30.0)
+    core = _run({k: v.clone() for k, v in args.items()}, sizes).double() / 30.0
+    args["z"] = z.repeat(64 * 128 // len(z) + 1)[:64 * 128].view(1, 64, 128).contiguous()
+    got, zz = _run(args, sizes).double(), args["z"].double()
+    want = core * zz * torch.sigmoid(zz)
+    fin = torch.isfinite(zz)
+    assert ((got - want).abs()[fin] <= 8e-7 * want.abs()[fin] + 1e-37 * core.abs()[fin]).all()
+    assert torch.equal(got[zz == inf], (core * inf)[zz == inf]) and got[zz == -inf].isnan().all()
