@@ -8,8 +8,8 @@
 // (the three left out are below 2^-24 of a term), small ones first, sums in the fp32 accumulators over at most 128 terms; decays, the state and everything
 // around the products stay fp32, the running sum of the exponents is taken in 64 bits (a chunk's exponents reach -200, neighbours differ by 1e-2).
 //
-//   prepare  (chunk, group, row): the parts of B and C as images of their shared-memory tiles, G = C B^T in fp32 on the CUDA cores, and whether any value is
-//            not a number or infinite (64 heads share them)
+//   prepare  (chunk, group, row): the parts of B and C as images of their shared-memory tiles, G = C B^T in fp32 on the CUDA cores, and the largest |G|, infinite
+//            where a value of B or C is large or no number (64 heads share them)
 //   scan     CTA = two heads of a row, chunks in order.  128 rows of the products = (head, channel) = TMEM lanes:
 //              update  W[(h,p)][n]  = X~^T B      A = the parts of dt 2^(cs_end - cs) x in TMEM, B image MN-major           K = 64
 //              inter   I[(h,p)][t]  = S^T C^T     A = the parts of the state in TMEM, C image K-major                       K = 128
@@ -21,8 +21,9 @@
 //   4 rows of 64 23.5 / 37.5, one of 48 23 / 22 (the host); 128 heads in 8 groups, 4 rows of up to 1024 207 / 734.  Error against 64 bits, 4 rows of up to
 //   1024: 1.0e-7, step by step 1.1e-7.  Tried: everything unrolled 217 us (2.3 warps waiting for instructions at every issue); four warps for
 //   the outputs 142; conditional loads of x, z 136 and more (the compiler waits for each).
-//   A chunk with a value that is not finite (or beyond bf16's range) runs step by step in the state's warps: a product with 0 must not spread it to
-//   earlier tokens.
+//   A chunk runs step by step in the state's warps where x, dt x, B, C, the state or a bound of M (largest |G| times dt, and D) is 1e18 or more or no number: a product
+//   with 0 must not spread what is not finite to earlier tokens, and products that the recurrence does not form (C B^T before it meets x, S^T C before S has
+//   decayed) must not leave fp32's range where its own values do not.
 // The chunked form: Dao and Gu, "Transformers are SSMs" (2024), section 6.
 #include <cuda_bf16.h>
 #include <math.h>
@@ -46,7 +47,7 @@ constexpr int S_WS = 2 * S_IMG + S_G;                     // workspace of a (row
 constexpr int SC_THREADS = 768;
 constexpr int W_M = 8, W_OUT = 12, W_MMA = 20, W_COPY = 21, W_STEP = 22;             // first warps of the roles; the state's are 0 .. 7
 constexpr uint32_t TM_I = 0, TM_W = 64, TM_S = 192, TM_X = 384;      // TMEM columns: inter, update / intra, state parts, x~ parts
-constexpr float S_FINITE = 3e38f;
+constexpr float S_LARGE = 1e18f;                          // 128 products of two values below it stay in fp32's range
 
 template <typename T> __device__ __forceinline__ float ldv(const T* p);
 template <> __device__ __forceinline__ float ldv<float>(const float* p) { return *p; }
@@ -102,8 +103,9 @@ __device__ __forceinline__ uint32_t swz(int row, int piece) { return (uint32_t)(
 
 // ---- prepare ---------------------------------------------------------------------------------------------------------------------
 constexpr int SP_THREADS = 512;
-__global__ void __launch_bounds__(SP_THREADS) ssd_prepare_kernel(SsdScanParams p, uint8_t* __restrict__ ws, int* __restrict__ odd, int chunks) {
+__global__ void __launch_bounds__(SP_THREADS) ssd_prepare_kernel(SsdScanParams p, uint8_t* __restrict__ ws, float* __restrict__ most_g, int chunks) {
   extern __shared__ __align__(16) float pm[];              // B, C [64][132]
+  __shared__ unsigned most;                                // as bits (of positive numbers: in order)
   constexpr int LD = SN + 4;
   const int c = blockIdx.x, g = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
   pdl_launch_dependents();
@@ -113,6 +115,7 @@ __global__ void __launch_bounds__(SP_THREADS) ssd_prepare_kernel(SsdScanParams p
   uint8_t* img = ws + slot * S_WS;
   const int inner = p.nh * SP, Cd = inner + 2 * p.G * SN;
   const float* src = p.xBC + ((long long)b * p.T + c * SQ) * Cd + inner + g * SN;
+  if (tid == 0) most = 0u;
   bool bad = false;
 #pragma unroll 4
   for (int i = tid; i < 2 * SQ * SN / 8; i += SP_THREADS) {       // 8 columns of a token
@@ -126,13 +129,12 @@ __global__ void __launch_bounds__(SP_THREADS) ssd_prepare_kernel(SsdScanParams p
     float* row = pm + (which * SQ + t) * LD + n0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      bad |= !(fabsf(v[k]) < S_FINITE);
+      bad |= !(fabsf(v[k]) < S_LARGE);
       row[k] = v[k];
     }
     store_parts(img + which * S_IMG + (n0 >> 6) * S_BLK + swz(t, (n0 & 63) >> 3), S_PART, v);
   }
-  const int any = __syncthreads_or(bad);
-  if (tid == 0) odd[slot] = any;
+  __syncthreads();
   // G[t][s], stored [s / 4][t][4]; 2 x 4 outputs of a thread (lanes along t: their rows of C miss each other's banks), sums over 16 columns added up in order
   const float *Bs = pm, *Cs = pm + SQ * LD;
   const int t0 = tid & 31, s0 = (tid >> 5) * 4;
@@ -158,16 +160,25 @@ __global__ void __launch_bounds__(SP_THREADS) ssd_prepare_kernel(SsdScanParams p
 #pragma unroll
       for (int j = 0; j < 4; ++j) tot[i][j] += acc[i][j];
   }
+  float big = 0.f;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) big = fmaxf(big, fabsf(tot[i][j]));
+  const unsigned m = __reduce_max_sync(0xffffffffu, bad ? 0x7f800000u : __float_as_uint(big));
+  if ((tid & 31) == 0) atomicMax(&most, m);
   float4* G = reinterpret_cast<float4*>(img + 2 * S_IMG);
 #pragma unroll
   for (int i = 0; i < 2; ++i) G[(s0 >> 2) * SQ + t0 + 32 * i] = make_float4(tot[i][0], tot[i][1], tot[i][2], tot[i][3]);
+  __syncthreads();
+  if (tid == 0) most_g[slot] = __uint_as_float(most);
 }
 
 // ---- scan ------------------------------------------------------------------------------------------------------------------------
 struct ScanArgs {
   SsdScanParams p;
   const uint8_t* ws;
-  const int* odd;
+  const float* most_g;
   int chunks;
   unsigned* wait_word;
 };
@@ -330,7 +341,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) ssd_chunk_kernel(const __grid_c
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           v[i] = S[i0 + i];
-          bad |= !(fabsf(v[i]) < S_FINITE);
+          bad |= !(fabsf(v[i]) < S_LARGE);
         }
         put_parts(tmem + lanes + TM_S + hf * 32 + i0 / 2, 64, v);
       }
@@ -360,14 +371,14 @@ __global__ void __launch_bounds__(SC_THREADS, 1) ssd_chunk_kernel(const __grid_c
     auto put_x = [&](int c) {                              // the parts of x~ of chunk c
       if (!wait(&sh.dt_ready[c & 1], c >> 1)) return false;
       const ChunkSteps& st = sh.st[c & 1];
-      bool bad = lane == 0 && a.odd[((long long)b * a.chunks + c) * p.G + g] != 0;
+      bool bad = false;
 #pragma unroll
       for (int t0 = 0; t0 < 32; t0 += 8) {
         float v[8];
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
           v[t] = x[t0 + t] * st.w[hl][hf * 32 + t0 + t];
-          bad |= !(fabsf(x[t0 + t]) < S_FINITE && fabsf(v[t]) < S_FINITE);
+          bad |= !(fabsf(x[t0 + t]) < S_LARGE && fabsf(v[t]) < S_LARGE);
         }
         put_parts(tmem + lanes + TM_X + hf * 16 + t0 / 2, 32, v);
       }
@@ -625,9 +636,11 @@ __global__ void __launch_bounds__(SC_THREADS, 1) ssd_chunk_kernel(const __grid_c
       const int hl = warp - W_STEP, h = h0 + hl;
       const T* dtp = (const T*)p.dt_raw + (long long)b * p.dt_sb + h;
       const double negA = -(double)expf(p.A_log[h]) * 1.4426950408889634;      // to log2
-      const float bias = p.dt_bias[h];
+      const float bias = p.dt_bias[h], Dh = fabsf(p.D_skip[h]);
+      const float* most_g = a.most_g + (long long)b * a.chunks * p.G + g;
       for (int c = 0; c < nc; ++c) {
         const int n = min(SQ, n_tok - c * SQ);
+        const float g_most = most_g[(long long)c * p.G];
         float dt[2];
         double cs[2];
 #pragma unroll
@@ -664,6 +677,8 @@ __global__ void __launch_bounds__(SC_THREADS, 1) ssd_chunk_kernel(const __grid_c
           st.e[hl][t] = exp2f(hi) * fmaf(lo, 0.69314718f, 1.f);
           st.w[hl][t] = dt[k] * exp2f((float)(end - cs[k]));
         }
+        // |M| <= |G| dt + |D|
+        if (!(fmaf(g_most, dt[0], Dh) < S_LARGE && fmaf(g_most, dt[1], Dh) < S_LARGE)) *const_cast<volatile int*>(&sh.odd_chunk[c & 1]) = c + 1;
         if (lane == 31) st.dA[hl] = exp2f((float)end) * fmaf((float)(end - (double)(float)end), 0.69314718f, 1.f);
         arrive(&sh.dt_ready[c & 1]);
       }
@@ -684,17 +699,17 @@ bool ssd_chunk_supported(const SsdScanParams& p) {
   return p.N == SN && p.P == SP && p.T >= SSD_CHUNK_MIN_T && p.G > 0 && (p.nh / p.G) % 2 == 0 && p.B <= 65535 && p.G <= 65535 &&
          reinterpret_cast<uintptr_t>(p.xBC) % 16 == 0;
 }
-// bytes of the images, then one int per (row, chunk, group)
+// bytes of the images, then the largest |G| per (row, chunk, group)
 long long ssd_chunk_workspace(const SsdScanParams& p) {
   const long long slots = (long long)p.B * ((p.T + SQ - 1) / SQ) * p.G;
-  return slots * (S_WS + (long long)sizeof(int));
+  return slots * (S_WS + (long long)sizeof(float));
 }
 void ssd_chunk_launch(const SsdScanParams& p, void* workspace, bool lp, cudaStream_t st) {
   ScanArgs a{};
   a.p = p;
   a.chunks = (p.T + SQ - 1) / SQ;
   a.ws = static_cast<const uint8_t*>(workspace);
-  a.odd = reinterpret_cast<const int*>(a.ws + (long long)p.B * a.chunks * p.G * S_WS);
+  a.most_g = reinterpret_cast<const float*>(a.ws + (long long)p.B * a.chunks * p.G * S_WS);
   check_waits();
   a.wait_word = wait_word(WAIT_SSD);
   count_launch(COUNT_SSD);
@@ -703,7 +718,7 @@ void ssd_chunk_launch(const SsdScanParams& p, void* workspace, bool lp, cudaStre
     if (cudaFuncSetAttribute(ssd_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PREP_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SC_SMEM) != cudaSuccess)
       throw std::runtime_error("ssd scan: shared memory size refused");
-    ssd_prepare_kernel<<<dim3(a.chunks, p.G, p.B), SP_THREADS, PREP_SMEM, st>>>(p, static_cast<uint8_t*>(workspace), const_cast<int*>(a.odd), a.chunks);
+    ssd_prepare_kernel<<<dim3(a.chunks, p.G, p.B), SP_THREADS, PREP_SMEM, st>>>(p, static_cast<uint8_t*>(workspace), const_cast<float*>(a.most_g), a.chunks);
     launch_pdl(kernel, dim3(p.nh / 2, p.B), dim3(SC_THREADS), SC_SMEM, st, a);
   };
   if (lp) go(ssd_chunk_kernel<__nv_bfloat16>); else go(ssd_chunk_kernel<float>);

@@ -85,3 +85,34 @@ def test_gate_at_the_ends_of_its_range():
     fin = torch.isfinite(zz)
     assert ((got - want).abs()[fin] <= 8e-7 * want.abs()[fin] + 1e-37 * core.abs()[fin]).all()
     assert torch.equal(got[zz == inf], (core * inf)[zz == inf]) and got[zz == -inf].isnan().all()
+
+
+@pytest.mark.parametrize("what", ["products", "state", "steps"])
+def test_operands_whose_products_leave_the_range(what):
+    """Products that the recurrence does not form (C B^T before it is weighted with x, S^T C before S has decayed) may leave fp32's range where its own values do not.
+    Bound: as above, and a decay e^-a carries an error of a * 2^-23 (a = A dt: 60 and more with the large state)."""
+    args, sizes = _inputs(2, 1, 128, (128,), torch.float32)
+    args["slots"].fill_(1)
+    inner = 128
+    args["A_log"].fill_(3.0)
+    x, Bm, Cm = args["xBC"][..., :inner], args["xBC"][..., inner:inner + 128], args["xBC"][..., inner + 128:]
+    if what == "products":                # C B^T near 1e39
+        x *= 1e-8
+        Bm *= 1e19
+        Cm *= 1e19
+    elif what == "state":                 # S^T C near 1e41; the state decays by e^-20 and more before the first token reads it
+        args["dt_bias"].fill_(3.0)
+        args["state"] *= 1e30
+        Cm *= 1e10
+    else:                                 # C B^T times the step size
+        args["A_log"].fill_(-70.0)
+        args["dt_bias"].fill_(600.0)
+        x *= 1e-20
+        Bm *= 1e18
+        Cm *= 1e18
+    want_state = args["state"].clone()
+    want, size = _definition(*(dict(args, state=want_state)).values(), *sizes)
+    got = _run(args, sizes)
+    assert torch.isfinite(got).all()
+    assert ((got[0].double() - want[0]).norm() / size[0].norm()).item() < (2e-5 if what == "state" else 1e-6)
+    assert ((args["state"][1].double() - want_state[1].double()).norm() / want_state[1].double().norm()).item() < 1e-6
