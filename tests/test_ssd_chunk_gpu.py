@@ -116,3 +116,25 @@ def test_operands_whose_products_leave_the_range(what):
     assert torch.isfinite(got).all()
     assert ((got[0].double() - want[0]).norm() / size[0].norm()).item() < (2e-5 if what == "state" else 1e-6)
     assert ((args["state"][1].double() - want_state[1].double()).norm() / want_state[1].double().norm()).item() < 1e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("nh,G", [(2, 1), (8, 2)])
+@pytest.mark.parametrize("T,lens", [(48, (1, 48, 23)), (130, (1, 130, 1, 22)), (64, (2, 5, 17, 40))])
+def test_rows_of_few_tokens_run_step_by_step(nh, G, T, lens, dtype):
+    """Decode rows beside a prompt portion in one padded call: the bits of the step-by-step kernel, which a call of the short rows alone takes."""
+    args, sizes = _inputs(nh, G, T, lens, dtype)
+    alone = {k: v.clone() for k, v in args.items()}
+    got = _run(args, sizes)
+    most = 23
+    short = [b for b, n in enumerate(lens) if n <= most]
+    for k in ("xBC", "dt_raw", "z"):
+        alone[k] = alone[k][short, :most]
+    for k in ("slots", "ctx_len", "q_len"):
+        alone[k] = alone[k][short]
+    before = dict(ops.kernel_launches())["ssd_chunk"]
+    want = ops.ssd_scan(*alone.values(), *sizes)
+    assert dict(ops.kernel_launches())["ssd_chunk"] == before
+    for i, b in enumerate(short):
+        assert torch.equal(got[b, :most], want[i]) and not got[b, most:].any()
+        assert torch.equal(args["state"][alone["slots"][i]], alone["state"][alone["slots"][i]])
