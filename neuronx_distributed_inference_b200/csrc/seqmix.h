@@ -164,10 +164,11 @@ struct SsdScanParams {
   int B, T, nh, P, N, G;
 };
 void ssd_scan_launch(const SsdScanParams& p, bool lp, cudaStream_t st);
-// the same over prompts in chunks on tensor cores (ssd_chunk.cu): every output row is written, zeros past q_len
+// the same over prompts in chunks on tensor cores (ssd_chunk.cu)
 constexpr int SSD_CHUNK_MIN_T = 48;       // padded width of the call; shorter: a chunk costs as much as 40 steps (times: ssd_chunk.cu)
 bool ssd_chunk_supported(const SsdScanParams& p);
 long long ssd_chunk_workspace(const SsdScanParams& p);
+bool ssd_chunk_pads(const SsdScanParams& p);            // zeros past q_len are written too
 void ssd_chunk_launch(const SsdScanParams& p, void* workspace, bool lp, cudaStream_t st);
 
 // Update of an fp32 residual stream whose sublayers are normalised on both sides, and the norm the next sublayer reads:

@@ -234,7 +234,7 @@ at::Tensor ssd_scan(const at::Tensor& xBC, const at::Tensor& dt_raw, const at::T
   a.state = state.data_ptr<float>(); a.lines = lines.data_ptr<int>(); a.ctx_len = ctx.data_ptr<int>(); a.q_len = qlen.data_ptr<int>();
   a.B = (int)B; a.T = (int)T; a.nh = (int)nh; a.P = (int)P; a.N = (int)N; a.G = (int)G;
   const bool chunked = B > 0 && ssd_chunk_supported(a);
-  auto y = chunked ? at::empty({B, T, inner}, xBC.options()) : at::zeros({B, T, inner}, xBC.options());
+  auto y = chunked && ssd_chunk_pads(a) ? at::empty({B, T, inner}, xBC.options()) : at::zeros({B, T, inner}, xBC.options());
   a.y = y.data_ptr<float>();
   if (chunked) {
     auto ws = at::empty({ssd_chunk_workspace(a)}, xBC.options().dtype(at::kByte));

@@ -54,7 +54,6 @@ constexpr int S_WS = 2 * S_IMG + S_G;                     // workspace of a (row
 constexpr int SC_THREADS = 768;
 constexpr int W_M = 8, W_OUT = 12, W_MMA = 20, W_COPY = 21, W_STEP = 22;             // first warps of the roles; the state's are 0 .. 7
 constexpr uint32_t TM_I = 0, TM_W = 64, TM_S = 192, TM_X = 384;      // TMEM columns: inter, update / intra, state parts, x~ parts
-constexpr int S_ORDER = 2048;                             // rows that are ordered by their length; more run as they come
 constexpr float S_LARGE = 1e18f;                          // 128 products of two values below it stay in fp32's range
 
 // two values -> their three bf16 parts.  w - v of a bf16 w and a fp32 v is one mixed-type instruction; it is the negative of what is left, so the
@@ -107,34 +106,31 @@ __device__ __forceinline__ uint32_t swz(int row, int piece) { return (uint32_t)(
 
 // ---- prepare ---------------------------------------------------------------------------------------------------------------------
 constexpr int SP_THREADS = 512;
-// {row, tokens, state line, earlier context} of all rows, the longest first, by one block
-__device__ __forceinline__ void order_rows(const SsdScanParams& p, int4* __restrict__ order, int* len) {
-  const bool sorted = p.B <= S_ORDER;
-  for (int i = threadIdx.x; sorted && i < p.B; i += SP_THREADS) len[i] = p.q_len[i];
+// {row, tokens of this window, state line, earlier context} of all rows, the longest first, by one block.  The window is `most` tokens after the first `done`
+__device__ __forceinline__ void order_rows(const SsdScanParams& p, int4* __restrict__ order, int* len, int done, int most) {
+  for (int i = threadIdx.x; i < p.B; i += SP_THREADS) len[i] = p.q_len[i];
   __syncthreads();
   for (int i = threadIdx.x; i < p.B; i += SP_THREADS) {
-    const int4 row = make_int4(i, min(p.q_len[i], p.T), p.lines[i], p.ctx_len[i]);
-    int at = sorted ? 0 : i;
-    if (sorted) {
-      const int own = len[i];
+    const int4 row = make_int4(i, min(min(p.q_len[i], p.T) - done, most), p.lines[i], done > 0 ? 1 : p.ctx_len[i]);
+    const int own = len[i];
+    int at = 0;
 #pragma unroll 4
-      for (int j = 0; j < p.B; ++j) at += len[j] > own || (len[j] == own && j < i);
-    }
+    for (int j = 0; j < p.B; ++j) at += len[j] > own || (len[j] == own && j < i);
     order[at] = row;
   }
 }
 __global__ void __launch_bounds__(SP_THREADS) ssd_prepare_kernel(SsdScanParams p, uint8_t* __restrict__ ws, float* __restrict__ most_g, int4* __restrict__ order,
-                                                                 int chunks, int min_tokens) {
+                                                                 int chunks, int min_tokens, int done) {
   extern __shared__ __align__(16) float pm[];              // B, C [64][132]
   __shared__ unsigned most;                                // as bits (of positive numbers: in order)
   constexpr int LD = SN + 4;
   const int c = blockIdx.x, g = blockIdx.y, b = (int)blockIdx.z - 1, tid = threadIdx.x;
   pdl_launch_dependents();
   if (b < 0) {
-    if (c == 0 && g == 0) order_rows(p, order, reinterpret_cast<int*>(pm));
+    if (c == 0 && g == 0) order_rows(p, order, reinterpret_cast<int*>(pm), done, chunks * SQ);
     return;
   }
-  const int n_tok = min(p.q_len[b], p.T), n = min(n_tok - c * SQ, SQ);
+  const int n_tok = min(min(p.q_len[b], p.T) - done, chunks * SQ), n = min(n_tok - c * SQ, SQ);
   if (n_tok < min_tokens || n <= 0) return;
   const long long slot = ((long long)b * chunks + c) * p.G + g;
   uint8_t* img = ws + slot * S_WS;
@@ -205,7 +201,7 @@ struct ScanArgs {
   const uint8_t* ws;
   const float* most_g;
   const int4* order;
-  int chunks, min_tokens;
+  int chunks, min_tokens, pad;
   unsigned* wait_word;
 };
 // what a chunk's step sizes give, per head; two chunks in flight
@@ -340,7 +336,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) ssd_chunk_kernel(const __grid_c
   const float* xrow = p.xBC + (long long)b * p.T * Cd + h0 * SP;
   float* yrow = p.y + (long long)b * p.T * inner + h0 * SP;
   auto pad = [&](int tid, int threads) {                   // padding tokens: zeros
-    for (int i = tid; i < (p.T - max(n_tok, 0)) * 32; i += threads)
+    for (int i = tid; i < (p.T - max(n_tok, 0)) * 32 * a.pad; i += threads)
       *reinterpret_cast<float4*>(yrow + (long long)(max(n_tok, 0) + (i >> 5)) * inner + (i & 31) * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
   };
   if (n_tok >= a.min_tokens) {
@@ -751,35 +747,69 @@ __global__ void __launch_bounds__(SC_THREADS, 1) ssd_chunk_kernel(const __grid_c
 }  // namespace
 
 bool ssd_chunk_supported(const SsdScanParams& p) {
-  return p.N == SN && p.P == SP && p.T >= SSD_CHUNK_MIN_T && p.G > 0 && (p.nh / p.G) % 2 == 0 && p.B < 65535 && p.G <= 65535 &&
+  return p.N == SN && p.P == SP && p.T >= SSD_CHUNK_MIN_T && p.G > 0 && (p.nh / p.G) % 2 == 0 && p.B <= 65535 && p.G <= 65535 &&
          (reinterpret_cast<uintptr_t>(p.xBC) | reinterpret_cast<uintptr_t>(p.state)) % 16 == 0;
 }
-// bytes of the images, then the order of the rows and the largest |G| per (row, chunk, group)
-long long ssd_chunk_workspace(const SsdScanParams& p) {
-  const long long slots = (long long)p.B * ((p.T + SQ - 1) / SQ) * p.G;
-  return slots * (S_WS + (long long)sizeof(float)) + p.B * (long long)sizeof(int4);
+// The images take 114.7 KB per (row, chunk of 64 tokens, group): 1.8 KB a token and group, padding included.  Calls that would take more than this run in windows of
+// tokens, the state carried in its place, and where one chunk of all rows is more, in groups of rows (at least one chunk of one row).  A window ends with an
+// emptying chip and costs the state's way through memory: with 128 MB, 16 rows of 1024 tokens (128 heads, 8 groups) ran in two windows, 971 us instead of 843.
+constexpr long long S_WS_MOST = 512LL << 20;
+static_assert(S_WS_MOST / S_WS <= 2 * SQ * (SN + 4), "a group's rows are ordered in the prepare kernel's shared memory");
+static void ssd_window(const SsdScanParams& p, int& rows, int& chunks) {
+  const long long per = (long long)p.G * S_WS;
+  rows = (int)std::max(1LL, std::min((long long)p.B, S_WS_MOST / per));
+  chunks = (int)std::max(1LL, std::min((long long)(p.T + SQ - 1) / SQ, S_WS_MOST / (per * rows)));
 }
-void ssd_chunk_launch(const SsdScanParams& p, void* workspace, bool lp, cudaStream_t st) {
+// images, order of the rows, largest |G| per (row, chunk, group)
+long long ssd_chunk_workspace(const SsdScanParams& p) {
+  int rows, chunks;
+  ssd_window(p, rows, chunks);
+  return (long long)rows * chunks * p.G * (S_WS + (long long)sizeof(float)) + rows * (long long)sizeof(int4);
+}
+bool ssd_chunk_pads(const SsdScanParams& p) {
+  int rows, chunks;
+  ssd_window(p, rows, chunks);
+  return (long long)chunks * SQ >= p.T;
+}
+void ssd_chunk_launch(const SsdScanParams& all, void* workspace, bool lp, cudaStream_t st) {
+  int rows, chunks;
+  ssd_window(all, rows, chunks);
   ScanArgs a{};
-  a.p = p;
-  a.chunks = (p.T + SQ - 1) / SQ;
+  a.chunks = chunks;
   a.ws = static_cast<const uint8_t*>(workspace);
-  a.order = reinterpret_cast<const int4*>(a.ws + (long long)p.B * a.chunks * p.G * S_WS);
-  a.most_g = reinterpret_cast<const float*>(a.order + p.B);
+  a.order = reinterpret_cast<const int4*>(a.ws + (long long)rows * chunks * all.G * S_WS);
+  a.most_g = reinterpret_cast<const float*>(a.order + rows);
   // tokens from which on a row takes chunks.  us, steps / chunks: one row of 16, 24 and 32 tokens 20.5 / 26.6, 24.6 / 26.6, 28.7 / 26.6; sixteen rows (several CTAs
   // per SM, one after the other) of 8 and 16 47 / 57, 61 / 59
-  a.min_tokens = (long long)p.B * p.nh > 4 * kNumSMs ? 16 : 28;
+  a.min_tokens = (long long)all.B * all.nh > 4 * kNumSMs ? 16 : 28;
+  a.pad = ssd_chunk_pads(all) ? 1 : 0;
   check_waits();
   a.wait_word = wait_word(WAIT_SSD);
   count_launch(COUNT_SSD);
   constexpr int PREP_SMEM = 2 * SQ * (SN + 4) * (int)sizeof(float);
+  const int esz = lp ? 2 : 4;
+  const long long inner = (long long)all.nh * SP, Cd = inner + 2LL * all.G * SN;
   auto go = [&](auto kernel) {
     if (cudaFuncSetAttribute(ssd_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PREP_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SC_SMEM) != cudaSuccess)
       throw std::runtime_error("ssd scan: shared memory size refused");
-    ssd_prepare_kernel<<<dim3(a.chunks, p.G, p.B + 1), SP_THREADS, PREP_SMEM, st>>>(p, static_cast<uint8_t*>(workspace), const_cast<float*>(a.most_g),
-                                                                                     const_cast<int4*>(a.order), a.chunks, a.min_tokens);
-    launch_pdl(kernel, dim3(p.nh / 2, p.B), dim3(SC_THREADS), SC_SMEM, st, a);
+    for (int b0 = 0; b0 < all.B; b0 += rows)
+      for (int done = 0; done < all.T; done += chunks * SQ) {
+        SsdScanParams& p = a.p;                            // the rows and tokens of this window; a row's stride stays T tokens
+        p = all;
+        p.B = std::min(rows, all.B - b0);
+        const long long at = (long long)b0 * all.T + done;
+        p.xBC += at * Cd;
+        p.y += at * inner;
+        p.dt_raw = static_cast<const char*>(all.dt_raw) + (b0 * all.dt_sb + done * all.dt_st) * esz;
+        p.z = static_cast<const char*>(all.z) + (b0 * all.z_sb + done * all.z_st) * esz;
+        p.lines += b0;
+        p.ctx_len += b0;
+        p.q_len += b0;
+        ssd_prepare_kernel<<<dim3(chunks, p.G, p.B + 1), SP_THREADS, PREP_SMEM, st>>>(p, static_cast<uint8_t*>(workspace), const_cast<float*>(a.most_g),
+                                                                                       const_cast<int4*>(a.order), chunks, a.min_tokens, done);
+        launch_pdl(kernel, dim3(p.nh / 2, p.B), dim3(SC_THREADS), SC_SMEM, st, a);
+      }
   };
   if (lp) go(ssd_chunk_kernel<__nv_bfloat16>); else go(ssd_chunk_kernel<float>);
 }

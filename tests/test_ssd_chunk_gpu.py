@@ -138,3 +138,42 @@ def test_rows_of_few_tokens_run_step_by_step(nh, G, T, lens, dtype):
     for i, b in enumerate(short):
         assert torch.equal(got[b, :most], want[i]) and not got[b, most:].any()
         assert torch.equal(args["state"][alone["slots"][i]], alone["state"][alone["slots"][i]])
+
+
+def test_workspace_is_bounded():
+    """Long prompts run in windows of tokens, many rows in groups: the bits of one window after the other, and no more than 514 MB beside the output."""
+    nh, G, P, N = 16, 8, 64, 128
+    T, cut = 40000, 37440                 # 585 chunks of 8 groups fill a window
+    args, sizes = _inputs(nh, G, T, (T,), torch.bfloat16)
+    args["slots"].fill_(1)
+    parts = {k: v.clone() for k, v in args.items()}
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    base = torch.cuda.memory_allocated()
+    got = _run(args, sizes)
+    assert torch.cuda.max_memory_allocated() - base - got.numel() * 4 < 514 << 20
+    first = {k: (v[:, :cut].contiguous() if k == "xBC" else v[:, :cut] if k in ("dt_raw", "z") else v) for k, v in parts.items()}
+    first["q_len"] = torch.full_like(parts["q_len"], cut)
+    y0 = _run(first, sizes)
+    rest = {k: (v[:, cut:].contiguous() if k == "xBC" else v[:, cut:] if k in ("dt_raw", "z") else v) for k, v in parts.items()}
+    rest["q_len"], rest["ctx_len"] = torch.full_like(parts["q_len"], T - cut), torch.full_like(parts["q_len"], cut)
+    y1 = _run(rest, sizes)
+    assert torch.equal(got, torch.cat([y0, y1], 1)) and torch.equal(args["state"], parts["state"])
+
+
+def test_rows_in_groups():
+    """More rows than the workspace holds chunks of: a short row, padding and prompts in every group."""
+    nh, G, T, B = 256, 128, 64, 40        # 36 rows of 128 groups fill the workspace
+    lens = [(64, 1, 50, 0, 33)[b % 5] for b in range(B)]
+    args, sizes = _inputs(nh, G, 1, (1,), torch.bfloat16)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")             # noqa: E731
+    P, N, inner = 64, 128, nh * 64
+    args.update(xBC=torch.randn(B, T, inner + 2 * G * N, device="cuda"), dt_raw=torch.randn(B, T, nh, device="cuda").bfloat16(),
+                z=torch.randn(B, T, inner, device="cuda").bfloat16(), state=torch.randn(B, nh, N, P, device="cuda"),
+                slots=i32(list(range(B))[::-1]), ctx_len=i32([b % 2 for b in range(B)]), q_len=i32(lens))
+    alone = args["state"].clone()
+    got = _run(args, sizes)
+    for b in range(B):
+        one = {k: (alone if k == "state" else v if k in ("A_log", "dt_bias", "D_skip") else v[b:b + 1]) for k, v in args.items()}
+        assert torch.equal(_run(one, sizes)[0], got[b])
+    assert torch.equal(alone, args["state"])
