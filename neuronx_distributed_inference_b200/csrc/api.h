@@ -101,8 +101,9 @@ enum WaitKernel { WAIT_ATTENTION, WAIT_GEMM_PAIR, WAIT_SKINNY, WAIT_SSD, WAIT_RO
 unsigned* wait_word(WaitKernel which);
 void check_waits();
 void wait_probe_launch(long long clocks, int* out, cudaStream_t stream);
-// launches of the tensor-core kernels by the host (a graph replay is none): which route calls took
-enum CountedKernel { COUNT_ATTENTION, COUNT_GEMM_PAIR, COUNT_SKINNY, COUNT_GEMM_TCGEN05, COUNT_SSD, COUNT_ROUTER, COUNT_KERNELS };
+// launches of the tensor-core kernels by the host (a graph replay is none): which route calls took (COUNT_ATTENTION_TWO: those of COUNT_ATTENTION with two
+// query tiles per CTA)
+enum CountedKernel { COUNT_ATTENTION, COUNT_ATTENTION_TWO, COUNT_GEMM_PAIR, COUNT_SKINNY, COUNT_GEMM_TCGEN05, COUNT_SSD, COUNT_ROUTER, COUNT_KERNELS };
 void count_launch(CountedKernel which);
 std::vector<std::pair<std::string, long long>> kernel_launches();
 

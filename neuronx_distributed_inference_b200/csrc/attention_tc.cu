@@ -689,6 +689,7 @@ static void fa_run(FaParams& p, cudaStream_t stream) {
   check_waits();
   p.wait_word = wait_word(WAIT_ATTENTION);
   count_launch(COUNT_ATTENTION);
+  if (NX == 2) count_launch(COUNT_ATTENTION_TWO);
   // grouped heads share their keys two by two; a head of its own takes 256 queries instead
   p.pair_heads = (p.Hq / p.Hkv) % 2 == 0 ? 1 : 0;
   const bool pair = NX == 2 && p.pair_heads;

@@ -48,7 +48,7 @@ void check_waits() {
 static std::atomic<long long> g_launches[COUNT_KERNELS];
 void count_launch(CountedKernel which) { g_launches[which].fetch_add(1, std::memory_order_relaxed); }
 std::vector<std::pair<std::string, long long>> kernel_launches() {
-  static const char* const names[COUNT_KERNELS] = {"attention_prefill_tc", "gemm_pair", "skinny_gemm", "gemm_tcgen05", "ssd_chunk", "router_logits_tc"};
+  static const char* const names[COUNT_KERNELS] = {"attention_prefill_tc", "attention_prefill_tc_two_tiles", "gemm_pair", "skinny_gemm", "gemm_tcgen05", "ssd_chunk", "router_logits_tc"};
   std::vector<std::pair<std::string, long long>> r;
   for (int i = 0; i < COUNT_KERNELS; ++i) r.emplace_back(names[i], g_launches[i].load(std::memory_order_relaxed));
   return r;

@@ -98,28 +98,54 @@ def test_soft_cap_does_not_depend_on_unseen_keys(D):
         want = got
 
 
+def _two_tiles():
+    return ops.kernel_launches()["attention_prefill_tc_two_tiles"]
+
+
 # rows of more than 1152 keys and at least 148 CTAs take two query tiles per CTA: one tile more or less than that, whole and odd lengths, heads in pairs
 # and alone; the bound above
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("B,T,Hq,Hkv,window,causal,sinks", [
-    (1, 1152, 34, 17, 0, True, False), (1, 1153, 32, 8, 0, True, True), (1, 1281, 30, 30, 0, True, False), (2, 1290, 16, 4, 1025, True, True),
-    (2, 1290, 16, 4, 1024, True, False), (1, 1217, 32, 16, 0, False, False), (2, 1408, 15, 5, 0, False, True)])
-def test_two_tiles(D, B, T, Hq, Hkv, window, causal, sinks):
+@pytest.mark.parametrize("B,T,Hq,Hkv,window,causal,sinks,two", [
+    (1, 1152, 34, 17, 0, True, False, 0), (1, 1153, 32, 8, 0, True, True, 1), (1, 1281, 30, 30, 0, True, False, 1), (2, 1290, 16, 4, 1025, True, True, 1),
+    (2, 1290, 16, 4, 1024, True, False, 0), (1, 1217, 32, 16, 0, False, False, 1), (2, 1408, 15, 5, 0, False, True, 1)])
+def test_two_tiles(D, B, T, Hq, Hkv, window, causal, sinks, two):
+    before = _two_tiles()
     test_contiguous(D, B, T, Hq, Hkv, window, causal, sinks)
+    assert _two_tiles() - before == two
 
 
 @pytest.mark.parametrize("D,cap", [(64, 20.0), (128, 20.0), (64, None), (128, None)])
-@pytest.mark.parametrize("Hq,G", [(16, 4), (17, 17)])
-@pytest.mark.parametrize("mask", [dict(), dict(window=1300, keep=70), dict(window=200, keep=4), dict(chunk=1200)])
-def test_two_tiles_paged(D, cap, Hq, G, mask):
+@pytest.mark.parametrize("Hq,G", [(32, 8), (17, 17)])
+@pytest.mark.parametrize("mask,two", [(dict(), 1), (dict(window=1300, keep=70), 1), (dict(window=200, keep=4), 0), (dict(chunk=1200), 1)])
+def test_two_tiles_paged(D, cap, Hq, G, mask, two):
     ctx, n = (0, 1517, 130, 64, 1000), (300, 16, 0, 257, 290)
     q, dirty, clean, table, c, m = _paged(5, 300, Hq, G, D, 64, ctx, n)
     args = (table, c, m, D ** -0.5, cap, mask.get("window", 0), mask.get("keep", 0))
+    before = _two_tiles()
     got = ops.paged_window_attention(q, *dirty, *args, chunk=mask.get("chunk"))
+    assert _two_tiles() - before == two
     want = ref.paged_window_attention(q.float(), *(t.float() for t in clean), *args, chunk=mask.get("chunk"))
     assert _rel(got, want) < 4e-3
     for b, live in enumerate(n):
         assert not got[b, live:].any()
+
+
+@pytest.mark.parametrize("std", [1.0, 6.0])          # scores inside and beyond the range of the polynomial for tanh (|score| <= cap)
+@pytest.mark.parametrize("Hq,G", [(32, 8), (17, 17)])
+@pytest.mark.parametrize("gate", [None, "channel", "odd", "head"])
+def test_two_tiles_cap_gate_sinks_temperature(std, Hq, G, gate):
+    D, ctx, n = 128, (0, 1100, 130, 64, 1000), (300, 140, 0, 257, 290)
+    q, dirty, clean, table, c, m = _paged(5, 300, Hq, G, D, 64, ctx, n, std)
+    wide = torch.randn(5, 300, Hq * D + 3, device=DEV, dtype=torch.bfloat16)
+    g = {None: None, "channel": wide[..., :Hq * D].contiguous(), "odd": wide[..., 3:], "head": wide[..., :Hq]}[gate]
+    kw = dict(gate=g, sinks=torch.randn(Hq, device=DEV), gate_per_head=gate == "head", head_scale=torch.linspace(-0.8, 2.0, Hq, device=DEV))
+    for cap in (None, 20.0):
+        before = _two_tiles()
+        got = ops.paged_window_attention(q, *dirty, table, c, m, D ** -0.5, cap, 0, 0, **kw)
+        assert _two_tiles() - before == 1
+        want = ref.paged_window_attention(q.float(), *(t.float() for t in clean), table, c, m, D ** -0.5, cap, 0, 0,
+                                          **dict(kw, gate=None if g is None else g.float()))
+        assert _rel(got, want) < 4e-3
 
 
 def test_soft_cap_of_scores_below_the_range():
