@@ -1,4 +1,4 @@
-// mbarriers of the warp-specialised tensor-core kernels (attention_tc.cu, gemm_pair.cu, skinny_gemm.cu) and their bounded waits.
+// mbarriers of the warp-specialised tensor-core kernels (attention_tc.cu, gemm_pair.cu, skinny_gemm.cu, ssd_chunk.cu, router_tc.cu) and their bounded waits.
 //
 // A wait that runs out is an error of the kernel, never a slow neighbour: every role waits for the kernels in front of its own (griddepcontrol.wait)
 // before it may block here.  The role then sets `stop`, which ends the other waits of the CTA, issues nothing more and runs to its end; the launch's

@@ -236,21 +236,8 @@ __global__ void __launch_bounds__(256) moe_scatter_kernel(const __nv_bfloat16* _
 void moe_plan256_launch(const int* topk_i, int id_step, int entries, int expert_offset, int e_local, int tiles, int* pos, int* tile_expert, int* tile_row,
                         cudaStream_t stream) {
   if (e_local > MOE_MAX_E) throw std::runtime_error("moe_plan: more than 512 local experts");
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(MOE_PLAN_CTAS);
-  cfg.blockDim = dim3(MOE_PLAN_THREADS);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = MOE_PLAN_CTAS;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, moe_plan256_kernel, topk_i, id_step, entries, expert_offset, e_local, tiles, pos, tile_expert, tile_row);
-  if (e != cudaSuccess) throw std::runtime_error(std::string("moe_plan launch failed: ") + cudaGetErrorString(e));
+  launch_pdl_cluster(moe_plan256_kernel, MOE_PLAN_CTAS, dim3(MOE_PLAN_CTAS), dim3(MOE_PLAN_THREADS), 0, stream, topk_i, id_step, entries, expert_offset, e_local,
+                     tiles, pos, tile_expert, tile_row);
 }
 void moe_scatter_launch(const void* x, const float* topk_w, const int* pos, void* xp, int N, int H, int k, int scale_input, cudaStream_t stream) {
   launch_pdl(moe_scatter_kernel, dim3(N), dim3(256), 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), topk_w, pos,

@@ -234,7 +234,7 @@ __device__ __forceinline__ void radix_select(unsigned* hist, unsigned* s_prefix,
 // large), and only groups that reach it can hold one of the k largest: k groups plus ties, 32 elements each, are read again.  Their elements
 // from the bound upwards (k plus a few percent for rows in no particular order) are ranked by counting (value, then lowest index).  More than
 // TOPK_CAND of them (long runs of equal values, or one group that holds most of the large ones): the row is selected by radix passes over all of
-// it, as every row was before (32 rows of 128256 bf16 values: 84 us a call, six scalar passes per row; 15 us with the groups, most of it the host).
+// it, as every row was before (32 rows of 128256 bf16 values: 84 us a call, six scalar passes per row; 15 us with the groups, in a graph too).
 template <typename T>
 __global__ void __launch_bounds__(TOPK_THREADS) topk_sample_kernel(const T* __restrict__ logits, const uint32_t* __restrict__ gmax, int groups,
                                                                    const int* __restrict__ top_k, const float* __restrict__ top_p,

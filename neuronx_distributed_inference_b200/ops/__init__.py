@@ -46,7 +46,7 @@ def _use_cuda(x: torch.Tensor) -> bool:
 
 
 def kernel_launches():
-    """{kernel: launches by the host} of the tensor-core GEMM and attention kernels: ``stats`` counts calls (``gemm_tcgen05``: those of :func:`linear` that run
+    """{kernel: launches by the host} of the tensor-core kernels (GEMMs, attention, Mamba-2 scan, router): ``stats`` counts calls (``gemm_tcgen05``: those of :func:`linear` that run
     on tensor cores), this tells which kernel the rules of the extension chose."""
     return dict(_C().kernel_launches())
 

@@ -1,4 +1,4 @@
-"""fp32 router on tensor cores (csrc/moe_plain.cu): logits against 64 bits at the edges of its blocks and column parts; choice and weights against the definition.
+"""fp32 router on tensor cores (csrc/router_tc.cu; choice: csrc/moe_plain.cu): logits against 64 bits at the edges of its blocks and column parts; choice and weights against the definition.
 
 Bound: products of bf16 rows and split fp32 weights are exact in fp32, sums of at most 64 go through the tensor core (its adder drops bits below
 2^-23 of the running sum: 64 * 2^-23 relative at worst, 1e-7 seen), the rest are fp32 additions; 1e-6 is asked for."""
