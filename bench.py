@@ -206,7 +206,7 @@ def token_checksum(tokens):
             "distinct_tokens": int(tokens.unique().numel())}
 
 
-# ---- the other BASELINE.json configs (bench.py --config ...): same JSON line, measured through the public generate() API ----
+# ---- the other benchmark configurations (bench.py --config ...): same JSON line, measured through the public generate() API ----
 DBRX_1L = dict(d_model=6144, n_heads=48, n_layers=1, max_seq_len=32768, vocab_size=100352,
                attn_config=dict(kv_n_heads=8, clip_qkv=8.0, rope_theta=500000.0),
                ffn_config=dict(ffn_hidden_size=10752, moe_num_experts=16, moe_top_k=4, hidden_size=6144))
@@ -334,7 +334,7 @@ def main():
     ap.add_argument("--skip-ci", action="store_true")
     ap.add_argument("--config", default="llama8b", choices=["llama8b", "dbrx", "quant", "spec", "fetodra", "sodudra", "tusipel", "zanivik", "balivik",
                                                                 "navulorn"],
-                    help="BASELINE.json config: llama8b (headline, default), dbrx (1-layer MoE), quant (Llama-2-7b fp8), "
+                    help="benchmark configuration: llama8b (headline, default), dbrx (1-layer MoE), quant (Llama-2-7b fp8), "
                          "spec (open_llama 7b + 3b draft), fetodra (1 GPU: prefill / decode tokens/s of the Fetodra stack beside the Bamba "
                          "stack at equal layer sizes + per-kernel roofline table; --size picks the layer sizes), sodudra (1 GPU: the same for the "
                          "Sodudra stack beside the DeepSeek stack; --size small|large), tusipel (1 GPU: the same for the Tusipel stack beside "

@@ -34,12 +34,12 @@ def annotate_layers(model):
     return model
 
 
-def ncu_launch_list_cmd(cmd: List[str], out_csv: str = "gpurun_out/launches.csv", skip: int = 0, count: int = 400) -> str:
+def ncu_launch_list_cmd(cmd: List[str], out_csv: str = "launches.csv", skip: int = 0, count: int = 400) -> str:
     return " ".join(["ncu", "--metrics", "gpu__time_duration.sum", "--clock-control", "none", "-s", str(skip), "-c", str(count),
                      "--csv", "--log-file", out_csv] + [shlex.quote(c) for c in cmd])
 
 
-def ncu_full_cmd(cmd: List[str], kernel_regex: str, out: str = "gpurun_out/prof", skip: int = 0, count: int = 3) -> str:
+def ncu_full_cmd(cmd: List[str], kernel_regex: str, out: str = "prof", skip: int = 0, count: int = 3) -> str:
     return " ".join(["ncu", "--set", "full", "--clock-control", "none", "-k", f"regex:{kernel_regex}",
                      "-s", str(skip), "-c", str(count), "-o", out, "-f"] + [shlex.quote(c) for c in cmd])
 

@@ -1,5 +1,5 @@
 """Micro-benchmarks of the hot kernels against the measured roofline (MEASURED_PEAKS.json).
-Usage (on the GPU box): python tools/bench_kernels.py [--json gpurun_out/kernels.json]"""
+Usage (on a machine with B200s): python tools/bench_kernels.py [--json kernels.json]"""
 import argparse
 import json
 import math

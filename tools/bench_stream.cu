@@ -1,6 +1,6 @@
 // Streaming micro-benchmark (design input for the decode GEMV): how fast can ONE SM / the whole chip pull weights into shared
 // memory with (a) 3-D tiled TMA boxes of 128-byte rows, (b) contiguous 1-D bulk copies (pre-tiled weights), (c) LDG.128?
-//   nvcc -gencode arch=compute_100a,code=sm_100a -O3 -o gpurun_out/bench_stream tools/bench_stream.cu -lcuda
+//   nvcc -gencode arch=compute_100a,code=sm_100a -O3 -o bench_stream tools/bench_stream.cu -lcuda
 //   ./bench_stream            -> table: variant, bytes per copy, ring KB, CTAs/SM, TB/s
 // No math: the consumer releases a stage as soon as it is full, so the number is the data-movement ceiling.
 #include <cuda.h>

@@ -15,7 +15,7 @@ def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
     ap.add_argument("--layers", type=int, default=4)
-    ap.add_argument("--out", default="gpurun_out/trace.json")
+    ap.add_argument("--out", default="trace.json")
     ap.add_argument("--shard-shapes", type=int, default=1, help="1 GPU: per-rank shapes of TP=N, no collectives")
     a = ap.parse_args()
     from neuronx_distributed_inference_b200.parallel import state as pstate
