@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(SP_THREADS) ssd_prepare_kernel(SsdScanParams p
   const float* src = p.xBC + ((long long)b * p.T + c * SQ) * Cd + inner + g * SN;
   if (tid == 0) most = 0u;
   bool bad = false;
-#pragma unroll 4
+#pragma unroll                                             // (by a factor, the compiler settles for 40 registers: 11.1 us instead of 10.5)
   for (int i = tid; i < 2 * SQ * SN / 8; i += SP_THREADS) {       // 8 columns of a token
     const int which = i >> 10, t = (i >> 4) & 63, n0 = (i & 15) * 8;
     float v[8] = {};
