@@ -94,7 +94,7 @@ __device__ __forceinline__ void attention_body(const AttnArgs& p, uint8_t* smem_
   // K/V tiles, cos/sin — runs BEFORE griddepcontrol.wait and overlaps the QKV projection; after the wait only the new rows are
   // fetched, rotated, written to the cache (for later steps) and patched into the resident tiles from shared memory.
   const bool fused = (MODE == ATTN_DECODE) && p.qkv != nullptr;
-  unsigned long long* prof = p.prof ? p.prof + (size_t)(bx + by * gdx) * 8 : nullptr;
+  unsigned long long* prof = p.prof ? p.prof + (size_t)(bx + by * gdx + (BY_LENGTH ? blockIdx.z * gdx * p.nsplit : 0)) * 8 : nullptr;
   if (prof && tid == 0) {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
