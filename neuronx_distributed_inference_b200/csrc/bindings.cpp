@@ -111,6 +111,33 @@ static void check_gemv_inputs(const at::Tensor& x, const at::Tensor& w) {
   TORCH_CHECK(x.size(1) % 64 == 0 && x.stride(1) == 1 && x.stride(0) % 8 == 0 && w.is_contiguous());
 }
 
+// Where the swapped, evenly split GEMM (skinny_gemm.cu) beats the 128-row token tiles of gemm_tcgen05.cu (us in a graph, skinny / tiles; 16, 64, 96 and 128 tokens):
+//   gate|up 28672 x 4096: 43 / 61, 48 / 62, 53 / 62, 56 / 63     17280 x 3200: 25 / 48, 30 / 34, 34 / 34, 38 / 34    16384 x 2048: 17 / 33, 22 / 26, 25 / 26, 28 / 26
+//           8192 x 3072:  17 / 36, 21 / 23, 24 / 23, 27 / 23      6144 x 2048: 14 / 28, 20 / 18, 22 / 18, 25 / 18     2048 x 1024:   9 / 17, 12 / 17, 14 / 17, 17 / 17
+//   plain 4096 x 14336:   26 / 57, 30 / 58, 34 / 58, 35 / 59      6144 x 4096: 16 / 25, 19 / 26, 21 / 26, 23 / 26      2048 x 8192:  14 / 39, 18 / 39, 21 / 39, 23 / 40
+//           3072 x 3072:  12 / 20, 15 / 20, 18 / 20, 20 / 20      4096 x 1024:  9 / 11, 11 / 11, 13 / 11, 14 / 11       512 x 512:    8 / 8,  10 / 8,  11 / 8,  13 / 8
+// A feature's tokens are in one lane, so its epilogue and the fix-up of the cut tiles grow with the tokens, while the tile kernel's time does not change up to 128.
+static bool skinny_pays(int M, int rows, int K, bool glu) {
+  const long long size = (long long)rows * K;
+  if (glu) return M <= 32 || (M <= 64 && size >= (16LL << 20)) || (M <= 96 && size >= (32LL << 20)) || (M <= SKINNY_MAX_T && size >= (64LL << 20));
+  return M <= 64 || (M <= SKINNY_MAX_T && (K >= 2 * rows || size >= (8LL << 20)));
+}
+
+static void run_skinny(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int act, const c10::optional<at::Tensor>& residual,
+                       at::Tensor& y, bool fresh_weight) {
+  const int M = x.size(0);
+  const int64_t nt = skinny_gemm_tickets(), nf = skinny_gemm_ws_floats(M, act != 0);
+  auto ws = at::empty({nf + nt}, x.options().dtype(at::kFloat));              // one per call: safe on any stream and inside captured graphs
+  SkinnyGemm a{};
+  a.x = x.data_ptr(); a.x_rows = M; a.ldx = x.stride(0); a.w = w.data_ptr(); a.bias = optr(bias); a.residual = optr(residual); a.y = y.data_ptr();
+  a.experts = 1; a.tokens = M; a.n_out = y.size(1); a.K = x.size(1); a.act = act; a.limit = 7.f; a.alpha = 1.702f;
+  a.w_fresh = fresh_weight ? 1 : 0;
+  a.ws = ws.data_ptr<float>();
+  a.tickets = reinterpret_cast<unsigned*>(ws.data_ptr<float>() + nf);
+  skinny_clear_launch(a.tickets, (int)nt, cur_stream());
+  skinny_gemm_launch(a, cur_stream());
+}
+
 at::Tensor gemv(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias,
                 const c10::optional<at::Tensor>& norm_w, double eps, double offset, int64_t act,
                 const c10::optional<at::Tensor>& scale, const c10::optional<at::Tensor>& residual) {
@@ -146,23 +173,23 @@ at::Tensor gemv(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
   const int N = w.size(0);
   const bool glu = act != 0;
   if (glu) TORCH_CHECK(N % 2 == 0);
-  bool x_in_smem;
-  at::Tensor xn = prenorm_if_needed(x, norm_w, eps, offset, x_in_smem);
   auto y = at::empty({x.size(0), glu ? N / 2 : N}, x.options());
   if (residual.has_value())
     TORCH_CHECK(!glu && residual->is_contiguous() && residual->size(0) == x.size(0) && residual->size(1) == N && is_bf16(*residual));
+  // rows too wide for the streaming kernel's shared memory (from 7 tokens of 14336, 8 of 11008).  us, here / one warp per weight row: 4096 x 14336 at 7 tokens
+  // 26 / 57, at 8 26 / 36; 4096 x 11008 at 8 21 / 39
+  if (!gemv2_supported(x.size(0), x.size(1), 0) && (glu ? N / 2 : N) % 8 == 0) {
+    run_skinny(norm_w.has_value() ? std::get<0>(rmsnorm(x.contiguous(), *norm_w, eps, offset, c10::nullopt)) : x, w, bias, (int)act, residual, y, false);
+    return y;
+  }
+  bool x_in_smem;
+  at::Tensor xn = prenorm_if_needed(x, norm_w, eps, offset, x_in_smem);
   GemvParams p{};
   fill_params(p, xn, w, bias, norm_w, eps, offset, (int)act, residual, scale, y, x_in_smem);
   run_gemv(p, 0, x.device());
   return y;
 }
 
-// tcgen05 GEMM for T > 8 tokens (prefill, long speculation windows)
-// Where the swapped, evenly split GEMM (skinny_gemm.cu) beats the 128-row token tiles of gemm_tcgen05.cu (us, skinny / tiles; 37, 64 and 128 tokens):
-//   gate|up 28672 x 4096: 52 / 62, 55 / 63, 69 / 63     17280 x 3200: 33 / 34, 35 / 34, 46 / 34    16384 x 2048: 23 / 26, 26 / 26, 36 / 26
-//   plain 4096 x 14336:   30 / 52, 31 / 52, 39 / 54     6144 x 4096:  18 / 23, 19 / 23, 25 / 24    2048 x 8192:  19 / 34, 20 / 35, 27 / 36
-// Its last tile's epilogue grows with the tokens (a feature per lane, all tokens in turn, twice that with a gate product), while the tile kernel's
-// time does not change up to 128; deep K leaves the tile kernel few tiles.
 // Where 256 x 256 tiles on CTA pairs (gemm_pair.cu) beat the one-CTA tiles (us, pairs / one CTA, isolated):
 //   28672 x 4096 gate|up: 62 / 84 at 256 tokens, 99 / 133 at 512, 624 / 725 at 4096      4096 x 14336: 74 / 55 at 256, 76 / 77 at 512, 80 / 94 at 768
 //   6144 x 4096: 26 / 26 at 256, 29 / 41 at 400, 71 / 82 at 2048                         2048 x 8192: 45 / 36 at 512, 45 / 49 at 768, 98 / 110 at 4096
@@ -171,13 +198,9 @@ static bool pair_pays(int M, int n_out, bool glu) {
   return M > 512 || (M > 128 && ((M + 255) / 256) * ((n_out + (glu ? 127 : 255)) / (glu ? 128 : 256)) >= 40);
 }
 
-static bool skinny_pays(int M, int rows, int K, bool glu) {
-  if (glu) return M <= 32 || (M <= 64 && (long long)rows * K >= (64LL << 20));
-  return M <= 64 || (M <= SKINNY_MAX_T && K >= 2 * rows);
-}
-
 // fresh_weight: w was written by a kernel enqueued just before (an expanded 8-bit weight).  The kernels fetch a parameter's first tiles before the
 // kernels in front of them have finished; such a weight has to be waited for.
+// tcgen05 GEMM for T > 8 tokens (prefill, long speculation windows)
 at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int64_t act,
                 const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& out, bool fresh_weight) {
   TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1));
@@ -194,17 +217,7 @@ at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
   if (residual.has_value())
     TORCH_CHECK(!glu && residual->is_contiguous() && residual->size(0) == M && residual->size(1) == n_out && is_bf16(*residual));
   if (skinny_pays(M, N, K, glu)) {
-    auto fopt = x.options().dtype(at::kFloat);
-    const int64_t nt = skinny_gemm_tickets(), nf = skinny_gemm_ws_floats(M, glu);
-    auto ws = at::empty({nf + nt}, fopt);              // one per call: safe on any stream and inside captured graphs
-    SkinnyGemm a{};
-    a.x = x.data_ptr(); a.x_rows = M; a.ldx = x.stride(0); a.w = w.data_ptr(); a.bias = optr(bias); a.residual = optr(residual); a.y = y.data_ptr();
-    a.experts = 1; a.tokens = M; a.n_out = n_out; a.K = K; a.act = (int)act; a.limit = 7.f; a.alpha = 1.702f;
-    a.w_fresh = fresh_weight ? 1 : 0;
-    a.ws = ws.data_ptr<float>();
-    a.tickets = reinterpret_cast<unsigned*>(ws.data_ptr<float>() + nf);
-    skinny_clear_launch(a.tickets, (int)nt, cur_stream());
-    skinny_gemm_launch(a, cur_stream());
+    run_skinny(x, w, bias, (int)act, residual, y, fresh_weight);
     return y;
   }
   if (pair_pays(M, n_out, glu)) {

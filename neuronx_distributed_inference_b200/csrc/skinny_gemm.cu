@@ -10,9 +10,13 @@
 //     in flight per SM), weights and tokens have a TMA producer warp each.
 //   * accumulators (128 features x tokens) sit in TMEM twice, so a tile's epilogue overlaps the stream of the next one.  A lane holds one output
 //     feature: a warp's store of one token is 64 contiguous bytes, gate and up of a feature meet in one thread.
-//   * eight epilogue warps: the last tile's epilogue is the tail of the launch (four warps: 56 instead of 51 us at 37 tokens, 28672 x 4096).
-// Measured (us, here / 128-row token tiles): see skinny_pays in bindings.cpp.  28672 x 4096 at 9 tokens 46 us = 5.1 TB/s; six of eight Mixtral-sized
-// experts, 6 tokens, with permutation and sum: 336 us = 6.3 TB/s (one warp per weight row and (token, slot) pair: 744 us).
+//   * 16 epilogue warps: the last tile's epilogue is the tail of the launch, and so is the fix-up of its parts.  Both are round trips to L2 and cold
+//     instructions, so: every load of a group of 8 tokens (residual, parts) before the first use, the activation chosen outside of the loops, one code path.
+//     With 8 warps, groups of 16 tokens, three copies of the epilogue and the residual read where it was added, the tail after the last weights was
+//     25 us at 37 tokens, 28672 x 4096 gate | up (now 8) and 17 us at 4096 x 14336 with a residual (now 6).
+// Measured (us, here / 128-row token tiles): see skinny_pays in bindings.cpp.  28672 x 4096 gate | up at 9 tokens 42.6 us = 5.5 TB/s (46 before), a gated MLP
+// of 8B sizes with norm and residual at 37 tokens 78 us in a graph (100 before); six of eight Mixtral-sized experts, 6 tokens, with permutation and sum: 336 us
+// = 6.3 TB/s (one warp per weight row and (token, slot) pair: 744 us).
 #include <algorithm>
 #include <stdexcept>
 #include <string>
@@ -25,7 +29,8 @@ namespace nxdi {
 
 constexpr int SK_BM = 128, SK_BK = 64;                 // weight rows, k elements per stage box (128-byte rows)
 constexpr int SK_W_BYTES = SK_BM * SK_BK * 2;
-constexpr int SK_THREADS = 384;                        // 4 warps: weights, MMA, TMEM, tokens; 8 epilogue warps
+constexpr int SK_EPI = 16;                             // epilogue warps: four per 32 features
+constexpr int SK_THREADS = 128 + SK_EPI * 32;          // 4 warps: weights, MMA, TMEM, tokens; epilogue warps
 constexpr int SK_MAX_STAGES = 12;
 constexpr int SK_SMEM = 220 * 1024;
 
@@ -63,10 +68,14 @@ __device__ __forceinline__ void sk_umma(uint32_t tmem_d, uint64_t da, uint64_t d
 __device__ __forceinline__ void sk_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar_s32(bar)) : "memory");
 }
-__device__ __forceinline__ void sk_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-                 "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(taddr));
+__device__ __forceinline__ void sk_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
+}
+__device__ __forceinline__ uint32_t ldg_act_u16(const __nv_bfloat16* p) {
+  unsigned short r;
+  asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(r) : "l"(p));
+  return r;
 }
 
 template <bool GLU>
@@ -90,7 +99,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tmem_full[b], 1);
-      mbar_init(&tmem_empty[b], 8);
+      mbar_init(&tmem_empty[b], SK_EPI);
     }
     s_stop = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -189,7 +198,9 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
     }
   } else if (warp >= 4) {
     // ================= epilogue: lane = output feature =================
-    const int n_in = (warp & 3) * 32 + lane, c0 = warp >= 8 ? 16 : 0;      // two warps per 32 features: even and odd groups of 16 tokens
+    // One code path for whole tiles and for tiles that meet in the workspace, the activation chosen outside of the loop over the tokens: the epilogue runs once or
+    // twice per CTA, so every instruction of it is fetched cold.
+    const int n_in = (warp & 3) * 32 + lane, c0 = ((warp - 4) >> 2) * 8;      // the warps of 32 features take groups of 8 tokens in turn
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     int seg = 0;
     bool live = true;          // false once a wait ran out: the warp still takes part in the barriers of the eight
@@ -198,134 +209,142 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
       u += kb1 - kb0;
       const int ei = tile / n_tiles, n = (tile % n_tiles) * SK_BM + n_in, e = grouped ? p.active[ei] : 0;
       const int row0 = grouped ? p.seg_start[ei] : 0, cnt = grouped ? p.seg_count[ei] : p.T;
+      const float bg = (p.bias && n < p.n_out) ? __bfloat162float(p.bias[(size_t)e * p.rows + n]) : 0.f;
+      const float bu = (GLU && p.bias && n < p.n_out) ? __bfloat162float(p.bias[(size_t)e * p.rows + p.n_out + n]) : 0.f;
+      const bool whole = kb0 == 0 && kb1 == nkb;
+      // CTAs that share the tile: those of its first and last k-block and all between
+      const long long f = (long long)tile * nkb;
+      const int c_first = whole ? blockIdx.x : (int)(((f + 1) * G - 1) / total), c_last = whole ? blockIdx.x : (int)(((f + nkb) * G - 1) / total);
       if (live) live = mbar_wait_warp(&tmem_full[buf], (uint32_t)((seg >> 1) & 1), stop, p.wait_word);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem + lanes + (uint32_t)(buf * acc_cols);
-      const bool whole = kb0 == 0 && kb1 == nkb;
-      const float bg = (p.bias && n < p.n_out) ? __bfloat162float(p.bias[(size_t)e * p.rows + n]) : 0.f;
-      const float bu = (GLU && p.bias && n < p.n_out) ? __bfloat162float(p.bias[(size_t)e * p.rows + p.n_out + n]) : 0.f;
-      auto finish = [&](int t, float g, float up) {
-        if (n >= p.n_out || t >= cnt) return;
-        float r = g + bg;
-        if (GLU) {
-          up += bu;
-          if (p.act == 4) {       // clamped, shifted gate product
-            const float gc = fminf(r, p.limit), uc = fminf(fmaxf(up, -p.limit), p.limit);
-            r = (uc + 1.f) * gc * (1.f / (1.f + __expf(-p.alpha * gc)));
-          } else {
-            r = (p.act == 1 ? silu(r) : (p.act == 2 ? gelu_tanh(r) : gelu_erf(r))) * up;
+      bool own = whole;          // this CTA's part comes straight from TMEM (it is the first in k order), the others' from the workspace
+      if (!whole) {
+        if (kb0 == 0) {
+          // the tile's first part is its CTA's last segment, so the other parts are often there already: then they are added to the sums in TMEM, which
+          // needs neither slot nor ticket
+          if (threadIdx.x == 128) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.tickets + c_first) : "memory");
+            s_last = v == (unsigned)(c_last - c_first);
           }
+          asm volatile("bar.sync 1, %0;" ::"n"(SK_EPI * 32) : "memory");
+          own = s_last != 0;
+          asm volatile("bar.sync 1, %0;" ::"n"(SK_EPI * 32) : "memory");     // s_last reusable
         }
-        const size_t at = (size_t)(row0 + t) * p.n_out + n;
-        if (!GLU && p.residual) r += ldg_act_bf16(p.residual + at);
-        if (p.y_f32) reinterpret_cast<float*>(p.y)[at] = r;
-        else reinterpret_cast<__nv_bfloat16*>(p.y)[at] = __float2bfloat16(r);
-      };
-      if (whole) {
+        if (!own) {
+          // slot 0 of this CTA if the tile began in an earlier one, else slot 1
+          float4* mine = reinterpret_cast<float4*>(p.ws + ((size_t)blockIdx.x * 2 + (kb0 == 0 ? 1 : 0)) * acc_cols * SK_BM) + n_in;
 #pragma unroll 1
-        for (int c = c0; c < cnt && live; c += 32) {
-          uint32_t g[16], up[16];
-          sk_ld16(acc + c, g);
-          if (GLU) sk_ld16(acc + p.xb + c, up);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          for (int c = c0; c < cnt && live; c += 2 * SK_EPI) {
 #pragma unroll
-          for (int k = 0; k < 16; ++k) finish(c + k, __uint_as_float(g[k]), GLU ? __uint_as_float(up[k]) : 0.f);
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tmem_empty[buf]);
-        continue;
-      }
-      // a part of the tile's k range.  CTAs that share the tile: those of its first and last k-block and all between
-      const long long f = (long long)tile * nkb;
-      const int c_first = (int)(((f + 1) * G - 1) / total), c_last = (int)(((f + nkb) * G - 1) / total);
-      // adds to the sums of 16 columns from column c the partials of CTAs q0 .. c_last (k order)
-      auto add_parts = [&](int c, int q0, float (&g)[16], float (&up)[16]) {
-#pragma unroll 2
-        for (int q = q0; q <= c_last; ++q) {              // 8 .. 16 16-byte loads in flight per thread: a round trip to L2 is most of the cost
-          const float4* src = reinterpret_cast<const float4*>(p.ws + ((size_t)q * 2 + (q == c_first ? 1 : 0)) * acc_cols * SK_BM) + n_in + (size_t)(c >> 2) * SK_BM;
-          float4 a[4], b[4];
+            for (int w = 0; w < NW; ++w) {
+              uint32_t v[8];
+              sk_ld8(acc + w * p.xb + c, v);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            a[k] = __ldcg(src + k * SK_BM);
-            if (GLU) b[k] = __ldcg(src + (size_t)((p.xb >> 2) + k) * SK_BM);
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            g[4 * k] += a[k].x; g[4 * k + 1] += a[k].y; g[4 * k + 2] += a[k].z; g[4 * k + 3] += a[k].w;
-            if (GLU) { up[4 * k] += b[k].x; up[4 * k + 1] += b[k].y; up[4 * k + 2] += b[k].z; up[4 * k + 3] += b[k].w; }
-          }
-        }
-      };
-      if (kb0 == 0) {
-        // the tile's first part is its CTA's last segment, so the other parts are usually there already: then it takes them to its own sums
-        // in TMEM and needs neither slot nor ticket
-        if (threadIdx.x == 128) {
-          unsigned v;
-          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.tickets + c_first) : "memory");
-          s_last = v == (unsigned)(c_last - c_first);
-        }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        const bool direct = s_last != 0;
-        asm volatile("bar.sync 1, 256;" ::: "memory");     // s_last reusable
-        if (direct) {
-          __threadfence();
-#pragma unroll 1
-          for (int c = c0; c < cnt && live; c += 32) {
-            uint32_t vg[16], vu[16];
-            sk_ld16(acc + c, vg);
-            if (GLU) sk_ld16(acc + p.xb + c, vu);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            float g[16], up[16];
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-              g[k] = __uint_as_float(vg[k]);
-              up[k] = GLU ? __uint_as_float(vu[k]) : 0.f;
+              for (int k = 0; k < 8; k += 4)
+                __stcg(mine + (size_t)((w * p.xb + c + k) >> 2) * SK_BM, make_float4(__uint_as_float(v[k]), __uint_as_float(v[k + 1]), __uint_as_float(v[k + 2]), __uint_as_float(v[k + 3])));
             }
-            add_parts(c, c_first + 1, g, up);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) finish(c + k, g[k], up[k]);
           }
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0) mbar_arrive(&tmem_empty[buf]);
-          continue;
+          __threadfence();
+          asm volatile("bar.sync 1, %0;" ::"n"(SK_EPI * 32) : "memory");
+          if (threadIdx.x == 128) s_last = atomicAdd(&p.tickets[c_first], 1u) == (unsigned)(c_last - c_first);
+          asm volatile("bar.sync 1, %0;" ::"n"(SK_EPI * 32) : "memory");
+          const bool last = s_last != 0;
+          asm volatile("bar.sync 1, %0;" ::"n"(SK_EPI * 32) : "memory");     // s_last reusable
+          if (!last) continue;
         }
+        __threadfence();
       }
-      // slot 0 of this CTA if the tile began in an earlier one, else slot 1
-      const int wcols = (cnt + 15) & ~15;
-      float* mine = p.ws + ((size_t)blockIdx.x * 2 + (kb0 == 0 ? 1 : 0)) * acc_cols * SK_BM;
 #pragma unroll 1
-      for (int w = 0; w < NW; ++w)
-#pragma unroll 1
-        for (int c = c0; c < wcols && live; c += 32) {
-          uint32_t v[16];
-          sk_ld16(acc + w * p.xb + c, v);
+      for (int c = c0; c < cnt && live; c += 2 * SK_EPI) {
+        float g[8], up[8];
+        uint32_t res[8];
+        const bool in = n < p.n_out;
+        const size_t at = (size_t)(row0 + c) * p.n_out + n;
+        if (!GLU && p.residual) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (in && c + k < cnt) res[k] = ldg_act_u16(p.residual + at + (size_t)k * p.n_out);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) g[k] = up[k] = 0.f;
+        if (own) {
+          uint32_t vg[8], vu[8];
+          sk_ld8(acc + c, vg);
+          if (GLU) sk_ld8(acc + p.xb + c, vu);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int k = 0; k < 16; k += 4)
-            __stcg(reinterpret_cast<uint4*>(mine) + (size_t)((w * p.xb + c + k) >> 2) * SK_BM + n_in, make_uint4(v[k], v[k + 1], v[k + 2], v[k + 3]));
+          for (int k = 0; k < 8; ++k) {
+            g[k] = __uint_as_float(vg[k]);
+            if (GLU) up[k] = __uint_as_float(vu[k]);
+          }
         }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tmem_empty[buf]);
-      __threadfence();
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (threadIdx.x == 128) s_last = atomicAdd(&p.tickets[c_first], 1u) == (unsigned)(c_last - c_first);
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (s_last) {
-        __threadfence();
+        // the other parts in k order, 8 or 12 16-byte loads in flight per thread: a round trip to L2 is most of the cost
+        constexpr int NP = GLU ? 2 : 6;
 #pragma unroll 1
-        for (int c = c0; c < cnt && live; c += 32) {
-          float g[16], up[16];
+        for (int q0 = own ? c_first + 1 : c_first; q0 <= c_last; q0 += NP) {
+          float4 a[NP][2], b[NP][2];
 #pragma unroll
-          for (int k = 0; k < 16; ++k) g[k] = up[k] = 0.f;
-          add_parts(c, c_first, g, up);
+          for (int i = 0; i < NP; ++i) {
+            const int q = q0 + i;
+            const float4* src = reinterpret_cast<const float4*>(p.ws + ((size_t)q * 2 + (q == c_first ? 1 : 0)) * acc_cols * SK_BM) + n_in + (size_t)(c >> 2) * SK_BM;
 #pragma unroll
-          for (int k = 0; k < 16; ++k) finish(c + k, g[k], up[k]);
+            for (int k = 0; k < 2; ++k) {
+              if (q <= c_last) a[i][k] = __ldcg(src + k * SK_BM);
+              if (GLU && q <= c_last) b[i][k] = __ldcg(src + (size_t)((p.xb >> 2) + k) * SK_BM);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < NP; ++i) {
+            if (q0 + i > c_last) break;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              g[4 * k] += a[i][k].x; g[4 * k + 1] += a[i][k].y; g[4 * k + 2] += a[i][k].z; g[4 * k + 3] += a[i][k].w;
+              if (GLU) { up[4 * k] += b[i][k].x; up[4 * k + 1] += b[i][k].y; up[4 * k + 2] += b[i][k].z; up[4 * k + 3] += b[i][k].w; }
+            }
+          }
         }
+        if (GLU) {
+          if (p.act == 4) {       // clamped, shifted gate product
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const float gc = fminf(g[k] + bg, p.limit), uc = fminf(fmaxf(up[k] + bu, -p.limit), p.limit);
+              g[k] = (uc + 1.f) * gc * (1.f / (1.f + __expf(-p.alpha * gc)));
+            }
+          } else if (p.act == 1) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) g[k] = silu(g[k] + bg) * (up[k] + bu);
+          } else if (p.act == 2) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) g[k] = gelu_tanh(g[k] + bg) * (up[k] + bu);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) g[k] = gelu_erf(g[k] + bg) * (up[k] + bu);
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            g[k] += bg;
+            if (p.residual) g[k] += __uint_as_float(res[k] << 16);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (in && c + k < cnt) {
+            if (p.y_f32) reinterpret_cast<float*>(p.y)[at + (size_t)k * p.n_out] = g[k];
+            else reinterpret_cast<__nv_bfloat16*>(p.y)[at + (size_t)k * p.n_out] = __float2bfloat16(g[k]);
+          }
       }
-      asm volatile("bar.sync 1, 256;" ::: "memory");     // s_last reusable
+      if (own) {
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+      }
     }
   }
   if (*stop) __nanosleep(1000000);        // gave up: let copies in flight land before the shared memory goes away

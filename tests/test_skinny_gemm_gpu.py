@@ -84,3 +84,25 @@ def test_a_token_may_name_an_expert_again(N, form):
     got = ops.moe_experts(x, wg, wd, w, i, "silu_mul", offset)
     want = ref.moe_experts(x.float(), wg.float(), wd.float(), w, i, "silu_mul", offset)
     assert _rel(got, want) < 5e-3
+
+
+@pytest.mark.parametrize("T", [6, 7, 8, 24, 25, 41, 96])
+@pytest.mark.parametrize("form", ["residual", "norm", "gate product"])
+def test_groups_of_eight_tokens(T, form):
+    """Rows of 6 .. 8 tokens that fill the streaming kernel's shared memory, and token counts around the epilogue's groups."""
+    K = 16384 if form == "norm" else 14336
+    x = torch.randn(T, K, device=DEV, dtype=BF)
+    w = (torch.randn(1040, K, device=DEV) / math.sqrt(K)).to(BF)
+    kw, kf = {}, {}
+    if form == "residual":
+        r, b = torch.randn(T, 1040, device=DEV, dtype=BF), torch.randn(1040, device=DEV, dtype=BF)
+        kw, kf = dict(residual=r, bias=b), dict(residual=r.float(), bias=b.float())
+    if form == "norm":
+        n = torch.randn(K, device=DEV, dtype=BF)
+        kw, kf = dict(norm_weight=n, norm_eps=1e-5), dict(norm_weight=n.float(), norm_eps=1e-5)
+    if form == "gate product":
+        kw = kf = dict(act="silu_mul")
+    res = kf.get("residual")
+    want = ref.linear(x.float(), w.float(), **{k: v for k, v in kf.items() if k != "residual"})
+    # the normalised rows are rounded to bf16 too
+    assert _rel(ops.linear(x, w, **kw), want if res is None else want + res) < (5e-3 if form == "norm" else 3e-3)
