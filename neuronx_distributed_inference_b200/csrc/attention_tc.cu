@@ -17,8 +17,7 @@
 //   the MMA warp's code (fa_umma), 27 us from the halves of P, 7 us from the mixed-type sums (fa_add_bf16x2), 20 us from masks outside the tiles
 //   that need none.  3 x 1000 tokens of head size 64, window 128: 24 us, 30 before.
 //   A soft cap (tanh) needs nine more fp32 pair operations per pair of scores; they run beside the exponentials, the maximum is taken before the cap and capped
-//   alone.  Three portions with cap, gate and window: 257 us; 267 with the cap as a pass of its own, 255 with the cap's size in the polynomial's coefficients
-//   (other bits for no gain in error).
+//   alone.  Three portions with cap, gate and window: 211 us in a graph (254 before the gate came through shared memory).
 //   Tried and slower: 64-key tiles with two score buffers per query tile (478 us: both tiles' softmax phases fall together, and a hand-over costs as
 //   much per 64 keys); sixteen softmax warps with half a row per thread (482 us); a share of the exponentials as polynomials on the FMA pipe (2 of 16: no
 //   gain, 4 of 16: 1 % slower: the fp32 pair operations cost more clocks than the exponentials they replace); the maximum beside the exponentials of
@@ -52,6 +51,7 @@ constexpr float FA_LOG2E = 1.4426950408889634f;
 
 struct FaParams {
   CUtensorMap tm_q, tm_k, tm_v, tm_o;   // q / o (and contiguous k / v): 4-D {D, heads, T, B}; paged k / v: 3-D {D, kv heads, slots}; boxes of 64 columns
+  CUtensorMap tm_g;                     // the gate, like q (gate_tma)
   const float* sinks;                   // [Hq] or null
   const float* head_scale;              // [Hq] or null: a further factor of the scores of a head
   const __nv_bfloat16* gate;            // [B, T, Hq * D] (or [B, T, Hq] with gate_per_head) with the strides below, or null
@@ -59,7 +59,7 @@ struct FaParams {
   __nv_bfloat16* out;                   // [B, T, Hq, D]
   const int *ctx_len, *q_len, *block_table;   // paged rows
   int max_blocks, page_shift;
-  int gate_per_head, gate_vec;
+  int gate_per_head, gate_tma;
   int B, T, Hq, Hkv, causal, window, keep, chunk, pair_heads;
   float scale, softcap;
   unsigned* wait_word;                  // mbar_wait.cuh
@@ -132,6 +132,11 @@ __device__ __forceinline__ void fa_tmem_ld32(uint32_t taddr, uint32_t* v) {
         "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
       : "r"(taddr));
 }
+__device__ __forceinline__ void fa_tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+                 "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(taddr));
+}
 __device__ __forceinline__ void fa_tmem_st32(uint32_t taddr, const uint32_t* v) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -147,6 +152,15 @@ __device__ __forceinline__ float fa_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// 1 / (1 + e^-g) without a division: its branch for the ends of the range keeps the compiler from running several of them side by side (200 clocks each, one
+// after the other).  The reciprocal's last bit comes from a Newton step, except where 1 + e^-g is infinite or nearly so.
+__device__ __forceinline__ float fa_sigmoid(float g) {
+  const float x = 1.f + expf(-g);
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  const float n = fmaf(r, fmaf(-x, r, 1.f), r);
+  return x < 0x1p126f ? n : r;
 }
 // two fp32 operations per instruction
 __device__ __forceinline__ uint64_t fa_pack2(float a, float b) {
@@ -224,6 +238,7 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_k) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_v) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_o) : "memory");
+    if (p.gate_tma) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_g) : "memory");
     mbar_init(q_full, 1);
     for (int s = 0; s < SLOTS; ++s) {
       mbar_init(&kv_full[s], 1);
@@ -325,6 +340,14 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
             for (int c = 0; c < D / 64; ++c) fa_tma_4d(dst + c * HALF, tm, c * 64, hk, key0, b, &kv_full[s]);
           }
         }
+      }
+      // the gate's tiles follow the last values through the ring: they are there when the epilogue starts
+      for (int x = 0; x < NX && go && p.gate_tma; ++x) {
+        const int it = 2 * n_tiles + x, s = it % SLOTS;
+        go = mbar_wait_warp(&kv_empty[s], (uint32_t)((it / SLOTS) & 1) ^ 1u, stop, p.wait_word);
+        if (!go || lane != 0) continue;
+        mbar_expect(&kv_full[s], TILE);
+        for (int c = 0; c < D / 64; ++c) fa_tma_4d(sKV + s * TILE + c * HALF, &p.tm_g, c * 64, pair ? h_first + x : h_first, pair ? q0 : q0 + x * FA_ROWS, b, &kv_full[s]);
       }
     } else if (warp == W_MMA) {
       // ================= MMA issuer =================
@@ -595,44 +618,69 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
       else tile(std::true_type{}, i, key0);
     }
     // ---- epilogue: O / l (times the gate) -> bf16 -> shared memory -> TMA store (rows past T are clipped, padding rows are zeros)
-    const bool done = mbar_wait_warp(&o_full[x], 0, stop, p.wait_word);
+    bool done = mbar_wait_warp(&o_full[x], 0, stop, p.wait_word);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     float l = l_run;
     if (p.sinks != nullptr) l = (m_run == -INFINITY) ? 1.f : l + fa_ex2(p.sinks[h] * FA_LOG2E - m_run);
     float inv = (m_run == -INFINITY || l == 0.f) ? 0.f : 1.f / l;
     const bool live_row = t < qn;
+    const uint32_t live_mask = live_row ? ~0u : 0u;
+    uint8_t* so = sQ + x * TILE + r * 128;
+    auto put = [&](int col, const float (&f)[8]) {       // 16-byte chunk of the 128-byte row, XOR-swizzled like TMA does
+      // (the choice is made on the packed words: one per element puts each sigmoid behind a branch of its own)
+      *reinterpret_cast<uint4*>(so + (col >> 6) * HALF + ((((col & 63) >> 3) ^ (r & 7)) << 4)) =
+          make_uint4(pack_bf16(f[0], f[1]) & live_mask, pack_bf16(f[2], f[3]) & live_mask, pack_bf16(f[4], f[5]) & live_mask, pack_bf16(f[6], f[7]) & live_mask);
+    };
     const __nv_bfloat16* gp = nullptr;
     if (p.gate != nullptr && live_row) {
       gp = p.gate + (long long)b * p.g_sb + (long long)t * p.g_st + (p.gate_per_head ? h : h * D);
       if (p.gate_per_head) inv *= 1.f / (1.f + expf(-__bfloat162float(*gp)));
     }
-    uint8_t* so = sQ + x * TILE + r * 128;
+    if (p.gate != nullptr && !p.gate_per_head) {
+      // The gate's tile is in shared memory, and the sigmoids of 16 columns run side by side; read from global memory where it is used, with a branch per
+      // element (for the division and for padding rows), the gate took 13 us of a CTA's last 16 (now 4.5; no gate: 0.9).
+      const int it = 2 * n_tiles + x;
+      const uint8_t* sg = sKV + (it % SLOTS) * TILE + r * 128;
+      if (p.gate_tma) done = mbar_wait_warp(&kv_full[it % SLOTS], (uint32_t)((it / SLOTS) & 1), stop, p.wait_word) && done;
 #pragma unroll 1
-    for (int c0 = 0; c0 < D; c0 += 32) {
-      uint32_t o[32];
-      fa_tmem_ld32(tO + c0, o);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      for (int c0 = 0; c0 < D; c0 += 16) {
+        uint32_t o[16], w[8];
+        fa_tmem_ld16(tO + c0, o);
+        if (p.gate_tma) {
 #pragma unroll
-      for (int e = 0; e < 32; e += 8) {
-        float f[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) f[k] = live_row ? __uint_as_float(o[e + k]) * inv : 0.f;
-        if (gp != nullptr && !p.gate_per_head) {
-          float g[8];
-          if (p.gate_vec) {
-            const uint4 w = ldg_act(gp + c0 + e);
-            g[0] = bf16lo(w.x); g[1] = bf16hi(w.x); g[2] = bf16lo(w.y); g[3] = bf16hi(w.y);
-            g[4] = bf16lo(w.z); g[5] = bf16hi(w.z); g[6] = bf16lo(w.w); g[7] = bf16hi(w.w);
-          } else {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) g[k] = ldg_act_bf16(gp + c0 + e + k);
+          for (int k = 0; k < 2; ++k) {
+            const uint4 q = *reinterpret_cast<const uint4*>(sg + (c0 >> 6) * HALF + (((((c0 & 63) >> 3) + k) ^ (r & 7)) << 4));
+            w[4 * k] = q.x; w[4 * k + 1] = q.y; w[4 * k + 2] = q.z; w[4 * k + 3] = q.w;
           }
+        } else {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) f[k] *= 1.f / (1.f + expf(-g[k]));
+          for (int k = 0; k < 8; ++k) w[k] = live_row ? ldg_act_u16(gp + c0 + 2 * k) | ldg_act_u16(gp + c0 + 2 * k + 1) << 16 : 0u;
         }
-        const int ch = ((c0 & 63) + e) >> 3;             // 16-byte chunk of the 128-byte row, XOR-swizzled like TMA does
-        *reinterpret_cast<uint4*>(so + (c0 >> 6) * HALF + ((ch ^ (r & 7)) << 4)) =
-            make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int k = 0; k < 16; k += 8) {
+          float f[8];
+#pragma unroll
+          for (int e = 0; e < 8; e += 2) {
+            f[e] = __uint_as_float(o[k + e]) * inv * fa_sigmoid(bf16lo(w[(k + e) >> 1]));
+            f[e + 1] = __uint_as_float(o[k + e + 1]) * inv * fa_sigmoid(bf16hi(w[(k + e) >> 1]));
+          }
+          put(c0 + k, f);
+        }
+      }
+    } else {
+#pragma unroll 1
+      for (int c0 = 0; c0 < D; c0 += 32) {
+        uint32_t o[32];
+        fa_tmem_ld32(tO + c0, o);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int e = 0; e < 32; e += 8) {
+          float f[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) f[k] = __uint_as_float(o[e + k]) * inv;
+          put(c0 + e, f);
+        }
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -732,7 +780,7 @@ void attention_prefill_tc_launch(const void* q, const void* k, const void* v, vo
 
 // Prompt portions over a paged cache.  Sizes this kernel takes: keys and values of one size, 64 or 128, rows on 16-byte boundaries, pages of
 // 2^k >= 8 tokens (smaller ones would break the 8-row swizzle atoms), no distance term; the rest is paged_window_attention_mma_kernel's.
-// 3 rows of up to 1024 tokens over contexts up to 3000, 32 / 8 heads x 128, window 2048, cap, gate: 0.257 ms, mma.sync kernel 0.89 ms.
+// 3 rows of up to 1024 tokens over contexts up to 3000, 32 / 8 heads x 128, window 2048, cap, gate: 0.21 ms, mma.sync kernel 0.89 ms.
 bool paged_attention_tc_supported(const WindowAttnParams& p, bool lp) {
   return lp && p.T >= 16 && p.maps != 2 && p.slopes == nullptr && p.D == p.Dv && (p.D == 64 || p.D == 128) && (p.v_rs * 2) % 16 == 0 && p.page >= 8 &&
          (p.page & (p.page - 1)) == 0 && (long long)p.B * p.Hq * ((p.T + FA_ROWS - 1) / FA_ROWS) <= 0x7fffffffLL &&
@@ -748,7 +796,12 @@ void paged_attention_tc_launch(const WindowAttnParams& w, long long slots, cudaS
   p.out = reinterpret_cast<__nv_bfloat16*>(w.out);
   p.sinks = w.sinks; p.head_scale = w.head_scale;
   p.gate = reinterpret_cast<const __nv_bfloat16*>(w.gate); p.g_sb = w.g_sb; p.g_st = w.g_st; p.gate_per_head = w.gate_per_head;
-  p.gate_vec = (reinterpret_cast<uintptr_t>(w.gate) % 16 == 0 && (w.g_sb * 2) % 16 == 0 && (w.g_st * 2) % 16 == 0) ? 1 : 0;
+  const long long g_sb = w.B == 1 ? w.T * w.g_st : w.g_sb;
+  p.gate_tma = w.gate != nullptr && !w.gate_per_head && reinterpret_cast<uintptr_t>(w.gate) % 16 == 0 && g_sb > 0 && g_sb % 8 == 0 && w.g_st > 0 && w.g_st % 8 == 0 ? 1 : 0;
+  if (p.gate_tma) {
+    const long long gd[4] = {w.D, w.Hq, w.T, w.B}, gs[4] = {1, w.D, w.g_st, g_sb};
+    fa_make_map(&p.tm_g, w.gate, 4, gd, gs, FA_ROWS);
+  }
   p.ctx_len = w.ctx_len; p.q_len = w.q_len; p.block_table = w.block_table; p.max_blocks = w.max_blocks;
   while ((1 << p.page_shift) < w.page) ++p.page_shift;
   p.B = w.B; p.T = w.T; p.Hq = w.Hq; p.Hkv = w.G; p.causal = 1; p.window = w.window; p.keep = w.keep_first; p.chunk = w.chunk;

@@ -48,11 +48,12 @@ __device__ __forceinline__ uint4 ldg_act(const void* p) {
   asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
   return r;
 }
-__device__ __forceinline__ float ldg_act_bf16(const __nv_bfloat16* p) {
+__device__ __forceinline__ uint32_t ldg_act_u16(const __nv_bfloat16* p) {
   unsigned short r;
   asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(r) : "l"(p));
-  return __uint_as_float(((uint32_t)r) << 16);
+  return r;
 }
+__device__ __forceinline__ float ldg_act_bf16(const __nv_bfloat16* p) { return __uint_as_float(ldg_act_u16(p) << 16); }
 
 __device__ __forceinline__ float bf16lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }

@@ -72,11 +72,6 @@ __device__ __forceinline__ void sk_ld8(uint32_t taddr, uint32_t (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
 }
-__device__ __forceinline__ uint32_t ldg_act_u16(const __nv_bfloat16* p) {
-  unsigned short r;
-  asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(r) : "l"(p));
-  return r;
-}
 
 template <bool GLU>
 __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid_constant__ SkinnyKernelParams p) {

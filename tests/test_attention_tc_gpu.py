@@ -161,3 +161,21 @@ def test_soft_cap_of_scores_below_the_range():
         got = ops.paged_window_attention(q, k, v, table, c, m, D ** -0.5, cap, 0, 0)
         want = ref.paged_window_attention(q.float(), k.float(), v.float(), table, c, m, D ** -0.5, cap, 0, 0)
         assert _rel(got, want) < 4e-3
+
+
+@pytest.mark.parametrize("D,B,T,Hq,G", [(128, 1, 40, 4, 2), (128, 5, 300, 8, 2), (64, 3, 140, 8, 8)])
+@pytest.mark.parametrize("at", [0, 8, 3])
+def test_gate_rows_of_a_wider_tensor(D, B, T, Hq, G, at):
+    """The gate comes as tiles where its rows lie on 16 bytes, else element by element; the ends of the sigmoid's range, infinities, and padding rows that hold NaN."""
+    ctx, n = [0, 77, 130, 64, 1000][:B], [T, T - 30, 0, T // 2, 290][:B]
+    q, dirty, clean, table, c, m = _paged(B, T, Hq, G, D, 64, ctx, n)
+    wide = torch.randn(B, T, Hq * D + 8, device=DEV, dtype=torch.bfloat16) * 4
+    wide[:, 5] = torch.tensor([100.0, -100.0, 3e38, -3e38, float("inf"), -float("inf"), 88.5, -88.5], device=DEV).bfloat16().repeat(Hq * D // 8 + 1)
+    for b in range(B):
+        wide[b, n[b]:] = float("nan")
+    gate = wide[..., at:at + Hq * D]
+    got = ops.paged_window_attention(q, *dirty, table, c, m, D ** -0.5, 0.0, 0, 0, gate)
+    want = ref.paged_window_attention(q.float(), *(t.float() for t in clean), table, c, m, D ** -0.5, 0.0, 0, 0, gate.nan_to_num(0.0, float("inf"), -float("inf")).float())
+    assert torch.isfinite(got).all() and _rel(got, want) < 4e-3
+    for b in range(B):
+        assert not got[b, n[b]:].any()
