@@ -17,7 +17,8 @@
 //   the MMA warp's code (fa_umma), 27 us from the halves of P, 7 us from the mixed-type sums (fa_add_bf16x2), 20 us from masks outside the tiles
 //   that need none.  3 x 1000 tokens of head size 64, window 128: 24 us, 30 before.
 //   A soft cap (tanh) needs nine more fp32 pair operations per pair of scores; they run beside the exponentials, the maximum is taken before the cap and capped
-//   alone.  Three portions with cap, gate and window: 211 us in a graph (254 before the gate came through shared memory).
+//   alone.  Three portions with cap, gate and window: 208 us in a graph (254 before the gate came
+//   through shared memory; 193 with a shorter polynomial up to half the cap, but 290 .. 340 for scores between that and the cap, which then take both).
 //   Tried and slower: 64-key tiles with two score buffers per query tile (478 us: both tiles' softmax phases fall together, and a hand-over costs as
 //   much per 64 keys); sixteen softmax warps with half a row per thread (482 us); a share of the exponentials as polynomials on the FMA pipe (2 of 16: no
 //   gain, 4 of 16: 1 % slower: the fp32 pair operations cost more clocks than the exponentials they replace); the maximum beside the exponentials of
@@ -47,6 +48,7 @@
 namespace nxdi {
 
 constexpr int FA_ROWS = 128;                   // queries per tile = keys per tile
+constexpr int FA_SHORT = 6;                    // key tiles of a CTA that does not wait for the large code of a tile (capped_tile)
 constexpr float FA_LOG2E = 1.4426950408889634f;
 
 struct FaParams {
@@ -137,6 +139,11 @@ __device__ __forceinline__ void fa_tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) 
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
                  "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(taddr));
 }
+__device__ __forceinline__ void fa_tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+               : "memory");
+}
 __device__ __forceinline__ void fa_tmem_st32(uint32_t taddr, const uint32_t* v) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -189,13 +196,19 @@ __device__ __forceinline__ void fa_add_bf16x2(float& s_lo, float& s_hi, uint32_t
   asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.bf16 %0, l, %0;\n\tadd.rn.f32.bf16 %1, h, %1;\n\t}" : "+f"(s_lo), "+f"(s_hi) : "r"(w));
 }
 // tanh on |x| <= 1: x times a polynomial in x^2 (weighted least squares on Chebyshev nodes, relative error 1.7e-7 with fp32 arithmetic)
-__device__ __forceinline__ uint64_t fa_tanh2_small(uint64_t x) {
+__device__ __forceinline__ uint64_t fa_tanh2_unit(uint64_t x) {
   const float t[7] = {0.00104102155f, -0.00620337576f, 0.0202899761f, -0.0534570292f, 0.13325204f, -0.333328396f, 0.99999994f};
   const uint64_t u = fa_mul2(x, x);
   uint64_t r = fa_pack2(t[0], t[0]);
 #pragma unroll
   for (int i = 1; i < 7; ++i) r = fa_fma2(r, u, fa_pack2(t[i], t[i]));
   return fa_mul2(x, r);
+}
+// tanh on |x| > 1: 1 - 2 / (1 + e^2|x|), without the branches of tanhf
+__device__ __forceinline__ float fa_tanh_large(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + fa_ex2(fabsf(x) * (2.f * FA_LOG2E))));
+  return copysignf(fmaf(-2.f, r, 1.f), x);
 }
 
 template <int D, int NX>
@@ -451,7 +464,29 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
     const int lb_min = reach(w_pos), lb_max = reach(w_pos + 31);
     const float hs = p.head_scale ? p.scale * p.head_scale[h] : p.scale;
     float m_run = -INFINITY, l_run = 0.f;
-    auto tile = [&](auto masked, int i, int key0) {
+    // O = alpha O: P V of the tile before has retired
+    auto rescale = [&](auto cols, float alpha) {
+      constexpr int C = decltype(cols)::value;
+#pragma unroll 1
+      for (int c0 = 0; c0 < D; c0 += C) {
+        uint32_t o[C];
+#pragma unroll
+        for (int c = 0; c < C; c += 32) fa_tmem_ld32(tO + c0 + c, o + c);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int e = 0; e < C; e += 2) {
+          float a, d;
+          fa_unpack2(fa_mul2(fa_pack2(__uint_as_float(o[e]), __uint_as_float(o[e + 1])), fa_pack2(alpha, alpha)), a, d);
+          o[e] = __float_as_uint(a);
+          o[e + 1] = __float_as_uint(d);
+        }
+#pragma unroll
+        for (int c = 0; c < C; c += 32) fa_tmem_st32(tO + c0 + c, o + c);
+      }
+    };
+    const float to_cap = CAP ? hs / p.softcap : 0.f;     // scores -> what the soft cap takes the tanh of
+    const uint64_t tc2 = fa_pack2(to_cap, to_cap);
+    auto tile = [&](auto masked, int i, int key0) {      // false: nothing done, scores beyond the cap
       constexpr bool MASKED = decltype(masked)::value;
       uint32_t v[128];
 #pragma unroll
@@ -467,27 +502,24 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
           dead[c] = k0 > up_max || (k0 + 63 < lb_min && k0 >= keep);
         }
       }
-      bool slow[2] = {false, false};                     // halves with scores beyond the cap (|x| > 1): tanhf for those scores
-      if (CAP) {
+      if constexpr (CAP) {
         // v = score / cap from here on; the cap itself is taken beside the exponentials, the maximum's alone before them (it is increasing)
-        const float to_cap = hs / p.softcap;
-        const uint64_t tc2 = fa_pack2(to_cap, to_cap);
+        float big[2] = {0.f, 0.f};
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           if (dead[c]) continue;
-          float big = 0.f;
 #pragma unroll
           for (int e = 64 * c; e < 64 * c + 64; e += 2) {
             float a, d;
             fa_unpack2(fa_mul2(fa_pack2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), tc2), a, d);
             v[e] = __float_as_uint(a);
             v[e + 1] = __float_as_uint(d);
-            big = fmaxf(big, fmaxf(fabsf(a), fabsf(d)));
+            big[c] = fmaxf(big[c], fmaxf(fabsf(a), fabsf(d)));
           }
-          // taken over scores that the row does not see too (later keys, rows of pages that were not fetched, whatever shared memory held): both
-          // ways give a score the same bits
-          slow[c] = __any_sync(0xffffffffu, !(big <= 1.f));
         }
+        // Looked for over scores that the row does not see too (later keys, rows of pages that were not fetched, whatever shared memory held): both ways give a
+        // score the same bits.
+        if (__any_sync(0xffffffffu, !(fmaxf(big[0], big[1]) <= 1.f))) return false;
         scl = p.softcap * FA_LOG2E;
       } else if (!(scl > 0.f)) {                         // a head's factor may be zero or negative: the maximum below needs a positive scale
 #pragma unroll
@@ -524,40 +556,18 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
       }
       const float mx_raw = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       float mx = (mx_raw == -INFINITY) ? -INFINITY : mx_raw * scl;
-      if (CAP) {
-        // a row that sees keys has a maximum, of scores below fp32's range too: -cap
-        const bool any = !MASKED || (!dead[0] && (see[0] | see[1]) != 0u) || (!dead[1] && (see[2] | see[3]) != 0u);
+      if (CAP && mx_raw > -INFINITY) {
         float t, unused;
-        fa_unpack2(fa_tanh2_small(fa_pack2(mx_raw, mx_raw)), t, unused);
-        mx = any ? (fabsf(mx_raw) <= 1.f ? t : tanhf(mx_raw)) * scl : -INFINITY;
+        fa_unpack2(fa_tanh2_unit(fa_pack2(mx_raw, mx_raw)), t, unused);
+        mx = t * scl;
       }
       const bool grow = mx > m_run + SLACK || (m_run == -INFINITY && mx > -INFINITY);
       const float m_new = grow ? mx : m_run;
       const float alpha = (m_run == -INFINITY) ? 0.f : fa_ex2(m_run - m_new);
       const bool move = i > 0 && __any_sync(0xffffffffu, grow);
-      l_run *= alpha;
+
       m_run = m_new;
-      // O = alpha O: P V of the tile before has retired
-      auto rescale = [&](auto cols) {
-        constexpr int C = decltype(cols)::value;
-#pragma unroll 1
-        for (int c0 = 0; c0 < D; c0 += C) {
-          uint32_t o[C];
-#pragma unroll
-          for (int c = 0; c < C; c += 32) fa_tmem_ld32(tO + c0 + c, o + c);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int e = 0; e < C; e += 2) {
-            float a, d;
-            fa_unpack2(fa_mul2(fa_pack2(__uint_as_float(o[e]), __uint_as_float(o[e + 1])), fa_pack2(alpha, alpha)), a, d);
-            o[e] = __float_as_uint(a);
-            o[e + 1] = __float_as_uint(d);
-          }
-#pragma unroll
-          for (int c = 0; c < C; c += 32) fa_tmem_st32(tO + c0 + c, o + c);
-        }
-      };
-      if (SLACK > 0.f && move) rescale(std::integral_constant<int, 32>{});       // seldom: in few registers, beside the scores
+      if (SLACK > 0.f && move) rescale(std::integral_constant<int, 32>{}, alpha);       // seldom: in few registers, beside the scores
       // ---- P = exp2(v * scl - m) -> bf16 -> TMEM, over the scores, 64 keys at a time: their P V runs while the next are exponentiated
       const float neg_m = (m_run == -INFINITY) ? 0.f : -m_run;
       const uint64_t scl2 = fa_pack2(scl, scl), neg2 = fa_pack2(neg_m, neg_m);
@@ -568,28 +578,12 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
         if (dead[c]) {
 #pragma unroll
           for (int e = 0; e < 32; ++e) pk[e] = 0u;
-        } else if (CAP && slow[c]) {
-#pragma unroll
-          for (int e = 0; e < 64; e += 2) {
-            const float s0 = __uint_as_float(v[64 * c + e]), s1 = __uint_as_float(v[64 * c + e + 1]);
-            float a, bb;
-            fa_unpack2(fa_fma2(fa_tanh2_small(fa_pack2(s0, s1)), scl2, neg2), a, bb);
-            if (!(fabsf(s0) <= 1.f)) a = fmaf(tanhf(s0), scl, neg_m);
-            if (!(fabsf(s1) <= 1.f)) bb = fmaf(tanhf(s1), scl, neg_m);
-            if (MASKED) {
-              if (!(see[2 * c + (e >> 5)] & (1u << (e & 31)))) a = -INFINITY;
-              if (!(see[2 * c + (e >> 5)] & (2u << (e & 31)))) bb = -INFINITY;
-            }
-            const uint32_t w = pack_bf16(fa_ex2(a), fa_ex2(bb));
-            fa_add_bf16x2(ls[e & 2], ls[(e & 2) + 1], w);
-            pk[e >> 1] = w;
-          }
         } else {
 #pragma unroll
           for (int e = 0; e < 64; e += 2) {
             const uint64_t v2 = fa_pack2(__uint_as_float(v[64 * c + e]), __uint_as_float(v[64 * c + e + 1]));
             float a, bb;
-            fa_unpack2(fa_fma2(CAP ? fa_tanh2_small(v2) : v2, scl2, neg2), a, bb);
+            fa_unpack2(fa_fma2(CAP ? fa_tanh2_unit(v2) : v2, scl2, neg2), a, bb);
             if (CAP && MASKED) {                         // the cap of a masked score is no -inf
               if (!(see[2 * c + (e >> 5)] & (1u << (e & 31)))) a = -INFINITY;
               if (!(see[2 * c + (e >> 5)] & (2u << (e & 31)))) bb = -INFINITY;
@@ -601,21 +595,129 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
           }
         }
         fa_tmem_st32(tS + 32 * c, pk);
-        if (SLACK == 0.f && c == 0 && move) rescale(std::integral_constant<int, 64>{});      // often: in the registers of the first scores
+        if (SLACK == 0.f && c == 0 && move) rescale(std::integral_constant<int, 64>{}, alpha);      // often: in the registers of the first scores
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(c == 0 ? &p_half[x] : &p_full[x]);
       }
-      l_run += (ls[0] + ls[2]) + (ls[1] + ls[3]);
+      l_run = fmaf(l_run, alpha, (ls[0] + ls[2]) + (ls[1] + ls[3]));
+      return true;
     };
+    // Soft cap, tiles with scores beyond the cap and CTAs of few key tiles: 64 or 32 keys at a time, the scores read from TMEM twice, in loops that are not unrolled
+    // (the same bits).  Slower per tile once `tile` is in the instruction cache (254 against 207 us for the three portions named above), but a tenth of its code: four
+    // portions of up to 287 tokens with a window of 500 38 us, 44 with `tile`; where an SM has one CTA alone (20 tokens: 16 CTAs) 27 and 25.  Scores up to twice
+    // the cap: 323 us, 1156 with a tanhf behind a branch for each of them in `tile`.
+    auto capped_tile = [&](int i, int key0) {
+      const float scl = p.softcap * FA_LOG2E;
+      auto visible = [&](int k0) {                       // which of 32 keys this row sees
+        const int e_hi = up - k0, e_lo = lb - k0, e_keep = keep - k0;
+        const uint32_t m_hi = e_hi >= 31 ? ~0u : e_hi < 0 ? 0u : (2u << e_hi) - 1u;
+        const uint32_t m_lo = e_lo <= 0 ? ~0u : e_lo > 31 ? 0u : ~0u << e_lo;
+        const uint32_t m_keep = e_keep > 31 ? ~0u : e_keep <= 0 ? 0u : (1u << e_keep) - 1u;
+        return m_hi & (m_lo | m_keep);
+      };
+      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      uint32_t any = 0u;
+#pragma unroll 1
+      for (int c = 0; c < 2; ++c) {
+        const uint32_t see[2] = {visible(key0 + 64 * c), visible(key0 + 64 * c + 32)};
+        any |= see[0] | see[1];
+        uint32_t v[64];
+        fa_tmem_ld32(tS + 64 * c, v);
+        fa_tmem_ld32(tS + 64 * c + 32, v + 32);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int e = 0; e < 64; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * to_cap);
+        if (__any_sync(0xffffffffu, (see[0] & see[1]) != ~0u)) {
+#pragma unroll
+          for (int e = 0; e < 64; ++e)
+            if (!(see[e >> 5] & (1u << (e & 31)))) v[e] = 0xff800000u;      // -inf
+        }
+#pragma unroll
+        for (int e = 0; e < 64; e += 8)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) m4[k] = fmaxf(m4[k], fmaxf(__uint_as_float(v[e + 2 * k]), __uint_as_float(v[e + 2 * k + 1])));
+      }
+      const float mx_raw = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+      // the cap is increasing: the maximum alone is capped.  A row that sees keys has one, of scores below fp32's range too: -cap
+      float mx;
+      {
+        float a, unused;
+        fa_unpack2(fa_tanh2_unit(fa_pack2(mx_raw, mx_raw)), a, unused);
+        mx = any != 0u ? (fabsf(mx_raw) <= 1.f ? a : fa_tanh_large(mx_raw)) * scl : -INFINITY;
+      }
+      const bool grow = mx > m_run + SLACK || (m_run == -INFINITY && mx > -INFINITY);
+      const float m_new = grow ? mx : m_run;
+      const float alpha = (m_run == -INFINITY) ? 0.f : fa_ex2(m_run - m_new);
+      if (i > 0 && __any_sync(0xffffffffu, grow)) rescale(std::integral_constant<int, 32>{}, alpha);
+
+      m_run = m_new;
+      const float neg_m = (m_run == -INFINITY) ? 0.f : -m_run;
+      const uint64_t scl2 = fa_pack2(scl, scl), neg2 = fa_pack2(neg_m, neg_m);
+      float ls[4] = {0.f, 0.f, 0.f, 0.f};
+      uint32_t v[32];
+      fa_tmem_ld32(tS, v);
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {
+        const uint32_t see = visible(key0 + 32 * c);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        float t[32], big = 0.f;
+#pragma unroll
+        for (int e = 0; e < 32; e += 2) {
+          float a, d;
+          const uint64_t y = fa_mul2(fa_pack2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), tc2);
+          fa_unpack2(y, a, d);
+          fa_unpack2(fa_tanh2_unit(y), t[e], t[e + 1]);
+          big = fmaxf(big, fmaxf(fabsf(a), fabsf(d)));
+        }
+        if (__any_sync(0xffffffffu, !(big <= 1.f))) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            const float a = __uint_as_float(v[e]) * to_cap, la = fa_tanh_large(a);
+            t[e] = fabsf(a) <= 1.f ? t[e] : la;
+          }
+        }
+        if (c < 3) fa_tmem_ld32(tS + 32 * c + 32, v);      // the next scores, beside the exponentials
+        if (__any_sync(0xffffffffu, see != ~0u)) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (!(see & (1u << e))) t[e] = -INFINITY;
+        }
+        uint32_t pk[16];
+#pragma unroll
+        for (int e = 0; e < 32; e += 2) {
+          float a, d;
+          fa_unpack2(fa_fma2(fa_pack2(t[e], t[e + 1]), scl2, neg2), a, d);
+          const uint32_t w = pack_bf16(fa_ex2(a), fa_ex2(d));          // -inf -> 0
+          fa_add_bf16x2(ls[e & 2], ls[(e & 2) + 1], w);
+          pk[e >> 1] = w;
+        }
+        fa_tmem_st16(tS + 16 * c, pk);
+        if (c & 1) {
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(c == 1 ? &p_half[x] : &p_full[x]);
+        }
+      }
+      l_run = fmaf(l_run, alpha, (ls[0] + ls[2]) + (ls[1] + ls[3]));
+    };
+    bool large = n_tiles <= FA_SHORT && gridDim.x > kNumSMs;      // or a tile of this warp had scores beyond the cap: no more tries
     for (int i = 0; i < n_tiles; ++i) {
       const int key0 = key_at(i);
       if (!mbar_wait_warp(&s_full[x], (uint32_t)(i & 1), stop, p.wait_word)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // masks only in a tile that has keys which some row of the warp does not see
-      if (key0 + FA_ROWS - 1 <= up_min && (key0 >= lb_max || key0 + FA_ROWS <= keep)) tile(std::false_type{}, i, key0);
-      else tile(std::true_type{}, i, key0);
+      const bool plain = key0 + FA_ROWS - 1 <= up_min && (key0 >= lb_max || key0 + FA_ROWS <= keep);
+      if constexpr (CAP) {
+        if (!large) large = !(plain ? tile(std::false_type{}, i, key0) : tile(std::true_type{}, i, key0));
+        if (large) capped_tile(i, key0);
+      } else if (plain) {
+        tile(std::false_type{}, i, key0);
+      } else {
+        tile(std::true_type{}, i, key0);
+      }
     }
     // ---- epilogue: O / l (times the gate) -> bf16 -> shared memory -> TMA store (rows past T are clipped, padding rows are zeros)
     bool done = mbar_wait_warp(&o_full[x], 0, stop, p.wait_word);

@@ -179,3 +179,20 @@ def test_gate_rows_of_a_wider_tensor(D, B, T, Hq, G, at):
     assert torch.isfinite(got).all() and _rel(got, want) < 4e-3
     for b in range(B):
         assert not got[b, n[b]:].any()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("std", [1.0, 4.0, 12.0, 1e20])
+@pytest.mark.parametrize("mask", [dict(), dict(window=100, keep=4), dict(chunk=96)])
+def test_cap_of_many_short_rows(D, std, mask):
+    """More CTAs than SMs, few key tiles each: the small code, with scores below, around and beyond the cap."""
+    ctx, n = (0, 517, 130, 64), (300, 16, 0, 129)
+    q, dirty, clean, table, c, m = _paged(4, 300, 16, 4, D, 64, ctx, n)
+    args = (table, c, m, D ** -0.5, 20.0, mask.get("window", 0), mask.get("keep", 0))
+    q = q * std
+    kw = dict(chunk=mask.get("chunk"), head_scale=torch.linspace(-0.8, 2.0, 16, device=DEV))
+    got = ops.paged_window_attention(q, *dirty, *args, **kw)
+    want = ref.paged_window_attention(q.double(), *(t.double() for t in clean), *args, **dict(kw, head_scale=kw["head_scale"].double()))
+    assert torch.isfinite(got).all() and _rel(got, want) < 4e-3
+    alone = ops.paged_window_attention(q[:1], *dirty, table[:1], c[:1], m[:1], *args[3:], **kw)      # fewer CTAs: the unrolled code, where the scores allow it
+    assert torch.equal(got[:1], alone)
