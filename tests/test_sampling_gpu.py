@@ -49,3 +49,18 @@ def test_more_rows_than_a_grid_dimension():
     one = torch.ones(B, device="cuda")
     got = ops.sample(logits, torch.ones(B, device="cuda", dtype=torch.int32), one, one, one * 0.5)
     assert torch.equal(got, logits.argmax(-1))
+
+
+@pytest.mark.parametrize("near", [1, 40, 70, 400, 32000])
+@pytest.mark.parametrize("k", [1, 50, 200])
+def test_values_that_share_their_leading_bytes(k, near):
+    """The bound's last bytes are looked at only where many groups share the leading ones."""
+    B, V = 4, 32000
+    logits = torch.randn(B, V)
+    for b in range(B):
+        at = torch.randperm(V)[:near]
+        logits[b, at] = 8.0 + torch.randperm(near).float() * 1e-6       # one 16-bit prefix
+    one = torch.ones(B)
+    top_k, rand = torch.full((B,), k, dtype=torch.int32), torch.rand(B)
+    got = ops.sample(logits.cuda(), top_k.cuda(), one.cuda(), one.cuda(), rand.cuda())
+    assert torch.equal(got.cpu(), ref.sample(logits, top_k, one, one, rand))
