@@ -68,8 +68,10 @@ struct GemmRsArgs {
 };
 void gemm_tcgen05_launch(const void* a, int lda, const void* b, const void* bias, const void* residual, void* c, int ldc, int M,
                          int N, int K, int act, cudaStream_t stream, const GemmRsArgs* rs = nullptr, bool w_fresh = false);
+// clear: n_clear words set to zero on the way (fewer than 1024 rows)
 void rmsnorm_launch(const void* x, const void* res_in, const void* w, void* y, void* res_out, int rows, int H, float eps,
-                    float offset, cudaStream_t stream);
+                    float offset, cudaStream_t stream,
+                    unsigned* clear = nullptr, int n_clear = 0);
 
 void rope_kv_append_launch(const void* qkv, const float* cos, const float* sin, void* q_out, void* k_cache, void* v_cache,
                            const int* lines, const int* positions, const void* q_norm, const void* k_norm, float eps, int B,

@@ -23,21 +23,33 @@ static inline const void* optr(const c10::optional<at::Tensor>& t) { return t.ha
 static inline bool is_bf16(const at::Tensor& t) { return t.scalar_type() == at::kBFloat16; }
 
 // ---- rmsnorm ------------------------------------------------------------------------------------------
-std::tuple<at::Tensor, at::Tensor> rmsnorm(const at::Tensor& x, const at::Tensor& w, double eps, double offset,
-                                           const c10::optional<at::Tensor>& residual) {
-  TORCH_CHECK(x.is_cuda() && x.dim() == 2 && is_bf16(x) && x.is_contiguous() && is_bf16(w));
-  const int rows = x.size(0), H = x.size(1);
+// x [.., H], a residual like it; clear: words set to zero on the way (the tickets of the GEMM that follows)
+static at::Tensor rmsnorm_rows(const at::Tensor& x, const at::Tensor& w, double eps, double offset, const at::Tensor* residual, at::Tensor* res_out,
+                               unsigned* clear = nullptr, int n_clear = 0) {
+  TORCH_CHECK(x.is_cuda() && is_bf16(x) && x.is_contiguous() && is_bf16(w));
+  const int64_t H = x.size(-1), rows = H ? x.numel() / H : 0;
   TORCH_CHECK(H % 8 == 0 && H <= 16384, "rmsnorm: hidden must be a multiple of 8 and <= 16384");
   c10::cuda::CUDAGuard guard(x.device());
   auto y = at::empty_like(x);
-  at::Tensor res_out;
-  if (residual.has_value()) {
-    TORCH_CHECK(residual->is_contiguous() && residual->sizes() == x.sizes() && is_bf16(*residual));
-    res_out = at::empty_like(x);
+  if (residual != nullptr) {
+    TORCH_CHECK(residual->is_contiguous() && residual->numel() == x.numel() && residual->size(-1) == H && is_bf16(*residual));
+    *res_out = at::empty_like(x);
   }
-  rmsnorm_launch(x.data_ptr(), optr(residual), w.data_ptr(), y.data_ptr(), res_out.defined() ? res_out.data_ptr() : nullptr,
-                 rows, H, (float)eps, (float)offset, cur_stream());
-  return {y, res_out.defined() ? res_out : y};
+  rmsnorm_launch(x.data_ptr(), residual != nullptr ? residual->data_ptr() : nullptr, w.data_ptr(), y.data_ptr(), residual != nullptr ? res_out->data_ptr() : nullptr,
+                 (int)rows, (int)H, (float)eps, (float)offset, cur_stream(), clear, n_clear);
+  return y;
+}
+std::tuple<at::Tensor, at::Tensor> rmsnorm(const at::Tensor& x, const at::Tensor& w, double eps, double offset, const c10::optional<at::Tensor>& residual) {
+  TORCH_CHECK(x.dim() >= 1);
+  const auto xc = x.contiguous();          // (a slice of a wider projection arrives strided)
+  if (!residual.has_value()) {
+    auto y = rmsnorm_rows(xc, w, eps, offset, nullptr, nullptr);
+    return {y, y};
+  }
+  at::Tensor r;
+  const auto rc = residual->contiguous();
+  auto y = rmsnorm_rows(xc, w, eps, offset, &rc, &r);
+  return {y, r};
 }
 
 struct Scratch {
@@ -100,7 +112,7 @@ static void fill_params(GemvParams& p, const at::Tensor& x, const at::Tensor& w,
 static at::Tensor prenorm_if_needed(const at::Tensor& x, const c10::optional<at::Tensor>& norm_w, double eps, double offset,
                                     bool& x_in_smem) {
   x_in_smem = gemv_smem_bytes(x.size(0), x.size(1), true) <= 220 * 1024;
-  if (!x_in_smem && norm_w.has_value()) return std::get<0>(rmsnorm(x.contiguous(), *norm_w, eps, offset, c10::nullopt));
+  if (!x_in_smem && norm_w.has_value()) return rmsnorm_rows(x.contiguous(), *norm_w, eps, offset, nullptr, nullptr);
   return x;
 }
 
@@ -123,18 +135,20 @@ static bool skinny_pays(int M, int rows, int K, bool glu) {
   return M <= 64 || (M <= SKINNY_MAX_T && (K >= 2 * rows || size >= (8LL << 20)));
 }
 
-static void run_skinny(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int act, const c10::optional<at::Tensor>& residual,
-                       at::Tensor& y, bool fresh_weight) {
+// norm_w: x is normalised first; its kernel clears the GEMM's tickets, which else takes a launch of its own (1.5 us in the stream)
+static void run_skinny(at::Tensor x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int act, const c10::optional<at::Tensor>& residual,
+                       at::Tensor& y, bool fresh_weight, const c10::optional<at::Tensor>& norm_w = c10::nullopt, double eps = 0., double offset = 0.) {
   const int M = x.size(0);
   const int64_t nt = skinny_gemm_tickets(), nf = skinny_gemm_ws_floats(M, act != 0);
   auto ws = at::empty({nf + nt}, x.options().dtype(at::kFloat));              // one per call: safe on any stream and inside captured graphs
   SkinnyGemm a{};
+  a.ws = ws.data_ptr<float>();
+  a.tickets = reinterpret_cast<unsigned*>(ws.data_ptr<float>() + nf);
+  if (norm_w.has_value()) x = rmsnorm_rows(x.contiguous(), *norm_w, eps, offset, nullptr, nullptr, a.tickets, (int)nt);
+  else skinny_clear_launch(a.tickets, (int)nt, cur_stream());
   a.x = x.data_ptr(); a.x_rows = M; a.ldx = x.stride(0); a.w = w.data_ptr(); a.bias = optr(bias); a.residual = optr(residual); a.y = y.data_ptr();
   a.experts = 1; a.tokens = M; a.n_out = y.size(1); a.K = x.size(1); a.act = act; a.limit = 7.f; a.alpha = 1.702f;
   a.w_fresh = fresh_weight ? 1 : 0;
-  a.ws = ws.data_ptr<float>();
-  a.tickets = reinterpret_cast<unsigned*>(ws.data_ptr<float>() + nf);
-  skinny_clear_launch(a.tickets, (int)nt, cur_stream());
   skinny_gemm_launch(a, cur_stream());
 }
 
@@ -179,7 +193,7 @@ at::Tensor gemv(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
   // rows too wide for the streaming kernel's shared memory (from 7 tokens of 14336, 8 of 11008).  us, here / one warp per weight row: 4096 x 14336 at 7 tokens
   // 26 / 57, at 8 26 / 36; 4096 x 11008 at 8 21 / 39
   if (!gemv2_supported(x.size(0), x.size(1), 0) && (glu ? N / 2 : N) % 8 == 0) {
-    run_skinny(norm_w.has_value() ? std::get<0>(rmsnorm(x.contiguous(), *norm_w, eps, offset, c10::nullopt)) : x, w, bias, (int)act, residual, y, false);
+    run_skinny(x, w, bias, (int)act, residual, y, false, norm_w, eps, offset);
     return y;
   }
   bool x_in_smem;
@@ -201,8 +215,9 @@ static bool pair_pays(int M, int n_out, bool glu) {
 // fresh_weight: w was written by a kernel enqueued just before (an expanded 8-bit weight).  The kernels fetch a parameter's first tiles before the
 // kernels in front of them have finished; such a weight has to be waited for.
 // tcgen05 GEMM for T > 8 tokens (prefill, long speculation windows)
-at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int64_t act,
-                const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& out, bool fresh_weight) {
+static at::Tensor gemm_rows(at::Tensor x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int64_t act,
+                const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& out, bool fresh_weight, const c10::optional<at::Tensor>& norm_w, double eps,
+                double offset) {
   TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1));
   TORCH_CHECK(is_bf16(x) && is_bf16(w) && x.stride(1) == 1 && w.is_contiguous());
   const int M = x.size(0), K = x.size(1), N = w.size(0);
@@ -217,9 +232,10 @@ at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
   if (residual.has_value())
     TORCH_CHECK(!glu && residual->is_contiguous() && residual->size(0) == M && residual->size(1) == n_out && is_bf16(*residual));
   if (skinny_pays(M, N, K, glu)) {
-    run_skinny(x, w, bias, (int)act, residual, y, fresh_weight);
+    run_skinny(x, w, bias, (int)act, residual, y, fresh_weight, norm_w, eps, offset);
     return y;
   }
+  if (norm_w.has_value()) x = rmsnorm_rows(x.contiguous(), *norm_w, eps, offset, nullptr, nullptr);
   if (pair_pays(M, n_out, glu)) {
     gemm_pair_launch(x.data_ptr(), x.stride(0), w.data_ptr(), optr(bias), optr(residual), y.data_ptr(), M, N, K, (int)act, cur_stream(),
                      fresh_weight);
@@ -228,6 +244,60 @@ at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
   gemm_tcgen05_launch(x.data_ptr(), (int)x.stride(0), w.data_ptr(), optr(bias), optr(residual), y.data_ptr(), n_out, M, N, K,
                       (int)act, cur_stream(), nullptr, fresh_weight);
   return y;
+}
+
+at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int64_t act, const c10::optional<at::Tensor>& residual,
+                const c10::optional<at::Tensor>& out, bool fresh_weight) {
+  return gemm_rows(x, w, bias, act, residual, out, fresh_weight, c10::nullopt, 0., 0.);
+}
+
+at::Tensor dequant_bf16(const at::Tensor& w, const at::Tensor& scale);
+
+// y = act(rmsnorm(x) w^T + bias) (+ residual) of rows x [.., K]: the choice between the kernels, made here because in Python it cost more than a launch.
+// -> result and what ran (the bits below), or none where no kernel takes the call (the caller's library path) or the norm's weight is of another type (LINEAR_NORM
+// alone: the caller normalises first).  bf16 x; w bf16, or int8 / fp8 with a scale per channel or one.
+enum { LINEAR_QGEMV = 1, LINEAR_GEMV = 2, LINEAR_DEQUANT = 4, LINEAR_GEMM = 8, LINEAR_NORM = 16 };
+std::tuple<c10::optional<at::Tensor>, int64_t> linear(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias,
+                                                      const c10::optional<at::Tensor>& norm_w, double eps, double offset, int64_t act,
+                                                      const c10::optional<at::Tensor>& scale, const c10::optional<at::Tensor>& residual,
+                                                      const c10::optional<at::Tensor>& out, bool tensor_cores) {
+  const auto none = std::make_tuple(c10::optional<at::Tensor>(), (int64_t)0);
+  const bool wq = w.scalar_type() == at::kChar || w.scalar_type() == at::kFloat8_e4m3fn;
+  const bool plain = is_bf16(w) && !scale.has_value();
+  if (!is_bf16(x) || x.dim() < 1 || x.size(-1) == 0 || w.dim() != 2 || !w.is_contiguous() || !(plain || (wq && scale.has_value() && scale->dim() == 1))) return none;
+  const int64_t K = x.size(-1), T = x.numel() / K, N = w.size(0), n_out = act != 0 ? N / 2 : N;
+  const bool few = T <= GEMV_MAX_T;
+  int64_t ran = 0;
+  if (few && wq && K % 16 == 0) ran = LINEAR_QGEMV;
+  else if (few && plain && K % 64 == 0 && (K % 256 == 0 || gemv2_supported((int)T, (int)K, 0))) ran = LINEAR_GEMV;
+  else if (!few && K % 64 == 0 && n_out % 8 == 0 && tensor_cores) ran = LINEAR_GEMM | (wq ? LINEAR_DEQUANT : 0);
+  else return none;
+  if ((ran & LINEAR_GEMM) && norm_w.has_value()) {
+    if (!is_bf16(*norm_w)) return std::make_tuple(c10::optional<at::Tensor>(), (int64_t)LINEAR_NORM);
+    ran |= LINEAR_NORM;
+  }
+  const auto x2 = x.reshape({T, K});
+  c10::optional<at::Tensor> r2, scale_f;
+  if (residual.has_value() && act == 0) r2 = wq && few ? residual->reshape({T, -1}).contiguous() : residual->reshape({T, -1});
+  if (scale.has_value()) scale_f = scale->to(at::kFloat).contiguous();
+  at::Tensor y;
+  if (ran & (LINEAR_QGEMV | LINEAR_GEMV)) {
+    y = gemv(x2, w, bias, norm_w, eps, offset, act, scale_f, r2);
+  } else {
+    // weight-only 8-bit layers: one expansion pass to bf16 (stays in L2), then the bf16 GEMM, which waits for it
+    c10::optional<at::Tensor> o2;
+    if (out.has_value()) o2 = out->view({T, -1});
+    y = gemm_rows(x2.contiguous(), wq ? dequant_bf16(w, *scale_f) : w, bias, act, r2, o2, wq, norm_w, eps, offset);
+  }
+  if ((ran & LINEAR_GEMM) && out.has_value()) {
+    y = *out;
+  } else {
+    auto shape = x.sizes().vec();
+    shape.back() = y.size(1);
+    y = y.view(shape);
+  }
+  if (residual.has_value() && !r2.has_value()) y = y + *residual;
+  return std::make_tuple(c10::optional<at::Tensor>(y), ran);
 }
 
 // Row-parallel GEMV -> one-shot all-reduce over NVLink peer buffers -> +bias +residual.  ONE kernel.
@@ -564,8 +634,10 @@ at::Tensor argmax(const at::Tensor& logits, const std::vector<int64_t>& slot_ptr
   return out;
 }
 
-at::Tensor topk_sample(const at::Tensor& logits, const at::Tensor& top_k, const at::Tensor& top_p,
-                       const at::Tensor& temperature, const at::Tensor& rand, int64_t global_topk) {
+at::Tensor topk_sample(const at::Tensor& logits_in, const at::Tensor& top_k_in, const at::Tensor& top_p_in,
+                       const at::Tensor& temperature_in, const c10::optional<at::Tensor>& rand_in, int64_t global_topk) {
+  const auto logits = logits_in.contiguous(), top_k = top_k_in.to(at::kInt), top_p = top_p_in.to(at::kFloat), temperature = temperature_in.to(at::kFloat);
+  const auto rand = rand_in.has_value() ? rand_in->to(at::kFloat) : at::full({logits.size(0)}, 0.5, logits.options().dtype(at::kFloat));
   TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.stride(1) == 1);
   TORCH_CHECK(logits.scalar_type() == at::kFloat || is_bf16(logits), "topk_sample: fp32 or bf16 logits");
   TORCH_CHECK(global_topk >= 1 && global_topk <= 256);
@@ -887,6 +959,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dstep_launch", &nxdi::dstep_launch_b);
   m.def("rmsnorm", &nxdi::rmsnorm);
   m.def("gemv", &nxdi::gemv);
+  m.def("linear", &nxdi::linear);
   m.def("gemv_allreduce", &nxdi::gemv_allreduce);
   m.def("set_prof", [](const c10::optional<at::Tensor>& buf) {
     if (!buf.has_value()) { nxdi::gemv2_set_prof(nullptr, 0); return; }

@@ -45,10 +45,13 @@ void gemv_launch(const GemvParams& p, int mode, cudaStream_t stream) {
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const __nv_bfloat16* __restrict__ x,
                                                       const __nv_bfloat16* __restrict__ res_in,
                                                       const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                                                      __nv_bfloat16* __restrict__ res_out, int H, float eps, float offset) {
+                                                      __nv_bfloat16* __restrict__ res_out, int H, float eps, float offset,
+                                                      unsigned* __restrict__ clear, int n_clear) {
   __shared__ float sred[8];
   pdl_launch_dependents();
   pdl_wait();
+  if (blockIdx.x == 0)                 // words that the kernel behind this one counts in
+    for (int i = threadIdx.x; i < n_clear; i += 256) clear[i] = 0u;
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * H);
   const uint4* rr = res_in ? reinterpret_cast<const uint4*>(res_in + (size_t)row * H) : nullptr;
@@ -172,7 +175,8 @@ __global__ void __launch_bounds__(256, 4) rmsnorm_rows_kernel(const __nv_bfloat1
 }
 
 void rmsnorm_launch(const void* x, const void* res_in, const void* w, void* y, void* res_out, int rows, int H, float eps,
-                    float offset, cudaStream_t stream) {
+                    float offset, cudaStream_t stream, unsigned* clear, int n_clear) {
+  if (n_clear > 0 && rows >= 1024) throw std::runtime_error("rmsnorm: words are cleared beside fewer than 1024 rows");
   // enough rows to fill the SMs that way; fewer, where a row's latency counts: a block per row
   if (rows >= 1024 && H <= 8192) {
     auto go = [&](auto kernel, int per_block) {
@@ -187,7 +191,7 @@ void rmsnorm_launch(const void* x, const void* res_in, const void* w, void* y, v
   }
   launch_pdl(rmsnorm_kernel, dim3(rows), dim3(256), 0, stream, reinterpret_cast<const __nv_bfloat16*>(x),
              reinterpret_cast<const __nv_bfloat16*>(res_in), reinterpret_cast<const __nv_bfloat16*>(w),
-             reinterpret_cast<__nv_bfloat16*>(y), reinterpret_cast<__nv_bfloat16*>(res_out), H, eps, offset);
+             reinterpret_cast<__nv_bfloat16*>(y), reinterpret_cast<__nv_bfloat16*>(res_out), H, eps, offset, clear, n_clear);
 }
 
 }  // namespace nxdi

@@ -67,18 +67,17 @@ def rmsnorm(x, weight, eps: float, offset: float = 0.0, residual=None):
     if _use_cuda(x) and x.dtype in _FAST_DTYPES and x.shape[-1] % 8 == 0 and weight is not None \
             and weight.dtype == x.dtype:
         stats["rmsnorm"] += 1
-        x2 = x.reshape(-1, x.shape[-1]).contiguous()        # (a slice of a wider projection arrives strided)
-        if residual is not None:
-            r2 = residual.reshape(-1, x.shape[-1]).contiguous()
-            y, r = _C().rmsnorm(x2, weight, eps, offset, r2)
-            return y.view(x.shape), r.view(x.shape)
-        y, _ = _C().rmsnorm(x2, weight, eps, offset, None)
-        return y.view(x.shape)
+        y, r = _C().rmsnorm(x, weight, eps, offset, residual)
+        return y if residual is None else (y, r)
     return ref.rmsnorm(x, weight, eps, offset, residual)
 
 
 _GATE_PRODUCTS = {"silu_mul": "silu", "gelu_tanh_mul": "gelu_tanh", "gelu_mul": "gelu"}
 _ACT_CODES = {None: 0, "silu_mul": 1, "gelu_tanh_mul": 2, "gelu_mul": 3}
+
+
+# what csrc/bindings.cpp::linear ran, by the bits that it returns
+_LINEAR_KINDS = [[kind for i, kind in enumerate(("qgemv", "gemv", "dequant_gemm", "gemm_tcgen05", "rmsnorm")) if bits >> i & 1] for bits in range(32)]
 
 
 def staging_for(group, x, w):
@@ -98,51 +97,28 @@ def linear(x, w, bias=None, norm_weight=None, norm_eps: float = 1e-6, norm_offse
            act: Optional[str] = None, scale=None, residual=None, out=None):
     """y = act(rmsnorm(x) @ w^T + bias) (+ residual).  w: [N,K] bf16, or int8/fp8 with per-channel ``scale``.
     ``out``: preallocated result (tcgen05 GEMM path only; used to land partial sums in the symmetric heap)."""
-    if _use_cuda(x) and x.dtype in _FAST_DTYPES:
-        K = x.shape[-1]
-        T = x.numel() // K
-        N = w.shape[0]
-        wq = w.dtype in (torch.int8, torch.float8_e4m3fn)
-        ok_w = (w.dtype == x.dtype and scale is None) or (wq and scale is not None and scale.dim() == 1)
-        if ok_w and act in _ACT_CODES and w.is_contiguous():
-            x2, fresh = x.reshape(T, K), False
-            if wq and T <= GEMV_MAX_TOKENS and K % 16 == 0 and w.dim() == 2:
-                stats["qgemv"] += 1
-                r2 = residual.reshape(T, -1).contiguous() if (residual is not None and act is None) else None
-                y = _C().gemv(x2, w, bias, norm_weight, norm_eps, norm_offset, _ACT_CODES[act], scale.float().contiguous(), r2)
-                y = y.view(*x.shape[:-1], y.shape[-1])
-                return y if (residual is None or r2 is not None) else y + residual
-            if not wq and T <= GEMV_MAX_TOKENS and K % 64 == 0 and (K % 256 == 0 or _C().gemv2_supported(T, K)):
-                stats["gemv"] += 1
-                r2 = residual.reshape(T, -1) if (residual is not None and act is None) else None
-                y = _C().gemv(x2, w, bias, norm_weight, norm_eps, norm_offset, _ACT_CODES[act], scale, r2)
-                y = y.view(*x.shape[:-1], y.shape[-1])
-                return y if (residual is None or r2 is not None) else y + residual
-            n_out = N // 2 if act is not None else N
-            if (wq and _ACT_QUANT and w.dtype == torch.float8_e4m3fn and T > GEMV_MAX_TOKENS and K % 128 == 0 and n_out % 8 == 0
-                    and w.dim() == 2 and K <= 16384):
+    if x.dtype in _FAST_DTYPES and act in _ACT_CODES and _use_cuda(x):
+        if _ACT_QUANT and w.dtype == torch.float8_e4m3fn and scale is not None and scale.dim() == 1 and w.is_contiguous():
+            K = x.shape[-1]
+            T = x.numel() // K
+            n_out = w.shape[0] // 2 if act is not None else w.shape[0]
+            if T > GEMV_MAX_TOKENS and K % 128 == 0 and n_out % 8 == 0 and w.dim() == 2 and K <= 16384:
                 # W8A8: RMSNorm + per-token fp8 quantisation in one kernel, then the fp8 tensor-core GEMM (2x the bf16 rate);
                 # acc * a_scale[row] * w_scale[col] in the epilogue
                 stats["gemm_fp8"] += 1
-                xq, a_s = _C().rmsnorm_quant(x2.contiguous(), norm_weight, float(norm_eps), float(norm_offset), float("inf"))
+                xq, a_s = _C().rmsnorm_quant(x.reshape(T, K).contiguous(), norm_weight, float(norm_eps), float(norm_offset), float("inf"))
                 r2 = residual.reshape(T, -1).contiguous() if (residual is not None and act is None) else None
                 y = _C().gemm_fp8(xq, a_s, w, scale.float().contiguous(), bias, _ACT_CODES[act], r2)
                 y = y.view(*x.shape[:-1], y.shape[-1])
                 return y if (residual is None or r2 is not None) else y + residual
-            if (wq and T > GEMV_MAX_TOKENS and w.dim() == 2 and K % 64 == 0 and n_out % 8 == 0 and _TCGEN05_GEMM
-                    and x.dtype == torch.bfloat16):
-                # weight-only 8-bit prefill: one expansion pass to bf16 (stays in L2), then the bf16 tensor-core GEMM, which waits for it
-                stats["dequant_gemm"] += 1
-                w, scale, wq, fresh = _C().dequant_bf16(w, scale.float().contiguous()), None, False, True
-            if not wq and n_out % 8 == 0 and K % 64 == 0 and _TCGEN05_GEMM and (T > GEMV_MAX_TOKENS or K % 64 != 0):
-                if norm_weight is not None:
-                    x2 = rmsnorm(x2, norm_weight, norm_eps, norm_offset)
-                stats["gemm_tcgen05"] += 1
-                r2 = residual.reshape(T, -1) if (residual is not None and act is None) else None
-                o2 = out.view(T, -1) if out is not None else None
-                y = _C().gemm(x2.contiguous(), w, bias, _ACT_CODES[act], r2, o2, fresh)
-                y = out if out is not None else y.view(*x.shape[:-1], y.shape[-1])
-                return y if (residual is None or r2 is not None) else y + residual
+        y, ran = _C().linear(x, w, bias, norm_weight, norm_eps, norm_offset, _ACT_CODES[act], scale, residual, out, _TCGEN05_GEMM)
+        if y is None and ran:              # the norm's weight is of another type than the rows
+            x, norm_weight = rmsnorm(x, norm_weight, norm_eps, norm_offset), None
+            y, ran = _C().linear(x, w, bias, None, norm_eps, norm_offset, _ACT_CODES[act], scale, residual, out, _TCGEN05_GEMM)
+        if y is not None:
+            for kind in _LINEAR_KINDS[ran]:
+                stats[kind] += 1
+            return y
     if act in _GATE_PRODUCTS and _mix_cuda(x) and w.dtype == x.dtype and scale is None and x.dim() >= 2:
         # fp32 rows and sizes the GEMM kernels do not take: library product, then the gate product as one elementwise kernel
         gu = ref.linear(x, w, bias, norm_weight, norm_eps, norm_offset)
@@ -343,11 +319,7 @@ def sample(logits, top_k, top_p, temperature, rand=None, global_topk: int = 256)
     if _use_cuda(logits) and logits.dim() == 2 and logits.dtype in (torch.float32, torch.bfloat16) \
             and global_topk <= 256:
         stats["topk_sample"] += 1
-        B = logits.shape[0]
-        if rand is None:
-            rand = torch.full((B,), 0.5, device=logits.device)
-        return _C().topk_sample(logits.contiguous(), top_k.to(torch.int32), top_p.float(), temperature.float(),
-                                rand.float(), int(global_topk))
+        return _C().topk_sample(logits, top_k, top_p, temperature, rand, int(global_topk))
     return ref.sample(logits, top_k, top_p, temperature, rand, global_topk)
 
 
