@@ -128,6 +128,9 @@ struct SkinnyGemm {
   int n_out, K, act;
   float limit, alpha;
   int w_fresh;                // w was written by a kernel just before: the weight producer waits for it
+  int wt;                     // 0 bf16; one weight of 1 int8, 2 e4m3 (skinny_gemm8_supported) with scale [rows], or [1] (scale_n)
+  const float* scale;
+  int scale_n;
   const int *n_active, *active, *seg_start, *seg_count;   // grouped: number of segments; each one's expert, first row of x and rows; null: one expert
   float* ws;                  // skinny_gemm_ws_floats
   unsigned* tickets;          // skinny_gemm_tickets, zero at launch
@@ -135,6 +138,7 @@ struct SkinnyGemm {
 int skinny_gemm_rows(int tokens);          // `tokens` rounded up to what a segment may hold
 long long skinny_gemm_ws_floats(int tokens, bool glu);
 int skinny_gemm_tickets();
+bool skinny_gemm8_supported(int tokens, int K, bool glu);
 void skinny_clear_launch(unsigned* tickets, int n, cudaStream_t stream);
 void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream);
 // id_step: 1, or 2 when topk_i points at int64 ids (their low words are read)

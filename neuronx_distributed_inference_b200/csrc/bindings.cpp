@@ -124,9 +124,9 @@ static void check_gemv_inputs(const at::Tensor& x, const at::Tensor& w) {
 }
 
 // Where the swapped, evenly split GEMM (skinny_gemm.cu) beats the 128-row token tiles of gemm_tcgen05.cu (us in a graph, skinny / tiles; 16, 64, 96 and 128 tokens):
-//   gate|up 28672 x 4096: 43 / 61, 48 / 62, 53 / 62, 56 / 63     17280 x 3200: 25 / 48, 30 / 34, 34 / 34, 38 / 34    16384 x 2048: 17 / 33, 22 / 26, 25 / 26, 28 / 26
+//   gate|up 28672 x 4096: 43 / 61, 49 / 62, 53 / 62, 57 / 63     17280 x 3200: 24 / 48, 30 / 34, 34 / 34, 34 / 34    16384 x 2048: 16 / 33, 21 / 26, 25 / 26, 26 / 26
 //           8192 x 3072:  17 / 36, 21 / 23, 24 / 23, 27 / 23      6144 x 2048: 14 / 28, 20 / 18, 22 / 18, 25 / 18     2048 x 1024:   9 / 17, 12 / 17, 14 / 17, 17 / 17
-//   plain 4096 x 14336:   26 / 57, 30 / 58, 34 / 58, 35 / 59      6144 x 4096: 16 / 25, 19 / 26, 21 / 26, 23 / 26      2048 x 8192:  14 / 39, 18 / 39, 21 / 39, 23 / 40
+//   plain 4096 x 14336:   25 / 57, 29 / 58, 32 / 58, 35 / 59      6144 x 4096: 14 / 25, 17 / 26, 20 / 26, 22 / 26      2048 x 8192:  14 / 39, 17 / 39, 20 / 39, 23 / 40
 //           3072 x 3072:  12 / 20, 15 / 20, 18 / 20, 20 / 20      4096 x 1024:  9 / 11, 11 / 11, 13 / 11, 14 / 11       512 x 512:    8 / 8,  10 / 8,  11 / 8,  13 / 8
 // A feature's tokens are in one lane, so its epilogue and the fix-up of the cut tiles grow with the tokens, while the tile kernel's time does not change up to 128.
 static bool skinny_pays(int M, int rows, int K, bool glu) {
@@ -137,7 +137,8 @@ static bool skinny_pays(int M, int rows, int K, bool glu) {
 
 // norm_w: x is normalised first; its kernel clears the GEMM's tickets, which else takes a launch of its own (1.5 us in the stream)
 static void run_skinny(at::Tensor x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int act, const c10::optional<at::Tensor>& residual,
-                       at::Tensor& y, bool fresh_weight, const c10::optional<at::Tensor>& norm_w = c10::nullopt, double eps = 0., double offset = 0.) {
+                       at::Tensor& y, bool fresh_weight, const c10::optional<at::Tensor>& norm_w = c10::nullopt, double eps = 0., double offset = 0.,
+                       const at::Tensor* scale = nullptr) {
   const int M = x.size(0);
   const int64_t nt = skinny_gemm_tickets(), nf = skinny_gemm_ws_floats(M, act != 0);
   auto ws = at::empty({nf + nt}, x.options().dtype(at::kFloat));              // one per call: safe on any stream and inside captured graphs
@@ -149,6 +150,11 @@ static void run_skinny(at::Tensor x, const at::Tensor& w, const c10::optional<at
   a.x = x.data_ptr(); a.x_rows = M; a.ldx = x.stride(0); a.w = w.data_ptr(); a.bias = optr(bias); a.residual = optr(residual); a.y = y.data_ptr();
   a.experts = 1; a.tokens = M; a.n_out = y.size(1); a.K = x.size(1); a.act = act; a.limit = 7.f; a.alpha = 1.702f;
   a.w_fresh = fresh_weight ? 1 : 0;
+  if (scale != nullptr) {
+    a.wt = w.scalar_type() == at::kChar ? 1 : 2;
+    a.scale = scale->data_ptr<float>();
+    a.scale_n = (int)scale->numel();
+  }
   skinny_gemm_launch(a, cur_stream());
 }
 
@@ -253,6 +259,21 @@ at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
 
 at::Tensor dequant_bf16(const at::Tensor& w, const at::Tensor& scale);
 
+// int8 / fp8 weights and 9 .. 128 tokens (64 with a gate product): the bytes are read once.  us, here / expanded to bf16 in memory first: 4096 x 4096 at 9 tokens 11 / 25,
+// at 128 24 / 33; 4096 x 11008 at 9 17 / 48, at 37 20 / 52, at 128 30 / 58; 11008 x 4096 at 47 20 / 51; 12288 x 4096 at 64 23 / 58, at 100 28 / 60.  The weight is not
+// rounded: the scale is applied to the fp32 sum.
+static at::Tensor linear8_few(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int64_t act, const at::Tensor& scale,
+                              const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& norm_w, double eps, double offset) {
+  const int64_t M = x.size(0), N = w.size(0), n_out = act != 0 ? N / 2 : N;
+  TORCH_CHECK(x.size(1) == w.size(1) && w.is_cuda() && (act == 0 || N % 2 == 0) && (scale.numel() == 1 || scale.numel() == N));
+  c10::cuda::CUDAGuard guard(x.device());
+  auto y = at::empty({M, n_out}, x.options());
+  if (residual.has_value())
+    TORCH_CHECK(act == 0 && residual->is_contiguous() && residual->size(0) == M && residual->size(1) == n_out && is_bf16(*residual));
+  run_skinny(x.contiguous(), w, bias, (int)act, residual, y, false, norm_w, eps, offset, &scale);
+  return y;
+}
+
 // y = act(rmsnorm(x) w^T + bias) (+ residual) of rows x [.., K]: the choice between the kernels, made here because in Python it cost more than a launch.
 // -> result and what ran (the bits below), or none where no kernel takes the call (the caller's library path) or the norm's weight is of another type (LINEAR_NORM
 // alone: the caller normalises first).  bf16 x; w bf16, or int8 / fp8 with a scale per channel or one.
@@ -266,11 +287,11 @@ std::tuple<c10::optional<at::Tensor>, int64_t> linear(const at::Tensor& x, const
   const bool plain = is_bf16(w) && !scale.has_value();
   if (!is_bf16(x) || x.dim() < 1 || x.size(-1) == 0 || w.dim() != 2 || !w.is_contiguous() || !(plain || (wq && scale.has_value() && scale->dim() == 1))) return none;
   const int64_t K = x.size(-1), T = x.numel() / K, N = w.size(0), n_out = act != 0 ? N / 2 : N;
-  const bool few = T <= GEMV_MAX_T;
+  const bool few = T <= GEMV_MAX_T, few8 = wq && !out.has_value() && skinny_gemm8_supported((int)std::min<int64_t>(T, SKINNY_MAX_T + 1), (int)K, act != 0);
   int64_t ran = 0;
   if (few && wq && K % 16 == 0) ran = LINEAR_QGEMV;
   else if (few && plain && K % 64 == 0 && (K % 256 == 0 || gemv2_supported((int)T, (int)K, 0))) ran = LINEAR_GEMV;
-  else if (!few && K % 64 == 0 && n_out % 8 == 0 && tensor_cores) ran = LINEAR_GEMM | (wq ? LINEAR_DEQUANT : 0);
+  else if (!few && K % 64 == 0 && n_out % 8 == 0 && tensor_cores) ran = LINEAR_GEMM | (wq && !few8 ? LINEAR_DEQUANT : 0);
   else return none;
   if ((ran & LINEAR_GEMM) && norm_w.has_value()) {
     if (!is_bf16(*norm_w)) return std::make_tuple(c10::optional<at::Tensor>(), (int64_t)LINEAR_NORM);
@@ -284,10 +305,11 @@ std::tuple<c10::optional<at::Tensor>, int64_t> linear(const at::Tensor& x, const
   if (ran & (LINEAR_QGEMV | LINEAR_GEMV)) {
     y = gemv(x2, w, bias, norm_w, eps, offset, act, scale_f, r2);
   } else {
-    // weight-only 8-bit layers: one expansion pass to bf16 (stays in L2), then the bf16 GEMM, which waits for it
     c10::optional<at::Tensor> o2;
     if (out.has_value()) o2 = out->view({T, -1});
-    y = gemm_rows(x2.contiguous(), wq ? dequant_bf16(w, *scale_f) : w, bias, act, r2, o2, wq, norm_w, eps, offset);
+    // weight-only 8-bit layers: few tokens read the bytes (linear8_few); more, one expansion pass to bf16 (stays in L2), then the bf16 GEMM, which waits for it
+    if (few8) y = linear8_few(x2, w, bias, act, *scale_f, r2, norm_w, eps, offset);
+    else y = gemm_rows(x2.contiguous(), wq ? dequant_bf16(w, *scale_f) : w, bias, act, r2, o2, wq, norm_w, eps, offset);
   }
   if ((ran & LINEAR_GEMM) && out.has_value()) {
     y = *out;

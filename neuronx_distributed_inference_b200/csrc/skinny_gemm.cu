@@ -6,17 +6,20 @@
 //   * CTA c of G takes the k-blocks [total c / G, total (c + 1) / G) of the concatenated (segment, 128-feature tile, k) space: every SM streams the
 //     same number of bytes whatever the shape (stream-K).  Tiles cut by a boundary meet in fp32 partials; the CTA that arrives last adds them in
 //     k order (deterministic) and runs the epilogue.
-//   * a stage is a 128 x 64 weight box (two for gate | up) plus the tokens' 64 columns; the ring takes all of shared memory (100 .. 180 KB of weights
-//     in flight per SM), weights and tokens have a TMA producer warp each.
+//   * a stage is a weight box of 128 rows x 64 k (two for gate | up; 128 k for one plain bf16 weight) plus the tokens' columns; the ring takes all of shared
+//     memory (100 .. 180 KB of weights in flight per SM), weights and tokens have a TMA producer warp each.  4096 x 4096 at 9 tokens 11.7 us with 128 k a stage,
+//     13.3 with 64.
+//   * int8 / e4m3 weights come as bytes, 128 k a box; eight warps expand them to bf16 (exactly) into TMEM, from where the MMAs read them as their A operand; the scale is
+//     applied to the fp32 sum.
 //   * accumulators (128 features x tokens) sit in TMEM twice, so a tile's epilogue overlaps the stream of the next one.  A lane holds one output
 //     feature: a warp's store of one token is 64 contiguous bytes, gate and up of a feature meet in one thread.
 //   * 16 epilogue warps: the last tile's epilogue is the tail of the launch, and so is the fix-up of its parts.  Both are round trips to L2 and cold
 //     instructions, so: every load of a group of 8 tokens (residual, parts) before the first use, the activation chosen outside of the loops, one code path.
 //     With 8 warps, groups of 16 tokens, three copies of the epilogue and the residual read where it was added, the tail after the last weights was
 //     25 us at 37 tokens, 28672 x 4096 gate | up (now 8) and 17 us at 4096 x 14336 with a residual (now 6).
-// Measured (us, here / 128-row token tiles): see skinny_pays in bindings.cpp.  28672 x 4096 gate | up at 9 tokens 42.6 us = 5.5 TB/s (46 before), a gated MLP
-// of 8B sizes with norm and residual at 37 tokens 78 us in a graph (100 before); six of eight Mixtral-sized experts, 6 tokens, with permutation and sum: 336 us
-// = 6.3 TB/s (one warp per weight row and (token, slot) pair: 744 us).
+// Measured (us, here / 128-row token tiles): see skinny_pays in bindings.cpp, 8-bit weights: linear8_few.  28672 x 4096 gate | up at 9 tokens 42.5 us = 5.5 TB/s
+// (46 before), a gated MLP of 8B sizes with norm and residual at 37 tokens 77 us in a graph (100 before); six of eight Mixtral-sized experts, 6 tokens, with permutation
+// and sum: 336 us = 6.3 TB/s (one warp per weight row and (token, slot) pair: 744 us).
 #include <algorithm>
 #include <stdexcept>
 #include <string>
@@ -29,16 +32,22 @@ namespace nxdi {
 
 constexpr int SK_BM = 128, SK_BK = 64;                 // weight rows, k elements per stage box (128-byte rows)
 constexpr int SK_W_BYTES = SK_BM * SK_BK * 2;
-constexpr int SK_EPI = 16;                             // epilogue warps: four per 32 features
-constexpr int SK_THREADS = 128 + SK_EPI * 32;          // 4 warps: weights, MMA, TMEM, tokens; epilogue warps
+constexpr int SK_THREADS = 640;                        // 4 warps: weights, MMA, TMEM, tokens; 16 epilogue warps, or 8 that expand 8-bit weights and 8 epilogue warps
+constexpr int SK_A_BUFS = 4, SK_A_COLS = 64;           // 8-bit weights: expanded boxes in TMEM, 128 k each
+__host__ __device__ constexpr int sk_epi(int wt) { return wt ? 8 : 16; }
+// k elements of a stage: with 128, one copy brings 32 KB of bf16 weights (or 16 KB of bytes) and one the tokens' columns.  A thread issues a copy in 0.25 us, in which an
+// SM's share of HBM brings 11 KB.
+__host__ __device__ constexpr int sk_bk(int wt, bool wide) { return wt || wide ? 128 : SK_BK; }
 constexpr int SK_MAX_STAGES = 12;
 constexpr int SK_SMEM = 220 * 1024;
 
 struct SkinnyKernelParams {
-  CUtensorMap tm_w;        // [experts * rows, K], box {64, 128}
-  CUtensorMap tm_x;        // [token rows, K], box {64, xbox}: xb rows for one expert, 16 when grouped (an expert loads as many as it has tokens for)
+  CUtensorMap tm_w;        // [experts * rows, K], box {64, 128} (bytes: {128, 128}); wide: as {64, rows, K / 64}, box {64, 128, 2}
+  CUtensorMap tm_x;        // [token rows, K], box {64, xbox}: xb rows for one expert, 16 when grouped (an expert loads as many as it has tokens for); 128 k: {64, xb, 2}
   const int *n_active, *active, *seg_start, *seg_count;     // grouped: segments (expert, first row of x, rows <= xb); null: one expert, T rows
   const __nv_bfloat16 *bias, *residual;                      // [experts * rows]; [T, n_out] (one expert)
+  const float* scale;      // 8-bit weights: [rows], or [1] with scale_step 0
+  int scale_step;
   void* y;                 // [token rows, n_out] bf16, or fp32 (y_f32)
   float* ws;               // [G][2][cols / 4][128][4] partial tiles
   unsigned* tickets;       // [G], zero at launch
@@ -47,6 +56,10 @@ struct SkinnyKernelParams {
   unsigned* wait_word;     // mbar_wait.cuh
 };
 
+__device__ __forceinline__ void sk_tma3(void* dst, const CUtensorMap* tm, int row, int group, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(mbar_s32(dst)), "l"(tm),
+               "r"(0), "r"(row), "r"(group), "r"(mbar_s32(bar)) : "memory");
+}
 __device__ __forceinline__ void sk_tma(void* dst, const CUtensorMap* tm, int c0, int c1, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(mbar_s32(dst)), "l"(tm),
                "r"(c0), "r"(c1), "r"(mbar_s32(bar)) : "memory");
@@ -61,40 +74,85 @@ __device__ __forceinline__ uint64_t sk_desc(const void* smem) {
   d |= (uint64_t)2 << 61;
   return d;
 }
-__device__ __forceinline__ void sk_umma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d), "l"(da),
-               "l"(db), "r"(idesc), "r"(acc) : "memory");
+// Called by a whole warp, issued by the lane whose `on` is 1: in code that all lanes run the descriptors stay in uniform registers.  (In a branch for one lane each
+// is moved there before its instruction: the issuing thread took 0.8 us for a box of 128 rows and eight instructions, more than its bytes take from HBM.)
+__device__ __forceinline__ void sk_umma(uint32_t on, uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d), "l"(da),
+               "l"(db), "r"(idesc), "r"(acc), "r"(on) : "memory");
 }
-__device__ __forceinline__ void sk_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar_s32(bar)) : "memory");
+__device__ __forceinline__ void sk_umma_ts(uint32_t on, uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+               "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc), "r"(on) : "memory");
+}
+__device__ __forceinline__ void sk_commit(uint32_t on, uint64_t* bar) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(mbar_s32(bar)),
+               "r"(on) : "memory");
+}
+__device__ __forceinline__ uint32_t sk_elect() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
 }
 __device__ __forceinline__ void sk_ld8(uint32_t taddr, uint32_t (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
 }
 
-template <bool GLU>
+__device__ __forceinline__ void sk_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
+      "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]),
+      "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]),
+      "r"(v[31])
+      : "memory");
+}
+// four one-byte weights (k ascending) -> two bf16 pairs, exact
+template <int WT>
+__device__ __forceinline__ void sk_expand4(uint32_t w, uint32_t& lo, uint32_t& hi) {
+  if constexpr (WT == 2) {        // e4m3
+    uint32_t a, b;
+    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(a) : "h"((unsigned short)(w & 0xffffu)));
+    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(b) : "h"((unsigned short)(w >> 16)));
+    const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&a)), fb = __half22float2(*reinterpret_cast<const __half2*>(&b));
+    lo = pack_bf16(fa.x, fa.y);
+    hi = pack_bf16(fb.x, fb.y);
+  } else {                        // int8: 128 + the low seven bits under the exponent of 128, minus 128 or (negative) 256
+    const uint32_t a = __byte_perm(w, 0x43434343u, 0x5140), b = __byte_perm(w, 0x43434343u, 0x5342);
+    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(lo) : "r"(a & 0xff7fff7fu), "r"(a & 0xff80ff80u));
+    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(hi) : "r"(b & 0xff7fff7fu), "r"(b & 0xff80ff80u));
+  }
+}
+
+// WT: 0 bf16 weights, 1 int8, 2 e4m3.  WIDE (bf16, one weight without a gate product): 128 k a stage
+template <bool GLU, int WT, bool WIDE>
 __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid_constant__ SkinnyKernelParams p) {
-  constexpr int NW = GLU ? 2 : 1;
+  constexpr int NW = GLU ? 2 : 1, EPI = sk_epi(WT), W_EPI = SK_THREADS / 32 - EPI, T_EPI = W_EPI * 32, BK = sk_bk(WT, WIDE), XBOX = BK / SK_BK;
+  constexpr int W_BYTES = WIDE ? 2 * SK_W_BYTES : SK_W_BYTES;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (mbar_s32(smem_raw) & 1023u)) & 1023u);
-  __shared__ uint64_t full_bar[SK_MAX_STAGES], empty_bar[SK_MAX_STAGES], tmem_full[2], tmem_empty[2];
+  __shared__ uint64_t full_bar[SK_MAX_STAGES], empty_bar[SK_MAX_STAGES], tmem_full[2], tmem_empty[2], a_full[SK_A_BUFS], a_empty[SK_A_BUFS];
   __shared__ uint32_t tmem_slot;
   __shared__ int s_stop, s_last;
   volatile int* stop = &s_stop;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ST = p.stages, x_bytes = p.xb * SK_BK * 2, stage_bytes = NW * SK_W_BYTES + x_bytes;     // xb % 16 == 0: multiples of 1024
+  const int ST = p.stages, x_bytes = p.xb * BK * 2, stage_bytes = NW * W_BYTES + x_bytes;     // xb % 16 == 0: multiples of 1024
 
   if (warp == 0 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_w) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_x) : "memory");
     for (int s = 0; s < ST; ++s) {
       mbar_init(&full_bar[s], 2);         // the two producers
-      mbar_init(&empty_bar[s], 1);
+      mbar_init(&empty_bar[s], WT ? 1 + 4 * NW : 1);      // the MMAs' commit, and the warps that expand the weights
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tmem_full[b], 1);
-      mbar_init(&tmem_empty[b], SK_EPI);
+      mbar_init(&tmem_empty[b], EPI);
+    }
+    for (int b = 0; b < SK_A_BUFS && WT; ++b) {
+      mbar_init(&a_full[b], 4);
+      mbar_init(&a_empty[b], 1);
     }
     s_stop = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -113,7 +171,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
   bool early = warp == 0 && !grouped && !p.w_fresh;
   if (!early) pdl_wait();
 
-  const int n_tiles = (p.n_out + SK_BM - 1) / SK_BM, nkb = p.K / SK_BK;
+  const int n_tiles = (p.n_out + SK_BM - 1) / SK_BM, nkb = p.K / BK;
   const long long total = (long long)(grouped ? *p.n_active : 1) * n_tiles * nkb;
   const long long G = max(1ll, min((long long)gridDim.x, total / 4));                // at least four k-blocks per CTA that works
   const long long u0 = blockIdx.x < G ? total * blockIdx.x / G : 0, u1 = blockIdx.x < G ? total * (blockIdx.x + 1) / G : 0;
@@ -139,12 +197,14 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
           if (!go) break;
           uint8_t* st = smem + (size_t)s * stage_bytes;
           if (warp == 0) {
-            mbar_expect(&full_bar[s], NW * SK_W_BYTES);
-            sk_tma(st, &p.tm_w, kb * SK_BK, row_w, &full_bar[s]);
-            if (GLU) sk_tma(st + SK_W_BYTES, &p.tm_w, kb * SK_BK, row_w + p.n_out, &full_bar[s]);
+            mbar_expect(&full_bar[s], NW * W_BYTES);
+            if (WIDE) sk_tma3(st, &p.tm_w, row_w, kb * 2, &full_bar[s]);
+            else sk_tma(st, &p.tm_w, kb * BK, row_w, &full_bar[s]);
+            if (GLU) sk_tma(st + W_BYTES, &p.tm_w, kb * BK, row_w + p.n_out, &full_bar[s]);
           } else {
-            mbar_expect(&full_bar[s], boxes * box_bytes);
-            for (int q = 0; q < boxes; ++q) sk_tma(st + NW * SK_W_BYTES + q * box_bytes, &p.tm_x, kb * SK_BK, row_x + q * p.xbox, &full_bar[s]);
+            mbar_expect(&full_bar[s], boxes * box_bytes * XBOX);
+            if (XBOX == 2) sk_tma3(st + NW * W_BYTES, &p.tm_x, 0, kb * 2, &full_bar[s]);
+            for (int q = 0; q < boxes && XBOX == 1; ++q) sk_tma(st + NW * W_BYTES + q * box_bytes, &p.tm_x, kb * BK, row_x + q * p.xbox, &full_bar[s]);
           }
           if (++s == ST) {
             s = 0;
@@ -156,46 +216,113 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
     }
   } else if (warp == 1) {
     // ================= MMA issuer =================
-    if (lane == 0) {
-      int seg = 0, s = 0;
-      uint32_t phase = 0;
-      bool go = true;
-      for (long long u = u0; u < u1 && go; ++seg) {
-        const int kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u)), buf = seg & 1;
-        // D = f32, A = B = bf16, both K-major, M = 128, N = the tokens in whole boxes (a multiple of 16)
-        const int nx = grouped ? (p.seg_count[(int)(u / nkb) / n_tiles] + 15) / 16 * 16 : p.xb;
-        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nx >> 3) << 17) | ((uint32_t)(SK_BM >> 4) << 24);
-        go = mbar_wait(&tmem_empty[buf], (uint32_t)((seg >> 1) & 1) ^ 1u, stop, p.wait_word);
+    const uint32_t on = sk_elect();
+    const uint64_t dw0 = sk_desc(smem), dx0 = sk_desc(smem + NW * W_BYTES);
+    const uint32_t half = (uint32_t)(x_bytes / XBOX) >> 4, stage = (uint32_t)stage_bytes >> 4;
+    uint32_t at = 0;                                       // of the ring's next stage, in 16-byte units like a descriptor
+    int seg = 0, s = 0, ab = 0;
+    uint32_t phase = 0, aphase = 0;
+    bool go = true;
+    for (long long u = u0; u < u1 && go; ++seg) {
+      const int kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u)), buf = seg & 1;
+      // D = f32, A = B = bf16, both K-major, M = 128, N = the tokens in whole boxes (a multiple of 16)
+      const int nx = grouped ? (p.seg_count[(int)(u / nkb) / n_tiles] + 15) / 16 * 16 : p.xb;
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nx >> 3) << 17) | ((uint32_t)(SK_BM >> 4) << 24);
+      const uint32_t d0 = tmem + (uint32_t)(buf * acc_cols);
+      go = mbar_wait_warp(&tmem_empty[buf], (uint32_t)((seg >> 1) & 1) ^ 1u, stop, p.wait_word);
+      if (!go) break;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        go = mbar_wait_warp(&full_bar[s], phase, stop, p.wait_word);
         if (!go) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int kb = kb0; kb < kb1; ++kb) {
-          go = mbar_wait(&full_bar[s], phase, stop, p.wait_word);
-          if (!go) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint8_t* st = smem + (size_t)s * stage_bytes;
-          const uint64_t db = sk_desc(st + NW * SK_W_BYTES);
+        const uint64_t db = dx0 + at;
 #pragma unroll
-          for (int w = 0; w < NW; ++w) {
-            const uint64_t da = sk_desc(st + w * SK_W_BYTES);
+        for (int w = 0; w < NW; ++w) {
+          const uint32_t d = d0 + (uint32_t)(w * p.xb), first = kb != kb0 ? 1u : 0u;
+          if constexpr (WT == 0) {
+            const uint64_t da = dw0 + at + (uint64_t)(w * (W_BYTES >> 4));
 #pragma unroll
-            for (int k = 0; k < SK_BK / 16; ++k)      // 16 k = 32 bytes inside the swizzle atom
-              sk_umma(tmem + (uint32_t)(buf * acc_cols + w * p.xb), da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb != kb0 || k != 0) ? 1u : 0u);
-          }
-          sk_commit(&empty_bar[s]);
-          if (++s == ST) {
-            s = 0;
-            phase ^= 1u;
+            for (int k = 0; k < BK / 16; ++k)         // 16 k = 32 bytes inside the swizzle atom of 64
+              sk_umma(on, d, da + (uint64_t)((k >> 2) * (SK_W_BYTES >> 4) + (k & 3) * 2), db + (uint64_t)((k >> 2) * half + (k & 3) * 2), idesc, k != 0 ? 1u : first);
+          } else {
+            go = mbar_wait_warp(&a_full[ab], aphase, stop, p.wait_word);
+            if (!go) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a = tmem + 2 * acc_cols + ab * SK_A_COLS;
+#pragma unroll
+            for (int k = 0; k < BK / 16; ++k)
+              sk_umma_ts(on, d, a + 8 * k, db + (uint64_t)((k >> 2) * half + (k & 3) * 2), idesc, k != 0 ? 1u : first);
+            sk_commit(on, &a_empty[ab]);
+            if (++ab == SK_A_BUFS) {
+              ab = 0;
+              aphase ^= 1u;
+            }
           }
         }
-        if (go) sk_commit(&tmem_full[buf]);
-        u += kb1 - kb0;
+        if (!go) break;
+        sk_commit(on, &empty_bar[s]);
+        at += stage;
+        if (++s == ST) {
+          s = 0;
+          at = 0;
+          phase ^= 1u;
+        }
+      }
+      if (go) sk_commit(on, &tmem_full[buf]);
+      u += kb1 - kb0;
+    }
+  } else if (WT != 0 && warp >= 4 && warp < W_EPI) {
+    // ================= 8-bit weights -> bf16 in TMEM, the MMAs' A operand =================
+    // Two sets of four warps (32 weight rows each) take the boxes in turn.  Through TMEM, because shared memory has no room for it: a box is written and read
+    // once there as bytes; as bf16 it would be written and read twice more.
+    if constexpr (WT != 0) {
+      const int set = (warp - 4) >> 2, row = (warp & 3) * 32 + lane;
+      const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+      const int n = (int)(u1 - u0) * NW;                  // boxes
+      int s = NW == 1 ? set : 0, ab = set;                // counted: divisions of the box's number cost more than its expansion
+      uint32_t phase = 0, aphase = 1;
+      for (int it = set; it < n; it += 2) {
+        // the buffer first: that its last MMAs are done tells that the stage's phase before this one is over, which its parity (this set sees every second
+        // phase) does not
+        if (!mbar_wait_warp(&a_empty[ab], aphase, stop, p.wait_word)) break;
+        if (!mbar_wait_warp(&full_bar[s], phase, stop, p.wait_word)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t src = mbar_s32(smem + (size_t)s * stage_bytes + (NW == 1 ? 0 : set) * W_BYTES) + row * 128;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {                      // 64 k: four 16-byte chunks of the row, XOR-swizzled by TMA
+          uint32_t v[32];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t q[4];
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(src + (((4 * h + c) ^ (row & 7)) << 4)));
+#pragma unroll
+            for (int k = 0; k < 4; ++k) sk_expand4<WT>(q[k], v[8 * c + 2 * k], v[8 * c + 2 * k + 1]);
+          }
+          sk_st32(tmem + lanes + 2 * acc_cols + ab * SK_A_COLS + 32 * h, v);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty_bar[s]);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&a_full[ab]);
+        ab += 2;
+        if (ab >= SK_A_BUFS) {
+          ab = set;
+          aphase ^= 1u;
+        }
+        s += 2 / NW;
+        if (s >= ST) {
+          s -= ST;
+          phase ^= 1u;
+        }
       }
     }
-  } else if (warp >= 4) {
+  } else if (warp >= W_EPI) {
     // ================= epilogue: lane = output feature =================
     // One code path for whole tiles and for tiles that meet in the workspace, the activation chosen outside of the loop over the tokens: the epilogue runs once or
     // twice per CTA, so every instruction of it is fetched cold.
-    const int n_in = (warp & 3) * 32 + lane, c0 = ((warp - 4) >> 2) * 8;      // the warps of 32 features take groups of 8 tokens in turn
+    const int n_in = (warp & 3) * 32 + lane, c0 = ((warp - W_EPI) >> 2) * 8;      // the warps of 32 features take groups of 8 tokens in turn
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     int seg = 0;
     bool live = true;          // false once a wait ran out: the warp still takes part in the barriers of the eight
@@ -206,6 +333,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
       const int row0 = grouped ? p.seg_start[ei] : 0, cnt = grouped ? p.seg_count[ei] : p.T;
       const float bg = (p.bias && n < p.n_out) ? __bfloat162float(p.bias[(size_t)e * p.rows + n]) : 0.f;
       const float bu = (GLU && p.bias && n < p.n_out) ? __bfloat162float(p.bias[(size_t)e * p.rows + p.n_out + n]) : 0.f;
+      const float sg = WT && n < p.n_out ? __ldcg(p.scale + (size_t)n * p.scale_step) : 1.f, su = WT && GLU && n < p.n_out ? __ldcg(p.scale + (size_t)(p.n_out + n) * p.scale_step) : 1.f;
       const bool whole = kb0 == 0 && kb1 == nkb;
       // CTAs that share the tile: those of its first and last k-block and all between
       const long long f = (long long)tile * nkb;
@@ -218,20 +346,20 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
         if (kb0 == 0) {
           // the tile's first part is its CTA's last segment, so the other parts are often there already: then they are added to the sums in TMEM, which
           // needs neither slot nor ticket
-          if (threadIdx.x == 128) {
+          if (threadIdx.x == T_EPI) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.tickets + c_first) : "memory");
             s_last = v == (unsigned)(c_last - c_first);
           }
-          asm volatile("bar.sync 1, %0;" ::"n"(SK_EPI * 32) : "memory");
+          asm volatile("bar.sync 1, %0;" ::"n"(EPI * 32) : "memory");
           own = s_last != 0;
-          asm volatile("bar.sync 1, %0;" ::"n"(SK_EPI * 32) : "memory");     // s_last reusable
+          asm volatile("bar.sync 1, %0;" ::"n"(EPI * 32) : "memory");     // s_last reusable
         }
         if (!own) {
           // slot 0 of this CTA if the tile began in an earlier one, else slot 1
           float4* mine = reinterpret_cast<float4*>(p.ws + ((size_t)blockIdx.x * 2 + (kb0 == 0 ? 1 : 0)) * acc_cols * SK_BM) + n_in;
 #pragma unroll 1
-          for (int c = c0; c < cnt && live; c += 2 * SK_EPI) {
+          for (int c = c0; c < cnt && live; c += 2 * EPI) {
 #pragma unroll
             for (int w = 0; w < NW; ++w) {
               uint32_t v[8];
@@ -246,17 +374,17 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
           __syncwarp();
           if (lane == 0) mbar_arrive(&tmem_empty[buf]);
           __threadfence();
-          asm volatile("bar.sync 1, %0;" ::"n"(SK_EPI * 32) : "memory");
-          if (threadIdx.x == 128) s_last = atomicAdd(&p.tickets[c_first], 1u) == (unsigned)(c_last - c_first);
-          asm volatile("bar.sync 1, %0;" ::"n"(SK_EPI * 32) : "memory");
+          asm volatile("bar.sync 1, %0;" ::"n"(EPI * 32) : "memory");
+          if (threadIdx.x == T_EPI) s_last = atomicAdd(&p.tickets[c_first], 1u) == (unsigned)(c_last - c_first);
+          asm volatile("bar.sync 1, %0;" ::"n"(EPI * 32) : "memory");
           const bool last = s_last != 0;
-          asm volatile("bar.sync 1, %0;" ::"n"(SK_EPI * 32) : "memory");     // s_last reusable
+          asm volatile("bar.sync 1, %0;" ::"n"(EPI * 32) : "memory");     // s_last reusable
           if (!last) continue;
         }
         __threadfence();
       }
 #pragma unroll 1
-      for (int c = c0; c < cnt && live; c += 2 * SK_EPI) {
+      for (int c = c0; c < cnt && live; c += 2 * EPI) {
         float g[8], up[8];
         uint32_t res[8];
         const bool in = n < p.n_out;
@@ -302,6 +430,13 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
               g[4 * k] += a[i][k].x; g[4 * k + 1] += a[i][k].y; g[4 * k + 2] += a[i][k].z; g[4 * k + 3] += a[i][k].w;
               if (GLU) { up[4 * k] += b[i][k].x; up[4 * k + 1] += b[i][k].y; up[4 * k + 2] += b[i][k].z; up[4 * k + 3] += b[i][k].w; }
             }
+          }
+        }
+        if constexpr (WT != 0) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            g[k] *= sg;
+            if (GLU) up[k] *= su;
           }
         }
         if (GLU) {
@@ -353,7 +488,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
 
 typedef CUresult (*SkEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static void sk_map(CUtensorMap* tm, const void* ptr, long long rows, int K, long long ld, int box_rows) {
+// rows of K elements, `groups` boxes of 64 elements (128 bytes, also for byte elements) side by side in one copy; groups > 1: as {64, rows, K / 64}
+static void sk_map(CUtensorMap* tm, const void* ptr, long long rows, int K, long long ld, int box_rows, bool bytes = false, int groups = 1) {
   static SkEncodeFn fn = [] {
     void* q = nullptr;
     cudaDriverEntryPointQueryResult r;
@@ -361,10 +497,11 @@ static void sk_map(CUtensorMap* tm, const void* ptr, long long rows, int K, long
       throw std::runtime_error("cuTensorMapEncodeTiled not available");
     return reinterpret_cast<SkEncodeFn>(q);
   }();
-  cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)rows}, gstride[1] = {(cuuint64_t)ld * 2};
-  cuuint32_t box[2] = {(cuuint32_t)SK_BK, (cuuint32_t)box_rows}, estr[2] = {1, 1};
-  CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const cuuint64_t es = bytes ? 1 : 2;
+  cuuint64_t gdim[3] = {(cuuint64_t)(groups > 1 ? SK_BK : K), (cuuint64_t)rows, (cuuint64_t)(K / SK_BK)}, gstride[2] = {(cuuint64_t)ld * es, 128};
+  cuuint32_t box[3] = {(cuuint32_t)(128 / es), (cuuint32_t)box_rows, (cuuint32_t)groups}, estr[3] = {1, 1, 1};
+  CUresult r = fn(tm, bytes ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, groups > 1 ? 3 : 2, const_cast<void*>(ptr), gdim, gstride, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled (skinny gemm) failed: " + std::to_string((int)r));
 }
 
@@ -391,33 +528,43 @@ __global__ void __launch_bounds__(256) skinny_clear_kernel(unsigned* __restrict_
 }
 void skinny_clear_launch(unsigned* tickets, int n, cudaStream_t stream) { launch_pdl(skinny_clear_kernel, dim3(1), dim3(256), 0, stream, tickets, n); }
 
+bool skinny_gemm8_supported(int tokens, int K, bool glu) { return tokens >= 1 && tokens <= (glu ? SKINNY_MAX_T / 2 : SKINNY_MAX_T) && K % sk_bk(1, false) == 0; }
+
 void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream) {
-  if (a.K % SK_BK != 0 || a.tokens < 1 || a.tokens > SKINNY_MAX_T) throw std::runtime_error("skinny gemm: K % 64 == 0, 1 .. 128 tokens per expert");
-  SkinnyKernelParams p{};
   const bool glu = a.act != 0;
+  if (a.K % SK_BK != 0 || a.tokens < 1 || a.tokens > SKINNY_MAX_T) throw std::runtime_error("skinny gemm: K % 64 == 0, 1 .. 128 tokens per expert");
+  if (a.wt != 0 && (!skinny_gemm8_supported(a.tokens, a.K, glu) || a.n_active != nullptr || a.scale == nullptr))
+    throw std::runtime_error("skinny gemm, 8-bit weights: one weight with scales, K % 128 == 0, 1 .. 128 tokens (64 with a gate product)");
+  SkinnyKernelParams p{};
   p.rows = glu ? 2 * a.n_out : a.n_out;
   p.xb = skinny_gemm_rows(a.tokens);
-  sk_map(&p.tm_w, a.w, (long long)a.experts * p.rows, a.K, a.K, SK_BM);
+  const bool wide = a.wt == 0 && !glu && a.n_active == nullptr && a.K % 128 == 0;
+  sk_map(&p.tm_w, a.w, (long long)a.experts * p.rows, a.K, a.K, SK_BM, a.wt != 0, wide ? 2 : 1);
   p.xbox = a.n_active ? 16 : p.xb;
-  sk_map(&p.tm_x, a.x, a.x_rows, a.K, a.ldx, p.xbox);
+  sk_map(&p.tm_x, a.x, a.x_rows, a.K, a.ldx, p.xbox, false, wide || a.wt ? 2 : 1);
   p.n_active = a.n_active; p.active = a.active; p.seg_start = a.seg_start; p.seg_count = a.seg_count;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(a.bias);
   p.residual = reinterpret_cast<const __nv_bfloat16*>(a.residual);
+  p.scale = a.scale; p.scale_step = a.scale_n > 1 ? 1 : 0;
   p.y = a.y; p.y_f32 = a.y_f32; p.ws = a.ws; p.tickets = a.tickets;
   p.T = a.tokens; p.n_out = a.n_out; p.K = a.K; p.act = a.act; p.limit = a.limit; p.alpha = a.alpha; p.w_fresh = a.w_fresh;
   check_waits();
   p.wait_word = wait_word(WAIT_SKINNY);
   count_launch(COUNT_SKINNY);
-  const int stage = (glu ? 2 : 1) * SK_W_BYTES + p.xb * SK_BK * 2;
-  p.stages = std::min(SK_MAX_STAGES, (SK_SMEM - 1024) / stage);
+  const int stage = (glu || wide ? 2 : 1) * SK_W_BYTES + p.xb * sk_bk(a.wt, wide) * 2;
+  p.stages = std::min(SK_MAX_STAGES, (SK_SMEM - 1024) / stage);       // at least SK_A_BUFS: see the order of waits in the warps that expand 8-bit weights
   int cols = 32;
-  while (cols < 2 * (glu ? 2 : 1) * p.xb) cols *= 2;
+  while (cols < 2 * (glu ? 2 : 1) * p.xb + (a.wt ? SK_A_BUFS * SK_A_COLS : 0)) cols *= 2;
   p.tmem_cols = cols;
   const size_t smem = (size_t)p.stages * stage + 1024;
-  auto kernel = glu ? skinny_gemm_kernel<true> : skinny_gemm_kernel<false>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM) != cudaSuccess)
-    throw std::runtime_error("skinny gemm: shared memory size refused");
-  launch_pdl(kernel, dim3(sk_grid()), dim3(SK_THREADS), smem, stream, p);
+  auto go = [&](auto kernel) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM) != cudaSuccess)
+      throw std::runtime_error("skinny gemm: shared memory size refused");
+    launch_pdl(kernel, dim3(sk_grid()), dim3(SK_THREADS), smem, stream, p);
+  };
+  if (a.wt == 0) glu ? go(skinny_gemm_kernel<true, 0, false>) : wide ? go(skinny_gemm_kernel<false, 0, true>) : go(skinny_gemm_kernel<false, 0, false>);
+  else if (a.wt == 1) glu ? go(skinny_gemm_kernel<true, 1, false>) : go(skinny_gemm_kernel<false, 1, false>);
+  else glu ? go(skinny_gemm_kernel<true, 2, false>) : go(skinny_gemm_kernel<false, 2, false>);
 }
 
 // ---- routed experts of a small step -------------------------------------------------------------------------------------------------------

@@ -1,0 +1,64 @@
+"""int8 / fp8 weights of 9 .. 128 tokens (csrc/skinny_gemm.cu): the bytes are expanded on their way to the tensor cores.
+
+Bound: rows are bf16, products and sums fp32, the scale is applied to the sum: results are rounded to bf16 once (2^-9 at most, 1.7e-3 rms)."""
+import pytest
+import torch
+
+from neuronx_distributed_inference_b200 import ops
+from neuronx_distributed_inference_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+DEV, BF = "cuda", torch.bfloat16
+TYPES = [torch.int8, torch.float8_e4m3fn]
+
+
+def _rel(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-9)).item()
+
+
+def _want(x, q, s, bias=None, act=None):
+    return ref.linear(x.double(), q.double() * s.double().view(-1, 1), None if bias is None else bias.double(), act=act)
+
+
+@pytest.mark.parametrize("wdtype", TYPES)
+@pytest.mark.parametrize("T", [9, 16, 17, 37, 64, 65, 100, 128])
+@pytest.mark.parametrize("N,K", [(8, 128), (136, 256), (4104, 384), (1000, 4096), (256, 14336), (20000, 128)])
+def test_plain(wdtype, T, N, K):
+    q, s = ref.quantize_per_channel(torch.randn(N, K, device=DEV) * 0.02, wdtype)
+    x = torch.randn(T, K, device=DEV, dtype=BF)
+    b, r = torch.randn(N, device=DEV, dtype=BF), torch.randn(T, N, device=DEV, dtype=BF)
+    assert _rel(ops.linear(x, q, scale=s), _want(x, q, s)) < 3e-3
+    assert _rel(ops.linear(x, q, b, scale=s, residual=r), _want(x, q, s, b) + r.double()) < 3e-3
+    assert _rel(ops.linear(x, q, scale=s.view(-1)[:1].contiguous()), _want(x, q, s.view(-1)[:1])) < 3e-3
+
+
+@pytest.mark.parametrize("wdtype", TYPES)
+@pytest.mark.parametrize("T,I,K", [(9, 72, 128), (32, 1344, 512), (37, 14336, 4096), (64, 8640, 3840), (65, 200, 2048)])
+@pytest.mark.parametrize("act", ["silu_mul", "gelu_tanh_mul"])
+def test_gate_product(wdtype, T, I, K, act):
+    q, s = ref.quantize_per_channel(torch.randn(2 * I, K, device=DEV) / K ** 0.5, wdtype)
+    x = torch.randn(T, K, device=DEV, dtype=BF)
+    b, n = torch.randn(2 * I, device=DEV, dtype=BF), torch.randn(K, device=DEV, dtype=BF)
+    # above 64 tokens the weight itself is rounded to bf16
+    assert _rel(ops.linear(x, q, b, scale=s, act=act), _want(x, q, s, b, act)) < (3e-3 if T <= 64 else 6e-3)
+    h = x.double() * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-5) * n.double()
+    assert _rel(ops.linear(x, q, b, norm_weight=n, norm_eps=1e-5, scale=s, act=act), _want(h, q, s, b, act)) < 8e-3
+
+
+@pytest.mark.parametrize("wdtype", TYPES)
+def test_every_byte(wdtype):
+    """All 256 values of a byte, in every position of a 16-byte piece: the expansion is exact (fp8: NaN stays NaN)."""
+    K = 256
+    q = torch.arange(256, device=DEV).view(256, 1).add(torch.arange(K, device=DEV)).remainder(256).to(torch.uint8).view(wdtype)
+    x = torch.zeros(16, K, device=DEV, dtype=BF)
+    for t in range(16):
+        x[t, 17 * t % K] = 1.0
+    got = ops.linear(x, q, scale=torch.ones(256, device=DEV))
+    want = torch.stack([q[:, 17 * t % K].float() for t in range(16)])
+    bad = torch.isnan(q.float()).any(-1)                       # 0 x NaN is NaN
+    assert torch.equal(got[:, ~bad].float(), want[:, ~bad])
+    assert torch.isnan(got[:, bad]).all()
+    if not bad.all():
+        return
+    q = torch.where(torch.isnan(q.float()), torch.zeros_like(q.float()), q.float()).to(wdtype)
+    assert torch.equal(ops.linear(x, q, scale=torch.ones(256, device=DEV)).float(), torch.stack([q[:, 17 * t % K].float() for t in range(16)]))
