@@ -388,7 +388,9 @@ at::Tensor moe_decode(const at::Tensor& x, const at::Tensor& w_gate_up, const at
   return y.to(x.scalar_type());
 }
 
-// Routed experts of a step of up to 128 tokens: every expert's weights are streamed once for all its tokens (bf16; act and biases as moe_grouped)
+constexpr int64_t MOE_SMALL_ENTRIES = 2560;       // (token, slot) pairs that moe_small_gather_kernel counts by comparing each with all
+// Routed experts of a step of up to 128 tokens, or of a few hundred: every expert's weights are streamed once for up to 128 of its tokens (bf16; act and biases as
+// moe_grouped)
 at::Tensor moe_small(const at::Tensor& x, const at::Tensor& w_gate_up, const at::Tensor& w_down, const at::Tensor& topk_w, const at::Tensor& topk_i,
                      int64_t expert_offset, int64_t act, bool scale_input, const c10::optional<at::Tensor>& gate_up_bias,
                      const c10::optional<at::Tensor>& down_bias, double limit, double alpha) {
@@ -396,7 +398,9 @@ at::Tensor moe_small(const at::Tensor& x, const at::Tensor& w_gate_up, const at:
   TORCH_CHECK(w_gate_up.dim() == 3 && w_down.dim() == 3 && w_gate_up.is_contiguous() && w_down.is_contiguous() && act >= 1 && act <= 4);
   const int N = x.size(0), H = x.size(1), E = w_gate_up.size(0), I = w_gate_up.size(1) / 2, k = topk_i.size(1);
   TORCH_CHECK(w_gate_up.size(1) == 2 * I && w_gate_up.size(2) == H && w_down.size(0) == E && w_down.size(1) == H && w_down.size(2) == I);
-  TORCH_CHECK(N >= 1 && N <= SKINNY_MAX_T && H % 64 == 0 && I % 64 == 0 && E <= 512, "moe_small: 1 .. 128 tokens, sizes in multiples of 64, <= 512 experts");
+  const int most = std::min(N, SKINNY_MAX_T);                      // rows of a segment
+  TORCH_CHECK(N >= 1 && (N <= SKINNY_MAX_T || (int64_t)N * k <= MOE_SMALL_ENTRIES) && H % 64 == 0 && I % 64 == 0 && E <= 512,
+              "moe_small: 1 .. 128 tokens (or 2560 entries), sizes in multiples of 64, <= 512 experts");
   TORCH_CHECK(topk_w.scalar_type() == at::kFloat && is_ids(topk_i) && topk_w.is_contiguous() && topk_i.is_contiguous() &&
               topk_w.numel() == (int64_t)N * k && topk_i.size(0) == N);
   if (gate_up_bias) TORCH_CHECK(is_bf16(*gate_up_bias) && gate_up_bias->is_contiguous() && gate_up_bias->numel() == (int64_t)E * 2 * I);
@@ -408,10 +412,10 @@ at::Tensor moe_small(const at::Tensor& x, const at::Tensor& w_gate_up, const at:
   auto y = at::empty({R, H}, fopt);
   // an expert has at most N entries when every token names it once, but nothing forbids a token to name it again (k times N): its rows are cut into
   // segments of what the GEMM's token tile holds
-  const int seg_rows = skinny_gemm_rows(N);
+  const int seg_rows = skinny_gemm_rows(most);
   const int64_t segs = std::min<int64_t>(E, R) + R / seg_rows;
   auto meta = at::empty({R + 1 + 3 * segs + 2 * nt}, iopt);       // pos | n_active | active | seg_start | seg_count | tickets of both GEMMs
-  auto ws = at::empty({std::max(skinny_gemm_ws_floats(N, true), skinny_gemm_ws_floats(N, false))}, fopt);
+  auto ws = at::empty({std::max(skinny_gemm_ws_floats(most, true), skinny_gemm_ws_floats(most, false))}, fopt);
   int* pos = meta.data_ptr<int>();
   int *n_active = pos + R, *active = n_active + 1, *seg_start = active + segs, *seg_count = seg_start + segs;
   unsigned* tickets = reinterpret_cast<unsigned*>(seg_count + segs);
@@ -420,7 +424,7 @@ at::Tensor moe_small(const at::Tensor& x, const at::Tensor& w_gate_up, const at:
                           scale_input ? 1 : 0, xp.data_ptr(), pos, n_active, active, seg_start, seg_count, tickets, (int)(2 * nt), st);
   SkinnyGemm a{};
   a.x = xp.data_ptr(); a.x_rows = R; a.ldx = H; a.w = w_gate_up.data_ptr(); a.bias = optr(gate_up_bias); a.y = h.data_ptr();
-  a.experts = E; a.tokens = N; a.n_out = I; a.K = H; a.act = (int)act; a.limit = (float)limit; a.alpha = (float)alpha;
+  a.experts = E; a.tokens = most; a.n_out = I; a.K = H; a.act = (int)act; a.limit = (float)limit; a.alpha = (float)alpha;
   a.n_active = n_active; a.active = active; a.seg_start = seg_start; a.seg_count = seg_count;
   a.ws = ws.data_ptr<float>(); a.tickets = tickets;
   skinny_gemm_launch(a, st);

@@ -44,6 +44,7 @@ constexpr int SK_SMEM = 220 * 1024;
 struct SkinnyKernelParams {
   CUtensorMap tm_w;        // [experts * rows, K], box {64, 128} (bytes: {128, 128}); wide: as {64, rows, K / 64}, box {64, 128, 2}
   CUtensorMap tm_x;        // [token rows, K], box {64, xbox}: xb rows for one expert, 16 when grouped (an expert loads as many as it has tokens for); 128 k: {64, xb, 2}
+  CUtensorMap tm_x64;      // grouped, segments of more than 48 rows: box {64, 64}
   const int *n_active, *active, *seg_start, *seg_count;     // grouped: segments (expert, first row of x, rows <= xb); null: one expert, T rows
   const __nv_bfloat16 *bias, *residual;                      // [experts * rows]; [T, n_out] (one expert)
   const float* scale;      // 8-bit weights: [rows], or [1] with scale_step 0
@@ -142,6 +143,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
   if (warp == 0 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_w) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_x) : "memory");
+    if (p.n_active) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tm_x64) : "memory");
     for (int s = 0; s < ST; ++s) {
       mbar_init(&full_bar[s], 2);         // the two producers
       mbar_init(&empty_bar[s], WT ? 1 + 4 * NW : 1);      // the MMAs' commit, and the warps that expand the weights
@@ -187,7 +189,14 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
         const int tile = (int)(u / nkb), kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u));
         const int ei = tile / n_tiles, n0 = (tile % n_tiles) * SK_BM, e = grouped ? p.active[ei] : 0;
         const int row_w = e * p.rows + n0, row_x = grouped ? p.seg_start[ei] : 0;
-        const int boxes = grouped ? (p.seg_count[ei] + p.xbox - 1) / p.xbox : 1, box_bytes = p.xbox * SK_BK * 2;
+        // a segment's rows in boxes of 64 as far as they go, the rest in one more (where it fits) or in up to two of 16: each copy costs the issuing thread 0.25 us
+        int boxes = 1, big = 0;
+        const int box_bytes = p.xbox * SK_BK * 2;
+        if (grouped) {
+          const int cnt = p.seg_count[ei];
+          big = cnt / 64 + (cnt % 64 > 32 && (cnt / 64 + 1) * 64 <= p.xb ? 1 : 0);
+          boxes = max(0, (cnt - big * 64 + 15) / 16);
+        }
         for (int kb = kb0; kb < kb1; ++kb) {
           if (early && phase != 0) {       // the ring is full: from here on a wait depends on the warps that wait for earlier kernels
             pdl_wait();
@@ -202,9 +211,14 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
             else sk_tma(st, &p.tm_w, kb * BK, row_w, &full_bar[s]);
             if (GLU) sk_tma(st + W_BYTES, &p.tm_w, kb * BK, row_w + p.n_out, &full_bar[s]);
           } else {
-            mbar_expect(&full_bar[s], boxes * box_bytes * XBOX);
-            if (XBOX == 2) sk_tma3(st + NW * W_BYTES, &p.tm_x, 0, kb * 2, &full_bar[s]);
-            for (int q = 0; q < boxes && XBOX == 1; ++q) sk_tma(st + NW * W_BYTES + q * box_bytes, &p.tm_x, kb * BK, row_x + q * p.xbox, &full_bar[s]);
+            mbar_expect(&full_bar[s], boxes * box_bytes * XBOX + big * (64 * SK_BK * 2));
+            uint8_t* xs = st + NW * W_BYTES;
+            if (XBOX == 2) {
+              sk_tma3(xs, &p.tm_x, 0, kb * 2, &full_bar[s]);
+            } else {
+              for (int q = 0; q < big; ++q) sk_tma(xs + q * (64 * SK_BK * 2), &p.tm_x64, kb * BK, row_x + q * 64, &full_bar[s]);
+              for (int q = 0; q < boxes; ++q) sk_tma(xs + big * (64 * SK_BK * 2) + q * box_bytes, &p.tm_x, kb * BK, row_x + big * 64 + q * p.xbox, &full_bar[s]);
+            }
           }
           if (++s == ST) {
             s = 0;
@@ -542,6 +556,7 @@ void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream) {
   sk_map(&p.tm_w, a.w, (long long)a.experts * p.rows, a.K, a.K, SK_BM, a.wt != 0, wide ? 2 : 1);
   p.xbox = a.n_active ? 16 : p.xb;
   sk_map(&p.tm_x, a.x, a.x_rows, a.K, a.ldx, p.xbox, false, wide || a.wt ? 2 : 1);
+  if (a.n_active) sk_map(&p.tm_x64, a.x, a.x_rows, a.K, a.ldx, 64);
   p.n_active = a.n_active; p.active = a.active; p.seg_start = a.seg_start; p.seg_count = a.seg_count;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(a.bias);
   p.residual = reinterpret_cast<const __nv_bfloat16*>(a.residual);

@@ -407,7 +407,8 @@ def moe_experts(x, w_gate_up, w_down, topk_w, topk_i, act="silu_mul", expert_off
                    and x.shape[1] % 8 == 0 and w_down.shape[2] % 8 == 0 and max(x.shape[1], w_down.shape[2]) * 2 <= 65536)
     # small steps: every expert's weights are streamed once for all its tokens, evenly over the SMs (csrc/skinny_gemm.cu)
     if (_use_cuda(x) and _MOE_GROUPED and x.dtype == torch.bfloat16 and w_gate_up.dtype == x.dtype and w_down.dtype == x.dtype
-            and kact in _MOE_ACTS and (_MOE_ROWS_TOKENS if rows_kernel else 0) < N <= _MOE_SMALL_TOKENS and topk_i.dim() == 2 and topk_i.shape[1] <= 64
+            and kact in _MOE_ACTS and (_MOE_ROWS_TOKENS if rows_kernel else 0) < N and topk_i.dim() == 2 and topk_i.shape[1] <= 64
+            and (N <= _MOE_SMALL_TOKENS or _few_rows_of_large_experts(N * topk_i.shape[1], w_gate_up))
             and w_gate_up.is_contiguous() and w_down.is_contiguous() and x.shape[1] % 64 == 0 and w_down.shape[2] % 64 == 0
             and w_gate_up.shape[0] <= 512
             and (gate_up_bias is None or gate_up_bias.dtype == x.dtype) and (down_bias is None or down_bias.dtype == x.dtype)):
@@ -443,8 +444,18 @@ def _expert_ids(ids):
 _MOE_GROUPED = os.environ.get("NXDI_B200_MOE_GROUPED", "1") == "1"
 # measured (us, rows kernel / small-step path): 128 experts, 8 chosen, 2048 x 768: 26 / 36, 37 / 57, 80 / 74, 137 / 105 at 1, 2, 4, 8 tokens; 8 experts, 2 chosen,
 # 4096 x 14336: 132 / 139, 222 / 185 and 697 / 386 at 1, 2 and 8.  Against the CTA-pair path at 12, 48 and 128 tokens: 147 / 129, 259 / 210, 271 / 219 and
-# 539 / 436, 568 / 461, 587 / 543; 16 experts, 4 chosen, 6144 x 1344: 254 / 186, 190 / 163, 201 / 175 at 16, 48 and 128
+# 539 / 436, 568 / 461, 587 / 481; 16 experts, 4 chosen, 6144 x 1344: 254 / 186, 190 / 163, 201 / 175 at 16, 48 and 128
 _MOE_ROWS_TOKENS, _MOE_SMALL_TOKENS = 2, 128
+
+
+def _few_rows_of_large_experts(entries: int, w_gate_up) -> bool:
+    """Steps of more than 128 tokens whose experts still wait for their weights: segments of up to 128 rows against 256-row tiles (us, segments / tiles; 8 experts of
+    4096 x 14336, 2 chosen: 480 / 560 at 150 and 192 tokens, 592 / 611 at 300, 774 / 629 at 512; 16 of 6144 x 1344, 4 chosen: 190 / 225 at 192, 243 / 240 at 400; 128 of
+    2048 x 768, 8 chosen: 250 / 272 at 129, 274 / 278 at 300, 286 / 284 at 512).  Small experts stay where they are."""
+    E, rows, H = w_gate_up.shape
+    return entries <= min(48 * E, 2560) and rows * H >= 1 << 20
+
+
 _MOE_ACTS = {"silu_mul": 1, "gelu_tanh_mul": 2, "gelu_mul": 3, "gpt_oss_glu": 4, "clamped_glu": 4}      # 4 takes (limit, alpha); gpt_oss_glu: 7, 1.702
 _UNARY_ACTS = {"relu": 1, "relu2": 2, "silu": 3, "gelu_tanh": 4, "sigmoid": 5, "gelu": 6}         # codes of csrc/seqmix.cu (unary_act, moe_plain, gated_act_mul)
 _MOE_PLAIN_ACTS = _UNARY_ACTS

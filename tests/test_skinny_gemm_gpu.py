@@ -106,3 +106,29 @@ def test_groups_of_eight_tokens(T, form):
     want = ref.linear(x.float(), w.float(), **{k: v for k, v in kf.items() if k != "residual"})
     # the normalised rows are rounded to bf16 too
     assert _rel(ops.linear(x, w, **kw), want if res is None else want + res) < (5e-3 if form == "norm" else 3e-3)
+
+
+@pytest.mark.parametrize("N,form", [(129, "even"), (190, "even"), (190, "one expert"), (191, "half"), (130, "bias"), (190, "scaled")])
+def test_large_experts_of_a_few_hundred_tokens(N, form):
+    """Segments of up to 128 rows where an expert has more, boxes of 64 and 16 token rows; the same bits every time."""
+    E, k, H, I = 8, 2, 1024, 512
+    x = torch.randn(N, H, device=DEV, dtype=BF)
+    wg = (torch.randn(E, 2 * I, H, device=DEV) / math.sqrt(H)).to(BF)
+    wd = (torch.randn(E, H, I, device=DEV) / math.sqrt(I)).to(BF)
+    w, i = torch.topk(torch.softmax(torch.randn(N, E, device=DEV), -1), k, -1)
+    if form == "one expert":
+        i[:, 0], i[:, 1] = 3, 5
+    if form == "half":
+        i[:N // 2, 0], i[:N // 2, 1] = 3, 6
+    kw, kf = {}, {}
+    if form == "bias":
+        bg, bd = torch.randn(E, 2 * I, device=DEV, dtype=BF), torch.randn(E, H, device=DEV, dtype=BF)
+        kw, kf = dict(gate_up_bias=bg, down_bias=bd), dict(gate_up_bias=bg.float(), down_bias=bd.float())
+    if form == "scaled":
+        kw = kf = dict(scale_input=True)
+    before = ops.kernel_launches()["skinny_gemm"]
+    got = ops.moe_experts(x, wg, wd, w, i, "silu_mul", 0, **kw)
+    assert ops.kernel_launches()["skinny_gemm"] == before + 2
+    assert _rel(got, ref.moe_experts(x.float(), wg.float(), wd.float(), w, i, "silu_mul", 0, **kf)) < 5e-3
+    for _ in range(5):
+        assert torch.equal(ops.moe_experts(x, wg, wd, w, i, "silu_mul", 0, **kw), got)
