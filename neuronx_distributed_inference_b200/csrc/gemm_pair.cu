@@ -65,13 +65,19 @@ __device__ __forceinline__ uint64_t gp_desc(const void* smem) {     // K-major, 
   d |= (uint64_t)2 << 61;
   return d;
 }
-__device__ __forceinline__ void gp_umma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d), "l"(da),
-               "l"(db), "r"(idesc), "r"(acc) : "memory");
+// Called by a whole warp, issued by the lane whose `on` is 1: in code that all lanes run the descriptors stay in uniform registers
+__device__ __forceinline__ void gp_umma(uint32_t on, uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d), "l"(da),
+               "l"(db), "r"(idesc), "r"(acc), "r"(on) : "memory");
 }
-__device__ __forceinline__ void gp_commit_both(uint64_t* bar) {      // arrives on the barrier at this offset in both CTAs
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(mbar_s32(bar)),
-               "h"((unsigned short)3) : "memory");
+__device__ __forceinline__ void gp_commit_both(uint32_t on, uint64_t* bar) {      // arrives on the barrier at this offset in both CTAs
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(mbar_s32(bar)),
+               "h"((unsigned short)3), "r"(on) : "memory");
+}
+__device__ __forceinline__ uint32_t gp_elect() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
 }
 __device__ __forceinline__ void gp_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -138,13 +144,14 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
   const uint32_t tmem = *tmem_slot;
   pdl_launch_dependents();
   // a weight that is a parameter does not depend on earlier kernels; everything else does
-  const bool early = warp == 0 && p.tile_expert == nullptr && !p.w_fresh;
+  bool early = warp == 0 && p.tile_expert == nullptr && !p.w_fresh;
   if (!early) pdl_wait();
 
   if (warp == 0 || warp == 3) {
     // ================= TMA producers: B (warp 0), A (warp 3) of this CTA =================
     if (lane == 0) {
-      long long it = 0;
+      int s = 0;
+      uint32_t phase = 0;
       bool go = true;
       for (int t = pair; t < total && go; t += pairs) {
         int mt, nt;
@@ -160,10 +167,12 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
         }
         const int row_a = m0 + (int)rank * 128;
         const int row_b = e * p.N + (glu ? nt * (BN / 2) + (rank ? p.n_out : 0) : nt * BN + (int)rank * (BN / 2));
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const int s = (int)(it % ST);
-          if (early && it == ST) pdl_wait();         // the ring is full: from here on a wait depends on the warps that wait for earlier kernels
-          go = mbar_wait<true>(&empty_bar[s], (uint32_t)((it / ST) & 1) ^ 1u, stop, p.wait_word);
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (early && phase != 0) {       // the ring is full: from here on a wait depends on the warps that wait for earlier kernels
+            pdl_wait();
+            early = false;
+          }
+          go = mbar_wait<true>(&empty_bar[s], phase ^ 1u, stop, p.wait_word);
           if (!go) break;
           uint8_t* st = smem + s * STAGE;
           const uint32_t bar = gp_leader(&full_bar[s]);
@@ -173,16 +182,22 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
             if (rank == 0) mbar_expect(&full_bar[s], 2 * STAGE - (second ? 0 : GP_A_BYTES));       // everything that both CTAs copy for this stage
             if (rank == 0 || second) gp_tma(st, &p.tma_a, kb * GP_BK, row_a, bar);
           }
+          if (++s == ST) {
+            s = 0;
+            phase ^= 1u;
+          }
         }
       }
     }
   } else if (warp == 1) {
-    // ================= MMA issuer: one thread of the leader =================
-    if (rank == 0 && lane == 0) {
+    // ================= MMA issuer: a warp of the leader =================
+    if (rank == 0) {
       // D = f32, A = B = bf16, both K-major, M = 256, N = BN
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
-      long long it = 0;
-      int tc = 0;
+      const uint32_t on = gp_elect();
+      const uint64_t da0 = gp_desc(smem), db0 = gp_desc(smem + GP_A_BYTES);
+      int tc = 0, s = 0;
+      uint32_t phase = 0;
       bool go = true;
       for (int t = pair; t < total && go; t += pairs) {
         if (p.tile_expert != nullptr) {
@@ -191,21 +206,24 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
           if (__ldg(p.tile_expert + mt) < 0) continue;
         }
         const int buf = tc & 1;
-        go = mbar_wait<true>(&tmem_empty[buf], (uint32_t)((tc >> 1) & 1) ^ 1u, stop, p.wait_word);
+        go = mbar_wait_warp<true>(&tmem_empty[buf], (uint32_t)((tc >> 1) & 1) ^ 1u, stop, p.wait_word);
         if (!go) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const int s = (int)(it % ST);
-          go = mbar_wait<true>(&full_bar[s], (uint32_t)((it / ST) & 1), stop, p.wait_word);
+        for (int kb = 0; kb < nkb; ++kb) {
+          go = mbar_wait_warp<true>(&full_bar[s], phase, stop, p.wait_word);
           if (!go) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint64_t da = gp_desc(smem + s * STAGE), db = gp_desc(smem + s * STAGE + GP_A_BYTES);
+          const uint64_t da = da0 + (uint64_t)(s * (STAGE >> 4)), db = db0 + (uint64_t)(s * (STAGE >> 4));
 #pragma unroll
           for (int k = 0; k < GP_BK / 16; ++k)       // 16 k = 32 bytes inside the swizzle atom
-            gp_umma(tmem + (uint32_t)(buf * BN), da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0 ? 1u : 0u);
-          gp_commit_both(&empty_bar[s]);
+            gp_umma(on, tmem + (uint32_t)(buf * BN), da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0 ? 1u : 0u);
+          gp_commit_both(on, &empty_bar[s]);
+          if (++s == ST) {
+            s = 0;
+            phase ^= 1u;
+          }
         }
-        if (go) gp_commit_both(&tmem_full[buf]);
+        if (go) gp_commit_both(on, &tmem_full[buf]);
         ++tc;
       }
     }
@@ -272,14 +290,19 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
 #pragma unroll
                 for (int k = 0; k < 8; ++k) up[k] += __bfloat162float(p.bias[eo + p.n_out + col0 + j + k]);
               }
+              // the activation is chosen once for eight values: chosen for each, they ran one after the other
+              if (p.act == 1) {
 #pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                if (p.act == 4) {        // (clamp(up, -limit, limit) + 1) * g * sigmoid(alpha g), g = min(gate, limit)
+                for (int k = 0; k < 8; ++k) f[k] = silu(f[k]) * up[k];
+              } else if (p.act == 4) {     // (clamp(up, -limit, limit) + 1) * g * sigmoid(alpha g), g = min(gate, limit)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
                   const float g = fminf(f[k], p.limit), u = fminf(fmaxf(up[k], -p.limit), p.limit);
                   f[k] = (u + 1.f) * g * (1.f / (1.f + __expf(-p.alpha * g)));
-                } else {
-                  f[k] = (p.act == 1 ? silu(f[k]) : (p.act == 2 ? gelu_tanh(f[k]) : gelu_erf(f[k]))) * up[k];
                 }
+              } else {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) f[k] = (p.act == 2 ? gelu_tanh(f[k]) : gelu_erf(f[k])) * up[k];
               }
             }
             uint4* at = stg_at(lane, (c - c0 + j) >> 3);

@@ -9,7 +9,7 @@
 //     <TM 1, BN 128>  M <= 128.
 //   * warp 0: TMA producer (cp.async.bulk.tensor.2d, SWIZZLE_128B) through a 4-deep mbarrier ring of 32/48 KB stages; the WEIGHT
 //     tiles of the first ring fill are issued BEFORE griddepcontrol.wait (weights never depend on the previous kernel);
-//   * warp 1: ONE elected thread issues tcgen05.mma.cta_group::1.kind::f16 with shared-memory descriptors; accumulators live in
+//   * warp 1: the warp issues, by one elected lane, tcgen05.mma.cta_group::1.kind::f16 with shared-memory descriptors; accumulators live in
 //     TMEM, double buffered (2 x TM x 128 columns): tcgen05.commit releases smem stages and hands a finished accumulator to the
 //     epilogue through mbarriers, and the mainloop of tile i+1 runs while tile i is being written out;
 //   * warps 4..7: epilogue — tcgen05.ld (32x32b: one TMEM lane = one output row per thread), bias / residual / SwiGLU (tile = 64
@@ -111,26 +111,33 @@ __device__ __forceinline__ uint64_t umma_desc(const void* smem) {
 __host__ __device__ constexpr uint32_t umma_idesc(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+// Called by a whole warp, issued by the lane whose `on` is 1: in code that all lanes run the descriptors stay in uniform registers
+__device__ __forceinline__ void umma_f16(uint32_t on, uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(on)
       : "memory");
 }
-__device__ __forceinline__ void umma_f8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_f8(uint32_t on, uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(on)
       : "memory");
 }
 // instruction descriptor for kind::f8f6f4: D = f32, A = B = e4m3 (format 0), both K-major
 __host__ __device__ constexpr uint32_t umma_idesc_f8(int M, int N) {
   return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s_u32(bar)) : "memory");
+__device__ __forceinline__ void umma_commit(uint32_t on, uint64_t* bar) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(s_u32(bar)), "r"(on)
+               : "memory");
+}
+__device__ __forceinline__ uint32_t umma_elect() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
@@ -206,7 +213,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tcgen05_kernel(const __gri
       const bool is_b = warp == 0;
       // (grouped: the routing plan comes from the preceding kernels; fresh: the weight does — the weight producer waits too)
       if (!is_b || p.grp_tile_expert != nullptr || p.w_fresh) pdl_wait();
-      long long it = 0;   // k-block counter across work items (ring position)
+      int s = 0;          // ring position, counted across work items
+      uint32_t ph = 0;
       for (int w = blockIdx.x; w < total_tiles; w += gridDim.x) {
         const int t = w / S, ks = w % S;
         const int m0 = (t % p.m_tiles) * (TM * GM_BM), n_out0 = (t / p.m_tiles) * tile_out;
@@ -217,9 +225,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tcgen05_kernel(const __gri
           if (e < 0) continue;
           eo = e * p.N;
         }
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = (int)(it % GM_STAGES);
-          const uint32_t ph = (uint32_t)((it / GM_STAGES) & 1);
+        for (int kb = kb0; kb < kb1; ++kb) {
           mb_wait(&empty_bar[s], ph ^ 1u);
           if (is_b) {
             mb_expect(&full_bar[s], B_BYTES);
@@ -234,46 +240,54 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tcgen05_kernel(const __gri
             mb_expect(&full_bar[s], TM * GM_A_BYTES);
             tma_2d(smem + s * STAGE_BYTES, &p.tma_a, kb * BKE, m0, &full_bar[s]);
           }
+          if (++s == GM_STAGES) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
       }
     }
   } else if (warp == 1) {
-    // ================= MMA issuer (one thread) =================
-    if (lane == 0) {
-      constexpr uint32_t idesc = FP8 ? umma_idesc_f8(GM_BM, BN) : umma_idesc(GM_BM, BN);
-      long long it = 0;
-      int tc = 0;
-      if (p.grp_tile_expert != nullptr) pdl_wait();
-      for (int w = blockIdx.x; w < total_tiles; w += gridDim.x) {
-        const int ks = w % S;
-        if (p.grp_tile_expert != nullptr && __ldg(p.grp_tile_expert + (w / S) % p.m_tiles) < 0) continue;
-        const int kb0 = (int)((long long)nkb * ks / S), kb1 = (int)((long long)nkb * (ks + 1) / S);
-        const int buf = tc & 1;
-        mb_wait(&tmem_empty[buf], (uint32_t)(((tc >> 1) & 1) ^ 1));   // the epilogue has drained this accumulator buffer
+    // ================= MMA issuer =================
+    constexpr uint32_t idesc = FP8 ? umma_idesc_f8(GM_BM, BN) : umma_idesc(GM_BM, BN);
+    const uint32_t on = umma_elect();
+    const uint64_t da0 = umma_desc(smem), db0 = umma_desc(smem + TM * GM_A_BYTES);
+    int tc = 0, s = 0;
+    uint32_t ph = 0;
+    if (p.grp_tile_expert != nullptr) pdl_wait();
+    for (int w = blockIdx.x; w < total_tiles; w += gridDim.x) {
+      const int ks = w % S;
+      if (p.grp_tile_expert != nullptr && __ldg(p.grp_tile_expert + (w / S) % p.m_tiles) < 0) continue;
+      const int kb0 = (int)((long long)nkb * ks / S), kb1 = (int)((long long)nkb * (ks + 1) / S);
+      const int buf = tc & 1;
+      mb_wait(&tmem_empty[buf], (uint32_t)(((tc >> 1) & 1) ^ 1));   // the epilogue has drained this accumulator buffer
+      __syncwarp();
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      for (int kb = kb0; kb < kb1; ++kb) {
+        mb_wait(&full_bar[s], ph);
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = (int)(it % GM_STAGES);
-          const uint32_t ph = (uint32_t)((it / GM_STAGES) & 1);
-          mb_wait(&full_bar[s], ph);
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint64_t db = umma_desc(smem + s * STAGE_BYTES + TM * GM_A_BYTES);
+        const uint64_t db = db0 + (uint64_t)(s * (STAGE_BYTES >> 4));
 #pragma unroll
-          for (int sub = 0; sub < TM; ++sub) {
-            const uint64_t da = umma_desc(smem + s * STAGE_BYTES + sub * GM_A_BYTES);
-            const uint32_t acc = tmem_base + (uint32_t)(buf * ACC_COLS + sub * BN);
+        for (int sub = 0; sub < TM; ++sub) {
+          const uint64_t da = da0 + (uint64_t)(s * (STAGE_BYTES >> 4) + sub * (GM_A_BYTES >> 4));
+          const uint32_t acc = tmem_base + (uint32_t)(buf * ACC_COLS + sub * BN);
 #pragma unroll
-            for (int k = 0; k < GM_BK / 16; ++k) {
-              // advance 16 bf16 = 32 bytes along K inside the 128-byte swizzle atom: +2 in the (addr >> 4) field
-              // (fp8: 32 elements = 32 bytes per instruction; bf16: 16 elements = 32 bytes — the same descriptor step)
-              if (FP8) umma_f8(acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb != kb0 || k != 0) ? 1u : 0u);
-              else umma_f16(acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb != kb0 || k != 0) ? 1u : 0u);
-            }
+          for (int k = 0; k < GM_BK / 16; ++k) {
+            // advance 16 bf16 = 32 bytes along K inside the 128-byte swizzle atom: +2 in the (addr >> 4) field
+            // (fp8: 32 elements = 32 bytes per instruction; bf16: 16 elements = 32 bytes — the same descriptor step)
+            if (FP8) umma_f8(on, acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+            else umma_f16(on, acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb != kb0 || k != 0) ? 1u : 0u);
           }
-          umma_commit(&empty_bar[s]);       // frees the smem stage when these MMAs retire
         }
-        umma_commit(&tmem_full[buf]);       // accumulator(s) of this tile complete
-        ++tc;
+        umma_commit(on, &empty_bar[s]);       // frees the smem stage when these MMAs retire
+        if (++s == GM_STAGES) {
+          s = 0;
+          ph ^= 1u;
+        }
       }
+      umma_commit(on, &tmem_full[buf]);       // accumulator(s) of this tile complete
+      ++tc;
     }
   } else if (warp >= 4) {
     // ================= epilogue: TMEM -> registers -> (split-K fix-up) -> global =================
@@ -316,40 +330,57 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tcgen05_kernel(const __gri
           sc_u[j] = u4.x * as; sc_u[j + 1] = u4.y * as; sc_u[j + 2] = u4.z * as; sc_u[j + 3] = u4.w * as;
         }
       }
+      uint4 r4[4];          // the residual's loads before their first use
+      if (res) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 8)
+          if (col0 + j + 8 <= n_out) r4[j >> 3] = ldg_act(res + j);
+      }
 #pragma unroll
       for (int j = 0; j < 32; j += 8) {
-        float f[8];
+        float f[8], up[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          float a = __uint_as_float(vg[j + e]);
-          const bool in = col0 + j + e < n_out;
-          float up_s = 1.f;
+          f[e] = __uint_as_float(vg[j + e]);
+          up[e] = __uint_as_float(vu[j + e]);
           if (FP8) {
-            a *= sc_g[j + e];
-            up_s = sc_u[j + e];
+            f[e] *= sc_g[j + e];
+            up[e] *= sc_u[j + e];
           }
-          if (p.bias && in) a += __bfloat162float(p.bias[cur_eo + col0 + j + e]);
-          if (glu) {
-            float up = __uint_as_float(vu[j + e]) * up_s;
-            if (p.bias && in) up += __bfloat162float(p.bias[cur_eo + n_out + col0 + j + e]);
-            if (p.act == 4) {   // clamped gate product: (clamp(up, -limit, limit) + 1) * g * sigmoid(alpha g), g = min(gate, limit)
-              const float g = fminf(a, p.glu_limit), u = fminf(fmaxf(up, -p.glu_limit), p.glu_limit);
-              a = (u + 1.f) * g * (1.f / (1.f + __expf(-p.glu_alpha * g)));
-            } else {
-              a = (p.act == 1 ? silu(a) : (p.act == 2 ? gelu_tanh(a) : gelu_erf(a))) * up;
+        }
+        if (p.bias) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            if (col0 + j + e >= n_out) break;
+            f[e] += __bfloat162float(p.bias[cur_eo + col0 + j + e]);
+            if (glu) up[e] += __bfloat162float(p.bias[cur_eo + n_out + col0 + j + e]);
+          }
+        }
+        if (glu) {            // the activation is chosen once for eight values: chosen for each, they ran one after the other
+          if (p.act == 1) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = silu(f[e]) * up[e];
+          } else if (p.act == 4) {   // clamped gate product: (clamp(up, -limit, limit) + 1) * g * sigmoid(alpha g), g = min(gate, limit)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float g = fminf(f[e], p.glu_limit), u = fminf(fmaxf(up[e], -p.glu_limit), p.glu_limit);
+              f[e] = (u + 1.f) * g * (1.f / (1.f + __expf(-p.glu_alpha * g)));
             }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = (p.act == 2 ? gelu_tanh(f[e]) : gelu_erf(f[e])) * up[e];
           }
-          f[e] = a;
         }
         if (col0 + j + 8 <= n_out) {
           if (res) {
-            const uint4 r = ldg_act(res + j);
+            const uint4 r = r4[j >> 3];
             f[0] += bf16lo(r.x); f[1] += bf16hi(r.x); f[2] += bf16lo(r.y); f[3] += bf16hi(r.y);
             f[4] += bf16lo(r.z); f[5] += bf16hi(r.z); f[6] += bf16lo(r.w); f[7] += bf16hi(r.w);
           }
           *reinterpret_cast<uint4*>(dst + j) =
               make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
         } else {
+#pragma unroll
           for (int e = 0; e < 8; ++e)
             if (col0 + j + e < n_out) dst[j + e] = __float2bfloat16(f[e] + (res ? ldg_act_bf16(res + j + e) : 0.f));
         }
