@@ -123,16 +123,20 @@ static void check_gemv_inputs(const at::Tensor& x, const at::Tensor& w) {
   TORCH_CHECK(x.size(1) % 64 == 0 && x.stride(1) == 1 && x.stride(0) % 8 == 0 && w.is_contiguous());
 }
 
-// Where the swapped, evenly split GEMM (skinny_gemm.cu) beats the 128-row token tiles of gemm_tcgen05.cu (us in a graph, skinny / tiles; 16, 64, 96 and 128 tokens):
-//   gate|up 28672 x 4096: 43 / 61, 49 / 62, 53 / 62, 57 / 63     17280 x 3200: 24 / 48, 30 / 34, 34 / 34, 34 / 34    16384 x 2048: 16 / 33, 21 / 26, 25 / 26, 26 / 26
-//           8192 x 3072:  17 / 36, 21 / 23, 24 / 23, 27 / 23      6144 x 2048: 14 / 28, 20 / 18, 22 / 18, 25 / 18     2048 x 1024:   9 / 17, 12 / 17, 14 / 17, 17 / 17
-//   plain 4096 x 14336:   25 / 57, 29 / 58, 32 / 58, 35 / 59      6144 x 4096: 14 / 25, 17 / 26, 20 / 26, 22 / 26      2048 x 8192:  14 / 39, 17 / 39, 20 / 39, 23 / 40
-//           3072 x 3072:  12 / 20, 15 / 20, 18 / 20, 20 / 20      4096 x 1024:  9 / 11, 11 / 11, 13 / 11, 14 / 11       512 x 512:    8 / 8,  10 / 8,  11 / 8,  13 / 8
-// A feature's tokens are in one lane, so its epilogue and the fix-up of the cut tiles grow with the tokens, while the tile kernel's time does not change up to 128.
+// Where the swapped, evenly split GEMM (skinny_gemm.cu) beats the 128-row token tiles of gemm_tcgen05.cu (us in a graph, skinny / tiles; 16, 32, 48, 64 and 128 tokens):
+//   gate|up 28672 x 4096: 42 / 44, 44 / 44, 47 / 45, 49 / 45, 57 / 45     17280 x 3200: 24 / 24, 26 / 24, 29 / 24, 30 / 24, 37 / 25
+//           16384 x 4096: 27 / 28, 29 / 29, 32 / 29, 33 / 29, 41 / 30     16384 x 2048: 16 / 25, 18 / 16, 20 / 16, 21 / 16, 28 / 16
+//           12288 x 4096: 22 / 26, 24 / 27, 26 / 27, 28 / 27, 34 / 27     10240 x 5120: 24 / 30, 26 / 30, 28 / 30, 30 / 31, 37 / 31
+//   plain 4096 x 14336:   25 / 50, 26 / 50, 28 / 51, 29 / 51, 35 / 52     12288 x 4096: 21 / 28, 22 / 29, 26 / 29, 27 / 29, 33 / 30 (80 tokens 29 / 30, 96 31 / 30)
+//          4096 x 4096:   12 / 21, 13 / 21, 15 / 21, 15 / 21, 20 / 22      6144 x 4096: 14 / 21, 15 / 22, 17 / 22, 17 / 22, 22 / 22
+//          2048 x 2048:    8 / 15,  8 / 14, 10 / 14, 10 / 14, 14 / 14      4096 x 1024:  8 / 8,   8 / 8,  10 / 8,  10 / 7,  13 / 8
+// A feature's tokens are in one lane, so its epilogue and the fix-up of the cut tiles grow with the tokens, twice as fast with a gate product, while the tile kernel's
+// time does not change up to 128; deep K leaves the tile kernel few tiles.  Between other kernels it gains what it prefetches: a whole gated MLP at 37 tokens takes
+// 78.1 / 79.7 us with 28672 x 4096 and 63.6 / 65.1 with 22016 x 4096.
 static bool skinny_pays(int M, int rows, int K, bool glu) {
   const long long size = (long long)rows * K;
-  if (glu) return M <= 32 || (M <= 64 && size >= (16LL << 20)) || (M <= 96 && size >= (32LL << 20)) || (M <= SKINNY_MAX_T && size >= (64LL << 20));
-  return M <= 64 || (M <= SKINNY_MAX_T && (K >= 2 * rows || size >= (8LL << 20)));
+  if (glu) return M <= 32 || (M <= 40 && size >= (64LL << 20)) || (M <= 64 && rows <= 16384 && K >= 4096);
+  return M <= 64 || (M <= SKINNY_MAX_T && (K >= 2 * rows || (size >= (8LL << 20) && (M <= 80 || size < (32LL << 20)))));
 }
 
 // norm_w: x is normalised first; its kernel clears the GEMM's tickets, which else takes a launch of its own (1.5 us in the stream)
@@ -210,13 +214,18 @@ at::Tensor gemv(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
   return y;
 }
 
-// Where 256 x 256 tiles on CTA pairs (gemm_pair.cu) beat the one-CTA tiles (us, pairs / one CTA, isolated):
-//   28672 x 4096 gate|up: 62 / 84 at 256 tokens, 99 / 133 at 512, 624 / 725 at 4096      4096 x 14336: 74 / 55 at 256, 76 / 77 at 512, 80 / 94 at 768
-//   6144 x 4096: 26 / 26 at 256, 29 / 41 at 400, 71 / 82 at 2048                         2048 x 8192: 45 / 36 at 512, 45 / 49 at 768, 98 / 110 at 4096
-// Up to 512 tokens the one-CTA kernel has smaller tiles and split-K to fill the chip; with 40 pair tiles or more (of 74 pairs) they are not needed.
+// Where 256 x 256 tiles on CTA pairs (gemm_pair.cu) beat the one-CTA tiles (us in a graph, pairs / one CTA, at 256, 384, 512 and 768 tokens):
+//   gate|up 28672 x 4096: 57 / 64, 91 / 86, 95 / 111, 124 / 140     17280 x 3200: 28 / 32, 43 / 48, 43 / 50, 61 / 68     16384 x 2048: 20 / 23, 31 / 35, 29 / 33, 40 / 45
+//           22016 x 4096: 51 / 60, 70 / 63, 73 / 88, 98 / 110
+//   plain 12288 x 4096:   31 / 39, 47 / 40, 49 / 63, 58 / 68        6144 x 4096: 26 / 26, 28 / 26, 28 / 35, 31 / 36      4096 x 4096: 26 / 22, 27 / 25, 27 / 25, 28 / 33
+//         4096 x 14336:   74 / 54, 75 / 75, 73 / 74, 78 / 91        2048 x 8192: 43 / 35, 44 / 35, 44 / 35, 44 / 53
+// Up to 512 tokens the one-CTA kernel has smaller tiles and split-K to fill the chip; with 40 pair tiles or more (of 74 pairs) they are not needed, except up to 384
+// tokens, a quarter of whose pair tiles is padding, where the last wave of pairs is short too.
 static bool pair_pays(int M, int n_out, bool glu) {
-  return M > 512 || (M > 128 && ((M + 255) / 256) * ((n_out + (glu ? 127 : 255)) / (glu ? 128 : 256)) >= 40);
+  const int tiles = ((M + 255) / 256) * ((n_out + (glu ? 127 : 255)) / (glu ? 128 : 256)), waves = (tiles + 73) / 74;
+  return M > 512 || (M > 128 && tiles >= 40 && (M <= 256 || M > 384 || 5 * tiles >= 4 * 74 * waves));
 }
+
 
 // fresh_weight: w was written by a kernel enqueued just before (an expanded 8-bit weight).  The kernels fetch a parameter's first tiles before the
 // kernels in front of them have finished; such a weight has to be waited for.
