@@ -281,17 +281,24 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const T* __restrict_
     }
 }
 
-// Logits of up to sixteen experts: the kernel above gives a warp four of them and leaves the other warps of the block idle (eight experts: two of eight
-// warps work).  Here KW warps share the columns of four experts, read the rows and the weights straight from memory (no staging, no barrier in the loop;
-// the row of one warp is in L1 for the next) and their sums are added in order at the end.  Bound by the latency of a few rounds of loads.  Eight experts
-// of 4096 columns, logits and choice together: 6.9 us for 6 tokens, 8.4 for 300 (28 with the kernel above), 9.1 for 1000, 23 for 4096.
+// Logits of few tokens or few experts: the kernel above gives a warp four experts (one for a few tokens) and stages the rows, which leaves most of the chip idle.
+// Here KW warps share the columns of four experts, read the rows and the weights straight from memory (no staging, no barrier in the loop) and their sums are added in
+// order at the end; a block takes 32 / KW experts.  Bound by the latency of a few rounds of loads.  us in a graph, logits and choice together, here / a block per 4 tokens
+// with two or four warps per four experts (8, 16 experts) or staged rows: 8 experts of 4096 columns at 6, 100 tokens 5.2 / 7.4, 6.4 / 8.2; 16 of 6144 at 6, 179
+// 6.4 / 13.9, 8.8 / 15.3; 128 of 2048 at 9, 48, 179 7.9 / 14.6, 9.7 / 16.3, 15.1 / 16.5 (255: 18.1 / 16.5); 256 of 4096 at 9, 100, 179 11.5 / 22.4, 23 / 26, 34 / 31.
+// Half a microsecond to 1.5 of that come from launching both kernels before the one in front has ended.
 constexpr int RS_EG = 4;
-template <typename T, int RT, int KW>
+// EARLY: launched before the kernel in front has ended (the rows then come past L1); with many tokens the rows' lines in L1 are worth more
+template <typename T, int RT, int KW, bool EARLY>
 __global__ void __launch_bounds__(256) router_logits_split_kernel(const T* __restrict__ x, const float* __restrict__ w, float* __restrict__ logits,
                                                                   int N, int W, int E) {
   __shared__ float part[8][RT * RS_EG];
+  if (EARLY) {                    // (blocks of the choice that wait on an SM would keep this kernel's from it)
+    pdl_launch_dependents();
+    pdl_wait();
+  }
   const int t0 = blockIdx.x * RT, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int e0 = (warp / KW) * RS_EG;
+  const int eb = EARLY ? blockIdx.y * (8 / KW) * RS_EG : 0, e0 = eb + (warp / KW) * RS_EG;
   float acc[RT][RS_EG] = {};
   if (e0 < E) {
     const float* wr[RS_EG];
@@ -308,9 +315,11 @@ __global__ void __launch_bounds__(256) router_logits_split_kernel(const T* __res
 #pragma unroll
       for (int t = 0; t < RT; ++t) {
         if constexpr (std::is_same<T, float>::value) {
-          xv[t] = __ldg(reinterpret_cast<const float4*>(xr[t] + c));
+          const float4* q = reinterpret_cast<const float4*>(xr[t] + c);
+          xv[t] = EARLY ? __ldcg(q) : __ldg(q);
         } else {
-          const uint2 r = __ldg(reinterpret_cast<const uint2*>(xr[t] + c));
+          const uint2* q = reinterpret_cast<const uint2*>(xr[t] + c);
+          const uint2 r = EARLY ? __ldcg(q) : __ldg(q);
           xv[t] = make_float4(bf16lo(r.x), bf16hi(r.x), bf16lo(r.y), bf16hi(r.y));
         }
       }
@@ -329,7 +338,7 @@ __global__ void __launch_bounds__(256) router_logits_split_kernel(const T* __res
       if (lane == 0) part[warp][t * RS_EG + g] = v;
     }
   __syncthreads();
-  const int i = threadIdx.x, grp = i / (RT * RS_EG), j = i % (RT * RS_EG), t = t0 + j / RS_EG, e = grp * RS_EG + j % RS_EG;
+  const int i = threadIdx.x, grp = i / (RT * RS_EG), j = i % (RT * RS_EG), t = t0 + j / RS_EG, e = eb + grp * RS_EG + j % RS_EG;
   if (grp < 8 / KW && t < N && e < E) {
     float v = part[grp * KW][j];
 #pragma unroll
@@ -341,6 +350,8 @@ __global__ void __launch_bounds__(256) router_logits_split_kernel(const T* __res
 __global__ void __launch_bounds__(256) router_select_kernel(float* __restrict__ logits, const float* __restrict__ parts, int n_parts, float* __restrict__ topk_w,
                                                             void* __restrict__ topk_i, int N, int E, int k, RouterSelect sel) {
   extern __shared__ float zsm[];                             // per warp: [E] scores, [E] choice scores, [groups] group bests
+  if (N < 256) pdl_launch_dependents();
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tok = blockIdx.x * 8 + warp;
   if (tok >= N) return;
@@ -353,11 +364,11 @@ __global__ void __launch_bounds__(256) router_select_kernel(float* __restrict__ 
   for (int c0 = lane; c0 < E; c0 += 128) {                    // four experts a lane: the loads of all parts in flight together
     float v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = c0 + 32 * u < E ? logits[(size_t)tok * E + c0 + 32 * u] : 0.f;
+    for (int u = 0; u < 4; ++u) v[u] = c0 + 32 * u < E ? __ldcg(logits + (size_t)tok * E + c0 + 32 * u) : 0.f;
 #pragma unroll 8
     for (int z = 0; z < n_parts; ++z)
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] += c0 + 32 * u < E ? __ldg(parts + ((size_t)z * N + tok) * E + c0 + 32 * u) : 0.f;
+      for (int u = 0; u < 4; ++u) v[u] += c0 + 32 * u < E ? __ldcg(parts + ((size_t)z * N + tok) * E + c0 + 32 * u) : 0.f;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int e = c0 + 32 * u;
@@ -462,19 +473,28 @@ void router_topk_launch(const void* x, const float* w, float* logits, float* par
   if (kparts > 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
     n_parts = kparts - 1;
     router_logits_tc_launch(x, w, logits, parts, N, W, E, kparts, st);
-  } else if (E <= 16 && W % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
-    // tokens per block: one for a few tokens; then four, and eight (half the weight reads) once four would give every SM eight blocks
+  } else if ((E <= 16 || (N < 256 && (long long)N * E <= 26000)) && W % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
+    // tokens per block: one for a few tokens; then four, and eight (half the weight reads) once four would give every SM eight blocks.  Eight warps per four experts
+    // as long as that takes no more than two blocks per SM
+    const bool early = N < 256;
     const int srt = few ? 1 : N <= 4 * 8 * kNumSMs ? 4 : 8;
-    auto split = [&](auto kernel, auto xp) { kernel<<<(N + srt - 1) / srt, 256, 0, st>>>(xp, w, logits, N, W, E); };
-    auto by_rows = [&](auto xp, auto kw) {
-      using X = std::remove_cv_t<std::remove_pointer_t<decltype(xp)>>;
-      constexpr int KW = decltype(kw)::value;
-      if (srt == 1) split(router_logits_split_kernel<X, 1, KW>, xp);
-      else if (srt == 4) split(router_logits_split_kernel<X, 4, KW>, xp);
-      else split(router_logits_split_kernel<X, 8, KW>, xp);
+    const long long blocks = (N + srt - 1) / srt;
+    auto split = [&](auto kernel, int kw, auto xp) {
+      const dim3 grid((unsigned)blocks, (E + 8 / kw * RS_EG - 1) / (8 / kw * RS_EG));
+      if (early) launch_pdl(kernel, grid, dim3(256), 0, st, xp, w, logits, N, W, E);
+      else kernel<<<grid, 256, 0, st>>>(xp, w, logits, N, W, E);
     };
     auto by_experts = [&](auto xp) {
-      if (E <= 8) by_rows(xp, std::integral_constant<int, 4>()); else by_rows(xp, std::integral_constant<int, 2>());
+      using X = std::remove_cv_t<std::remove_pointer_t<decltype(xp)>>;
+      if (early) {
+        const bool wide = blocks * ((E + RS_EG - 1) / RS_EG) <= 2 * kNumSMs;
+        if (few) wide ? split(router_logits_split_kernel<X, 1, 8, true>, 8, xp) : split(router_logits_split_kernel<X, 1, 4, true>, 4, xp);
+        else wide ? split(router_logits_split_kernel<X, 4, 8, true>, 8, xp) : split(router_logits_split_kernel<X, 4, 4, true>, 4, xp);
+      } else if (E <= 8) {
+        srt == 4 ? split(router_logits_split_kernel<X, 4, 4, false>, 4, xp) : split(router_logits_split_kernel<X, 8, 4, false>, 4, xp);
+      } else {
+        srt == 4 ? split(router_logits_split_kernel<X, 4, 2, false>, 2, xp) : split(router_logits_split_kernel<X, 8, 2, false>, 2, xp);
+      }
     };
     if (lp) by_experts((const __nv_bfloat16*)x); else by_experts((const float*)x);
   } else if (lp) {
@@ -484,7 +504,7 @@ void router_topk_launch(const void* x, const float* w, float* logits, float* par
   }
   const size_t sel_smem = sizeof(float) * 8 * (size_t)(2 * E + (sel.groups > 1 ? sel.groups : 0));
   if (sel_smem > 48 * 1024) cudaFuncSetAttribute(router_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem);
-  router_select_kernel<<<(N + 7) / 8, 256, sel_smem, st>>>(logits, parts, n_parts, topk_w, topk_i, N, E, k, sel);
+  launch_pdl(router_select_kernel, dim3((N + 7) / 8), dim3(256), sel_smem, st, logits, parts, n_parts, topk_w, topk_i, N, E, k, sel);
 }
 
 void moe_plain_gather_launch(const void* x, const int* row_entry, const int* tile_expert, void* xp, int R, int H, int k, bool lp, cudaStream_t st) {

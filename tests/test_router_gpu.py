@@ -49,3 +49,22 @@ def test_module_ids_keep_their_type():
     x = torch.randn(5, 256, device="cuda", dtype=torch.bfloat16)
     assert r(x)[2].dtype == torch.int64 and ops.router_topk(x, r.linear_router.weight, 2)[2].dtype == torch.int64
     assert ops.router_topk(x, r.linear_router.weight, 2, "sigmoid")[2].dtype == torch.int32
+
+
+@pytest.mark.parametrize("N", [1, 5, 32, 33, 100, 203, 204, 255, 256])
+@pytest.mark.parametrize("E,W,k", [(5, 64, 2), (8, 4096, 2), (16, 516, 4), (17, 128, 4), (128, 2048, 8), (127, 260, 8), (512, 1024, 8)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_split_columns(N, E, W, k, dtype):
+    """Experts over the grid's second dimension, four and eight warps per four of them, ragged counts on both; rows that the kernel in front is still writing."""
+    base = torch.randn(N, W, device="cuda", dtype=dtype)
+    w = torch.randn(E, W, device="cuda") / W ** 0.5
+    for i in range(3):
+        x = base * (i + 1)                              # a kernel of the same stream
+        logits, tw, ti = ops.router_topk(x, w, k)
+        want = x.double() @ w.double().t()
+        # fp32 sums of W products with independent rounding errors
+        assert ((logits.double() - want).norm() / want.norm()).item() < 2e-6
+        p = torch.softmax(logits.double(), -1)
+        top = p.gather(1, ti.long())
+        assert torch.allclose(top.sort(-1, descending=True).values, p.topk(k, -1).values, rtol=1e-5)
+        assert torch.allclose(tw.double(), top / top.sum(-1, keepdim=True), rtol=1e-5)
