@@ -73,6 +73,8 @@ void rmsnorm_launch(const void* x, const void* res_in, const void* w, void* y, v
                     float offset, cudaStream_t stream,
                     unsigned* clear = nullptr, int n_clear = 0);
 
+void rope_rows_launch(const void* pos, bool wide, const float* cos_table, const float* sin_table, float* cos_out, float* sin_out, int rows, int half, int table, cudaStream_t stream);
+void cache_lines_launch(const void* ids, bool wide, void* lines, long long n, long long n_lines, cudaStream_t stream);
 void rope_kv_append_launch(const void* qkv, const float* cos, const float* sin, void* q_out, void* k_cache, void* v_cache,
                            const int* lines, const int* positions, const void* q_norm, const void* k_norm, float eps, int B,
                            int T, int nq, int nkv, int D, int L, int S, cudaStream_t stream, void* k_out = nullptr, void* v_out = nullptr);

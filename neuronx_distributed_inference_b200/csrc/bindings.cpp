@@ -561,6 +561,31 @@ at::Tensor symm_as_tensor(int64_t ptr, int64_t nbytes, int64_t device) {
 }
 
 // ---- rope / cache appends -------------------------------------------------------------------------------------
+// cos / sin [.., half] of positions [..] (int32 or int64), clamped to the tables [length, half]
+std::tuple<at::Tensor, at::Tensor> rope_rows(const at::Tensor& positions, const at::Tensor& cos_table, const at::Tensor& sin_table) {
+  TORCH_CHECK(is_ids(positions) && positions.is_cuda() && cos_table.is_cuda() && cos_table.dim() == 2 && cos_table.scalar_type() == at::kFloat && cos_table.is_contiguous() &&
+              sin_table.sizes() == cos_table.sizes() && sin_table.scalar_type() == at::kFloat && sin_table.is_contiguous() && cos_table.size(0) > 0 &&
+              cos_table.size(0) <= std::numeric_limits<int>::max() && positions.numel() <= std::numeric_limits<int>::max());
+  c10::cuda::CUDAGuard guard(positions.device());
+  const auto pos = positions.contiguous();
+  auto shape = positions.sizes().vec();
+  shape.push_back(cos_table.size(1));
+  auto c = at::empty(shape, cos_table.options()), s = at::empty(shape, cos_table.options());
+  if (c.numel() > 0)
+    rope_rows_launch(pos.data_ptr(), pos.scalar_type() == at::kLong, cos_table.data_ptr<float>(), sin_table.data_ptr<float>(), c.data_ptr<float>(), s.data_ptr<float>(),
+                     (int)pos.numel(), (int)cos_table.size(1), (int)cos_table.size(0), cur_stream());
+  return {c, s};
+}
+// ids (int32 or int64) with those outside 0 .. n_lines - 1 replaced by n_lines
+at::Tensor cache_lines(const at::Tensor& ids, int64_t n_lines) {
+  TORCH_CHECK(is_ids(ids) && ids.is_cuda() && n_lines >= 0 && n_lines <= std::numeric_limits<int>::max());
+  c10::cuda::CUDAGuard guard(ids.device());
+  const auto in = ids.contiguous();
+  auto lines = at::empty(in.sizes(), in.options());
+  if (in.numel() > 0) cache_lines_launch(in.data_ptr(), in.scalar_type() == at::kLong, lines.data_ptr(), in.numel(), n_lines, cur_stream());
+  return lines;
+}
+
 at::Tensor rope_kv_append(const at::Tensor& qkv, const at::Tensor& cos, const at::Tensor& sin, at::Tensor& k_cache,
                           at::Tensor& v_cache, const at::Tensor& lines, const at::Tensor& positions, int64_t nq, int64_t nkv,
                           int64_t D, const c10::optional<at::Tensor>& q_norm, const c10::optional<at::Tensor>& k_norm,
@@ -1022,6 +1047,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("symm_close", &nxdi::symm_close);
   m.def("symm_free", &nxdi::symm_free);
   m.def("symm_as_tensor", &nxdi::symm_as_tensor);
+  m.def("rope_rows", &nxdi::rope_rows);
+  m.def("cache_lines", &nxdi::cache_lines);
   m.def("rope_kv_append", &nxdi::rope_kv_append);
   m.def("rope_kv_split_append", &nxdi::rope_kv_split_append);
   m.def("kv_append", &nxdi::kv_append);

@@ -2,6 +2,8 @@
 // output, plus stand-alone contiguous / paged cache appends.
 // reference kernels: K10 write_kv_cache_at_batch_kernel (kvcache/utils.py:17-67, OOB-skip semantics),
 // the RoPE/QK-norm stages of K2/K3 (attention_base.py:1186-1381, gqa.py:566-631).
+#include <algorithm>
+
 #include "api.h"
 #include "common.cuh"
 
@@ -127,6 +129,41 @@ void paged_kv_append_launch(const void* k_new, const void* v_new, void* k_cache,
   launch_pdl(paged_kv_append_kernel, dim3((total + 255) / 256), dim3(256), 0, stream, reinterpret_cast<const uint4*>(k_new),
              reinterpret_cast<const uint4*>(v_new), reinterpret_cast<uint4*>(k_cache), reinterpret_cast<uint4*>(v_cache), slots,
              HDV, n_slots, total);
+}
+
+// cos / sin rows of positions, clamped to the table, and cache lines of sequence ids, where an unknown id takes line n_lines: what a decode step does once in front of
+// its first attention.  As nine elementwise kernels of the library (casts, comparisons, gathers) they took 17 us of the step, with nothing else running; bound by two launches,
+// 3 us.  No early launch of the kernel behind: the decode attention reads what these write before it waits for the kernel in front of it.  POS: int or long long
+template <typename POS>
+__global__ void __launch_bounds__(256) rope_rows_kernel(const POS* __restrict__ pos, const float* __restrict__ cos_table, const float* __restrict__ sin_table,
+                                                        float* __restrict__ cos_out, float* __restrict__ sin_out, int rows, int half, int table) {
+  pdl_wait();
+  const long long total = (long long)rows * half;
+  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
+    const long long p = __ldcg(pos + i / half);
+    const long long at = (p < 0 ? 0 : p >= table ? table - 1 : p) * half + i % half;
+    cos_out[i] = __ldg(cos_table + at);
+    sin_out[i] = __ldg(sin_table + at);
+  }
+}
+template <typename ID>
+__global__ void __launch_bounds__(256) cache_lines_kernel(const ID* __restrict__ ids, ID* __restrict__ lines, long long n, long long n_lines) {
+  pdl_wait();
+  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+    const ID id = __ldcg(ids + i);
+    lines[i] = id < 0 || id >= n_lines ? (ID)n_lines : id;
+  }
+}
+static unsigned rows_grid(long long n) { return (unsigned)std::min<long long>((n + 255) / 256, 8 * kNumSMs); }
+void rope_rows_launch(const void* pos, bool wide, const float* cos_table, const float* sin_table, float* cos_out, float* sin_out, int rows, int half, int table, cudaStream_t stream) {
+  const dim3 grid(rows_grid((long long)rows * half));
+  if (wide) launch_pdl(rope_rows_kernel<long long>, grid, dim3(256), 0, stream, static_cast<const long long*>(pos), cos_table, sin_table, cos_out, sin_out, rows, half, table);
+  else launch_pdl(rope_rows_kernel<int>, grid, dim3(256), 0, stream, static_cast<const int*>(pos), cos_table, sin_table, cos_out, sin_out, rows, half, table);
+}
+void cache_lines_launch(const void* ids, bool wide, void* lines, long long n, long long n_lines, cudaStream_t stream) {
+  const dim3 grid(rows_grid(n));
+  if (wide) launch_pdl(cache_lines_kernel<long long>, grid, dim3(256), 0, stream, static_cast<const long long*>(ids), static_cast<long long*>(lines), n, n_lines);
+  else launch_pdl(cache_lines_kernel<int>, grid, dim3(256), 0, stream, static_cast<const int*>(ids), static_cast<int*>(lines), n, n_lines);
 }
 
 }  // namespace nxdi

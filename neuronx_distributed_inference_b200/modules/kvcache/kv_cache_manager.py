@@ -77,8 +77,7 @@ class KVCacheManager(nn.Module):
         """Map seq_ids to cache lines; negative / out-of-range ids go to the garbage line (or are
         skipped by the kernels when there is none)."""
         if self.garbage:
-            bad = (seq_ids < 0) | (seq_ids >= self.num_lines)
-            return torch.where(bad, torch.full_like(seq_ids, self.num_lines), seq_ids)
+            return ops.cache_lines(seq_ids, self.num_lines)
         return seq_ids
 
     def update(self, layer: int, k_new, v_new, seq_ids, positions, lines=None):

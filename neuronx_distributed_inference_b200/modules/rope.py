@@ -12,6 +12,8 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
+from .. import ops
+
 
 def _yarn_find_dim(num_rot, dim, base, max_pos):
     return (dim * math.log(max_pos / (num_rot * 2 * math.pi))) / (2 * math.log(base))
@@ -99,8 +101,7 @@ class RotaryEmbedding(nn.Module):
         need = self.max_position_embeddings
         if self._table_len < need or self.cos_table.device != position_ids.device:
             self.build_tables(need, position_ids.device)
-        p = position_ids.long().clamp(0, self._table_len - 1)
-        return self.cos_table[p], self.sin_table[p]
+        return ops.rope_rows(position_ids, self.cos_table, self.sin_table)
 
 
 class MRotaryEmbedding(RotaryEmbedding):

@@ -175,6 +175,23 @@ def apply_rope(x, cos, sin, interleaved: bool = False):
     return ref.apply_rope(x, cos, sin, interleaved)
 
 
+def rope_rows(positions, cos_table, sin_table):
+    """cos / sin rows of ``positions`` (any shape), clamped to the tables ``[length, rot_dim / 2]``."""
+    if positions.dtype in (torch.int32, torch.int64) and cos_table.dtype == torch.float32 and cos_table.is_cuda and cos_table.is_contiguous() and _use_cuda(positions):
+        stats["rope_rows"] += 1
+        return _C().rope_rows(positions, cos_table, sin_table)
+    p = positions.long().clamp(0, cos_table.shape[0] - 1)
+    return cos_table[p], sin_table[p]
+
+
+def cache_lines(ids, n_lines: int):
+    """Cache lines of sequence ids: ids that are none of ``0 .. n_lines - 1`` take line ``n_lines``."""
+    if ids.dtype in (torch.int32, torch.int64) and _use_cuda(ids):
+        stats["cache_lines"] += 1
+        return _C().cache_lines(ids, int(n_lines))
+    return torch.where((ids < 0) | (ids >= n_lines), torch.full_like(ids, n_lines), ids)
+
+
 def rope_kv_append(qkv, cos, sin, k_cache, v_cache, seq_ids, positions, n_q, n_kv, head_dim,
                    interleaved: bool = False, q_norm=None, k_norm=None, norm_eps: float = 1e-6):
     """Split fused qkv [B,T,(n_q+2n_kv)*D], optional per-head q/k RMSNorm (Qwen3), RoPE on q,k,

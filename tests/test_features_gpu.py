@@ -271,3 +271,19 @@ def test_odd_head_dims_run_on_padded_kernels(head_dim, heads, kv, monkeypatch):
     assert ops.stats["rope_attn_decode"] > n0
     rel = ((l1 - l0).norm() / l0.norm()).item()
     assert rel < 3e-2, rel
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+@pytest.mark.parametrize("shape,half", [((1, 1), 64), ((2, 1), 32), ((3, 17), 5), ((3, 2, 300), 48), ((2, 4096), 64), ((0, 1), 8)])
+def test_rope_rows_and_cache_lines(dtype, shape, half):
+    from neuronx_distributed_inference_b200 import ops
+    cos, sin = torch.randn(500, half, device="cuda"), torch.randn(500, half, device="cuda")
+    pos = torch.randint(-20, 600, shape, device="cuda", dtype=dtype)
+    wide = torch.randint(-20, 600, (*shape[:-1], shape[-1] + 3), device="cuda", dtype=dtype)[..., 1:-2]           # strided
+    for p in (pos, wide, pos[..., :1].expand(shape)):
+        want = p.long().clamp(0, 499)
+        c, s = ops.rope_rows(p, cos, sin)
+        assert torch.equal(c, cos[want]) and torch.equal(s, sin[want])
+        lines = ops.cache_lines(p, 37)
+        assert lines.dtype == dtype and torch.equal(lines, torch.where((p < 0) | (p >= 37), torch.full_like(p, 37), p))
