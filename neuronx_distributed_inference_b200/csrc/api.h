@@ -117,7 +117,7 @@ void gemm_pair_launch(const void* a, long long lda, const void* b, const void* b
                       float limit = 7.f, float alpha = 1.702f);
 
 // few tokens x large weights with the weights streamed evenly over the SMs (skinny_gemm.cu): one weight [rows, K], or the experts that have tokens
-constexpr int SKINNY_MAX_T = 128;
+constexpr int SKINNY_MAX_T = 128, SKINNY8_MAX_T = 512;      // tokens of a tile; of 8-bit weights without a gate product
 struct SkinnyGemm {
   const void* x;              // [x_rows, K] bf16, row stride ldx
   long long x_rows, ldx;
@@ -141,6 +141,7 @@ int skinny_gemm_rows(int tokens);          // `tokens` rounded up to what a segm
 long long skinny_gemm_ws_floats(int tokens, bool glu);
 int skinny_gemm_tickets();
 bool skinny_gemm8_supported(int tokens, int K, bool glu);
+int skinny_gemm8_block(int tokens);        // tokens of a token tile there (before skinny_gemm_rows)
 void skinny_clear_launch(unsigned* tickets, int n, cudaStream_t stream);
 void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream);
 // id_step: 1, or 2 when topk_i points at int64 ids (their low words are read)

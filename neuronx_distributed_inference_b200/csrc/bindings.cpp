@@ -144,7 +144,7 @@ static void run_skinny(at::Tensor x, const at::Tensor& w, const c10::optional<at
                        at::Tensor& y, bool fresh_weight, const c10::optional<at::Tensor>& norm_w = c10::nullopt, double eps = 0., double offset = 0.,
                        const at::Tensor* scale = nullptr) {
   const int M = x.size(0);
-  const int64_t nt = skinny_gemm_tickets(), nf = skinny_gemm_ws_floats(M, act != 0);
+  const int64_t nt = skinny_gemm_tickets(), nf = skinny_gemm_ws_floats(scale != nullptr ? skinny_gemm8_block(M) : M, act != 0);
   auto ws = at::empty({nf + nt}, x.options().dtype(at::kFloat));              // one per call: safe on any stream and inside captured graphs
   SkinnyGemm a{};
   a.ws = ws.data_ptr<float>();
@@ -268,9 +268,10 @@ at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
 
 at::Tensor dequant_bf16(const at::Tensor& w, const at::Tensor& scale);
 
-// int8 / fp8 weights and 9 .. 128 tokens (64 with a gate product): the bytes are read once.  us, here / expanded to bf16 in memory first: 4096 x 4096 at 9 tokens 11 / 25,
-// at 128 24 / 33; 4096 x 11008 at 9 17 / 48, at 37 20 / 52, at 128 30 / 58; 11008 x 4096 at 47 20 / 51; 12288 x 4096 at 64 23 / 58, at 100 28 / 60.  The weight is not
-// rounded: the scale is applied to the fp32 sum.
+// int8 / fp8 weights and 9 .. 512 tokens (64 with a gate product): the bytes are read once, by blocks of up to 128 tokens at the same time.  us, here / expanded to bf16
+// in memory first: 4096 x 4096 at 9 tokens 11 / 25, at 128 24 / 33, at 256 25 / 34, at 512 32 / 37; 4096 x 11008 at 9 17 / 48, at 37 20 / 52, at 128 30 / 58, at 256
+// 37 / 73, at 512 57 / 88; 11008 x 4096 at 47 20 / 51; 12288 x 4096 at 64 23 / 58, at 256 41 / 57, at 384 51 / 77, at 512 64 / 78.  The weight is not rounded: the
+// scale is applied to the fp32 sum.
 static at::Tensor linear8_few(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int64_t act, const at::Tensor& scale,
                               const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& norm_w, double eps, double offset) {
   const int64_t M = x.size(0), N = w.size(0), n_out = act != 0 ? N / 2 : N;
@@ -296,7 +297,7 @@ std::tuple<c10::optional<at::Tensor>, int64_t> linear(const at::Tensor& x, const
   const bool plain = is_bf16(w) && !scale.has_value();
   if (!is_bf16(x) || x.dim() < 1 || x.size(-1) == 0 || w.dim() != 2 || !w.is_contiguous() || !(plain || (wq && scale.has_value() && scale->dim() == 1))) return none;
   const int64_t K = x.size(-1), T = x.numel() / K, N = w.size(0), n_out = act != 0 ? N / 2 : N;
-  const bool few = T <= GEMV_MAX_T, few8 = wq && !out.has_value() && skinny_gemm8_supported((int)std::min<int64_t>(T, SKINNY_MAX_T + 1), (int)K, act != 0);
+  const bool few = T <= GEMV_MAX_T, few8 = wq && !out.has_value() && skinny_gemm8_supported((int)std::min<int64_t>(T, SKINNY8_MAX_T + 1), (int)K, act != 0);
   int64_t ran = 0;
   if (few && wq && K % 16 == 0) ran = LINEAR_QGEMV;
   else if (few && plain && K % 64 == 0 && (K % 256 == 0 || gemv2_supported((int)T, (int)K, 0))) ran = LINEAR_GEMV;

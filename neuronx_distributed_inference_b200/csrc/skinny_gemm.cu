@@ -174,7 +174,9 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
   if (!early) pdl_wait();
 
   const int n_tiles = (p.n_out + SK_BM - 1) / SK_BM, nkb = p.K / BK;
-  const long long total = (long long)(grouped ? *p.n_active : 1) * n_tiles * nkb;
+  // 8-bit weights: more tokens than a token tile holds are blocks of xb rows, which share the weights in L2
+  const int n_seg = grouped ? *p.n_active : WT ? (p.T + p.xb - 1) / p.xb : 1;
+  const long long total = (long long)n_seg * n_tiles * nkb;
   const long long G = max(1ll, min((long long)gridDim.x, total / 4));                // at least four k-blocks per CTA that works
   const long long u0 = blockIdx.x < G ? total * blockIdx.x / G : 0, u1 = blockIdx.x < G ? total * (blockIdx.x + 1) / G : 0;
   const int acc_cols = NW * p.xb;
@@ -188,7 +190,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
       for (long long u = u0; u < u1 && go;) {
         const int tile = (int)(u / nkb), kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u));
         const int ei = tile / n_tiles, n0 = (tile % n_tiles) * SK_BM, e = grouped ? p.active[ei] : 0;
-        const int row_w = e * p.rows + n0, row_x = grouped ? p.seg_start[ei] : 0;
+        const int row_w = e * p.rows + n0, row_x = grouped ? p.seg_start[ei] : ei * p.xb;
         // a segment's rows in boxes of 64 as far as they go, the rest in one more (where it fits) or in up to two of 16: each copy costs the issuing thread 0.25 us
         int boxes = 1, big = 0;
         const int box_bytes = p.xbox * SK_BK * 2;
@@ -214,7 +216,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
             mbar_expect(&full_bar[s], boxes * box_bytes * XBOX + big * (64 * SK_BK * 2));
             uint8_t* xs = st + NW * W_BYTES;
             if (XBOX == 2) {
-              sk_tma3(xs, &p.tm_x, 0, kb * 2, &full_bar[s]);
+              sk_tma3(xs, &p.tm_x, row_x, kb * 2, &full_bar[s]);
             } else {
               for (int q = 0; q < big; ++q) sk_tma(xs + q * (64 * SK_BK * 2), &p.tm_x64, kb * BK, row_x + q * 64, &full_bar[s]);
               for (int q = 0; q < boxes; ++q) sk_tma(xs + big * (64 * SK_BK * 2) + q * box_bytes, &p.tm_x, kb * BK, row_x + big * 64 + q * p.xbox, &full_bar[s]);
@@ -344,7 +346,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
       const int tile = (int)(u / nkb), kb0 = (int)(u % nkb), kb1 = (int)min((long long)nkb, kb0 + (u1 - u)), buf = seg & 1;
       u += kb1 - kb0;
       const int ei = tile / n_tiles, n = (tile % n_tiles) * SK_BM + n_in, e = grouped ? p.active[ei] : 0;
-      const int row0 = grouped ? p.seg_start[ei] : 0, cnt = grouped ? p.seg_count[ei] : p.T;
+      const int row0 = grouped ? p.seg_start[ei] : ei * p.xb, cnt = grouped ? p.seg_count[ei] : WT ? min(p.xb, p.T - row0) : p.T;
       const float bg = (p.bias && n < p.n_out) ? __bfloat162float(p.bias[(size_t)e * p.rows + n]) : 0.f;
       const float bu = (GLU && p.bias && n < p.n_out) ? __bfloat162float(p.bias[(size_t)e * p.rows + p.n_out + n]) : 0.f;
       const float sg = WT && n < p.n_out ? __ldcg(p.scale + (size_t)n * p.scale_step) : 1.f, su = WT && GLU && n < p.n_out ? __ldcg(p.scale + (size_t)(p.n_out + n) * p.scale_step) : 1.f;
@@ -542,16 +544,17 @@ __global__ void __launch_bounds__(256) skinny_clear_kernel(unsigned* __restrict_
 }
 void skinny_clear_launch(unsigned* tickets, int n, cudaStream_t stream) { launch_pdl(skinny_clear_kernel, dim3(1), dim3(256), 0, stream, tickets, n); }
 
-bool skinny_gemm8_supported(int tokens, int K, bool glu) { return tokens >= 1 && tokens <= (glu ? SKINNY_MAX_T / 2 : SKINNY_MAX_T) && K % sk_bk(1, false) == 0; }
+bool skinny_gemm8_supported(int tokens, int K, bool glu) { return tokens >= 1 && tokens <= (glu ? SKINNY_MAX_T / 2 : SKINNY8_MAX_T) && K % sk_bk(1, false) == 0; }
+int skinny_gemm8_block(int tokens) { return (tokens + (tokens + SKINNY_MAX_T - 1) / SKINNY_MAX_T - 1) / ((tokens + SKINNY_MAX_T - 1) / SKINNY_MAX_T); }
 
 void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream) {
   const bool glu = a.act != 0;
-  if (a.K % SK_BK != 0 || a.tokens < 1 || a.tokens > SKINNY_MAX_T) throw std::runtime_error("skinny gemm: K % 64 == 0, 1 .. 128 tokens per expert");
+  if (a.K % SK_BK != 0 || a.tokens < 1 || (a.wt == 0 && a.tokens > SKINNY_MAX_T)) throw std::runtime_error("skinny gemm: K % 64 == 0, 1 .. 128 tokens per expert");
   if (a.wt != 0 && (!skinny_gemm8_supported(a.tokens, a.K, glu) || a.n_active != nullptr || a.scale == nullptr))
-    throw std::runtime_error("skinny gemm, 8-bit weights: one weight with scales, K % 128 == 0, 1 .. 128 tokens (64 with a gate product)");
+    throw std::runtime_error("skinny gemm, 8-bit weights: one weight with scales, K % 128 == 0, 1 .. 512 tokens (64 with a gate product)");
   SkinnyKernelParams p{};
   p.rows = glu ? 2 * a.n_out : a.n_out;
-  p.xb = skinny_gemm_rows(a.tokens);
+  p.xb = skinny_gemm_rows(a.wt ? skinny_gemm8_block(a.tokens) : a.tokens);
   const bool wide = a.wt == 0 && !glu && a.n_active == nullptr && a.K % 128 == 0;
   sk_map(&p.tm_w, a.w, (long long)a.experts * p.rows, a.K, a.K, SK_BM, a.wt != 0, wide ? 2 : 1);
   p.xbox = a.n_active ? 16 : p.xb;

@@ -1,4 +1,4 @@
-"""int8 / fp8 weights of 9 .. 128 tokens (csrc/skinny_gemm.cu): the bytes are expanded on their way to the tensor cores.
+"""int8 / fp8 weights of 9 .. 512 tokens (csrc/skinny_gemm.cu): the bytes are expanded on their way to the tensor cores.
 
 Bound: rows are bf16, products and sums fp32, the scale is applied to the sum: results are rounded to bf16 once (2^-9 at most, 1.7e-3 rms)."""
 import pytest
@@ -21,7 +21,7 @@ def _want(x, q, s, bias=None, act=None):
 
 
 @pytest.mark.parametrize("wdtype", TYPES)
-@pytest.mark.parametrize("T", [9, 16, 17, 37, 64, 65, 100, 128])
+@pytest.mark.parametrize("T", [9, 16, 17, 37, 64, 65, 100, 128, 129, 250, 257, 512])
 @pytest.mark.parametrize("N,K", [(8, 128), (136, 256), (4104, 384), (1000, 4096), (256, 14336), (20000, 128)])
 def test_plain(wdtype, T, N, K):
     q, s = ref.quantize_per_channel(torch.randn(N, K, device=DEV) * 0.02, wdtype)
