@@ -185,6 +185,13 @@ at::Tensor gemv(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
       run_gemv(p, 0, x.device());
       return y;
     }
+    // rows too wide for its shared memory (from 8 tokens of 11008, 7 of 14336): bytes expanded on the way to the tensor cores.  us in a graph, fp8 / one warp per
+    // few weight rows: 4096 x 11008 at 8 tokens 16.6 / 98, 4096 x 14336 at 7 19.3 / 112, 1024 x 16384 at 6 12.3 / 59, 256 x 28672 at 4 14.1 / 64; int8 alike.  Both
+    // keep products and sums in fp32 (errors against 64 bits are the same).  A norm stays with the warps, which scale the fp32 sums by 1 / rms instead of the rows.
+    if (q2 && !norm_w.has_value() && x.stride(0) % 8 == 0 && y.size(1) % 8 == 0 && (!glu || N % 2 == 0) && skinny_gemm8_supported((int)x.size(0), (int)x.size(1), glu)) {
+      run_skinny(x.contiguous(), w, bias, (int)act, residual, y, false, c10::nullopt, 0., 0., &*scale);
+      return y;
+    }
     static int n_sms = 0;
     if (n_sms == 0) n_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
     qgemv_launch(x.data_ptr(), w.data_ptr(), scale->data_ptr<float>(), (int)scale->numel(), optr(bias), optr(norm_w), optr(residual),

@@ -1,5 +1,7 @@
 // Weight-only quantised skinny GEMM for decode:  Y[T<=8, N] = epi( norm(X)[T,K] . dequant(Wq[N,K])^T )
 //   Wq: int8 or fp8-e4m3 (one byte per weight), scale: fp32 per output channel ([N]) or per tensor ([1]).
+// Runs what the streaming kernel (gemv2.cu) and the tensor cores (skinny_gemm.cu) do not take: K that is no multiple of 128, rows too wide for shared memory with a
+// norm or with an output width that is no multiple of 8.
 // Decode is bound by weight bytes; 8-bit weights halve them, but only if nothing materialises a bf16 copy — the torch
 // fallback dequantises the whole matrix (1 + 2 + 2 bytes of traffic per weight).  Here the bytes go HBM -> registers once:
 //   * warp-per-row-group: a warp owns R consecutive output rows and accumulates T x R fp32 sums; lanes stride K with

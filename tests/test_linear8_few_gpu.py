@@ -1,4 +1,4 @@
-"""int8 / fp8 weights of 9 .. 512 tokens (csrc/skinny_gemm.cu): the bytes are expanded on their way to the tensor cores.
+"""int8 / fp8 weights of 9 .. 512 tokens, and of fewer with rows too wide for the GEMV (csrc/skinny_gemm.cu): the bytes are expanded on their way to the tensor cores.
 
 Bound: rows are bf16, products and sums fp32, the scale is applied to the sum: results are rounded to bf16 once (2^-9 at most, 1.7e-3 rms)."""
 import pytest
@@ -62,3 +62,21 @@ def test_every_byte(wdtype):
         return
     q = torch.where(torch.isnan(q.float()), torch.zeros_like(q.float()), q.float()).to(wdtype)
     assert torch.equal(ops.linear(x, q, scale=torch.ones(256, device=DEV)).float(), torch.stack([q[:, 17 * t % K].float() for t in range(16)]))
+
+
+@pytest.mark.parametrize("wdtype", TYPES)
+@pytest.mark.parametrize("T,N,K", [(8, 4096, 11008), (7, 256, 14336), (8, 1000, 10624), (3, 136, 32768), (1, 8, 110592), (8, 1001, 11008)])
+def test_rows_too_wide_for_the_gemv(wdtype, T, N, K):
+    """1 .. 8 rows that do not fit one SM's shared memory; 1001 weight rows and a norm stay with the warp-per-row kernel."""
+    q, s = ref.quantize_per_channel(torch.randn(N, K, device=DEV) / K ** 0.5, wdtype)
+    x, b = torch.randn(T, K, device=DEV, dtype=BF), torch.randn(N, device=DEV, dtype=BF)
+    r, n = torch.randn(T, N, device=DEV, dtype=BF), torch.randn(K, device=DEV, dtype=BF)
+    wide = torch.randn(T, K + 8, device=DEV, dtype=BF)
+    assert _rel(ops.linear(x, q, scale=s), _want(x, q, s)) < 3e-3
+    assert _rel(ops.linear(wide[:, 8:], q, scale=s), _want(wide[:, 8:], q, s)) < 3e-3
+    assert _rel(ops.linear(x, q, b, scale=s, residual=r), _want(x, q, s, b) + r.double()) < 3e-3
+    assert _rel(ops.linear(x, q, scale=s.view(-1)[:1].contiguous()), _want(x, q, s.view(-1)[:1])) < 3e-3
+    if N % 16 == 0:
+        assert _rel(ops.linear(x, q, b, scale=s, act="silu_mul"), _want(x, q, s, b, "silu_mul")) < 3e-3
+    h = x.double() * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-5) * n.double()
+    assert _rel(ops.linear(x, q, norm_weight=n, norm_eps=1e-5, scale=s), _want(h, q, s)) < 6e-3
