@@ -3,6 +3,8 @@
 // design notes.  A "phase" is one skinny GEMM  Y[T<=8, N] = f(rmsnorm(X)[T,K] · W[N,K]^T)  (+ fused LL all-reduce).
 #pragma once
 #include "api.h"
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace nxdi {
@@ -275,39 +277,55 @@ __device__ __forceinline__ void g2_consume(const G2Phase& p, const G2Symm& sy, c
   if (has_norm || WT != 0) {
     // one in-place pass over x: sum of squares (fused RMSNorm), x gamma, and for the 8-bit weight paths bf16 -> f16
     const float o = p.norm_offset;
+    auto rows = [&](int t, auto count) {
+      constexpr int R = decltype(count)::value;
+      float acc[R];
+      const uint32_t row = xs_u + t * xs_stride + ctid * 16;
 #pragma unroll
-    for (int t = 0; t < GEMV_MAX_T; ++t) {
-      if (t < T) {
-        float acc = 0.f;
+      for (int h = 0; h < R; ++h) acc[h] = 0.f;
 #pragma unroll
-        for (int j = 0; j < G2_MAXV; ++j) {
-          if (j < per_thread) {
-            const uint32_t a = xs_u + t * xs_stride + (ctid + 256 * j) * 16;
-            uint4 w = lds128(a);
-            float f[8] = {bf16lo(w.x), bf16hi(w.x), bf16lo(w.y), bf16hi(w.y), bf16lo(w.z), bf16hi(w.z), bf16lo(w.w), bf16hi(w.w)};
+      for (int j = 0; j < G2_MAXV; ++j) {
+        if (j < per_thread) {
+          const uint32_t a = row + 4096 * j;
+          uint4 w[R];
+#pragma unroll
+          for (int h = 0; h < R; ++h) w[h] = lds128(a + h * xs_stride);
+#pragma unroll
+          for (int h = 0; h < R; ++h) {
+            float f[8] = {bf16lo(w[h].x), bf16hi(w[h].x), bf16lo(w[h].y), bf16hi(w[h].y), bf16lo(w[h].z), bf16hi(w[h].z), bf16lo(w[h].w), bf16hi(w[h].w)};
             if (has_norm) {
               const uint4 gm = gq[j];
               const float gf[8] = {bf16lo(gm.x), bf16hi(gm.x), bf16lo(gm.y), bf16hi(gm.y), bf16lo(gm.z), bf16hi(gm.z), bf16lo(gm.w), bf16hi(gm.w)};
 #pragma unroll
               for (int e = 0; e < 8; ++e) {
-                acc += f[e] * f[e];
+                acc[h] += f[e] * f[e];
                 f[e] *= gf[e] + o;
               }
             }
             if (WT != 0) {
-              w = make_uint4(pack_f16_sat(f[0], f[1]), pack_f16_sat(f[2], f[3]), pack_f16_sat(f[4], f[5]), pack_f16_sat(f[6], f[7]));
+              w[h] = make_uint4(pack_f16_sat(f[0], f[1]), pack_f16_sat(f[2], f[3]), pack_f16_sat(f[4], f[5]), pack_f16_sat(f[6], f[7]));
             } else {
-              w = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+              w[h] = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
             }
-            sts128(a, w);
+            sts128(a + h * xs_stride, w[h]);
           }
         }
-        if (has_norm) {
-          acc = warp_sum(acc);
-          if (lane == 0) sts_f32(rstd_u + (warp * 8 + t) * 4, acc);
-        }
       }
-    }
+      if (has_norm) {
+#pragma unroll
+        for (int h = 0; h < R; ++h) acc[h] = warp_sum(acc[h]);
+#pragma unroll
+        for (int h = 0; h < R; ++h)
+          if (lane == 0) sts_f32(rstd_u + (warp * 8 + t + h) * 4, acc[h]);
+      }
+    };
+    // The pass was unrolled over the tokens: code that no warp had fetched before for each of them, 0.5 to 0.7 us a token whatever K.  A rolled loop runs it from
+    // the instruction cache; two tokens at a time, since one token's is a serial chain.  us in a graph, this / unrolled: with a norm, bf16 6144 x 4096 at 4 tokens
+    // 10.3 / 11.5, at 8 11.7 / 14.4, gate|up 28672 x 4096 at 8 40.3 / 42.8; fp8 4096 x 4096 at 3 6.2 / 7.0, at 8 7.0 / 9.8, 4096 x 11008 at 3 10.6 / 11.1.
+    int t = 0;
+#pragma unroll 1
+    for (; t + 1 < T; t += 2) rows(t, std::integral_constant<int, 2>{});
+    if (t < T) rows(t, std::integral_constant<int, 1>{});
     asm volatile("bar.sync 1, 256;" ::: "memory");
   }
   if (prof && ctid == 0) prof[3] = clock64();

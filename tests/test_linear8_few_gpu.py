@@ -80,3 +80,16 @@ def test_rows_too_wide_for_the_gemv(wdtype, T, N, K):
         assert _rel(ops.linear(x, q, b, scale=s, act="silu_mul"), _want(x, q, s, b, "silu_mul")) < 3e-3
     h = x.double() * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-5) * n.double()
     assert _rel(ops.linear(x, q, norm_weight=n, norm_eps=1e-5, scale=s), _want(h, q, s)) < 6e-3
+
+
+@pytest.mark.parametrize("wdtype", [BF, *TYPES])
+@pytest.mark.parametrize("K", [128, 2048, 4096, 4224])
+@pytest.mark.parametrize("norm", [False, True])
+def test_rows_of_a_step_do_not_depend_on_their_number(wdtype, K, norm):
+    """1 .. 8 rows are normalised and converted in pairs and a rest: each row has the bits that it has alone."""
+    x, w = torch.randn(8, K, device=DEV, dtype=BF), torch.randn(512, K, device=DEV) / K ** 0.5
+    w, s = (w.to(BF), None) if wdtype == BF else ref.quantize_per_channel(w, wdtype)
+    n = torch.randn(K, device=DEV, dtype=BF) if norm else None
+    one = torch.cat([ops.linear(x[t:t + 1], w, norm_weight=n, scale=s) for t in range(8)])
+    for T in range(1, 9):
+        assert torch.equal(ops.linear(x[:T], w, norm_weight=n, scale=s), one[:T])
