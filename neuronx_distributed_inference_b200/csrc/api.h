@@ -153,7 +153,7 @@ void moe_small_combine_launch(const float* y, const float* topk_w, const int* po
 // MoE decode: routed experts for T <= 8 tokens as two batched streaming launches (moe_decode.cu)
 void moe_decode_launch(const void* x, const void* w_gate_up, const void* w_down, const float* topk_w, const int* topk_i, int id_step, void* u,
                        float* y_acc, int T, int topk, int H, int I, int E, int expert_offset, int act /*1 silu*up, 4 clamped gate product*/, float limit,
-                       float alpha, int n_sms, cudaStream_t stream);
+                       float alpha, cudaStream_t stream);
 
 constexpr int ATT_MAX_ORDER = 64;      // rows that a warp orders in two registers a lane
 struct AttnDecodeParams {

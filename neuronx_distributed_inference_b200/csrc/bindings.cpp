@@ -397,11 +397,9 @@ at::Tensor moe_decode(const at::Tensor& x, const at::Tensor& w_gate_up, const at
               topk_i.is_contiguous() && topk_w.numel() == (int64_t)T * k && topk_i.size(0) == T);
   c10::cuda::CUDAGuard guard(x.device());
   auto u = at::empty({(int64_t)T * k, I}, x.options());
-  auto y = at::zeros({T, H}, x.options().dtype(at::kFloat));
-  static int n_sms = 0;
-  if (n_sms == 0) n_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  auto y = at::empty({T, H}, x.options().dtype(at::kFloat));     // cleared by the first kernel
   moe_decode_launch(x.data_ptr(), w_gate_up.data_ptr(), w_down.data_ptr(), topk_w.data_ptr<float>(), id_ptr(topk_i), id_step(topk_i),
-                    u.data_ptr(), y.data_ptr<float>(), T, k, H, I, E, (int)expert_offset, (int)act, (float)limit, (float)alpha, n_sms, cur_stream());
+                    u.data_ptr(), y.data_ptr<float>(), T, k, H, I, E, (int)expert_offset, (int)act, (float)limit, (float)alpha, cur_stream());
   return y.to(x.scalar_type());
 }
 

@@ -424,7 +424,7 @@ def moe_experts(x, w_gate_up, w_down, topk_w, topk_i, act="silu_mul", expert_off
                    and x.shape[1] % 8 == 0 and w_down.shape[2] % 8 == 0 and max(x.shape[1], w_down.shape[2]) * 2 <= 65536)
     # small steps: every expert's weights are streamed once for all its tokens, evenly over the SMs (csrc/skinny_gemm.cu)
     if (_use_cuda(x) and _MOE_GROUPED and x.dtype == torch.bfloat16 and w_gate_up.dtype == x.dtype and w_down.dtype == x.dtype
-            and kact in _MOE_ACTS and (_MOE_ROWS_TOKENS if rows_kernel else 0) < N and topk_i.dim() == 2 and topk_i.shape[1] <= 64
+            and kact in _MOE_ACTS and (_rows_kernel_tokens(w_gate_up) if rows_kernel else 0) < N and topk_i.dim() == 2 and topk_i.shape[1] <= 64
             and (N <= _MOE_SMALL_TOKENS or _few_rows_of_large_experts(N * topk_i.shape[1], w_gate_up))
             and w_gate_up.is_contiguous() and w_down.is_contiguous() and x.shape[1] % 64 == 0 and w_down.shape[2] % 64 == 0
             and w_gate_up.shape[0] <= 512
@@ -463,6 +463,12 @@ _MOE_GROUPED = os.environ.get("NXDI_B200_MOE_GROUPED", "1") == "1"
 # 4096 x 14336: 132 / 139, 222 / 185 and 697 / 386 at 1, 2 and 8.  Against the CTA-pair path at 12, 48 and 128 tokens: 147 / 129, 259 / 210, 271 / 219 and
 # 539 / 436, 568 / 461, 587 / 481; 16 experts, 4 chosen, 6144 x 1344: 254 / 186, 190 / 163, 201 / 175 at 16, 48 and 128
 _MOE_ROWS_TOKENS, _MOE_SMALL_TOKENS = 2, 128
+
+
+def _rows_kernel_tokens(w_gate_up) -> int:
+    """Up to how many tokens a warp per weight row and (token, slot) pair beats reading every chosen expert once (us in a graph, rows / once: 2 tokens of 2 in 8
+    4096 x 14336 218 / 205, 4096 x 7168 119 / 120, 6144 x 4096 100 / 105, 4 in 16 6144 x 1344 79 / 92; 1 token of 4096 x 14336 128 / 137, 6144 x 1344 53 / 68)."""
+    return _MOE_ROWS_TOKENS if w_gate_up.shape[1] * w_gate_up.shape[2] < 1 << 26 else 1
 
 
 def _few_rows_of_large_experts(entries: int, w_gate_up) -> bool:

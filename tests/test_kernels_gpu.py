@@ -525,3 +525,40 @@ def test_fp8_w8a8_gemm_and_rmsnorm_quant(M, N, K, act, per_tensor):
         ops.set_activation_quant(False)
     yr = ref.linear((xq.float() * a_s), wq.float() * (ws if per_tensor else ws[:, None]), b.float(), act=act)
     assert y.shape == yr.shape and _rel(y, yr) < 8e-3, _rel(y, yr)
+
+
+@pytest.mark.parametrize("T", [1, 2])
+@pytest.mark.parametrize("k,E,H,I,off", [(1, 1, 8, 8, 0), (2, 4, 72, 264, 0), (4, 16, 520, 248, 0), (3, 8, 2048, 72, 3), (2, 8, 264, 1032, 8), (4, 4, 4096, 1344, 0)])
+def test_moe_decode_edges(T, k, E, H, I, off):
+    """Ends of a warp's eight loads, of a block's eight units and of the four down rows; pairs of other ranks, all of them too (offset 8 of ids below 8).
+    Bound: u and the result are rounded to bf16 once each (2^-9), sums are fp32."""
+    x = torch.randn(T, H, device=DEV, dtype=torch.bfloat16)
+    gu = (torch.randn(E, 2 * I, H, device=DEV) / H ** 0.5).bfloat16()
+    dn = (torch.randn(E, H, I, device=DEV) / I ** 0.5).bfloat16()
+    w = torch.rand(T, k, device=DEV)
+    ids = torch.stack([torch.randperm(max(E, k), device=DEV)[:k] for _ in range(T)]).to(torch.int32)
+    torch.full((T, H), float("nan"), device=DEV)               # freed: the accumulator is not clean memory
+    y = ops._C().moe_decode(x, gu, dn, w, ids, off, 1, 7.0, 1.702)
+    want = torch.zeros(T, H, device=DEV, dtype=torch.float64)
+    for t in range(T):
+        for j in range(k):
+            e = int(ids[t, j]) - off
+            if 0 <= e < E:
+                g = gu[e].double() @ x[t].double()
+                want[t] += w[t, j].double() * (dn[e].double() @ (torch.nn.functional.silu(g[:I]) * g[I:]))
+    if not (want != 0).any():
+        assert (y == 0).all()
+    else:
+        assert ((y.double() - want).norm() / want.norm()).item() < 6e-3
+
+
+def test_two_tokens_of_the_largest_experts():
+    """From 2^26 gate and up weights on, two tokens read each chosen expert once."""
+    E, H, I = 3, 4096, 8192
+    x = torch.randn(2, H, device=DEV, dtype=torch.bfloat16)
+    gu, dn = (torch.randn(E, 2 * I, H, device=DEV) / 64).bfloat16(), (torch.randn(E, H, I, device=DEV) / 90).bfloat16()
+    ids, w = torch.tensor([[0, 2], [2, 1]], device=DEV), torch.rand(2, 2, device=DEV)
+    before = ops.stats["moe_small"], ops.stats["moe_decode"]
+    two, one = ops.moe_experts(x, gu, dn, w, ids), torch.cat([ops.moe_experts(x[t:t + 1], gu, dn, w[t:t + 1], ids[t:t + 1]) for t in range(2)])
+    assert (ops.stats["moe_small"], ops.stats["moe_decode"]) == (before[0] + 1, before[1] + 2)
+    assert ((two.double() - one.double()).norm() / one.double().norm()).item() < 6e-3        # as above: two roundings to bf16
