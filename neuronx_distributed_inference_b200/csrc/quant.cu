@@ -97,7 +97,7 @@ void rmsnorm_quant_launch(const void* x, const void* gamma, void* q, float* scal
              reinterpret_cast<const __nv_bfloat16*>(gamma), reinterpret_cast<uint8_t*>(q), scale, H, eps, offset, clamp);
 }
 
-// Weight-only 8-bit layers at prefill sizes without activation quantisation: expand W (int8 / fp8-e4m3, per-channel or per-tensor
+// Weight-only 8-bit layers above 512 tokens (64 with a gate product; fewer read the bytes) without activation quantisation: expand W (int8 / fp8-e4m3, per-channel or per-tensor
 // scale) to bf16 ONCE per call into a scratch buffer (1 B read + 2 B written per weight; the copy is consumed from L2 by the
 // tcgen05 GEMM that follows, which therefore waits for it before its first weight tile: `fresh_weight`) instead of the three elementwise passes of the PyTorch composite.
 template <int WT>
