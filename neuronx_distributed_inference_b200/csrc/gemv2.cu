@@ -37,7 +37,7 @@ struct Gemv2Params {
   int max_inflight;
 };
 
-template <bool GLU, int MODE, int WT>
+template <bool GLU, int MODE, int WT, bool WIDE>
 __global__ void __launch_bounds__(G2_THREADS, 1) gemv2_kernel(const __grid_constant__ Gemv2Params pp) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemv2_kernel(const __grid_const
   }
   int stage = 0;
   uint32_t lap = 0, xph = 0;
-  g2_consume<GLU, MODE, WT>(ph, pp.symm, sm, blockIdx.x, tid, stage, lap, xph, [] { pdl_wait(); });
+  g2_consume<GLU, MODE, WT, WIDE>(ph, pp.symm, sm, blockIdx.x, tid, stage, lap, xph, [] { pdl_wait(); });
 }
 
 static int g2_num_sms() {
@@ -158,9 +158,12 @@ int gemv2_pmax(int N, int K, bool glu, int wt) {
   return gemv2_grid(N, K, glu, wt) / n_tiles + 3;
 }
 
-template <bool GLU, int MODE, int WT>
+template <bool GLU, int MODE, int WT, bool WIDE = false>
 static void launch_gemv2(const Gemv2Params& pp, cudaStream_t stream) {
-  auto kern = gemv2_kernel<GLU, MODE, WT>;
+  if constexpr (!WIDE) {
+    if (pp.ph.K > G2_ROUND && (WT != 0 || pp.ph.norm_w != nullptr)) return launch_gemv2<GLU, MODE, WT, true>(pp, stream);
+  }
+  auto kern = gemv2_kernel<GLU, MODE, WT, WIDE>;
   static bool configured = false;
   if (!configured) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_BUDGET);

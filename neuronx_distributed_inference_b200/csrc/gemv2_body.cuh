@@ -210,7 +210,10 @@ __device__ __forceinline__ uint32_t pack_f16_sat(float lo, float hi) {
   return r;
 }
 
-template <bool GLU, int MODE, int WT = 0, class WaitDep>
+constexpr int G2_MAXV = 7, G2_ROUND = 256 * 8 * G2_MAXV;   // 16-byte vectors of a row that a thread normalises or converts in a round; its columns (14336)
+// WIDE: rows of more than G2_ROUND columns that are normalised or converted take several rounds.  A kernel that looks for such rows at run time costs the others
+// 0.1 us (fp8 4096 x 4096 at 3 tokens 6.3, 6.2 without; 6.5 with one loop over all rounds)
+template <bool GLU, int MODE, int WT = 0, bool WIDE = true, class WaitDep>
 __device__ __forceinline__ void g2_consume(const G2Phase& p, const G2Symm& sy, const G2Smem& sm, const int c, const int tid,
                                            int& stage, uint32_t& lap, uint32_t& xph, WaitDep&& wait_dep) {
   const int lane = tid & 31, warp = tid >> 5;
@@ -240,15 +243,15 @@ __device__ __forceinline__ void g2_consume(const G2Phase& p, const G2Symm& sy, c
   const bool has_norm = p.norm_w != nullptr;
   // ---- before the dependency resolves: everything that does not depend on the previous kernel ----
   // gamma -> registers (this thread's vectors ctid, ctid+256, ...); zero the k padding of every x row (K..Kp)
-  constexpr int G2_MAXV = 7;   // K <= 14336
   uint4 gq[G2_MAXV];
   const int per_thread = (nvec - ctid + 255) / 256;   // vectors of this thread
-  if (has_norm) {
-    const uint4* gw = reinterpret_cast<const uint4*>(p.norm_w);
+  auto load_gamma = [&](int first) {
+    const uint4* gw = reinterpret_cast<const uint4*>(p.norm_w) + ctid + 256 * first;
 #pragma unroll
     for (int j = 0; j < G2_MAXV; ++j)
-      if (j < per_thread) gq[j] = ldg_cached(gw + ctid + 256 * j);
-  }
+      if (first + j < per_thread) gq[j] = ldg_cached(gw + 256 * j);
+  };
+  if (has_norm) load_gamma(0);
   if (Kp != K) {
     const int padv = (Kp - K) >> 3;
     for (int i = ctid; i < T * padv; i += 256)
@@ -277,15 +280,15 @@ __device__ __forceinline__ void g2_consume(const G2Phase& p, const G2Symm& sy, c
   if (has_norm || WT != 0) {
     // one in-place pass over x: sum of squares (fused RMSNorm), x gamma, and for the 8-bit weight paths bf16 -> f16
     const float o = p.norm_offset;
-    auto rows = [&](int t, auto count) {
+    auto rows = [&](int t, auto first, auto count) {
       constexpr int R = decltype(count)::value;
       float acc[R];
-      const uint32_t row = xs_u + t * xs_stride + ctid * 16;
+      const uint32_t row = xs_u + t * xs_stride + ctid * 16 + 4096 * first;
 #pragma unroll
       for (int h = 0; h < R; ++h) acc[h] = 0.f;
 #pragma unroll
       for (int j = 0; j < G2_MAXV; ++j) {
-        if (j < per_thread) {
+        if (first + j < per_thread) {
           const uint32_t a = row + 4096 * j;
           uint4 w[R];
 #pragma unroll
@@ -315,17 +318,29 @@ __device__ __forceinline__ void g2_consume(const G2Phase& p, const G2Symm& sy, c
 #pragma unroll
         for (int h = 0; h < R; ++h) acc[h] = warp_sum(acc[h]);
 #pragma unroll
-        for (int h = 0; h < R; ++h)
-          if (lane == 0) sts_f32(rstd_u + (warp * 8 + t + h) * 4, acc[h]);
+        for (int h = 0; h < R; ++h) {
+          const uint32_t sum = rstd_u + (warp * 8 + t + h) * 4;
+          if (lane == 0) sts_f32(sum, std::is_same<decltype(first), int>::value ? lds_f32(sum) + acc[h] : acc[h]);
+        }
       }
     };
     // The pass was unrolled over the tokens: code that no warp had fetched before for each of them, 0.5 to 0.7 us a token whatever K.  A rolled loop runs it from
     // the instruction cache; two tokens at a time, since one token's is a serial chain.  us in a graph, this / unrolled: with a norm, bf16 6144 x 4096 at 4 tokens
     // 10.3 / 11.5, at 8 11.7 / 14.4, gate|up 28672 x 4096 at 8 40.3 / 42.8; fp8 4096 x 4096 at 3 6.2 / 7.0, at 8 7.0 / 9.8, 4096 x 11008 at 3 10.6 / 11.1.
+    const std::integral_constant<int, 0> start;
+    const std::integral_constant<int, 1> one;
     int t = 0;
 #pragma unroll 1
-    for (; t + 1 < T; t += 2) rows(t, std::integral_constant<int, 2>{});
-    if (t < T) rows(t, std::integral_constant<int, 1>{});
+    for (; t + 1 < T; t += 2) rows(t, start, std::integral_constant<int, 2>{});
+    if (t < T) rows(t, start, one);
+    if constexpr (WIDE) {
+#pragma unroll 1
+      for (int first = G2_MAXV; 256 * first < nvec; first += G2_MAXV) {
+        if (has_norm) load_gamma(first);
+#pragma unroll 1
+        for (t = 0; t < T; ++t) rows(t, first, one);
+      }
+    }
     asm volatile("bar.sync 1, 256;" ::: "memory");
   }
   if (prof && ctid == 0) prof[3] = clock64();
