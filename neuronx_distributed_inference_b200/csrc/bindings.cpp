@@ -23,12 +23,13 @@ static inline const void* optr(const c10::optional<at::Tensor>& t) { return t.ha
 static inline bool is_bf16(const at::Tensor& t) { return t.scalar_type() == at::kBFloat16; }
 
 // ---- rmsnorm ------------------------------------------------------------------------------------------
+constexpr int64_t RMSNORM_MAX_H = 16384;
 // x [.., H], a residual like it; clear: words set to zero on the way (the tickets of the GEMM that follows)
 static at::Tensor rmsnorm_rows(const at::Tensor& x, const at::Tensor& w, double eps, double offset, const at::Tensor* residual, at::Tensor* res_out,
                                unsigned* clear = nullptr, int n_clear = 0) {
   TORCH_CHECK(x.is_cuda() && is_bf16(x) && x.is_contiguous() && is_bf16(w));
   const int64_t H = x.size(-1), rows = H ? x.numel() / H : 0;
-  TORCH_CHECK(H % 8 == 0 && H <= 16384, "rmsnorm: hidden must be a multiple of 8 and <= 16384");
+  TORCH_CHECK(H % 8 == 0 && H <= RMSNORM_MAX_H, "rmsnorm: hidden must be a multiple of 8 and <= 16384");
   c10::cuda::CUDAGuard guard(x.device());
   auto y = at::empty_like(x);
   if (residual != nullptr) {
@@ -208,8 +209,8 @@ at::Tensor gemv(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
   if (residual.has_value())
     TORCH_CHECK(!glu && residual->is_contiguous() && residual->size(0) == x.size(0) && residual->size(1) == N && is_bf16(*residual));
   // rows too wide for the streaming kernel's shared memory (from 7 tokens of 14336, 8 of 11008).  us, here / one warp per weight row: 4096 x 14336 at 7 tokens
-  // 26 / 57, at 8 26 / 36; 4096 x 11008 at 8 21 / 39
-  if (!gemv2_supported(x.size(0), x.size(1), 0) && (glu ? N / 2 : N) % 8 == 0) {
+  // 26 / 57, at 8 26 / 36; 4096 x 11008 at 8 21 / 39.  With a norm, rows wider than its kernel takes stay with the kernel that normalises them itself
+  if (!gemv2_supported(x.size(0), x.size(1), 0) && (glu ? N / 2 : N) % 8 == 0 && (!norm_w.has_value() || x.size(1) <= RMSNORM_MAX_H)) {
     run_skinny(x, w, bias, (int)act, residual, y, false, norm_w, eps, offset);
     return y;
   }

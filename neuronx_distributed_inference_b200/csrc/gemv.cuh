@@ -13,8 +13,8 @@
 //   * the first weight batch is issued BEFORE griddepcontrol.wait (PDL): weights never depend on the
 //     previous kernel, so HBM streaming continues across kernel boundaries inside the decode CUDA graph;
 //   * epilogues: bias, residual, SwiGLU/GeGLU (tile = 8 gate rows + 8 up rows).
-// Role since round 2: the fallback for activations too wide for shared memory (T*K*2 > ~200 KB, e.g. 8 tokens x K=14336);
-// everything else — and every fused all-reduce — runs on the TMA-pipelined gemv2.cu.
+// Role: rows too wide for the ring of the TMA-pipelined gemv2.cu (8 x 14336 and the like) that skinny_gemm.cu does not take either: output widths that are
+// no multiple of 8, and rows of more than 16384 columns with a norm.  Everything else, and every fused all-reduce, runs on those two.
 #pragma once
 #include "api.h"
 #include "common.cuh"

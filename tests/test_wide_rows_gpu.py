@@ -34,3 +34,14 @@ def test_every_column_counts(wdtype, T, K, N):
     assert _rel(ops.linear(x, q, scale=s, act="silu_mul"), ref.linear(x.double(), w, act="silu_mul")) < 5e-3
     assert _rel(ops.linear(x, q, norm_weight=n, norm_eps=1e-5, scale=s), h @ w.t()) < 6e-3
     assert _rel(ops.linear(x, q, norm_weight=n, norm_eps=1e-5, scale=s, act="silu_mul"), ref.linear(h, w, act="silu_mul")) < 1e-2
+
+
+@pytest.mark.parametrize("T,K", [(1, 87296), (2, 43776), (2, 54016), (3, 28928), (4, 22016), (4, 26880), (5, 17664), (5, 18432), (6, 16640), (6, 17920)])
+@pytest.mark.parametrize("N", [64, 2064])
+def test_norm_of_rows_wider_than_the_norm_kernel_takes(T, K, N):
+    """Rows above 16384 columns that the streaming kernel has no shared memory for: the kernel that normalises them itself."""
+    x, w, _, n, wd = _layer(T, N, K, BF)
+    h = x.double() * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-5) * (n.double() + 1)
+    r = torch.randn(T, N, device=DEV, dtype=BF)
+    assert _rel(ops.linear(x, w, norm_weight=n, norm_eps=1e-5, norm_offset=1.0, residual=r), h @ wd.t() + r.double()) < 6e-3
+    assert _rel(ops.linear(x, w, norm_weight=n, norm_eps=1e-5, norm_offset=1.0, act="silu_mul"), ref.linear(h, wd, act="silu_mul")) < 1e-2
