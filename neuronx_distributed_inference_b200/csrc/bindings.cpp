@@ -24,11 +24,16 @@ static inline bool is_bf16(const at::Tensor& t) { return t.scalar_type() == at::
 
 // ---- rmsnorm ------------------------------------------------------------------------------------------
 constexpr int64_t RMSNORM_MAX_H = 16384;
+// the kernels read a norm's weight as K bf16 values side by side
+static void check_norm_weight(const at::Tensor& w, int64_t K) {
+  TORCH_CHECK(w.is_cuda() && is_bf16(w) && w.numel() == K && w.is_contiguous(), "norm weight: ", K, " contiguous bf16 values on the GPU expected");
+}
 // x [.., H], a residual like it; clear: words set to zero on the way (the tickets of the GEMM that follows)
 static at::Tensor rmsnorm_rows(const at::Tensor& x, const at::Tensor& w, double eps, double offset, const at::Tensor* residual, at::Tensor* res_out,
                                unsigned* clear = nullptr, int n_clear = 0) {
-  TORCH_CHECK(x.is_cuda() && is_bf16(x) && x.is_contiguous() && is_bf16(w));
+  TORCH_CHECK(x.is_cuda() && is_bf16(x) && x.is_contiguous());
   const int64_t H = x.size(-1), rows = H ? x.numel() / H : 0;
+  check_norm_weight(w, H);
   TORCH_CHECK(H % 8 == 0 && H <= RMSNORM_MAX_H, "rmsnorm: hidden must be a multiple of 8 and <= 16384");
   c10::cuda::CUDAGuard guard(x.device());
   auto y = at::empty_like(x);
@@ -42,14 +47,14 @@ static at::Tensor rmsnorm_rows(const at::Tensor& x, const at::Tensor& w, double 
 }
 std::tuple<at::Tensor, at::Tensor> rmsnorm(const at::Tensor& x, const at::Tensor& w, double eps, double offset, const c10::optional<at::Tensor>& residual) {
   TORCH_CHECK(x.dim() >= 1);
-  const auto xc = x.contiguous();          // (a slice of a wider projection arrives strided)
+  const auto xc = x.contiguous(), wc = w.contiguous();          // (a slice of a wider projection arrives strided)
   if (!residual.has_value()) {
-    auto y = rmsnorm_rows(xc, w, eps, offset, nullptr, nullptr);
+    auto y = rmsnorm_rows(xc, wc, eps, offset, nullptr, nullptr);
     return {y, y};
   }
   at::Tensor r;
   const auto rc = residual->contiguous();
-  auto y = rmsnorm_rows(xc, w, eps, offset, &rc, &r);
+  auto y = rmsnorm_rows(xc, wc, eps, offset, &rc, &r);
   return {y, r};
 }
 
@@ -166,6 +171,7 @@ static void run_skinny(at::Tensor x, const at::Tensor& w, const c10::optional<at
 at::Tensor gemv(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias,
                 const c10::optional<at::Tensor>& norm_w, double eps, double offset, int64_t act,
                 const c10::optional<at::Tensor>& scale, const c10::optional<at::Tensor>& residual) {
+  if (norm_w.has_value()) check_norm_weight(*norm_w, x.size(-1));
   if (scale.has_value()) {
     // weight-only quantised path (int8 / fp8-e4m3, per-channel or per-tensor scale)
     TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && is_bf16(x));
@@ -297,7 +303,7 @@ static at::Tensor linear8_few(const at::Tensor& x, const at::Tensor& w, const c1
 // alone: the caller normalises first).  bf16 x; w bf16, or int8 / fp8 with a scale per channel or one.
 enum { LINEAR_QGEMV = 1, LINEAR_GEMV = 2, LINEAR_DEQUANT = 4, LINEAR_GEMM = 8, LINEAR_NORM = 16 };
 std::tuple<c10::optional<at::Tensor>, int64_t> linear(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias,
-                                                      const c10::optional<at::Tensor>& norm_w, double eps, double offset, int64_t act,
+                                                      const c10::optional<at::Tensor>& norm_in, double eps, double offset, int64_t act,
                                                       const c10::optional<at::Tensor>& scale, const c10::optional<at::Tensor>& residual,
                                                       const c10::optional<at::Tensor>& out, bool tensor_cores) {
   const auto none = std::make_tuple(c10::optional<at::Tensor>(), (int64_t)0);
@@ -311,9 +317,11 @@ std::tuple<c10::optional<at::Tensor>, int64_t> linear(const at::Tensor& x, const
   else if (few && plain && K % 64 == 0 && (K % 256 == 0 || gemv2_supported((int)T, (int)K, 0))) ran = LINEAR_GEMV;
   else if (!few && K % 64 == 0 && n_out % 8 == 0 && tensor_cores) ran = LINEAR_GEMM | (wq && !few8 ? LINEAR_DEQUANT : 0);
   else return none;
-  if ((ran & LINEAR_GEMM) && norm_w.has_value()) {
-    if (!is_bf16(*norm_w)) return std::make_tuple(c10::optional<at::Tensor>(), (int64_t)LINEAR_NORM);
-    ran |= LINEAR_NORM;
+  c10::optional<at::Tensor> norm_w;
+  if (norm_in.has_value()) {
+    if (!is_bf16(*norm_in)) return std::make_tuple(c10::optional<at::Tensor>(), (int64_t)LINEAR_NORM);
+    norm_w = norm_in->contiguous();
+    if (ran & LINEAR_GEMM) ran |= LINEAR_NORM;
   }
   const auto x2 = x.reshape({T, K});
   c10::optional<at::Tensor> r2, scale_f;

@@ -1,0 +1,45 @@
+"""Arguments of ops.linear that its kernels do not take as they are: the few-row kernels read norm weights and biases as dense bf16."""
+import pytest
+import torch
+
+from neuronx_distributed_inference_b200 import ops
+from neuronx_distributed_inference_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+DEV, BF = "cuda", torch.bfloat16
+TYPES = [BF, torch.int8, torch.float8_e4m3fn]
+
+
+def _rel(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-9)).item()
+
+
+def _layer(T, N, K, wdtype):
+    x, w, n = torch.randn(T, K, device=DEV, dtype=BF), torch.randn(N, K, device=DEV) / K ** 0.5, torch.randn(K, device=DEV)
+    q, s = (w.to(BF), None) if wdtype == BF else ref.quantize_per_channel(w, wdtype)
+    h = x.double() * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-5)
+    return x, q, s, n, h, q.double() if s is None else q.double() * s.double().view(-1, 1)
+
+
+@pytest.mark.parametrize("wdtype", TYPES)
+@pytest.mark.parametrize("T,K", [(1, 512), (8, 512), (9, 512), (8, 11008), (600, 512)])
+def test_norm_weight_of_another_type(wdtype, T, K):
+    """fp32 norm weights, as checkpoints keep them, at every number of rows (rows, x gamma and result are rounded to bf16; from 513 rows on 8-bit weights too)."""
+    x, q, s, n, h, w = _layer(T, 136, K, wdtype)
+    assert _rel(ops.linear(x, q, norm_weight=n, norm_eps=1e-5, scale=s), (h * n.double()) @ w.t()) < 8e-3
+
+
+@pytest.mark.parametrize("wdtype", TYPES)
+@pytest.mark.parametrize("T", [1, 8, 9])
+def test_strided_norm_weight(wdtype, T):
+    x, q, s, n, h, w = _layer(T, 136, 512, wdtype)
+    n2 = torch.stack([n.to(BF), torch.zeros_like(n, dtype=BF)], -1)[:, 0]
+    assert _rel(ops.linear(x, q, norm_weight=n2, norm_eps=1e-5, scale=s), (h * n2.double()) @ w.t()) < 8e-3
+
+
+@pytest.mark.parametrize("wdtype", TYPES)
+@pytest.mark.parametrize("T", [1, 8, 9, 600])
+def test_norm_weight_of_another_length(wdtype, T):
+    x, q, s, n, _, _ = _layer(T, 136, 512, wdtype)
+    with pytest.raises(RuntimeError):
+        ops.linear(x, q, norm_weight=n.to(BF)[:256].contiguous(), scale=s)
