@@ -302,7 +302,7 @@ static at::Tensor linear8_few(const at::Tensor& x, const at::Tensor& w, const c1
 // -> result and what ran (the bits below), or none where no kernel takes the call (the caller's library path) or the norm's weight is of another type (LINEAR_NORM
 // alone: the caller normalises first).  bf16 x; w bf16, or int8 / fp8 with a scale per channel or one.
 enum { LINEAR_QGEMV = 1, LINEAR_GEMV = 2, LINEAR_DEQUANT = 4, LINEAR_GEMM = 8, LINEAR_NORM = 16 };
-std::tuple<c10::optional<at::Tensor>, int64_t> linear(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias,
+std::tuple<c10::optional<at::Tensor>, int64_t> linear(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias_in,
                                                       const c10::optional<at::Tensor>& norm_in, double eps, double offset, int64_t act,
                                                       const c10::optional<at::Tensor>& scale, const c10::optional<at::Tensor>& residual,
                                                       const c10::optional<at::Tensor>& out, bool tensor_cores) {
@@ -323,6 +323,12 @@ std::tuple<c10::optional<at::Tensor>, int64_t> linear(const at::Tensor& x, const
     norm_w = norm_in->contiguous();
     if (ran & LINEAR_GEMM) ran |= LINEAR_NORM;
   }
+  c10::optional<at::Tensor> bias;
+  if (bias_in.has_value()) {
+    TORCH_CHECK(bias_in->is_cuda() && is_bf16(*bias_in) && bias_in->numel() == N, "linear: a bias of ", N, " bf16 values on the GPU expected");
+    bias = bias_in->contiguous();
+  }
+  if (scale.has_value()) TORCH_CHECK(scale->is_cuda() && (scale->numel() == 1 || scale->numel() == N), "linear: scales on the GPU, one or ", N, " expected");
   const auto x2 = x.reshape({T, K});
   c10::optional<at::Tensor> r2, scale_f;
   if (residual.has_value() && act == 0) r2 = wq && few ? residual->reshape({T, -1}).contiguous() : residual->reshape({T, -1});

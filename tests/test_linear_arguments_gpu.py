@@ -43,3 +43,24 @@ def test_norm_weight_of_another_length(wdtype, T):
     x, q, s, n, _, _ = _layer(T, 136, 512, wdtype)
     with pytest.raises(RuntimeError):
         ops.linear(x, q, norm_weight=n.to(BF)[:256].contiguous(), scale=s)
+
+
+@pytest.mark.parametrize("wdtype", TYPES)
+@pytest.mark.parametrize("T", [1, 8, 9, 600])
+def test_bias(wdtype, T):
+    """A strided bias counts as its dense copy; one of another type is refused, as F.linear refuses it, and so is one of another length."""
+    x, q, s, _, _, w = _layer(T, 136, 512, wdtype)
+    b = torch.randn(136, device=DEV)
+    b2 = torch.stack([b.to(BF), torch.zeros_like(b, dtype=BF)], -1)[:, 0]
+    assert _rel(ops.linear(x, q, b2, scale=s), x.double() @ w.t() + b2.double()) < 5e-3
+    for bad in (b, b.to(BF)[:64].contiguous()):
+        with pytest.raises(RuntimeError):
+            ops.linear(x, q, bad, scale=s)
+
+
+@pytest.mark.parametrize("wdtype", TYPES[1:])
+@pytest.mark.parametrize("T", [1, 9, 600])
+def test_scale_in_host_memory(wdtype, T):
+    x, q, s, _, _, _ = _layer(T, 136, 512, wdtype)
+    with pytest.raises(RuntimeError):
+        ops.linear(x, q, scale=s.cpu())
