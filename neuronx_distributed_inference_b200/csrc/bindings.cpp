@@ -717,14 +717,16 @@ at::Tensor argmax(const at::Tensor& logits, const std::vector<int64_t>& slot_ptr
 
 at::Tensor topk_sample(const at::Tensor& logits_in, const at::Tensor& top_k_in, const at::Tensor& top_p_in,
                        const at::Tensor& temperature_in, const c10::optional<at::Tensor>& rand_in, int64_t global_topk) {
-  const auto logits = logits_in.contiguous(), top_k = top_k_in.to(at::kInt), top_p = top_p_in.to(at::kFloat), temperature = temperature_in.to(at::kFloat);
-  const auto rand = rand_in.has_value() ? rand_in->to(at::kFloat) : at::full({logits.size(0)}, 0.5, logits.options().dtype(at::kFloat));
+  // (columns of one parameter matrix arrive strided)
+  const auto logits = logits_in.contiguous(), top_k = top_k_in.to(at::kInt).contiguous(), top_p = top_p_in.to(at::kFloat).contiguous(),
+             temperature = temperature_in.to(at::kFloat).contiguous();
+  const auto rand = rand_in.has_value() ? rand_in->to(at::kFloat).contiguous() : at::full({logits.size(0)}, 0.5, logits.options().dtype(at::kFloat));
   TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.stride(1) == 1);
   TORCH_CHECK(logits.scalar_type() == at::kFloat || is_bf16(logits), "topk_sample: fp32 or bf16 logits");
   TORCH_CHECK(global_topk >= 1 && global_topk <= 256);
   const int B = logits.size(0), V = logits.size(1);
-  TORCH_CHECK(top_k.scalar_type() == at::kInt && top_k.numel() == B && top_p.scalar_type() == at::kFloat &&
-              temperature.scalar_type() == at::kFloat && rand.scalar_type() == at::kFloat && rand.numel() == B);
+  for (const auto* t : {&top_k, &top_p, &temperature, &rand})
+    TORCH_CHECK(t->is_cuda() && t->numel() == B, "topk_sample: top_k, top_p, temperature and rand hold a value per row, on the GPU");
   c10::cuda::CUDAGuard guard(logits.device());
   auto out = at::empty({B}, logits.options().dtype(at::kLong));
   if (B == 0) return out;

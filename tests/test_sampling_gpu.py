@@ -64,3 +64,24 @@ def test_values_that_share_their_leading_bytes(k, near):
     top_k, rand = torch.full((B,), k, dtype=torch.int32), torch.rand(B)
     got = ops.sample(logits.cuda(), top_k.cuda(), one.cuda(), one.cuda(), rand.cuda())
     assert torch.equal(got.cpu(), ref.sample(logits, top_k, one, one, rand))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_strided_parameters(dtype):
+    """Columns of one parameter matrix, and of one matrix of draws, give what dense copies of them give."""
+    B, V = 5, 4000
+    logits = (torch.randn(B, V, device="cuda") * 3).to(dtype)
+    params = torch.stack([torch.randint(1, 200, (B,), device="cuda").float(), torch.linspace(0.2, 1.0, B, device="cuda"), torch.linspace(1.5, 0.3, B, device="cuda")], -1)
+    ks, rand = torch.stack([params[:, 0].int(), torch.ones(B, device="cuda", dtype=torch.int32)], -1), torch.rand(B, 7, device="cuda")
+    got = ops.sample(logits, ks[:, 0], params[:, 1], params[:, 2], rand[:, 3], global_topk=256)
+    dense = [t.clone(memory_format=torch.contiguous_format) for t in (ks[:, 0], params[:, 1], params[:, 2], rand[:, 3])]
+    assert torch.equal(got, ops.sample(logits, *dense, global_topk=256))
+    assert torch.equal(got, ops.sample(logits, params[:, 0], params[:, 1], params[:, 2], rand[:, 3], global_topk=256))
+    assert torch.equal(ops.sample(logits, ks[:, 0], params[:, 1], params[:, 2], global_topk=256), ops.sample(logits, *dense[:3], global_topk=256))
+
+
+@pytest.mark.parametrize("bad", range(4))
+def test_parameters_of_another_length(bad):
+    args = [torch.ones(3 if i == bad else 4, device="cuda") for i in range(4)]
+    with pytest.raises(RuntimeError):
+        ops.sample(torch.randn(4, 100, device="cuda"), *args)
