@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <memory>
 #include <string>
 #include <utility>
 #include <vector>
@@ -13,6 +14,17 @@ namespace nxdi {
 constexpr int SYMM_MAX_RANKS = 8;
 constexpr int SYMM_MAX_TILES = 1024;
 constexpr int GEMV_MAX_T = 8;
+
+// workspace.cpp: `nf` floats, `ni` ints and `nt` tickets (zero, and left zero) for launches on `stream` of the current device, until `keep` goes.  A launch takes them
+// after it has waited for the launch in front: those of one stream share them.
+struct Workspace {
+  float* f;
+  int* i;
+  unsigned* tickets;
+  std::shared_ptr<const void> keep;
+};
+Workspace workspace(cudaStream_t stream, int64_t nf, int64_t ni, int64_t nt);
+int workspace_rows_in_use(int device);
 
 struct SymmArgs {
   float* recv[SYMM_MAX_RANKS];  // peer-mapped LL receive buffers  [2 parity][world src][8 tok][n_max] x {fp32 value, u32 tag}

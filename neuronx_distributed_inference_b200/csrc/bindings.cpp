@@ -6,8 +6,6 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <cuda_runtime.h>
 
-#include <map>
-
 #include "api.h"
 
 namespace nxdi {
@@ -58,31 +56,13 @@ std::tuple<at::Tensor, at::Tensor> rmsnorm(const at::Tensor& x, const at::Tensor
   return {y, r};
 }
 
-struct Scratch {
-  at::Tensor f, i, tickets, gemv_ws, gemv_tickets;
-  // Buffers that were outgrown are RETIRED, never freed: CUDA graphs captured earlier hold their addresses (a decode graph of a
-  // small sequence bucket keeps replaying after a larger bucket made the workspace grow); freeing them would hand the memory to
-  // the caching allocator while those graphs still write their split-KV partials / stream-K tickets there.
-  std::vector<at::Tensor> retired;
-  void grow(at::Tensor& t, int64_t n, const at::TensorOptions& o, bool zero) {
-    if (t.defined() && t.numel() >= n) return;
-    if (t.defined()) retired.push_back(t);
-    t = zero ? at::zeros({n}, o) : at::empty({n}, o);
-  }
-};
-static Scratch& scratch(const at::Device& dev, int64_t nf, int64_t ni, int64_t nt);
-
-static void run_gemv(GemvParams& p, int mode, const at::Device& dev) {
+static void run_gemv(GemvParams& p, int mode) {
   const int wt = p.scale != nullptr ? p.wdtype : 0;
   if (gemv2_supported(p.T, p.K, wt) && p.x_in_smem) {
-    auto& s = scratch(dev, 0, 0, 0);
     const bool glu = p.act != 0;
     const int n_tiles = gemv2_ntiles(p.N, glu);
-    const int64_t need = (int64_t)n_tiles * gemv2_pmax(p.N, p.K, glu, wt) * 128;
-    auto o = at::TensorOptions().device(dev);
-    s.grow(s.gemv_ws, std::max<int64_t>(need, 4 << 20), o.dtype(at::kFloat), false);
-    s.grow(s.gemv_tickets, std::max<int64_t>(n_tiles, 1 << 15), o.dtype(at::kInt), true);
-    gemv2_launch(p, mode, s.gemv_ws.data_ptr<float>(), reinterpret_cast<unsigned*>(s.gemv_tickets.data_ptr<int>()), cur_stream());
+    const auto ws = workspace(cur_stream(), (int64_t)n_tiles * gemv2_pmax(p.N, p.K, glu, wt) * 128, 0, n_tiles);
+    gemv2_launch(p, mode, ws.f, ws.tickets, cur_stream());
   } else {
     TORCH_CHECK(wt == 0, "gemv: 8-bit weights need the TMA streaming kernel");
     TORCH_CHECK(p.K % 256 == 0, "gemv: K must be a multiple of 256 on the wide-activation fallback");
@@ -189,7 +169,7 @@ at::Tensor gemv(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
     if (q2 && gemv2_supported((int)x.size(0), (int)x.size(1), i8 ? 1 : 2) && x.stride(0) % 8 == 0 && (!glu || N % 2 == 0)) {
       GemvParams p{};
       fill_params(p, x, w, bias, norm_w, eps, offset, (int)act, residual, scale, y, true);
-      run_gemv(p, 0, x.device());
+      run_gemv(p, 0);
       return y;
     }
     // rows too wide for its shared memory (from 8 tokens of 11008, 7 of 14336): bytes expanded on the way to the tensor cores.  us in a graph, fp8 / one warp per
@@ -224,7 +204,7 @@ at::Tensor gemv(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
   at::Tensor xn = prenorm_if_needed(x, norm_w, eps, offset, x_in_smem);
   GemvParams p{};
   fill_params(p, xn, w, bias, norm_w, eps, offset, (int)act, residual, scale, y, x_in_smem);
-  run_gemv(p, 0, x.device());
+  run_gemv(p, 0);
   return y;
 }
 
@@ -390,7 +370,7 @@ at::Tensor gemv_allreduce(const at::Tensor& x, const at::Tensor& w, const c10::o
   p.symm.parity = parity;
   p.symm.call = call;
   p.symm.n_max = n_max;
-  run_gemv(p, 1, x.device());
+  run_gemv(p, 1);
   return y;
 }
 
@@ -680,17 +660,6 @@ void paged_kv_append(at::Tensor& k_cache, at::Tensor& v_cache, const at::Tensor&
 }
 
 // ---- sampling ---------------------------------------------------------------------------------------------------
-static Scratch& scratch(const at::Device& dev, int64_t nf, int64_t ni, int64_t nt) {
-  static std::map<int, Scratch> all;
-  auto& s = all[dev.index()];
-  auto o = at::TensorOptions().device(dev);
-  // generous first sizes (16 MB of partials covers B = 8, 8 kv heads, 32 splits at head_dim 128) so that growth is rare
-  s.grow(s.f, std::max<int64_t>(nf, 4 << 20), o.dtype(at::kFloat), false);
-  s.grow(s.i, std::max<int64_t>(ni, 1 << 16), o.dtype(at::kInt), false);
-  s.grow(s.tickets, std::max<int64_t>(nt, 1 << 14), o.dtype(at::kInt), true);
-  return s;
-}
-
 at::Tensor argmax(const at::Tensor& logits, const std::vector<int64_t>& slot_ptrs, const c10::optional<at::Tensor>& step,
                   int64_t rank, int64_t parity, int64_t call, int64_t rows_max) {
   TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.stride(1) == 1);
@@ -699,7 +668,7 @@ at::Tensor argmax(const at::Tensor& logits, const std::vector<int64_t>& slot_ptr
   c10::cuda::CUDAGuard guard(logits.device());
   auto out = at::empty({B}, logits.options().dtype(at::kLong));
   const int nsplit = std::max(1, std::min(64, V / 2048));
-  auto& ws = scratch(logits.device(), (int64_t)B * nsplit, (int64_t)B * nsplit, B);
+  const auto ws = workspace(cur_stream(), (int64_t)B * nsplit, (int64_t)B * nsplit, B);
   ArgmaxSymm sy{};
   const int world = slot_ptrs.size();
   if (world > 1) {
@@ -709,8 +678,8 @@ at::Tensor argmax(const at::Tensor& logits, const std::vector<int64_t>& slot_ptr
     sy.step = reinterpret_cast<const uint32_t*>(step->data_ptr<int>());
     sy.rank = rank; sy.world = world; sy.parity = parity; sy.call = call; sy.rows_max = rows_max;
   }
-  argmax_launch(logits.data_ptr(), is_bf16(logits) ? 1 : 0, out.data_ptr<int64_t>(), ws.f.data_ptr<float>(), ws.i.data_ptr<int>(),
-                reinterpret_cast<unsigned*>(ws.tickets.data_ptr<int>()), B, V, (int)logits.stride(0), nsplit,
+  argmax_launch(logits.data_ptr(), is_bf16(logits) ? 1 : 0, out.data_ptr<int64_t>(), ws.f, ws.i,
+                ws.tickets, B, V, (int)logits.stride(0), nsplit,
                 world > 1 ? &sy : nullptr, cur_stream());
   return out;
 }
@@ -766,10 +735,10 @@ at::Tensor attention_decode(const at::Tensor& q, const at::Tensor& k_cache, cons
   p.sinks = sinks.has_value() ? sinks->data_ptr<float>() : nullptr;
   p.B = B; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.S = S; p.L = L; p.window = window; p.scale = (float)scale;
   p.nsplit = pick_nsplit(B, Hkv, s_hint > 0 ? (int)std::min<int64_t>(s_hint, S) : S);
-  auto& ws = scratch(q.device(), (int64_t)B * Hkv * p.nsplit * 64 * (D + 2), 0, (int64_t)B * Hkv);
-  p.ws_o = ws.f.data_ptr<float>();
+  const auto ws = workspace(cur_stream(), (int64_t)B * Hkv * p.nsplit * 64 * (D + 2), 0, (int64_t)B * Hkv);
+  p.ws_o = ws.f;
   p.ws_ml = p.ws_o + (int64_t)B * Hkv * p.nsplit * 64 * D;
-  p.tickets = reinterpret_cast<unsigned*>(ws.tickets.data_ptr<int>());
+  p.tickets = ws.tickets;
   attention_decode_launch(p, cur_stream());
   return out;
 }
@@ -801,10 +770,10 @@ at::Tensor rope_attention_decode(const at::Tensor& qkv, const at::Tensor& cos, c
   p.qkv = qkv.data_ptr(); p.cos = cos.data_ptr<float>(); p.sin = sin.data_ptr<float>();
   p.q_norm = optr(q_norm); p.k_norm = optr(k_norm); p.write_pos = write_pos.data_ptr<int>(); p.norm_eps = (float)eps;
   p.nsplit = pick_nsplit(B, nkv, s_hint > 0 ? (int)std::min<int64_t>(s_hint, S) : S);
-  auto& ws = scratch(qkv.device(), (int64_t)B * nkv * p.nsplit * 64 * (D + 2), 0, (int64_t)B * nkv);
-  p.ws_o = ws.f.data_ptr<float>();
+  const auto ws = workspace(cur_stream(), (int64_t)B * nkv * p.nsplit * 64 * (D + 2), 0, (int64_t)B * nkv);
+  p.ws_o = ws.f;
   p.ws_ml = p.ws_o + (int64_t)B * nkv * p.nsplit * 64 * D;
-  p.tickets = reinterpret_cast<unsigned*>(ws.tickets.data_ptr<int>());
+  p.tickets = ws.tickets;
   attention_decode_launch(p, cur_stream());
   return out;
 }
@@ -856,10 +825,10 @@ at::Tensor paged_attention_decode(const at::Tensor& q, const at::Tensor& k_cache
   p.nsplit = paged_nsplit(B * Hkv, p.max_blocks * bs);
   p.by_length = B > 1 && B <= ATT_MAX_ORDER && B * Hkv >= 96 && B * Hkv < 1024 ? 1 : 0;
   const int64_t rows = (int64_t)B * Hkv * p.nsplit * T * (Hq / Hkv);
-  auto& ws = scratch(q.device(), rows * (D + 2), 0, (int64_t)B * Hkv);
-  p.ws_o = ws.f.data_ptr<float>();
+  const auto ws = workspace(cur_stream(), rows * (D + 2), 0, (int64_t)B * Hkv);
+  p.ws_o = ws.f;
   p.ws_ml = p.ws_o + rows * D;
-  p.tickets = reinterpret_cast<unsigned*>(ws.tickets.data_ptr<int>());
+  p.tickets = ws.tickets;
   attention_decode_launch(p, cur_stream());
   return out;
 }
@@ -1070,6 +1039,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("symm_close", &nxdi::symm_close);
   m.def("symm_free", &nxdi::symm_free);
   m.def("symm_as_tensor", &nxdi::symm_as_tensor);
+  m.def("workspace_rows_in_use", [](int64_t device) { return nxdi::workspace_rows_in_use((int)device); });
   m.def("rope_rows", &nxdi::rope_rows);
   m.def("cache_lines", &nxdi::cache_lines);
   m.def("rope_kv_append", &nxdi::rope_kv_append);
