@@ -620,28 +620,8 @@ static void make_2d(CUtensorMap* tm, const void* ptr, int rows, int K, int ld_el
   if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled (gemm) failed: " + std::to_string((int)r));
 }
 
-// split-K scratch (per device): fp32 partial tiles + tickets
-static size_t gemm_ws_bytes() { return (size_t)96 << 20; }
-static int gemm_max_tickets() { return 1 << 16; }
-static float* g_gemm_ws[16] = {nullptr};
-static unsigned* g_gemm_tk[16] = {nullptr};
-static float* gemm_ws() {
-  int dev;
-  cudaGetDevice(&dev);
-  if (g_gemm_ws[dev] == nullptr) {
-    if (cudaMalloc(&g_gemm_ws[dev], gemm_ws_bytes()) != cudaSuccess) throw std::runtime_error("gemm: split-K workspace allocation failed");
-  }
-  return g_gemm_ws[dev];
-}
-static unsigned* gemm_tickets() {
-  int dev;
-  cudaGetDevice(&dev);
-  if (g_gemm_tk[dev] == nullptr) {
-    if (cudaMalloc(&g_gemm_tk[dev], gemm_max_tickets() * sizeof(unsigned)) != cudaSuccess) throw std::runtime_error("gemm: ticket allocation failed");
-    cudaMemset(g_gemm_tk[dev], 0, gemm_max_tickets() * sizeof(unsigned));
-  }
-  return g_gemm_tk[dev];
-}
+// most that the partial tiles of a split K may take
+constexpr size_t GM_WS_BYTES = (size_t)96 << 20;
 
 static void gemm_launch_impl(const void* a, int lda, const void* b, const void* bias, const void* residual, void* c, int ldc, int M, int N,
                              int K, int act, cudaStream_t stream, const GemmRsArgs* rs, const float* a_scale, const float* w_scale,
@@ -737,18 +717,20 @@ static void gemm_launch_impl(const void* a, int lda, const void* b, const void* 
   // such as gate_up at M = 256 — 224 tiles — is better left alone: 86 us unsplit vs 280 us with 3 slices)
   if (tiles * 4 <= n_sms) {
     for (int sgl = 1; sgl <= 4; ++sgl) {
-      if (sgl > 1 && (nkb / sgl < 8 || (size_t)tiles * sgl * tile_ws_bytes > gemm_ws_bytes())) break;
+      if (sgl > 1 && (nkb / sgl < 8 || (size_t)tiles * sgl * tile_ws_bytes > GM_WS_BYTES)) break;
       const double cost = (double)((tiles * sgl + n_sms - 1) / n_sms) / sgl + (sgl > 1 ? 0.06 : 0.0);
       if (cost < best - 1e-9) { best = cost; best_s = sgl; }
     }
   }
   if (model_split > 0 && force_s <= 0 && !force_tm) best_s = model_split;
   p.splits = force_s > 0 ? std::min({force_s, 4, std::max(1, nkb / 2)}) : best_s;
-  if (force_s > 0 && (size_t)tiles * p.splits * tile_ws_bytes > gemm_ws_bytes()) p.splits = 1;
+  if (force_s > 0 && (size_t)tiles * p.splits * tile_ws_bytes > GM_WS_BYTES) p.splits = 1;
   if (rs != nullptr || tile_expert != nullptr) p.splits = 1;
-  if ((size_t)tiles * p.splits * tile_ws_bytes > gemm_ws_bytes() || tiles > gemm_max_tickets()) p.splits = 1;
-  p.ws = p.splits > 1 ? gemm_ws() : nullptr;
-  p.tickets = gemm_tickets();
+  if ((size_t)tiles * p.splits * tile_ws_bytes > GM_WS_BYTES) p.splits = 1;
+  Workspace ws{};
+  if (p.splits > 1) ws = workspace(stream, (int64_t)((size_t)tiles * p.splits * tile_ws_bytes / 4), 0, tiles);
+  p.ws = ws.f;
+  p.tickets = ws.tickets;
   if (rs != nullptr) {
     const int rows_per_seg = rs->rows_per_seg;
     if (rows_per_seg % (GM_BM * rs->world) != 0 || M % rows_per_seg != 0 || N % 8 != 0 || ldc != N)

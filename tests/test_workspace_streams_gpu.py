@@ -13,15 +13,16 @@ ROUNDS = 60
 
 
 def _calls(seed):
-    """Stream-K GEMVs (bf16 and fp8 weights), split decode attention, argmax: (call, result alone) pairs."""
+    """Stream-K GEMVs (bf16 and fp8 weights), GEMMs with a split K, split decode attention, argmax: (call, result alone) pairs."""
     g = torch.Generator(DEV).manual_seed(seed)
     rnd = lambda *s: torch.randn(*s, device=DEV, dtype=BF, generator=g)
     x, w = rnd(2, 4096), rnd(5000, 4096) * 0.02
     x8, w8 = rnd(3, 8192), (rnd(2056, 8192) * 0.02).to(torch.float8_e4m3fn)
     s8 = torch.rand(2056, device=DEV, generator=g)
     q, cache, lines, pos = rnd(2, 1, 8, 128), rnd(3, 2, 4096, 128), torch.tensor([0, 1], device=DEV, dtype=torch.int32), torch.tensor([[4000], [2500]], device=DEV, dtype=torch.int32)
+    xk, wk, xs, ws = rnd(200, 8192), rnd(1024, 8192) * 0.02, rnd(130, 4096), rnd(512, 4096) * 0.02
     logits = torch.randn(4, 50000, device=DEV, generator=g)
-    calls = [lambda: ops.linear(x, w), lambda: ops.linear(x, w, act="silu_mul"), lambda: ops.linear(x8, w8, scale=s8),
+    calls = [lambda: ops.linear(x, w), lambda: ops.linear(x, w, act="silu_mul"), lambda: ops.linear(x8, w8, scale=s8), lambda: ops.linear(xk, wk), lambda: ops.linear(xs, ws, act="silu_mul"),
              lambda: ops.attention_decode(q, cache, cache, lines, pos, 0.09), lambda: ops.argmax(logits)]
     return [(f, f()) for f in calls]
 
