@@ -5,17 +5,18 @@
 //   * eager calls: kept for the KEPT (device, stream) pairs that were used last.  Buffers that are outgrown or given up go back to the caching allocator, which
 //     hands them out again in the order of their stream; a call holds its own until its kernel is enqueued.
 //   * calls under capture: the graph may be replayed on any stream, beside eager calls and other graphs.  Partials come from the graph's memory pool, call by call.
-//     Tickets would have to be cleared by a launch of their own then (1.5 us a call); they are a row of a slab that was cleared before, one for each stream of a
-//     capture, and the row is free again once the graph is gone.  With no row left they are cleared call by call.
+//     Tickets would have to be cleared by a launch of their own then (1.5 us a call); they are a row of a slab that was cleared before, one for each memory pool of
+//     graphs and stream of a capture.  (Graphs of one pool share the rest of their memory too, and are not replayed at the same time.)  The row is free again once
+//     the pool has no graph left: a CUDA user object, which would tell of that, costs every replay 2 us.  With no row left tickets are cleared call by call.
 #include <algorithm>
 #include <array>
-#include <atomic>
 #include <map>
 #include <memory>
 #include <mutex>
 #include <vector>
 
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <cuda_runtime.h>
 #include <torch/types.h>
@@ -26,8 +27,9 @@ namespace nxdi {
 namespace {
 
 constexpr size_t KEPT = 8;
-constexpr int64_t FLOATS = 4 << 20, INTS = 1 << 16, TICKETS = 1 << 15;      // first sizes: growth is rare
-constexpr int ROWS = 64;                                                     // of the slab, TICKETS each
+constexpr int64_t FLOATS = 4 << 20, INTS = 1 << 16, TICKETS = 1 << 14;      // first sizes: growth is rare
+constexpr int ROWS = 256;                                                    // of the slab, TICKETS each: 16 MB
+constexpr c10::MempoolId_t NO_POOL{0, 0};
 
 struct Buffers {
   at::Tensor f, i, t;
@@ -46,8 +48,7 @@ struct Entry {
   std::shared_ptr<const Buffers> b;
 };
 struct Row {
-  std::atomic<bool> busy{false};
-  unsigned long long capture = 0;
+  c10::MempoolId_t pool = NO_POOL;      // of the graphs that use it; none: free
   cudaStream_t stream = nullptr;
 };
 struct Slab {
@@ -59,10 +60,11 @@ struct State {
   std::mutex m;
   std::vector<Entry> entries;
   std::map<int, Slab> slabs;
+  std::vector<std::pair<unsigned long long, c10::MempoolId_t>> captures;      // the last few and their pools
   unsigned long long clock = 0;
 };
 State& state() {
-  static State* s = new State;      // never destroyed: graphs that outlive the module give their rows back to it
+  static State* s = new State;      // never destroyed: its tensors would meet an allocator that is gone
   return *s;
 }
 
@@ -70,26 +72,46 @@ void check(cudaError_t e, const char* what) { TORCH_CHECK(e == cudaSuccess, what
 
 Workspace give(const std::shared_ptr<const Buffers>& b) { return {b->ws.f, b->ws.i, b->ws.tickets, b}; }
 
+// the memory pool that a capture allocates from (one look at the allocator's segments for each capture)
+c10::MempoolId_t pool_of(State& st, int device, unsigned long long capture) {
+  for (auto& c : st.captures)
+    if (c.first == capture) return c.second;
+  const auto probe = at::empty({1}, at::TensorOptions().device(at::kCUDA, (c10::DeviceIndex)device).dtype(at::kInt));
+  const size_t p = reinterpret_cast<size_t>(probe.data_ptr());
+  c10::MempoolId_t pool = NO_POOL;
+  for (const auto& segment : c10::cuda::CUDACachingAllocator::snapshot(NO_POOL, false).segments)
+    if (segment.device == device && p >= segment.address && p - segment.address < segment.total_size) pool = segment.owner_private_pool_id;
+  if (st.captures.size() == KEPT) st.captures.erase(st.captures.begin());
+  st.captures.emplace_back(capture, pool);
+  return pool;
+}
+// rows whose pools have no graph any more
+void free_rows(Slab& s, int device) {
+  for (auto& row : s.rows) {
+    if (row.pool == NO_POOL) continue;
+    int graphs = 0;
+    try {
+      graphs = c10::cuda::CUDACachingAllocator::getPoolUseCount((c10::DeviceIndex)device, row.pool);
+    } catch (const c10::Error&) {      // the allocator has forgotten the pool
+    }
+    if (graphs == 0) row = Row{};
+  }
+}
 // the capture's row of the slab, or null
-unsigned* captured_tickets(State& st, int device, unsigned long long capture, cudaStream_t stream, cudaGraph_t graph) {
+unsigned* captured_tickets(State& st, int device, unsigned long long capture, cudaStream_t stream) {
   auto it = st.slabs.find(device);
   if (it == st.slabs.end()) return nullptr;
+  const c10::MempoolId_t pool = pool_of(st, device, capture);
+  if (pool == NO_POOL) return nullptr;
   Slab& s = it->second;
   auto at_row = [&](int r) { return reinterpret_cast<unsigned*>(s.t.data_ptr<int>()) + (int64_t)r * TICKETS; };
   for (int r = 0; r < ROWS; ++r)
-    if (s.rows[r].busy.load() && s.rows[r].capture == capture && s.rows[r].stream == stream) return at_row(r);
-  for (int k = 0; k < ROWS; ++k) {
+    if (s.rows[r].pool == pool && s.rows[r].stream == stream) return at_row(r);
+  free_rows(s, device);
+  for (int k = 0; k < ROWS; ++k) {      // in turn: a row rests as long as possible before it is used again
     const int r = (s.next + k) % ROWS;
-    Row& row = s.rows[r];
-    if (row.busy.load()) continue;
-    cudaUserObject_t object;
-    check(cudaUserObjectCreate(&object, &row, [](void* p) { static_cast<Row*>(p)->busy.store(false); }, 1, cudaUserObjectNoDestructorSync), "cudaUserObjectCreate");
-    row.capture = capture;
-    row.stream = stream;
-    row.busy.store(true);
-    const cudaError_t e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
-    if (e != cudaSuccess) cudaUserObjectRelease(object, 1);
-    check(e, "cudaGraphRetainUserObject");
+    if (s.rows[r].pool != NO_POOL) continue;
+    s.rows[r] = Row{pool, stream};
     s.next = (r + 1) % ROWS;
     return at_row(r);
   }
@@ -107,10 +129,9 @@ Workspace workspace(cudaStream_t stream, int64_t nf, int64_t ni, int64_t nt) {
   std::lock_guard<std::mutex> lock(st.m);
   if (status != cudaStreamCaptureStatusNone) {
     unsigned long long capture = 0;
-    cudaGraph_t graph = nullptr;
-    check(cudaStreamGetCaptureInfo(stream, &status, &capture, &graph), "cudaStreamGetCaptureInfo");
+    check(cudaStreamGetCaptureInfo(stream, &status, &capture), "cudaStreamGetCaptureInfo");
     auto b = std::make_shared<Buffers>();
-    if (nt <= TICKETS) b->ws.tickets = captured_tickets(st, device, capture, stream, graph);
+    if (nt <= TICKETS) b->ws.tickets = captured_tickets(st, device, capture, stream);
     b->take(nf, ni, b->ws.tickets != nullptr ? 0 : nt, options());
     return give(b);
   }
@@ -141,10 +162,9 @@ int workspace_rows_in_use(int device) {
   State& st = state();
   std::lock_guard<std::mutex> lock(st.m);
   auto it = st.slabs.find(device);
-  int n = 0;
-  if (it != st.slabs.end())
-    for (auto& r : it->second.rows) n += r.busy.load() ? 1 : 0;
-  return n;
+  if (it == st.slabs.end()) return 0;
+  free_rows(it->second, device);
+  return (int)std::count_if(it->second.rows.begin(), it->second.rows.end(), [](const Row& r) { return r.pool != NO_POOL; });
 }
 
 }  // namespace nxdi

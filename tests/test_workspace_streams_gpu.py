@@ -117,22 +117,24 @@ def test_a_capture_with_two_branches():
         assert _same([out_a], a * 4) and _same([out_b], b * 4)
 
 
+def _capture(calls, **kw):
+    graph, out = torch.cuda.CUDAGraph(), []
+    with torch.cuda.graph(graph, **kw):
+        for f, _ in calls:
+            out.append(f())
+    return graph, out
+
+
 def test_rows_of_graphs_are_given_back():
-    """70 graphs at once: 64 take a row of cleared tickets, the others clear theirs; all rows are free once the graphs are gone."""
-    ext = ops._C()
-    pairs = _calls(0)
+    """260 graphs at once: 256 take a row of cleared tickets, the others clear theirs; the rows are free again when the graphs are gone."""
+    ext, pairs = ops._C(), _calls(0)
+    pairs = [pairs[0], pairs[-1]]
     gc.collect()
     torch.cuda.synchronize()
     before = ext.workspace_rows_in_use(0)
     for _ in range(2):
-        graphs = []
-        for _ in range(70):
-            graph, out = torch.cuda.CUDAGraph(), []
-            with torch.cuda.graph(graph):
-                for f, _ in pairs:
-                    out.append(f())
-            graphs.append((graph, out))
-        assert ext.workspace_rows_in_use(0) == 64
+        graphs = [_capture(pairs) for _ in range(260)]
+        assert ext.workspace_rows_in_use(0) == 256
         for _ in range(2):
             for graph, out in graphs:
                 graph.replay()
@@ -142,3 +144,26 @@ def test_rows_of_graphs_are_given_back():
         gc.collect()
         torch.cuda.synchronize()
         assert ext.workspace_rows_in_use(0) == before
+        torch.cuda.empty_cache()
+        assert ext.workspace_rows_in_use(0) == before
+
+
+def test_graphs_of_one_pool_share_a_row():
+    """They share their other memory too, and are replayed one after the other; the row stays until the last of them is gone."""
+    ext, pairs = ops._C(), _calls(0)
+    gc.collect()
+    before = ext.workspace_rows_in_use(0)
+    stream, pool = torch.cuda.Stream(), torch.cuda.graph_pool_handle()
+    graphs = [_capture(pairs, pool=pool, stream=stream)[0] for _ in range(3)]
+    assert ext.workspace_rows_in_use(0) == before + 1
+    del graphs[:2]
+    gc.collect()
+    assert ext.workspace_rows_in_use(0) == before + 1
+    more, out = _capture(pairs, pool=pool, stream=stream)
+    graphs[0].replay()
+    more.replay()
+    torch.cuda.synchronize()
+    assert _same([out], pairs) and ext.workspace_rows_in_use(0) == before + 1
+    del graphs, more, out
+    gc.collect()
+    assert ext.workspace_rows_in_use(0) == before
