@@ -37,8 +37,8 @@ struct Gemv2Params {
   int max_inflight;
 };
 
-template <bool GLU, int MODE, int WT, bool WIDE>
-__global__ void __launch_bounds__(G2_THREADS, 1) gemv2_kernel(const __grid_constant__ Gemv2Params pp) {
+template <bool GLU, int MODE, int WT, bool WIDE, int CTAS>
+__global__ void __launch_bounds__(G2_THREADS, CTAS) gemv2_kernel(const __grid_constant__ Gemv2Params pp) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   G2Phase ph = pp.ph;
@@ -158,19 +158,26 @@ int gemv2_pmax(int N, int K, bool glu, int wt) {
   return gemv2_grid(N, K, glu, wt) / n_tiles + 3;
 }
 
-template <bool GLU, int MODE, int WT, bool WIDE = false>
+// Registers.  With up to 112 of them the next kernel's CTAs start beside this one's, as long as shared memory holds both, and fetch their first weights: that pays where
+// the busiest CTA has a second tile to do meanwhile.  Elsewhere the 140 that the compiler takes are worth more.  us in a graph, two CTAs per SM / one, 1 and 8
+// tokens: bf16 4096 x 1024 3.2 / 3.8, 3.5 / 3.9, with a norm 3.6 / 4.0, 4.9 / 5.5; 8192 x 512 4.0 / 4.5, 4.3 / 4.5; fp8 4096 x 2048 3.7 / 4.0, 5.0 / 5.5; one tile per CTA:
+// bf16 2048 x 2048 3.5 / 3.4, 4.0 / 3.6, fp8 3.1 / 2.9, 4.6 / 4.4; tiles that fill shared memory: bf16 6144 x 4096 with a norm 9.8 / 9.6, 11.5 / 11.4.
+constexpr size_t G2_TWO_SMEM = 112 * 1024;
+
+template <bool GLU, int MODE, int WT, bool WIDE = false, int CTAS = 1>
 static void launch_gemv2(const Gemv2Params& pp, cudaStream_t stream) {
-  if constexpr (!WIDE) {
+  const size_t smem = g2_fixed_smem(pp.ph.T, pp.ph.K, WT) + (size_t)pp.n_stages * G2_STAGE_BYTES;
+  const int grid = gemv2_grid(pp.ph.N, pp.ph.K, GLU, WT);
+  if constexpr (!WIDE && CTAS == 1) {
     if (pp.ph.K > G2_ROUND && (WT != 0 || pp.ph.norm_w != nullptr)) return launch_gemv2<GLU, MODE, WT, true>(pp, stream);
+    if (smem <= G2_TWO_SMEM && g2_ntiles(pp.ph.N, GLU) > grid) return launch_gemv2<GLU, MODE, WT, false, 2>(pp, stream);
   }
-  auto kern = gemv2_kernel<GLU, MODE, WT, WIDE>;
+  auto kern = gemv2_kernel<GLU, MODE, WT, WIDE, CTAS>;
   static bool configured = false;
   if (!configured) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G2_SMEM_BUDGET);
     configured = true;
   }
-  const size_t smem = g2_fixed_smem(pp.ph.T, pp.ph.K, WT) + (size_t)pp.n_stages * G2_STAGE_BYTES;
-  const int grid = gemv2_grid(pp.ph.N, pp.ph.K, GLU, WT);
   launch_pdl(kern, dim3(grid), dim3(G2_THREADS), smem, stream, pp);
 }
 
