@@ -158,11 +158,19 @@ int gemv2_pmax(int N, int K, bool glu, int wt) {
   return gemv2_grid(N, K, glu, wt) / n_tiles + 3;
 }
 
-// Registers.  With up to 112 of them the next kernel's CTAs start beside this one's, as long as shared memory holds both, and fetch their first weights: that pays where
-// the busiest CTA has a second tile to do meanwhile.  Elsewhere the 140 that the compiler takes are worth more.  us in a graph, two CTAs per SM / one, 1 and 8
-// tokens: bf16 4096 x 1024 3.2 / 3.8, 3.5 / 3.9, with a norm 3.6 / 4.0, 4.9 / 5.5; 8192 x 512 4.0 / 4.5, 4.3 / 4.5; fp8 4096 x 2048 3.7 / 4.0, 5.0 / 5.5; one tile per CTA:
-// bf16 2048 x 2048 3.5 / 3.4, 4.0 / 3.6, fp8 3.1 / 2.9, 4.6 / 4.4; tiles that fill shared memory: bf16 6144 x 4096 with a norm 9.8 / 9.6, 11.5 / 11.4.
+// Registers.  With up to 112 of them the next kernel's CTAs start beside this one's, as long as shared memory holds both, and fetch their first weights; elsewhere the
+// 140 that the compiler takes are worth more.  us in a graph, two CTAs per SM / one, 1 and 8 tokens:
+//   a second tile for the busiest CTA: bf16 4096 x 1024 3.2 / 3.8, 3.5 / 3.9, with a norm 3.6 / 4.0, 4.9 / 5.5; 8192 x 512 4.0 / 4.5, 4.3 / 4.5; fp8 4096 x 2048 3.7 / 4.0, 5.0 / 5.5
+//   a CTA on every SM: bf16 2368 x 2048 2.8 / 3.6, 3.3 / 3.9, with a norm 3.2 / 3.9, 4.9 / 5.7; fp8 2368 x 3072 with a norm 3.1 / 3.8, 5.4 / 5.9
+//   100 CTAs or more of one stage: bf16 1600 x 512 2.1 / 2.2, 2.4 / 2.5; 2048 x 512 2.4 / 2.5, 2.7 / 2.6, with a norm 2.7 / 2.7, 4.1 / 4.2; fp8 1152 x 1024 2.6 / 2.7, 3.7 / 3.9
+//   of two stages of bf16: 1600 x 1024 2.4 / 2.7 at one token, 2304 x 1024 2.7 / 2.9 at one, 2.8 / 2.9 at four, but 3.3 / 3.1 at 8
+//   neither: bf16 2048 x 2048 3.4 / 3.4, 4.0 / 3.6; 512 x 1024 2.2 / 2.1, 2.7 / 2.4; fp8 2048 x 3072 3.6 / 3.4, 6.7 / 5.7
 constexpr size_t G2_TWO_SMEM = 112 * 1024;
+static bool g2_two_ctas(const G2Phase& ph, bool glu, size_t smem, int grid) {
+  if (smem > G2_TWO_SMEM) return false;
+  const int stages = (ph.K + g2_kc(ph.wt) - 1) / g2_kc(ph.wt);      // of a tile
+  return g2_ntiles(ph.N, glu) > grid || grid == g2_num_sms() || (grid >= 100 && (stages == 1 || (stages == 2 && ph.wt == 0 && ph.T <= 4)));
+}
 
 template <bool GLU, int MODE, int WT, bool WIDE = false, int CTAS = 1>
 static void launch_gemv2(const Gemv2Params& pp, cudaStream_t stream) {
@@ -170,7 +178,7 @@ static void launch_gemv2(const Gemv2Params& pp, cudaStream_t stream) {
   const int grid = gemv2_grid(pp.ph.N, pp.ph.K, GLU, WT);
   if constexpr (!WIDE && CTAS == 1) {
     if (pp.ph.K > G2_ROUND && (WT != 0 || pp.ph.norm_w != nullptr)) return launch_gemv2<GLU, MODE, WT, true>(pp, stream);
-    if (smem <= G2_TWO_SMEM && g2_ntiles(pp.ph.N, GLU) > grid) return launch_gemv2<GLU, MODE, WT, false, 2>(pp, stream);
+    if (g2_two_ctas(pp.ph, GLU, smem, grid)) return launch_gemv2<GLU, MODE, WT, false, 2>(pp, stream);
   }
   auto kern = gemv2_kernel<GLU, MODE, WT, WIDE, CTAS>;
   static bool configured = false;
