@@ -319,8 +319,8 @@ __device__ __forceinline__ void g2_consume(const G2Phase& p, const G2Symm& sy, c
         for (int h = 0; h < R; ++h) acc[h] = warp_sum(acc[h]);
 #pragma unroll
         for (int h = 0; h < R; ++h) {
-          const uint32_t sum = rstd_u + (warp * 8 + t + h) * 4;
-          if (lane == 0) sts_f32(sum, std::is_same<decltype(first), int>::value ? lds_f32(sum) + acc[h] : acc[h]);
+          if constexpr (std::is_same<decltype(first), int>::value) acc[h] += lds_f32(rstd_u + (warp * 8 + t + h) * 4);
+          if (lane == 0) sts_f32(rstd_u + (warp * 8 + t + h) * 4, acc[h]);
         }
       }
     };
