@@ -79,7 +79,7 @@ struct GemmRsArgs {
   void* cta_counter;
 };
 void gemm_tcgen05_launch(const void* a, int lda, const void* b, const void* bias, const void* residual, void* c, int ldc, int M,
-                         int N, int K, int act, cudaStream_t stream, const GemmRsArgs* rs = nullptr, bool w_fresh = false);
+                         int N, int K, int act, cudaStream_t stream, const GemmRsArgs* rs = nullptr, bool w_fresh = false, const float* w_scale = nullptr, int w_scale_n = 0);
 // clear: n_clear words set to zero on the way (fewer than 1024 rows)
 void rmsnorm_launch(const void* x, const void* res_in, const void* w, void* y, void* res_out, int rows, int H, float eps,
                     float offset, cudaStream_t stream,
@@ -126,7 +126,7 @@ std::vector<std::pair<std::string, long long>> kernel_launches();
 // prompt-sized GEMM on CTA pairs (gemm_pair.cu); tile_expert / tile_row: grouped, m_tiles tiles of up to 256 rows of the M permuted ones (moe_plan256)
 void gemm_pair_launch(const void* a, long long lda, const void* b, const void* bias, const void* residual, void* c, int M, int N, int K, int act,
                       cudaStream_t stream, bool w_fresh = false, const int* tile_expert = nullptr, const int* tile_row = nullptr, int m_tiles = 0, int experts = 1,
-                      float limit = 7.f, float alpha = 1.702f);
+                      float limit = 7.f, float alpha = 1.702f, const float* scale = nullptr, int scale_n = 0);
 
 // few tokens x large weights with the weights streamed evenly over the SMs (skinny_gemm.cu): one weight [rows, K], or the experts that have tokens
 constexpr int SKINNY_MAX_T = 128, SKINNY8_MAX_T = 512;      // tokens of a tile; of 8-bit weights without a gate product

@@ -223,10 +223,11 @@ static bool pair_pays(int M, int n_out, bool glu) {
 
 // fresh_weight: w was written by a kernel enqueued just before (an expanded 8-bit weight).  The kernels fetch a parameter's first tiles before the
 // kernels in front of them have finished; such a weight has to be waited for.
+// w_scale: of the sums, per output channel or one (a weight expanded from bytes; not in the kernel of few tokens).
 // tcgen05 GEMM for T > 8 tokens (prefill, long speculation windows)
 static at::Tensor gemm_rows(at::Tensor x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int64_t act,
                 const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& out, bool fresh_weight, const c10::optional<at::Tensor>& norm_w, double eps,
-                double offset) {
+                double offset, const at::Tensor* w_scale = nullptr) {
   TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1));
   TORCH_CHECK(is_bf16(x) && is_bf16(w) && x.stride(1) == 1 && w.is_contiguous());
   const int M = x.size(0), K = x.size(1), N = w.size(0);
@@ -240,18 +241,20 @@ static at::Tensor gemm_rows(at::Tensor x, const at::Tensor& w, const c10::option
   auto y = out.has_value() ? *out : at::empty({M, n_out}, x.options());
   if (residual.has_value())
     TORCH_CHECK(!glu && residual->is_contiguous() && residual->size(0) == M && residual->size(1) == n_out && is_bf16(*residual));
-  if (skinny_pays(M, N, K, glu)) {
+  const float* ws = w_scale != nullptr ? w_scale->data_ptr<float>() : nullptr;
+  const int ws_n = w_scale != nullptr ? (int)w_scale->numel() : 0;
+  if (ws == nullptr && skinny_pays(M, N, K, glu)) {
     run_skinny(x, w, bias, (int)act, residual, y, fresh_weight, norm_w, eps, offset);
     return y;
   }
   if (norm_w.has_value()) x = rmsnorm_rows(x.contiguous(), *norm_w, eps, offset, nullptr, nullptr);
   if (pair_pays(M, n_out, glu)) {
     gemm_pair_launch(x.data_ptr(), x.stride(0), w.data_ptr(), optr(bias), optr(residual), y.data_ptr(), M, N, K, (int)act, cur_stream(),
-                     fresh_weight);
+                     fresh_weight, nullptr, nullptr, 0, 1, 7.f, 1.702f, ws, ws_n);
     return y;
   }
   gemm_tcgen05_launch(x.data_ptr(), (int)x.stride(0), w.data_ptr(), optr(bias), optr(residual), y.data_ptr(), n_out, M, N, K,
-                      (int)act, cur_stream(), nullptr, fresh_weight);
+                      (int)act, cur_stream(), nullptr, fresh_weight, ws, ws_n);
   return y;
 }
 
@@ -260,12 +263,31 @@ at::Tensor gemm(const at::Tensor& x, const at::Tensor& w, const c10::optional<at
   return gemm_rows(x, w, bias, act, residual, out, fresh_weight, c10::nullopt, 0., 0.);
 }
 
+static at::Tensor expand_bf16(const at::Tensor& w, const at::Tensor* scale);
 at::Tensor dequant_bf16(const at::Tensor& w, const at::Tensor& scale);
 
-// int8 / fp8 weights and 9 .. 512 tokens (64 with a gate product): the bytes are read once, by blocks of up to 128 tokens at the same time.  us, here / expanded to bf16
-// in memory first: 4096 x 4096 at 9 tokens 11 / 25, at 128 24 / 33, at 256 25 / 34, at 512 32 / 37; 4096 x 11008 at 9 17 / 48, at 37 20 / 52, at 128 30 / 58, at 256
-// 37 / 73, at 512 57 / 88; 11008 x 4096 at 47 20 / 51; 12288 x 4096 at 64 23 / 58, at 256 41 / 57, at 384 51 / 77, at 512 64 / 78.  The weight is not rounded: the
-// scale is applied to the fp32 sum.
+// Whether 8-bit weights of 9 .. 512 tokens (64 with a gate product) are read as bytes (linear8_few) or expanded to bf16 in front of a tile GEMM.  Bytes cost their
+// stream, once, and an epilogue that grows with the tokens of a block; the expansion costs a launch and two passes over bf16 weights, the tile GEMM behind it the
+// same whatever the tokens of a tile.  us in a graph, bytes / expanded (fp8):
+//   1024 x 1024: 16.3 / 13.5 at 128 tokens, 15.4 / 9.6 at 320      4096 x 1024: 16.7 / 12.0 at 128, 14.7 / 12.1 at 192, 19.7 / 14.3 at 512
+//   2048 x 1024: 12.4 / 14.8 at 65                                 8192 x 1024: 19.9 / 16.4 at 256, 26.5 / 18.9 at 512
+//   4096 x 512:  9.0 / 10.0 at 129, 10.6 / 11.7 at 320             8192 x 512:  9.3 / 12.5 at 129, 11.5 / 12.6 at 256, 20.9 / 14.5 at 320
+//   2048 x 2048: 18.7 / 15.1 at 256, 21.8 / 15.5 at 512            8192 x 2048: 25.8 / 28.3 at 257, 33.3 / 28.9 at 512
+//   512 x 2048:  14.8 / 18.6 at 257                                2048 x 3072: 16.9 / 18.6 at 129
+//   gate products: 512 x 512 8.6 / 7.3 at 33, 2048 x 1024 12.7 / 14.3 at 48, 4096 x 1024 14.2 / 12.1 at 64
+static bool linear8_bytes_pay(int64_t T, int64_t N, int64_t K, bool glu) {
+  if (K < 512) return T <= 32;
+  if (glu) return T <= 32 || K >= 2048 || (K >= 1024 ? T <= 48 || N >= 8192 : N >= 4096);
+  if (T <= 64 || K >= 4096) return true;
+  const int64_t b = (T + 127) / 128;
+  const bool low = (T + b - 1) / b <= 96;        // tokens of a block
+  if (K >= 2048) return b == 1 || (b == 2 && (low || N <= 1024)) || N <= 512 || (N >= 8192 && (b <= 3 || N * K >= (24LL << 20)));
+  if (K >= 1024) return b <= 2 && ((N >= 8192 && (b == 1 || low)) || (N <= (b == 1 ? 2048 : 1024) && low));
+  return N >= 4096 && N * T <= (2LL << 20);
+}
+
+// int8 / fp8 weights and 9 .. 512 tokens (64 with a gate product): the bytes are read once, by blocks of up to 128 tokens at the same time.  The weight is not rounded:
+// the scale is applied to the fp32 sum.
 static at::Tensor linear8_few(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias, int64_t act, const at::Tensor& scale,
                               const c10::optional<at::Tensor>& residual, const c10::optional<at::Tensor>& norm_w, double eps, double offset) {
   const int64_t M = x.size(0), N = w.size(0), n_out = act != 0 ? N / 2 : N;
@@ -295,7 +317,7 @@ std::tuple<c10::optional<at::Tensor>, int64_t> linear(const at::Tensor& x, const
   int64_t ran = 0;
   if (few && wq && K % 16 == 0) ran = LINEAR_QGEMV;
   else if (few && plain && K % 64 == 0 && (K % 256 == 0 || gemv2_supported((int)T, (int)K, 0))) ran = LINEAR_GEMV;
-  else if (!few && K % 64 == 0 && n_out % 8 == 0 && tensor_cores) ran = LINEAR_GEMM | (wq && !few8 ? LINEAR_DEQUANT : 0);
+  else if (!few && K % 64 == 0 && n_out % 8 == 0 && tensor_cores) ran = LINEAR_GEMM | (wq && !(few8 && linear8_bytes_pay(T, N, K, act != 0)) ? LINEAR_DEQUANT : 0);
   else return none;
   c10::optional<at::Tensor> norm_w;
   if (norm_in.has_value()) {
@@ -312,15 +334,20 @@ std::tuple<c10::optional<at::Tensor>, int64_t> linear(const at::Tensor& x, const
   const auto x2 = x.reshape({T, K});
   c10::optional<at::Tensor> r2, scale_f;
   if (residual.has_value() && act == 0) r2 = wq && few ? residual->reshape({T, -1}).contiguous() : residual->reshape({T, -1});
-  if (scale.has_value()) scale_f = scale->to(at::kFloat).contiguous();
+  if (scale.has_value()) {
+    scale_f = scale->to(at::kFloat).contiguous();
+    if (reinterpret_cast<uintptr_t>(scale_f->data_ptr()) % 16 != 0) scale_f = scale_f->clone();      // (a slice; the tile kernels load four at a time)
+  }
   at::Tensor y;
   if (ran & (LINEAR_QGEMV | LINEAR_GEMV)) {
     y = gemv(x2, w, bias, norm_w, eps, offset, act, scale_f, r2);
   } else {
     c10::optional<at::Tensor> o2;
     if (out.has_value()) o2 = out->view({T, -1});
-    // weight-only 8-bit layers: few tokens read the bytes (linear8_few); more, one expansion pass to bf16 (stays in L2), then the bf16 GEMM, which waits for it
-    if (few8) y = linear8_few(x2, w, bias, act, *scale_f, r2, norm_w, eps, offset);
+    // weight-only 8-bit layers: few tokens read the bytes (linear8_few) where that pays; else one expansion pass to bf16 (stays in L2), then the bf16 GEMM, which waits
+    // for it.  Up to 512 tokens (64 with a gate product) the weight is not rounded either way: its scale goes to the fp32 sum
+    if (few8 && linear8_bytes_pay(T, N, K, act != 0)) y = linear8_few(x2, w, bias, act, *scale_f, r2, norm_w, eps, offset);
+    else if (few8) y = gemm_rows(x2.contiguous(), expand_bf16(w, nullptr), bias, act, r2, o2, true, norm_w, eps, offset, &*scale_f);
     else y = gemm_rows(x2.contiguous(), wq ? dequant_bf16(w, *scale_f) : w, bias, act, r2, o2, wq, norm_w, eps, offset);
   }
   if ((ran & LINEAR_GEMM) && out.has_value()) {
@@ -447,16 +474,19 @@ at::Tensor moe_small(const at::Tensor& x, const at::Tensor& w_gate_up, const at:
 
 // int8 / fp8 weight [N, K] x scale -> bf16.  A result per call: two streams may expand weights at the same time, and the stream order of the caching
 // allocator hands the same memory to the next layer
-at::Tensor dequant_bf16(const at::Tensor& w, const at::Tensor& scale) {
-  TORCH_CHECK(w.is_cuda() && w.dim() == 2 && w.is_contiguous() && scale.scalar_type() == at::kFloat && scale.is_contiguous());
+static at::Tensor expand_bf16(const at::Tensor& w, const at::Tensor* scale) {
+  TORCH_CHECK(w.is_cuda() && w.dim() == 2 && w.is_contiguous());
   const bool i8 = w.scalar_type() == at::kChar;
   TORCH_CHECK(i8 || w.scalar_type() == at::kFloat8_e4m3fn, "dequant_bf16: int8 or float8_e4m3fn weights");
-  TORCH_CHECK(scale.numel() == 1 || scale.numel() == w.size(0));
   c10::cuda::CUDAGuard guard(w.device());
   auto out = at::empty({w.size(0), w.size(1)}, w.options().dtype(at::kBFloat16));
-  dequant_bf16_launch(w.data_ptr(), i8 ? 1 : 2, scale.data_ptr<float>(), (int)scale.numel(), out.data_ptr(), (int)w.size(0), (int)w.size(1),
-                      cur_stream());
+  dequant_bf16_launch(w.data_ptr(), i8 ? 1 : 2, scale != nullptr ? scale->data_ptr<float>() : nullptr, scale != nullptr ? (int)scale->numel() : 0, out.data_ptr(),
+                      (int)w.size(0), (int)w.size(1), cur_stream());
   return out;
+}
+at::Tensor dequant_bf16(const at::Tensor& w, const at::Tensor& scale) {
+  TORCH_CHECK(scale.is_cuda() && scale.scalar_type() == at::kFloat && scale.is_contiguous() && (scale.numel() == 1 || scale.numel() == w.size(0)));
+  return expand_bf16(w, &scale);
 }
 
 // Routed experts of a prefill-sized batch (any N): permutation on the device + two grouped tcgen05 GEMMs + weighted combine.

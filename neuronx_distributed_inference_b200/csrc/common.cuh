@@ -174,4 +174,15 @@ template <typename... KArgs, typename... Args>
 inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   launch_pdl_cluster(kernel, 1, grid, block, smem, stream, std::forward<Args>(args)...);
 }
+// scales of 32 output columns from col0 on (n_out % 8 == 0, 16-byte aligned), or the one of all: their loads side by side
+__device__ __forceinline__ void load_scales(const float* scale, bool one, int col0, int n_out, float (&s)[32]) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 4) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (one) v.x = v.y = v.z = v.w = __ldg(scale);
+    else if (col0 + j < n_out) v = __ldg(reinterpret_cast<const float4*>(scale + col0 + j));
+    s[j] = v.x; s[j + 1] = v.y; s[j + 2] = v.z; s[j + 3] = v.w;
+  }
+}
+
 }  // namespace nxdi

@@ -39,6 +39,8 @@ struct PairParams {
   __nv_bfloat16* c;               // [M, n_out]
   int M, N, K, n_out, act;        // act: 0 none, 1 silu*up, 2 gelu_tanh*up, 3 gelu*up, 4 clamped gate product (n_out = N / 2)
   float limit, alpha;
+  const float* scale;             // SCALED: of the sums, [N], or [1] (scale_one)
+  int scale_one;
   int m_tiles, n_tiles, band;
   int w_fresh;                    // B was written by a kernel just before this one
   unsigned* wait_word;            // mbar_wait.cuh
@@ -100,6 +102,8 @@ __device__ __forceinline__ void gp_tile(const PairParams& p, int t, int& mt, int
   nt = r / rows;
 }
 
+// SCALED: of a weight that was expanded from bytes without its scale
+template <bool SCALED>
 __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_constant__ PairParams p) {
   constexpr int BN = GP_BN, ST = GP_STAGES, STAGE = GP_STAGE;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -266,6 +270,11 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
         if (p.residual != nullptr) move_rows(row0, row_end, col_t + c0, true);
 #pragma unroll 1
         for (int c = c0; c < c0 + 64; c += 32) {
+          float sg[32], su[32];      // SCALED: loaded in front of the sums
+          if (SCALED) {
+            load_scales(p.scale, p.scale_one != 0, col_t + c, p.n_out, sg);
+            if (glu) load_scales(p.scale + (p.scale_one ? 0 : p.n_out), p.scale_one != 0, col_t + c, p.n_out, su);
+          }
           uint32_t vg[32], vu[32];
           gp_ld32(acc + c, vg);
           if (glu) gp_ld32(acc + BN / 2 + c, vu);
@@ -278,6 +287,10 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
             float f[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) f[k] = __uint_as_float(vg[j + k]);
+            if (SCALED) {
+#pragma unroll
+              for (int k = 0; k < 8; ++k) f[k] *= sg[j + k];
+            }
             if (p.bias != nullptr) {
 #pragma unroll
               for (int k = 0; k < 8; ++k) f[k] += __bfloat162float(p.bias[eo + col0 + j + k]);
@@ -286,6 +299,10 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
               float up[8];
 #pragma unroll
               for (int k = 0; k < 8; ++k) up[k] = __uint_as_float(vu[j + k]);
+              if (SCALED) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) up[k] *= su[j + k];
+              }
               if (p.bias != nullptr) {
 #pragma unroll
                 for (int k = 0; k < 8; ++k) up[k] += __bfloat162float(p.bias[eo + p.n_out + col0 + j + k]);
@@ -363,13 +380,15 @@ static int gp_sms() {
 
 // a [M, K] (row stride lda), b [experts * N, K], c [M, n_out]; tile_expert / tile_row (device, [m_tiles]) for the grouped flavour
 void gemm_pair_launch(const void* a, long long lda, const void* b, const void* bias, const void* residual, void* c, int M, int N, int K, int act,
-                      cudaStream_t stream, bool w_fresh, const int* tile_expert, const int* tile_row, int m_tiles, int experts, float limit, float alpha) {
+                      cudaStream_t stream, bool w_fresh, const int* tile_expert, const int* tile_row, int m_tiles, int experts, float limit, float alpha,
+                      const float* scale, int scale_n) {
   if (K % GP_BK != 0 || M < 1) throw std::runtime_error("gemm pair: K must be a multiple of 64");
   PairParams p{};
   const bool glu = act != 0;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   p.c = reinterpret_cast<__nv_bfloat16*>(c);
+  p.scale = scale; p.scale_one = scale_n == 1 ? 1 : 0;
   p.M = M; p.N = N; p.K = K; p.act = act; p.n_out = glu ? N / 2 : N; p.limit = limit; p.alpha = alpha;
   check_waits();
   p.wait_word = wait_word(WAIT_GEMM_PAIR);
@@ -381,7 +400,8 @@ void gemm_pair_launch(const void* a, long long lda, const void* b, const void* b
   p.band = tile_expert == nullptr ? p.m_tiles : std::min(4, p.m_tiles);
   gp_map(&p.tma_a, a, M, K, lda, 128);
   gp_map(&p.tma_b, b, (long long)experts * N, K, K, GP_BN / 2);
-  if (cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM) != cudaSuccess)
+  auto kernel = scale != nullptr ? gemm_pair_kernel<true> : gemm_pair_kernel<false>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM) != cudaSuccess)
     throw std::runtime_error("gemm pair: shared memory size refused");
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2 * std::min(gp_sms() / 2, p.m_tiles * p.n_tiles));
@@ -397,7 +417,7 @@ void gemm_pair_launch(const void* a, long long lda, const void* b, const void* b
   attr[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel, p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
   if (e != cudaSuccess) throw std::runtime_error(std::string("gemm pair launch failed: ") + cudaGetErrorString(e));
 }
 

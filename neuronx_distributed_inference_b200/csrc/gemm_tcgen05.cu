@@ -40,7 +40,7 @@ struct GemmParams {
   // fp8 (e4m3 x e4m3 -> fp32, tcgen05 kind::f8f6f4): acc * a_scale[row] * w_scale[col] (dynamic per-token activation scale,
   // per-output-channel or per-tensor weight scale); null for bf16
   const float* a_scale;
-  const float* w_scale;
+  const float* w_scale;      // (bf16: of a weight that was expanded from bytes without its scale, or null)
   int w_scale_n;
   int splits;                     // split-K factor: work item = (tile, k slice); partial accumulators meet in `ws`
   float* ws;                      // [tiles][splits][TM*128][128] fp32 partials (L2 resident)
@@ -154,7 +154,7 @@ __device__ __forceinline__ void mb_arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s_u32(b)) : "memory");
 }
 
-template <int TM, int BN, bool FP8>
+template <int TM, int BN, bool FP8, bool SCALED = false>
 __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   constexpr int B_BYTES = BN * GM_BK * 2;
   constexpr int STAGE_BYTES = TM * GM_A_BYTES + B_BYTES;
@@ -296,6 +296,13 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tcgen05_kernel(const __gri
     const int q = warp & 3;                 // TMEM lane quarter this warp may access
     const int etid = threadIdx.x - 128;     // 0..127 inside the epilogue group
     const int n_out = glu ? (p.N >> 1) : p.N;
+    // SCALED (a weight that was expanded from bytes without its scale): scales of the next 32 columns, loaded in front of their sums
+    float xs_g[32], xs_u[32];
+    auto load_sc = [&](int col0) {
+      if (!SCALED) return;
+      load_scales(p.w_scale, p.w_scale_n == 1, col0, n_out, xs_g);
+      if (glu) load_scales(p.w_scale + (p.w_scale_n == 1 ? 0 : n_out), p.w_scale_n == 1, col0, n_out, xs_u);
+    };
     // final math + store of 32 accumulator columns [c0, c0+32) of one row (GLU: gate chunk + matching up chunk)
     int cur_eo = 0;   // grouped: offset of the current tile's expert inside bias / w_scale ([E][N])
     auto store_chunk = [&](int row, int n_out0, int c0, const uint32_t (&vg)[32], const uint32_t (&vu)[32]) {
@@ -346,6 +353,13 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tcgen05_kernel(const __gri
           if (FP8) {
             f[e] *= sc_g[j + e];
             up[e] *= sc_u[j + e];
+          }
+        }
+        if (SCALED) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            f[e] *= xs_g[j + e];
+            up[e] *= xs_u[j + e];
           }
         }
         if (p.bias) {
@@ -418,6 +432,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tcgen05_kernel(const __gri
         } else {
 #pragma unroll 1
           for (int c0 = 0; c0 < half; c0 += 32) {
+            load_sc(n_out0 + c0);
             uint32_t vg[32], vu[32];
             tmem_ld32(lane_addr + c0, vg);
             if (glu) tmem_ld32(lane_addr + BN / 2 + c0, vu);
@@ -459,6 +474,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tcgen05_kernel(const __gri
             const int r_in = sub * GM_BM + q * 32 + lane;
 #pragma unroll 1
             for (int c0 = 0; c0 < half; c0 += 32) {
+              load_sc(n_out0 + c0);
               uint32_t vg[32], vu[32];
 #pragma unroll
               for (int j = 0; j < 32; ++j) vg[j] = vu[j] = 0u;
@@ -751,14 +767,11 @@ static void gemm_launch_impl(const void* a, int lda, const void* b, const void* 
   static bool configured = false;
   if (!configured) {
     const int max_smem = GM_STAGES * (2 * GM_A_BYTES + 128 * GM_BK * 2) + 256 + 1024;   // == 1 x A + 256-row B
-    cudaFuncSetAttribute(gemm_tcgen05_kernel<1, 128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    cudaFuncSetAttribute(gemm_tcgen05_kernel<2, 128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    cudaFuncSetAttribute(gemm_tcgen05_kernel<1, 256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    cudaFuncSetAttribute(gemm_tcgen05_kernel<1, 64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    cudaFuncSetAttribute(gemm_tcgen05_kernel<1, 128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    cudaFuncSetAttribute(gemm_tcgen05_kernel<2, 128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    cudaFuncSetAttribute(gemm_tcgen05_kernel<1, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    cudaFuncSetAttribute(gemm_tcgen05_kernel<1, 64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+    auto allow = [&](auto kernel) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem); };
+    allow(gemm_tcgen05_kernel<1, 128, false>); allow(gemm_tcgen05_kernel<2, 128, false>); allow(gemm_tcgen05_kernel<1, 256, false>); allow(gemm_tcgen05_kernel<1, 64, false>);
+    allow(gemm_tcgen05_kernel<1, 128, true>); allow(gemm_tcgen05_kernel<2, 128, true>); allow(gemm_tcgen05_kernel<1, 256, true>); allow(gemm_tcgen05_kernel<1, 64, true>);
+    allow(gemm_tcgen05_kernel<1, 128, false, true>); allow(gemm_tcgen05_kernel<2, 128, false, true>); allow(gemm_tcgen05_kernel<1, 256, false, true>);
+    allow(gemm_tcgen05_kernel<1, 64, false, true>);
     configured = true;
   }
   const int grid = std::min(n_sms, p.m_tiles * p.n_tiles * p.splits);
@@ -769,6 +782,11 @@ static void gemm_launch_impl(const void* a, int lda, const void* b, const void* 
     else if (BN == 256) launch_pdl(gemm_tcgen05_kernel<1, 256, true>, g, b3, smem, stream, p);
     else if (BN == 64) launch_pdl(gemm_tcgen05_kernel<1, 64, true>, g, b3, smem, stream, p);
     else launch_pdl(gemm_tcgen05_kernel<1, 128, true>, g, b3, smem, stream, p);
+  } else if (w_scale != nullptr) {
+    if (TM == 2) launch_pdl(gemm_tcgen05_kernel<2, 128, false, true>, g, b3, smem, stream, p);
+    else if (BN == 256) launch_pdl(gemm_tcgen05_kernel<1, 256, false, true>, g, b3, smem, stream, p);
+    else if (BN == 64) launch_pdl(gemm_tcgen05_kernel<1, 64, false, true>, g, b3, smem, stream, p);
+    else launch_pdl(gemm_tcgen05_kernel<1, 128, false, true>, g, b3, smem, stream, p);
   } else {
     if (TM == 2) launch_pdl(gemm_tcgen05_kernel<2, 128, false>, g, b3, smem, stream, p);
     else if (BN == 256) launch_pdl(gemm_tcgen05_kernel<1, 256, false>, g, b3, smem, stream, p);
@@ -778,8 +796,8 @@ static void gemm_launch_impl(const void* a, int lda, const void* b, const void* 
 }
 
 void gemm_tcgen05_launch(const void* a, int lda, const void* b, const void* bias, const void* residual, void* c, int ldc, int M,
-                         int N, int K, int act, cudaStream_t stream, const GemmRsArgs* rs, bool w_fresh) {
-  gemm_launch_impl(a, lda, b, bias, residual, c, ldc, M, N, K, act, stream, rs, nullptr, nullptr, 0, nullptr, 1, 7.f, 1.702f, w_fresh);
+                         int N, int K, int act, cudaStream_t stream, const GemmRsArgs* rs, bool w_fresh, const float* w_scale, int w_scale_n) {
+  gemm_launch_impl(a, lda, b, bias, residual, c, ldc, M, N, K, act, stream, rs, nullptr, w_scale, w_scale_n, nullptr, 1, 7.f, 1.702f, w_fresh);
 }
 
 // grouped GEMM of the mixture-of-experts layers: a [R, K] tokens permuted by expert (R % 128 == 0), b [E, N, K] stacked expert
@@ -788,7 +806,7 @@ void gemm_grouped_launch(const void* a, const void* b, const void* bias, void* c
                          const int* tile_expert, const float* a_scale, const float* w_scale, cudaStream_t stream, float glu_limit, float glu_alpha) {
   if (K % (a_scale ? 128 : 64) != 0) throw std::runtime_error("grouped gemm: K must be a multiple of 64 (128 for fp8)");
   const int n_out = act ? N / 2 : N;
-  gemm_launch_impl(a, K, b, bias, nullptr, c, n_out, R, N, K, act, stream, nullptr, a_scale, w_scale, a_scale ? N : 0, tile_expert,
+  gemm_launch_impl(a, K, b, bias, nullptr, c, n_out, R, N, K, act, stream, nullptr, a_scale, a_scale ? w_scale : nullptr, a_scale ? N : 0, tile_expert,
                    n_experts, glu_limit, glu_alpha);
 }
 

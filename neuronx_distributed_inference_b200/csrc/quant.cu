@@ -97,9 +97,10 @@ void rmsnorm_quant_launch(const void* x, const void* gamma, void* q, float* scal
              reinterpret_cast<const __nv_bfloat16*>(gamma), reinterpret_cast<uint8_t*>(q), scale, H, eps, offset, clamp);
 }
 
-// Weight-only 8-bit layers above 512 tokens (64 with a gate product; fewer read the bytes) without activation quantisation: expand W (int8 / fp8-e4m3, per-channel or per-tensor
-// scale) to bf16 ONCE per call into a scratch buffer (1 B read + 2 B written per weight; the copy is consumed from L2 by the
-// tcgen05 GEMM that follows, which therefore waits for it before its first weight tile: `fresh_weight`) instead of the three elementwise passes of the PyTorch composite.
+// Weight-only 8-bit layers that do not read the bytes (linear8_bytes_pay in bindings.cpp, and all above 512 tokens, 64 with a gate product): expand W (int8 / fp8-e4m3,
+// per-channel or per-tensor scale, or without one, exactly) to bf16 ONCE per call into a scratch buffer (1 B read + 2 B written per weight; the copy is consumed
+// from L2 by the tcgen05 GEMM that follows, which therefore waits for it before its first weight tile: `fresh_weight`) instead of the three elementwise passes of
+// the PyTorch composite.
 template <int WT>
 __global__ void __launch_bounds__(256) dequant_bf16_kernel(const uint8_t* __restrict__ w, const float* __restrict__ scale, int scale_n,
                                                            __nv_bfloat16* __restrict__ out, int N, int K) {
@@ -109,7 +110,7 @@ __global__ void __launch_bounds__(256) dequant_bf16_kernel(const uint8_t* __rest
   const long long total = (long long)N * kv;
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
     const int n = (int)(i / kv);
-    const float sc = scale[scale_n == 1 ? 0 : n];
+    const float sc = scale == nullptr ? 1.f : scale[scale_n == 1 ? 0 : n];
     const uint4 q = ldg_stream(reinterpret_cast<const uint4*>(w) + i);
     const uint32_t words[4] = {q.x, q.y, q.z, q.w};
     uint32_t o[8];

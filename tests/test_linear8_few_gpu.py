@@ -93,3 +93,29 @@ def test_rows_of_a_step_do_not_depend_on_their_number(wdtype, K, norm):
     one = torch.cat([ops.linear(x[t:t + 1], w, norm_weight=n, scale=s) for t in range(8)])
     for T in range(1, 9):
         assert torch.equal(ops.linear(x[:T], w, norm_weight=n, scale=s), one[:T])
+
+
+@pytest.mark.parametrize("wdtype", TYPES)
+@pytest.mark.parametrize("T,N,K", [(65, 512, 512), (128, 4096, 1024), (129, 1000, 384), (200, 8192, 1024), (257, 2048, 2048), (300, 8200, 512), (512, 136, 256), (512, 16384, 1024)])
+def test_expanded_weights_are_not_rounded(wdtype, T, N, K):
+    """Sizes whose bytes are expanded in memory first (both tile kernels, cut tiles): the scale goes to the sum, so only the result is rounded (1.7e-3 rms; 2.4e-3
+    with a rounded weight)."""
+    q, s = ref.quantize_per_channel(torch.randn(N, K, device=DEV) / K ** 0.5, wdtype)
+    x, b, r = torch.randn(T, K, device=DEV, dtype=BF), torch.randn(N, device=DEV, dtype=BF), torch.randn(T, N, device=DEV, dtype=BF)
+    before = dict(ops.stats)
+    assert _rel(ops.linear(x, q, scale=s), _want(x, q, s)) < 1.9e-3
+    assert ops.stats["dequant_gemm"] == before["dequant_gemm"] + 1
+    assert _rel(ops.linear(x, q, b, scale=s, residual=r), _want(x, q, s, b) + r.double()) < 3e-3
+    assert _rel(ops.linear(x, q, scale=s.view(-1)[:1].contiguous()), _want(x, q, s.view(-1)[:1])) < 1.9e-3
+
+
+@pytest.mark.parametrize("wdtype", TYPES)
+@pytest.mark.parametrize("T,I,K", [(33, 72, 128), (64, 500 * 8, 256), (64, 1024, 1024)])
+def test_expanded_weights_with_a_gate_product(wdtype, T, I, K):
+    q, s = ref.quantize_per_channel(torch.randn(2 * I, K, device=DEV) / K ** 0.5, wdtype)
+    x, b = torch.randn(T, K, device=DEV, dtype=BF), torch.randn(2 * I, device=DEV, dtype=BF)
+    before = dict(ops.stats)
+    for act in ("silu_mul", "gelu_mul"):
+        assert _rel(ops.linear(x, q, b, scale=s, act=act), _want(x, q, s, b, act)) < 3e-3
+        assert _rel(ops.linear(x, q, scale=s.view(-1)[:1].contiguous(), act=act), _want(x, q, s.view(-1)[:1], None, act)) < 3e-3
+    assert ops.stats["dequant_gemm"] == before["dequant_gemm"] + 4
