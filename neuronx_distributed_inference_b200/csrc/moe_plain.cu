@@ -285,7 +285,9 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const T* __restrict_
 // Here KW warps share the columns of four experts, read the rows and the weights straight from memory (no staging, no barrier in the loop) and their sums are added in
 // order at the end; a block takes 32 / KW experts.  Bound by the latency of a few rounds of loads.  us in a graph, logits and choice together, here / a block per 4 tokens
 // with two or four warps per four experts (8, 16 experts) or staged rows: 8 experts of 4096 columns at 6, 100 tokens 5.2 / 7.4, 6.4 / 8.2; 16 of 6144 at 6, 179
-// 6.4 / 13.9, 8.8 / 15.3; 128 of 2048 at 9, 48, 179 7.9 / 14.6, 9.7 / 16.3, 15.1 / 16.5 (255: 18.1 / 16.5); 256 of 4096 at 9, 100, 179 11.5 / 22.4, 23 / 26, 34 / 31.
+// 6.4 / 13.9, 8.8 / 15.3; 128 of 2048 at 9, 48, 179 7.9 / 14.6, 9.7 / 16.3, 15.1 / 16.5; 256 of 4096 at 9, 100, 179 11.5 / 22.4, 23 / 26, 34 / 31.  Its blocks read every
+// weight once for four tokens, so staged rows win from about 5000 + 8 W tokens times experts: 128 of 2048 at 200 20.5 / 17.8, 384 of 1024 at 64 25.6 / 19.7, 128 of 1024 at
+// 100 11.5 / 13.6, at 128 16.2 / 13.7.  A token a block up to 32 tokens and 10000 of that product: 512 of 4096 at 32 38.9 so, 27.6 with four tokens a block, 34.1 staged.
 // Half a microsecond to 1.5 of that come from launching both kernels before the one in front has ended.
 constexpr int RS_EG = 4;
 // EARLY: launched before the kernel in front has ended (the rows then come past L1); with many tokens the rows' lines in L1 are worth more
@@ -473,11 +475,11 @@ void router_topk_launch(const void* x, const float* w, float* logits, float* par
   if (kparts > 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
     n_parts = kparts - 1;
     router_logits_tc_launch(x, w, logits, parts, N, W, E, kparts, st);
-  } else if ((E <= 16 || (N < 256 && (long long)N * E <= 26000)) && W % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
+  } else if ((E <= 16 || (N < 256 && (long long)N * E <= std::min(26000, 5000 + 8 * W))) && W % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
     // tokens per block: one for a few tokens; then four, and eight (half the weight reads) once four would give every SM eight blocks.  Eight warps per four experts
     // as long as that takes no more than two blocks per SM
-    const bool early = N < 256;
-    const int srt = few ? 1 : N <= 4 * 8 * kNumSMs ? 4 : 8;
+    const bool early = N < 256, one = few && N * E <= 10000;
+    const int srt = one ? 1 : N <= 4 * 8 * kNumSMs ? 4 : 8;
     const long long blocks = (N + srt - 1) / srt;
     auto split = [&](auto kernel, int kw, auto xp) {
       const dim3 grid((unsigned)blocks, (E + 8 / kw * RS_EG - 1) / (8 / kw * RS_EG));
@@ -488,7 +490,7 @@ void router_topk_launch(const void* x, const float* w, float* logits, float* par
       using X = std::remove_cv_t<std::remove_pointer_t<decltype(xp)>>;
       if (early) {
         const bool wide = blocks * ((E + RS_EG - 1) / RS_EG) <= 2 * kNumSMs;
-        if (few) wide ? split(router_logits_split_kernel<X, 1, 8, true>, 8, xp) : split(router_logits_split_kernel<X, 1, 4, true>, 4, xp);
+        if (one) wide ? split(router_logits_split_kernel<X, 1, 8, true>, 8, xp) : split(router_logits_split_kernel<X, 1, 4, true>, 4, xp);
         else wide ? split(router_logits_split_kernel<X, 4, 8, true>, 8, xp) : split(router_logits_split_kernel<X, 4, 4, true>, 4, xp);
       } else if (E <= 8) {
         srt == 4 ? split(router_logits_split_kernel<X, 4, 4, false>, 4, xp) : split(router_logits_split_kernel<X, 8, 4, false>, 4, xp);

@@ -68,3 +68,10 @@ def test_split_columns(N, E, W, k, dtype):
         top = p.gather(1, ti.long())
         assert torch.allclose(top.sort(-1, descending=True).values, p.topk(k, -1).values, rtol=1e-5)
         assert torch.allclose(tw.double(), top / top.sum(-1, keepdim=True), rtol=1e-5)
+
+
+@pytest.mark.parametrize("N,E,W", [(19, 512, 2048), (20, 512, 2048), (32, 512, 4096), (32, 384, 2052), (25, 400, 2880), (13, 512, 1024), (26, 512, 1024), (64, 206, 1024), (65, 206, 1024)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_split_columns_at_the_limits(N, E, W, dtype):
+    """One or four tokens a block up to 32 tokens, and the last sizes before staged rows (tokens x experts up to 5000 + 8 W)."""
+    test_split_columns(N, E, W, 8, dtype)
