@@ -606,8 +606,9 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
     };
     // Soft cap, tiles with scores beyond the cap and CTAs of few key tiles: 64 or 32 keys at a time, the scores read from TMEM twice, in loops that are not unrolled
     // (the same bits).  Slower per tile once `tile` is in the instruction cache (254 against 207 us for the three portions named above), but a tenth of its code: four
-    // portions of up to 287 tokens with a window of 500 38 us, 44 with `tile`; where an SM has one CTA alone (20 tokens: 16 CTAs) 27 and 25.  Scores up to twice
-    // the cap: 323 us, 1156 with a tanhf behind a branch for each of them in `tile`.
+    // portions of up to 287 tokens with a window of 500 38 us, 44 with `tile`; where an SM has one CTA alone (20 tokens: 16 CTAs) 27 and 25.  A window of up to a tile
+    // leaves a warp two of six halves that it sees, and `tile` skips the others: 4 x 1024 tokens of head size 64, window 128, 45 us, 52 here (192: 59 and 57).
+    // Scores up to twice the cap: 323 us, 1156 with a tanhf behind a branch for each of them in `tile`.
     auto capped_tile = [&](int i, int key0) {
       const float scl = p.softcap * FA_LOG2E;
       auto visible = [&](int k0) {                       // which of 32 keys this row sees
@@ -703,7 +704,8 @@ __global__ void __launch_bounds__(FaShape<D, NX>::THREADS, 3 - NX) attention_pre
       }
       l_run = fmaf(l_run, alpha, (ls[0] + ls[2]) + (ls[1] + ls[3]));
     };
-    bool large = n_tiles <= FA_SHORT && gridDim.x > kNumSMs;      // or a tile of this warp had scores beyond the cap: no more tries
+    // (a choice for the whole launch, but for the row's number of tiles: CTAs of both kinds on an SM fetch both codes)
+    bool large = n_tiles <= FA_SHORT && !(p.window > 0 && p.window <= FA_ROWS) && gridDim.x > kNumSMs;      // or a tile of this warp had scores beyond the cap: no more tries
     for (int i = 0; i < n_tiles; ++i) {
       const int key0 = key_at(i);
       if (!mbar_wait_warp(&s_full[x], (uint32_t)(i & 1), stop, p.wait_word)) break;
