@@ -116,13 +116,16 @@ static void check_gemv_inputs(const at::Tensor& x, const at::Tensor& w) {
 //   plain 4096 x 14336:   25 / 50, 26 / 50, 28 / 51, 29 / 51, 35 / 52     12288 x 4096: 21 / 28, 22 / 29, 26 / 29, 27 / 29, 33 / 30 (80 tokens 29 / 30, 96 31 / 30)
 //          4096 x 4096:   12 / 21, 13 / 21, 15 / 21, 15 / 21, 20 / 22      6144 x 4096: 14 / 21, 15 / 22, 17 / 22, 17 / 22, 22 / 22
 //          2048 x 2048:    8 / 15,  8 / 14, 10 / 14, 10 / 14, 14 / 14      4096 x 1024:  8 / 8,   8 / 8,  10 / 8,  10 / 7,  13 / 8
+//   at 65, 80 and 128:    8192 x 2048: 15 / 12, 15 / 12, 17 / 12    17280 x 3200: 28 / 24, 28 / 24, ..    3200 x 3200: 14 / 17, 15 / 17, 19 / 17
+//   gate|up at 33 and 64: 2048 x 4096: 18 / 16, 22 / 16    1024 x 7168: 23 / 18, 28 / 18    2048 x 5120: 21 / 17, 25 / 17
 // A feature's tokens are in one lane, so its epilogue and the fix-up of the cut tiles grow with the tokens, twice as fast with a gate product, while the tile kernel's
-// time does not change up to 128; deep K leaves the tile kernel few tiles.  Between other kernels it gains what it prefetches: a whole gated MLP at 37 tokens takes
-// 78.1 / 79.7 us with 28672 x 4096 and 63.6 / 65.1 with 22016 x 4096.
+// time does not change up to 128; deep K leaves the tile kernel few tiles.  Between other kernels it gains what it prefetches: a whole gated MLP takes 75.0 / 74.9 us at 33
+// tokens, 75.9 / 75.2 at 40 with 28672 x 4096 and 62.8 / 63.9, 63.2 / 64.1 with 22016 x 4096.  The line at 40 tokens is the break-even of these two.  Gate products of
+// 16384 x 4096 stay here up to 64 tokens, where the tiles have been ahead since their MMA warp issues from uniform code (31 / 29 at 33, 33 / 29 at 64).
 static bool skinny_pays(int M, int rows, int K, bool glu) {
   const long long size = (long long)rows * K;
-  if (glu) return M <= 32 || (M <= 40 && size >= (64LL << 20)) || (M <= 64 && rows <= 16384 && K >= 4096);
-  return M <= 64 || (M <= SKINNY_MAX_T && (K >= 2 * rows || (size >= (8LL << 20) && (M <= 80 || size < (32LL << 20)))));
+  if (glu) return M <= 32 || (M <= 40 && size >= (64LL << 20)) || (M <= 64 && rows <= 16384 && K >= (rows >= 4096 ? 4096 : 8192));
+  return M <= 64 || (M <= SKINNY_MAX_T && (K >= 2 * rows || (K >= 4096 && size >= (8LL << 20) && (M <= 80 || size < (32LL << 20))) || (K >= 3072 && rows <= 8192 && M <= 80)));
 }
 
 // norm_w: x is normalised first; its kernel clears the GEMM's tickets, which else takes a launch of its own (1.5 us in the stream)
