@@ -459,22 +459,24 @@ def _expert_ids(ids):
 
 
 _MOE_GROUPED = os.environ.get("NXDI_B200_MOE_GROUPED", "1") == "1"
-# measured (us, rows kernel / small-step path): 128 experts, 8 chosen, 2048 x 768: 26 / 36, 37 / 57, 80 / 74, 137 / 105 at 1, 2, 4, 8 tokens; 8 experts, 2 chosen,
-# 4096 x 14336: 132 / 139, 222 / 185 and 697 / 386 at 1, 2 and 8.  Against the CTA-pair path at 12, 48 and 128 tokens: 147 / 129, 259 / 210, 271 / 219 and
-# 539 / 436, 568 / 461, 587 / 481; 16 experts, 4 chosen, 6144 x 1344: 254 / 186, 190 / 163, 201 / 175 at 16, 48 and 128
+# us in a graph, rows kernel / every chosen expert once, at 1, 2, 3, 4 and 8 tokens: 128 experts, 8 chosen, 2048 x 768: 19 / 34, 31 / 45, 43 / 57, 56 / 67, 99 / 101; 16, 4,
+# 6144 x 1344: 42 / 53, 68 / 77, 89 / 90, 114 / 107, 194 / 134; 8, 2, 4096 x 14336: 117 / 127, 210 / 207, 299 / 270, 384 / 324, 732 / 379.  (The line at two tokens is older
+# than the rows kernel of these figures, which wins at 3 and 4 tokens of the smallest experts too.)  Once / the CTA-pair path at 12, 48 and 128 tokens, as first
+# measured: 129 / 147, 210 / 259, 219 / 271 and 436 / 539, 461 / 568, 481 / 587; 16 experts, 4 chosen, 6144 x 1344: 186 / 254, 163 / 190, 175 / 201 at 16, 48 and 128
 _MOE_ROWS_TOKENS, _MOE_SMALL_TOKENS = 2, 128
 
 
 def _rows_kernel_tokens(w_gate_up) -> int:
-    """Up to how many tokens a warp per weight row and (token, slot) pair beats reading every chosen expert once (us in a graph, rows / once: 2 tokens of 2 in 8
-    4096 x 14336 218 / 205, 4096 x 7168 119 / 120, 6144 x 4096 100 / 105, 4 in 16 6144 x 1344 79 / 92; 1 token of 4096 x 14336 128 / 137, 6144 x 1344 53 / 68)."""
+    """Up to how many tokens a warp per weight row and (token, slot) pair beats reading every chosen expert once: two, one from 2^26 gate and up weights on, where two
+    tokens that share an expert count (us in a graph, rows / once, 2 tokens of 2 in 8: 4096 x 14336 210 / 207, 4096 x 7168 110 / 107, 6144 x 4096 93 / 96)."""
     return _MOE_ROWS_TOKENS if w_gate_up.shape[1] * w_gate_up.shape[2] < 1 << 26 else 1
 
 
 def _few_rows_of_large_experts(entries: int, w_gate_up) -> bool:
     """Steps of more than 128 tokens whose experts still wait for their weights: segments of up to 128 rows against 256-row tiles (us, segments / tiles; 8 experts of
     4096 x 14336, 2 chosen: 480 / 560 at 150 and 192 tokens, 592 / 611 at 300, 774 / 629 at 512; 16 of 6144 x 1344, 4 chosen: 190 / 225 at 192, 243 / 240 at 400; 128 of
-    2048 x 768, 8 chosen: 250 / 272 at 129, 274 / 278 at 300, 286 / 284 at 512).  Small experts stay where they are."""
+    2048 x 768, 8 chosen: 216 / 255 at 129, 263 / 248 at 200, 244 / 255 at 300, 286 / 284 at 512; 64 of 1024 x 512, 4 chosen: 53 / 56 at 129, 57 / 58 at 300; 32 of
+    2048 x 256: 41 / 43 and 49 / 46).  Below 2^20 gate and up weights an expert the two are within 5 % (64 of 1024 x 256: 40 / 41, 42 / 42)."""
     E, rows, H = w_gate_up.shape
     return entries <= min(48 * E, 2560) and rows * H >= 1 << 20
 
