@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Headline benchmark: Llama-3.1-8B (32 layers, bf16, random-init weights, synthetic prompts) decode
 tokens/s and p50 TTFT at TP = --gpus on one B200 box, batch 2, 128-token prompt -> 128 generated tokens
-(the shape of the reference's Llama-3.1-8B CI perf test, BASELINE.md; the reference quotes a 4-layer
+(the shape of the reference's Llama-3.1-8B CI perf test; the reference quotes a 4-layer
 truncation at TP=32 on Trn1 — that config is reproduced too and reported under ``ci_4layer``).
 
     python bench.py --gpus 1 --steps 128 --warmup 8
@@ -22,7 +22,7 @@ import time
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-BASELINE_TOK_S = 1665.0   # reference Llama-3.1-8B(4-layer) Trn1 TP=32 e2e throughput (BASELINE.md)
+BASELINE_TOK_S = 1665.0   # reference Llama-3.1-8B(4-layer) Trn1 TP=32 e2e throughput
 BASELINE_E2E_MS = 306.0
 
 LLAMA31_8B = dict(hidden_size=4096, intermediate_size=14336, num_hidden_layers=32, num_attention_heads=32,
@@ -83,7 +83,7 @@ class ClockSampler:
 
 def run_reference(args):
     """The unmodified reference cannot execute on B200: it imports neuronx_distributed / torch_neuronx /
-    neuronxcc (AWS Trainium compiler + runtime) at module import time.  See DESIGN.md "Reference arm"."""
+    neuronxcc (AWS Trainium compiler + runtime) at module import time."""
     why = "reference requires AWS Neuron SDK (neuronx_distributed, torch_neuronx, neuronxcc, libnrt) - no CUDA path"
     try:
         sys.path.insert(0, os.path.join(ROOT, "baseline", "_ref"))
@@ -466,7 +466,7 @@ def main():
             torch.cuda.empty_cache()
             tpg = pstate.get_tensor_model_parallel_group()
             tpg.symm = None
-            # the published 306 ms / 1665 tok/s were measured with output_logits=True (BASELINE.md): that is the headline
+            # the published 306 ms / 1665 tok/s were measured with output_logits=True: that is the headline
             # like-for-like block; the logits-off variant is reported next to it
             app4 = build_app(LLAMA31_8B_CI4, args.gpus, 2, 256, 128, async_mode=False, output_logits=True)
             ci = ci_harness(app4, 2, 128, 256, output_logits=True)

@@ -2,7 +2,7 @@
 //
 // Why: a decode layer is five dependent kernels (qkv -> attention -> o_proj(+all-reduce) -> gate_up -> down(+all-reduce)).  With
 // the weights sharded 8 ways a layer streams 55 MB (8 us of HBM time) but took ~38 us: every kernel boundary costs 5-6 us of
-// grid drain + dependency release + activation reload + ring refill (profiles/decode_r2.md, tools/prof_decode.py), and no
+// grid drain + dependency release + activation reload + ring refill (profiles/decode_step.md, tools/prof_decode.py), and no
 // amount of PDL overlap hides it because the next kernel cannot consume before its input exists.  Here one CTA per SM stays
 // resident for the whole step:
 //   * the TMA producer thread walks the phase list and streams the weights of EVERY projection of EVERY layer back to back
@@ -14,7 +14,7 @@
 //   * attention is a phase too (the same `attention_body` as the stand-alone kernel, run by warps 0-3 of the first
 //     B*Hkv*nsplit CTAs; those CTAs give the tail of their ring to the K/V tiles);
 //   * the tensor-parallel all-reduces stay fused in the o_proj / down epilogues (LL stores into every peer over NVLink).
-// Reference: the per-layer kernels this replaces are K2-K5 of SURVEY §2.3 (attention_block_tkg, fused QKV, o_proj + reduce,
+// Reference: the per-layer kernels this replaces are the decode kernels (attention_block_tkg, fused QKV, o_proj + reduce,
 // MLP) — the reference fuses WITHIN a block; on B200 the step itself is the unit.
 #include <algorithm>
 #include <stdexcept>

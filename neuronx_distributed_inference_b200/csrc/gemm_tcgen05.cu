@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tcgen05_kernel(const __gri
 
   if (warp == 0 || warp == 3) {
     // ================= TMA producers =================
-    // One issuing thread sustains ~one TMA instruction per 0.2 us (tools/bench_stream.cu); a k-block of 48 KB issued as three
+    // One issuing thread sustains ~one TMA instruction per 0.2 us; a k-block of 48 KB issued as three
     // instructions by ONE thread took 0.5 us while the tensor pipe needs 0.26 us for it.  So the two operands have their own
     // producer warp — warp 0 streams the WEIGHT tile (and starts before griddepcontrol.wait: weights do not depend on the previous
     // kernel), warp 3 the ACTIVATION tile (one 256-row box when TM = 2) — both post to the same full barrier.
@@ -674,7 +674,7 @@ static void gemm_launch_impl(const void* a, int lda, const void* b, const void* 
   if (M <= 4 * GM_BM) {
     // Weight-dominated sizes (M <= 512): a CTA is bound by its shared-memory fill rate (~100 GB/s per SM), so a tile costs
     // (TM*128 + BN) operand rows per k-block and the launch costs  waves x that  — pick the shape that minimises it (ties: the larger
-    // tile).  Measured (profiles/r2/skinny_gemm_sweep.txt): M = 256 qkv 51 -> 37 us with 128x128 instead of 128x64 tiles (192 tiles were
+    // tile).  Measured: M = 256 qkv 51 -> 37 us with 128x128 instead of 128x64 tiles (192 tiles were
     // two waves), o_proj best with 128x64 (one wave of 128 tiles).  Split-K only pays for very deep K with less than half the SMs
     // busy (down: 84 -> 68 us with two k slices); everywhere else the partial round trip costs more than it gains.
     const int n_out_ = glu ? N / 2 : N;

@@ -3,15 +3,12 @@
 //
 // Design:
 //   * ONE elected producer thread streams W with TMA tensor loads (cp.async.bulk.tensor.3d, completion on an
-//     mbarrier): W[N,K] is described as a 3-D tensor {64 k, K/64 groups, N rows}; one instruction fetches the box
-//     {64, 2, 16} = 16 weight rows x 128 k = 4 KB into a 128B-swizzled stage.
-//   * CO-RESIDENCY: the CTA is sized to <= ~108 KB of shared memory so that TWO consecutive decode kernels fit on an SM.
-//     Under programmatic dependent launch the NEXT kernel's producer then fills its ring (weights never depend on the
-//     previous kernel) while THIS kernel is still computing: HBM no longer idles for the ~5 us launch / wait / x-prologue /
-//     flush window between dependent GEMVs, which was what separated 3.17 ms/step from the 2.28 ms streaming floor at TP1 and
-//     dominated the step at TP4/TP8 (profiles/decode_overheads_r1.md).
-//   * 8 consumer warps; a stage always belongs to warp (stage & 7), so a warp meets its stages lap after lap in order and the
-//     mbarrier phase parity is unambiguous for ANY ring depth >= 8.  A-fragments of mma.sync m16n8k16 come straight from the
+//     mbarrier): W[N,K] is described as a 3-D tensor {64 k, N rows, K/64 groups}; one instruction fetches 16 weight rows x 512 k
+//     = 16 KB into a 128B-swizzled stage (8-bit weights: 1024 k; two boxes of 8 rows for gate and up).
+//   * the ring takes what it can of an SM's shared memory; under programmatic dependent launch the next kernel starts when this one
+//     leaves, or beside it where both are small (g2_two_ctas), and fills its ring: weights never depend on the kernel in front.  (Rings
+//     of at most 108 KB, so that two kernels always fit: 3.40 against 2.82 ms a step of an 8B model.)
+//   * 8 consumer warps; each takes its k group (64 k) of every stage, so it meets the stages in order.  A-fragments of mma.sync m16n8k16 come straight from the
 //     swizzled stage (8-lane LDS.128 phases are conflict free); the token fragments of X (gamma folded in, bf16) sit in shared
 //     memory; 1/rms is applied to the fp32 accumulators in the epilogue (single pass over x).
 //   * stream-K for large weights (equal bytes per SM, ticketed deterministic fix-up), whole 16-row tiles per CTA for small ones.
@@ -142,7 +139,7 @@ int g2_max_inflight() {
   static int v = -1;
   if (v < 0) {
     const char* e = getenv("NXDI_B200_GEMV_INFLIGHT");
-    v = e ? atoi(e) : 6;   // measured (profiles/decode_r2.md): TP1 2.94 ms/step uncapped -> 2.82 with 6 stages (96 KB) in flight
+    v = e ? atoi(e) : 6;   // measured (profiles/decode_step.md): TP1 2.94 ms/step uncapped -> 2.82 with 6 stages (96 KB) in flight
   }
   return v;
 }
@@ -220,9 +217,8 @@ void make_weight_tmap(CUtensorMap* tm, const void* w, int N, int K, int box_rows
   if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
 }
 
-// Ring depth.  Default budget G2_SMEM_CORES keeps the CTA small enough for TWO decode kernels per SM (see the header);
-// never deeper than the busiest CTA's unit count (a 2-tile CTA does not need 22 stages); at least 8 stages (one per warp).
-// If even 8 stages do not fit the co-residency budget (wide K x many tokens) the kernel takes what it needs up to 224 KB.
+// Ring depth: what the budget (G2_SMEM_CORES) leaves beside the rows, never deeper than the busiest CTA's unit count (a 2-tile CTA does not need 22 stages).  With fewer
+// than 3 stages (wide K x many tokens under a smaller budget) the kernel takes what it needs up to 224 KB.
 static int g2_pick_stages(const GemvParams& p, bool glu, bool whole) {
   static int budget_kb = -1;
   if (budget_kb < 0) {

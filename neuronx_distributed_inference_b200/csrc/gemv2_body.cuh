@@ -16,7 +16,7 @@ constexpr int G2_KC = 64 * G2_KG;                          // 512 k elements per
 constexpr int G2_STAGE_BYTES = 16 * G2_KC * 2;             // 16384: [8 k groups][16 rows][64 k], 128B-swizzled
 constexpr int G2_MAX_STAGES = 13;
 constexpr int G2_SMEM_BUDGET = 224 * 1024;   // hard cap (dynamic); leaves room for the few static __shared__ words
-constexpr int G2_SMEM_CORES = 224 * 1024;    // default ring budget.  Measured (profiles/decode_r2.md): one deep ring per SM (224 KB) beats
+constexpr int G2_SMEM_CORES = 224 * 1024;    // default ring budget.  Measured (profiles/decode_step.md): one deep ring per SM (224 KB) beats
                                              // two co-resident 108 KB CTAs at TP1 (3.17 vs 3.64 ms/step) and on TP8 shard shapes (1.22 vs 1.36)
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -151,7 +151,7 @@ __device__ __forceinline__ G2Units g2_units(const G2Phase& p, bool GLU, int c) {
 }
 
 // ---- producer: ONE thread streams this CTA's units of the phase through the ring ----
-// One issuing thread sustains one copy per ~150-230 ns whatever its size (tools/bench_stream.cu: 4 KB boxes 2.7 TB/s,
+// One issuing thread sustains one copy per ~150-230 ns whatever its size (4 KB boxes 2.7 TB/s,
 // 8 KB 5.4 TB/s, 16 KB 7.2 TB/s chip-wide): the stage is therefore ONE 16 KB box (two 8 KB boxes for GLU tiles).
 __device__ __forceinline__ void g2_produce(const G2Phase& p, const G2Smem& sm, const int c, int& stage, uint32_t& ph, int& issued) {
   const bool GLU = p.act != 0;
@@ -264,7 +264,7 @@ __device__ __forceinline__ void g2_consume(const G2Phase& p, const G2Symm& sy, c
   uint32_t ar_tag = 1u;
   if (MODE == 1) ar_tag = ll_tag(sy.step, p.call);
   // ---- X prologue: ONE bulk copy (TMA, cp.async.bulk) per token row brings the activations into shared memory — a single
-  //      request stream per CTA instead of 1024 scattered 16-byte loads (measured: 1-3.5 us -> see profiles/decode_r2.md).
+  //      request stream per CTA instead of 1024 scattered 16-byte loads (measured: 1-3.5 us -> see profiles/decode_step.md).
   //      With a fused RMSNorm the rows are then scaled by gamma IN PLACE (bf16); the per-token 1/rms is a scalar, so it is
   //      applied to the fp32 accumulators in the epilogue instead of to x.
   if (ctid == 0) {

@@ -10,7 +10,7 @@
 // Everything is sized by the static bound R = roundup128(N * k + E_local * 127): no host synchronisation, no data-dependent
 // launch shapes — the whole layer replays inside a CUDA graph whatever the router decides.  The reference gets the same effect
 // from its blockwise matmul over a padded token->block table (modules/moe_v2.py:25-133 and the blockwise kernels behind
-// ExpertMLPsV2, SURVEY §2.8); tokens of one expert are contiguous here so that one TMA box feeds one UMMA tile.
+// ExpertMLPsV2); tokens of one expert are contiguous here so that one TMA box feeds one UMMA tile.
 #include <stdexcept>
 
 #include "api.h"

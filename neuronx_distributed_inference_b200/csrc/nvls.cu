@@ -8,7 +8,7 @@
 // Every kernel brackets its data phase with a cross-GPU barrier on signal words of the heap: rank r stores the collective's tag
 // into slot [cta][r] of every peer (st.release.sys over the peer mapping) and spins on its own slots (ld.acquire.sys, bounded).
 // Reference call sites these replace: reduce_scatter / all_gather of models/model_base.py:1471-1583, all_reduce of the
-// row-parallel layers (SURVEY §2.4 P1, P2), mappings of the external parallel_layers package.
+// row-parallel layers, mappings of the external parallel_layers package.
 #include <stdexcept>
 #include <string>
 

@@ -40,6 +40,8 @@ __host__ __device__ constexpr int sk_epi(int wt) { return wt ? 8 : 16; }
 __host__ __device__ constexpr int sk_bk(int wt, bool wide) { return wt || wide ? 128 : SK_BK; }
 constexpr int SK_MAX_STAGES = 12;
 constexpr int SK_SMEM = 220 * 1024;
+// the warps that expand 8-bit weights count on as many stages as there are expanded boxes, for the largest blocks too (128 tokens; 64 beside two weight boxes)
+static_assert((SK_SMEM - 1024) / (SK_W_BYTES + SKINNY_MAX_T * 128 * 2) >= SK_A_BUFS && (SK_SMEM - 1024) / (2 * SK_W_BYTES + SKINNY_MAX_T / 2 * 128 * 2) >= SK_A_BUFS, "ring of 8-bit weights");
 
 struct SkinnyKernelParams {
   CUtensorMap tm_w;        // [experts * rows, K], box {64, 128} (bytes: {128, 128}); wide: as {64, rows, K / 64}, box {64, 128, 2}
@@ -570,7 +572,7 @@ void skinny_gemm_launch(const SkinnyGemm& a, cudaStream_t stream) {
   p.wait_word = wait_word(WAIT_SKINNY);
   count_launch(COUNT_SKINNY);
   const int stage = (glu || wide ? 2 : 1) * SK_W_BYTES + p.xb * sk_bk(a.wt, wide) * 2;
-  p.stages = std::min(SK_MAX_STAGES, (SK_SMEM - 1024) / stage);       // at least SK_A_BUFS: see the order of waits in the warps that expand 8-bit weights
+  p.stages = std::min(SK_MAX_STAGES, (SK_SMEM - 1024) / stage);       // (8-bit weights: at least SK_A_BUFS, asserted above)
   int cols = 32;
   while (cols < 2 * (glu ? 2 : 1) * p.xb + (a.wt ? SK_A_BUFS * SK_A_COLS : 0)) cols *= 2;
   p.tmem_cols = cols;

@@ -8,8 +8,8 @@
 // a kernel needs only (local base, peer bases[], multicast base).
 //
 // The file descriptors travel between the processes over Unix-domain sockets (SCM_RIGHTS) from Python
-// (parallel/symm_heap.py); this file owns the driver calls.  Reference: the Neuron runtime's collective buffers are opaque to
-// the reference; SURVEY §5.8 asks for the B200 equivalent (peer-mapped + multicast symmetric memory).
+// (parallel/symm_heap.py); this file owns the driver calls.  Reference: the Neuron runtime's collective buffers, opaque
+// there; peer-mapped and multicast symmetric memory here.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <unistd.h>

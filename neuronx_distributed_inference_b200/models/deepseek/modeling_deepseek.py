@@ -4,7 +4,7 @@ heads), sigmoid group-limited top-k router with a score-correction bias, routed 
 
 Attention here is the *decompressed* MLA formulation (K = [k_nope | k_rope], V per head in the cache), which is exact and
 matches Hugging Face; the weight-absorbed form that caches ``(k_pe, compressed_kv)`` (reference :79-326) is a memory
-optimisation of the same function and is tracked as follow-up work in DESIGN.md."""
+optimisation of the same function and is not built."""
 from __future__ import annotations
 
 import math

@@ -2,7 +2,7 @@
 sliding-window / full layers, biased q/k/v/o, YaRN RoPE, MoE with a biased router that soft-maxes over the
 selected top-k, clamped SwiGLU experts with biases (``(up+1) * gate*sigmoid(1.702*gate)``).
 MXFP4 expert checkpoints are de-quantised at load (``mx_layout_transform.py`` of the reference repacks them for the
-Neuron engines; on B200 the block-scaled path would feed ``tcgen05.mma.kind::mxf4`` — see DESIGN.md)."""
+Neuron engines; on B200 the block-scaled path would feed ``tcgen05.mma.kind::mxf4``)."""
 from __future__ import annotations
 
 import torch

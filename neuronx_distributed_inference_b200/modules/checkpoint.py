@@ -2,7 +2,7 @@
 
 reference: modules/checkpoint.py:24-285 (HF safetensors / sharded safetensors / .bin loading, sharded
 safetensors saving, ``create_n_layer_checkpoint``, ``prune_state_dict``) and the external
-``ModelBuilder.shard_checkpoint`` walk (SURVEY §3.5).  Sharding here is driven by per-parameter
+``ModelBuilder.shard_checkpoint`` walk.  Sharding here is driven by per-parameter
 metadata set by the parallel layers (``partition_dim``, ``partition_stride``, optional ``shard_fn``).
 """
 from __future__ import annotations

@@ -6,9 +6,8 @@ Use case: a projection whose WEIGHT is sharded (to save memory) but whose input 
 (the draft's ``fc`` feature-fusion layer during long prefills).  ``y = x @ all_gather(W_shard)^T`` is evaluated tile by tile along K so
 only one ``[out, tile]`` slab of the gathered weight is alive at a time and tile ``i+1``'s gather overlaps tile ``i``'s GEMM.
 
-On B200 the decode path does not use this (a 2H x H weight is 64 MB for an 8B model and is simply replicated — DESIGN.md §8); the
-prefill path can, when ``weight_gather_seq_len_threshold`` is set.  The collective is NCCL all-gather on a side stream; the fused
-single-kernel AG->GEMM is a round-2 item."""
+On B200 the decode path does not use this (a 2H x H weight is 64 MB for an 8B model and is simply replicated); the
+prefill path can, when ``weight_gather_seq_len_threshold`` is set.  The collective is NCCL all-gather on a side stream."""
 from __future__ import annotations
 
 from typing import Optional

@@ -1,7 +1,6 @@
 """Mixture-of-experts block: router + routed experts (+ shared experts), tensor- and expert-parallel.
 
-Rebuild of the external ``neuronx_distributed.modules.moe`` surface used by the reference (SURVEY §2.10:
-``RouterTopK``, ``ExpertMLPs(V2)``, ``SharedExperts``, ``MoE``; glue in modules/moe.py:6-45, moe_v2.py:23-161).
+Rebuild of the external ``neuronx_distributed.modules.moe`` surface used by the reference (``RouterTopK``, ``ExpertMLPs(V2)``, ``SharedExperts``, ``MoE``; glue in modules/moe.py:6-45, moe_v2.py:23-161).
 
 Parallel layout on B200 (one NVSwitch domain, activations replicated across the TP group as in every TP decoder):
   * experts are split over ``moe_ep`` groups (contiguous ownership), each expert's intermediate dim over ``moe_tp``;

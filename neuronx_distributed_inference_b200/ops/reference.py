@@ -312,7 +312,7 @@ def identity_expert_add(y, x, topk_w, topk_i, num_experts: int):
 def moe_experts(x, w_gate_up, w_down, topk_w, topk_i, act: str = "silu_mul", expert_offset: int = 0,
                 gate_up_bias=None, down_bias=None, act_fn=None, scale_input: bool = False, gate_up_scale=None, down_scale=None, act_params=None):
     """Dropless expert MLPs.  x [N,H]; w_gate_up [E_local, 2I, H] ([gate; up] rows, K-major like nn.Linear — the
-    reference stores [E,H,2I], SURVEY §2.8; K-major is what TMA/UMMA and the GEMV kernels stream); w_down
+    reference stores [E,H,2I]; K-major is what TMA/UMMA and the GEMV kernels stream); w_down
     [E_local, H, I]; experts owned here are [expert_offset, expert_offset+E_local).
     -> partial output [N,H] (sum over owned experts; all-reduce across expert/tensor shards outside).  ``act = "clamped_glu"``: the
     product of :func:`clamped_glu` with ``act_params = (limit, alpha)``."""

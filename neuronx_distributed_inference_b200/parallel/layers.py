@@ -1,7 +1,7 @@
 """Tensor-parallel layers: ColumnParallelLinear / RowParallelLinear / ParallelEmbedding.
 
 Inferred API of the external ``neuronx_distributed.parallel_layers`` package that every model
-of the reference is wired with (SURVEY §2.10; call sites modeling_llama.py:354-387,1112-1133,
+of the reference is wired with (call sites modeling_llama.py:354-387,1112-1133,
 gqa.py:411-467,998-1010).  B200 design: each process owns its shard as a plain ``nn.Parameter``
 in ``nn.Linear`` layout ``[out, in]``; forward runs
 

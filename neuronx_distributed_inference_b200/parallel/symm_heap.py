@@ -15,7 +15,7 @@ Collectives (bf16, prefill-sized; the decode-sized all-reduce is fused into the 
     all_reduce      two-shot in-switch: rank r pulls the reduced slice r and multicasts it
     reduce_scatter  rank r pulls its reduced slice (sequence-parallel row-parallel layers), residual add fused
     all_gather      rank r multicasts its slice
-reference: the collectives of the external ``neuronx_distributed.parallel_layers.mappings`` (SURVEY §2.4 P1/P2, §5.8).
+reference: the collectives of the external ``neuronx_distributed.parallel_layers.mappings``.
 """
 from __future__ import annotations
 

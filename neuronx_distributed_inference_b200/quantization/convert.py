@@ -1,6 +1,6 @@
 """Weight quantisation: offline checkpoint generation + module conversion.
 
-Rebuild of the external ``neuronx_distributed.quantization`` surface the reference drives (SURVEY §2.7):
+Rebuild of the external ``neuronx_distributed.quantization`` surface the reference drives:
 ``quantize_pytorch_model_per_{tensor,channel}_symmetric`` + ``prepare_quantized_state_dict`` (application_base.py:746-799)
 and ``convert(model, q_config, modules_to_not_convert)`` swapping parallel linears for quantised ones holding
 ``weight`` (int8 / fp8) + ``scale`` (fp32, never down-cast; model_wrapper.py:1477-1529).

@@ -7,8 +7,8 @@ step (residual stream ping-pong, qkv, attention output, MLP activation) and the 
                 h1  = W_o · attn (+all-reduce) + h      ->  u = swiglu(W_gu · rmsnorm(h1))      ->  h = W_d · u (+all-reduce) + h1
 
 Eligibility (`eligible`) mirrors the conditions of the per-kernel fast path (modules/attention/attention_base.py) for dense
-Llama-style blocks; everything else keeps the layer-by-layer path.  Reference: the reference fuses within a block (SURVEY §2.3
-K2-K5: attention_block_tkg, fused QKV, MLP kernels); on B200 the whole step is one resident kernel.
+Llama-style blocks; everything else keeps the layer-by-layer path.  Reference: the reference fuses within a block
+(attention_block_tkg, fused QKV, MLP kernels); on B200 the whole step is one resident kernel.
 """
 from __future__ import annotations
 
@@ -20,7 +20,7 @@ import torch
 from .. import ops
 
 # Opt-in: correct (tests/test_features_gpu.py) but measured SLOWER than the per-kernel path on B200 so far (Llama-3.1-8B bs 2:
-# 4.27 vs 2.82 ms/step at TP1, 1.57 vs 1.15 ms on TP8 shard shapes — profiles/decode_r2.md has the phase timeline and the analysis).
+# 4.27 vs 2.82 ms/step at TP1, 1.57 vs 1.15 ms on TP8 shard shapes — profiles/decode_step.md has the phase timeline and the analysis).
 _ENABLED = os.environ.get("NXDI_B200_DECODE_STEP", "0") == "1"
 
 

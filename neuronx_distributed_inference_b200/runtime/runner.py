@@ -2,7 +2,7 @@
 CUDA-graph replay.
 
 Role of reference ``ModelWrapper`` (models/model_wrapper.py:50-1440) + ``ModelBuilder``/``NxDModel``
-routing (SURVEY §2.10).  What remains of it on B200:
+routing.  What remains of it on B200:
 * a *bucket* is a CUDA-graph key ``(batch bucket, seq bucket, n_active)``; kernels read real
   lengths from device memory so no attention masks are padded or shipped;
 * batch rows are never sorted by ``seq_ids`` (kernels index cache lines directly); short batches

@@ -116,7 +116,7 @@ def test_llama4_fp8_checkpoint_expert_fusion():
 
 @pytest.mark.parametrize("qdtype", ["int8", "f8e4m3"])
 def test_mixtral_expert_wise_quantized_checkpoint_flow(qdtype, tmp_path):
-    """``expert_wise_per_channel_symmetric`` (SURVEY §2.7): the MoE expert banks are stored 8-bit with one scale per expert and output
+    """``expert_wise_per_channel_symmetric``: the MoE expert banks are stored 8-bit with one scale per expert and output
     channel, attention projections per channel; the quantised model tracks the fp32 one."""
     from transformers import MixtralConfig
     from neuronx_distributed_inference_b200.models.mixtral.modeling_mixtral import NeuronMixtralForCausalLM as A

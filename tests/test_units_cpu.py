@@ -1,5 +1,5 @@
 """Unit tests of the host-side logic (config validation, bucketing, GQA plans, sampling, checkpoint I/O, CLI parsing) —
-the CPU tier of the reference's test strategy (SURVEY §4: test/unit/**)."""
+the CPU tier of the reference's test strategy (test/unit/**)."""
 import json
 import os
 

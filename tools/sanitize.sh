@@ -1,5 +1,5 @@
 #!/usr/bin/env bash
-# compute-sanitizer targets for the hand-written kernels (SURVEY §5.2: the reference has no race tooling; every kernel here
+# compute-sanitizer targets for the hand-written kernels (the reference has no race tooling; every kernel here
 # that synchronises through shared memory, mbarriers, tickets or peer flags gets a memcheck / racecheck / synccheck pass).
 # Usage on a GPU box:  tools/sanitize.sh [memcheck|racecheck|synccheck|initcheck] [pytest -k expression]
 set -euo pipefail
