@@ -890,21 +890,33 @@ namespace nxdi {
 std::tuple<at::Tensor, at::Tensor> rmsnorm_quant(const at::Tensor& x, const c10::optional<at::Tensor>& gamma, double eps, double offset,
                                                  double clamp) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.is_contiguous() && is_bf16(x));
-  if (gamma.has_value()) TORCH_CHECK(is_bf16(*gamma) && gamma->numel() == x.size(1));
+  c10::optional<at::Tensor> g;
+  if (gamma.has_value()) {
+    g = gamma->contiguous();
+    check_norm_weight(*g, x.size(1));
+  }
   c10::cuda::CUDAGuard guard(x.device());
   auto q = at::empty(x.sizes(), x.options().dtype(at::kFloat8_e4m3fn));
   auto scale = at::empty({x.size(0)}, x.options().dtype(at::kFloat));
-  rmsnorm_quant_launch(x.data_ptr(), optr(gamma), q.data_ptr(), scale.data_ptr<float>(), (int)x.size(0), (int)x.size(1), (float)eps,
+  rmsnorm_quant_launch(x.data_ptr(), optr(g), q.data_ptr(), scale.data_ptr<float>(), (int)x.size(0), (int)x.size(1), (float)eps,
                        (float)offset, (float)clamp, cur_stream());
   return {q, scale};
 }
-at::Tensor gemm_fp8(const at::Tensor& xq, const at::Tensor& a_scale, const at::Tensor& w, const at::Tensor& w_scale,
-                    const c10::optional<at::Tensor>& bias, int64_t act, const c10::optional<at::Tensor>& residual) {
+at::Tensor gemm_fp8(const at::Tensor& xq, const at::Tensor& a_scale, const at::Tensor& w, const at::Tensor& w_scale_in,
+                    const c10::optional<at::Tensor>& bias_in, int64_t act, const c10::optional<at::Tensor>& residual) {
   TORCH_CHECK(xq.is_cuda() && xq.dim() == 2 && xq.is_contiguous() && xq.scalar_type() == at::kFloat8_e4m3fn);
   TORCH_CHECK(w.dim() == 2 && w.is_contiguous() && w.scalar_type() == at::kFloat8_e4m3fn && w.size(1) == xq.size(1));
   const int M = xq.size(0), K = xq.size(1), N = w.size(0);
-  TORCH_CHECK(K % 128 == 0 && a_scale.scalar_type() == at::kFloat && a_scale.numel() == M && w_scale.scalar_type() == at::kFloat &&
-              (w_scale.numel() == 1 || w_scale.numel() == N) && a_scale.is_contiguous() && w_scale.is_contiguous());
+  TORCH_CHECK(K % 128 == 0 && a_scale.scalar_type() == at::kFloat && a_scale.numel() == M && w_scale_in.scalar_type() == at::kFloat &&
+              (w_scale_in.numel() == 1 || w_scale_in.numel() == N) && a_scale.is_contiguous() && w_scale_in.is_contiguous());
+  TORCH_CHECK(w.is_cuda() && a_scale.is_cuda() && w_scale_in.is_cuda(), "gemm_fp8: weights and scales on the GPU expected");
+  // (the kernel loads four scales at a time: those of a slice are copied)
+  const at::Tensor w_scale = reinterpret_cast<uintptr_t>(w_scale_in.data_ptr()) % 16 == 0 ? w_scale_in : w_scale_in.clone();
+  c10::optional<at::Tensor> bias;
+  if (bias_in.has_value()) {
+    TORCH_CHECK(bias_in->is_cuda() && is_bf16(*bias_in) && bias_in->numel() == N, "gemm_fp8: a bias of ", N, " bf16 values on the GPU expected");
+    bias = bias_in->contiguous();
+  }
   const bool glu = act != 0;
   const int n_out = glu ? N / 2 : N;
   TORCH_CHECK(n_out % 8 == 0);

@@ -64,3 +64,24 @@ def test_scale_in_host_memory(wdtype, T):
     x, q, s, _, _, _ = _layer(T, 136, 512, wdtype)
     with pytest.raises(RuntimeError):
         ops.linear(x, q, scale=s.cpu())
+
+
+def test_fp8_rows_and_weights(monkeypatch):
+    """W8A8: strided norm weights and biases count as their dense copies, scales may be a slice; other types and lengths are refused."""
+    monkeypatch.setattr(ops, "_ACT_QUANT", True)
+    x, q, s, n, _, _ = _layer(20, 136, 512, torch.float8_e4m3fn)
+    n2, b2 = torch.randn(512, 2, device=DEV).to(BF)[:, 0], torch.randn(136, 2, device=DEV).to(BF)[:, 0]
+    want = ops.linear(x, q, b2.contiguous(), norm_weight=n2.contiguous(), scale=s)
+    assert torch.equal(ops.linear(x, q, b2, norm_weight=n2, scale=s), want)
+    assert torch.equal(ops.linear(x, q, b2, norm_weight=n2, scale=torch.cat([s[:1], s])[1:]), want)
+    for kw in (dict(bias=b2.float()), dict(bias=b2[:64].contiguous()), dict(norm_weight=n2[:64].contiguous())):
+        with pytest.raises(RuntimeError):
+            ops.linear(x, q, scale=s, **kw)
+
+
+@pytest.mark.parametrize("wdtype", TYPES[1:])
+@pytest.mark.parametrize("T,N,K", [(20, 136, 512), (100, 512, 512), (300, 8192, 512), (200, 1024, 1024)])
+def test_scales_of_a_slice(wdtype, T, N, K):
+    """Scales that start off a 16-byte boundary, through every kernel that loads several at a time (the last size: a split K)."""
+    x, q, s, _, _, w = _layer(T, N, K, wdtype)
+    assert _rel(ops.linear(x, q, scale=torch.cat([s[:1], s])[1:]), x.double() @ w.t()) < 3e-3
